@@ -1,5 +1,7 @@
-"""ctypes binding of libhyc.so.  One entry per declaration of include/hyc.h."""
+"""ctypes binding of libhyc.so (one entry per declaration of include/hyc.h) and the native host path ``host``
+(csrc/host), which the operators call: it checks arguments, allocates and launches without Python in between."""
 import ctypes
+import importlib.util
 import os
 import threading
 
@@ -13,7 +15,16 @@ if not os.path.exists(LIB_PATH):
         "libhyc.so is not built (%s). Build it with `python hyc_lora_release_b200/build.py`; "
         "there is no fallback implementation." % LIB_PATH)
 
+HOST_PATH = os.path.join(_HERE, "lib", "_hyc_host.so")
+if not os.path.exists(HOST_PATH):
+    raise ImportError(
+        "_hyc_host.so is not built (%s). Build it with `python hyc_lora_release_b200/build.py`; "
+        "there is no fallback implementation." % HOST_PATH)
+
 _cdll = ctypes.CDLL(LIB_PATH)
+_spec = importlib.util.spec_from_file_location("_hyc_host", HOST_PATH)
+host = importlib.util.module_from_spec(_spec)
+_spec.loader.exec_module(host)
 
 _p, _i, _l, _f, _z = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_float, ctypes.c_size_t
 
@@ -92,8 +103,7 @@ class _DeviceGuardedLibrary:
 lib = _DeviceGuardedLibrary()
 
 
-class HycError(RuntimeError):
-    pass
+HycError = host.HycError           # a RuntimeError; raised by both paths
 
 
 def check(code, what):

@@ -25,12 +25,12 @@ from typing import Optional
 
 import torch
 
-from ._lib import require_cuda
-from .mlp import _status_tensor, gemm, linear_lora_save, lora_a_products, lora_grad_a, padded_block
+from ._lib import host, require_cuda
+from .mlp import _status_tensor, gemm, linear_lora_save, lora_a_products, padded_block
 from .operators import compress_function as cf
-from .operators.rmsnorm_kernels import rmsnorm_backward_packed, rmsnorm_forward, rmsnorm_forward_save
+from .operators.rmsnorm_kernels import rmsnorm_forward, rmsnorm_forward_save
 from .operators.rope_kernels import rope_inplace
-from .operators.softmax_kernels import softmax_backward, softmax_forward_scale_mask, softmax_forward_topk_save
+from .operators.softmax_kernels import softmax_forward_scale_mask, softmax_forward_topk_save
 
 BF16 = torch.bfloat16
 
@@ -120,22 +120,9 @@ def _repeat_kv(x, n_rep):
     return x[:, :, None].expand(b, n, n_rep, m, d).reshape(b, n * n_rep, m, d)
 
 
-def _repeat_kv_backward(g, n_rep):
-    if n_rep == 1:
-        return g
-    b, n, m, d = g.shape
-    return g.reshape(b, n // n_rep, n_rep, m, d).sum(dim=2)
-
-
 def _heads(x2, B, M, n):
     """[B*M, n*d] (contiguous) -> [B, n, M, d] view."""
     return x2.view(B, M, n, -1).transpose(1, 2)
-
-
-def _hidden(xh):
-    """[B, n, M, d] -> contiguous [B*M, n*d]."""
-    b, n, m, d = xh.shape
-    return xh.transpose(1, 2).reshape(b * m, n * d)
 
 
 def _matmul_to_hidden(a4, b4, out=None):
@@ -172,11 +159,54 @@ def attention_forward(x, w: AttnWeights, state: AttnState, cos, sin, attention_m
                       num_key_value_heads, eps=1e-5, status=None):
     """-> (x_medium [B,M,H], saved dict).  Advances the calibration state like the layer does."""
     require_cuda(x)
+    q = state.q_bit
+    st = status if status is not None else _status_tensor(x.device)
+    it, sv = state.iteration, state.static_value
+    if state.map_mode not in ("topk", "prune"):
+        raise ValueError("map_mode must be 'topk' or 'prune'")
+    calib = it < state.iteration_threshold
+    if calib or any(b is not None for b in (w.bias_q, w.bias_k, w.bias_v)) or (state.map_mode == "topk" and state.fuse_softmax_with_save):
+        out = _attention_forward_stepwise(x, w, state, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, eps, st, calib)
+        state.iteration += 1
+        return out
+    # steady state: two calls into the native host path around the save of the probability map
+    B, M, H = x.shape
+    pad = w.padded()
+    xs, xn_scale = sv['x'], sv['x_norm_1']['scale']
+    a, o2, rstd, x_o, x_q, xn_q, q_q, k_q, v_q, xa3 = host.attn_forward_map(
+        x, [w.norm_w, w.wq, w.wk, w.wv, w.bq, w.bk, w.bv, pad["aqkv_t"]],
+        [xs['outlier_channel_index'], xs['scale'], xn_scale, sv['q']['scale'], sv['k']['scale'], sv['v']['scale']],
+        cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, q, eps, st)
+    a_saved = _save_map(a, state)
+    a_shape = tuple(a.shape)
+    del a
+    x_medium, o_q, o_xa64 = host.attn_forward_out(x, o2, w.wo, pad["ao_cols"], pad["bo_cols"], sv['o']['scale'], w.bias_o, q, st)
+    state.iteration += 1
+    saved = dict(rstd=rstd, x_o=x_o, x_q=x_q, x_scale=xs['scale'], x_idx=xs['outlier_channel_index'], xn_q=xn_q, xn_scale=xn_scale,
+                 q_q=q_q, q_scale=sv['q']['scale'], k_q=k_q, k_scale=sv['k']['scale'], v_q=v_q, v_scale=sv['v']['scale'],
+                 q_xa=xa3[0], k_xa=xa3[1], v_xa=xa3[2], qkv_xa=xa3, a_saved=a_saved, a_shape=a_shape, map_mode=state.map_mode,
+                 o_q=o_q, o_scale=sv['o']['scale'], o_xa=o_xa64[:, :w.ao.shape[0]], q_bit=q, shape=(B, M, H),
+                 cos=cos, sin=sin, num_heads=num_heads, head_dim=head_dim, num_key_value_heads=num_key_value_heads)
+    return x_medium, saved
+
+
+def _save_map(a, state):
+    """The saved form of the probability map in steady state."""
+    if state.map_mode == "topk":
+        return cf.compression_softmax_topk(a, state.softmax_outlier_ratio, state.map_q_bit)
+    # the calibrated threshold as a host number (read once), fixed-capacity buffers and the count left on the device
+    # -> no host synchronisation in the step
+    if state.threshold_host is None:
+        state.threshold_host = float(state.static_value['a']['outlier'])
+    return cf.compression_softmax_static(a, state.threshold_host, ratio=state.softmax_outlier_ratio, margin=state.prune_capacity_margin)
+
+
+def _attention_forward_stepwise(x, w, state, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, eps, st, calib):
+    """Calibration iterations (every save takes its statistics from the finished tensor), projections with a bias, and
+    the softmax fused with the save: the same steps as separate operators."""
     B, M, H = x.shape
     T, q = B * M, state.q_bit
-    st = status if status is not None else _status_tensor(x.device)
     it, thd = state.iteration, state.iteration_threshold
-    calib = it < thd
     sv = state.static_value
     n_rep = num_heads // num_key_value_heads
 
@@ -202,32 +232,18 @@ def attention_forward(x, w: AttnWeights, state: AttnState, cos, sin, attention_m
     kh = _repeat_kv(_heads(ky, B, M, num_key_value_heads), n_rep)
     vh = _repeat_kv(_heads(vy, B, M, num_key_value_heads), n_rep)
     scores = torch.matmul(qh, kh.transpose(-2, -1))
+    a_thr = a_saved = None
     if state.map_mode == "topk" and state.fuse_softmax_with_save:
         # scale + mask + softmax and the save of the map in one pass over the scores
         a, a_saved = softmax_forward_topk_save(scores, 1.0 / math.sqrt(head_dim), attention_mask,
                                                state.softmax_outlier_ratio, state.map_q_bit, inplace=True)
     else:
         a = softmax_forward_scale_mask(scores, 1.0 / math.sqrt(head_dim), attention_mask, inplace=True)
-        a_saved = None
     del scores
-
-    if state.map_mode == "topk":
-        if a_saved is None:
-            a_saved = cf.compression_softmax_topk(a, state.softmax_outlier_ratio, state.map_q_bit)
-        a_thr = None
-    elif state.map_mode == "prune":
-        if calib:
-            a_saved, a_thr = cf.compression_pack_softmax_base(a, state.softmax_outlier_ratio, it, thd, sv['a'])
-        else:
-            # steady state: the calibrated threshold as a host number (read once), fixed-capacity buffers and the
-            # count left on the device -> no host synchronisation in the step
-            if state.threshold_host is None:
-                state.threshold_host = float(sv['a']['outlier'])
-            a_thr = None
-            a_saved = cf.compression_softmax_static(a, state.threshold_host, ratio=state.softmax_outlier_ratio,
-                                                    margin=state.prune_capacity_margin)
-    else:
-        raise ValueError("map_mode must be 'topk' or 'prune'")
+    if state.map_mode == "prune" and calib:
+        a_saved, a_thr = cf.compression_pack_softmax_base(a, state.softmax_outlier_ratio, it, thd, sv['a'])
+    elif a_saved is None:
+        a_saved = _save_map(a, state)
     o2 = _matmul_to_hidden(a, vh)
     a_shape = tuple(a.shape)
     del a
@@ -248,7 +264,6 @@ def attention_forward(x, w: AttnWeights, state: AttnState, cos, sin, attention_m
         if a_thr is not None:
             sv['a'] = cf.update_dict(sv['a'], {'outlier': a_thr}, it)
         sv['o'] = cf.update_dict(sv['o'], {'scale': o_scale}, it)
-    state.iteration += 1
 
     saved = dict(rstd=rstd, x_o=x_o, x_q=x_q, x_scale=x_scale, x_idx=x_idx, xn_q=xn_q, xn_scale=xn_scale,
                  q_q=q_q, q_scale=q_scale, k_q=k_q, k_scale=k_scale, v_q=v_q, v_scale=v_scale,
@@ -258,16 +273,6 @@ def attention_forward(x, w: AttnWeights, state: AttnState, cos, sin, attention_m
     return x_medium.reshape(B, M, H), saved
 
 
-def _rebuild(codes, scale, xa, b, q_bit):
-    """De-quantized main branch + LoRA product of a projection, [T, N] (b = lora_B.weight [N, r])."""
-    T = codes.shape[0]
-    return cf.decompression_dequantization_lora_add(codes.view(1, T, -1), scale, xa.view(1, T, -1), b.t(), q_bit).view(T, -1)
-
-
-def _vec(s):
-    return s.to(BF16).reshape(-1).contiguous()
-
-
 def attention_backward(grad_medium, saved, w: AttnWeights, status=None, on_lora_grads=None):
     """-> dict(grad_x, grad_aq, grad_bq, grad_ak, grad_bk, grad_av, grad_bv, grad_ao, grad_bo), the LoRA
     gradients in the layout of the weights they belong to ([r, in] / [out, r]).  ``on_lora_grads(dict)`` is
@@ -275,92 +280,38 @@ def attention_backward(grad_medium, saved, w: AttnWeights, status=None, on_lora_
     B, M, H = saved['shape']
     T, q = B * M, saved['q_bit']
     nh, d, nkv = saved['num_heads'], saved['head_dim'], saved['num_key_value_heads']
-    n_rep = nh // nkv
-    cos, sin = saved['cos'], saved['sin']
     dev = grad_medium.device
     st = status if status is not None else _status_tensor(dev)
     g = grad_medium.to(BF16).reshape(T, H).contiguous()
     pad = w.padded()
-    r = w.ao.shape[0]
 
-    # ---- o projection
-    gm64 = g @ pad["bo_cols"]                                # [T, 64]; first r columns = g @ Bo
-    grad_bo = g.t() @ saved['o_xa']                          # [H, r]
-    grad_ao = lora_grad_a(saved['o_q'], _vec(saved['o_scale']), gm64, 16, q)[:r]     # [r, heads*d], o de-quantized in the kernel
-    grad_o2 = gemm(g, w.wo, b_is_kn=True, a2=gm64, b2=pad["ao_rows"], status=st)      # [T, heads*d]
-    grad_oh = _heads(grad_o2, B, M, nh)
-
-    # ---- P.V backward on the restored map
-    m = saved['a_saved']
+    # ---- o projection (the LoRA-A gradient de-quantizes o inside its kernel)
+    grad_bo, grad_ao, grad_o2 = host.attn_backward_out(g, w.wo, pad["bo_cols"], pad["ao_rows"], saved['o_xa'], saved['o_q'],
+                                                       saved['o_scale'], q, st)
+    # ---- the map: P.V backward, softmax backward (for the top-k form fused with a second restore: the map is not
+    # re-read), scores backward with q, k rebuilt from their codes
+    m, topk, map_q = saved['a_saved'], [], 0
     if saved['map_mode'] == "topk":
-        a = m.to_dense()
+        a, topk, map_q = m.to_dense(), list(m.tensors()), m.q_bit
     else:
         a = m.to_dense().reshape(saved['a_shape']) if isinstance(m, (cf.PrunedMap, cf.TiledPrunedMap)) else \
             cf.decompression_softmax(m).reshape(saved['a_shape'])
-    v2 = _rebuild(saved['v_q'], saved['v_scale'], saved['v_xa'], w.bv, q)
-    vh = _repeat_kv(_heads(v2, B, M, nkv), n_rep)
-    # without grouped key/value heads grad_q, grad_k and grad_v have one shape: kept in one buffer, their rank-16
-    # products below run as one batched library call each
-    gqkv = torch.empty((3, T, nh * d), dtype=BF16, device=dev) if n_rep == 1 else None
-    if n_rep == 1:
-        grad_v = _matmul_to_hidden(a.transpose(-2, -1), grad_oh, out=gqkv[2])
-    else:
-        grad_v = _hidden(_repeat_kv_backward(torch.matmul(a.transpose(-2, -1), grad_oh), n_rep))
-    grad_a = torch.matmul(grad_oh, vh.transpose(-2, -1))
-    del vh, v2
-    # ---- softmax backward (for the top-k form fused with a second restore: the map is not re-read)
-    if saved['map_mode'] == "topk":
-        del a
-        grad_s = m.softmax_backward(grad_a, scale=1.0 / math.sqrt(d))
-        del grad_a
-    else:
-        grad_s = softmax_backward(a, grad_a, scale=1.0 / math.sqrt(d))
-        del a
-
-    # ---- q, k rebuilt from their codes, rotary re-applied
-    q2 = _rebuild(saved['q_q'], saved['q_scale'], saved['q_xa'], w.bq, q)
-    rope_inplace(q2.view(B, M, nh, d), cos, sin)
-    if n_rep == 1:
-        grad_k = _matmul_to_hidden(grad_s.transpose(-2, -1), _heads(q2, B, M, nh), out=gqkv[1])
-    else:
-        grad_k = _hidden(_repeat_kv_backward(torch.matmul(grad_s.transpose(-2, -1), _heads(q2, B, M, nh)), n_rep))
-    del q2
-    k2 = _rebuild(saved['k_q'], saved['k_scale'], saved['k_xa'], w.bk, q)
-    rope_inplace(k2.view(B, M, nkv, d), cos, sin)
-    grad_q = _matmul_to_hidden(grad_s, _repeat_kv(_heads(k2, B, M, nkv), n_rep), out=None if gqkv is None else gqkv[0])
-    del k2, grad_s
-    rope_inplace(grad_q.view(B, M, nh, d), cos, sin, backward=True)
-    rope_inplace(grad_k.view(B, M, nkv, d), cos, sin, backward=True)
+    grad_q, grad_k, grad_v, gqkv = host.attn_backward_map(
+        grad_o2, a, topk, map_q, [saved[n] for n in ('q_q', 'q_scale', 'q_xa', 'k_q', 'k_scale', 'k_xa', 'v_q', 'v_scale', 'v_xa')],
+        [w.bq, w.bk, w.bv], saved['cos'], saved['sin'], B, M, nh, d, nkv, q)
+    del a, grad_o2
 
     # ---- q/k/v projections: LoRA gradients, then grad_x_norm as one GEMM over the three K segments
     gmq = padded_block(w, "_gmq", T, dev)                    # g_q @ Bq | g_k @ Bk | g_v @ Bv side by side
     qkv_xa = saved.get('qkv_xa')
-    if gqkv is not None and r == 16:
-        # (B200, 2048 tokens: 11.5 us against 25.6 us as three products, 9.9 us against 19.7 us for the B gradients)
-        gmq.view(T, 4, 16)[:, :3].copy_(torch.bmm(gqkv, pad["bqkv"]).transpose(0, 1))
-        if qkv_xa is None:
-            qkv_xa = torch.stack((saved['q_xa'], saved['k_xa'], saved['v_xa']))
-        grad_b3 = torch.bmm(gqkv.transpose(1, 2), qkv_xa)     # [3, heads*d, r]
-    else:
-        torch.mm(grad_q, w.bq, out=gmq[:, :r])
-        torch.mm(grad_k, w.bk, out=gmq[:, r:2 * r])
-        torch.mm(grad_v, w.bv, out=gmq[:, 2 * r:3 * r])
-        grad_b3 = None
-    ga = lora_grad_a(saved['xn_q'].reshape(T, -1), _vec(saved['xn_scale']), gmq, 48, q)
-    grad_aq, grad_ak, grad_av = ga[:r], ga[r:2 * r], ga[2 * r:3 * r]
-    if grad_b3 is not None:
-        grad_bq, grad_bk, grad_bv = grad_b3[0], grad_b3[1], grad_b3[2]
-    else:
-        grad_bq = grad_q.t() @ saved['q_xa']
-        grad_bk = grad_k.t() @ saved['k_xa']
-        grad_bv = grad_v.t() @ saved['v_xa']
+    if qkv_xa is None:
+        qkv_xa = torch.stack((saved['q_xa'], saved['k_xa'], saved['v_xa']))
+    ga, grad_bq, grad_bk, grad_bv = host.attn_backward_lora([grad_q, grad_k, grad_v], gqkv, gmq, pad["bqkv"], [w.bq, w.bk, w.bv],
+                                                            qkv_xa, saved['xn_q'], saved['xn_scale'], q)
+    grads = dict(grad_aq=ga[:16], grad_bq=grad_bq, grad_ak=ga[16:32], grad_bk=grad_bk, grad_av=ga[32:48], grad_bv=grad_bv,
+                 grad_ao=grad_ao, grad_bo=grad_bo)
     if on_lora_grads is not None:
-        on_lora_grads(dict(grad_aq=grad_aq, grad_bq=grad_bq, grad_ak=grad_ak, grad_bk=grad_bk, grad_av=grad_av,
-                           grad_bv=grad_bv, grad_ao=grad_ao, grad_bo=grad_bo))
-    lora_x = gmq @ pad["aqkv_rows"]                          # [T, H]: the three LoRA-A back-projections
-    grad_xn = gemm(grad_q, w.wq, b_is_kn=True, a2=grad_k, b2=w.wk, a3=grad_v, b3=w.wv, residual=lora_x, status=st)
-    grad_x = rmsnorm_backward_packed(grad_xn.reshape(B, M, H), saved['x_q'], saved['x_scale'], saved['x_o'],
-                                     saved['x_idx'], w.norm_w, saved['rstd'], q, residual_grad=g.reshape(B, M, H))
-    return dict(grad_x=grad_x, grad_aq=grad_aq, grad_bq=grad_bq, grad_ak=grad_ak, grad_bk=grad_bk,
-                grad_av=grad_av, grad_bv=grad_bv, grad_ao=grad_ao, grad_bo=grad_bo,
-                grad_q=grad_q, grad_k=grad_k, grad_v=grad_v)
+        on_lora_grads(dict(grads))
+    grad_x = host.attn_backward_x(g, [grad_q, grad_k, grad_v], gmq, [w.wq, w.wk, w.wv, pad["aqkv_rows"], w.norm_w],
+                                  [saved['x_q'], saved['x_scale'], saved['x_o'], saved['x_idx'], saved['rstd']], [B, M, H], q, st)
+    return dict(grads, grad_x=grad_x, grad_q=grad_q, grad_k=grad_k, grad_v=grad_v)

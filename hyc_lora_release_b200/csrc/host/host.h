@@ -1,0 +1,83 @@
+// Native host path: the operator wrappers of this package on at::Tensor, so that a call costs its launches and
+// little else.  The same work in Python (argument checks, allocations, ctypes marshalling) cost 10-15 us per
+// launch, more than most kernels of a short sequence run for.
+#pragma once
+#include <torch/extension.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <initializer_list>
+#include <optional>
+#include <stdexcept>
+#include <string>
+#include <vector>
+#include "../../../include/hyc.h"
+
+namespace hyc_host {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+struct Error : std::runtime_error { using std::runtime_error::runtime_error; };
+void check(int rc, const char* what);
+
+// makes the device of `t` current for the scope and hands out torch's current stream there
+struct OnDevice {
+  c10::cuda::CUDAGuard guard;
+  void* stream;
+  explicit OnDevice(const Tensor& t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.get_device()).stream()) {}
+};
+
+void require_cuda(std::initializer_list<const Tensor*> ts);
+void check_q(int64_t q);
+inline const Tensor* opt(const OptTensor& t) { return t.has_value() && t->defined() ? &*t : nullptr; }
+inline bool given(const OptTensor& t) { return t.has_value() && t->defined(); }
+inline Tensor bf16c(const Tensor& t) { return t.to(at::kBFloat16).contiguous(); }
+inline Tensor vec(const Tensor& s) { return s.to(at::kBFloat16).reshape({-1}).contiguous(); }
+inline Tensor empty(at::IntArrayRef sz, const Tensor& like, at::ScalarType ty = at::kBFloat16) {
+  return at::empty(sz, like.options().dtype(ty).requires_grad(false));
+}
+inline void* data(const Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr; }
+inline void* data(const OptTensor& t) { return given(t) ? data(*t) : nullptr; }
+Tensor scale_vec(const Tensor& s, int64_t n);
+
+// ---- operators (host_ops.cpp)
+std::tuple<Tensor, OptTensor> quant(const Tensor& x, const Tensor& s, int64_t q_bit, const OptTensor& z, const OptTensor& channel,
+                                    const OptTensor& out_q, const OptTensor& out_xo);
+Tensor dequant(const Tensor& q, const Tensor& s, int64_t q_bit, const OptTensor& z, const OptTensor& channel, const OptTensor& xo,
+               const OptTensor& out);
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit);
+void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& val, const Tensor& col, const Tensor& q,
+                        const Tensor& s, const Tensor& z);
+Tensor topk_restore(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
+                    at::IntArrayRef shape, int64_t q_bit, const OptTensor& out);
+Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
+                             at::IntArrayRef shape, int64_t q_bit, const Tensor& grad, const OptTensor& out, double scale);
+Tensor prune_sparse(const Tensor& x, double thr);
+Tensor prune_restore(const Tensor& idx, const Tensor& val, int64_t numel);
+std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity);
+Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out);
+std::tuple<Tensor, Tensor, Tensor> silu_forward(const Tensor& xa1, const Tensor& b1, const Tensor& x1, const Tensor& s1,
+                                                const Tensor& xa2, const Tensor& b2, const Tensor& x2, const Tensor& s2, int64_t q_bit);
+std::tuple<Tensor, Tensor, Tensor> silu_backward(const Tensor& xa1, const Tensor& b1, const Tensor& q1, const Tensor& s1,
+                                                 const Tensor& xa2, const Tensor& b2, const Tensor& q2, const Tensor& s2,
+                                                 const Tensor& grad_o, int64_t q_bit);
+std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor& x, const Tensor& w, double eps, int64_t q_bit,
+                                                                   const Tensor& sx, const OptTensor& idx, const OptTensor& sy);
+Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor& sx, const OptTensor& xo, const OptTensor& idx,
+                               const Tensor& w, const Tensor& rstd, int64_t q_bit, const OptTensor& res);
+Tensor softmax_backward(const Tensor& y, const Tensor& g, double scale);
+Tensor softmax_forward(const Tensor& scores, double scale, const OptTensor& mask, bool inplace);
+Tensor rope(const Tensor& x, const Tensor& cos, const Tensor& sin, bool backward, bool inplace);
+Tensor dequant_lora_add(const Tensor& q, const Tensor& s, const Tensor& xa, const Tensor& b, int64_t q_bit);
+Tensor dequant_nf4(const Tensor& packed, const Tensor& code, const Tensor& absmax, const OptTensor& code2, const OptTensor& absmax2,
+                   int64_t blocksize2, double offset, int64_t blocksize, at::IntArrayRef shape);
+
+// ---- GEMMs and the two halves of the layer (host_blocks.cpp)
+struct Lora { const Tensor* xa = nullptr; const Tensor* bt = nullptr; };
+Tensor gemm(const Tensor& a, const Tensor& b, bool b_is_kn, const OptTensor& a2, const OptTensor& b2, const OptTensor& a3,
+            const OptTensor& b3, const OptTensor& residual, const Tensor& status);
+Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64_t r2, int64_t q_bit);
+void bind_ops(pybind11::module_& m);
+void bind_blocks(pybind11::module_& m);
+
+}  // namespace hyc_host

@@ -1,0 +1,269 @@
+// The two halves of the fused decoder layer in steady state (statistics calibrated), as fixed launch sequences.
+// What each step is and which rounding points it has is documented in mlp.py and attention.py, which own the
+// calibration branch and the weight records.
+#include "host.h"
+#include <cmath>
+
+namespace hyc_host {
+
+static int* status_ptr(const Tensor& st) { return (int*)st.data_ptr(); }
+
+Tensor gemm(const Tensor& a, const Tensor& b, bool b_is_kn, const OptTensor& a2, const OptTensor& b2, const OptTensor& a3,
+            const OptTensor& b3, const OptTensor& residual, const Tensor& status) {
+  OnDevice on(a);
+  const int64_t M = a.size(0), K = a.size(1), N = b_is_kn ? b.size(1) : b.size(0);
+  Tensor d = empty({M, N}, a);
+  check(hyc_gemm_bf16_tcgen05(data(a), data(b), (int)M, (int)N, (int)K, b_is_kn ? 1 : 0, data(a2), data(b2), given(a2) ? (int)a2->size(1) : 0,
+                              data(a3), data(b3), given(a3) ? (int)a3->size(1) : 0, nullptr, nullptr, 0, 0, nullptr, nullptr, 0, 0,
+                              data(residual), data(d), status_ptr(status), on.stream), "hyc_gemm_bf16_tcgen05");
+  return d;
+}
+
+// several rank-16 products x A_i^T with a shared left operand (stride 0) as one batched library call
+static Tensor lora_a_products(const Tensor& x2, const Tensor& stacked) {
+  return at::bmm(x2.unsqueeze(0).expand({stacked.size(0), -1, -1}), stacked);
+}
+
+static std::tuple<Tensor, Tensor> linear_lora_save(const Tensor& x, const Tensor& w, const Tensor& xa, const Tensor& b, const Tensor& scale,
+                                                   int64_t q_bit, const Tensor& status) {
+  OnDevice on(x);
+  const int64_t T = x.size(0), K = x.size(1), N = w.size(0);
+  const Tensor sc = vec(scale), bc = b.contiguous();
+  Tensor y = empty({T, N}, x), qm = empty({T, N * q_bit / 8}, x, at::kByte);
+  check(hyc_linear_lora_save_fwd_tcgen05(data(x), data(w), (int)T, (int)K, (int)N, data(xa), data(bc), bc.size(1), 1, data(sc), data(qm),
+                                         data(y), nullptr, (int)q_bit, status_ptr(status), on.stream), "hyc_linear_lora_save_fwd_tcgen05");
+  return {y, qm};
+}
+
+Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64_t r2, int64_t q_bit) {
+  require_cuda({&q, &scale, &gm});
+  OnDevice on(q);
+  const int64_t T = q.size(0), H = scale.numel();
+  Tensor out = empty({r2, H}, q);
+  const size_t nbytes = hyc_lora_grad_a_workspace_bytes((int)T, (int)H, (int)r2);
+  Tensor ws = empty({(int64_t)(nbytes / 4)}, q, at::kFloat);
+  check(hyc_lora_grad_a_dequant(data(q), data(scale), data(gm), gm.stride(0), (int)r2, (int)T, (int)H, (int)q_bit, data(out), data(ws),
+                                nbytes, on.stream), "hyc_lora_grad_a_dequant");
+  return out;
+}
+
+// ------------------------------------------------------------------ MLP half
+struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa, down_xa64; };
+
+static std::vector<Tensor> mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
+                                       const OptTensor& bias_d, int64_t q, double eps, const Tensor& status) {
+  const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &wd = w[3], &bg = w[4], &bu = w[5], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
+  const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
+  const Tensor gs = vec(stats[3]), us = vec(stats[4]);
+  require_cuda({&x_medium, &wg});
+  OnDevice on(x_medium);
+  const int64_t B = x_medium.size(0), M = x_medium.size(1), H = x_medium.size(2), T = B * M, I = wg.size(0);
+  auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale);
+  const Tensor xn2 = x_norm.view({T, H});
+  const Tensor gu_xa = lora_a_products(xn2, agu_t);
+  const char* xa = (const char*)gu_xa.data_ptr();
+  Tensor q1 = empty({B, M, I * q / 8}, x_norm, at::kByte), q2 = empty({B, M, I * q / 8}, x_norm, at::kByte), had = empty({T, I}, x_norm);
+  check(hyc_mlp_gateup_fwd_tcgen05(data(xn2), data(wg), data(wu), (int)T, (int)H, (int)I, xa, data(bg), 16, 1, xa + T * 16 * 2, data(bu), 16, 1,
+                                   data(gs), data(us), data(q1), data(q2), data(had), nullptr, nullptr, (int)q, status_ptr(status), on.stream),
+        "hyc_mlp_gateup_fwd_tcgen05");
+  const Tensor down_xa64 = at::mm(had, ad_cols);
+  Tensor x_out = gemm(had, wd, false, down_xa64, bd_cols, std::nullopt, std::nullopt, bf16c(x_medium).view({T, H}), status);
+  if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
+  return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
+}
+
+// up to and including the six LoRA gradients: -> had, ggu, gm64, grad_bd, grad_ad, ga, grad_bgu
+static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, const Tensor& gm64,
+                                             int64_t q, const Tensor& status) {
+  const Tensor &wd = w[0], &bg = w[1], &bu = w[2], &bd_cols = w[3], &ad_rows = w[4], &bgu = w[5];
+  const Tensor &gate_q = saved[0], &gate_s = saved[1], &up_q = saved[2], &up_s = saved[3], &gu_xa = saved[4], &down_xa = saved[5],
+               &xn_q = saved[6], &xn_scale = saved[7];
+  OnDevice on(g);
+  const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
+  Tensor grad_bd = at::mm(g.t(), down_xa);
+  const Tensor gdm64 = at::mm(g, bd_cols);
+  Tensor had = empty({T, I}, g), ggu = empty({2, T, I}, g);
+  char* gp = (char*)ggu.data_ptr();
+  const char* xa = (const char*)gu_xa.data_ptr();
+  check(hyc_mlp_graddown_bwd_tcgen05(data(g), data(wd), (int)T, (int)H, (int)I, data(gdm64), data(ad_rows), 64, xa, data(bg), 16, 1,
+                                     xa + T * 16 * 2, data(bu), 16, 1, data(gate_q), data(gate_s), data(up_q), data(up_s), nullptr, nullptr, 0,
+                                     data(had), gp, gp + T * I * 2, (int)q, status_ptr(status), on.stream), "hyc_mlp_graddown_bwd_tcgen05");
+  Tensor grad_ad = at::mm(gdm64.narrow(1, 0, 16).t(), had);
+  gm64.view({T, 4, 16}).narrow(1, 0, 2).copy_(at::bmm(ggu, bgu).transpose(0, 1));
+  Tensor ga = lora_grad_a(xn_q.view({T, -1}), vec(xn_scale), gm64, 32, q);
+  Tensor grad_bgu = at::bmm(ggu.transpose(1, 2), gu_xa);
+  return {had, ggu, grad_bd, grad_ad, ga, grad_bgu};
+}
+
+static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
+                             at::IntArrayRef shape, int64_t q, const Tensor& status) {
+  const Tensor &wg = w[0], &wu = w[1], &agu_rows = w[2], &norm_w = w[3];
+  Tensor grad_xn = gemm(ggu[0], wg, true, ggu[1], wu, gm64, agu_rows, std::nullopt, status);
+  return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
+}
+
+// ------------------------------------------------------------------ attention half
+static Tensor heads(const Tensor& x2, int64_t B, int64_t M, int64_t n) { return x2.view({B, M, n, -1}).transpose(1, 2); }
+static Tensor hidden(const Tensor& xh) { return xh.transpose(1, 2).reshape({xh.size(0) * xh.size(2), xh.size(1) * xh.size(3)}); }
+static Tensor repeat_kv(const Tensor& x, int64_t n) {
+  if (n == 1) return x;
+  const auto b = x.size(0), h = x.size(1), m = x.size(2), d = x.size(3);
+  return x.unsqueeze(2).expand({b, h, n, m, d}).reshape({b, h * n, m, d});
+}
+static Tensor repeat_kv_backward(const Tensor& g, int64_t n) {
+  if (n == 1) return g;
+  return g.reshape({g.size(0), g.size(1) / n, n, g.size(2), g.size(3)}).sum(2);
+}
+// [B, n, M, K] @ [B, n, K, d] written straight into the hidden layout
+static Tensor matmul_to_hidden(const Tensor& a4, const Tensor& b4, const OptTensor& out_in) {
+  const int64_t B = a4.size(0), n = a4.size(1), M = a4.size(2), d = b4.size(3);
+  Tensor out = given(out_in) ? out_in->view({B, M, n, d}) : empty({B, M, n, d}, a4);
+  for (int64_t b = 0; b < B; ++b) {
+    Tensor o = out[b].transpose(0, 1);
+    at::bmm_out(o, a4[b], b4[b]);
+  }
+  return out.view({B * M, n * d});
+}
+
+struct Geometry { int64_t heads, d, kv; };
+
+// the q, k, v projections with their saves, rotary embedding, scores and probabilities
+static std::vector<Tensor> attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos,
+                                            const Tensor& sin, const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps,
+                                            const Tensor& status) {
+  const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
+  const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
+  require_cuda({&x, &wq});
+  OnDevice on(x);
+  const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M, rep = nh / nkv;
+  auto [x_norm, rstd, x_o, x_q, xn_q] = rmsnorm_save(x, norm_w, eps, q, x_scale, x_idx, xn_scale);
+  const Tensor xn2 = x_norm.view({T, H});
+  const Tensor xa3 = lora_a_products(xn2, aqkv_t);
+  auto [qy, q_q] = linear_lora_save(xn2, wq, xa3[0], bq, q_scale, q, status);
+  auto [ky, k_q] = linear_lora_save(xn2, wk, xa3[1], bk, k_scale, q, status);
+  auto [vy, v_q] = linear_lora_save(xn2, wv, xa3[2], bv, v_scale, q, status);
+  rope(qy.view({B, M, nh, d}), cos, sin, false, true);
+  rope(ky.view({B, M, nkv, d}), cos, sin, false, true);
+  const Tensor kh = repeat_kv(heads(ky, B, M, nkv), rep), vh = repeat_kv(heads(vy, B, M, nkv), rep);
+  Tensor scores = at::matmul(heads(qy, B, M, nh), kh.transpose(-2, -1));
+  const Tensor a = softmax_forward(scores, 1.0 / std::sqrt((double)d), mask, true);
+  const Tensor o2 = matmul_to_hidden(a, vh, std::nullopt);
+  return {a, o2, rstd, x_o, x_q, *xn_q, q_q, k_q, v_q, xa3};
+}
+
+// o projection with residual and the save of its input
+static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols,
+                                            const Tensor& o_scale, const OptTensor& bias_o, int64_t q, const Tensor& status) {
+  const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
+  const Tensor o_xa64 = at::mm(o2, ao_cols);
+  Tensor x_medium = gemm(o2, wo, false, o_xa64, bo_cols, std::nullopt, std::nullopt, bf16c(x).view({T, H}), status);
+  if (given(bias_o)) x_medium.add_(bias_o->to(at::kBFloat16));
+  const Tensor o_q = std::get<0>(quant(o2.view({B, M, -1}), o_scale, q, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
+  return {x_medium.view({B, M, H}), o_q.view({T, -1}), o_xa64};
+}
+
+static Tensor rebuild(const Tensor& codes, const Tensor& scale, const Tensor& xa, const Tensor& b, int64_t q) {
+  const int64_t T = codes.size(0);
+  return dequant_lora_add(codes.view({1, T, -1}), scale, xa.view({1, T, -1}), b.t(), q).view({T, -1});
+}
+
+// o projection backward: -> gm64, grad_bo, grad_ao, grad_o2
+static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, const Tensor& bo_cols, const Tensor& ao_rows, const Tensor& o_xa,
+                                             const Tensor& o_q, const Tensor& o_scale, int64_t q, const Tensor& status) {
+  const Tensor gm64 = at::mm(g, bo_cols);
+  Tensor grad_bo = at::mm(g.t(), o_xa);
+  Tensor grad_ao = lora_grad_a(o_q, vec(o_scale), gm64, 16, q);
+  Tensor grad_o2 = gemm(g, wo, true, gm64, ao_rows, std::nullopt, std::nullopt, std::nullopt, status);
+  return {grad_bo, grad_ao, grad_o2};
+}
+
+// the map's backward.  `a`: the restored map; `topk`: the five tensors of the top-k form (the softmax backward then
+// restores once more on chip), empty for the pruned form.  -> grad_q, grad_k, grad_v [T, n*d] after the inverse
+// rotation, and the buffer that holds all three when the head counts agree
+static std::vector<OptTensor> attn_backward_map(const Tensor& grad_o2, Tensor a, const std::vector<Tensor>& topk, int64_t map_q_bit,
+                                                const std::vector<Tensor>& saved, const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin,
+                                                int64_t B, int64_t M, int64_t nh, int64_t d, int64_t nkv, int64_t q) {
+  const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
+               &v_s = saved[7], &v_xa = saved[8];
+  OnDevice on(grad_o2);
+  const int64_t T = B * M, rep = nh / nkv;
+  const double scale = 1.0 / std::sqrt((double)d);
+  const Tensor grad_oh = heads(grad_o2, B, M, nh);
+  Tensor v2 = rebuild(v_q, v_s, v_xa, w[2], q);
+  OptTensor gqkv;
+  if (rep == 1) gqkv = empty({3, T, nh * d}, grad_o2);
+  auto slot = [&](int i) -> OptTensor { return gqkv.has_value() ? OptTensor((*gqkv)[i]) : OptTensor(); };
+  Tensor grad_v = rep == 1 ? matmul_to_hidden(a.transpose(-2, -1), grad_oh, slot(2))
+                           : hidden(repeat_kv_backward(at::matmul(a.transpose(-2, -1), grad_oh), rep));
+  Tensor grad_a = at::matmul(grad_oh, repeat_kv(heads(v2, B, M, nkv), rep).transpose(-2, -1));
+  v2.reset();
+  Tensor grad_s;
+  if (!topk.empty()) {
+    const std::vector<int64_t> shape(a.sizes().begin(), a.sizes().end());
+    a.reset();
+    grad_s = topk_softmax_backward(topk[0], topk[1], topk[2], topk[3], topk[4], shape, map_q_bit, grad_a, std::nullopt, scale);
+  } else {
+    grad_s = softmax_backward(a, grad_a, scale);
+    a.reset();
+  }
+  grad_a.reset();
+  Tensor q2 = rebuild(q_q, q_s, q_xa, w[0], q);
+  rope(q2.view({B, M, nh, d}), cos, sin, false, true);
+  Tensor grad_k = rep == 1 ? matmul_to_hidden(grad_s.transpose(-2, -1), heads(q2, B, M, nh), slot(1))
+                           : hidden(repeat_kv_backward(at::matmul(grad_s.transpose(-2, -1), heads(q2, B, M, nh)), rep));
+  q2.reset();
+  Tensor k2 = rebuild(k_q, k_s, k_xa, w[1], q);
+  rope(k2.view({B, M, nkv, d}), cos, sin, false, true);
+  Tensor grad_q = matmul_to_hidden(grad_s, repeat_kv(heads(k2, B, M, nkv), rep), slot(0));
+  rope(grad_q.view({B, M, nh, d}), cos, sin, true, true);
+  rope(grad_k.view({B, M, nkv, d}), cos, sin, true, true);
+  return {grad_q, grad_k, grad_v, gqkv};
+}
+
+// LoRA gradients of q/k/v: -> ga [48, H], grad_bq, grad_bk, grad_bv (gmq is filled)
+static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, const OptTensor& gqkv, const Tensor& gmq, const OptTensor& bqkv,
+                                              const std::vector<Tensor>& b, const Tensor& qkv_xa, const Tensor& xn_q, const Tensor& xn_scale, int64_t q) {
+  OnDevice on(gmq);
+  const int64_t T = gmq.size(0), r = 16;
+  Tensor gb[3];
+  const bool batched = given(gqkv) && given(bqkv);
+  if (batched) {
+    gmq.view({T, 4, 16}).narrow(1, 0, 3).copy_(at::bmm(*gqkv, *bqkv).transpose(0, 1));
+    const Tensor g3 = at::bmm(gqkv->transpose(1, 2), qkv_xa);
+    for (int i = 0; i < 3; ++i) gb[i] = g3[i];
+  } else {
+    for (int i = 0; i < 3; ++i) {
+      Tensor o = gmq.narrow(1, i * r, r);
+      at::mm_out(o, grads[i], b[i]);
+      gb[i] = at::mm(grads[i].t(), qkv_xa[i]);
+    }
+  }
+  Tensor ga = lora_grad_a(xn_q.view({T, -1}), vec(xn_scale), gmq, 48, q);
+  return {ga, gb[0], gb[1], gb[2]};
+}
+
+static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
+                              const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
+  const Tensor &wq = w[0], &wk = w[1], &wv = w[2], &aqkv_rows = w[3], &norm_w = w[4];
+  const Tensor lora_x = at::mm(gmq, aqkv_rows);
+  Tensor grad_xn = gemm(grads[0], wq, true, grads[1], wk, grads[2], wv, lora_x, status);
+  return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
+}
+
+void bind_blocks(pybind11::module_& m) {
+  m.def("lora_grad_a", &lora_grad_a);
+  m.def("mlp_forward", &mlp_forward);
+  m.def("mlp_backward_lora", &mlp_backward_lora);
+  m.def("mlp_backward_x", [](const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
+                             std::vector<int64_t> shape, int64_t q, const Tensor& st) { return mlp_backward_x(g, ggu, gm64, w, saved, shape, q, st); });
+  m.def("attn_forward_map", &attn_forward_map);
+  m.def("attn_forward_out", &attn_forward_out);
+  m.def("attn_backward_out", &attn_backward_out);
+  m.def("attn_backward_map", &attn_backward_map);
+  m.def("attn_backward_lora", &attn_backward_lora);
+  m.def("attn_backward_x", [](const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
+                              const std::vector<Tensor>& saved, std::vector<int64_t> shape, int64_t q, const Tensor& st) {
+    return attn_backward_x(g, grads, gmq, w, saved, shape, q, st); });
+}
+
+}  // namespace hyc_host

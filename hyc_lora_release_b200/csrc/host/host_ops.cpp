@@ -1,0 +1,386 @@
+#include "host.h"
+
+namespace hyc_host {
+
+void check(int rc, const char* what) {
+  if (rc == HYC_OK) return;
+  std::string msg = std::string(what) + ": " + hyc_strerror(rc);
+  if (rc == HYC_ERR_LAUNCH) msg += " [cudaError " + std::to_string(hyc_last_cuda_error()) + "]";
+  throw Error(msg);
+}
+
+void require_cuda(std::initializer_list<const Tensor*> ts) {
+  const Tensor* first = nullptr;
+  for (const Tensor* t : ts) {
+    if (t == nullptr) continue;
+    if (!t->is_cuda()) throw std::runtime_error("this operator runs only on CUDA tensors (sm_100a kernels); there is no CPU path");
+    if (first == nullptr) first = t;
+    else if (t->device() != first->device())
+      throw std::runtime_error("the tensors of one call live on different devices (" + first->device().str() + " and " + t->device().str() + ")");
+  }
+}
+
+void check_q(int64_t q) { TORCH_CHECK_VALUE(q == 2 || q == 4 || q == 8, "quantize_bit must be 2, 4 or 8"); }
+
+Tensor scale_vec(const Tensor& s, int64_t n) {
+  Tensor v = s.to(at::kBFloat16).reshape({-1});
+  TORCH_CHECK_VALUE(v.numel() == n, "per-channel scale with ", v.numel(), " entries for ", n,
+                    " channels (per-tensor scales cannot be quantized with)");
+  return v.contiguous();
+}
+
+// [B, M, N] (or [B, heads, M, d], which becomes [B, M, heads*d]) -> bf16 with one row stride
+static Tensor rows_view(const Tensor& x_in) {
+  Tensor x = x_in;
+  if (x.dim() == 4) x = x.transpose(1, 2).reshape({x.size(0), x.size(2), -1});
+  TORCH_CHECK_VALUE(x.dim() == 3, "expected a [B, M, N] or [B, heads, M, d] tensor, got shape ", x_in.sizes());
+  x = x.to(at::kBFloat16);
+  const int64_t M = x.size(1), N = x.size(2);
+  if (x.stride(2) != 1 || (x.size(0) > 1 && x.stride(0) != M * x.stride(1)) || x.stride(1) < N || x.stride(1) % 8 != 0 ||
+      reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0)
+    x = x.contiguous();
+  return x;
+}
+
+static Tensor index_of(const Tensor& channel, const Tensor& like) {
+  return channel.to(like.device(), at::kLong).contiguous();
+}
+
+std::tuple<Tensor, OptTensor> quant(const Tensor& x_in, const Tensor& s_in, int64_t q_bit, const OptTensor& z, const OptTensor& channel,
+                                    const OptTensor& out_q, const OptTensor& out_xo) {
+  require_cuda({&x_in, &s_in});
+  check_q(q_bit);
+  OnDevice on(x_in);
+  const Tensor x = rows_view(x_in);
+  const int64_t B = x.size(0), M = x.size(1), N = x.size(2), rows = B * M;
+  TORCH_CHECK_VALUE(N % 32 == 0, "the hidden size must be a multiple of 32");
+  const Tensor s = scale_vec(s_in, N);
+  Tensor zt, idx;
+  if (given(z)) zt = z->reshape({-1}).to(at::kChar).contiguous();
+  int64_t k = 0;
+  if (given(channel)) { idx = index_of(*channel, x); k = idx.numel(); }
+  Tensor q = given(out_q) ? *out_q : empty({B, M, N * q_bit / 8}, x, at::kByte);
+  OptTensor xo = out_xo;
+  if (!given(out_q) && given(channel)) xo = empty({B, M, k}, x);
+  if (rows > 0)
+    check(hyc_quant_pack(data(x), rows, (int)N, x.stride(1), data(s), (const int8_t*)data(zt), k ? (const int64_t*)data(idx) : nullptr,
+                         (int)k, data(q), k ? data(xo) : nullptr, (int)q_bit, on.stream), "hyc_quant_pack");
+  return {q, xo};
+}
+
+Tensor dequant(const Tensor& q_in, const Tensor& s_in, int64_t q_bit, const OptTensor& z, const OptTensor& channel, const OptTensor& xo_in,
+               const OptTensor& out) {
+  require_cuda({&q_in, &s_in});
+  check_q(q_bit);
+  OnDevice on(q_in);
+  TORCH_CHECK_VALUE(q_in.dim() == 3, "expected [B, M, bytes] codes, got shape ", q_in.sizes());
+  const int64_t B = q_in.size(0), M = q_in.size(1), N = s_in.size(-1);
+  const Tensor q = q_in.contiguous(), s = scale_vec(s_in, N);
+  Tensor zt, idx, xo;
+  if (given(z)) zt = z->reshape({-1}).to(at::kChar).contiguous();
+  Tensor x = given(out) ? *out : empty({B, M, N}, q);
+  if (B * M == 0) return x;
+  int64_t k = 0;
+  if (given(channel)) {
+    idx = index_of(*channel, q);
+    k = idx.numel();
+    xo = bf16c(*xo_in);
+  }
+  check(hyc_unpack_dequant(data(q), B * M, (int)N, data(s), (const int8_t*)data(zt), k ? (const int64_t*)data(idx) : nullptr, (int)k,
+                           k ? data(xo) : nullptr, data(x), N, (int)q_bit, on.stream), "hyc_unpack_dequant");
+  return x;
+}
+
+// ---- attention map, per-row top-k
+void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& val, const Tensor& col, const Tensor& q,
+                        const Tensor& s, const Tensor& z) {
+  require_cuda({&x});
+  check_q(q_bit);
+  OnDevice on(x);
+  const Tensor xb = bf16c(x);
+  const int64_t S = xb.size(-1), rows = xb.numel() / S;
+  check(hyc_softmax_topk_compress(data(xb), rows, (int)S, (int)k, k ? data(val) : nullptr, k ? (uint16_t*)data(col) : nullptr, data(q),
+                                  data(s), (int8_t*)data(z), (int)q_bit, on.stream), "hyc_softmax_topk_compress");
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit) {
+  require_cuda({&x});
+  check_q(q_bit);
+  const int64_t S = x.size(-1), rows = x.numel() / S;
+  Tensor val = empty({rows, k}, x), col = empty({rows, k}, x, at::kShort), q = empty({rows, S * q_bit / 8}, x, at::kByte),
+         s = empty({rows, S / 64}, x), z = empty({rows, S / 64}, x, at::kChar);
+  topk_compress_into(x, k, q_bit, val, col, q, s, z);
+  return {val, col, q, s, z};
+}
+
+Tensor topk_restore(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
+                    at::IntArrayRef shape, int64_t q_bit, const OptTensor& out) {
+  OnDevice on(q);
+  Tensor x = given(out) ? *out : empty(shape, q);
+  const int64_t k = val.size(1);
+  check(hyc_softmax_topk_restore(k ? data(val) : nullptr, k ? (const uint16_t*)data(col) : nullptr, (int)k, data(q), data(s),
+                                 (const int8_t*)data(z), q.size(0), (int)shape.back(), data(x), (int)q_bit, on.stream), "hyc_softmax_topk_restore");
+  return x;
+}
+
+Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
+                             at::IntArrayRef shape, int64_t q_bit, const Tensor& grad, const OptTensor& out, double scale) {
+  require_cuda({&grad, &q});
+  OnDevice on(q);
+  const Tensor g = bf16c(grad);
+  TORCH_CHECK_VALUE(g.sizes() == shape, "the gradient must have the map's shape ", shape);
+  Tensor o = given(out) ? *out : empty(shape, q);
+  const int64_t k = val.size(1);
+  const int rc = hyc_softmax_topk_restore_bwd(k ? data(val) : nullptr, k ? (const uint16_t*)data(col) : nullptr, (int)k, data(q), data(s),
+                                              (const int8_t*)data(z), q.size(0), (int)shape.back(), data(g), data(o), (int)q_bit,
+                                              (float)scale, on.stream);
+  if (rc == HYC_ERR_UNSUPPORTED) {      // shape outside the fused kernel: restore, then the softmax backward in place
+    Tensor a = topk_restore(val, col, q, s, z, shape, q_bit, std::nullopt);
+    check(hyc_softmax_bwd(data(a), data(g), data(o), a.numel() / shape.back(), (int)shape.back(), (float)scale, on.stream), "hyc_softmax_bwd");
+    return o;
+  }
+  check(rc, "hyc_softmax_topk_restore_bwd");
+  return o;
+}
+
+// ---- attention map, threshold prune
+Tensor prune_sparse(const Tensor& x, double thr) {
+  require_cuda({&x});
+  OnDevice on(x);
+  const Tensor xf = bf16c(x);
+  const int64_t numel = xf.numel();
+  const size_t ws_bytes = hyc_softmax_prune_workspace_bytes(numel);
+  Tensor ws = empty({(int64_t)((ws_bytes + 7) / 8)}, x, at::kLong);
+  check(hyc_softmax_prune_count(data(xf), numel, (float)thr, data(ws), ws_bytes, on.stream), "hyc_softmax_prune_count");
+  const int64_t nnz = ws.narrow(0, 0, 1).item<int64_t>();
+  Tensor idx = empty({1, nnz}, x, at::kLong), val = empty({nnz}, x);
+  check(hyc_softmax_prune_fill(data(xf), numel, (float)thr, data(ws), (int64_t*)data(idx), data(val), nnz, on.stream), "hyc_softmax_prune_fill");
+  Tensor sp = at::_sparse_coo_tensor_unsafe(idx, val, {numel}, val.options().layout(at::kSparse));
+  return sp._coalesced_(true);      // the fill writes ascending indices
+}
+
+Tensor prune_restore(const Tensor& idx_in, const Tensor& val_in, int64_t numel) {
+  require_cuda({&idx_in, &val_in});
+  OnDevice on(val_in);
+  const Tensor idx = idx_in.reshape({-1}).contiguous(), val = bf16c(val_in);
+  Tensor out = empty({numel}, val);
+  check(hyc_softmax_prune_restore((const int64_t*)data(idx), data(val), idx.numel(), data(out), numel, on.stream), "hyc_softmax_prune_restore");
+  return out;
+}
+
+std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity) {
+  require_cuda({&x});
+  OnDevice on(x);
+  const Tensor xf = bf16c(x);
+  const int64_t numel = xf.numel();
+  Tensor nnz = empty({1}, x, at::kLong), words = empty({capacity}, x, at::kInt),
+         dir = empty({(int64_t)(hyc_softmax_prune_tiled_directory_bytes(numel) / 4)}, x, at::kInt);
+  check(hyc_softmax_prune_tiled(data(xf), numel, (float)thr, (uint32_t*)data(words), capacity, data(dir), (int64_t*)data(nnz), on.stream),
+        "hyc_softmax_prune_tiled");
+  return {words, dir, nnz};
+}
+
+Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out) {
+  OnDevice on(words);
+  Tensor x = given(out) ? *out : empty(shape, words);
+  check(hyc_softmax_prune_tiled_restore((const uint32_t*)data(words), words.numel(), data(directory), data(x), x.numel(), on.stream),
+        "hyc_softmax_prune_tiled_restore");
+  return x;
+}
+
+// ---- fused LoRA-SiLU-Hadamard
+// [R, N] LoRA-B operand -> the [N, R] row-major matrix the kernels read; ``lora_B.weight.T`` is a view of exactly that storage
+static Tensor b_transposed(const Tensor& b) {
+  TORCH_CHECK_VALUE(b.dim() == 2, "LoRA B must be [R, N]");
+  return b.t().to(at::kBFloat16).contiguous();
+}
+
+static void check_fused(int64_t q_bit, int64_t n, int64_t r, std::initializer_list<const Tensor*> ts) {
+  require_cuda(ts);
+  check_q(q_bit);
+  TORCH_CHECK_VALUE(n % 32 == 0, "N must be a multiple of 32");
+  TORCH_CHECK_VALUE(r == 16, "LoRA rank must be 16");
+}
+
+std::tuple<Tensor, Tensor, Tensor> silu_forward(const Tensor& xa1, const Tensor& b1, const Tensor& x1, const Tensor& s1,
+                                                const Tensor& xa2, const Tensor& b2, const Tensor& x2, const Tensor& s2, int64_t q_bit) {
+  TORCH_CHECK_VALUE(x1.dim() == 3, "expected [B, M, N] main branches, got shape ", x1.sizes());
+  const int64_t B = x1.size(0), M = x1.size(1), N = x1.size(2), R = b1.size(0);
+  check_fused(q_bit, N, R, {&xa1, &b1, &x1, &s1, &xa2, &b2, &x2, &s2});
+  OnDevice on(x1);
+  const Tensor x1c = bf16c(x1), x2c = bf16c(x2), a1 = bf16c(xa1), a2 = bf16c(xa2), bt1 = b_transposed(b1), bt2 = b_transposed(b2),
+               sc1 = scale_vec(s1, N), sc2 = scale_vec(s2, N);
+  Tensor q1 = empty({B, M, N * q_bit / 8}, x1, at::kByte), q2 = empty({B, M, N * q_bit / 8}, x1, at::kByte), o = empty({B, M, N}, x1);
+  check(hyc_fused_lora_silu_hadamard_fwd(data(a1), data(bt1), data(x1c), data(sc1), data(a2), data(bt2), data(x2c), data(sc2), data(q1),
+                                         data(q2), data(o), B * M, (int)N, (int)R, (int)q_bit, on.stream), "hyc_fused_lora_silu_hadamard_fwd");
+  return {q1, q2, o};
+}
+
+std::tuple<Tensor, Tensor, Tensor> silu_backward(const Tensor& xa1, const Tensor& b1, const Tensor& q1, const Tensor& s1,
+                                                 const Tensor& xa2, const Tensor& b2, const Tensor& q2, const Tensor& s2,
+                                                 const Tensor& grad_o, int64_t q_bit) {
+  TORCH_CHECK_VALUE(grad_o.dim() == 3, "expected a [B, M, N] gradient, got shape ", grad_o.sizes());
+  const int64_t B = grad_o.size(0), M = grad_o.size(1), N = grad_o.size(2), R = b1.size(0);
+  check_fused(q_bit, N, R, {&xa1, &b1, &q1, &s1, &xa2, &b2, &q2, &s2, &grad_o});
+  OnDevice on(grad_o);
+  const Tensor g = bf16c(grad_o), a1 = bf16c(xa1), a2 = bf16c(xa2), bt1 = b_transposed(b1), bt2 = b_transposed(b2),
+               sc1 = scale_vec(s1, N), sc2 = scale_vec(s2, N), q1c = q1.contiguous(), q2c = q2.contiguous();
+  Tensor o = empty({B, M, N}, g), gg = empty({B, M, N}, g), gu = empty({B, M, N}, g);
+  check(hyc_fused_lora_silu_hadamard_bwd(data(a1), data(bt1), data(q1c), data(sc1), data(a2), data(bt2), data(q2c), data(sc2), data(g),
+                                         data(o), data(gg), data(gu), B * M, (int)N, (int)R, (int)q_bit, on.stream),
+        "hyc_fused_lora_silu_hadamard_bwd");
+  return {o, gg, gu};
+}
+
+Tensor dequant_lora_add(const Tensor& q, const Tensor& s, const Tensor& xa, const Tensor& b, int64_t q_bit) {
+  require_cuda({&q, &s, &xa, &b});
+  check_q(q_bit);
+  OnDevice on(q);
+  const int64_t B = q.size(0), M = q.size(1), N = s.size(-1);
+  const Tensor sc = scale_vec(s, N), xac = bf16c(xa), bt = b_transposed(b), qc = q.contiguous();
+  Tensor y = empty({B, M, N}, q);
+  if (B * M)
+    check(hyc_dequant_lora_add(data(qc), data(sc), data(xac), data(bt), data(y), B * M, (int)N, (int)xac.size(-1), (int)q_bit, on.stream),
+          "hyc_dequant_lora_add");
+  return y;
+}
+
+// ---- norms, softmax, rotary embedding
+std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor& x, const Tensor& w_in, double eps, int64_t q_bit,
+                                                                   const Tensor& sx_in, const OptTensor& idx_in, const OptTensor& sy_in) {
+  require_cuda({&x, &w_in, &sx_in});
+  check_q(q_bit);
+  OnDevice on(x);
+  const Tensor xc = bf16c(x), w = bf16c(w_in);
+  const int64_t N = xc.size(-1), rows = xc.numel() / N;
+  const Tensor sx = scale_vec(sx_in, N);
+  Tensor idx, sy;
+  int64_t k = 0;
+  if (given(idx_in)) { idx = index_of(*idx_in, x); k = idx.numel(); }
+  if (given(sy_in)) sy = vec(*sy_in);
+  std::vector<int64_t> qs(xc.sizes().begin(), xc.sizes().end()), os = qs;
+  qs.back() = N * q_bit / 8;
+  os.back() = k;
+  Tensor y = at::empty_like(xc), rstd = empty({rows}, x, at::kFloat), qx = empty(qs, x, at::kByte), xo = empty(os, x);
+  OptTensor qy;
+  if (sy.defined()) qy = empty(qs, x, at::kByte);
+  if (rows)
+    check(hyc_rmsnorm_fwd_save(data(xc), data(w), (float)eps, rows, (int)N, data(sx), k ? (const int64_t*)data(idx) : nullptr, (int)k,
+                               data(sy), data(y), (float*)data(rstd), data(qx), k ? data(xo) : nullptr, data(qy), (int)q_bit, on.stream),
+          "hyc_rmsnorm_fwd_save");
+  return {y, rstd, xo, qx, qy};
+}
+
+Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor& sx_in, const OptTensor& xo_in, const OptTensor& idx_in,
+                               const Tensor& w_in, const Tensor& rstd, int64_t q_bit, const OptTensor& res_in) {
+  require_cuda({&dy, &qx, &sx_in, &w_in, &rstd});
+  OnDevice on(dy);
+  const Tensor dyc = bf16c(dy), sx = vec(sx_in), w = bf16c(w_in), q = qx.contiguous(), rs = rstd.contiguous();
+  const int64_t N = dyc.size(-1), rows = dyc.numel() / N;
+  Tensor idx, xo, res;
+  int64_t k = 0;
+  if (given(idx_in)) { idx = index_of(*idx_in, dy); k = idx.numel(); }
+  if (k) xo = bf16c(*xo_in);
+  if (given(res_in)) res = bf16c(*res_in);
+  Tensor dx = at::empty_like(dyc);
+  if (rows)
+    check(hyc_rmsnorm_bwd_packed(data(dyc), data(q), data(sx), k ? (const int64_t*)data(idx) : nullptr, (int)k, data(xo), data(w),
+                                 (const float*)data(rs), data(res), data(dx), rows, (int)N, (int)q_bit, on.stream), "hyc_rmsnorm_bwd_packed");
+  return dx;
+}
+
+Tensor softmax_backward(const Tensor& y, const Tensor& g, double scale) {
+  require_cuda({&y, &g});
+  OnDevice on(y);
+  const Tensor yc = bf16c(y), gc = bf16c(g);
+  Tensor o = at::empty_like(yc);
+  const int64_t S = yc.size(-1);
+  check(hyc_softmax_bwd(data(yc), data(gc), data(o), yc.numel() / S, (int)S, (float)scale, on.stream), "hyc_softmax_bwd");
+  return o;
+}
+
+Tensor softmax_forward(const Tensor& scores, double scale, const OptTensor& mask, bool inplace) {
+  require_cuda({&scores, opt(mask)});
+  TORCH_CHECK_VALUE(scores.dim() == 4, "scores must be [batch, heads, n, S]");
+  TORCH_CHECK_VALUE(!inplace || (scores.scalar_type() == at::kBFloat16 && scores.is_contiguous()), "inplace needs contiguous bf16 scores");
+  OnDevice on(scores);
+  const Tensor sc = bf16c(scores);
+  const int64_t b = sc.size(0), h = sc.size(1), n = sc.size(2), S = sc.size(3);
+  Tensor out = inplace ? sc : at::empty_like(sc), mk;
+  int64_t mb = 0, mh = 0, mr = 0;
+  if (given(mask)) {
+    mk = mask->to(at::kBFloat16);
+    TORCH_CHECK_VALUE(mk.dim() == 4 && mk.size(3) == S && mk.size(2) == n && (mk.size(0) == 1 || mk.size(0) == b) &&
+                      (mk.size(1) == 1 || mk.size(1) == h), "attention_mask must be [b or 1, h or 1, n, S]");
+    auto strides = [&]() { mb = mk.size(0) == 1 ? 0 : mk.stride(0); mh = mk.size(1) == 1 ? 0 : mk.stride(1); mr = mk.stride(2); };
+    if (mk.stride(3) != 1) mk = mk.contiguous();
+    strides();
+    if (((mb | mh | mr) & 7) || (reinterpret_cast<uintptr_t>(mk.data_ptr()) & 15)) { mk = mk.contiguous(); strides(); }
+  }
+  check(hyc_softmax_fwd_scale_mask(data(sc), (float)scale, data(mk), mb, mh, mr, (int)h, (int)n, data(out), b * h * n, (int)S, on.stream),
+        "hyc_softmax_fwd_scale_mask");
+  return out;
+}
+
+Tensor rope(const Tensor& x, const Tensor& cos_in, const Tensor& sin_in, bool backward, bool inplace) {
+  require_cuda({&x, &cos_in, &sin_in});
+  TORCH_CHECK_VALUE(x.dim() == 4, "expected a [batch, seq_len, n_heads, head_dim] tensor");
+  OnDevice on(x);
+  const int64_t batch = x.size(0), seq = x.size(1), heads = x.size(2), d = x.size(3);
+  Tensor cos = cos_in.squeeze(), sin = sin_in.squeeze();
+  TORCH_CHECK_VALUE(cos.dim() == 2 && sin.sizes() == cos.sizes(), "cos / sin must squeeze to [seq_len, head_dim] tables");
+  if (seq > cos.size(0)) {
+    PyErr_SetString(PyExc_AssertionError, "the rotary tables are shorter than the sequence");
+    throw pybind11::error_already_set();
+  }
+  TORCH_CHECK_VALUE(cos.size(1) >= d / 2, "cos / sin tables are narrower than head_dim / 2");
+  if (cos.scalar_type() != at::kBFloat16 && cos.scalar_type() != at::kFloat) { cos = cos.to(at::kFloat); sin = sin.to(at::kFloat); }
+  sin = sin.to(cos.scalar_type());
+  if (cos.stride(1) != 1 || sin.stride(1) != 1 || sin.stride(0) != cos.stride(0)) { cos = cos.contiguous(); sin = sin.contiguous(); }
+  const Tensor xc = bf16c(x);
+  Tensor out = inplace || xc.data_ptr() != x.data_ptr() ? xc : at::empty_like(xc);
+  check(hyc_rope(data(xc), heads * d, data(out), heads * d, data(cos), data(sin), cos.stride(0), cos.scalar_type() == at::kFloat ? 1 : 0,
+                 batch * seq, (int)seq, (int)heads, (int)d, backward ? 1 : 0, on.stream), "hyc_rope");
+  return out.view({batch, seq, heads, d});
+}
+
+Tensor dequant_nf4(const Tensor& packed, const Tensor& code, const Tensor& absmax, const OptTensor& code2, const OptTensor& absmax2,
+                   int64_t blocksize2, double offset, int64_t blocksize, at::IntArrayRef shape) {
+  OnDevice on(packed);
+  Tensor out = empty(shape, packed);
+  const bool nested = given(code2);
+  check(hyc_dequant_nf4(data(packed), (const float*)data(code), nested ? nullptr : (const float*)data(absmax),
+                        nested ? (const uint8_t*)data(absmax) : nullptr, (const float*)data(code2), (const float*)data(absmax2),
+                        (int)blocksize2, (float)offset, out.numel(), (int)blocksize, data(out), on.stream), "hyc_dequant_nf4");
+  return out;
+}
+
+void bind_ops(pybind11::module_& m) {
+  m.def("quant", &quant);
+  m.def("dequant", &dequant);
+  m.def("topk_compress", &topk_compress);
+  m.def("topk_compress_into", &topk_compress_into);
+  m.def("topk_restore", [](const Tensor& v, const Tensor& c, const Tensor& q, const Tensor& s, const Tensor& z, std::vector<int64_t> shape,
+                           int64_t q_bit, const OptTensor& out) { return topk_restore(v, c, q, s, z, shape, q_bit, out); });
+  m.def("topk_softmax_backward", [](const Tensor& v, const Tensor& c, const Tensor& q, const Tensor& s, const Tensor& z,
+                                    std::vector<int64_t> shape, int64_t q_bit, const Tensor& g, const OptTensor& out, double scale) {
+    return topk_softmax_backward(v, c, q, s, z, shape, q_bit, g, out, scale); });
+  m.def("prune_sparse", &prune_sparse);
+  m.def("prune_restore", &prune_restore);
+  m.def("prune_tiled", &prune_tiled);
+  m.def("prune_tiled_restore", [](const Tensor& w, const Tensor& d, std::vector<int64_t> shape, const OptTensor& out) {
+    return prune_tiled_restore(w, d, shape, out); });
+  m.def("silu_forward", &silu_forward);
+  m.def("silu_backward", &silu_backward);
+  m.def("dequant_lora_add", &dequant_lora_add);
+  m.def("rmsnorm_save", &rmsnorm_save);
+  m.def("rmsnorm_backward_packed", &rmsnorm_backward_packed);
+  m.def("softmax_backward", &softmax_backward);
+  m.def("softmax_forward", &softmax_forward);
+  m.def("rope", &rope);
+  m.def("dequant_nf4", [](const Tensor& p, const Tensor& code, const Tensor& absmax, const OptTensor& code2, const OptTensor& absmax2,
+                          int64_t bs2, double offset, int64_t bs, std::vector<int64_t> shape) {
+    return dequant_nf4(p, code, absmax, code2, absmax2, bs2, offset, bs, shape); });
+}
+
+}  // namespace hyc_host

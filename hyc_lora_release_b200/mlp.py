@@ -15,15 +15,14 @@ Only packed codes, scales, the outlier slab, the rank-16 LoRA activations and rs
 between the two passes.  Weights use the nn.Linear layout ([out, in]); the LoRA factors are
 ``lora_A.weight`` [r, in] and ``lora_B.weight`` [out, r].
 """
-import ctypes
 from dataclasses import dataclass, field
 from typing import Optional
 
 import torch
 
-from ._lib import HycError, check, lib, ptr, require_cuda, stream_of
+from ._lib import HycError, check, host, lib, ptr, require_cuda, stream_of
 from .operators import compress_function as cf
-from .operators.rmsnorm_kernels import rmsnorm_backward_packed, rmsnorm_forward, rmsnorm_forward_save
+from .operators.rmsnorm_kernels import rmsnorm_forward
 
 BF16 = torch.bfloat16
 _KERNEL_STATUS = {1: "TMA producer wait timed out", 2: "MMA issuer wait timed out", 3: "epilogue wait timed out"}
@@ -109,15 +108,7 @@ def linear_lora_save(x, w, a, b, scale, q_bit, *, want_main=False, status=None, 
 def lora_grad_a(q, scale, gm, r2, q_bit):
     """out [r2, H] = gm[:, :r2]^T @ dequant(q, scale), the packed activation de-quantized inside the kernel.
     q [T, H*q_bit/8] uint8, scale [H] bf16, gm [T, >= r2] bf16 (row stride a multiple of 8)."""
-    require_cuda(q, scale, gm)
-    T = q.shape[0]
-    H = scale.numel()
-    out = torch.empty((r2, H), dtype=BF16, device=q.device)
-    nbytes = lib.hyc_lora_grad_a_workspace_bytes(T, H, r2)
-    ws = torch.empty(nbytes // 4, dtype=torch.float32, device=q.device)
-    check(lib.hyc_lora_grad_a_dequant(ptr(q), ptr(scale), ptr(gm), gm.stride(0), r2, T, H, q_bit, ptr(out), ptr(ws),
-                                      nbytes, stream_of(q)), "hyc_lora_grad_a_dequant")
-    return out
+    return host.lora_grad_a(q, scale, gm, r2, q_bit)
 
 
 @dataclass
@@ -178,30 +169,39 @@ def mlp_forward(x_medium, w: MLPWeights, state: MLPState, eps=1e-5, status=None)
     """-> (x_out [B,M,H], saved tuple).  Advances the calibration state like the layer does."""
     require_cuda(x_medium)
     B, M, H = x_medium.shape
-    T, I, q = B * M, w.wg.shape[0], state.q_bit
     st = status if status is not None else _status_tensor(x_medium.device)
-    calib = state.iteration < state.iteration_threshold
-    sv = state.static_value
-
-    if calib:
-        x_norm, _, rstd, _, _ = rmsnorm_forward(x_medium, w.norm_w, eps)
-        xm_o, xm_q, xm_idx, xm_scale = cf.compression_pack_channel_base(
-            x_medium, state.layernorm_outlier_ratio, q, 'per-channel', state.iteration, state.iteration_threshold,
-            sv['x_medium'])
-        xn_q = None
+    q, sv = state.q_bit, state.static_value
+    if state.iteration < state.iteration_threshold:
+        x_out, saved = _mlp_forward_calibrating(x_medium, w, state, eps, st)
     else:
-        # steady state: the norm, the save of its input (codes + outlier channels) and the save of its output
-        # are one pass over x_medium
-        xm_idx, xm_scale, xn_scale = sv['x_medium']['outlier_channel_index'], sv['x_medium']['scale'], sv['x_norm_2']['scale']
-        x_norm, rstd, xm_o, xm_q, xn_q = rmsnorm_forward_save(x_medium, w.norm_w, eps, q, xm_scale, xm_idx, xn_scale)
+        # steady state: the norm, the save of its input (codes + outlier channels) and the save of its output are one
+        # pass over x_medium, then gate/up and down; one call into the native host path for the whole sequence
+        pad = w.padded()
+        xm, xn_scale = sv['x_medium'], sv['x_norm_2']['scale']
+        x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa, down_xa64 = host.mlp_forward(
+            x_medium, [w.norm_w, w.wg, w.wu, w.wd, w.bg, w.bu, pad["agu_t"], pad["ad_cols"], pad["bd_cols"]],
+            [xm['outlier_channel_index'], xm['scale'], xn_scale, sv['gate']['scale'], sv['up']['scale']], w.bias_d, q, eps, st)
+        saved = dict(rstd=rstd, xm_o=xm_o, xm_q=xm_q, xm_scale=xm['scale'], xm_idx=xm['outlier_channel_index'], xn_q=xn_q,
+                     xn_scale=xn_scale, gate_q=q1, gate_scale=gs, up_q=q2, up_scale=us, gate_xa=gu_xa[0], up_xa=gu_xa[1],
+                     gu_xa=gu_xa, down_xa=down_xa64[:, :16], q_bit=q, shape=(B, M, H))
+    state.iteration += 1
+    return x_out, saved
+
+
+def _mlp_forward_calibrating(x_medium, w, state, eps, st):
+    """A calibration iteration: every save takes its statistics from the finished tensor."""
+    B, M, H = x_medium.shape
+    T, I, q, it, thd = B * M, w.wg.shape[0], state.q_bit, state.iteration, state.iteration_threshold
+    sv, dev = state.static_value, x_medium.device
+    x_norm, _, rstd, _, _ = rmsnorm_forward(x_medium, w.norm_w, eps)
+    xm_o, xm_q, xm_idx, xm_scale = cf.compression_pack_channel_base(x_medium, state.layernorm_outlier_ratio, q, 'per-channel', it, thd,
+                                                                    sv['x_medium'])
     xn2 = x_norm.reshape(T, H)
     gu_xa = lora_a_products(xn2, w.padded()["agu_t"])                # x_norm @ Ag^T and x_norm @ Au^T in one call
     gate_xa, up_xa = gu_xa[0], gu_xa[1]
-    dev = x_medium.device
-    epp = 8 // q
-    q1 = torch.empty((B, M, I // epp), dtype=torch.uint8, device=dev)
-    q2 = torch.empty((B, M, I // epp), dtype=torch.uint8, device=dev)
-    had = torch.empty((B, M, I), dtype=BF16, device=dev)
+    q1 = torch.empty((B, M, I * q // 8), dtype=torch.uint8, device=dev)
+    q2 = torch.empty((B, M, I * q // 8), dtype=torch.uint8, device=dev)
+    had = torch.empty((T, I), dtype=BF16, device=dev)
 
     def gateup(s1, s2, m1=None, m2=None):
         check(lib.hyc_mlp_gateup_fwd_tcgen05(
@@ -210,45 +210,32 @@ def mlp_forward(x_medium, w: MLPWeights, state: MLPState, eps=1e-5, status=None)
             ptr(s1), ptr(s2), ptr(q1), ptr(q2), ptr(had), ptr(m1), ptr(m2), q, ptr(st), stream_of(x_medium)),
             "hyc_mlp_gateup_fwd_tcgen05")
 
-    if calib:
-        # calibration iterations: the scales depend on the finished main branches, so the GEMM runs
-        # twice (first pass only materialises gate_main / up_main); steady state is single-pass
-        ones = torch.ones(I, dtype=BF16, device=dev)
-        m1 = torch.empty((B, M, I), dtype=BF16, device=dev)
-        m2 = torch.empty((B, M, I), dtype=BF16, device=dev)
-        gateup(ones, ones, m1, m2)
-        gate_scale = cf.get_statistics_only_quant(m1, q, 'per-channel')
-        up_scale = cf.get_statistics_only_quant(m2, q, 'per-channel')
-        del m1, m2
-    else:
-        gate_scale, up_scale = sv['gate']['scale'], sv['up']['scale']
+    # the scales depend on the finished main branches, so the GEMM runs twice (the first pass only materialises
+    # gate_main / up_main)
+    ones = torch.ones(I, dtype=BF16, device=dev)
+    m1 = torch.empty((B, M, I), dtype=BF16, device=dev)
+    m2 = torch.empty((B, M, I), dtype=BF16, device=dev)
+    gateup(ones, ones, m1, m2)
+    gate_scale = cf.get_statistics_only_quant(m1, q, 'per-channel')
+    up_scale = cf.get_statistics_only_quant(m2, q, 'per-channel')
+    del m1, m2
     gs = gate_scale.to(BF16).reshape(-1).contiguous()
     us = up_scale.to(BF16).reshape(-1).contiguous()
     gateup(gs, us)
-
-    if xn_q is None:
-        xn_q, xn_scale = cf.compression_pack_quant_base(x_norm, q, 'per-channel', state.iteration,
-                                                        state.iteration_threshold, sv['x_norm_2'])
-    had2 = had.reshape(T, I)
+    xn_q, xn_scale = cf.compression_pack_quant_base(x_norm, q, 'per-channel', it, thd, sv['x_norm_2'])
     pad = w.padded()
-    down_xa64 = had2 @ pad["ad_cols"]              # [T, 64]: the LoRA-A activation of the down projection, zero-padded
-    down_xa = down_xa64[:, :16]
+    down_xa64 = had @ pad["ad_cols"]               # [T, 64]: the LoRA-A activation of the down projection, zero-padded
     # down = hadamard @ Wd^T + down_xa @ Bd^T (one more K block) + residual
-    x_out = gemm(had2, w.wd, a2=down_xa64, b2=pad["bd_cols"], residual=x_medium.reshape(T, H).contiguous(), status=st)
+    x_out = gemm(had, w.wd, a2=down_xa64, b2=pad["bd_cols"], residual=x_medium.reshape(T, H).to(BF16).contiguous(), status=st)
     if w.bias_d is not None:
         x_out += w.bias_d.to(BF16)
-
-    if calib:
-        it = state.iteration
-        sv['x_medium'] = cf.update_dict(sv['x_medium'], {'outlier_channel_index': xm_idx, 'scale': xm_scale}, it)
-        sv['x_norm_2'] = cf.update_dict(sv['x_norm_2'], {'scale': xn_scale}, it)
-        sv['gate'] = cf.update_dict(sv['gate'], {'scale': gate_scale}, it)
-        sv['up'] = cf.update_dict(sv['up'], {'scale': up_scale}, it)
-    state.iteration += 1
-
+    sv['x_medium'] = cf.update_dict(sv['x_medium'], {'outlier_channel_index': xm_idx, 'scale': xm_scale}, it)
+    sv['x_norm_2'] = cf.update_dict(sv['x_norm_2'], {'scale': xn_scale}, it)
+    sv['gate'] = cf.update_dict(sv['gate'], {'scale': gate_scale}, it)
+    sv['up'] = cf.update_dict(sv['up'], {'scale': up_scale}, it)
     saved = dict(rstd=rstd, xm_o=xm_o, xm_q=xm_q, xm_scale=xm_scale, xm_idx=xm_idx, xn_q=xn_q, xn_scale=xn_scale,
-                 gate_q=q1, gate_scale=gs, up_q=q2, up_scale=us, gate_xa=gate_xa, up_xa=up_xa, gu_xa=gu_xa, down_xa=down_xa,
-                 q_bit=q, shape=(B, M, H))
+                 gate_q=q1, gate_scale=gs, up_q=q2, up_scale=us, gate_xa=gate_xa, up_xa=up_xa, gu_xa=gu_xa,
+                 down_xa=down_xa64[:, :16], q_bit=q, shape=(B, M, H))
     return x_out.reshape(B, M, H), saved
 
 
@@ -258,46 +245,28 @@ def mlp_backward(grad_out, saved, w: MLPWeights, status=None, on_lora_grads=None
     as soon as the six LoRA gradients are enqueued, before the grad_x GEMM and the RMSNorm backward: the
     place to start their all-reduce so that it overlaps the rest of the pass."""
     B, M, H = saved['shape']
-    T, I, q = B * M, w.wg.shape[0], saved['q_bit']
+    T, q = B * M, saved['q_bit']
     dev = grad_out.device
     st = status if status is not None else _status_tensor(dev)
     g = grad_out.to(BF16).reshape(T, H).contiguous()
-    down_xa, gate_xa, up_xa = saved['down_xa'], saved['gate_xa'], saved['up_xa']
-
     pad = w.padded()
-    grad_bd = g.t() @ down_xa                      # [H, r]
-    gdm64 = g @ pad["bd_cols"]                     # [T, 64], first 16 columns = g @ Bd
-    gdm = gdm64[:, :16]
-    had = torch.empty((T, I), dtype=BF16, device=dev)
-    ggu = torch.empty((2, T, I), dtype=BF16, device=dev)       # grad_gate and grad_up in one buffer: their rank-16
-    gg, gu = ggu[0], ggu[1]                                    # products below run as one batched call each
-    check(lib.hyc_mlp_graddown_bwd_tcgen05(
-        ptr(g), ptr(w.wd), T, H, I, ptr(gdm64), ptr(pad["ad_rows"]), 64,
-        ptr(gate_xa), ptr(w.bg), 16, 1, ptr(up_xa), ptr(w.bu), 16, 1,
-        ptr(saved['gate_q']), ptr(saved['gate_scale']), ptr(saved['up_q']), ptr(saved['up_scale']),
-        None, None, 0,
-        ptr(had), ptr(gg), ptr(gu), q, ptr(st), stream_of(grad_out)), "hyc_mlp_graddown_bwd_tcgen05")
-    grad_ad = gdm.t() @ had                        # [r, I]
-
     gm64 = padded_block(w, "_gm64", T, dev)
-    # g_gate @ Bg and g_up @ Bu ([T, r] each) as one batched product, then side by side into the zero-padded K block
-    # (B200, 2048 tokens: 19.8 us against 34.1 us as two products)
-    gm64.view(T, 4, 16)[:, :2].copy_(torch.bmm(ggu, pad["bgu"]).transpose(0, 1))
-    # LoRA-A gradients of gate and up in one pass over the packed x_norm (de-quantized in shared memory)
-    ga = lora_grad_a(saved['xn_q'].reshape(T, -1), saved['xn_scale'].to(BF16).reshape(-1).contiguous(), gm64, 32, q)
-    grad_ag, grad_au = ga[:16], ga[16:32]          # [r, H] each
     gu_xa = saved.get('gu_xa')
     if gu_xa is None:
-        gu_xa = torch.stack((gate_xa, up_xa))
-    grad_bgu = torch.bmm(ggu.transpose(1, 2), gu_xa)           # [2, I, r]
-    grad_bg, grad_bu = grad_bgu[0], grad_bgu[1]
+        gu_xa = torch.stack((saved['gate_xa'], saved['up_xa']))
+    # grad_down GEMM with the SiLU-Hadamard backward in its epilogue (grad_gate and grad_up land in one buffer, their
+    # rank-16 products run as one batched call each), then the six LoRA gradients: the A side of gate and up in one
+    # pass over the packed x_norm, de-quantized in shared memory
+    had, ggu, grad_bd, grad_ad, ga, grad_bgu = host.mlp_backward_lora(
+        g, [w.wd, w.bg, w.bu, pad["bd_cols"], pad["ad_rows"], pad["bgu"]],
+        [saved['gate_q'], saved['gate_scale'], saved['up_q'], saved['up_scale'], gu_xa, saved['down_xa'], saved['xn_q'],
+         saved['xn_scale']], gm64, q, st)
+    grads = dict(grad_ag=ga[:16], grad_bg=grad_bgu[0], grad_au=ga[16:32], grad_bu=grad_bgu[1], grad_ad=grad_ad, grad_bd=grad_bd)
     if on_lora_grads is not None:
-        on_lora_grads(dict(grad_ag=grad_ag, grad_bg=grad_bg, grad_au=grad_au, grad_bu=grad_bu, grad_ad=grad_ad,
-                           grad_bd=grad_bd))
-    # grad wrt x_norm: gate and up products accumulate in one tensor-memory tile
-    grad_xn = gemm(gg, w.wg, b_is_kn=True, a2=gu, b2=w.wu, a3=gm64, b3=pad["agu_rows"], status=st)
-    # RMSNorm backward straight from the saved form of x_medium, residual gradient added in the same pass
-    grad_x = rmsnorm_backward_packed(grad_xn.reshape(B, M, H), saved['xm_q'], saved['xm_scale'], saved['xm_o'],
-                                     saved['xm_idx'], w.norm_w, saved['rstd'], q, residual_grad=g.reshape(B, M, H))
-    return dict(grad_x=grad_x, grad_ag=grad_ag, grad_bg=grad_bg, grad_au=grad_au, grad_bu=grad_bu,
-                grad_ad=grad_ad, grad_bd=grad_bd, hadamard=had, g_gate=gg, g_up=gu)
+        on_lora_grads(dict(grads))
+    # grad wrt x_norm (gate, up and LoRA products accumulate in one tensor-memory tile), then the RMSNorm backward
+    # straight from the saved form of x_medium with the residual gradient added in the same pass
+    grad_x = host.mlp_backward_x(g, ggu, gm64, [w.wg, w.wu, pad["agu_rows"], w.norm_w],
+                                 [saved['xm_q'], saved['xm_scale'], saved['xm_o'], saved['xm_idx'], saved['rstd']],
+                                 [B, M, H], q, st)
+    return dict(grads, grad_x=grad_x, hadamard=had, g_gate=ggu[0], g_up=ggu[1])

@@ -20,7 +20,7 @@ format above.
 """
 import torch
 
-from ._lib import check, lib, ptr, require_cuda, stream_of
+from ._lib import host, require_cuda
 
 BF16 = torch.bfloat16
 
@@ -79,15 +79,10 @@ class QuantizedWeight:
             self.absmax = qs.absmax.to(device=dev, dtype=torch.float32).contiguous()
 
     def dequantize(self):
-        out = torch.empty(self.shape, dtype=BF16, device=self.device)
         if self.nested:
-            check(lib.hyc_dequant_nf4(ptr(self.packed), ptr(self.code), None, ptr(self.absmax), ptr(self.code2),
-                                      ptr(self.absmax2), self.blocksize2, self.offset, self.numel, self.blocksize,
-                                      ptr(out), stream_of(self.packed)), "hyc_dequant_nf4")
-        else:
-            check(lib.hyc_dequant_nf4(ptr(self.packed), ptr(self.code), ptr(self.absmax), None, None, None, 1, 0.0,
-                                      self.numel, self.blocksize, ptr(out), stream_of(self.packed)), "hyc_dequant_nf4")
-        return out
+            return host.dequant_nf4(self.packed, self.code, self.absmax, self.code2, self.absmax2, self.blocksize2, self.offset,
+                                    self.blocksize, self.shape)
+        return host.dequant_nf4(self.packed, self.code, self.absmax, None, None, 1, 0.0, self.blocksize, self.shape)
 
 
 _CACHE_ATTRS = ("_pad", "_pad_key", "_gm64", "_gmq")      # what AttnWeights / MLPWeights keep between steps

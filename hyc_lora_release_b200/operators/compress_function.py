@@ -17,7 +17,7 @@ import ctypes
 import torch
 
 from .. import _lib
-from .._lib import check, lib, ptr, require_cuda, stream_of
+from .._lib import check, host, lib, ptr, require_cuda, stream_of
 
 BF16 = torch.bfloat16
 
@@ -53,23 +53,6 @@ def _as_hidden(x):
     if x.dim() != 3:
         raise ValueError("expected a [B, M, N] or [B, heads, M, d] tensor, got shape %s" % (tuple(x.shape),))
     return x
-
-
-def _rows_view(x):
-    """[B, M, N] bf16 -> (tensor whose memory is [B*M rows, N] with one row stride, rows, ld)."""
-    x = x.to(BF16)
-    B, M, N = x.shape
-    if x.stride(2) != 1 or (B > 1 and x.stride(0) != M * x.stride(1)) or x.stride(1) < N \
-            or x.stride(1) % 8 != 0 or x.data_ptr() % 16 != 0:
-        x = x.contiguous()
-    return x, B * M, x.stride(1)
-
-
-def _scale_vec(s, N):
-    s = s.to(BF16).reshape(-1)
-    if s.numel() != N:
-        raise ValueError("per-channel scale with %d entries for %d channels (per-tensor scales cannot be quantized with)" % (s.numel(), N))
-    return s.contiguous()
 
 
 def _check_q(q_bit):
@@ -147,56 +130,12 @@ def get_statistics_channel_base(x: torch.Tensor, outlier_ratio: float, q_bit: in
 # ******************** compress / decompress interface ********************
 
 def _quant(x, s, q_bit, z=None, channel=None, out=None):
-    require_cuda(x, s)
-    _check_q(q_bit)
-    x = _as_hidden(x)
-    xr, rows, ld = _rows_view(x)
-    B, M, N = x.shape
-    if N % 32 != 0:
-        raise ValueError("the hidden size must be a multiple of 32")
-    s = _scale_vec(s, N)
-    zt = None
-    if z is not None:
-        zt = z.reshape(-1).to(torch.int8).contiguous()
-    epp = 8 // q_bit
-    k, idx, xo = 0, None, None
-    if channel is not None:
-        idx = channel.to(device=x.device, dtype=torch.int64).contiguous()
-        k = idx.numel()
     if out is not None:      # caller-provided (q, x_outlier) buffers, e.g. reused across steps
-        q, xo = out
-    else:
-        q = torch.empty((B, M, N // epp), dtype=torch.uint8, device=x.device)
-        if channel is not None:
-            xo = torch.empty((B, M, k), dtype=BF16, device=x.device)
-    if rows == 0:
-        return q, xo
-    check(lib.hyc_quant_pack(ptr(xr), rows, N, ld, ptr(s), ptr(zt), ptr(idx) if k else None, k, ptr(q),
-                             ptr(xo) if k else None, q_bit, stream_of(x)), "hyc_quant_pack")
-    return q, xo
+        return host.quant(x, s, q_bit, z, channel, out[0], out[1])
+    return host.quant(x, s, q_bit, z, channel, None, None)
 
 
-def _dequant(q, s, q_bit, z=None, channel=None, x_outlier=None, out=None):
-    require_cuda(q, s)
-    _check_q(q_bit)
-    B, M, _ = q.shape
-    N = s.shape[-1]
-    q = q.contiguous()
-    s = _scale_vec(s, N)
-    zt = None
-    if z is not None:
-        zt = z.reshape(-1).to(torch.int8).contiguous()
-    x = out if out is not None else torch.empty((B, M, N), dtype=BF16, device=q.device)
-    if B * M == 0:
-        return x
-    k, idx, xo = 0, None, None
-    if channel is not None:
-        idx = channel.to(device=q.device, dtype=torch.int64).contiguous()
-        k = idx.numel()
-        xo = x_outlier.to(BF16).contiguous()
-    check(lib.hyc_unpack_dequant(ptr(q), B * M, N, ptr(s), ptr(zt), ptr(idx) if k else None, k,
-                                 ptr(xo) if k else None, ptr(x), N, q_bit, stream_of(q)), "hyc_unpack_dequant")
-    return x
+_dequant = host.dequant      # (q, s, q_bit, zero point, channel, x_outlier, out)
 
 
 def outlier_subtraction_fuse_compression_quantization(x, s, channel, quantize_bit=8, dtype=torch.bfloat16, out=None):
@@ -210,7 +149,7 @@ def outlier_subtraction_fuse_compression_quantization(x, s, channel, quantize_bi
 def outlier_addition_fuse_decompression_dequantization(q, s, x_outlier, channel, quantize_bit=8, is_head=False,
                                                        num_heads=1, dtype=torch.bfloat16, out=None):
     """compress_function.py:147-174.  ``out`` (not in the reference): an existing [B,M,N] bf16 buffer."""
-    x = _dequant(q, s, quantize_bit, channel=channel, x_outlier=x_outlier, out=out)
+    x = _dequant(q, s, quantize_bit, None, channel, x_outlier, out)
     return hidden_to_head_shape(x, num_heads=num_heads) if is_head else x
 
 
@@ -221,7 +160,7 @@ def compression_quantization(x, s, quantize_bit=8, dtype=torch.bfloat16):
 
 def decompression_dequantization(q, s, quantize_bit=8, is_head=False, num_heads=1, dtype=torch.bfloat16):
     """compress_function.py:214-241 (the result is bf16 whatever ``dtype`` says, as there)."""
-    x = _dequant(q, s, quantize_bit)
+    x = _dequant(q, s, quantize_bit, None, None, None, None)
     return hidden_to_head_shape(x, num_heads=num_heads) if is_head else x
 
 
@@ -229,19 +168,7 @@ def decompression_dequantization_lora_add(q, s, x_lora_a, w_lora_b, quantize_bit
     """``decompression_dequantization(q, s, quantize_bit) + x_lora_a @ w_lora_b`` in one kernel (no counterpart
     in the reference, which runs the two steps: fused_llama_layer_intra_inter_full_fuse.py:416-452).
     q [B, M, N*bit/8], s [.., N], x_lora_a [B, M, 16], w_lora_b [16, N] (``lora_B.weight.T``) -> [B, M, N] bf16."""
-    from ._fused_common import lora_b_transposed
-    require_cuda(q, s, x_lora_a, w_lora_b)
-    _check_q(quantize_bit)
-    B, M, _ = q.shape
-    N = s.shape[-1]
-    sc = _scale_vec(s, N)
-    xa = x_lora_a.to(BF16).contiguous()
-    bt = lora_b_transposed(w_lora_b)
-    y = torch.empty((B, M, N), dtype=BF16, device=q.device)
-    if B * M:
-        check(lib.hyc_dequant_lora_add(ptr(q.contiguous()), ptr(sc), ptr(xa), ptr(bt), ptr(y), B * M, N, xa.shape[-1],
-                                       quantize_bit, stream_of(q)), "hyc_dequant_lora_add")
-    return y
+    return host.dequant_lora_add(q, s, x_lora_a, w_lora_b, quantize_bit)
 
 
 def compression_quantization_with_zero_point(x, s, z, quantize_bit=8, dtype=torch.bfloat16):
@@ -252,7 +179,7 @@ def compression_quantization_with_zero_point(x, s, z, quantize_bit=8, dtype=torc
 def decompression_dequantization_with_zero_point(q, s, z, quantize_bit=8, is_head=False, num_heads=1,
                                                  dtype=torch.bfloat16):
     """compress_function.py:278-306."""
-    x = _dequant(q, s, quantize_bit, z=z)
+    x = _dequant(q, s, quantize_bit, z, None, None, None)
     return hidden_to_head_shape(x, num_heads=num_heads) if is_head else x
 
 
@@ -263,31 +190,13 @@ def compression_softmax(x: torch.Tensor, outlier):
     of the flattened map (int64 indices, values in x's dtype), built by a two-phase stream
     compaction.  One device-to-host copy of the count sizes the result, as in ``to_sparse``."""
     require_cuda(x)
-    xf = x.to(BF16).contiguous()
-    numel = xf.numel()
-    thr = float(outlier)
-    ws_bytes = lib.hyc_softmax_prune_workspace_bytes(numel)
-    ws = torch.empty((ws_bytes + 7) // 8, dtype=torch.int64, device=x.device)
-    st = stream_of(x)
-    check(lib.hyc_softmax_prune_count(ptr(xf), numel, thr, ptr(ws), ws_bytes, st), "hyc_softmax_prune_count")
-    nnz = int(ws[0].item())
-    idx = torch.empty((1, nnz), dtype=torch.int64, device=x.device)
-    val = torch.empty(nnz, dtype=BF16, device=x.device)
-    check(lib.hyc_softmax_prune_fill(ptr(xf), numel, thr, ptr(ws), ptr(idx) if nnz else None,
-                                     ptr(val) if nnz else None, nnz, st), "hyc_softmax_prune_fill")
-    return torch.sparse_coo_tensor(idx, val, (numel,), is_coalesced=True)
+    return host.prune_sparse(x, float(outlier))
 
 
 def decompression_softmax(x_sparse: torch.Tensor):
     """compress_function.py:316-317 (flattened dense map; callers reshape)."""
     require_cuda(x_sparse)
-    idx = x_sparse.indices().reshape(-1).contiguous()
-    val = x_sparse.values().to(BF16).contiguous()
-    numel = x_sparse.shape[0]
-    out = torch.empty(numel, dtype=BF16, device=val.device)
-    check(lib.hyc_softmax_prune_restore(ptr(idx) if idx.numel() else None, ptr(val) if idx.numel() else None,
-                                        idx.numel(), ptr(out), numel, stream_of(val)), "hyc_softmax_prune_restore")
-    return out
+    return host.prune_restore(x_sparse.indices(), x_sparse.values(), x_sparse.shape[0])
 
 
 class PrunedMap:
@@ -350,13 +259,9 @@ class TiledPrunedMap:
         numel = 1
         for d in self.shape:
             numel *= d
-        if out is None:
-            out = torch.empty(self.shape, dtype=BF16, device=self.words.device)
-        elif out.numel() != numel or out.dtype != BF16 or not out.is_contiguous():
+        if out is not None and (out.numel() != numel or out.dtype != BF16 or not out.is_contiguous()):
             raise ValueError("`out` must be a contiguous bf16 tensor with the map's number of elements")
-        check(lib.hyc_softmax_prune_tiled_restore(ptr(self.words), self.capacity, ptr(self.directory), ptr(out), numel,
-                                                  stream_of(self.words)), "hyc_softmax_prune_tiled_restore")
-        return out
+        return host.prune_tiled_restore(self.words, self.directory, self.shape, out)
 
     def entries(self):
         """(flattened index int64, value bf16) of the stored entries in ascending index order, decoded with torch
@@ -391,20 +296,16 @@ def compression_softmax_static(x: torch.Tensor, outlier, capacity=None, margin=1
     library's built-in scratch: maps of up to 268,435,456 elements, calls on one GPU must not overlap (they share
     that scratch), and the first call on a device must be made outside of stream capture."""
     require_cuda(x)
-    xf = x.to(BF16).contiguous()
-    numel = xf.numel()
+    numel = x.numel()
     if capacity is None:
         if ratio is None:
             raise ValueError("give `capacity` or the calibrated `ratio`")
         capacity = int(numel * ratio * margin) + 1024
     capacity = min(int(capacity), numel)
-    nnz = torch.empty(1, dtype=torch.int64, device=x.device)
     if not ordered:
-        words = torch.empty(capacity, dtype=torch.int32, device=x.device)
-        directory = torch.empty(lib.hyc_softmax_prune_tiled_directory_bytes(numel) // 4, dtype=torch.int32, device=x.device)
-        check(lib.hyc_softmax_prune_tiled(ptr(xf), numel, float(outlier), ptr(words), capacity, ptr(directory), ptr(nnz),
-                                          stream_of(x)), "hyc_softmax_prune_tiled")
-        return TiledPrunedMap(words, directory, nnz, x.shape)
+        return TiledPrunedMap(*host.prune_tiled(x, float(outlier), capacity), x.shape)
+    xf = x.to(BF16).contiguous()
+    nnz = torch.empty(1, dtype=torch.int64, device=x.device)
     idx = torch.empty(capacity, dtype=torch.int64, device=x.device)
     val = torch.empty(capacity, dtype=BF16, device=x.device)
     check(lib.hyc_softmax_prune_static(ptr(xf), numel, float(outlier), ptr(idx), ptr(val), capacity, ptr(nnz),
@@ -466,66 +367,31 @@ class TopkMap:
         """``softmax_backward(self.to_dense(), grad)`` (operators/softmax_kernels.py:41) without writing the
         restored map: one kernel where the shapes allow it, restore + softmax backward otherwise.  ``scale``: the
         bf16 result times ``scale`` as a second bf16 operation (the layer's ``grad_s / sqrt(head_dim)``)."""
-        require_cuda(grad, self.q)
-        g = grad.to(BF16).contiguous()
-        if tuple(g.shape) != self.shape:
-            raise ValueError("the gradient must have the map's shape %s" % (self.shape,))
-        S, rows, k = self.shape[-1], self.q.shape[0], self.val.shape[1]
-        if out is None:
-            out = torch.empty(self.shape, dtype=BF16, device=self.q.device)
-        rc = lib.hyc_softmax_topk_restore_bwd(ptr(self.val) if k else None, ptr(self.col) if k else None, k, ptr(self.q),
-                                              ptr(self.scale), ptr(self.zp), rows, S, ptr(g), ptr(out), self.q_bit,
-                                              float(scale), stream_of(self.q))
-        if rc == -8:      # HYC_ERR_UNSUPPORTED: shape outside the fused kernel
-            from .softmax_kernels import softmax_backward as _sb
-            res = _sb(self.to_dense(), g, scale)
-            out.copy_(res.reshape(self.shape))
-            return out
-        check(rc, "hyc_softmax_topk_restore_bwd")
-        return out
+        return host.topk_softmax_backward(self.val, self.col, self.q, self.scale, self.zp, self.shape, self.q_bit, grad,
+                                          out, float(scale))
 
 
 def compression_softmax_topk(x, outlier_ratio, quantize_bit=4, out=None):
     """Top-k per row (k = int(S * ratio)) as bf16 value + uint16 column, the remainder
     group-quantized.  x [..., S] with S % 64 == 0, S <= 4096.  ``out``: a TopkMap of an earlier call
     on the same shape, ratio and bit width whose buffers are overwritten (a ring of saved maps)."""
-    require_cuda(x)
-    _check_q(quantize_bit)
-    xb = x.to(BF16).contiguous()
-    S = xb.shape[-1]
-    rows = xb.numel() // S
+    S = x.shape[-1]
     k = int(S * outlier_ratio)
-    dev = x.device
-    if out is not None:
-        if (out.shape != tuple(x.shape) or out.q_bit != quantize_bit or out.val.shape != (rows, k)
-                or out.q.device != dev):
-            raise ValueError("`out` was made for another shape, ratio, bit width or device")
-        val, col, q, s, z = out.tensors()
-    else:
-        val = torch.empty((rows, k), dtype=BF16, device=dev)
-        col = torch.empty((rows, k), dtype=torch.int16, device=dev)   # holds uint16 column numbers
-        q = torch.empty((rows, S * quantize_bit // 8), dtype=torch.uint8, device=dev)
-        s = torch.empty((rows, S // 64), dtype=BF16, device=dev)
-        z = torch.empty((rows, S // 64), dtype=torch.int8, device=dev)
-    check(lib.hyc_softmax_topk_compress(ptr(xb), rows, S, k, ptr(val) if k else None, ptr(col) if k else None,
-                                        ptr(q), ptr(s), ptr(z), quantize_bit, stream_of(x)),
-          "hyc_softmax_topk_compress")
-    return out if out is not None else TopkMap(val, col, q, s, z, x.shape, quantize_bit)
+    if out is None:
+        return TopkMap(*host.topk_compress(x, k, quantize_bit), x.shape, quantize_bit)
+    require_cuda(x)
+    if (out.shape != tuple(x.shape) or out.q_bit != quantize_bit or out.val.shape != (x.numel() // S, k)
+            or out.q.device != x.device):
+        raise ValueError("`out` was made for another shape, ratio, bit width or device")
+    host.topk_compress_into(x, k, quantize_bit, *out.tensors())
+    return out
 
 
 def decompression_softmax_topk(m: TopkMap, out=None):
     """``out``: an existing contiguous bf16 tensor of the map's shape."""
-    S = m.shape[-1]
-    rows = m.q.shape[0]
-    k = m.val.shape[1]
-    if out is None:
-        out = torch.empty(m.shape, dtype=BF16, device=m.q.device)
-    elif tuple(out.shape) != m.shape or out.dtype != BF16 or not out.is_contiguous() or out.device != m.q.device:
+    if out is not None and (tuple(out.shape) != m.shape or out.dtype != BF16 or not out.is_contiguous() or out.device != m.q.device):
         raise ValueError("`out` must be a contiguous bf16 tensor of shape %s on the map's device" % (m.shape,))
-    check(lib.hyc_softmax_topk_restore(ptr(m.val) if k else None, ptr(m.col) if k else None, k, ptr(m.q),
-                                       ptr(m.scale), ptr(m.zp), rows, S, ptr(out), m.q_bit, stream_of(m.q)),
-          "hyc_softmax_topk_restore")
-    return out
+    return host.topk_restore(m.val, m.col, m.q, m.scale, m.zp, m.shape, m.q_bit, out)
 
 
 # ******************** pack "get statistics" and "compress" ********************

@@ -1,7 +1,7 @@
 """Drop-in for the reference's ``operators/softmax_kernels.py`` wrapper (:41-56)."""
 import torch
 
-from .._lib import check, lib, ptr, require_cuda, stream_of
+from .._lib import check, host, lib, ptr, require_cuda, stream_of
 
 BF16 = torch.bfloat16
 
@@ -9,13 +9,8 @@ BF16 = torch.bfloat16
 def softmax_backward(y, grad_y, scale=1.0):
     """o = (grad_y - sum(y * grad_y, -1)) * y for a [b, h, n, n] map.  ``scale`` (extension): the bf16 result
     times ``scale`` as a second bf16 operation, for the layer's ``grad_s / sqrt(head_dim)``."""
-    require_cuda(y, grad_y)
     assert grad_y.shape == y.shape
-    yc, gc = y.to(BF16).contiguous(), grad_y.to(BF16).contiguous()
-    S = yc.shape[-1]
-    o = torch.empty_like(yc)
-    check(lib.hyc_softmax_bwd(ptr(yc), ptr(gc), ptr(o), yc.numel() // S, S, float(scale), stream_of(y)), "hyc_softmax_bwd")
-    return o
+    return host.softmax_backward(y, grad_y, float(scale))
 
 
 def _mask_args(attention_mask, b, h, n, S):
@@ -81,30 +76,4 @@ def softmax_forward_scale_mask(scores, scale, attention_mask=None, inplace=False
     operations, the softmax is fp32 inside with a bf16 result;
     models/llama/fused_llama_layer_intra_inter_full_fuse.py:150-160).  ``attention_mask``: additive, broadcastable
     as [b, 1 or h, n, S].  ``inplace`` overwrites ``scores`` (which must then be contiguous bf16)."""
-    require_cuda(scores, attention_mask)
-    if scores.dim() != 4:
-        raise ValueError("scores must be [batch, heads, n, S]")
-    if inplace and (scores.dtype != BF16 or not scores.is_contiguous()):
-        raise ValueError("inplace needs contiguous bf16 scores")
-    sc = scores.to(BF16).contiguous()
-    b, h, n, S = sc.shape
-    out = sc if inplace else torch.empty_like(sc)
-    mb = mh = mr = 0
-    mk = None
-    if attention_mask is not None:
-        mk = attention_mask.to(BF16)
-        if mk.dim() != 4 or mk.shape[-1] != S or mk.shape[-2] != n or mk.shape[0] not in (1, b) or mk.shape[1] not in (1, h):
-            raise ValueError("attention_mask must be [b or 1, h or 1, n, S]")
-        if mk.stride(-1) != 1:
-            mk = mk.contiguous()
-        mb = 0 if mk.shape[0] == 1 else mk.stride(0)
-        mh = 0 if mk.shape[1] == 1 else mk.stride(1)
-        mr = mk.stride(2)
-        if (mb | mh | mr) & 7 or mk.data_ptr() & 15:
-            mk = mk.contiguous()
-            mb = 0 if mk.shape[0] == 1 else mk.stride(0)
-            mh = 0 if mk.shape[1] == 1 else mk.stride(1)
-            mr = mk.stride(2)
-    check(lib.hyc_softmax_fwd_scale_mask(ptr(sc), float(scale), ptr(mk), mb, mh, mr, h, n, ptr(out), b * h * n, S,
-                                         stream_of(scores)), "hyc_softmax_fwd_scale_mask")
-    return out
+    return host.softmax_forward(scores, float(scale), attention_mask, inplace)
