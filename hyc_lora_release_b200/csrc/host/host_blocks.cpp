@@ -2,6 +2,7 @@
 // What each step is and which rounding points it has is documented in mlp.py and attention.py, which own the
 // calibration branch and the weight records.
 #include "host.h"
+#include <array>
 #include <cmath>
 
 namespace hyc_host {
@@ -24,15 +25,28 @@ static Tensor lora_a_products(const Tensor& x2, const Tensor& stacked) {
   return at::bmm(x2.unsqueeze(0).expand({stacked.size(0), -1, -1}), stacked);
 }
 
-static std::tuple<Tensor, Tensor> linear_lora_save(const Tensor& x, const Tensor& w, const Tensor& xa, const Tensor& b, const Tensor& scale,
-                                                   int64_t q_bit, const Tensor& status) {
+// the q, k and v projections with the saves of their main branches in one launch: -> {y, codes} of each
+static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, const std::array<const Tensor*, 3>& w, const Tensor& xa3,
+                                                              const std::array<const Tensor*, 3>& b, const std::array<const Tensor*, 3>& scale,
+                                                              int64_t q_bit, const Tensor& status) {
   OnDevice on(x);
-  const int64_t T = x.size(0), K = x.size(1), N = w.size(0);
-  const Tensor sc = vec(scale), bc = b.contiguous();
-  Tensor y = empty({T, N}, x), qm = empty({T, N * q_bit / 8}, x, at::kByte);
-  check(hyc_linear_lora_save_fwd_tcgen05(data(x), data(w), (int)T, (int)K, (int)N, data(xa), data(bc), bc.size(1), 1, data(sc), data(qm),
-                                         data(y), nullptr, (int)q_bit, status_ptr(status), on.stream), "hyc_linear_lora_save_fwd_tcgen05");
-  return {y, qm};
+  const int64_t T = x.size(0), K = x.size(1);
+  std::array<std::pair<Tensor, Tensor>, 3> out;
+  Tensor keep[6];
+  const void *wp[3], *xp[3], *bp[3], *sp[3];
+  void *qp[3], *yp[3];
+  int n[3];
+  for (int i = 0; i < 3; ++i) {
+    n[i] = (int)w[i]->size(0);
+    out[i] = {empty({T, n[i]}, x), empty({T, n[i] * q_bit / 8}, x, at::kByte)};
+    keep[2 * i] = vec(*scale[i]);
+    keep[2 * i + 1] = b[i]->contiguous();
+    wp[i] = data(*w[i]); xp[i] = (const char*)xa3.data_ptr() + i * T * 16 * 2; bp[i] = data(keep[2 * i + 1]); sp[i] = data(keep[2 * i]);
+    yp[i] = data(out[i].first); qp[i] = data(out[i].second);
+  }
+  check(hyc_linears_lora_save_fwd_tcgen05(data(x), (int)T, (int)K, 3, wp, n, xp, bp, sp, qp, yp, (int)q_bit, status_ptr(status), on.stream),
+        "hyc_linears_lora_save_fwd_tcgen05");
+  return out;
 }
 
 Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64_t r2, int64_t q_bit) {
@@ -139,9 +153,10 @@ static std::vector<Tensor> attn_forward_map(const Tensor& x, const std::vector<T
   auto [x_norm, rstd, x_o, x_q, xn_q] = rmsnorm_save(x, norm_w, eps, q, x_scale, x_idx, xn_scale);
   const Tensor xn2 = x_norm.view({T, H});
   const Tensor xa3 = lora_a_products(xn2, aqkv_t);
-  auto [qy, q_q] = linear_lora_save(xn2, wq, xa3[0], bq, q_scale, q, status);
-  auto [ky, k_q] = linear_lora_save(xn2, wk, xa3[1], bk, k_scale, q, status);
-  auto [vy, v_q] = linear_lora_save(xn2, wv, xa3[2], bv, v_scale, q, status);
+  auto p3 = qkv_lora_save(xn2, {&wq, &wk, &wv}, xa3, {&bq, &bk, &bv}, {&q_scale, &k_scale, &v_scale}, q, status);
+  const auto &[qy, q_q] = p3[0];
+  const auto &[ky, k_q] = p3[1];
+  const auto &[vy, v_q] = p3[2];
   rope(qy.view({B, M, nh, d}), cos, sin, false, true);
   rope(ky.view({B, M, nkv, d}), cos, sin, false, true);
   const Tensor kh = repeat_kv(heads(ky, B, M, nkv), rep), vh = repeat_kv(heads(vy, B, M, nkv), rep);

@@ -1,0 +1,358 @@
+// The GEMMs of the layer for few tokens: one 128 x 128 tile per cluster of S = 1, 2 or 4 CTAs, each CTA contracting
+// one S-th of K; the partial accumulators meet in distributed shared memory and every CTA finishes 1/S of the tile's
+// columns with the same epilogues as the persistent kernel (mlp_tcgen05.cu).
+//
+// Why: below about a thousand tokens a 256 x 256 tile per CTA pair leaves most of the chip idle ([128, 4096] x
+// [4096, 4096]: 16 tiles on 74 pairs) while the product is bound by streaming the weights from HBM.  Here every SM
+// streams its own slice of the weight with two CTAs of three 32 KB stages (or one of six) in flight; the A tile comes
+// from L2.  With 129 tokens and more the tile belongs to a CTA pair (M 256, tcgen05 cta_group::2, each CTA loading half
+// of the B block), which cuts what an SM pulls out of L2 per k-block from 32 to 24 KB; a cluster is then 2 S CTAs.
+// The reduction order is fixed (rank 0, 1, ...), so results do not depend on the run.
+#include "tc_split.cuh"
+#include <stdlib.h>
+
+namespace hyc {
+namespace tc {
+
+constexpr int SBN = 128;                          // accumulator columns per tile
+constexpr int S_PIPE_BYTES = 98304;               // pipeline memory of a CTA that shares its SM (twice that if it does not)
+constexpr int S_MAX_STAGES = 8;
+constexpr int S_EPI_BYTES = 1024;                 // per-column constants
+constexpr int S_THREADS = 64 + 128;
+constexpr int S_PART_BYTES = SBN * BM * 4;        // the CTA's accumulators as [column][row], over the drained stages
+static_assert(S_PART_BYTES + 4 * 4096 <= S_PIPE_BYTES, "partials and the GRADDOWN tiles fit in the drained pipeline");
+constexpr int split_smem_bytes(int pipe) { return 1024 + pipe + S_EPI_BYTES + 256; }
+
+__device__ __forceinline__ void s_epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
+// 32 accumulator columns from `col` of the thread's row: this CTA's tensor memory, or the sum over the cluster
+// (its CTAs that hold the same rows: ranks first, first + step, ...)
+__device__ __forceinline__ void gather32(int split, int first, int step, uint32_t t_lane, uint32_t part, int col, int r,
+                                         uint32_t (&acc)[32]) {
+  if (split == 1) {
+    tc_ld32(t_lane + (uint32_t)col, acc);
+    return;
+  }
+  float f[32];
+#pragma unroll
+  for (int c = 0; c < 32; ++c) f[c] = 0.f;
+  for (int s = 0; s < split; ++s) {
+    uint32_t base;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base) : "r"(part + (uint32_t)(col * BM + r) * 4u), "r"(first + s * step));
+#pragma unroll
+    for (int c = 0; c < 32; ++c) f[c] += ld_cluster_f32(base + (uint32_t)(c * BM * 4));
+  }
+#pragma unroll
+  for (int c = 0; c < 32; ++c) acc[c] = __float_as_uint(f[c]);
+}
+
+template <int EPI, int QBIT, bool B_MN, bool PAIR>
+__global__ void __launch_bounds__(S_THREADS, 2)
+split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, int stages, int a_bytes) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  constexpr int TILE_M = PAIR ? 2 * BM : BM;
+  constexpr int B_BYTES = (PAIR ? SBN / 2 : SBN) * BK * 2;        // this CTA's part of the B block
+  const int stage_bytes = a_bytes + B_BYTES;
+  uint8_t* epi = smem + (stages * stage_bytes + 1023) / 1024 * 1024;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epi + S_EPI_BYTES);
+  uint64_t *full = bars, *empty = bars + S_MAX_STAGES, *acc_full = bars + 2 * S_MAX_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S_MAX_STAGES + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int crank = PAIR || split > 1 ? (int)cluster_ctarank() : 0;
+  const int half = PAIR ? crank & 1 : 0, rank = PAIR ? crank >> 1 : crank;      // which rows of the tile, which slice of K
+  const uint32_t leader = (uint32_t)(crank & ~1);                               // PAIR: the CTA that issues the pair's MMAs
+  constexpr int TILE_N = EPI == EPI_GATEUP ? SBN / 2 : SBN;
+  constexpr int UNITS = TILE_N / 32;
+  const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
+  const int tile = (int)blockIdx.x / (PAIR ? 2 * split : split);
+  const int m0 = (tile % tiles_m) * TILE_M + half * BM, nt = (tile / tiles_m) * TILE_N;
+  const int kb1 = p.K1 / BK, kb2 = (p.K1 + p.K2) / BK, kb_total = (p.K1 + p.K2 + p.K3) / BK;
+  const int kb_lo = (int)((int64_t)kb_total * rank / split), kb_hi = (int)((int64_t)kb_total * (rank + 1) / split);
+  const StoreView sv = store_view(p, nt);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(SBN) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(SBN) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();      // the peer's barriers exist before anything is signalled there
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int et = (int)threadIdx.x - 64, quad = warp & 3;
+  const int64_t row0 = (int64_t)m0 + quad * 32;
+  const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+  float* part = reinterpret_cast<float*>(smem);
+  float* sV = reinterpret_cast<float*>(epi);                       // quantizer constants (GATEUP: second vector at sV + 64)
+  __nv_bfloat16* sS = reinterpret_cast<__nv_bfloat16*>(sV);        // GRADDOWN: two bf16 scale vectors of 128
+  const int per = UNITS / split, first = rank * per;               // the 32-column blocks this CTA finishes
+  LoraA a1, a2;
+  LoraB b1, b2;
+  uint4 res[4];
+  GdInputs<QBIT> gin;
+  bool ok = true;
+
+  if (warp == 0) {
+    {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1u, abort_flag)) {
+          if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_PRODUCER); }
+          break;
+        }
+        const int seg = kb < kb1 ? 0 : (kb < kb2 ? 1 : 2);
+        const int wsel = EPI == EPI_STORE && sv.group > 0 ? sv.group : seg;
+        const CUtensorMap *ma = &maps.a[seg], *mb = &maps.b[wsel];
+        const int k0 = (seg == 0 ? kb : (seg == 1 ? kb - kb1 : kb - kb2)) * BK;
+        const int n0 = EPI == EPI_STORE ? sv.n0 : nt;
+        const uint32_t sa = smem_u32(smem + stage * stage_bytes), sb = sa + (uint32_t)a_bytes;
+        const uint32_t fbar = PAIR ? map_to_cta(&full[stage], leader) : smem_u32(&full[stage]);
+        if (elect_one()) {
+        if (half == 0) mbar_expect_tx(&full[stage], (uint32_t)((PAIR ? 2 : 1) * stage_bytes));      // the leader counts both CTAs' bytes
+        if (EPI == EPI_GATEUP) {
+          if (PAIR) {
+            tma_load_2d<PAIR>(sb, half == 0 ? &maps.b[0] : &maps.b[1], fbar, k0, n0);
+          } else {
+            tma_load_2d<PAIR>(sb, &maps.b[0], fbar, k0, n0);
+            tma_load_2d<PAIR>(sb + 8192, &maps.b[1], fbar, k0, n0);
+          }
+        } else if (B_MN) {
+          tma_load_2d<PAIR>(sb, mb, fbar, n0 + 64 * half, k0);
+          if (!PAIR) tma_load_2d<PAIR>(sb + 8192, mb, fbar, n0 + 64, k0);
+        } else {
+          tma_load_2d<PAIR>(sb, mb, fbar, k0, n0 + 64 * half);
+        }
+        tma_load_2d<PAIR>(sa, ma, fbar, k0, m0);
+        }
+        __syncwarp();
+        if (++stage == stages) { stage = 0; phase ^= 1u; }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (half == 0) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((B_MN ? 1u : 0u) << 16) | ((uint32_t)(SBN >> 3) << 17) |
+                             ((uint32_t)(TILE_M >> 4) << 24);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool fine = true;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait_warp(&full[stage], phase, abort_flag)) {
+          if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_MMA); }
+          fine = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + stage * stage_bytes), sb = sa + (uint32_t)a_bytes;
+        const uint64_t adesc = make_desc(sa, 16, 1024);
+        const uint64_t bdesc = B_MN ? make_desc(sb, 64 * 128, 1024) : make_desc(sb, 16, 1024);
+        if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk)
+          tc_mma<PAIR>(tmem_base, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(B_MN ? kk * 128 : kk * 2), idesc,
+                        (kb > kb_lo || kk > 0) ? 1u : 0u);
+        tc_commit<PAIR>(&empty[stage], leader);
+        }
+        __syncwarp();
+        if (++stage == stages) { stage = 0; phase ^= 1u; }
+      }
+      if (fine && elect_one()) tc_commit<PAIR>(acc_full, leader);
+    }
+    __syncwarp();
+  } else {
+    // what the epilogue needs besides the accumulators is fetched while the main loop runs
+    if (EPI == EPI_STORE) {
+      if (sv.q != nullptr) sV[et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(sv.s[sv.n0 + et])));
+      if (sv.l0.bt != nullptr) {
+        lora_load_a(sv.l0.xa, row0, p.M, lane, a1);
+        lora_load_b(sv.l0, (int64_t)sv.n0 + 32 * first, lane, b1);
+      }
+      if (sv.residual != nullptr) tile_fetch(sv.residual, row0, p.M, sv.ld, (int64_t)sv.n0 + 32 * first, lane, res);
+    } else if (EPI == EPI_GATEUP) {
+      if (et < TILE_N) {
+        sV[et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(p.s1[nt + et])));
+        sV[64 + et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(p.s2[nt + et])));
+      }
+      lora_load_a(p.l0.xa, row0, p.M, lane, a1);
+      lora_load_a(p.l1.xa, row0, p.M, lane, a2);
+      lora_load_b(p.l0, (int64_t)nt + 32 * first, lane, b1);
+      lora_load_b(p.l1, (int64_t)nt + 32 * first, lane, b2);
+    } else {
+      sS[et] = p.s1[nt + et];
+      sS[128 + et] = p.s2[nt + et];
+      lora_load_a(p.l1.xa, row0, p.M, lane, a1);
+      lora_load_a(p.l2.xa, row0, p.M, lane, a2);
+      gd_fetch<QBIT>(p, row0, lane, (int64_t)nt + 32 * first, gin);
+    }
+    s_epi_sync();
+    ok = mbar_wait(acc_full, 0, abort_flag);
+    if (!ok && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_EPILOGUE); }
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    if (ok && split > 1) {
+      // the stages are drained (the accumulators are complete): they hold the partial sums now
+#pragma unroll 1
+      for (int c0 = 0; c0 < SBN; c0 += 32) {
+        uint32_t v[32];
+        tc_ld32(t_lane + (uint32_t)c0, v);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) part[(c0 + c) * BM + quad * 32 + lane] = __uint_as_float(v[c]);
+      }
+    }
+  }
+  // every CTA of the cluster has its partial sums in place (or has given up: the status word says so)
+  if (split > 1) cluster_sync_all();
+
+  if (warp >= 2 && ok) {
+    const uint32_t part_addr = smem_u32(part);
+    const int r = quad * 32 + lane;
+    // behind the partial sums
+    uint32_t *R1 = reinterpret_cast<uint32_t*>(smem + S_PART_BYTES) + (warp - 2) * 1024, *R2 = R1 + 512;
+#pragma unroll 1
+    for (int u = first; u < first + per; ++u) {
+      const int cb = 32 * u;
+      const bool more = u + 1 < first + per;
+      uint32_t acc[32];
+      if (EPI == EPI_GATEUP) {
+        uint32_t up[32];
+        const LoraB n1 = b1, n2 = b2;
+        if (more) {
+          lora_load_b(p.l0, (int64_t)nt + cb + 32, lane, b1);
+          lora_load_b(p.l1, (int64_t)nt + cb + 32, lane, b2);
+        }
+        gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
+        gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, TILE_N + cb, r, up);
+        epi_gateup_block<QBIT>(p, row0, lane, nt, cb, acc, up, a1, a2, n1, n2, sV, sV + 64, R1, R2);
+      } else if (EPI == EPI_STORE) {
+        const uint4 now[4] = {res[0], res[1], res[2], res[3]};
+        const LoraB n1 = b1;
+        if (more && sv.residual != nullptr) tile_fetch(sv.residual, row0, p.M, sv.ld, (int64_t)sv.n0 + cb + 32, lane, res);
+        if (more && sv.l0.bt != nullptr) lora_load_b(sv.l0, (int64_t)sv.n0 + cb + 32, lane, b1);
+        gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
+        epi_store_block<QBIT>(sv, row0, lane, p.M, cb, acc, a1, n1, sV, now, R1, R2);
+      } else {
+        const GdInputs<QBIT> cur = gin;
+        if (more) gd_fetch<QBIT>(p, row0, lane, (int64_t)nt + cb + 32, gin);
+        gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
+        epi_graddown_block<QBIT>(p, row0, lane, nt, cb, acc, cur, a1, a2, R1, R2, reinterpret_cast<const uint32_t*>(sS),
+                                 reinterpret_cast<const uint32_t*>(sS + 128));
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR || split > 1) cluster_sync_all();      // nobody leaves while a peer may still read its partial sums
+  if (warp == 1) {
+    tc_fence_after();
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(SBN) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(SBN) : "memory");
+  }
+}
+
+template <int EPI, int QBIT, bool B_MN, bool PAIR>
+static int launch_one(int split, const Operands& ops, const Params& p, cudaStream_t st) {
+  auto kern = split_gemm_kernel<EPI, QBIT, B_MN, PAIR>;
+  static bool attr[64] = {false};
+  const int slot = current_device_slot();
+  if (slot < 0 || !attr[slot]) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem_bytes(2 * S_PIPE_BYTES)) != cudaSuccess) {
+      hyc_set_last_cuda_error((int)cudaGetLastError());
+      return HYC_ERR_LAUNCH;
+    }
+    if (slot >= 0) attr[slot] = true;
+  }
+  constexpr int TILE_N = EPI == EPI_GATEUP ? SBN / 2 : SBN, TILE_M = PAIR ? 2 * BM : BM;
+  const int cluster = (PAIR ? 2 : 1) * split;
+  const int ctas = ((p.M + TILE_M - 1) / TILE_M) * (p.N / TILE_N) * cluster;
+  const int pipe = ctas <= num_sms() ? 2 * S_PIPE_BYTES : S_PIPE_BYTES;       // one CTA per SM, or room for two
+  const int a_bytes = (p.M <= 64 ? 64 : BM) * BK * 2;
+  const int stage_bytes = a_bytes + (PAIR ? SBN / 2 : SBN) * BK * 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(S_THREADS);
+  cfg.dynamicSmemBytes = split_smem_bytes(pipe);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  int stages = pipe / stage_bytes;
+  if (stages > S_MAX_STAGES) stages = S_MAX_STAGES;
+  Maps maps;
+  if (!make_maps(&maps, ops, B_MN, a_bytes / (BK * 2), EPI == EPI_GATEUP || PAIR ? 64 : 128, false)) return HYC_ERR_UNSUPPORTED;
+  if (cudaLaunchKernelEx(&cfg, kern, maps, p, split, stages, a_bytes) != cudaSuccess) {
+    hyc_set_last_cuda_error((int)cudaGetLastError());
+    return HYC_ERR_LAUNCH;
+  }
+  return HYC_OK;
+}
+
+int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Operands& ops, const Params& p, cudaStream_t st) {
+#define HYC_SPLIT(E, Q, MN) \
+  return plan.pair ? launch_one<E, Q, MN, true>(plan.split, ops, p, st) : launch_one<E, Q, MN, false>(plan.split, ops, p, st)
+  if (epi == EPI_STORE) {
+    if (b_mn) HYC_SPLIT(EPI_STORE, 4, true);
+    if (q_bit == 2) HYC_SPLIT(EPI_STORE, 2, false);
+    if (q_bit == 8) HYC_SPLIT(EPI_STORE, 8, false);
+    HYC_SPLIT(EPI_STORE, 4, false);
+  }
+  if (epi == EPI_GATEUP) {
+    if (q_bit == 2) HYC_SPLIT(EPI_GATEUP, 2, false);
+    if (q_bit == 8) HYC_SPLIT(EPI_GATEUP, 8, false);
+    HYC_SPLIT(EPI_GATEUP, 4, false);
+  }
+  if (q_bit == 2) HYC_SPLIT(EPI_GRADDOWN, 2, true);
+  if (q_bit == 8) HYC_SPLIT(EPI_GRADDOWN, 8, true);
+  HYC_SPLIT(EPI_GRADDOWN, 4, true);
+#undef HYC_SPLIT
+}
+
+// Where the line lies (B200, Llama-2-7B weights, us per product, persistent / split):
+//   up to 128 tokens, S = the largest of 4, 2, 1 with at most one CTA per SM: [128,4096]x[4096,4096] 21.8 / 16.6,
+//     x[4096,11008] 42 / 26.5, the three-segment grad_x 67 / 37, gate/up 48.9 / 43.8, q/k/v 38 / 33.  The grad_down
+//     product has more column tiles than SMs can take at once either way and stays persistent: 28.8 / 30.3
+//   129 to 256 tokens, pair form, S = 2: 21.8 / 19.0, 43 / 30.6, 69 / 45; wider products fill the chip without it
+//   512 tokens: 45 / 47, 75 / 77: persistent
+SplitPlan choose_split(int epi, const Params& p) {
+  SplitPlan plan = {0, false};
+#ifdef HYC_TUNE
+  if (const char* e = getenv("HYC_SPLIT")) { if (atoi(e) >= 100) return plan; plan.split = atoi(e) % 10; plan.pair = atoi(e) >= 10; return plan; }
+#endif
+  if (epi == EPI_GRADDOWN || p.M > 2 * BM) return plan;
+  if (epi == EPI_STORE && p.l1.bt != nullptr) return plan;         // a second LoRA term: the persistent kernel's own epilogue
+  const int tiles = p.N / (epi == EPI_GATEUP ? SBN / 2 : SBN), sms = num_sms();
+  if (p.M <= BM) {
+    plan.split = 1;
+    for (int s = 2; s <= (epi == EPI_GATEUP ? 2 : 4); s *= 2)
+      if (tiles * s <= sms) plan.split = s;
+  } else if (epi == EPI_STORE && tiles * 4 <= sms) {
+    plan = {2, true};
+  }
+  return plan;
+}
+
+}  // namespace tc
+}  // namespace hyc

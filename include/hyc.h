@@ -310,6 +310,12 @@ int hyc_linear_lora_save_fwd_tcgen05(const void* x, const void* w, int T, int K,
                                      const void* scale, void* q_out, void* y, void* main_or_null, int q_bit,
                                      int* status, void* stream);
 
+/* The same for up to three weights on one x (q, k and v) in ONE launch: host arrays of `count` entries; w[i] is
+ * [n[i], K], xa[i] [T,16], bt[i] [n[i],16], q_out[i] / y[i] with n[i] columns. n[i] % 256 == 0, K % 64 == 0. */
+int hyc_linears_lora_save_fwd_tcgen05(const void* x, int T, int K, int count, const void* const* w, const int* n,
+                                      const void* const* xa, const void* const* bt, const void* const* scale,
+                                      void* const* q_out, void* const* y, int q_bit, int* status, void* stream);
+
 /* gate/up projections and triton_fuse_silu_forward in one kernel
  * (fused_llama_layer_intra_inter_full_fuse.py:218-235 + triton_fuse_lora_silu_hadamard_forward_kernels.py):
  * gate_main = x * wg^T and up_main = x * wu^T stay in tensor memory; the epilogue rounds them to bf16,
