@@ -336,6 +336,8 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
 //     product has more column tiles than SMs can take at once either way and stays persistent: 28.8 / 30.3
 //   129 to 256 tokens, pair form, S = 2: 21.8 / 19.0, 43 / 30.6, 69 / 45; wider products fill the chip without it
 //   512 tokens: 45 / 47, 75 / 77: persistent
+// A CTA keeps at least 16 k-blocks: below that its share of the main loop is shorter than set-up and reduction (about
+// 3 us), and the sum over all of K stays in one accumulator.
 SplitPlan choose_split(int epi, const Params& p) {
   SplitPlan plan = {0, false};
 #ifdef HYC_TUNE
@@ -344,11 +346,12 @@ SplitPlan choose_split(int epi, const Params& p) {
   if (epi == EPI_GRADDOWN || p.M > 2 * BM) return plan;
   if (epi == EPI_STORE && p.l1.bt != nullptr) return plan;         // a second LoRA term: the persistent kernel's own epilogue
   const int tiles = p.N / (epi == EPI_GATEUP ? SBN / 2 : SBN), sms = num_sms();
+  const int kb = (p.K1 + p.K2 + p.K3) / BK;
   if (p.M <= BM) {
     plan.split = 1;
     for (int s = 2; s <= (epi == EPI_GATEUP ? 2 : 4); s *= 2)
-      if (tiles * s <= sms) plan.split = s;
-  } else if (epi == EPI_STORE && tiles * 4 <= sms) {
+      if (tiles * s <= sms && kb >= 16 * s) plan.split = s;
+  } else if (epi == EPI_STORE && tiles * 4 <= sms && kb >= 32) {
     plan = {2, true};
   }
   return plan;

@@ -1,0 +1,69 @@
+"""The forms of the GEMM kernels that depend on the shape: clusters that split K (few rows), pairs and half-width column
+tiles, and several weights in one launch, at the edges of their ranges.
+
+Tolerance: fp32 sums of K products carry at most K * 2^-24 * (|A| |B|) of rounding, and every rounding to bf16 adds
+2^-8 (half a unit of an 8-bit significand) of the value it rounds."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF16 = torch.bfloat16
+
+
+def _rn(g, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=g) * scale).to(BF16).to(DEV)
+
+
+@pytest.mark.parametrize("M", [1, 64, 65, 128, 129, 255, 256, 257, 640, 641])
+@pytest.mark.parametrize("N,K,K2", [(256, 4096, 0), (256, 1984, 64), (1024, 1024, 1024), (4352, 2048, 64)])
+@pytest.mark.parametrize("b_is_kn", [False, True])
+def test_gemm_splits_and_tiles(M, N, K, K2, b_is_kn):
+    from hyc_lora_release_b200 import mlp
+    g = torch.Generator().manual_seed(M + N + K)
+    a, a2 = _rn(g, M, K), (_rn(g, M, K2) if K2 else None)
+    shape = (lambda k: (k, N)) if b_is_kn else (lambda k: (N, k))
+    b, b2 = _rn(g, *shape(K), scale=0.05), (_rn(g, *shape(K2), scale=0.05) if K2 else None)
+    res = _rn(g, M, N)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    d = mlp.gemm(a, b, b_is_kn=b_is_kn, a2=a2, b2=b2, residual=res, status=st)
+    assert int(st.item()) == 0
+    op = (lambda t: t.double()) if b_is_kn else (lambda t: t.double().t())
+    main, mag = a.double() @ op(b), a.double().abs() @ op(b).abs()
+    if K2:
+        main, mag = main + a2.double() @ op(b2), mag + a2.double().abs() @ op(b2).abs()
+    want = main + res.double()
+    bound = (K + K2) * 2.0 ** -24 * mag + 2.0 ** -8 * (main.abs() + want.abs()) * 1.01
+    assert bool(((d.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("T", [1, 100, 128, 200, 300])
+@pytest.mark.parametrize("ns", [(512, 256, 256), (256, 256), (768,)])
+def test_projections_in_one_launch(T, ns):
+    """Outputs and codes of several weights at once against each weight on its own (another split of K may round a
+    main branch the other way: its code then moves by one step, counted)."""
+    from hyc_lora_release_b200 import mlp
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(T + len(ns))
+    K, q = 2048, 4
+    x = _rn(g, T, K)
+    ws, bs = [_rn(g, n, K, scale=0.03) for n in ns], [_rn(g, n, 16, scale=0.05) for n in ns]
+    xas = [_rn(g, T, 16) for _ in ns]
+    scs = [torch.full((n,), 0.2 + 0.1 * i, dtype=BF16, device=DEV) for i, n in enumerate(ns)]
+    ys = [torch.full((T, n), float("nan"), dtype=BF16, device=DEV) for n in ns]
+    qs = [torch.zeros((T, n * q // 8), dtype=torch.uint8, device=DEV) for n in ns]
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    arr = lambda ts: (ctypes.c_void_p * len(ns))(*[t.data_ptr() for t in ts])
+    check(lib.hyc_linears_lora_save_fwd_tcgen05(ptr(x), T, K, len(ns), arr(ws), (ctypes.c_int * len(ns))(*ns), arr(xas), arr(bs),
+                                                arr(scs), arr(qs), arr(ys), q, ptr(st), stream_of(x)), "linears")
+    for w, b, xa, sc, y, codes in zip(ws, bs, xas, scs, ys, qs):
+        y1, q1, _ = mlp.linear_lora_save(x, w, None, b, sc, q, xa=xa, status=st)
+        assert int(st.item()) == 0
+        main, mag = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+        lora = xa.double() @ b.double().t()
+        bound = K * 2.0 ** -24 * mag + 2.0 ** -8 * (main.abs() + lora.abs() + (main + lora).abs()) * 1.01 + 1e-6
+        assert bool(((y.double() - main - lora).abs() <= bound).all())
+        flips = ((codes ^ q1) != 0).double().mean()
+        assert float(flips) < 2e-3 and bool(((y.double() - y1.double()).abs() <= 2 * bound).all())
