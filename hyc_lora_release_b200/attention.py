@@ -173,19 +173,20 @@ def attention_forward(x, w: AttnWeights, state: AttnState, cos, sin, attention_m
     B, M, H = x.shape
     pad = w.padded()
     xs, xn_scale = sv['x'], sv['x_norm_1']['scale']
-    a, o2, rstd, x_o, x_q, xn_q, q_q, k_q, v_q, xa3 = host.attn_forward_map(
+    a, o2, rstd, x_o, x_q, xn_q, q_q, k_q, v_q, xa3, o_codes, *map_class = host.attn_forward_map(
         x, [w.norm_w, w.wq, w.wk, w.wv, w.bq, w.bk, w.bv, pad["aqkv_t"]],
-        [xs['outlier_channel_index'], xs['scale'], xn_scale, sv['q']['scale'], sv['k']['scale'], sv['v']['scale']],
+        [xs['outlier_channel_index'], xs['scale'], xn_scale, sv['q']['scale'], sv['k']['scale'], sv['v']['scale'],
+         sv['o']['scale']],
         cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, q, eps, st)
     a_saved = _save_map(a, state)
     a_shape = tuple(a.shape)
     del a
-    x_medium, o_q, o_xa64 = host.attn_forward_out(x, o2, w.wo, pad["ao_cols"], pad["bo_cols"], sv['o']['scale'], w.bias_o, q, st)
+    x_medium, o_q, o_xa64 = host.attn_forward_out(x, o2, w.wo, pad["ao_cols"], pad["bo_cols"], sv['o']['scale'], o_codes, w.bias_o, q, st)
     state.iteration += 1
     saved = dict(rstd=rstd, x_o=x_o, x_q=x_q, x_scale=xs['scale'], x_idx=xs['outlier_channel_index'], xn_q=xn_q, xn_scale=xn_scale,
                  q_q=q_q, q_scale=sv['q']['scale'], k_q=k_q, k_scale=sv['k']['scale'], v_q=v_q, v_scale=sv['v']['scale'],
                  q_xa=xa3[0], k_xa=xa3[1], v_xa=xa3[2], qkv_xa=xa3, a_saved=a_saved, a_shape=a_shape, map_mode=state.map_mode,
-                 o_q=o_q, o_scale=sv['o']['scale'], o_xa=o_xa64[:, :w.ao.shape[0]], q_bit=q, shape=(B, M, H),
+                 map_class=map_class, o_q=o_q, o_scale=sv['o']['scale'], o_xa=o_xa64[:, :w.ao.shape[0]], q_bit=q, shape=(B, M, H),
                  cos=cos, sin=sin, num_heads=num_heads, head_dim=head_dim, num_key_value_heads=num_key_value_heads)
     return x_medium, saved
 
@@ -298,7 +299,7 @@ def attention_backward(grad_medium, saved, w: AttnWeights, status=None, on_lora_
             cf.decompression_softmax(m).reshape(saved['a_shape'])
     grad_q, grad_k, grad_v, gqkv = host.attn_backward_map(
         grad_o2, a, topk, map_q, [saved[n] for n in ('q_q', 'q_scale', 'q_xa', 'k_q', 'k_scale', 'k_xa', 'v_q', 'v_scale', 'v_xa')],
-        [w.bq, w.bk, w.bv], saved['cos'], saved['sin'], B, M, nh, d, nkv, q)
+        [w.bq, w.bk, w.bv], saved['cos'], saved['sin'], B, M, nh, d, nkv, q, *saved.get('map_class', (None, 0, 0)), st)
     del a, grad_o2
 
     # ---- q/k/v projections: LoRA gradients, then grad_x_norm as one GEMM over the three K segments

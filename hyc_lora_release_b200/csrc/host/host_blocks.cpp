@@ -139,10 +139,24 @@ static Tensor matmul_to_hidden(const Tensor& a4, const Tensor& b4, const OptTens
   return out.view({B * M, n * d});
 }
 
-struct Geometry { int64_t heads, d, kv; };
+// additive mask as the attention kernels take it: bf16, [b or 1, h or 1, M, M], strides in multiples of 8 elements
+struct MaskView { Tensor t; int64_t b = 0, h = 0, row = 0; };
+static MaskView mask_view(const OptTensor& mask, int64_t B, int64_t nh, int64_t M) {
+  MaskView v;
+  if (!given(mask)) return v;
+  v.t = mask->to(at::kBFloat16);
+  TORCH_CHECK_VALUE(v.t.dim() == 4 && v.t.size(3) == M && v.t.size(2) == M && (v.t.size(0) == 1 || v.t.size(0) == B) &&
+                    (v.t.size(1) == 1 || v.t.size(1) == nh), "attention_mask must be [b or 1, h or 1, n, S]");
+  auto strides = [&]() { v.b = v.t.size(0) == 1 ? 0 : v.t.stride(0); v.h = v.t.size(1) == 1 ? 0 : v.t.stride(1); v.row = v.t.stride(2); };
+  strides();
+  if (v.t.stride(3) != 1 || ((v.b | v.h | v.row) & 7) || (reinterpret_cast<uintptr_t>(v.t.data_ptr()) & 15)) { v.t = v.t.contiguous(); strides(); }
+  return v;
+}
+static bool attn_kernels_take(int64_t M, int64_t d) { return d == 128 && M % 8 == 0 && M <= 4096; }
 
 // the q, k, v projections with their saves, rotary embedding, scores and probabilities
-static std::vector<Tensor> attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos,
+using MapForward = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor, OptTensor, int64_t, int64_t>;
+static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos,
                                             const Tensor& sin, const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps,
                                             const Tensor& status) {
   const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
@@ -159,21 +173,39 @@ static std::vector<Tensor> attn_forward_map(const Tensor& x, const std::vector<T
   const auto &[vy, v_q] = p3[2];
   rope(qy.view({B, M, nh, d}), cos, sin, false, true);
   rope(ky.view({B, M, nkv, d}), cos, sin, false, true);
+  if (attn_kernels_take(M, d)) {
+    // one kernel from q, k, v to the probabilities, o and the codes of o
+    const MaskView mv = mask_view(mask, B, nh, M);
+    Tensor cls, a = empty({B, nh, M, M}, x_norm), o2 = empty({T, nh * d}, x_norm), o_q = empty({T, nh * d * q / 8}, x_norm, at::kByte);
+    const Tensor os = vec(stats[6]);
+    int64_t cls_b = 0, cls_h = 0;
+    if (mv.t.defined()) {
+      const int64_t nb = mv.t.size(0), nhm = mv.t.size(1);
+      cls = empty({(int64_t)hyc_attn_mask_class_bytes((int)nb, (int)nhm, (int)M)}, x_norm, at::kByte);
+      check(hyc_attn_mask_class(data(mv.t), mv.b, mv.h, mv.row, (int)nb, (int)nhm, (int)M, data(cls), on.stream), "hyc_attn_mask_class");
+      cls_b = nb == 1 ? 0 : nhm;
+      cls_h = nhm == 1 ? 0 : 1;
+    }
+    check(hyc_attn_fwd_tcgen05(data(qy), data(ky), data(vy), (int)B, (int)M, (int)nh, (int)nkv, (int)d, (float)(1.0 / std::sqrt((double)d)),
+                               data(mv.t), mv.b, mv.h, mv.row, data(cls), cls_b, cls_h, data(a), data(o2), data(os), data(o_q), (int)q,
+                               status_ptr(status), on.stream), "hyc_attn_fwd_tcgen05");
+    return {a, o2, rstd, x_o, x_q, *xn_q, q_q, k_q, v_q, xa3, o_q, cls, cls_b, cls_h};
+  }
   const Tensor kh = repeat_kv(heads(ky, B, M, nkv), rep), vh = repeat_kv(heads(vy, B, M, nkv), rep);
   Tensor scores = at::matmul(heads(qy, B, M, nh), kh.transpose(-2, -1));
   const Tensor a = softmax_forward(scores, 1.0 / std::sqrt((double)d), mask, true);
   const Tensor o2 = matmul_to_hidden(a, vh, std::nullopt);
-  return {a, o2, rstd, x_o, x_q, *xn_q, q_q, k_q, v_q, xa3};
+  return {a, o2, rstd, x_o, x_q, *xn_q, q_q, k_q, v_q, xa3, std::nullopt, std::nullopt, 0, 0};
 }
 
 // o projection with residual and the save of its input
 static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols,
-                                            const Tensor& o_scale, const OptTensor& bias_o, int64_t q, const Tensor& status) {
+                                            const Tensor& o_scale, const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& status) {
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
   const Tensor o_xa64 = at::mm(o2, ao_cols);
   Tensor x_medium = gemm(o2, wo, false, o_xa64, bo_cols, std::nullopt, std::nullopt, bf16c(x).view({T, H}), status);
   if (given(bias_o)) x_medium.add_(bias_o->to(at::kBFloat16));
-  const Tensor o_q = std::get<0>(quant(o2.view({B, M, -1}), o_scale, q, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
+  const Tensor o_q = given(o_codes) ? *o_codes : std::get<0>(quant(o2.view({B, M, -1}), o_scale, q, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
   return {x_medium.view({B, M, H}), o_q.view({T, -1}), o_xa64};
 }
 
@@ -197,16 +229,31 @@ static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, 
 // rotation, and the buffer that holds all three when the head counts agree
 static std::vector<OptTensor> attn_backward_map(const Tensor& grad_o2, Tensor a, const std::vector<Tensor>& topk, int64_t map_q_bit,
                                                 const std::vector<Tensor>& saved, const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin,
-                                                int64_t B, int64_t M, int64_t nh, int64_t d, int64_t nkv, int64_t q) {
+                                                int64_t B, int64_t M, int64_t nh, int64_t d, int64_t nkv, int64_t q,
+                                                const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status) {
   const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
                &v_s = saved[7], &v_xa = saved[8];
   OnDevice on(grad_o2);
   const int64_t T = B * M, rep = nh / nkv;
   const double scale = 1.0 / std::sqrt((double)d);
-  const Tensor grad_oh = heads(grad_o2, B, M, nh);
-  Tensor v2 = rebuild(v_q, v_s, v_xa, w[2], q);
   OptTensor gqkv;
   if (rep == 1) gqkv = empty({3, T, nh * d}, grad_o2);
+  if (attn_kernels_take(M, d)) {
+    const Tensor q2 = rebuild(q_q, q_s, q_xa, w[0], q), k2 = rebuild(k_q, k_s, k_xa, w[1], q), v2 = rebuild(v_q, v_s, v_xa, w[2], q);
+    rope(q2.view({B, M, nh, d}), cos, sin, false, true);
+    rope(k2.view({B, M, nkv, d}), cos, sin, false, true);
+    Tensor gs = empty({B, nh, M, M}, grad_o2);
+    Tensor gq = rep == 1 ? (*gqkv)[0] : empty({T, nh * d}, grad_o2), gk = rep == 1 ? (*gqkv)[1] : empty({T, nkv * d}, grad_o2),
+           gv = rep == 1 ? (*gqkv)[2] : empty({T, nkv * d}, grad_o2);
+    check(hyc_attn_bwd_tcgen05(data(q2), data(k2), data(v2), data(grad_o2), data(a), data(gs), (int)B, (int)M, (int)nh, (int)nkv, (int)d,
+                               (float)scale, data(cls), cls_b, cls_h, data(gq), data(gk), data(gv), status_ptr(status), on.stream),
+          "hyc_attn_bwd_tcgen05");
+    rope(gq.view({B, M, nh, d}), cos, sin, true, true);
+    rope(gk.view({B, M, nkv, d}), cos, sin, true, true);
+    return {gq, gk, gv, gqkv};
+  }
+  const Tensor grad_oh = heads(grad_o2, B, M, nh);
+  Tensor v2 = rebuild(v_q, v_s, v_xa, w[2], q);
   auto slot = [&](int i) -> OptTensor { return gqkv.has_value() ? OptTensor((*gqkv)[i]) : OptTensor(); };
   Tensor grad_v = rep == 1 ? matmul_to_hidden(a.transpose(-2, -1), grad_oh, slot(2))
                            : hidden(repeat_kv_backward(at::matmul(a.transpose(-2, -1), grad_oh), rep));

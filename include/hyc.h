@@ -347,6 +347,30 @@ int hyc_mlp_graddown_bwd_tcgen05(const void* g, const void* wd, int T, int H, in
                                  const void* lora_gate, const void* lora_up, int64_t ld_lora,
                                  void* o, void* grad_gate, void* grad_up, int q_bit, int* status, void* stream);
 
+/* ---- attention of the fused layer (heads of 128 columns, M % 8 == 0, M <= 4096) ----------------
+ *
+ * softmax(q k^T * scale + mask) v with the rounding points of the layer's separate steps
+ * (fused_llama_layer_intra_inter_full_fuse.py:150-170), q [B,M,heads*128], k / v [B,M,kv_heads*128] bf16.
+ * hyc_attn_mask_class sorts the 128 x 128 tiles of an additive mask (element strides, multiples of 8) into all-zero,
+ * mixed and ruled out; both directions skip the tiles of the last kind.  cls_b / cls_h: stride of a batch entry / head
+ * in the class array, in units of tiles^2 entries (0 where the mask is shared).
+ * forward: o [B,M,heads*128]; map (optional) [B,heads,M,M] the probabilities; o_codes (optional) the per-channel codes
+ *   of o under o_scale [heads*128].
+ * backward: map = the restored probabilities (zero in every tile that cls rules out), grad_s = scratch of its size;
+ *   grad_s = ((grad_a - rowsum(map * grad_a)) * map) * scale, grad_q, grad_k, grad_v.  HYC_ERR_UNSUPPORTED: another
+ *   head size or a longer sequence; nothing was launched. */
+size_t hyc_attn_mask_class_bytes(int mask_batch, int mask_heads, int M);
+int hyc_attn_mask_class(const void* mask, int64_t stride_b, int64_t stride_h, int64_t stride_row, int mask_batch, int mask_heads,
+                        int M, void* out, void* stream);
+int hyc_attn_fwd_tcgen05(const void* q, const void* k, const void* v, int B, int M, int heads, int kv_heads, int head_dim, float scale,
+                         const void* mask_or_null, int64_t mask_b, int64_t mask_h, int64_t mask_row,
+                         const void* cls_or_null, int64_t cls_b, int64_t cls_h, void* map_or_null, void* o,
+                         const void* o_scale_or_null, void* o_codes_or_null, int q_bit, int* status, void* stream);
+int hyc_attn_bwd_tcgen05(const void* q, const void* k, const void* v, const void* grad_o, const void* map, void* grad_s,
+                         int B, int M, int heads, int kv_heads, int head_dim, float scale,
+                         const void* cls_or_null, int64_t cls_b, int64_t cls_h, void* grad_q, void* grad_k, void* grad_v,
+                         int* status, void* stream);
+
 /* LoRA-A gradient with the de-quantizer inside the contraction:
  *   out[r, h] = sum_t gm[t, r] * x_hat[t, h],   x_hat = decompression_dequantization(q, scale)
  * Replaces `decompression_dequantization` followed by `x.mT @ grad_medium` of lora_backward
