@@ -69,6 +69,9 @@ SIGNATURES = {
     "hyc_mlp_gateup_fwd_tcgen05": (_i, [_p, _p, _p, _i, _i, _i, _p, _p, _l, _l, _p, _p, _l, _l,
                                         _p, _p, _p, _p, _p, _p, _p, _i, _p, _p]),
     "hyc_linear_lora_save_fwd_tcgen05": (_i, [_p, _p, _i, _i, _i, _p, _p, _l, _l, _p, _p, _p, _p, _i, _p, _p]),
+    "hyc_gemm_segments_tcgen05": (_i, [_i, _p, _p, _p, _i, _i, _i, _p, _p, _p, _p]),
+    "hyc_skinny_workspace_bytes": (_z, [_i, _p, _i]),
+    "hyc_skinny_products": (_i, [_i, _p, _i, _p, _z, _p, _p]),
     "hyc_attn_mask_class_bytes": (_z, [_i, _i, _i]),
     "hyc_attn_mask_class": (_i, [_p, _l, _l, _l, _i, _i, _i, _p, _p]),
     "hyc_attn_fwd_tcgen05": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _f, _p, _l, _l, _l, _p, _l, _l, _p, _p, _p, _p, _i, _p, _p]),

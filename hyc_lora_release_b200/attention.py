@@ -26,7 +26,7 @@ from typing import Optional
 import torch
 
 from ._lib import host, require_cuda
-from .mlp import _status_tensor, gemm, linear_lora_save, lora_a_products, padded_block
+from .mlp import _status_tensor, gemm, linear_lora_save, lora_a_products
 from .operators import compress_function as cf
 from .operators.rmsnorm_kernels import rmsnorm_forward, rmsnorm_forward_save
 from .operators.rope_kernels import rope_inplace
@@ -66,9 +66,8 @@ class AttnWeights:
           bo_cols  [H, 64]        columns 0..15 = Bo     ([N, K] operand of the o projection's LoRA block)
           ao_rows  [64, heads*d]  rows 0..15 = Ao        ([K, N] operand of grad_o's LoRA block)
           aqkv_rows [64, H]       rows 0..15 = Aq, 16..31 = Ak, 32..47 = Av ([K, N] operand of grad_x's LoRA block)
-        and the stacked factors of the batched rank-16 products:
-          aqkv_t   [3, H, r]        Aq^T, Ak^T, Av^T (x_norm @ all three in one call)
-          bqkv     [3, heads*d, r]  Bq, Bk, Bv (None with grouped key/value heads, whose shapes differ)"""
+        and the transposed factors of the rank-16 products:
+          aqkv_t   [3, H, r]        Aq^T, Ak^T, Av^T (x_norm @ all three in one call)"""
         ts = (self.aq, self.ak, self.av, self.ao, self.bo, self.bq, self.bk, self.bv)
         key = tuple((t.data_ptr(), t._version) for t in ts)
         if getattr(self, "_pad_key", None) != key:
@@ -80,10 +79,8 @@ class AttnWeights:
             aqkv = torch.zeros(64, self.aq.shape[1], dtype=dt, device=dev)
             aqkv[:r] = self.aq; aqkv[r:2 * r] = self.ak; aqkv[2 * r:3 * r] = self.av
             aqkv_t = torch.stack((self.aq.t(), self.ak.t(), self.av.t())).contiguous()      # [3, H, r]
-            same = self.bq.shape == self.bk.shape == self.bv.shape
-            bqkv = torch.stack((self.bq, self.bk, self.bv)).contiguous() if same else None   # [3, heads*d, r]
             self._pad = dict(ao_rows=ao_rows, ao_cols=ao_rows.t().contiguous(), bo_cols=bo_cols, aqkv_rows=aqkv,
-                             aqkv_t=aqkv_t, bqkv=bqkv)
+                             aqkv_t=aqkv_t)
             self._pad_key = key
         return self._pad
 
@@ -287,7 +284,7 @@ def attention_backward(grad_medium, saved, w: AttnWeights, status=None, on_lora_
     pad = w.padded()
 
     # ---- o projection (the LoRA-A gradient de-quantizes o inside its kernel)
-    grad_bo, grad_ao, grad_o2 = host.attn_backward_out(g, w.wo, pad["bo_cols"], pad["ao_rows"], saved['o_xa'], saved['o_q'],
+    grad_bo, grad_ao, grad_o2 = host.attn_backward_out(g, w.wo, w.bo, pad["ao_rows"], saved['o_xa'], saved['o_q'],
                                                        saved['o_scale'], q, st)
     # ---- the map: P.V backward, softmax backward (for the top-k form fused with a second restore: the map is not
     # re-read), scores backward with q, k rebuilt from their codes
@@ -297,18 +294,18 @@ def attention_backward(grad_medium, saved, w: AttnWeights, status=None, on_lora_
     else:
         a = m.to_dense().reshape(saved['a_shape']) if isinstance(m, (cf.PrunedMap, cf.TiledPrunedMap)) else \
             cf.decompression_softmax(m).reshape(saved['a_shape'])
-    grad_q, grad_k, grad_v, gqkv = host.attn_backward_map(
+    grad_q, grad_k, grad_v = host.attn_backward_map(
         grad_o2, a, topk, map_q, [saved[n] for n in ('q_q', 'q_scale', 'q_xa', 'k_q', 'k_scale', 'k_xa', 'v_q', 'v_scale', 'v_xa')],
         [w.bq, w.bk, w.bv], saved['cos'], saved['sin'], B, M, nh, d, nkv, q, *saved.get('map_class', (None, 0, 0)), st)
     del a, grad_o2
 
-    # ---- q/k/v projections: LoRA gradients, then grad_x_norm as one GEMM over the three K segments
-    gmq = padded_block(w, "_gmq", T, dev)                    # g_q @ Bq | g_k @ Bk | g_v @ Bv side by side
+    # ---- q/k/v projections: LoRA gradients, then grad_x_norm as one GEMM over four K segments
     qkv_xa = saved.get('qkv_xa')
     if qkv_xa is None:
         qkv_xa = torch.stack((saved['q_xa'], saved['k_xa'], saved['v_xa']))
-    ga, grad_bq, grad_bk, grad_bv = host.attn_backward_lora([grad_q, grad_k, grad_v], gqkv, gmq, pad["bqkv"], [w.bq, w.bk, w.bv],
-                                                            qkv_xa, saved['xn_q'], saved['xn_scale'], q)
+    # gmq: g_q @ Bq | g_k @ Bk | g_v @ Bv side by side
+    gmq, ga, grad_bq, grad_bk, grad_bv = host.attn_backward_lora([grad_q, grad_k, grad_v], [w.bq, w.bk, w.bv], qkv_xa,
+                                                                 saved['xn_q'], saved['xn_scale'], q, st)
     grads = dict(grad_aq=ga[:16], grad_bq=grad_bq, grad_ak=ga[16:32], grad_bk=grad_bk, grad_av=ga[32:48], grad_bv=grad_bv,
                  grad_ao=grad_ao, grad_bo=grad_bo)
     if on_lora_grads is not None:

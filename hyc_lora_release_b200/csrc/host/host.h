@@ -73,9 +73,6 @@ Tensor dequant_nf4(const Tensor& packed, const Tensor& code, const Tensor& absma
                    int64_t blocksize2, double offset, int64_t blocksize, at::IntArrayRef shape);
 
 // ---- GEMMs and the two halves of the layer (host_blocks.cpp)
-struct Lora { const Tensor* xa = nullptr; const Tensor* bt = nullptr; };
-Tensor gemm(const Tensor& a, const Tensor& b, bool b_is_kn, const OptTensor& a2, const OptTensor& b2, const OptTensor& a3,
-            const OptTensor& b3, const OptTensor& residual, const Tensor& status);
 Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64_t r2, int64_t q_bit);
 void bind_ops(pybind11::module_& m);
 void bind_blocks(pybind11::module_& m);

@@ -9,21 +9,59 @@ namespace hyc_host {
 
 static int* status_ptr(const Tensor& st) { return (int*)st.data_ptr(); }
 
-Tensor gemm(const Tensor& a, const Tensor& b, bool b_is_kn, const OptTensor& a2, const OptTensor& b2, const OptTensor& a3,
-            const OptTensor& b3, const OptTensor& residual, const Tensor& status) {
+// sum of a_i op(b_i) (+ residual), one to four K segments
+struct Segment { const Tensor *a, *b; };
+static Tensor gemm(std::initializer_list<Segment> segs, bool b_is_kn, const Tensor* residual, const Tensor& status) {
+  const Tensor& a = *segs.begin()->a;
   OnDevice on(a);
-  const int64_t M = a.size(0), K = a.size(1), N = b_is_kn ? b.size(1) : b.size(0);
+  const int64_t M = a.size(0), N = segs.begin()->b->size(b_is_kn ? 1 : 0);
+  const void *pa[4], *pb[4];
+  int k[4], n = 0;
+  for (const Segment& s : segs) { pa[n] = data(*s.a); pb[n] = data(*s.b); k[n++] = (int)s.a->size(1); }
   Tensor d = empty({M, N}, a);
-  check(hyc_gemm_bf16_tcgen05(data(a), data(b), (int)M, (int)N, (int)K, b_is_kn ? 1 : 0, data(a2), data(b2), given(a2) ? (int)a2->size(1) : 0,
-                              data(a3), data(b3), given(a3) ? (int)a3->size(1) : 0, nullptr, nullptr, 0, 0, nullptr, nullptr, 0, 0,
-                              data(residual), data(d), status_ptr(status), on.stream), "hyc_gemm_bf16_tcgen05");
+  check(hyc_gemm_segments_tcgen05(n, pa, pb, k, (int)M, (int)N, b_is_kn ? 1 : 0, residual ? data(*residual) : nullptr, data(d),
+                                  status_ptr(status), on.stream), "hyc_gemm_segments_tcgen05");
   return d;
 }
 
-// several rank-16 products x A_i^T with a shared left operand (stride 0) as one batched library call
+// The forward LoRA-A products stay library calls, batched where they share the left operand (stride 0): saved codes
+// behind them depend on every bit of their results, and with 2-bit codes one that flips moves a value by a third of its
+// range.  The backward products go through the kernel below.
 static Tensor lora_a_products(const Tensor& x2, const Tensor& stacked) {
   return at::bmm(x2.unsqueeze(0).expand({stacked.size(0), -1, -1}), stacked);
 }
+
+// rank-16 products (one launch for up to three operands)
+struct Skinny {
+  hyc_skinny_job jobs[3] = {};
+  int count = 0;
+  // x [T, n]
+  Skinny& on(const Tensor& x) {
+    hyc_skinny_job& j = jobs[count++];
+    j.x = data(x); j.ldx = x.stride(0); j.n = (int)x.size(1);
+    return *this;
+  }
+  // y (columns [col, col + 16) of a row of ld elements) = x w, then `pad` zero columns
+  Skinny& rows(const void* w, int64_t ld_w, const Tensor& y, int64_t offset, int64_t ld_y, int pad = 0) {
+    hyc_skinny_job& j = jobs[count - 1];
+    j.w[j.n_w] = w; j.ld_w = ld_w;
+    j.y[j.n_w++] = (char*)y.data_ptr() + offset * 2;
+    j.ld_y = ld_y; j.y_pad = pad;
+    return *this;
+  }
+  // z = x^T xa
+  Skinny& cols(const void* xa, int64_t ld_xa, void* z, bool transposed = false) {
+    hyc_skinny_job& j = jobs[count - 1];
+    j.xa = xa; j.ld_xa = ld_xa; j.z = z; j.z_transposed = transposed ? 1 : 0;
+    return *this;
+  }
+  void run(int64_t T, const Tensor& like, const Tensor& status, void* stream) {
+    const size_t bytes = hyc_skinny_workspace_bytes(count, jobs, (int)T);
+    Tensor ws = empty({(int64_t)(bytes / 4)}, like, at::kFloat);
+    check(hyc_skinny_products(count, jobs, (int)T, data(ws), bytes, status_ptr(status), stream), "hyc_skinny_products");
+  }
+};
+static const char* at_row(const Tensor& t, int64_t i) { return (const char*)t.data_ptr() + i * t.stride(0) * t.element_size(); }
 
 // the q, k and v projections with the saves of their main branches in one launch: -> {y, codes} of each
 static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, const std::array<const Tensor*, 3>& w, const Tensor& xa3,
@@ -81,38 +119,44 @@ static std::vector<Tensor> mlp_forward(const Tensor& x_medium, const std::vector
                                    data(gs), data(us), data(q1), data(q2), data(had), nullptr, nullptr, (int)q, status_ptr(status), on.stream),
         "hyc_mlp_gateup_fwd_tcgen05");
   const Tensor down_xa64 = at::mm(had, ad_cols);
-  Tensor x_out = gemm(had, wd, false, down_xa64, bd_cols, std::nullopt, std::nullopt, bf16c(x_medium).view({T, H}), status);
+  const Tensor res = bf16c(x_medium);
+  Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, false, &res, status);
   if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
   return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
 }
 
 // up to and including the six LoRA gradients: -> had, ggu, gm64, grad_bd, grad_ad, ga, grad_bgu
-static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, const Tensor& gm64,
-                                             int64_t q, const Tensor& status) {
-  const Tensor &wd = w[0], &bg = w[1], &bu = w[2], &bd_cols = w[3], &ad_rows = w[4], &bgu = w[5];
+static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q,
+                                             const Tensor& status) {
+  const Tensor &wd = w[0], &ad_rows = w[4];
+  const Tensor bg = w[1].contiguous(), bu = w[2].contiguous(), bd = w[3].contiguous();
   const Tensor &gate_q = saved[0], &gate_s = saved[1], &up_q = saved[2], &up_s = saved[3], &gu_xa = saved[4], &down_xa = saved[5],
                &xn_q = saved[6], &xn_scale = saved[7];
   OnDevice on(g);
   const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
-  Tensor grad_bd = at::mm(g.t(), down_xa);
-  const Tensor gdm64 = at::mm(g, bd_cols);
+  Tensor grad_bd = empty({H, 16}, g), gdm64 = empty({T, 64}, g), gm64 = empty({T, 64}, g), grad_ad = empty({16, I}, g),
+         grad_bgu = empty({2, I, 16}, g);
+  Skinny().on(g).rows(data(bd), 16, gdm64, 0, 64, 48).cols(data(down_xa), down_xa.stride(0), data(grad_bd)).run(T, g, status, on.stream);
   Tensor had = empty({T, I}, g), ggu = empty({2, T, I}, g);
   char* gp = (char*)ggu.data_ptr();
   const char* xa = (const char*)gu_xa.data_ptr();
   check(hyc_mlp_graddown_bwd_tcgen05(data(g), data(wd), (int)T, (int)H, (int)I, data(gdm64), data(ad_rows), 64, xa, data(bg), 16, 1,
                                      xa + T * 16 * 2, data(bu), 16, 1, data(gate_q), data(gate_s), data(up_q), data(up_s), nullptr, nullptr, 0,
                                      data(had), gp, gp + T * I * 2, (int)q, status_ptr(status), on.stream), "hyc_mlp_graddown_bwd_tcgen05");
-  Tensor grad_ad = at::mm(gdm64.narrow(1, 0, 16).t(), had);
-  gm64.view({T, 4, 16}).narrow(1, 0, 2).copy_(at::bmm(ggu, bgu).transpose(0, 1));
+  // g_gate Bg | g_up Bu side by side, the two B gradients and grad_ad, each operand read once
+  const Tensor g0 = ggu[0], g1 = ggu[1];
+  Skinny().on(g0).rows(data(bg), 16, gm64, 0, 64).cols(xa, 16, data(grad_bgu))
+          .on(g1).rows(data(bu), 16, gm64, 16, 64, 32).cols(xa + T * 32, 16, (char*)data(grad_bgu) + I * 32)
+          .on(had).cols(data(gdm64), 64, data(grad_ad), true).run(T, g, status, on.stream);
   Tensor ga = lora_grad_a(xn_q.view({T, -1}), vec(xn_scale), gm64, 32, q);
-  Tensor grad_bgu = at::bmm(ggu.transpose(1, 2), gu_xa);
-  return {had, ggu, grad_bd, grad_ad, ga, grad_bgu};
+  return {had, ggu, gm64, grad_bd, grad_ad, ga, grad_bgu};
 }
 
 static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
                              at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wg = w[0], &wu = w[1], &agu_rows = w[2], &norm_w = w[3];
-  Tensor grad_xn = gemm(ggu[0], wg, true, ggu[1], wu, gm64, agu_rows, std::nullopt, status);
+  const Tensor g0 = ggu[0], g1 = ggu[1];
+  Tensor grad_xn = gemm({{&g0, &wg}, {&g1, &wu}, {&gm64, &agu_rows}}, true, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 
@@ -129,9 +173,9 @@ static Tensor repeat_kv_backward(const Tensor& g, int64_t n) {
   return g.reshape({g.size(0), g.size(1) / n, n, g.size(2), g.size(3)}).sum(2);
 }
 // [B, n, M, K] @ [B, n, K, d] written straight into the hidden layout
-static Tensor matmul_to_hidden(const Tensor& a4, const Tensor& b4, const OptTensor& out_in) {
+static Tensor matmul_to_hidden(const Tensor& a4, const Tensor& b4) {
   const int64_t B = a4.size(0), n = a4.size(1), M = a4.size(2), d = b4.size(3);
-  Tensor out = given(out_in) ? out_in->view({B, M, n, d}) : empty({B, M, n, d}, a4);
+  Tensor out = empty({B, M, n, d}, a4);
   for (int64_t b = 0; b < B; ++b) {
     Tensor o = out[b].transpose(0, 1);
     at::bmm_out(o, a4[b], b4[b]);
@@ -194,7 +238,7 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
   const Tensor kh = repeat_kv(heads(ky, B, M, nkv), rep), vh = repeat_kv(heads(vy, B, M, nkv), rep);
   Tensor scores = at::matmul(heads(qy, B, M, nh), kh.transpose(-2, -1));
   const Tensor a = softmax_forward(scores, 1.0 / std::sqrt((double)d), mask, true);
-  const Tensor o2 = matmul_to_hidden(a, vh, std::nullopt);
+  const Tensor o2 = matmul_to_hidden(a, vh);
   return {a, o2, rstd, x_o, x_q, *xn_q, q_q, k_q, v_q, xa3, std::nullopt, std::nullopt, 0, 0};
 }
 
@@ -203,7 +247,8 @@ static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, c
                                             const Tensor& o_scale, const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& status) {
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
   const Tensor o_xa64 = at::mm(o2, ao_cols);
-  Tensor x_medium = gemm(o2, wo, false, o_xa64, bo_cols, std::nullopt, std::nullopt, bf16c(x).view({T, H}), status);
+  const Tensor res = bf16c(x);
+  Tensor x_medium = gemm({{&o2, &wo}, {&o_xa64, &bo_cols}}, false, &res, status);
   if (given(bias_o)) x_medium.add_(bias_o->to(at::kBFloat16));
   const Tensor o_q = given(o_codes) ? *o_codes : std::get<0>(quant(o2.view({B, M, -1}), o_scale, q, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
   return {x_medium.view({B, M, H}), o_q.view({T, -1}), o_xa64};
@@ -214,20 +259,23 @@ static Tensor rebuild(const Tensor& codes, const Tensor& scale, const Tensor& xa
   return dequant_lora_add(codes.view({1, T, -1}), scale, xa.view({1, T, -1}), b.t(), q).view({T, -1});
 }
 
-// o projection backward: -> gm64, grad_bo, grad_ao, grad_o2
-static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, const Tensor& bo_cols, const Tensor& ao_rows, const Tensor& o_xa,
+// o projection backward: -> grad_bo, grad_ao, grad_o2
+static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, const Tensor& bo_in, const Tensor& ao_rows, const Tensor& o_xa,
                                              const Tensor& o_q, const Tensor& o_scale, int64_t q, const Tensor& status) {
-  const Tensor gm64 = at::mm(g, bo_cols);
-  Tensor grad_bo = at::mm(g.t(), o_xa);
+  OnDevice on(g);
+  const int64_t T = g.size(0);
+  const Tensor bo = bo_in.contiguous();
+  Tensor gm64 = empty({T, 64}, g), grad_bo = empty({g.size(1), 16}, g);
+  Skinny().on(g).rows(data(bo), 16, gm64, 0, 64, 48).cols(data(o_xa), o_xa.stride(0), data(grad_bo)).run(T, g, status, on.stream);
   Tensor grad_ao = lora_grad_a(o_q, vec(o_scale), gm64, 16, q);
-  Tensor grad_o2 = gemm(g, wo, true, gm64, ao_rows, std::nullopt, std::nullopt, std::nullopt, status);
+  Tensor grad_o2 = gemm({{&g, &wo}, {&gm64, &ao_rows}}, true, nullptr, status);
   return {grad_bo, grad_ao, grad_o2};
 }
 
 // the map's backward.  `a`: the restored map; `topk`: the five tensors of the top-k form (the softmax backward then
 // restores once more on chip), empty for the pruned form.  -> grad_q, grad_k, grad_v [T, n*d] after the inverse
-// rotation, and the buffer that holds all three when the head counts agree
-static std::vector<OptTensor> attn_backward_map(const Tensor& grad_o2, Tensor a, const std::vector<Tensor>& topk, int64_t map_q_bit,
+// rotation
+static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, const std::vector<Tensor>& topk, int64_t map_q_bit,
                                                 const std::vector<Tensor>& saved, const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin,
                                                 int64_t B, int64_t M, int64_t nh, int64_t d, int64_t nkv, int64_t q,
                                                 const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status) {
@@ -236,26 +284,22 @@ static std::vector<OptTensor> attn_backward_map(const Tensor& grad_o2, Tensor a,
   OnDevice on(grad_o2);
   const int64_t T = B * M, rep = nh / nkv;
   const double scale = 1.0 / std::sqrt((double)d);
-  OptTensor gqkv;
-  if (rep == 1) gqkv = empty({3, T, nh * d}, grad_o2);
   if (attn_kernels_take(M, d)) {
     const Tensor q2 = rebuild(q_q, q_s, q_xa, w[0], q), k2 = rebuild(k_q, k_s, k_xa, w[1], q), v2 = rebuild(v_q, v_s, v_xa, w[2], q);
     rope(q2.view({B, M, nh, d}), cos, sin, false, true);
     rope(k2.view({B, M, nkv, d}), cos, sin, false, true);
     Tensor gs = empty({B, nh, M, M}, grad_o2);
-    Tensor gq = rep == 1 ? (*gqkv)[0] : empty({T, nh * d}, grad_o2), gk = rep == 1 ? (*gqkv)[1] : empty({T, nkv * d}, grad_o2),
-           gv = rep == 1 ? (*gqkv)[2] : empty({T, nkv * d}, grad_o2);
+    Tensor gq = empty({T, nh * d}, grad_o2), gk = empty({T, nkv * d}, grad_o2), gv = empty({T, nkv * d}, grad_o2);
     check(hyc_attn_bwd_tcgen05(data(q2), data(k2), data(v2), data(grad_o2), data(a), data(gs), (int)B, (int)M, (int)nh, (int)nkv, (int)d,
                                (float)scale, data(cls), cls_b, cls_h, data(gq), data(gk), data(gv), status_ptr(status), on.stream),
           "hyc_attn_bwd_tcgen05");
     rope(gq.view({B, M, nh, d}), cos, sin, true, true);
     rope(gk.view({B, M, nkv, d}), cos, sin, true, true);
-    return {gq, gk, gv, gqkv};
+    return {gq, gk, gv};
   }
   const Tensor grad_oh = heads(grad_o2, B, M, nh);
   Tensor v2 = rebuild(v_q, v_s, v_xa, w[2], q);
-  auto slot = [&](int i) -> OptTensor { return gqkv.has_value() ? OptTensor((*gqkv)[i]) : OptTensor(); };
-  Tensor grad_v = rep == 1 ? matmul_to_hidden(a.transpose(-2, -1), grad_oh, slot(2))
+  Tensor grad_v = rep == 1 ? matmul_to_hidden(a.transpose(-2, -1), grad_oh)
                            : hidden(repeat_kv_backward(at::matmul(a.transpose(-2, -1), grad_oh), rep));
   Tensor grad_a = at::matmul(grad_oh, repeat_kv(heads(v2, B, M, nkv), rep).transpose(-2, -1));
   v2.reset();
@@ -271,44 +315,38 @@ static std::vector<OptTensor> attn_backward_map(const Tensor& grad_o2, Tensor a,
   grad_a.reset();
   Tensor q2 = rebuild(q_q, q_s, q_xa, w[0], q);
   rope(q2.view({B, M, nh, d}), cos, sin, false, true);
-  Tensor grad_k = rep == 1 ? matmul_to_hidden(grad_s.transpose(-2, -1), heads(q2, B, M, nh), slot(1))
+  Tensor grad_k = rep == 1 ? matmul_to_hidden(grad_s.transpose(-2, -1), heads(q2, B, M, nh))
                            : hidden(repeat_kv_backward(at::matmul(grad_s.transpose(-2, -1), heads(q2, B, M, nh)), rep));
   q2.reset();
   Tensor k2 = rebuild(k_q, k_s, k_xa, w[1], q);
   rope(k2.view({B, M, nkv, d}), cos, sin, false, true);
-  Tensor grad_q = matmul_to_hidden(grad_s, repeat_kv(heads(k2, B, M, nkv), rep), slot(0));
+  Tensor grad_q = matmul_to_hidden(grad_s, repeat_kv(heads(k2, B, M, nkv), rep));
   rope(grad_q.view({B, M, nh, d}), cos, sin, true, true);
   rope(grad_k.view({B, M, nkv, d}), cos, sin, true, true);
-  return {grad_q, grad_k, grad_v, gqkv};
+  return {grad_q, grad_k, grad_v};
 }
 
-// LoRA gradients of q/k/v: -> ga [48, H], grad_bq, grad_bk, grad_bv (gmq is filled)
-static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, const OptTensor& gqkv, const Tensor& gmq, const OptTensor& bqkv,
-                                              const std::vector<Tensor>& b, const Tensor& qkv_xa, const Tensor& xn_q, const Tensor& xn_scale, int64_t q) {
-  OnDevice on(gmq);
-  const int64_t T = gmq.size(0), r = 16;
-  Tensor gb[3];
-  const bool batched = given(gqkv) && given(bqkv);
-  if (batched) {
-    gmq.view({T, 4, 16}).narrow(1, 0, 3).copy_(at::bmm(*gqkv, *bqkv).transpose(0, 1));
-    const Tensor g3 = at::bmm(gqkv->transpose(1, 2), qkv_xa);
-    for (int i = 0; i < 3; ++i) gb[i] = g3[i];
-  } else {
-    for (int i = 0; i < 3; ++i) {
-      Tensor o = gmq.narrow(1, i * r, r);
-      at::mm_out(o, grads[i], b[i]);
-      gb[i] = at::mm(grads[i].t(), qkv_xa[i]);
-    }
+// LoRA gradients of q/k/v: -> gmq [T, 64], ga [48, H], grad_bq, grad_bk, grad_bv
+static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, const std::vector<Tensor>& b_in, const Tensor& qkv_xa, const Tensor& xn_q,
+                                              const Tensor& xn_scale, int64_t q, const Tensor& status) {
+  OnDevice on(grads[0]);
+  const int64_t T = grads[0].size(0);
+  Tensor gmq = empty({T, 64}, grads[0]), gb[3], b[3];
+  Skinny s;
+  for (int i = 0; i < 3; ++i) {
+    gb[i] = empty({grads[i].size(1), 16}, grads[0]);
+    b[i] = b_in[i].contiguous();
+    s.on(grads[i]).rows(data(b[i]), 16, gmq, 16 * i, 64, i == 2 ? 16 : 0).cols(at_row(qkv_xa, i), 16, data(gb[i]));
   }
+  s.run(T, gmq, status, on.stream);
   Tensor ga = lora_grad_a(xn_q.view({T, -1}), vec(xn_scale), gmq, 48, q);
-  return {ga, gb[0], gb[1], gb[2]};
+  return {gmq, ga, gb[0], gb[1], gb[2]};
 }
 
 static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wq = w[0], &wk = w[1], &wv = w[2], &aqkv_rows = w[3], &norm_w = w[4];
-  const Tensor lora_x = at::mm(gmq, aqkv_rows);
-  Tensor grad_xn = gemm(grads[0], wq, true, grads[1], wk, grads[2], wv, lora_x, status);
+  Tensor grad_xn = gemm({{&grads[0], &wq}, {&grads[1], &wk}, {&grads[2], &wv}, {&gmq, &aqkv_rows}}, true, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 

@@ -36,6 +36,27 @@ inline int current_device_slot() {
   return dev;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_pdl may begin before the kernel in front of it in the
+// stream has ended, and has to call pdl_wait() before it touches memory (pdl_wait returns once that kernel, and with
+// it everything before, is complete and visible).  pdl_trigger() in the kernel in front lets the launch go out.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename K, typename... A>
+inline int launch_pdl(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, args...) != cudaSuccess) {
+    hyc_set_last_cuda_error((int)cudaGetLastError());
+    return HYC_ERR_LAUNCH;
+  }
+  return HYC_OK;
+}
+
 __host__ __device__ inline bool aligned(const void* p, size_t a) {
   return (reinterpret_cast<uintptr_t>(p) & (a - 1)) == 0;
 }

@@ -75,7 +75,7 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
   const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
   constexpr int TILE_N = (EPI == EPI_GATEUP) ? BN / 2 : BN;     // output columns per tile
   const int num_tiles = tiles_m * (p.n_wide + (p.N / TILE_N - p.n_wide) * 2);
-  const int kb1 = p.K1 / BK, kb2 = (p.K1 + p.K2) / BK, kb_total = (p.K1 + p.K2 + p.K3) / BK;
+  const int kb1 = p.K1 / BK, kb2 = (p.K1 + p.K2) / BK, kb3 = (p.K1 + p.K2 + p.K3) / BK, kb_total = kb3 + p.K4 / BK;
 
   if (warp == 0 && elect_one()) {
     for (int i = 0; i < 3; ++i) {
@@ -126,11 +126,11 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
             ok = false;
             break;
           }
-          const int seg = kb < kb1 ? 0 : (kb < kb2 ? 1 : 2);
+          const int seg = kb < kb1 ? 0 : (kb < kb2 ? 1 : (kb < kb3 ? 2 : 3));
           const int wsel = EPI == EPI_STORE && grp > 0 ? grp : seg;      // weights side by side along N, or K segments
           const CUtensorMap* ma = &maps.a[seg];
           const CUtensorMap* mb = wide ? &maps.b[wsel] : &maps.n[wsel];
-          const int k0 = (seg == 0 ? kb : (seg == 1 ? kb - kb1 : kb - kb2)) * BK;
+          const int k0 = (kb - (seg == 0 ? 0 : (seg == 1 ? kb1 : (seg == 2 ? kb2 : kb3)))) * BK;
           const uint32_t sa = smem_u32(stage_base + stage * stage_bytes);
           const uint32_t sb = sa + STAGE_A_BYTES;
           // pair form: the leader's barrier counts both CTAs' bytes
@@ -425,7 +425,7 @@ static int launch_as(const Operands& ops, const Params& p, cudaStream_t st) {
 
 template <int EPI, int QBIT, bool B_MN>
 static int launch(const Operands& ops, const Params& p, cudaStream_t st) {
-  const SplitPlan plan = choose_split(EPI, p);
+  const SplitPlan plan = choose_split(EPI, B_MN, p);
   if (plan.split > 0) return launch_split(EPI, QBIT, B_MN, plan, ops, p, st);
   // Pairs, except where few rows would leave half of the tile empty, and for grad_down with many tiles: its epilogue is
   // the longest (mma.sync products, which queue behind a busy tensor pipe) and in a pair a stall of either SM holds up
@@ -477,6 +477,30 @@ extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
   p.l0 = make_term(xa0, bt0, bt0_ld_col, bt0_ld_r);
   p.l1 = make_term(xa1, bt1, bt1_ld_col, bt1_ld_r);
   p.l2 = make_term(nullptr, nullptr, 0, 0);
+  p.residual = (const __nv_bfloat16*)residual;
+  p.out0 = (__nv_bfloat16*)D;
+  p.status = status;
+  p.g_end0 = p.g_end1 = N;
+  cudaStream_t st = (cudaStream_t)stream;
+  return b_is_kn ? launch<EPI_STORE, 4, true>(ops, p, st) : launch<EPI_STORE, 4, false>(ops, p, st);
+}
+
+extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
+                                                int b_is_kn, const void* residual, void* D, int* status, void* stream) {
+  if (!A || !B || !K || !D || !status) return HYC_ERR_NULL;
+  if (count < 1 || count > 4 || M <= 0 || N <= 0 || N % BN != 0) return HYC_ERR_SHAPE;
+  if (!aligned(D, 16) || (residual && !aligned(residual, 16))) return HYC_ERR_ALIGN;
+  Operands ops = {};
+  for (int i = 0; i < count; ++i) {
+    if (!A[i] || !B[i]) return HYC_ERR_NULL;
+    if (K[i] <= 0 || K[i] % BK != 0) return HYC_ERR_SHAPE;
+    if (!aligned(A[i], 16) || !aligned(B[i], 16)) return HYC_ERR_ALIGN;
+    ops.a[i] = {A[i], M, K[i]};
+    ops.b[i] = b_is_kn ? Matrix{B[i], K[i], N} : Matrix{B[i], N, K[i]};
+  }
+  Params p = {};
+  p.M = M; p.N = N; p.epi = EPI_STORE;
+  p.K1 = K[0]; p.K2 = count > 1 ? K[1] : 0; p.K3 = count > 2 ? K[2] : 0; p.K4 = count > 3 ? K[3] : 0;
   p.residual = (const __nv_bfloat16*)residual;
   p.out0 = (__nv_bfloat16*)D;
   p.status = status;

@@ -41,12 +41,12 @@ struct LoraTerm {
   int64_t ld_col, ld_r;
 };
 
-// tensor maps of a launch: up to three K segments (A, B) or three weights side by side; n: the B operands again in boxes of
+// tensor maps of a launch: up to four K segments (A, B) or three weights side by side; n: the B operands again in boxes of
 // 64 rows, for the half-width tiles of a K-major B
-struct Maps { CUtensorMap a[3], b[3], n[3]; };
+struct Maps { CUtensorMap a[4], b[4], n[4]; };
 
 struct Params {
-  int M, N, K1, K2, K3;       // K2, K3 > 0: further (A, B) pairs accumulated into the same tile
+  int M, N, K1, K2, K3, K4;   // K2, K3, K4 > 0: further (A, B) pairs accumulated into the same tile
   int epi, q_bit;
   LoraTerm l0, l1, l2;        // STORE: l0/l1 added; GATEUP: l0 gate, l1 up; GRADDOWN: l0 grad LoRA, l1 gate, l2 up
   const __nv_bfloat16* residual;   // STORE, [M, N] or null
@@ -673,6 +673,13 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 #define HYC_PROMO CU_TENSOR_MAP_L2_PROMOTION_L2_128B
 #endif
 inline EncodeTiledFn get_encode() {
+  // the encoder is a driver function: a thread whose first CUDA work is this call has no context current yet (the
+  // runtime binds the device's primary context, once per thread)
+  static thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+  }
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void* sym = nullptr;
@@ -700,9 +707,9 @@ inline bool make_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols
 
 // the matrices behind the maps: row-major, p == nullptr repeats entry 0
 struct Matrix { const void* p; int64_t rows, cols; };
-struct Operands { Matrix a[3], b[3]; };
+struct Operands { Matrix a[4], b[4]; };
 inline bool make_maps(Maps* m, const Operands& o, bool b_mn, int a_rows, int b_rows, bool narrow) {
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < 4; ++i) {
     if (o.a[i].p == nullptr) m->a[i] = m->a[0];
     else if (!make_map(&m->a[i], o.a[i].p, o.a[i].rows, o.a[i].cols, a_rows)) return false;
     if (o.b[i].p == nullptr) { m->b[i] = m->b[0]; m->n[i] = m->n[0]; continue; }

@@ -74,7 +74,7 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
   const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
   const int tile = (int)blockIdx.x / (PAIR ? 2 * split : split);
   const int m0 = (tile % tiles_m) * TILE_M + half * BM, nt = (tile / tiles_m) * TILE_N;
-  const int kb1 = p.K1 / BK, kb2 = (p.K1 + p.K2) / BK, kb_total = (p.K1 + p.K2 + p.K3) / BK;
+  const int kb1 = p.K1 / BK, kb2 = (p.K1 + p.K2) / BK, kb3 = (p.K1 + p.K2 + p.K3) / BK, kb_total = kb3 + p.K4 / BK;
   const int kb_lo = (int)((int64_t)kb_total * rank / split), kb_hi = (int)((int64_t)kb_total * (rank + 1) / split);
   const StoreView sv = store_view(p, nt);
 
@@ -121,10 +121,10 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
           if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_PRODUCER); }
           break;
         }
-        const int seg = kb < kb1 ? 0 : (kb < kb2 ? 1 : 2);
+        const int seg = kb < kb1 ? 0 : (kb < kb2 ? 1 : (kb < kb3 ? 2 : 3));
         const int wsel = EPI == EPI_STORE && sv.group > 0 ? sv.group : seg;
         const CUtensorMap *ma = &maps.a[seg], *mb = &maps.b[wsel];
-        const int k0 = (seg == 0 ? kb : (seg == 1 ? kb - kb1 : kb - kb2)) * BK;
+        const int k0 = (kb - (seg == 0 ? 0 : (seg == 1 ? kb1 : (seg == 2 ? kb2 : kb3)))) * BK;
         const int n0 = EPI == EPI_STORE ? sv.n0 : nt;
         const uint32_t sa = smem_u32(smem + stage * stage_bytes), sb = sa + (uint32_t)a_bytes;
         const uint32_t fbar = PAIR ? map_to_cta(&full[stage], leader) : smem_u32(&full[stage]);
@@ -331,14 +331,17 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
 }
 
 // Where the line lies (B200, Llama-2-7B weights, us per product, persistent / split):
-//   up to 128 tokens, S = the largest of 4, 2, 1 with at most one CTA per SM: [128,4096]x[4096,4096] 21.8 / 16.6,
-//     x[4096,11008] 42 / 26.5, the three-segment grad_x 67 / 37, gate/up 48.9 / 43.8, q/k/v 38 / 33.  The grad_down
-//     product has more column tiles than SMs can take at once either way and stays persistent: 28.8 / 30.3
+//   up to 128 tokens, S = the largest of 4, 2, 1 with at most one CTA per SM: x[4096,11008] 42 / 26.5, grad_o 21.8 / 16.6,
+//     the three-segment grad_x 67 / 37; unsplit (S = 1) gate/up 48.9 / 43.8, q/k/v 38 / 33.  The grad_down product has
+//     more column tiles than SMs can take at once either way and stays persistent: 28.8 / 30.3
 //   129 to 256 tokens, pair form, S = 2: 21.8 / 19.0, 43 / 30.6, 69 / 45; wider products fill the chip without it
 //   512 tokens: 45 / 47, 75 / 77: persistent
 // A CTA keeps at least 16 k-blocks: below that its share of the main loop is shorter than set-up and reduction (about
 // 3 us), and the sum over all of K stays in one accumulator.
-SplitPlan choose_split(int epi, const Params& p) {
+// Products whose results the layer quantizes, or that feed tensors it quantizes (gate/up, q/k/v, the K-major ones of fewer
+// than 128 k-blocks: the o projection), are not split: the saved codes then do not depend on how many rows are computed
+// together (with 2-bit codes one that flips moves a value by a third of its range).  That leaves 5 us on the o projection.
+SplitPlan choose_split(int epi, bool b_mn, const Params& p) {
   SplitPlan plan = {0, false};
 #ifdef HYC_TUNE
   if (const char* e = getenv("HYC_SPLIT")) { if (atoi(e) >= 100) return plan; plan.split = atoi(e) % 10; plan.pair = atoi(e) >= 10; return plan; }
@@ -346,12 +349,15 @@ SplitPlan choose_split(int epi, const Params& p) {
   if (epi == EPI_GRADDOWN || p.M > 2 * BM) return plan;
   if (epi == EPI_STORE && p.l1.bt != nullptr) return plan;         // a second LoRA term: the persistent kernel's own epilogue
   const int tiles = p.N / (epi == EPI_GATEUP ? SBN / 2 : SBN), sms = num_sms();
-  const int kb = (p.K1 + p.K2 + p.K3) / BK;
-  if (p.M <= BM) {
+  const int kb = (p.K1 + p.K2 + p.K3 + p.K4) / BK;
+  const bool whole = epi == EPI_GATEUP || p.q1 != nullptr || (!b_mn && kb < 128);
+  if (whole) {
+    if (p.M <= BM && tiles >= sms / 4) plan.split = 1;      // fewer tiles: half-width tiles of the persistent kernel
+  } else if (p.M <= BM) {
     plan.split = 1;
-    for (int s = 2; s <= (epi == EPI_GATEUP ? 2 : 4); s *= 2)
+    for (int s = 2; s <= 4; s *= 2)
       if (tiles * s <= sms && kb >= 16 * s) plan.split = s;
-  } else if (epi == EPI_STORE && tiles * 4 <= sms && kb >= 32) {
+  } else if (tiles * 4 <= sms && kb >= 32) {
     plan = {2, true};
   }
   return plan;

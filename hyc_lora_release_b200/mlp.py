@@ -39,17 +39,6 @@ def check_status(status, what):
         raise HycError("%s: %s" % (what, _KERNEL_STATUS.get(v, "status %d" % v)))
 
 
-def padded_block(owner, name, T, dev):
-    """A [T, 64] bf16 block of zeros kept on ``owner`` between steps (the rank-16 products of a backward pass are
-    written side by side into its first columns and ride a GEMM as one K block of 64; the other columns are never
-    written and stay zero, so the block is filled once, not once per step)."""
-    buf = getattr(owner, name, None)
-    if buf is None or buf.shape[0] != T or buf.device != dev:
-        buf = torch.zeros((T, 64), dtype=BF16, device=dev)
-        setattr(owner, name, buf)
-    return buf
-
-
 def _lora(xa, bt, ld_col, ld_r):
     if xa is None:
         return [None, None, 0, 0]
@@ -133,9 +122,8 @@ class MLPWeights:
           ad_cols  [I, 64]  columns 0..15 = Ad^T       (projects hadamard to the padded down LoRA activation)
           bd_cols  [H, 64]  columns 0..15 = Bd         (second operand of the down projection's LoRA part, [N, K])
           agu_rows [64, H]  rows 0..15 = Ag, 16..31 = Au (second operand of grad_x's LoRA part, [K, N])
-        and the stacked factors of the batched rank-16 products:
-          agu_t    [2, H, r]  Ag^T, Au^T  (x_norm @ both in one call)
-          bgu      [2, I, r]  Bg, Bu      (grad_gate @ Bg and grad_up @ Bu in one call)"""
+        and the transposed factors of the rank-16 products:
+          agu_t    [2, H, r]  Ag^T, Au^T  (x_norm @ both in one call)"""
         key = tuple(t._version for t in (self.ag, self.au, self.ad, self.bd, self.bg, self.bu))
         if getattr(self, "_pad_key", None) != key:
             r, I = self.ad.shape
@@ -145,9 +133,8 @@ class MLPWeights:
             bd_cols = torch.zeros(H, 64, dtype=dt, device=dev); bd_cols[:, :r] = self.bd
             agu_rows = torch.zeros(64, H, dtype=dt, device=dev); agu_rows[:r] = self.ag; agu_rows[r:2 * r] = self.au
             agu_t = torch.stack((self.ag.t(), self.au.t())).contiguous()      # [2, H, r]
-            bgu = torch.stack((self.bg, self.bu)).contiguous()                # [2, I, r]
             self._pad = dict(ad_rows=ad_rows, ad_cols=ad_rows.t().contiguous(), bd_cols=bd_cols, agu_rows=agu_rows,
-                             agu_t=agu_t, bgu=bgu)
+                             agu_t=agu_t)
             self._pad_key = key
         return self._pad
 
@@ -250,17 +237,16 @@ def mlp_backward(grad_out, saved, w: MLPWeights, status=None, on_lora_grads=None
     st = status if status is not None else _status_tensor(dev)
     g = grad_out.to(BF16).reshape(T, H).contiguous()
     pad = w.padded()
-    gm64 = padded_block(w, "_gm64", T, dev)
     gu_xa = saved.get('gu_xa')
     if gu_xa is None:
         gu_xa = torch.stack((saved['gate_xa'], saved['up_xa']))
-    # grad_down GEMM with the SiLU-Hadamard backward in its epilogue (grad_gate and grad_up land in one buffer, their
-    # rank-16 products run as one batched call each), then the six LoRA gradients: the A side of gate and up in one
-    # pass over the packed x_norm, de-quantized in shared memory
-    had, ggu, grad_bd, grad_ad, ga, grad_bgu = host.mlp_backward_lora(
-        g, [w.wd, w.bg, w.bu, pad["bd_cols"], pad["ad_rows"], pad["bgu"]],
+    # grad_down GEMM with the SiLU-Hadamard backward in its epilogue, then the six LoRA gradients: the rank-16 products of
+    # grad_gate, grad_up and hadamard from one read of each, the A side of gate and up in one pass over the packed
+    # x_norm, de-quantized in shared memory
+    had, ggu, gm64, grad_bd, grad_ad, ga, grad_bgu = host.mlp_backward_lora(
+        g, [w.wd, w.bg, w.bu, w.bd, pad["ad_rows"]],
         [saved['gate_q'], saved['gate_scale'], saved['up_q'], saved['up_scale'], gu_xa, saved['down_xa'], saved['xn_q'],
-         saved['xn_scale']], gm64, q, st)
+         saved['xn_scale']], q, st)
     grads = dict(grad_ag=ga[:16], grad_bg=grad_bgu[0], grad_au=ga[16:32], grad_bu=grad_bgu[1], grad_ad=grad_ad, grad_bd=grad_bd)
     if on_lora_grads is not None:
         on_lora_grads(dict(grads))

@@ -85,7 +85,7 @@ class QuantizedWeight:
         return host.dequant_nf4(self.packed, self.code, self.absmax, None, None, 1, 0.0, self.blocksize, self.shape)
 
 
-_CACHE_ATTRS = ("_pad", "_pad_key", "_gm64", "_gmq")      # what AttnWeights / MLPWeights keep between steps
+_CACHE_ATTRS = ("_pad", "_pad_key")      # what AttnWeights / MLPWeights keep between steps
 
 
 def materialize(record):
@@ -103,7 +103,7 @@ def materialize(record):
 
 
 def release(record, used):
-    """After the pass: keep the scratch the pass created on the copy (padded factors, zero blocks), drop the bf16
+    """After the pass: keep what the pass created on the copy (padded factors), drop the bf16
     weights."""
     if used is record:
         return

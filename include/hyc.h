@@ -297,6 +297,10 @@ int hyc_gemm_bf16_tcgen05(const void* A, const void* B, int M, int N, int K, int
                           const void* xa1, const void* bt1, int64_t bt1_ld_col, int64_t bt1_ld_r,
                           const void* residual, void* D, int* status, void* stream);
 
+/* The same without LoRA terms for one to four (A, B) pairs: host arrays of `count` entries, A[i] [M, K[i]]. */
+int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
+                              int b_is_kn, const void* residual_or_null, void* D, int* status, void* stream);
+
 /* A LoRA projection with the save of its main branch in the GEMM epilogue (the q/k/v/o projections of the
  * attention half: `lora_forward` followed by `compression_pack_quant_base(x=q_main, ...)`,
  * fused_llama_layer_intra_inter_full_fuse.py:112-142; models/utils/compute_utils.py:18-25):
@@ -346,6 +350,25 @@ int hyc_mlp_graddown_bwd_tcgen05(const void* g, const void* wd, int T, int H, in
                                  const void* q1, const void* s1, const void* q2, const void* s2,
                                  const void* lora_gate, const void* lora_up, int64_t ld_lora,
                                  void* o, void* grad_gate, void* grad_up, int q_bit, int* status, void* stream);
+
+/* ---- rank-16 products with a large operand ------------------------------------------------------
+ *
+ * For each of up to three x [T, n] (bf16, row stride ldx, n % 8 == 0), from one read of it:
+ *   y[i] = x * w[i]     w[i] [n, 16] (row stride ld_w), y[i] [T, 16] bf16 (row stride ld_y); after the last y the next
+ *                       y_pad columns are set to zero (the product then rides a GEMM as a K block of 64)
+ *   z = x^T * xa        xa [T, 16] (row stride ld_xa), z [n, 16] bf16, or [16, n] if z_transposed; NULL: not wanted
+ * fp32 accumulation in a fixed order.  These are the LoRA terms of lora_forward / lora_backward
+ * (models/utils/compute_utils.py:18-36). */
+typedef struct {
+  const void* x; int64_t ldx;
+  const void* w[3]; int64_t ld_w;
+  void* y[3]; int64_t ld_y;
+  const void* xa; int64_t ld_xa;
+  void* z;
+  int n, n_w, y_pad, z_transposed;
+} hyc_skinny_job;
+size_t hyc_skinny_workspace_bytes(int count, const hyc_skinny_job* jobs, int T);
+int hyc_skinny_products(int count, const hyc_skinny_job* jobs, int T, void* workspace, size_t workspace_bytes, int* status, void* stream);
 
 /* ---- attention of the fused layer (heads of 128 columns, M % 8 == 0, M <= 4096) ----------------
  *
