@@ -458,21 +458,47 @@ fused_silu_wide_kernel(const __nv_bfloat16* __restrict__ xa1, const __nv_bfloat1
 // main branch was saved as codes (the q/k/v projections: `decompression_dequantization` followed by
 // `+ x_lora_a @ w_lora_b`, fused_llama_layer_intra_inter_full_fuse.py:416-452).  Same layout as the wide
 // kernel above with one branch.
-template <int QBIT>
+// HEADS: up to three projections side by side in the grid, each a whole number of heads of 128 columns wide, and for the
+// ones with `rope` set the rotary embedding behind the sum.  A warp then owns columns [32 w, 32 w + 32) of BOTH halves of a
+// head, so that the partner of a value sits four lanes away.  Three launches and the two of the embedding become one:
+// 2048 tokens, 32 heads, 4 bits: 24.7 + 14.6 us before.
+struct RebuildJob { const __nv_bfloat16 *xa, *bt, *s; const uint8_t* q; __nv_bfloat16* y; int n, first_block; bool rope; };
+struct RebuildJobs { RebuildJob job[3]; const void *cos, *sin; int64_t ld_table; int table_f32, seq_len, count; };
+
+// the rotation of a packed pair; own: the lane's half, other: the other half; `upper`: the lane has the second half.
+// Rounding points: rope.cu
+__device__ __forceinline__ uint32_t rotate_bf16(uint32_t own, uint32_t other, uint32_t c, uint32_t s, bool upper) {
+  const uint32_t a = mul2(own, c), b = mul2(other, s);
+  return upper ? add2(a, b) : sub2(a, b);
+}
+__device__ __forceinline__ float rotate_f32(float own, float other, float c, float s, bool upper) {
+  const float a = __fmul_rn(own, c), b = __fmul_rn(other, s);
+  return upper ? __fadd_rn(a, b) : __fsub_rn(a, b);
+}
+
+template <int QBIT, bool HEADS>
 __global__ void __launch_bounds__(256, HYC_FUSED_MINB)
-dequant_lora_add_kernel(const __nv_bfloat16* __restrict__ xa, const __nv_bfloat16* __restrict__ bt,
-                        const __nv_bfloat16* __restrict__ sv, const uint8_t* __restrict__ q,
-                        __nv_bfloat16* __restrict__ y, int64_t rows, int N) {
+dequant_lora_add_kernel(const RebuildJobs jobs, int64_t rows) {
+  const int which = !HEADS || jobs.count < 2 || (int)blockIdx.x < jobs.job[1].first_block ? 0 : ((int)blockIdx.x < jobs.job[2].first_block ? 1 : 2);
+  const __nv_bfloat16* __restrict__ xa = jobs.job[which].xa;
+  const __nv_bfloat16* __restrict__ bt = jobs.job[which].bt;
+  const __nv_bfloat16* __restrict__ sv = jobs.job[which].s;
+  const uint8_t* __restrict__ q = jobs.job[which].q;
+  __nv_bfloat16* __restrict__ y = jobs.job[which].y;
+  const int N = jobs.job[which].n;
+  const bool rope = HEADS && jobs.job[which].rope;
   constexpr int EPP = 8 / QBIT;
   constexpr uint32_t CM = (1u << QBIT) - 1u, BM = CM * 0x01010101u;
   __shared__ __align__(16) uint32_t s_l[8][16 * kWideLd];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int c0 = 64 * (blockIdx.x * 8 + warp);
-  if (c0 >= N) return;
+  const int wi = ((int)blockIdx.x - jobs.job[which].first_block) * 8 + warp;      // 64 columns per warp
+  if (64 * wi >= N) return;
+  // first column of the warp's octet o (0..7)
+  auto octet = [&](int o) { return HEADS ? 128 * (wi >> 1) + 32 * (wi & 1) + 8 * (o & 3) + 64 * (o >> 2) : 64 * wi + 8 * o; };
   const int64_t qld = (int64_t)N / EPP;
   uint32_t* sl = s_l[warp];
   const int cl = lane & 7, rsub = lane >> 3;
-  const int col = c0 + 8 * cl;
+  const int col = octet(cl);
   const bool col_ok = col < N;
   const int blk = col >> 5, cg = (col >> 3) & 3;
   uint32_t sp[4] = {0u, 0u, 0u, 0u};
@@ -506,7 +532,7 @@ dequant_lora_add_kernel(const __nv_bfloat16* __restrict__ xa, const __nv_bfloat1
       }
 #pragma unroll 2
       for (int nt = 0; nt < 8; ++nt) {
-        const int n = c0 + 8 * nt + g;
+        const int n = octet(nt) + g;
         uint32_t ba = 0u, bb = 0u;
         if (n < N) {
           ba = *reinterpret_cast<const uint32_t*>(bt + (int64_t)n * 16 + 2 * t);
@@ -542,6 +568,31 @@ dequant_lora_add_kernel(const __nv_bfloat16* __restrict__ xa, const __nv_bfloat1
         }
         o[j] = add2(x, lw[j]);
       }
+      if (HEADS && rope) {      // block-uniform
+        uint32_t other[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) other[j] = __shfl_xor_sync(0xffffffffu, o[j], 4);
+        const int pos = (int)((uint32_t)row % (uint32_t)jobs.seq_len), j0 = (col & 63);
+        const bool upper = cl >= 4;
+        if (row < rows) {
+          if (jobs.table_f32) {
+            const float* cp = reinterpret_cast<const float*>(jobs.cos) + pos * jobs.ld_table + j0;
+            const float* sp = reinterpret_cast<const float*>(jobs.sin) + pos * jobs.ld_table + j0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 c = *reinterpret_cast<const float2*>(cp + 2 * j), s = *reinterpret_cast<const float2*>(sp + 2 * j);
+              o[j] = pack_bf16x2_rn(rotate_f32(bf16lo_to_f32(o[j]), bf16lo_to_f32(other[j]), c.x, s.x, upper),
+                                    rotate_f32(bf16hi_to_f32(o[j]), bf16hi_to_f32(other[j]), c.y, s.y, upper));
+            }
+          } else {
+            const uint4 c = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(jobs.cos) + pos * jobs.ld_table + j0);
+            const uint4 s = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(jobs.sin) + pos * jobs.ld_table + j0);
+            const uint32_t cw[4] = {c.x, c.y, c.z, c.w}, sw[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = rotate_bf16(o[j], other[j], cw[j], sw[j], upper);
+          }
+        }
+      }
       if (row < rows && col_ok) st_stream_v4(y + row * N + col, make_uint4(o[0], o[1], o[2], o[3]));
     }
     __syncwarp();
@@ -551,8 +602,7 @@ dequant_lora_add_kernel(const __nv_bfloat16* __restrict__ xa, const __nv_bfloat1
 // one resident wave: every block walks down the rows with a fixed stride, so a second, partial wave would
 // only add a tail
 template <typename K>
-static inline dim3 fused_wide_grid(K kern, int64_t rows, int N) {
-  const int cgroups = ((N + 63) / 64 + 7) / 8;
+static inline dim3 wide_grid(K kern, int64_t rows, int cgroups) {
   const int64_t tiles = (rows + 15) / 16;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 2;
@@ -562,6 +612,9 @@ static inline dim3 fused_wide_grid(K kern, int64_t rows, int N) {
   if (slots > 65535) slots = 65535;
   return dim3((unsigned)cgroups, (unsigned)slots, 1);
 }
+
+template <typename K>
+static inline dim3 fused_wide_grid(K kern, int64_t rows, int N) { return wide_grid(kern, rows, ((N + 63) / 64 + 7) / 8); }
 
 static inline dim3 fused_grid(int64_t rows, int N) {
   const int cgroups = (N / 32 + 7) / 8;
@@ -659,8 +712,37 @@ extern "C" HYC_API int hyc_dequant_lora_add(const void* q, const void* scale, co
   if (rc) return rc;
   if (!aligned(q, 8) || !aligned(scale, 16) || !aligned(xa, 4) || !aligned(bt, 4) || !aligned(y, 16)) return HYC_ERR_ALIGN;
   if (rows == 0) return HYC_OK;
-#define DL(QB) dequant_lora_add_kernel<QB><<<fused_wide_grid(dequant_lora_add_kernel<QB>, rows, N), 256, 0, (cudaStream_t)stream>>>( \
-      (const __nv_bfloat16*)xa, (const __nv_bfloat16*)bt, (const __nv_bfloat16*)scale, (const uint8_t*)q, (__nv_bfloat16*)y, rows, N)
+  RebuildJobs jobs = {};
+  jobs.job[0] = {(const __nv_bfloat16*)xa, (const __nv_bfloat16*)bt, (const __nv_bfloat16*)scale, (const uint8_t*)q, (__nv_bfloat16*)y, N, 0, false};
+  jobs.count = 1;
+#define DL(QB) dequant_lora_add_kernel<QB, false><<<fused_wide_grid(dequant_lora_add_kernel<QB, false>, rows, N), 256, 0, (cudaStream_t)stream>>>(jobs, rows)
+  if (q_bit == 2) DL(2); else if (q_bit == 4) DL(4); else DL(8);
+#undef DL
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
+}
+
+extern "C" HYC_API int hyc_rebuild_qkv(const void* const* q, const void* const* scale, const void* const* xa, const void* const* bt, void* const* y,
+                                       const int* n, const void* cos_t, const void* sin_t, int64_t ld_table, int table_is_f32,
+                                       int64_t rows, int seq_len, int q_bit, void* stream) {
+  if (!q || !scale || !xa || !bt || !y || !n || !cos_t || !sin_t) return HYC_ERR_NULL;
+  if (rows < 0 || rows > 0xffffffffll || seq_len < 1 || ld_table < 64) return HYC_ERR_SHAPE;
+  if ((ld_table & (table_is_f32 ? 3 : 7)) != 0 || !aligned(cos_t, 16) || !aligned(sin_t, 16)) return HYC_ERR_ALIGN;
+  RebuildJobs jobs = {};
+  int blocks = 0;
+  for (int i = 0; i < 3; ++i) {
+    if (!q[i] || !scale[i] || !xa[i] || !bt[i] || !y[i]) return HYC_ERR_NULL;
+    const int rc = check_fused(rows, n[i], 16, q_bit);
+    if (rc) return rc;
+    if (n[i] % 128 != 0) return HYC_ERR_SHAPE;
+    if (!aligned(q[i], 8) || !aligned(scale[i], 16) || !aligned(xa[i], 4) || !aligned(bt[i], 4) || !aligned(y[i], 16)) return HYC_ERR_ALIGN;
+    jobs.job[i] = {(const __nv_bfloat16*)xa[i], (const __nv_bfloat16*)bt[i], (const __nv_bfloat16*)scale[i], (const uint8_t*)q[i],
+                   (__nv_bfloat16*)y[i], n[i], blocks, i < 2};
+    blocks += (n[i] / 64 + 7) / 8;
+  }
+  jobs.cos = cos_t; jobs.sin = sin_t; jobs.ld_table = ld_table; jobs.table_f32 = table_is_f32; jobs.seq_len = seq_len; jobs.count = 3;
+  if (rows == 0) return HYC_OK;
+#define DL(QB) dequant_lora_add_kernel<QB, true><<<wide_grid(dequant_lora_add_kernel<QB, true>, rows, blocks), 256, 0, (cudaStream_t)stream>>>(jobs, rows)
   if (q_bit == 2) DL(2); else if (q_bit == 4) DL(4); else DL(8);
 #undef DL
   HYC_CHECK_LAUNCH();

@@ -3,6 +3,7 @@
 // launch, more than most kernels of a short sequence run for.
 #pragma once
 #include <torch/extension.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <initializer_list>
@@ -32,9 +33,12 @@ void check_q(int64_t q);
 inline const Tensor* opt(const OptTensor& t) { return t.has_value() && t->defined() ? &*t : nullptr; }
 inline bool given(const OptTensor& t) { return t.has_value() && t->defined(); }
 inline Tensor bf16c(const Tensor& t) { return t.to(at::kBFloat16).contiguous(); }
-inline Tensor vec(const Tensor& s) { return s.to(at::kBFloat16).reshape({-1}).contiguous(); }
+inline Tensor vec(const Tensor& s) {
+  if (s.dim() == 1 && s.scalar_type() == at::kBFloat16 && s.is_contiguous()) return s;
+  return s.to(at::kBFloat16).reshape({-1}).contiguous();
+}
 inline Tensor empty(at::IntArrayRef sz, const Tensor& like, at::ScalarType ty = at::kBFloat16) {
-  return at::empty(sz, like.options().dtype(ty).requires_grad(false));
+  return at::detail::empty_cuda(sz, ty, like.device(), std::nullopt);
 }
 inline void* data(const Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr; }
 inline void* data(const OptTensor& t) { return given(t) ? data(*t) : nullptr; }
@@ -73,6 +77,11 @@ Tensor dequant_nf4(const Tensor& packed, const Tensor& code, const Tensor& absma
                    int64_t blocksize2, double offset, int64_t blocksize, at::IntArrayRef shape);
 
 // ---- GEMMs and the two halves of the layer (host_blocks.cpp)
+struct RopeTables {                              // [>= seq, >= d / 2], bf16 or fp32, the same row stride
+  Tensor cos, sin;
+  int f32() const { return cos.scalar_type() == at::kFloat ? 1 : 0; }
+};
+RopeTables rope_tables(const Tensor& cos, const Tensor& sin, int64_t seq, int64_t d);
 Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64_t r2, int64_t q_bit);
 void bind_ops(pybind11::module_& m);
 void bind_blocks(pybind11::module_& m);

@@ -102,7 +102,7 @@ Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64
 // ------------------------------------------------------------------ MLP half
 struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa, down_xa64; };
 
-static std::vector<Tensor> mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
+static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
                                        const OptTensor& bias_d, int64_t q, double eps, const Tensor& status) {
   const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &wd = w[3], &bg = w[4], &bu = w[5], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
@@ -198,11 +198,31 @@ static MaskView mask_view(const OptTensor& mask, int64_t B, int64_t nh, int64_t 
 }
 static bool attn_kernels_take(int64_t M, int64_t d) { return d == 128 && M % 8 == 0 && M <= 4096; }
 
+RopeTables rope_tables(const Tensor& cos_in, const Tensor& sin_in, int64_t seq, int64_t d) {
+  RopeTables t{cos_in.dim() == 2 ? cos_in : cos_in.squeeze(), sin_in.dim() == 2 ? sin_in : sin_in.squeeze()};
+  TORCH_CHECK_VALUE(t.cos.dim() == 2 && t.sin.sizes() == t.cos.sizes(), "cos / sin must squeeze to [seq_len, head_dim] tables");
+  if (seq > t.cos.size(0)) {
+    PyErr_SetString(PyExc_AssertionError, "the rotary tables are shorter than the sequence");
+    throw pybind11::error_already_set();
+  }
+  TORCH_CHECK_VALUE(t.cos.size(1) >= d / 2, "cos / sin tables are narrower than head_dim / 2");
+  if (t.cos.scalar_type() != at::kBFloat16 && t.cos.scalar_type() != at::kFloat) t.cos = t.cos.to(at::kFloat);
+  if (t.sin.scalar_type() != t.cos.scalar_type()) t.sin = t.sin.to(t.cos.scalar_type());
+  if (t.cos.stride(1) != 1 || t.sin.stride(1) != 1 || t.sin.stride(0) != t.cos.stride(0)) { t.cos = t.cos.contiguous(); t.sin = t.sin.contiguous(); }
+  return t;
+}
+// q and k (contiguous [rows, heads*d]) in place
+static void rope_pair(const Tensor& q, int64_t nh, const Tensor& k, int64_t nkv, const RopeTables& t, int64_t seq, int64_t d, bool backward,
+                      void* stream) {
+  require_cuda({&q, &k, &t.cos, &t.sin});
+  check(hyc_rope_pair(data(q), (int)nh, data(k), (int)nkv, data(t.cos), data(t.sin), t.cos.stride(0), t.f32(), q.size(0), (int)seq, (int)d,
+                      backward ? 1 : 0, stream), "hyc_rope_pair");
+}
+
 // the q, k, v projections with their saves, rotary embedding, scores and probabilities
 using MapForward = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor, OptTensor, int64_t, int64_t>;
-static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos,
-                                            const Tensor& sin, const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps,
-                                            const Tensor& status) {
+static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const RopeTables& tables,
+                                   const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status) {
   const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
   require_cuda({&x, &wq});
@@ -215,8 +235,7 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
   const auto &[qy, q_q] = p3[0];
   const auto &[ky, k_q] = p3[1];
   const auto &[vy, v_q] = p3[2];
-  rope(qy.view({B, M, nh, d}), cos, sin, false, true);
-  rope(ky.view({B, M, nkv, d}), cos, sin, false, true);
+  rope_pair(qy, nh, ky, nkv, tables, M, d, false, on.stream);
   if (attn_kernels_take(M, d)) {
     // one kernel from q, k, v to the probabilities, o and the codes of o
     const MaskView mv = mask_view(mask, B, nh, M);
@@ -276,7 +295,7 @@ static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, 
 // restores once more on chip), empty for the pruned form.  -> grad_q, grad_k, grad_v [T, n*d] after the inverse
 // rotation
 static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, const std::vector<Tensor>& topk, int64_t map_q_bit,
-                                                const std::vector<Tensor>& saved, const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin,
+                                                const std::vector<Tensor>& saved, const std::vector<Tensor>& w, const RopeTables& tables,
                                                 int64_t B, int64_t M, int64_t nh, int64_t d, int64_t nkv, int64_t q,
                                                 const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status) {
   const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
@@ -285,16 +304,27 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
   const int64_t T = B * M, rep = nh / nkv;
   const double scale = 1.0 / std::sqrt((double)d);
   if (attn_kernels_take(M, d)) {
-    const Tensor q2 = rebuild(q_q, q_s, q_xa, w[0], q), k2 = rebuild(k_q, k_s, k_xa, w[1], q), v2 = rebuild(v_q, v_s, v_xa, w[2], q);
-    rope(q2.view({B, M, nh, d}), cos, sin, false, true);
-    rope(k2.view({B, M, nkv, d}), cos, sin, false, true);
+    // q, k (rotated) and v from their codes in one launch
+    Tensor rebuilt[3], keep[9];
+    const void *cp[3], *sp[3], *xp[3], *bp[3];
+    void* yp[3];
+    int n[3];
+    for (int i = 0; i < 3; ++i) {
+      n[i] = (int)((i == 0 ? nh : nkv) * d);
+      rebuilt[i] = empty({T, n[i]}, grad_o2);
+      cp[i] = data(keep[3 * i] = saved[3 * i].contiguous()); sp[i] = data(keep[3 * i + 1] = vec(saved[3 * i + 1]));
+      xp[i] = data(saved[3 * i + 2]); bp[i] = data(keep[3 * i + 2] = w[i].contiguous()); yp[i] = data(rebuilt[i]);
+    }
+    require_cuda({&q_q, &k_q, &v_q, &w[0], &tables.cos, &tables.sin});
+    check(hyc_rebuild_qkv(cp, sp, xp, bp, yp, n, data(tables.cos), data(tables.sin), tables.cos.stride(0), tables.f32(), T, (int)M, (int)q, on.stream),
+          "hyc_rebuild_qkv");
+    const Tensor &q2 = rebuilt[0], &k2 = rebuilt[1], &v2 = rebuilt[2];
     Tensor gs = empty({B, nh, M, M}, grad_o2);
     Tensor gq = empty({T, nh * d}, grad_o2), gk = empty({T, nkv * d}, grad_o2), gv = empty({T, nkv * d}, grad_o2);
     check(hyc_attn_bwd_tcgen05(data(q2), data(k2), data(v2), data(grad_o2), data(a), data(gs), (int)B, (int)M, (int)nh, (int)nkv, (int)d,
                                (float)scale, data(cls), cls_b, cls_h, data(gq), data(gk), data(gv), status_ptr(status), on.stream),
           "hyc_attn_bwd_tcgen05");
-    rope(gq.view({B, M, nh, d}), cos, sin, true, true);
-    rope(gk.view({B, M, nkv, d}), cos, sin, true, true);
+    rope_pair(gq, nh, gk, nkv, tables, M, d, true, on.stream);
     return {gq, gk, gv};
   }
   const Tensor grad_oh = heads(grad_o2, B, M, nh);
@@ -314,15 +344,14 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
   }
   grad_a.reset();
   Tensor q2 = rebuild(q_q, q_s, q_xa, w[0], q);
-  rope(q2.view({B, M, nh, d}), cos, sin, false, true);
+  rope(q2.view({B, M, nh, d}), tables.cos, tables.sin, false, true);
   Tensor grad_k = rep == 1 ? matmul_to_hidden(grad_s.transpose(-2, -1), heads(q2, B, M, nh))
                            : hidden(repeat_kv_backward(at::matmul(grad_s.transpose(-2, -1), heads(q2, B, M, nh)), rep));
   q2.reset();
   Tensor k2 = rebuild(k_q, k_s, k_xa, w[1], q);
-  rope(k2.view({B, M, nkv, d}), cos, sin, false, true);
+  rope(k2.view({B, M, nkv, d}), tables.cos, tables.sin, false, true);
   Tensor grad_q = matmul_to_hidden(grad_s, repeat_kv(heads(k2, B, M, nkv), rep));
-  rope(grad_q.view({B, M, nh, d}), cos, sin, true, true);
-  rope(grad_k.view({B, M, nkv, d}), cos, sin, true, true);
+  rope_pair(grad_q, nh, grad_k, nkv, tables, M, d, true, on.stream);
   return {grad_q, grad_k, grad_v};
 }
 
@@ -350,20 +379,228 @@ static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads,
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 
+// ------------------------------------------------------------------ the whole layer
+// Forward and backward of a calibrated layer as one call each: between the launches there is then no Python (attribute and
+// dictionary look-ups, argument conversion), which cost more than the kernels of a short sequence run for.
+// 128 tokens, Llama-2-7B, bf16 weights, host work per forward + backward: 863 us as ten calls.
+
+// a frozen projection: a bf16 matrix, or 4-bit codes that become one for the half of the pass that uses it
+struct FrozenWeight {
+  Tensor plain;
+  Tensor packed, code, absmax;
+  OptTensor code2, absmax2;
+  int64_t blocksize2 = 1, blocksize = 64;
+  double offset = 0;
+  std::vector<int64_t> shape;
+  Tensor get() const {
+    return plain.defined() ? plain : dequant_nf4(packed, code, absmax, code2, absmax2, blocksize2, offset, blocksize, shape);
+  }
+};
+
+enum { PQ, PK, PV, PO, PGATE, PUP, PDOWN, PROJECTIONS };
+enum { AQKV_T, AQKV_ROWS, AO_COLS, AO_ROWS, BO_COLS, AGU_T, AGU_ROWS, AD_ROWS, AD_COLS, BD_COLS, PADS };
+
+struct Stamp {                                  // a tensor as it was: the same storage, nothing written since
+  const void* p = nullptr;
+  uint32_t version = 0;
+  static Stamp of(const Tensor& t) { return {t.data_ptr(), t.is_inference() ? 0u : (uint32_t)t._version()}; }
+  bool operator==(const Stamp& o) const { return p == o.p && version == o.version; }
+};
+
+struct LayerPlan {
+  Tensor norm1, norm2;
+  FrozenWeight w[PROJECTIONS];
+  Tensor lora[2 * PROJECTIONS];                 // A, B of each projection
+  OptTensor bias_o, bias_d;
+  std::vector<Tensor> pad;                      // what AttnWeights.padded / MLPWeights.padded make of the LoRA factors
+  Stamp pad_of[2 * PROJECTIONS];
+  std::vector<Tensor> stats_in, stats;          // calibrated statistics as given, and as the kernels read them
+  std::vector<Stamp> stats_of;
+
+  // false: the padded factors are out of date, or a weight is no longer what it was checked to be
+  bool fresh() const {
+    if ((int)pad.size() != PADS) return false;
+    for (const FrozenWeight& f : w)
+      if (f.plain.defined() && f.plain.scalar_type() != at::kBFloat16) return false;
+    for (int i = 0; i < 2 * PROJECTIONS; ++i)
+      if (lora[i].scalar_type() != at::kBFloat16 || !(Stamp::of(lora[i]) == pad_of[i])) return false;
+    return true;
+  }
+  void set_padded(const std::vector<Tensor>& p) {
+    TORCH_CHECK_VALUE((int)p.size() == PADS, "LayerPlan: ", (int)PADS, " padded factors expected");
+    pad = p;
+    for (int i = 0; i < 2 * PROJECTIONS; ++i) pad_of[i] = Stamp::of(lora[i]);
+  }
+  void set_stats(const std::vector<Tensor>& s) {
+    bool same = s.size() == stats_in.size();
+    for (size_t i = 0; same && i < s.size(); ++i) same = s[i].unsafeGetTensorImpl() == stats_in[i].unsafeGetTensorImpl() && Stamp::of(s[i]) == stats_of[i];
+    if (same) return;
+    stats_in = s;
+    stats.clear();
+    stats_of.clear();
+    for (const Tensor& t : s) {
+      stats_of.push_back(Stamp::of(t));
+      stats.push_back(t.scalar_type() == at::kLong ? t.contiguous() : vec(t));
+    }
+  }
+};
+
+// order of the statistics
+enum { X_IDX, X_SCALE, XN1_SCALE, Q_SCALE, K_SCALE, V_SCALE, O_SCALE, XM_IDX, XM_SCALE, XN2_SCALE, GATE_SCALE, UP_SCALE, STATS };
+
+struct LayerSaved {
+  MlpForward mlp;
+  Tensor rstd, x_o, x_q, xn_q, q_q, k_q, v_q, xa3, o_q, o_xa64;
+  std::vector<Tensor> map;                      // top-k form: five tensors; pruned form: words, directory, nnz
+  OptTensor cls;
+  int64_t cls_b = 0, cls_h = 0;
+  std::vector<Tensor> stats;
+  RopeTables tables;
+  int64_t B, M, H, nh, d, nkv, q_attn, q_mlp, map_q;    // map_q = 0: pruned form
+  at::ScalarType x_type;
+};
+
+static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p, const Tensor& x_in, const std::vector<Tensor>& stats, const Tensor& cos,
+                                                                    const Tensor& sin, const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv,
+                                                                    int64_t q_attn, int64_t q_mlp, int64_t map_q, int64_t map_k, double threshold,
+                                                                    int64_t capacity, double eps, const Tensor& status) {
+  at::AutoDispatchBelowADInplaceOrView below;
+  TORCH_CHECK_VALUE((int)stats.size() == STATS, "layer_forward: ", (int)STATS, " statistics expected");
+  TORCH_CHECK_VALUE(x_in.dim() == 3, "expected a [B, M, H] input, got shape ", x_in.sizes());
+  require_cuda({&x_in, &p.norm1, &p.lora[0], &status});
+  p.set_stats(stats);
+  const std::vector<Tensor>& st = p.stats;
+  const Tensor x = bf16c(x_in);
+  auto s = std::make_shared<LayerSaved>();
+  s->B = x.size(0); s->M = x.size(1); s->H = x.size(2);
+  s->nh = nh; s->d = d; s->nkv = nkv; s->q_attn = q_attn; s->q_mlp = q_mlp; s->map_q = map_q;
+  s->stats = st;
+  s->x_type = x_in.scalar_type();
+  s->tables = rope_tables(cos, sin, s->M, d);
+  Tensor x_medium;
+  {
+    Tensor a, o2;
+    OptTensor o_codes;
+    std::tie(a, o2, s->rstd, s->x_o, s->x_q, s->xn_q, s->q_q, s->k_q, s->v_q, s->xa3, o_codes, s->cls, s->cls_b, s->cls_h) = attn_forward_map(
+        x, {p.norm1, p.w[PQ].get(), p.w[PK].get(), p.w[PV].get(), p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
+        {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status);
+    if (map_q > 0) {
+      auto [val, col, q, sc, z] = topk_compress(a, map_k, map_q);
+      s->map = {val, col, q, sc, z};
+    } else {
+      auto [words, directory, nnz] = prune_tiled(a, threshold, capacity);
+      s->map = {words, directory, nnz};
+    }
+    a.reset();
+    auto out = attn_forward_out(x, o2, p.w[PO].get(), p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
+    x_medium = out[0]; s->o_q = out[1]; s->o_xa64 = out[2];
+  }
+  s->mlp = mlp_forward(x_medium, {p.norm2, p.w[PGATE].get(), p.w[PUP].get(), p.w[PDOWN].get(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
+                                  p.pad[AGU_T], p.pad[AD_COLS], p.pad[BD_COLS]},
+                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status);
+  Tensor y = std::move(s->mlp.x_out);
+  s->mlp.x_out = Tensor();
+  return {y.to(s->x_type), s};
+}
+
+// -> grad_x and the fourteen LoRA gradients (A, B of q, k, v, o, gate, up, down).  hook: see mlp.mlp_backward
+static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad_y, LayerSaved& s, const pybind11::object& hook, const Tensor& overflow,
+                                          const Tensor& status) {
+  at::AutoDispatchBelowADInplaceOrView below;
+  const std::vector<Tensor>& st = s.stats;
+  const int64_t T = s.B * s.M;
+  const std::vector<int64_t> shape = {s.B, s.M, s.H};
+  require_cuda({&grad_y, &s.rstd});
+  OnDevice on(s.rstd);
+  std::vector<Tensor> out(1 + 2 * PROJECTIONS);
+  auto lora = [&](int proj, const Tensor& a, const Tensor& b) { out[1 + 2 * proj] = a; out[2 + 2 * proj] = b; };
+  auto report = [&](std::initializer_list<std::pair<const char*, int>> which) {
+    if (hook.is_none()) return;
+    pybind11::dict d;
+    for (const auto& [name, proj] : which) {
+      d[(std::string("grad_a") + name).c_str()] = out[1 + 2 * proj];
+      d[(std::string("grad_b") + name).c_str()] = out[2 + 2 * proj];
+    }
+    hook(d);
+  };
+  Tensor g_medium;
+  {
+    const Tensor g = bf16c(grad_y).view({T, s.H});
+    const MlpForward& m = s.mlp;
+    auto r = mlp_backward_lora(g, {p.w[PDOWN].get(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
+                               {m.q1, m.gs, m.q2, m.us, m.gu_xa, m.down_xa64, m.xn_q, st[XN2_SCALE]}, s.q_mlp, status);
+    lora(PGATE, r[5].narrow(0, 0, 16), r[6].select(0, 0));
+    lora(PUP, r[5].narrow(0, 16, 16), r[6].select(0, 1));
+    lora(PDOWN, r[4], r[3]);
+    report({{"g", PGATE}, {"u", PUP}, {"d", PDOWN}});
+    r[0].reset();
+    g_medium = mlp_backward_x(g, r[1], r[2], {p.w[PGATE].get(), p.w[PUP].get(), p.pad[AGU_ROWS], p.norm2},
+                              {m.xm_q, st[XM_SCALE], m.xm_o, st[XM_IDX], m.rstd}, shape, s.q_mlp, status).view({T, s.H});
+  }
+  std::vector<Tensor> grads;
+  {
+    auto r = attn_backward_out(g_medium, p.w[PO].get(), p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
+    lora(PO, r[1], r[0]);
+    const std::vector<int64_t> a_shape = {s.B, s.nh, s.M, s.M};
+    const bool topk = s.map_q > 0;
+    Tensor a = topk ? topk_restore(s.map[0], s.map[1], s.map[2], s.map[3], s.map[4], a_shape, s.map_q, std::nullopt)
+                    : prune_tiled_restore(s.map[0], s.map[1], a_shape, std::nullopt);
+    grads = attn_backward_map(r[2], std::move(a), topk ? s.map : std::vector<Tensor>(), s.map_q,
+                              {s.q_q, st[Q_SCALE], s.xa3.select(0, 0), s.k_q, st[K_SCALE], s.xa3.select(0, 1), s.v_q, st[V_SCALE], s.xa3.select(0, 2)},
+                              {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.tables, s.B, s.M, s.nh, s.d, s.nkv, s.q_attn,
+                              s.cls, s.cls_b, s.cls_h, status);
+    if (!topk)
+      check(hyc_prune_overflow_flag((const int64_t*)data(s.map[2]), s.map[0].numel(), (int*)data(overflow), on.stream), "hyc_prune_overflow_flag");
+  }
+  auto r = attn_backward_lora(grads, {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.xa3, s.xn_q, st[XN1_SCALE], s.q_attn, status);
+  for (int i = 0; i < 3; ++i) lora(PQ + i, r[1].narrow(0, 16 * i, 16), r[2 + i]);
+  report({{"q", PQ}, {"k", PK}, {"v", PV}, {"o", PO}});
+  out[0] = attn_backward_x(g_medium, grads, r[0], {p.w[PQ].get(), p.w[PK].get(), p.w[PV].get(), p.pad[AQKV_ROWS], p.norm1},
+                           {s.x_q, st[X_SCALE], s.x_o, st[X_IDX], s.rstd}, shape, s.q_attn, status).to(s.x_type);
+  return out;
+}
+
 void bind_blocks(pybind11::module_& m) {
   m.def("lora_grad_a", &lora_grad_a);
-  m.def("mlp_forward", &mlp_forward);
+  m.def("mlp_forward", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const OptTensor& bias_d, int64_t q,
+                          double eps, const Tensor& st) {
+    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st);
+    return std::vector<Tensor>{f.x_out, f.rstd, f.xm_o, f.xm_q, f.xn_q, f.q1, f.q2, f.gs, f.us, f.gu_xa, f.down_xa64}; });
   m.def("mlp_backward_lora", &mlp_backward_lora);
   m.def("mlp_backward_x", [](const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
                              std::vector<int64_t> shape, int64_t q, const Tensor& st) { return mlp_backward_x(g, ggu, gm64, w, saved, shape, q, st); });
-  m.def("attn_forward_map", &attn_forward_map);
+  m.def("attn_forward_map", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos, const Tensor& sin,
+                               const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& st) {
+    return attn_forward_map(x, w, stats, rope_tables(cos, sin, x.size(1), d), mask, nh, d, nkv, q, eps, st); });
   m.def("attn_forward_out", &attn_forward_out);
   m.def("attn_backward_out", &attn_backward_out);
-  m.def("attn_backward_map", &attn_backward_map);
+  m.def("attn_backward_map", [](const Tensor& grad_o2, const Tensor& a, const std::vector<Tensor>& topk, int64_t map_q_bit, const std::vector<Tensor>& saved,
+                                const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin, int64_t B, int64_t M, int64_t nh, int64_t d,
+                                int64_t nkv, int64_t q, const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& st) {
+    return attn_backward_map(grad_o2, a, topk, map_q_bit, saved, w, rope_tables(cos, sin, M, d), B, M, nh, d, nkv, q, cls, cls_b, cls_h, st); });
   m.def("attn_backward_lora", &attn_backward_lora);
   m.def("attn_backward_x", [](const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, std::vector<int64_t> shape, int64_t q, const Tensor& st) {
     return attn_backward_x(g, grads, gmq, w, saved, shape, q, st); });
+  pybind11::class_<FrozenWeight>(m, "FrozenWeight")
+      .def(pybind11::init([](const Tensor& w) { FrozenWeight f; f.plain = w; return f; }))
+      .def(pybind11::init([](const Tensor& packed, const Tensor& code, const Tensor& absmax, const OptTensor& code2, const OptTensor& absmax2,
+                             int64_t blocksize2, double offset, int64_t blocksize, std::vector<int64_t> shape) {
+        return FrozenWeight{Tensor(), packed, code, absmax, code2, absmax2, blocksize2, blocksize, offset, std::move(shape)}; }));
+  pybind11::class_<LayerSaved, std::shared_ptr<LayerSaved>>(m, "LayerSaved");
+  pybind11::class_<LayerPlan>(m, "LayerPlan")
+      .def(pybind11::init([](const Tensor& norm1, const Tensor& norm2, const std::vector<FrozenWeight>& w, const std::vector<Tensor>& lora,
+                             const OptTensor& bias_o, const OptTensor& bias_d) {
+        TORCH_CHECK_VALUE(w.size() == PROJECTIONS && lora.size() == 2 * PROJECTIONS, "LayerPlan: seven weights and fourteen LoRA factors expected");
+        auto p = std::make_unique<LayerPlan>();
+        p->norm1 = norm1; p->norm2 = norm2; p->bias_o = bias_o; p->bias_d = bias_d;
+        std::copy(w.begin(), w.end(), p->w);
+        std::copy(lora.begin(), lora.end(), p->lora);
+        return p; }))
+      .def("fresh", &LayerPlan::fresh)
+      .def("set_padded", &LayerPlan::set_padded)
+      .def("forward", &layer_forward)
+      .def("backward", &layer_backward);
 }
 
 }  // namespace hyc_host

@@ -23,10 +23,10 @@ void require_cuda(std::initializer_list<const Tensor*> ts) {
 void check_q(int64_t q) { TORCH_CHECK_VALUE(q == 2 || q == 4 || q == 8, "quantize_bit must be 2, 4 or 8"); }
 
 Tensor scale_vec(const Tensor& s, int64_t n) {
-  Tensor v = s.to(at::kBFloat16).reshape({-1});
+  const Tensor v = vec(s);
   TORCH_CHECK_VALUE(v.numel() == n, "per-channel scale with ", v.numel(), " entries for ", n,
                     " channels (per-tensor scales cannot be quantized with)");
-  return v.contiguous();
+  return v;
 }
 
 // [B, M, N] (or [B, heads, M, d], which becomes [B, M, heads*d]) -> bf16 with one row stride
@@ -327,16 +327,7 @@ Tensor rope(const Tensor& x, const Tensor& cos_in, const Tensor& sin_in, bool ba
   TORCH_CHECK_VALUE(x.dim() == 4, "expected a [batch, seq_len, n_heads, head_dim] tensor");
   OnDevice on(x);
   const int64_t batch = x.size(0), seq = x.size(1), heads = x.size(2), d = x.size(3);
-  Tensor cos = cos_in.squeeze(), sin = sin_in.squeeze();
-  TORCH_CHECK_VALUE(cos.dim() == 2 && sin.sizes() == cos.sizes(), "cos / sin must squeeze to [seq_len, head_dim] tables");
-  if (seq > cos.size(0)) {
-    PyErr_SetString(PyExc_AssertionError, "the rotary tables are shorter than the sequence");
-    throw pybind11::error_already_set();
-  }
-  TORCH_CHECK_VALUE(cos.size(1) >= d / 2, "cos / sin tables are narrower than head_dim / 2");
-  if (cos.scalar_type() != at::kBFloat16 && cos.scalar_type() != at::kFloat) { cos = cos.to(at::kFloat); sin = sin.to(at::kFloat); }
-  sin = sin.to(cos.scalar_type());
-  if (cos.stride(1) != 1 || sin.stride(1) != 1 || sin.stride(0) != cos.stride(0)) { cos = cos.contiguous(); sin = sin.contiguous(); }
+  const auto [cos, sin] = rope_tables(cos_in, sin_in, seq, d);
   const Tensor xc = bf16c(x);
   Tensor out = inplace || xc.data_ptr() != x.data_ptr() ? xc : at::empty_like(xc);
   check(hyc_rope(data(xc), heads * d, data(out), heads * d, data(cos), data(sin), cos.stride(0), cos.scalar_type() == at::kFloat ? 1 : 0,

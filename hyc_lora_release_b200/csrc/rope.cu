@@ -14,25 +14,32 @@
 // store rounds to bf16.  No multiply-add contraction in either form.
 // One thread owns eight adjacent j of one head: two 16-byte loads and two 16-byte stores of x, 16 (bf16
 // tables) or 2 x 32 (fp32 tables) bytes of each table; the tables stay in L1/L2 (seq_len * head_dim values).
+// Bound by memory.  Blocks are laid out over (octets of a row, rows), so that no index needs a 64-bit division, and a
+// launch takes up to two tensors with the same rows (q and k of a layer).
 #include "hyc_common.cuh"
 
 namespace hyc {
 
+struct RopeTensor { const __nv_bfloat16* x; __nv_bfloat16* out; int64_t ldx, ldo; int heads; };
+
 template <bool TABLE_F32>
 __global__ void __launch_bounds__(256)
-rope_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bfloat16* __restrict__ out, int64_t ldo,
-            const void* __restrict__ cos_t, const void* __restrict__ sin_t, int64_t ld_table,
-            int64_t rows, int seq_len, int n_heads, int head_dim, float sin_sign) {
+rope_kernel(const RopeTensor t0, const RopeTensor t1, const void* __restrict__ cos_t, const void* __restrict__ sin_t, int64_t ld_table,
+            int64_t rows, int seq_len, int head_dim, float sin_sign) {
   const int half = head_dim >> 1;
   const int per_head = half >> 3;                       // octets of j per head
-  const int per_row = n_heads * per_head;
-  const int64_t total = rows * per_row;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = i / per_row;
-    const int w = (int)(i - row * per_row);
-    const int head = w / per_head, j0 = (w - head * per_head) << 3;
-    const int pos = (int)(row % seq_len);
-    const __nv_bfloat16* xp = x + row * ldx + (int64_t)head * head_dim + j0;
+  const int w = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  int head = w / per_head;
+  const int j0 = (w - head * per_head) << 3;
+  if (head >= t0.heads + t1.heads) return;
+  const bool second = head >= t0.heads;
+  if (second) head -= t0.heads;
+  const int64_t ldx = second ? t1.ldx : t0.ldx, ldo = second ? t1.ldo : t0.ldo;
+  const __nv_bfloat16* __restrict__ x = (second ? t1.x : t0.x) + (int64_t)head * head_dim + j0;
+  __nv_bfloat16* __restrict__ out = (second ? t1.out : t0.out) + (int64_t)head * head_dim + j0;
+  for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
+    const int pos = (int)((uint32_t)row % (uint32_t)seq_len);      // rows < 2^32: checked by the caller
+    const __nv_bfloat16* xp = x + row * ldx;
     const uint4 a = *reinterpret_cast<const uint4*>(xp);
     const uint4 b = *reinterpret_cast<const uint4*>(xp + half);
     const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
@@ -74,7 +81,7 @@ rope_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bfloat16* __r
         o2[e] = *reinterpret_cast<const uint32_t*>(&r2);
       }
     }
-    __nv_bfloat16* op = out + row * ldo + (int64_t)head * head_dim + j0;
+    __nv_bfloat16* op = out + row * ldo;
     *reinterpret_cast<uint4*>(op) = make_uint4(o1[0], o1[1], o1[2], o1[3]);
     *reinterpret_cast<uint4*>(op + half) = make_uint4(o2[0], o2[1], o2[2], o2[3]);
   }
@@ -84,26 +91,45 @@ rope_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bfloat16* __r
 
 using namespace hyc;
 
+static int launch_rope(const RopeTensor& t0, const RopeTensor& t1, const void* cos_t, const void* sin_t, int64_t ld_table, int table_is_f32,
+                       int64_t rows, int seq_len, int head_dim, int backward, void* stream) {
+  const int64_t per_row = (int64_t)(t0.heads + t1.heads) * (head_dim / 16), bx = (per_row + 255) / 256;
+  // one resident wave of blocks of 256 threads, each walking down the rows
+  int64_t by = (int64_t)num_sms() * 8 / bx;
+  by = by < 1 ? 1 : (by > rows ? rows : by);
+  if (by > 65535) by = 65535;
+  const dim3 grid((unsigned)bx, (unsigned)by);
+  const float sgn = backward ? -1.f : 1.f;
+  if (table_is_f32)
+    rope_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(t0, t1, cos_t, sin_t, ld_table, rows, seq_len, head_dim, sgn);
+  else
+    rope_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(t0, t1, cos_t, sin_t, ld_table, rows, seq_len, head_dim, sgn);
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
+}
+
 extern "C" HYC_API int hyc_rope(const void* x, int64_t ldx, void* out, int64_t ldo, const void* cos_t, const void* sin_t,
                                 int64_t ld_table, int table_is_f32, int64_t rows, int seq_len, int n_heads, int head_dim,
                                 int backward, void* stream) {
   if (!x || !out || !cos_t || !sin_t) return HYC_ERR_NULL;
-  if (rows < 0 || seq_len < 1 || n_heads < 1 || head_dim < 16 || (head_dim & 15) != 0) return HYC_ERR_SHAPE;
+  if (rows < 0 || rows > 0xffffffffll || seq_len < 1 || n_heads < 1 || head_dim < 16 || (head_dim & 15) != 0) return HYC_ERR_SHAPE;
   if (ldx < (int64_t)n_heads * head_dim || ldo < (int64_t)n_heads * head_dim || ld_table < head_dim / 2) return HYC_ERR_SHAPE;
   if ((ldx & 7) != 0 || (ldo & 7) != 0 || (ld_table & (table_is_f32 ? 3 : 7)) != 0) return HYC_ERR_ALIGN;
   if (!aligned(x, 16) || !aligned(out, 16) || !aligned(cos_t, 16) || !aligned(sin_t, 16)) return HYC_ERR_ALIGN;
   if (rows == 0) return HYC_OK;
-  const int64_t total = rows * n_heads * (head_dim / 16);
-  int64_t blocks = (total + 255) / 256;
-  const int64_t cap = (int64_t)num_sms() * 8;
-  if (blocks > cap) blocks = cap;
-  const float sgn = backward ? -1.f : 1.f;
-  if (table_is_f32)
-    rope_kernel<true><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)out, ldo, cos_t, sin_t,
-                                                                    ld_table, rows, seq_len, n_heads, head_dim, sgn);
-  else
-    rope_kernel<false><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)out, ldo, cos_t, sin_t,
-                                                                     ld_table, rows, seq_len, n_heads, head_dim, sgn);
-  HYC_CHECK_LAUNCH();
-  return HYC_OK;
+  return launch_rope({(const __nv_bfloat16*)x, (__nv_bfloat16*)out, ldx, ldo, n_heads}, {nullptr, nullptr, 0, 0, 0}, cos_t, sin_t, ld_table,
+                     table_is_f32, rows, seq_len, head_dim, backward, stream);
+}
+
+extern "C" HYC_API int hyc_rope_pair(void* x0, int n_heads0, void* x1, int n_heads1, const void* cos_t, const void* sin_t, int64_t ld_table,
+                                     int table_is_f32, int64_t rows, int seq_len, int head_dim, int backward, void* stream) {
+  if (!x0 || !x1 || !cos_t || !sin_t) return HYC_ERR_NULL;
+  if (rows < 0 || rows > 0xffffffffll || seq_len < 1 || n_heads0 < 1 || n_heads1 < 1 || head_dim < 16 || (head_dim & 15) != 0 ||
+      ld_table < head_dim / 2) return HYC_ERR_SHAPE;
+  if ((ld_table & (table_is_f32 ? 3 : 7)) != 0 || !aligned(x0, 16) || !aligned(x1, 16) || !aligned(cos_t, 16) || !aligned(sin_t, 16))
+    return HYC_ERR_ALIGN;
+  if (rows == 0) return HYC_OK;
+  const int64_t ld0 = (int64_t)n_heads0 * head_dim, ld1 = (int64_t)n_heads1 * head_dim;
+  return launch_rope({(const __nv_bfloat16*)x0, (__nv_bfloat16*)x0, ld0, ld0, n_heads0}, {(const __nv_bfloat16*)x1, (__nv_bfloat16*)x1, ld1, ld1, n_heads1},
+                     cos_t, sin_t, ld_table, table_is_f32, rows, seq_len, head_dim, backward, stream);
 }

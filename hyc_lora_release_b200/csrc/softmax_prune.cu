@@ -611,6 +611,17 @@ extern "C" HYC_API int hyc_softmax_prune_tiled_restore(const uint32_t* words, in
   return HYC_OK;
 }
 
+static __global__ void prune_overflow_kernel(const int64_t* nnz, int64_t capacity, int* flag) {
+  if (*nnz > capacity) *flag += 1;
+}
+
+extern "C" HYC_API int hyc_prune_overflow_flag(const int64_t* nnz, int64_t capacity, int* flag, void* stream) {
+  if (!nnz || !flag) return HYC_ERR_NULL;
+  prune_overflow_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(nnz, capacity, flag);
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Variant for callers that must not allocate device memory when they call: a training loop whose
 // HBM is handed out up front by a fixed memory plan, or a host framework that forbids allocation

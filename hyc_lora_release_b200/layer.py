@@ -22,9 +22,11 @@ host has to read back.
 """
 import torch
 
+from ._lib import host
 from .attention import AttnState, AttnWeights, attention_backward, attention_forward
 from . import nf4
 from .mlp import MLPState, MLPWeights, _status_tensor, check_status, mlp_backward, mlp_forward
+from .operators.compress_function import static_capacity
 
 BF16 = torch.bfloat16
 
@@ -88,14 +90,33 @@ class FusedLayerFunction(torch.autograd.Function):
         # fixed-capacity prune buffers: entries beyond the capacity were dropped; the flag stays on the device
         if hasattr(saved_map, "nnz") and hasattr(saved_map, "capacity"):
             module._overflow.add_((saved_map.nnz > saved_map.capacity).to(torch.int32))
-        module._steps_since_check += 1
-        every = 1 if module.check_kernel_status else module.check_every
-        if every and module._steps_since_check >= every and not torch.cuda.is_current_stream_capturing():
-            module.raise_on_device_errors()
+        module._after_backward()
         grads = [ga['grad_aq'], ga['grad_bq'], ga['grad_ak'], ga['grad_bk'], ga['grad_av'], ga['grad_bv'],
                  ga['grad_ao'], ga['grad_bo'], gm['grad_ag'], gm['grad_bg'], gm['grad_au'], gm['grad_bu'],
                  gm['grad_ad'], gm['grad_bd']]
         return (ga['grad_x'].to(x_dtype),) + (None,) * 9 + tuple(grads)
+
+
+class SteadyLayerFunction(torch.autograd.Function):
+    """The calibrated layer through the native host path: one call forward, one backward.  Arguments as in
+    ``FusedLayerFunction`` with the layer's plan in place of the two weight records."""
+
+    @staticmethod
+    def forward(ctx, x, module, plan, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, *lora):
+        st = module._status_for(x.device)
+        y, saved = module._steady_forward(plan, x, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, st)
+        ctx.hyc = (saved, plan, st, module)
+        return y
+
+    @staticmethod
+    def backward(ctx, grad_y):
+        saved, plan, st, module = ctx.hyc
+        ctx.hyc = None
+        if not plan.fresh():
+            module._refresh_plan(plan)
+        grads = plan.backward(grad_y, saved, module.on_lora_grads, module._overflow, st)
+        module._after_backward()
+        return (grads[0], None, None, None, None, None, None, None, None, *grads[1:])
 
 
 def _frozen(base, name):
@@ -131,11 +152,25 @@ def _bias(base, name):
     return b
 
 
+_MISSING = object()
+
+
+def _entry(mod, table, name, default=_MISSING):
+    """``getattr(mod, name)`` past the slow look-up of a Module (a layer call makes three dozen of them)."""
+    try:
+        return mod.__dict__[table][name]
+    except (AttributeError, KeyError):
+        return getattr(mod, name) if default is _MISSING else getattr(mod, name, default)
+
+
+def _adapter_weight(mod):
+    return _entry(_entry(mod, "_modules", "default", mod), "_parameters", "weight")
+
+
 def _adapter(mod, name, rank_dim):
     """``lora_A`` / ``lora_B`` module dictionary of a PEFT layer (``.default``) or a bare ``nn.Linear``.
     The kernels are built for bf16 adapters of rank 16."""
-    inner = getattr(mod, "default", mod)
-    w = inner.weight
+    w = _adapter_weight(mod)
     if w.dtype != BF16:
         raise NotImplementedError("%s: LoRA adapters must be bf16 (got %s)" % (name, w.dtype))
     if w.dim() != 2 or w.shape[rank_dim] != 16:
@@ -165,12 +200,19 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
         self._overflow = None
         self._steps_since_check = 0
         self._weights = None
+        self._plan = None
 
     def _status_for(self, device):
         if self._status is None or self._status.device != device:
             self._status = torch.zeros(1, dtype=torch.int32, device=device)
             self._overflow = torch.zeros(1, dtype=torch.int32, device=device)
         return self._status
+
+    def _after_backward(self):
+        self._steps_since_check += 1
+        every = 1 if self.check_kernel_status else self.check_every
+        if every and self._steps_since_check >= every and not torch.cuda.is_current_stream_capturing():
+            self.raise_on_device_errors()
 
     def raise_on_device_errors(self):
         """Read the two persistent device words (synchronises) and raise if a tensor-core kernel gave up on a bounded
@@ -221,17 +263,20 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
 
     def _bind(self, norm_w1, norm_w2, mods):
         """Weight records for the two halves, rebuilt only when a tensor was replaced."""
+        key = [id(norm_w1), id(norm_w2)]
+        for base, la, lb in mods.values():            # in the order q, k, v, o, gate, up, down
+            w = _entry(base, "_parameters", "weight")
+            # (a 4-bit weight is wrapped once: the parameter and its quant state are what identify it)
+            key += (id(w), id(w.__dict__.get("quant_state") if type(w) is torch.nn.Parameter else getattr(w, "quant_state", None)),
+                    id(_adapter_weight(la)), id(_adapter_weight(lb)), id(_entry(base, "_parameters", "bias", None)))
+        if self._weights is not None and self._weights[0] == key and (self._plan is None or self._plan.fresh()):
+            return self._weights[1:]
         tensors = [norm_w1, norm_w2]
-        idents = [id(norm_w1), id(norm_w2)]
         biases = {}
-        for name in ("q", "k", "v", "o", "gate", "up", "down"):
-            base, la, lb = mods[name]
+        for name, (base, la, lb) in mods.items():
             tensors += [_frozen(base, name + "_proj"), _adapter(la, name + "_proj lora_A", 0),
                         _adapter(lb, name + "_proj lora_B", 1)]
-            # (a 4-bit weight is wrapped anew on every call: the parameter it wraps is what identifies it)
-            idents += [id(base.weight), id(tensors[-2]), id(tensors[-1])]
             biases[name] = _bias(base, name + "_proj")
-        key = tuple(idents) + tuple(id(b) for b in biases.values())
         if self._weights is None or self._weights[0] != key:
             (n1, n2, wq, aq, bq, wk, ak, bk, wv, av, bv, wo, ao, bo, wg, ag, bg, wu, au, bu, wd, ad, bd) = tensors
             aw = AttnWeights(norm_w=n1, wq=wq, wk=wk, wv=wv, wo=wo, aq=aq, bq=bq, ak=ak, bk=bk, av=av, bv=bv, ao=ao, bo=bo,
@@ -239,7 +284,44 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
             mw = MLPWeights(norm_w=n2, wg=wg, wu=wu, wd=wd, ag=ag, bg=bg, au=au, bu=bu, ad=ad, bd=bd, bias_d=biases["down"])
             lora = (aq, bq, ak, bk, av, bv, ao, bo, ag, bg, au, bu, ad, bd)
             self._weights = (key, aw, mw, lora)
+            # q/k/v projections with a bias run as separate launches
+            self._plan = None if any(biases[n] is not None for n in ("q", "k", "v")) else host.LayerPlan(
+                n1, n2, [w.native() if isinstance(w, nf4.QuantizedWeight) else host.FrozenWeight(w) for w in (wq, wk, wv, wo, wg, wu, wd)],
+                list(lora), biases["o"], biases["down"])
+        if self._plan is not None:
+            self._refresh_plan(self._plan)
         return self._weights[1:]
+
+    def _refresh_plan(self, plan):
+        """The LoRA factors in the layouts of the kernels, rebuilt when one changed."""
+        a, m = self._weights[1].padded(), self._weights[2].padded()
+        plan.set_padded([a["aqkv_t"], a["aqkv_rows"], a["ao_cols"], a["ao_rows"], a["bo_cols"], m["agu_t"], m["agu_rows"], m["ad_rows"],
+                         m["ad_cols"], m["bd_cols"]])
+
+    def _steady(self):
+        """True when a call is one of the fixed launch sequence: statistics calibrated and nothing wanted of the steps between."""
+        a, m = self.attn_state, self.mlp_state
+        return (self._plan is not None and a.iteration >= a.iteration_threshold and m.iteration >= m.iteration_threshold
+                and not (self.track_saved_bytes or self.keep_saved or a.fuse_softmax_with_save) and a.map_mode in ("topk", "prune"))
+
+    def _steady_forward(self, plan, x, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, status):
+        a, m = self.attn_state, self.mlp_state
+        av, mv = a.static_value, m.static_value
+        stats = [av['x']['outlier_channel_index'], av['x']['scale'], av['x_norm_1']['scale'], av['q']['scale'], av['k']['scale'],
+                 av['v']['scale'], av['o']['scale'], mv['x_medium']['outlier_channel_index'], mv['x_medium']['scale'],
+                 mv['x_norm_2']['scale'], mv['gate']['scale'], mv['up']['scale']]
+        if a.map_mode == "topk":
+            save = (a.map_q_bit, int(x.shape[1] * a.softmax_outlier_ratio), 0.0, 0)
+        else:
+            if a.threshold_host is None:
+                a.threshold_host = float(av['a']['outlier'])
+            entries = x.shape[0] * num_heads * x.shape[1] ** 2
+            save = (0, 0, a.threshold_host, static_capacity(entries, a.softmax_outlier_ratio, a.prune_capacity_margin))
+        out = plan.forward(x, stats, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, a.q_bit, m.q_bit, *save,
+                           1e-5, status)
+        a.iteration += 1
+        m.iteration += 1
+        return out
 
     def named_lora_weights(self):
         """{"grad_aq": q lora_A weight, "grad_bq": q lora_B weight, ...}: the 14 adapter weights of the last forward
@@ -264,6 +346,9 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
                     up=(up_proj_base, up_proj_lora_a, up_proj_lora_b),
                     down=(down_proj_base, down_proj_lora_a, down_proj_lora_b))
         aw, mw, lora = self._bind(norm_weight_1, norm_weight_2, mods)
+        if self._steady():
+            return SteadyLayerFunction.apply(input, self, self._plan, cos, sin, attention_mask, num_heads, head_dim,
+                                             num_key_value_heads, *lora)
         return FusedLayerFunction.apply(input, self, aw, mw, cos, sin, attention_mask, num_heads, head_dim,
                                         num_key_value_heads, *lora)
 

@@ -78,6 +78,13 @@ class QuantizedWeight:
         else:
             self.absmax = qs.absmax.to(device=dev, dtype=torch.float32).contiguous()
 
+    def native(self):
+        """The same record for the native host path of the layer."""
+        if self.nested:
+            return host.FrozenWeight(self.packed, self.code, self.absmax, self.code2, self.absmax2, self.blocksize2, self.offset,
+                                     self.blocksize, self.shape)
+        return host.FrozenWeight(self.packed, self.code, self.absmax, None, None, 1, 0.0, self.blocksize, self.shape)
+
     def dequantize(self):
         if self.nested:
             return host.dequant_nf4(self.packed, self.code, self.absmax, self.code2, self.absmax2, self.blocksize2, self.offset,

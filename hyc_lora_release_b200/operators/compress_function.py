@@ -282,6 +282,11 @@ class TiledPrunedMap:
         return idx[order], val[order]
 
 
+def static_capacity(numel, ratio, margin=1.5):
+    """Entries that the buffers of a fixed-capacity save hold for a threshold calibrated to keep ``ratio`` of ``numel``."""
+    return min(int(numel * ratio * margin) + 1024, numel)
+
+
 def compression_softmax_static(x: torch.Tensor, outlier, capacity=None, margin=1.5, ratio=None, ordered=False):
     """``compression_softmax`` (compress_function.py:309-313) without the device-to-host read of the count: the
     kept entries go into buffers of a fixed ``capacity`` (default: ``margin`` x ``ratio`` x numel + 1024, for a
@@ -300,7 +305,7 @@ def compression_softmax_static(x: torch.Tensor, outlier, capacity=None, margin=1
     if capacity is None:
         if ratio is None:
             raise ValueError("give `capacity` or the calibrated `ratio`")
-        capacity = int(numel * ratio * margin) + 1024
+        capacity = static_capacity(numel, ratio, margin)
     capacity = min(int(capacity), numel)
     if not ordered:
         return TiledPrunedMap(*host.prune_tiled(x, float(outlier), capacity), x.shape)

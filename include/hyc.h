@@ -140,6 +140,9 @@ int hyc_softmax_prune_tiled(const void* a, int64_t numel, float threshold,
 int hyc_softmax_prune_tiled_restore(const uint32_t* words, int64_t capacity, const void* directory,
                                     void* a_out, int64_t numel, void* stream);
 
+/* *flag += 1 if *nnz > capacity (entries of a fixed-capacity save were dropped). */
+int hyc_prune_overflow_flag(const int64_t* nnz, int64_t capacity, int* flag, void* stream);
+
 /* No counterpart in the reference.  The same threshold prune for callers that must not allocate
  * device memory at call time (a fixed up-front memory plan, or a host that forbids allocation inside
  * operator callbacks) and so have no workspace to pass: the tile offsets live in a 512 KiB array built
@@ -212,6 +215,13 @@ int hyc_fused_lora_silu_hadamard_bwd(const void* xa1, const void* bt1, const voi
 int hyc_dequant_lora_add(const void* q, const void* scale, const void* xa, const void* bt,
                          void* y, int64_t rows, int N, int R, int q_bit, void* stream);
 
+/* hyc_dequant_lora_add of the q, k and v projections in one launch, q and k followed by the rotary embedding (bf16 in between,
+ * as the separate steps have it): what the backward pass rebuilds from the saved codes.  n[0] = heads*128, n[1] = n[2] =
+ * kv_heads*128; tables as in hyc_rope.  q_bit is that of the codes. */
+int hyc_rebuild_qkv(const void* const* q, const void* const* scale, const void* const* xa, const void* const* bt, void* const* y,
+                    const int* n, const void* cos_table, const void* sin_table, int64_t ld_table, int table_is_f32,
+                    int64_t rows, int seq_len, int q_bit, void* stream);
+
 /* ---- producers / consumers of the saved tensors ----------------------------------------- */
 
 /* rmsnorm_forward / rmsnorm_backward (operators/rmsnorm_kernels.py:10-54, 58-113, wrappers
@@ -249,6 +259,10 @@ int hyc_rmsnorm_bwd_packed(const void* dy, const void* qx, const void* scale_x, 
 int hyc_rope(const void* x, int64_t ldx, void* out, int64_t ldo, const void* cos_table, const void* sin_table,
              int64_t ld_table, int table_is_f32, int64_t rows, int seq_len, int n_heads, int head_dim,
              int backward, void* stream);
+/* The same in place on two contiguous tensors with the same rows ([rows, n_heads0*head_dim] and [rows, n_heads1*head_dim],
+ * a layer's q and k) in one launch. */
+int hyc_rope_pair(void* x0, int n_heads0, void* x1, int n_heads1, const void* cos_table, const void* sin_table, int64_t ld_table,
+                  int table_is_f32, int64_t rows, int seq_len, int head_dim, int backward, void* stream);
 /* Attention probabilities from raw scores in one pass (fused_llama_layer_intra_inter_full_fuse.py:150-160:
  * `s = q @ k^T / sqrt(d)`, `s + attention_mask`, `softmax(s, -1, dtype=bf16)`): a = softmax(bf16(bf16(scores * scale)
  * + mask)) per row, fp32 inside, bf16 result.  scores, a [rows, S] bf16 (a may alias scores), rows = batch * heads * M;
