@@ -65,7 +65,10 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
   uint64_t* empty = bars + MAX_STAGES;             // [STAGES]
   uint64_t* tmem_full = bars + 2 * MAX_STAGES;     // [2]
   uint64_t* tmem_empty = bars + 2 * MAX_STAGES + 2;  // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 4);
+  uint64_t* main_read = bars + 2 * MAX_STAGES + 4;   // [2] pair form: the main branch of the tile (GRADDOWN: also the first half of
+                                                     // the LoRA terms) is in registers, its columns may be overwritten
+  uint64_t* lora_full = bars + 2 * MAX_STAGES + 6;   // [2] pair form: LoRA terms are in those columns
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -77,6 +80,11 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
   const int num_tiles = tiles_m * (p.n_wide + (p.N / TILE_N - p.n_wide) * 2);
   const int kb1 = p.K1 / BK, kb2 = (p.K1 + p.K2) / BK, kb3 = (p.K1 + p.K2 + p.K3) / BK, kb_total = kb3 + p.K4 / BK;
 
+  // pair form: rounds of LoRA products per tile (GRADDOWN has two terms per column and room for one: two rounds)
+  const int lora_rounds = !PAIR ? 0 : (EPI == EPI_GATEUP ? 1 : (EPI == EPI_GRADDOWN ? (p.lpre1 == nullptr ? 2 : 0) : (p.l0.bt != nullptr ? 1 : 0)));
+  LoraStage lst;
+  lst.a1 = smem + PIPE_BYTES + 16384; lst.a2 = lst.a1 + 4096; lst.b1 = lst.a1 + 8192; lst.b2 = lst.a1 + 12288;
+
   if (warp == 0 && elect_one()) {
     for (int i = 0; i < 3; ++i) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.a[i])) : "memory");
@@ -87,7 +95,10 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
     // full / tmem_empty are used in the leader only: the loads of both CTAs and the epilogue warps of both CTAs
     // arrive there; empty / tmem_full exist in both CTAs and are signalled together by the leader's commits
     for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], (PAIR ? 2 : 1) * EPI_WARPS); }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], (PAIR ? 2 : 1) * EPI_WARPS);
+      mbar_init(&main_read[b], 2 * EPI_WARPS); mbar_init(&lora_full[b], 1);
+    }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -178,6 +189,37 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
+      // LoRA products of the tile before: due as soon as the epilogue has taken its main branch out, so between the k-blocks
+      // of the present tile
+      int due = 0, due_buf = 0, due_cols = 0;
+      uint32_t due_parity = 0u;             // one bit per accumulator
+      auto lora_products = [&](bool wait) {
+        while (due > 0) {
+          if (wait) {
+            if (!mbar_wait_warp(&main_read[due_buf], (due_parity >> due_buf) & 1u, abort_flag)) {
+              if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_MMA); }
+              return false;
+            }
+          } else if (!__all_sync(0xffffffffu, mbar_test(&main_read[due_buf], (due_parity >> due_buf) & 1u))) {
+            return true;
+          }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t d = tmem_base + (uint32_t)(due_buf * BN);
+            // columns of one product; GRADDOWN takes a quarter of the tile's columns from each CTA's operand per round
+            const int n = EPI == EPI_GRADDOWN ? due_cols / 2 : due_cols;
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TILE_M >> 4) << 24) | ((uint32_t)(n >> 3) << 17);
+            const uint32_t b_off = EPI == EPI_GRADDOWN && due == 1 ? k16_offset(due_cols / 4, 0) : 0u;
+            tc_mma<PAIR>(d, make_desc_k16(smem_u32(lst.a1)), make_desc_k16(smem_u32(lst.b1) + b_off), idesc, 0u);
+            if (EPI != EPI_STORE) tc_mma<PAIR>(d + (uint32_t)n, make_desc_k16(smem_u32(lst.a2)), make_desc_k16(smem_u32(lst.b2) + b_off), idesc, 0u);
+            tc_commit<PAIR>(&lora_full[due_buf]);
+          }
+          __syncwarp();
+          due_parity ^= 1u << due_buf;
+          --due;
+        }
+        return true;
+      };
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++it) {
         const uint32_t idesc = tile / tiles_m < p.n_wide ? idesc_wide : idesc_narrow;
         const int buf = it & 1;
@@ -213,11 +255,18 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
           }
           __syncwarp();
           if (++stage == stages) { stage = 0; phase ^= 1u; }
+          if (PAIR && due > 0) lora_products(false);
         }
         if (ok && elect_one()) tc_commit<PAIR>(&tmem_full[buf]);
         __syncwarp();
+        if (PAIR) {
+          // what is left of the tile before: its accumulator is the next one to be written
+          if (ok && !lora_products(true)) ok = false;
+          due = lora_rounds; due_buf = buf; due_cols = tile / tiles_m < p.n_wide ? TILE_N : TILE_N / 2;
+        }
         TC_STAMP(1, it, 2);
       }
+      if (PAIR && ok) lora_products(true);
     }
   } else {
     // ------------------------------------------------ epilogue warps
@@ -233,6 +282,217 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
     const uint32_t tmem_empty_leader[2] = {PAIR ? map_to_cta(&tmem_empty[0], 0) : smem_u32(&tmem_empty[0]),
                                            PAIR ? map_to_cta(&tmem_empty[1], 0) : smem_u32(&tmem_empty[1])};
     bool fine = true;                    // false: a wait gave up; the barriers below are still kept
+    if constexpr (PAIR) {
+      uint32_t* R = reinterpret_cast<uint32_t*>(epi_b) + (warp - 2) * 512;      // this warp's tile
+      const uint32_t main_read_leader = map_to_cta(&main_read[0], 0);
+      uint32_t lora_parity = 0u;           // one bit per accumulator
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (fine && !mbar_wait(bar, parity, abort_flag)) {
+          if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_EPILOGUE); }
+          fine = false;
+        }
+        fine = __all_sync(0xffffffffu, fine);
+        tc_fence_after();
+      };
+      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
+        const int m0 = (tile % tiles_m) * TILE_M + (int)rank * BM, ct = tile / tiles_m;
+        const bool wide = ct < p.n_wide;
+        const int n0 = column_tile(p.n_wide, TILE_N, ct), cols = wide ? TILE_N : TILE_N / 2;
+        const int buf = it & 1;
+        const int64_t row0 = (int64_t)m0 + quad * 32, row = row0 + lane;
+        const bool valid = row < p.M;
+        const int cb0 = cols / 2 * chalf, blocks = cols / 64;                   // this warp's columns of the tile, in blocks of 32
+        const StoreView sv = store_view(p, n0);
+        // ---- constants and LoRA operands of the tile (the readers of the previous ones are done: barrier at the end)
+        if (EPI == EPI_STORE) {
+          if (sv.q != nullptr && et < cols) sGV[et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(sv.s[sv.n0 + et])));
+          if (lora_rounds) {
+            stage_lora_a(lst.a1, sv.l0.xa, m0, p.M, et);
+            stage_lora_b(lst.b1, sv.l0, sv.n0 + (int)rank * (cols / 2), cols / 2, et);
+          }
+        } else if (EPI == EPI_GATEUP) {
+          if (et < cols) {
+            sGV[et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(p.s1[n0 + et])));
+            sGV[BN / 2 + et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(p.s2[n0 + et])));
+          }
+        } else if (et < cols) {      // the scales stay bf16: column pairs are read as one packed word
+          sGS[et] = p.s1[n0 + et];
+          sGS[BN + et] = p.s2[n0 + et];
+        }
+        if (EPI != EPI_STORE && lora_rounds) {
+          const LoraTerm &la = EPI == EPI_GATEUP ? p.l0 : p.l1, &lb = EPI == EPI_GATEUP ? p.l1 : p.l2;
+          stage_lora_a(lst.a1, la.xa, m0, p.M, et);
+          stage_lora_a(lst.a2, lb.xa, m0, p.M, et);
+          stage_lora_b(lst.b1, la, n0 + (int)rank * (cols / 2), cols / 2, et);
+          stage_lora_b(lst.b2, lb, n0 + (int)rank * (cols / 2), cols / 2, et);
+        }
+        if (lora_rounds) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        uint4 res[4];                        // STORE: the residual of the next block
+        GdCodes<QBIT> codes;                 // GRADDOWN: codes of the next block
+        if (EPI == EPI_STORE && sv.residual != nullptr) tile_fetch(sv.residual, row0, p.M, sv.ld, (int64_t)sv.n0 + cb0, lane, res);
+        if (EPI == EPI_GRADDOWN) gd_codes<QBIT>(p, row, (int64_t)n0 + cb0, codes);
+        epi_bar_sync();
+        wait(&tmem_full[buf], (uint32_t)(it >> 1) & 1u);
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
+        auto columns_read = [&]() {          // what this warp needed of the accumulator is in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(main_read_leader + 8u * (uint32_t)buf);
+        };
+        auto lora_wait = [&]() {
+          wait(&lora_full[buf], (lora_parity >> buf) & 1u);
+          lora_parity ^= 1u << buf;
+        };
+        if (fine) {
+          if constexpr (EPI == EPI_GATEUP) {
+            uint32_t xg[2][16], xu[2][16];
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+              if (b < blocks) {
+                tc_ld_pairs(t_lane + (uint32_t)(cb0 + 32 * b), xg[b]);
+                tc_ld_pairs(t_lane + (uint32_t)(cols + cb0 + 32 * b), xu[b]);
+              }
+            columns_read();
+            // the codes while the LoRA products wait their turn on the tensor pipe
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+              if (b < blocks) {
+                const int64_t n = (int64_t)n0 + cb0 + 32 * b;
+                uint32_t w1[BlockGeo<QBIT>::NW], w2[BlockGeo<QBIT>::NW];
+                pack_codes<QBIT>(xg[b], sGV + cb0 + 32 * b, w1);
+                pack_codes<QBIT>(xu[b], sGV + BN / 2 + cb0 + 32 * b, w2);
+                if (valid) {
+                  store_block_words<QBIT>(p.q1 + (row * p.N + n) * QBIT / 8, w1);
+                  store_block_words<QBIT>(p.q2 + (row * p.N + n) * QBIT / 8, w2);
+                  if (p.dbg1 != nullptr) { store_pairs(xg[b], p.dbg1 + row * p.N + n); store_pairs(xu[b], p.dbg2 + row * p.N + n); }
+                }
+              }
+            lora_wait();
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+              if (b < blocks) {
+                uint32_t l1[16], l2[16];
+                tc_ld_pairs(t_lane + (uint32_t)(cb0 + 32 * b), l1);
+                tc_ld_pairs(t_lane + (uint32_t)(cols + cb0 + 32 * b), l2);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  const uint32_t y1 = add2(xg[b][i], l1[i]);
+                  l1[i] = mul2(mul2(y1, sigmoid2(y1)), add2(xu[b][i], l2[i]));
+                }
+                flush_pairs(l1, R, p.out0, row0, p.M, p.N, (int64_t)n0 + cb0 + 32 * b, lane);
+              }
+          } else if constexpr (EPI == EPI_GRADDOWN) {
+            uint32_t gd[4][16];
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+              if (b < blocks) tc_ld_pairs(t_lane + (uint32_t)(cb0 + 32 * b), gd[b]);
+            if (lora_rounds) columns_read();
+            // round r: blocks r * blocks / 2 ..; the first half of the tile's columns hold the gate terms of both column halves, the
+            // second half the up terms
+            const int per = blocks / 2;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+              if (b < blocks) {
+                const int64_t n = (int64_t)n0 + cb0 + 32 * b;
+                const GdCodes<QBIT> cur = codes;
+                if (b + 1 < blocks) gd_codes<QBIT>(p, row, n + 32, codes);
+                uint32_t t1[16], t2[16], o[16];
+                if (lora_rounds) {
+                  if (b == 0 || b == per) lora_wait();
+                  const uint32_t at = t_lane + (uint32_t)(chalf * (cols / 4) + 32 * (b < per ? b : b - per));
+                  tc_ld_pairs(at, t1);
+                  tc_ld_pairs(at + (uint32_t)(cols / 2), t2);
+                  if (b == per - 1) columns_read();
+                } else {
+#pragma unroll
+                  for (int c8 = 0; c8 < 4; ++c8) {      // the terms of a launch that prepared them
+                    uint4 a = make_uint4(0u, 0u, 0u, 0u), c = a;
+                    if (valid) {
+                      a = *reinterpret_cast<const uint4*>(p.lpre1 + row * p.ld_pre + n + 8 * c8);
+                      c = *reinterpret_cast<const uint4*>(p.lpre2 + row * p.ld_pre + n + 8 * c8);
+                    }
+                    t1[4 * c8] = a.x; t1[4 * c8 + 1] = a.y; t1[4 * c8 + 2] = a.z; t1[4 * c8 + 3] = a.w;
+                    t2[4 * c8] = c.x; t2[4 * c8 + 1] = c.y; t2[4 * c8 + 2] = c.z; t2[4 * c8 + 3] = c.w;
+                  }
+                }
+                const uint32_t* sS1 = reinterpret_cast<const uint32_t*>(sGS) + (cb0 + 32 * b) / 2;
+                const uint32_t* sS2 = reinterpret_cast<const uint32_t*>(sGS + BN) + (cb0 + 32 * b) / 2;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  const uint32_t x1 = dequant_pair<QBIT>(cur.w1, 2 * i, sS1[i]), x2 = dequant_pair<QBIT>(cur.w2, 2 * i, sS2[i]);
+                  const uint32_t y1 = add2(x1, t1[i]), sig = sigmoid2(y1), y1s = mul2(y1, sig), y2 = add2(x2, t2[i]);
+                  o[i] = mul2(y1s, y2);
+                  const uint32_t inner = add2(kOne2, mul2(y1, sub2(kOne2, sig)));
+                  t1[i] = mul2(mul2(gd[b][i], y2), mul2(sig, inner));
+                  t2[i] = mul2(gd[b][i], y1s);
+                }
+                flush_pairs(o, R, p.out0, row0, p.M, p.N, n, lane);
+                flush_pairs(t1, R, p.out1, row0, p.M, p.N, n, lane);
+                flush_pairs(t2, R, p.out2, row0, p.M, p.N, n, lane);
+              }
+          } else {
+            const bool has1 = sv.l1.bt != nullptr, has_res = sv.residual != nullptr;
+            uint32_t x[4][16];
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+              if (b < blocks) tc_ld_pairs(t_lane + (uint32_t)(cb0 + 32 * b), x[b]);
+            if (lora_rounds) columns_read();
+            if (sv.q != nullptr || sv.main != nullptr) {
+#pragma unroll
+              for (int b = 0; b < 4; ++b)
+                if (b < blocks && valid) {
+                  const int64_t n = (int64_t)sv.n0 + cb0 + 32 * b;
+                  if (sv.q != nullptr) {
+                    uint32_t w1[BlockGeo<QBIT>::NW];
+                    pack_codes<QBIT>(x[b], sGV + cb0 + 32 * b, w1);
+                    store_block_words<QBIT>(sv.q + (row * sv.ld + n) * QBIT / 8, w1);
+                  }
+                  if (sv.main != nullptr) store_pairs(x[b], sv.main + row * sv.ld + n);
+                }
+            }
+            if (lora_rounds) lora_wait();
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+              if (b < blocks) {
+                const int64_t n = (int64_t)sv.n0 + cb0 + 32 * b;
+                if (lora_rounds) {
+                  uint32_t l[16];
+                  tc_ld_pairs(t_lane + (uint32_t)(cb0 + 32 * b), l);
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) x[b][i] = add2(x[b][i], l[i]);
+                }
+                if (has1) {
+#pragma unroll 1
+                  for (int i = 0; i < 16; ++i) {
+                    const uint32_t l = pack_bf16x2_rn(lora_dot_global(sv.l1, n + 2 * i, row, valid), lora_dot_global(sv.l1, n + 2 * i + 1, row, valid));
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                      if (j == i) x[b][j] = add2(x[b][j], l);
+                  }
+                }
+                if (has_res) {
+                  const uint4 now[4] = {res[0], res[1], res[2], res[3]};
+                  if (b + 1 < blocks) tile_fetch(sv.residual, row0, p.M, sv.ld, n + 32, lane, res);
+                  tile_put(R, lane, now);
+                  __syncwarp();
+#pragma unroll
+                  for (int c8 = 0; c8 < 4; ++c8) {
+                    const uint4 r = *reinterpret_cast<const uint4*>(R + gd_chunk(lane, c8));
+                    x[b][4 * c8] = add2(x[b][4 * c8], r.x); x[b][4 * c8 + 1] = add2(x[b][4 * c8 + 1], r.y);
+                    x[b][4 * c8 + 2] = add2(x[b][4 * c8 + 2], r.z); x[b][4 * c8 + 3] = add2(x[b][4 * c8 + 3], r.w);
+                  }
+                  __syncwarp();
+                }
+                flush_pairs(x[b], R, sv.out, row0, p.M, sv.ld, n, lane);
+              }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tmem_empty_leader[buf]);
+        epi_bar_sync();    // everyone is done with the staged tile before the next one overwrites it
+      }
+    } else
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
       const int m0 = (tile % tiles_m) * TILE_M + (int)rank * BM, ct = tile / tiles_m;
       const bool wide = ct < p.n_wide;
@@ -427,10 +687,8 @@ template <int EPI, int QBIT, bool B_MN>
 static int launch(const Operands& ops, const Params& p, cudaStream_t st) {
   const SplitPlan plan = choose_split(EPI, B_MN, p);
   if (plan.split > 0) return launch_split(EPI, QBIT, B_MN, plan, ops, p, st);
-  // Pairs, except where few rows would leave half of the tile empty, and for grad_down with many tiles: its epilogue is
-  // the longest (mma.sync products, which queue behind a busy tensor pipe) and in a pair a stall of either SM holds up
-  // both.  2048 tokens, Llama-2-7B: 159 us single, 182 us as pairs; 512 tokens: 61 / 55 us; 256: 45 / 42 us
-  bool pair = p.M > BM && (EPI != EPI_GRADDOWN || p.M <= 5 * BM);
+  // pairs, except where few rows would leave half of the tile empty
+  bool pair = p.M > BM;
 #ifdef HYC_TUNE
   if (const char* e = getenv("HYC_SPLIT")) { int v = atoi(e); if (v >= 200) pair = v >= 300; }
 #endif

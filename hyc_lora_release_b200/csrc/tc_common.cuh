@@ -120,6 +120,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {      // does not suspend
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
 // bounded wait; false = gave up (either the limit was hit here or another role raised abort)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < SPIN_LIMIT; ++i) {
@@ -221,6 +230,12 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_b
   d |= (uint64_t)2 << 61;
   return d;
 }
+
+// no swizzle, K-major: core matrices of 8 rows x 16 bytes, the two of a K = 16 slice 128 bytes apart, row groups 256
+__device__ __forceinline__ uint64_t make_desc_k16(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr & 0x3ffffu) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46);
+}
+__device__ __forceinline__ uint32_t k16_offset(int row, int k_half) { return (uint32_t)((row >> 3) * 256 + k_half * 128 + (row & 7) * 16); }
 
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * EPI_WARPS) : "memory"); }
 
@@ -539,6 +554,15 @@ __device__ __forceinline__ void gd_fetch(const Params& p, int64_t row0, int lane
   lora_load_b(p.l2, n, lane, in.b2);
 }
 
+// the codes alone (pair form)
+template <int QBIT> struct GdCodes { uint32_t w1[BlockGeo<QBIT>::NW], w2[BlockGeo<QBIT>::NW]; };
+template <int QBIT>
+__device__ __forceinline__ void gd_codes(const Params& p, int64_t row, int64_t n, GdCodes<QBIT>& in) {
+  const bool valid = row < p.M;
+  load_block_words<QBIT>(p.q1 + (row * p.N + n) * QBIT / 8, valid, in.w1);
+  load_block_words<QBIT>(p.q2 + (row * p.N + n) * QBIT / 8, valid, in.w2);
+}
+
 // One block of 32 rows x 32 columns of the GRADDOWN epilogue, a whole warp at a time (lane = row for the
 // accumulator and the element-wise chain).  The LoRA terms of the two branches are rank-16 products on the legacy
 // tensor path: fragments -> bf16 pairs -> the warp's two shared-memory tiles, from which every lane reads its own
@@ -660,6 +684,71 @@ __device__ __forceinline__ void epi_store_block(const StoreView& v, int64_t row0
   gd_flush(R, v.out, row0, M, v.ld, n, lane);
   __syncwarp();
   if (save && valid) store_block_words<QBIT>(v.q + (row * v.ld + n) * QBIT / 8, w1);
+}
+
+// ------------------------------------------------------------------ epilogues of the pair form
+// The rank-16 LoRA terms come from tcgen05 as well: once the warps of both CTAs have the main branch of a tile in registers
+// (as bf16 pairs), its tensor-memory columns are free and take bf16 xa B^T as one K = 16 product each.  From mma.sync
+// fragments the same terms queued behind the busy tensor pipe: the epilogue of the gate/up product took 38 k cycles where
+// the main loop of the next tile takes 34 k (2048 tokens, Llama-2-7B: 293 us; without those instructions 237).
+struct LoraStage { uint8_t *a1, *a2, *b1, *b2; };      // [128][16] and [columns / 2][16] operands, k16_offset layout
+
+// 16-byte chunks of operand rows, by the 256 epilogue threads (et)
+__device__ __forceinline__ void stage_lora_a(uint8_t* dst, const __nv_bfloat16* xa, int64_t m0, int64_t M, int et) {
+  const int row = et >> 1, kh = et & 1;
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (m0 + row < M) v = *reinterpret_cast<const uint4*>(xa + (m0 + row) * 16 + 8 * kh);
+  *reinterpret_cast<uint4*>(dst + k16_offset(row, kh)) = v;
+}
+__device__ __forceinline__ void stage_lora_b(uint8_t* dst, const LoraTerm& l, int64_t n, int rows, int et) {
+  const int row = et >> 1, kh = et & 1;
+  if (row >= rows) return;
+  const __nv_bfloat16* p = l.bt + (n + row) * l.ld_col + 8 * kh * l.ld_r;
+  uint4 v;
+  if (l.ld_r == 1 && (l.ld_col & 7) == 0 && (reinterpret_cast<uintptr_t>(l.bt) & 15) == 0) {
+    v = *reinterpret_cast<const uint4*>(p);
+  } else {
+    auto two = [&](int r) { return (uint32_t)__bfloat16_as_ushort(p[r * l.ld_r]) | ((uint32_t)__bfloat16_as_ushort(p[(r + 1) * l.ld_r]) << 16); };
+    v = make_uint4(two(0), two(2), two(4), two(6));
+  }
+  *reinterpret_cast<uint4*>(dst + k16_offset(row, kh)) = v;
+}
+
+// 32 accumulator columns of the lane's row as 16 bf16 pairs
+__device__ __forceinline__ void tc_ld_pairs(uint32_t taddr, uint32_t (&x)[16]) {
+  uint32_t v[32];
+  tc_ld32(taddr, v);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = pack_bf16x2_rn(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+}
+// the block's codes; r: its quantizer constants in shared memory
+template <int QBIT>
+__device__ __forceinline__ void pack_codes(const uint32_t (&x)[16], const float* r, uint32_t (&w)[BlockGeo<QBIT>::NW]) {
+  using G = BlockGeo<QBIT>;
+#pragma unroll
+  for (int i = 0; i < G::NW; ++i) w[i] = 0u;
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) {
+    const float4 k = *reinterpret_cast<const float4*>(r + c);
+    put_code<QBIT>(w, c, fastq_code_bits<QBIT>(bf16lo_to_f32(x[c / 2]), k.x) & G::CM);
+    put_code<QBIT>(w, c + 1, fastq_code_bits<QBIT>(bf16hi_to_f32(x[c / 2]), k.y) & G::CM);
+    put_code<QBIT>(w, c + 2, fastq_code_bits<QBIT>(bf16lo_to_f32(x[c / 2 + 1]), k.z) & G::CM);
+    put_code<QBIT>(w, c + 3, fastq_code_bits<QBIT>(bf16hi_to_f32(x[c / 2 + 1]), k.w) & G::CM);
+  }
+}
+// a lane's 16 pairs through the warp's tile: out as whole 64-byte row segments
+__device__ __forceinline__ void flush_pairs(const uint32_t (&o)[16], uint32_t* R, __nv_bfloat16* out, int64_t row0, int64_t M, int64_t ldo, int64_t n,
+                                            int lane) {
+#pragma unroll
+  for (int c8 = 0; c8 < 4; ++c8)
+    *reinterpret_cast<uint4*>(R + gd_chunk(lane, c8)) = make_uint4(o[4 * c8], o[4 * c8 + 1], o[4 * c8 + 2], o[4 * c8 + 3]);
+  __syncwarp();
+  gd_flush(R, out, row0, M, ldo, n, lane);
+  __syncwarp();
+}
+__device__ __forceinline__ void store_pairs(const uint32_t (&o)[16], __nv_bfloat16* dst) {
+#pragma unroll
+  for (int c8 = 0; c8 < 4; ++c8) *reinterpret_cast<uint4*>(dst + 8 * c8) = make_uint4(o[4 * c8], o[4 * c8 + 1], o[4 * c8 + 2], o[4 * c8 + 3]);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
