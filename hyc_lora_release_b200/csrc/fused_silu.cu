@@ -506,43 +506,42 @@ dequant_lora_add_kernel(const RebuildJobs jobs, int64_t rows) {
     const uint4 a = *reinterpret_cast<const uint4*>(sv + col);
     sp[0] = a.x; sp[1] = a.y; sp[2] = a.z; sp[3] = a.w;
   }
+  // the B fragments of the warp's 64 columns stay in registers; a tile's codes and xa rows are fetched one tile ahead
+  uint32_t fb[8][2];
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    const int n = octet(nt) + g;
+    fb[nt][0] = n < N ? *reinterpret_cast<const uint32_t*>(bt + (int64_t)n * 16 + 2 * t) : 0u;
+    fb[nt][1] = n < N ? *reinterpret_cast<const uint32_t*>(bt + (int64_t)n * 16 + 2 * t + 8) : 0u;
+  }
   const int64_t n_tiles = (rows + 15) / 16;
-  for (int64_t rt = blockIdx.y; rt < n_tiles; rt += gridDim.y) {
-    uint2 pq[4];
+  const int qcol = QBIT == 8 ? col : (QBIT == 4 ? 16 * blk + 8 * (cg & 1) : 8 * blk);
+  uint2 nq[4];
+  uint32_t na[4];
+  auto fetch = [&](int64_t rt) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int64_t row = rt * 16 + 4 * i + rsub;
-      pq[i] = make_uint2(0u, 0u);
-      if (row < rows && col_ok) {
-        if (QBIT == 8) pq[i] = ld_stream_v2(q + row * qld + col);
-        else if (QBIT == 4) pq[i] = ld_stream_v2(q + row * qld + 16 * blk + 8 * (cg & 1));
-        else pq[i] = ld_stream_v2(q + row * qld + 8 * blk);
-      }
+      nq[i] = make_uint2(0u, 0u);
+      if (row < rows && col_ok) nq[i] = ld_stream_v2(q + row * qld + qcol);
     }
-    {
-      const int64_t ra = rt * 16 + g, rb = ra + 8;
-      uint32_t a[4] = {0u, 0u, 0u, 0u};
-      if (ra < rows) {
-        a[0] = *reinterpret_cast<const uint32_t*>(xa + ra * 16 + 2 * t);
-        a[2] = *reinterpret_cast<const uint32_t*>(xa + ra * 16 + 2 * t + 8);
-      }
-      if (rb < rows) {
-        a[1] = *reinterpret_cast<const uint32_t*>(xa + rb * 16 + 2 * t);
-        a[3] = *reinterpret_cast<const uint32_t*>(xa + rb * 16 + 2 * t + 8);
-      }
-#pragma unroll 2
-      for (int nt = 0; nt < 8; ++nt) {
-        const int n = octet(nt) + g;
-        uint32_t ba = 0u, bb = 0u;
-        if (n < N) {
-          ba = *reinterpret_cast<const uint32_t*>(bt + (int64_t)n * 16 + 2 * t);
-          bb = *reinterpret_cast<const uint32_t*>(bt + (int64_t)n * 16 + 2 * t + 8);
-        }
-        float l[4];
-        mma_bf16_16816(l, a, ba, bb);
-        sl[g * kWideLd + 4 * nt + t] = pack_bf16x2_rn(l[0], l[1]);
-        sl[(g + 8) * kWideLd + 4 * nt + t] = pack_bf16x2_rn(l[2], l[3]);
-      }
+    const int64_t ra = rt * 16 + g, rb = ra + 8;
+    na[0] = ra < rows ? *reinterpret_cast<const uint32_t*>(xa + ra * 16 + 2 * t) : 0u;
+    na[2] = ra < rows ? *reinterpret_cast<const uint32_t*>(xa + ra * 16 + 2 * t + 8) : 0u;
+    na[1] = rb < rows ? *reinterpret_cast<const uint32_t*>(xa + rb * 16 + 2 * t) : 0u;
+    na[3] = rb < rows ? *reinterpret_cast<const uint32_t*>(xa + rb * 16 + 2 * t + 8) : 0u;
+  };
+  fetch(blockIdx.y);
+  for (int64_t rt = blockIdx.y; rt < n_tiles; rt += gridDim.y) {
+    const uint2 pq[4] = {nq[0], nq[1], nq[2], nq[3]};
+    const uint32_t a[4] = {na[0], na[1], na[2], na[3]};
+    if (rt + gridDim.y < n_tiles) fetch(rt + gridDim.y);
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      float l[4];
+      mma_bf16_16816(l, a, fb[nt][0], fb[nt][1]);
+      sl[g * kWideLd + 4 * nt + t] = pack_bf16x2_rn(l[0], l[1]);
+      sl[(g + 8) * kWideLd + 4 * nt + t] = pack_bf16x2_rn(l[2], l[3]);
     }
     __syncwarp();
 #pragma unroll

@@ -134,11 +134,30 @@ __device__ __forceinline__ void lane_load_dequant(const uint8_t* __restrict__ qg
   }
 }
 
+// Which lane owns group g of a warp's run.  RAGGED: rows of `groups` groups where LPR (the power of two above) lanes serve a
+// row; the last LPR - groups lanes of every row own nothing.
+template <int LPR, bool RAGGED> struct LaneMap {
+  int groups;
+  uint32_t inv;                  // 65536 / groups + 1: g * inv >> 16 is g / groups for g < 32
+  __device__ __forceinline__ explicit LaneMap(int n) : groups(n), inv(RAGGED ? 65536u / (uint32_t)n + 1u : 0u) {}
+  __device__ __forceinline__ int owner(int g) const {
+    if (!RAGGED) return g;
+    const int r = (int)(((uint32_t)g * inv) >> 16);
+    return r * LPR + (g - r * groups);
+  }
+  static constexpr bool ragged = RAGGED;
+};
+typedef LaneMap<32, false> LaneMapWhole;
+
 // global -> shared: pieces [0, n_pieces) of the run, zeros beyond (slots = the warp's 32 x 32 words)
-__device__ __forceinline__ void lane_run_to_shared(const __nv_bfloat16* __restrict__ run, int n_pieces, uint32_t* slots, int lane) {
+// (RAGGED: slots beyond the run are left as they are)
+template <typename MAP = LaneMapWhole>
+__device__ __forceinline__ void lane_run_to_shared(const __nv_bfloat16* __restrict__ run, int n_pieces, uint32_t* slots, int lane,
+                                                   const MAP& map = MAP(32)) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int p = 32 * i + lane;
+    if (MAP::ragged && p >= n_pieces) continue;
     uint32_t t[8];
     if (p < n_pieces) {
       ld_stream_v8(run + 16 * p, t);
@@ -146,7 +165,7 @@ __device__ __forceinline__ void lane_run_to_shared(const __nv_bfloat16* __restri
 #pragma unroll
       for (int j = 0; j < 8; ++j) t[j] = 0u;
     }
-    const int owner = p >> 2, c0 = 2 * (p & 3);
+    const int owner = map.owner(p >> 2), c0 = 2 * (p & 3);
     uint32_t* dst = slots + owner * 32;
     *reinterpret_cast<uint4*>(dst + park_chunk(c0, owner)) = make_uint4(t[0], t[1], t[2], t[3]);
     *reinterpret_cast<uint4*>(dst + park_chunk(c0 + 1, owner)) = make_uint4(t[4], t[5], t[6], t[7]);
@@ -154,11 +173,14 @@ __device__ __forceinline__ void lane_run_to_shared(const __nv_bfloat16* __restri
 }
 // global -> shared without passing through registers (cp.async): the same placement as lane_run_to_shared.  The
 // copy is in flight while the warp does other work; lane_async_wait() + __syncwarp() before the slots are read.
-__device__ __forceinline__ void lane_run_to_shared_async(const __nv_bfloat16* __restrict__ run, int n_pieces, uint32_t* slots, int lane) {
+template <typename MAP = LaneMapWhole>
+__device__ __forceinline__ void lane_run_to_shared_async(const __nv_bfloat16* __restrict__ run, int n_pieces, uint32_t* slots, int lane,
+                                                         const MAP& map = MAP(32)) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int p = 32 * i + lane;
-    const int owner = p >> 2, c0 = 2 * (p & 3);
+    if (MAP::ragged && p >= n_pieces) continue;
+    const int owner = map.owner(p >> 2), c0 = 2 * (p & 3);
     uint32_t* dst = slots + owner * 32;
     const bool in = p < n_pieces;
     const __nv_bfloat16* src = run + 16 * (in ? p : 0);
@@ -172,11 +194,14 @@ __device__ __forceinline__ void lane_run_to_shared_async(const __nv_bfloat16* __
 }
 __device__ __forceinline__ void lane_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 // shared -> global
-__device__ __forceinline__ void lane_shared_to_run(const uint32_t* slots, __nv_bfloat16* __restrict__ run, int n_pieces, int lane) {
+template <typename MAP = LaneMapWhole>
+__device__ __forceinline__ void lane_shared_to_run(const uint32_t* slots, __nv_bfloat16* __restrict__ run, int n_pieces, int lane,
+                                                   const MAP& map = MAP(32)) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int p = 32 * i + lane;
-    const int owner = p >> 2, c0 = 2 * (p & 3);
+    if (MAP::ragged && p >= n_pieces) continue;
+    const int owner = map.owner(p >> 2), c0 = 2 * (p & 3);
     const uint32_t* src = slots + owner * 32;
     const uint4 t0 = *reinterpret_cast<const uint4*>(src + park_chunk(c0, owner));
     const uint4 t1 = *reinterpret_cast<const uint4*>(src + park_chunk(c0 + 1, owner));

@@ -584,7 +584,7 @@ extern "C" HYC_API int hyc_softmax_bwd(const void* y, const void* g, void* o, in
   if (rows < 0 || S <= 0 || S % 8 != 0 || S > 32 * 8 * kSmMaxVec) return HYC_ERR_SHAPE;
   if (!aligned(y, 16) || !aligned(g, 16) || !aligned(o, 16)) return HYC_ERR_ALIGN;
   if (rows == 0) return HYC_OK;
-  if (softmax_bwd_lane(y, g, rows, S, out_scale, o, (cudaStream_t)stream)) {   // rows of 64 * 2^n columns: staged, coalesced
+  if (softmax_bwd_lane(y, g, rows, S, out_scale, o, (cudaStream_t)stream)) {   // rows of 64 n <= 2048 columns: staged, coalesced
     HYC_CHECK_LAUNCH();
     return HYC_OK;
   }

@@ -4,7 +4,8 @@
 // every lane owning ONE quantization group: 64 consecutive columns = 128 contiguous bytes = 32 packed
 // bf16 pairs.  A warp therefore works on 32 / LPR rows at a time, and everything that costs one warp
 // instruction per row in a warp-per-row layout (reductions, scans, group parameters) is shared by
-// those rows; group min/max needs no shuffle at all.
+// those rows; group min/max needs no shuffle at all.  Rows whose groups are not a power of two (RAGGED) get the next power
+// of two of lanes, of which the last ones own no group.
 //
 // Selection of the k largest magnitudes of a row is an exact radix select on BIT PLANES:
 //   1. the lane's 64 magnitude patterns (15 bits) are bit-transposed in registers into 15 planes of
@@ -63,17 +64,20 @@ struct SoftmaxPrologue {
 };
 
 // ---------------------------------------------------------------- compress
-template <int QBIT, int LPR, bool SOFTMAX>
+template <int QBIT, int LPR, bool SOFTMAX, bool RAGGED>
 __global__ void __launch_bounds__(256, HYC_LANE_MINB)
-topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int k,
+topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int groups, int k,
                           __nv_bfloat16* __restrict__ val_out, uint16_t* __restrict__ col_out,
                           uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scale, int8_t* __restrict__ zp,
                           SoftmaxPrologue sp) {
   constexpr int RPW = 32 / LPR;          // rows per warp
-  constexpr int S = 64 * LPR;
-  constexpr int64_t QLD = (int64_t)S * QBIT / 8;
+  const int GPR = RAGGED ? groups : LPR; // groups per row
+  const int S = 64 * GPR;
+  const int64_t QLD = (int64_t)S * QBIT / 8;
+  const LaneMap<LPR, RAGGED> map(GPR);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int lr = lane & (LPR - 1), rw = lane / LPR;
+  const bool owns = !RAGGED || lr < GPR;
   __shared__ __align__(16) uint32_t s_x[8][32 * 32];          // the warp's rows, 128 bytes per lane
   __shared__ uint32_t s_out[8][kLaneStageEntries];            // staged (column << 16 | value) words
   uint32_t* sx = s_x[warp] + lane * 32;
@@ -85,7 +89,7 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
     // the warp's rows are one contiguous run of 4 KB: fetch it, park it, read the lane's own group back
     const int64_t left = rows - row0;
     const int n_rows = (int)(left < RPW ? left : RPW);
-    lane_run_to_shared(a + row0 * S, n_rows * (S / 16), s_x[warp], lane);
+    lane_run_to_shared(a + row0 * S, n_rows * (S / 16), s_x[warp], lane, map);
     __syncwarp();
     uint32_t xw[32];
     lane_slot_load(sx, lane, xw);
@@ -187,7 +191,7 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
         }
       // ---- radix select, most significant plane first
       // (branch-free: the rows of a warp take different sides)
-      uint32_t A0 = kFull, A1 = kFull, G0 = 0u, G1 = 0u;
+      uint32_t A0 = owns ? kFull : 0u, A1 = A0, G0 = 0u, G1 = 0u;
       int rem = k;                       // k - (number of magnitudes known to be above the threshold)
 #pragma unroll
       for (int b = 14; b >= 0; --b) {
@@ -255,10 +259,10 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
     float mn, mx;
     lane_minmax(xw, mn, mx);
     const GroupParams p = group_params<QBIT>(mn, mx);
-    if (valid) {
+    if (valid && owns) {
       lane_quant_store<QBIT>(xw, p, q + row * QLD + (64 * QBIT / 8) * lr);
-      scale[row * LPR + lr] = __ushort_as_bfloat16(f32_to_bf16bits_rn(p.s));
-      zp[row * LPR + lr] = (int8_t)(int)p.z;
+      scale[row * GPR + lr] = __ushort_as_bfloat16(f32_to_bf16bits_rn(p.s));
+      zp[row * GPR + lr] = (int8_t)(int)p.z;
     }
     __syncwarp();   // the slots and the staging area are rewritten by other lanes in the next round
   }
@@ -268,18 +272,21 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
 // SMBWD: instead of the restored map y itself, write the softmax backward of it for the upstream gradient
 // `grad`:  out = (g - sum_row(bf16(y * g))) * y  (operators/softmax_kernels.py:7-38: the product is a bf16
 // operation, the row sum and the rest fp32).  The restored map never goes to HBM.
-template <int QBIT, int LPR, bool SMBWD>
+template <int QBIT, int LPR, bool SMBWD, bool RAGGED>
 __global__ void __launch_bounds__(256, SMBWD ? 3 : HYC_LANE_MINB)      // SMBWD: two tiles per warp, 3 blocks fill the SM
 topk_lane_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* __restrict__ colv, int k, float inv_k,
                          const uint8_t* __restrict__ q, const __nv_bfloat16* __restrict__ scale,
-                         const int8_t* __restrict__ zp, int64_t rows, const __nv_bfloat16* __restrict__ grad,
+                         const int8_t* __restrict__ zp, int64_t rows, int groups, const __nv_bfloat16* __restrict__ grad,
                          float oscale, __nv_bfloat16* __restrict__ ao) {
   constexpr int RPW = 32 / LPR;
-  constexpr int S = 64 * LPR;
-  constexpr int64_t QLD = (int64_t)S * QBIT / 8;
+  const int GPR = RAGGED ? groups : LPR;
+  const int S = 64 * GPR;
+  const int64_t QLD = (int64_t)S * QBIT / 8;
+  const LaneMap<LPR, RAGGED> map(GPR);
   constexpr int PRE = 4;                 // list entries per lane fetched before the de-quantization
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int lr = lane & (LPR - 1), rw = lane / LPR;
+  const bool owns = !RAGGED || lr < GPR;
   // dynamic shared memory: per warp its rows (128 bytes per lane) and, SMBWD, a second tile for the gradient rows
   extern __shared__ __align__(16) uint32_t s_dyn[];
   uint32_t* s_xw = s_dyn + warp * 1024;
@@ -294,7 +301,7 @@ topk_lane_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* 
     const int n_rows = (int)(left < RPW ? left : RPW);
     const int n_ent = n_rows * k;
     // the gradient rows start their way into shared memory now and arrive while the map is being rebuilt
-    if (SMBWD) lane_run_to_shared_async(grad + row0 * S, n_rows * (S / 16), s_gw, lane);
+    if (SMBWD) lane_run_to_shared_async(grad + row0 * S, n_rows * (S / 16), s_gw, lane, map);
     const __nv_bfloat16* vrun = val + row0 * k;
     const uint16_t* crun = colv + row0 * k;
     uint16_t pc[PRE], pv[PRE];
@@ -307,9 +314,9 @@ topk_lane_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* 
     // de-quantize the lane's group into its shared-memory slot
     {
       uint32_t o[32];
-      if (valid) {
-        const float s = __bfloat162float(scale[row * LPR + lr]);
-        const float z = (float)zp[row * LPR + lr];
+      if (valid && owns) {
+        const float s = __bfloat162float(scale[row * GPR + lr]);
+        const float z = (float)zp[row * GPR + lr];
         lane_load_dequant<QBIT>(q + row * QLD + (64 * QBIT / 8) * lr, s, z, o);
       } else {
 #pragma unroll
@@ -350,6 +357,7 @@ topk_lane_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* 
                                             *reinterpret_cast<const __nv_bfloat162*>(&gv[j]));
         acc += __bfloat162float(p.x) + __bfloat162float(p.y);
       }
+      if (!owns) acc = 0.f;
 #pragma unroll
       for (int o = 1; o < LPR; o <<= 1) acc += __shfl_xor_sync(kFull, acc, o);     // stays inside the row's lanes
 #pragma unroll
@@ -365,19 +373,21 @@ topk_lane_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* 
       __syncwarp();
     }
     // the warp's rows leave as four fully coalesced 1 KB stores
-    lane_shared_to_run(s_xw, ao + row0 * S, n_rows * (S / 16), lane);
+    lane_shared_to_run(s_xw, ao + row0 * S, n_rows * (S / 16), lane, map);
     __syncwarp();
   }
 }
 
 // ---------------------------------------------------------------- softmax backward on dense maps
-// out = (g - sum_row(bf16(y * g))) * y for rows of 64 * LPR columns, same layout and staging as above
-template <int LPR>
+// out = (g - sum_row(bf16(y * g))) * y, same layout and staging as above
+template <int LPR, bool RAGGED>
 __global__ void __launch_bounds__(256, 3)
-softmax_bwd_lane_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ g, int64_t rows,
+softmax_bwd_lane_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ g, int64_t rows, int groups,
                         float oscale, __nv_bfloat16* __restrict__ out) {
   constexpr int RPW = 32 / LPR;
-  constexpr int S = 64 * LPR;
+  const int GPR = RAGGED ? groups : LPR;
+  const int S = 64 * GPR;
+  const LaneMap<LPR, RAGGED> map(GPR);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   // dynamic shared memory: two 4 KB tiles per warp, so that both operands are on their way at once (cp.async)
   extern __shared__ __align__(16) uint32_t s_dyn[];
@@ -389,8 +399,8 @@ softmax_bwd_lane_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16
     const int64_t row0 = item * RPW, left = rows - row0;
     const int n_pieces = (int)(left < RPW ? left : RPW) * (S / 16);
     uint32_t yv[32], gv[32];
-    lane_run_to_shared_async(y + row0 * S, n_pieces, s_yw, lane);
-    lane_run_to_shared_async(g + row0 * S, n_pieces, s_gw, lane);
+    lane_run_to_shared_async(y + row0 * S, n_pieces, s_yw, lane, map);
+    lane_run_to_shared_async(g + row0 * S, n_pieces, s_gw, lane, map);
     lane_async_wait();
     __syncwarp();
     lane_slot_load(sx, lane, yv);
@@ -402,6 +412,7 @@ softmax_bwd_lane_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16
                                           *reinterpret_cast<const __nv_bfloat162*>(&gv[j]));
       acc += __bfloat162float(p.x) + __bfloat162float(p.y);
     }
+    if (RAGGED && (lane & (LPR - 1)) >= GPR) acc = 0.f;
 #pragma unroll
     for (int o = 1; o < LPR; o <<= 1) acc += __shfl_xor_sync(kFull, acc, o);
 #pragma unroll
@@ -415,14 +426,14 @@ softmax_bwd_lane_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16
     __syncwarp();
     lane_slot_store(sx, lane, gv);
     __syncwarp();
-    lane_shared_to_run(s_yw, out + row0 * S, n_pieces, lane);
+    lane_shared_to_run(s_yw, out + row0 * S, n_pieces, lane, map);
     __syncwarp();
   }
 }
 
-template <int LPR>
-static void launch_softmax_bwd(const void* y, const void* g, int64_t rows, float oscale, void* out, cudaStream_t st) {
-  auto kern = softmax_bwd_lane_kernel<LPR>;
+template <int LPR, bool RAGGED>
+static void launch_softmax_bwd(const void* y, const void* g, int64_t rows, int groups, float oscale, void* out, cudaStream_t st) {
+  auto kern = softmax_bwd_lane_kernel<LPR, RAGGED>;
   static bool attr[64] = {false};      // up to 64 KB of dynamic shared memory per block: set per device
   const int slot = current_device_slot();
   if (slot < 0 || !attr[slot]) {
@@ -431,52 +442,57 @@ static void launch_softmax_bwd(const void* y, const void* g, int64_t rows, float
   }
   int grid, threads;
   lane_launch_shape(kern, rows, 32 / LPR, grid, threads, 8192);
-  kern<<<grid, threads, (threads / 32) * 8192, st>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)g, rows, oscale,
+  kern<<<grid, threads, (threads / 32) * 8192, st>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)g, rows, groups, oscale,
                                                      (__nv_bfloat16*)out);
 }
 
-// rows of 64 * 2^n <= 2048 columns, 32-byte aligned tensors; false = not covered (nothing launched)
-bool softmax_bwd_lane(const void* y, const void* g, int64_t rows, int S, float oscale, void* out, cudaStream_t st) {
-  if (S < 64 || S > 2048 || (S & (S - 1)) != 0 || !aligned(y, 32) || !aligned(g, 32) || !aligned(out, 32)) return false;
-  switch (S / 64) {
-    case 1: launch_softmax_bwd<1>(y, g, rows, oscale, out, st); break;
-    case 2: launch_softmax_bwd<2>(y, g, rows, oscale, out, st); break;
-    case 4: launch_softmax_bwd<4>(y, g, rows, oscale, out, st); break;
-    case 8: launch_softmax_bwd<8>(y, g, rows, oscale, out, st); break;
-    case 16: launch_softmax_bwd<16>(y, g, rows, oscale, out, st); break;
-    default: launch_softmax_bwd<32>(y, g, rows, oscale, out, st); break;
+#define HYC_LANE_DISPATCH(FN, ...)                                                                    \
+  switch (topk_lanes_per_row(S)) {                                                                    \
+    case 1: FN(1, false)(__VA_ARGS__); break;                                                         \
+    case 2: FN(2, false)(__VA_ARGS__); break;                                                         \
+    case 4: if (S == 256) FN(4, false)(__VA_ARGS__); else FN(4, true)(__VA_ARGS__); break;            \
+    case 8: if (S == 512) FN(8, false)(__VA_ARGS__); else FN(8, true)(__VA_ARGS__); break;            \
+    case 16: if (S == 1024) FN(16, false)(__VA_ARGS__); else FN(16, true)(__VA_ARGS__); break;        \
+    default: if (S == 2048) FN(32, false)(__VA_ARGS__); else FN(32, true)(__VA_ARGS__); break;        \
   }
+
+// rows of 64 n <= 2048 columns, 32-byte aligned tensors; false = not covered (nothing launched)
+bool softmax_bwd_lane(const void* y, const void* g, int64_t rows, int S, float oscale, void* out, cudaStream_t st) {
+  if (S < 64 || S > 2048 || S % 64 != 0 || !aligned(y, 32) || !aligned(g, 32) || !aligned(out, 32)) return false;
+#define FN(L, RG) launch_softmax_bwd<L, RG>
+  HYC_LANE_DISPATCH(FN, y, g, rows, S / 64, oscale, out, st);
+#undef FN
   return true;
 }
 
 // ---------------------------------------------------------------- launchers
-template <int QBIT, int LPR>
-static void launch_compress(const void* a, int64_t rows, int k, void* val, uint16_t* col, void* q, void* scale,
+template <int QBIT, int LPR, bool RAGGED>
+static void launch_compress(const void* a, int64_t rows, int groups, int k, void* val, uint16_t* col, void* q, void* scale,
                             int8_t* zp, const SoftmaxPrologue* sp, cudaStream_t st) {
   int grid, threads;
   if (sp == nullptr) {
-    auto kern = topk_lane_compress_kernel<QBIT, LPR, false>;
+    auto kern = topk_lane_compress_kernel<QBIT, LPR, false, RAGGED>;
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads);
-    kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)a, rows, k, (__nv_bfloat16*)val, col,
+    kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)a, rows, groups, k, (__nv_bfloat16*)val, col,
                                    (uint8_t*)q, (__nv_bfloat16*)scale, zp, SoftmaxPrologue{});
-  } else {
-    auto kern = topk_lane_compress_kernel<QBIT, LPR, true>;
+  } else if constexpr (!RAGGED) {
+    auto kern = topk_lane_compress_kernel<QBIT, LPR, true, false>;
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads);
-    kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)a, rows, k, (__nv_bfloat16*)val, col,
+    kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)a, rows, groups, k, (__nv_bfloat16*)val, col,
                                    (uint8_t*)q, (__nv_bfloat16*)scale, zp, *sp);
   }
 }
-template <int QBIT, int LPR>
+template <int QBIT, int LPR, bool RAGGED>
 static void launch_restore(const void* val, const uint16_t* col, int k, const void* q, const void* scale,
-                           const int8_t* zp, int64_t rows, const void* grad, float oscale, void* ao, cudaStream_t st) {
+                           const int8_t* zp, int64_t rows, int groups, const void* grad, float oscale, void* ao, cudaStream_t st) {
   int grid, threads;
   if (grad == nullptr) {
-    auto kern = topk_lane_restore_kernel<QBIT, LPR, false>;
+    auto kern = topk_lane_restore_kernel<QBIT, LPR, false, RAGGED>;
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads, 4096);
     kern<<<grid, threads, (threads / 32) * 4096, st>>>((const __nv_bfloat16*)val, col, k, k > 0 ? 1.0f / (float)k : 0.f,
-                                   (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows, nullptr, 1.f, (__nv_bfloat16*)ao);
+                                   (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows, groups, nullptr, 1.f, (__nv_bfloat16*)ao);
   } else {
-    auto kern = topk_lane_restore_kernel<QBIT, LPR, true>;
+    auto kern = topk_lane_restore_kernel<QBIT, LPR, true, RAGGED>;
     // two 4 KB tiles per warp: up to 64 KB per block, above the default limit (set per device)
     static bool attr[64] = {false};
     const int slot = current_device_slot();
@@ -486,32 +502,25 @@ static void launch_restore(const void* val, const uint16_t* col, int k, const vo
     }
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads, 8192);
     kern<<<grid, threads, (threads / 32) * 8192, st>>>((const __nv_bfloat16*)val, col, k, k > 0 ? 1.0f / (float)k : 0.f,
-                                   (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows,
+                                   (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows, groups,
                                    (const __nv_bfloat16*)grad, oscale, (__nv_bfloat16*)ao);
   }
 }
 
-#define HYC_LANE_DISPATCH(FN, ...)                                            \
-  switch (S / 64) {                                                           \
-    case 1: FN<QB, 1>(__VA_ARGS__); break;                                    \
-    case 2: FN<QB, 2>(__VA_ARGS__); break;                                    \
-    case 4: FN<QB, 4>(__VA_ARGS__); break;                                    \
-    case 8: FN<QB, 8>(__VA_ARGS__); break;                                    \
-    case 16: FN<QB, 16>(__VA_ARGS__); break;                                  \
-    case 32: FN<QB, 32>(__VA_ARGS__); break;                                  \
-    default: return HYC_ERR_SHAPE;                                            \
-  }
-
 template <int QB>
 static int compress_q(const void* a, int64_t rows, int S, int k, void* val, uint16_t* col, void* q, void* scale,
                       int8_t* zp, const SoftmaxPrologue* sp, cudaStream_t st) {
-  HYC_LANE_DISPATCH(launch_compress, a, rows, k, val, col, q, scale, zp, sp, st);
+#define FN(L, RG) launch_compress<QB, L, RG>
+  HYC_LANE_DISPATCH(FN, a, rows, S / 64, k, val, col, q, scale, zp, sp, st);
+#undef FN
   return HYC_OK;
 }
 template <int QB>
 static int restore_q(const void* val, const uint16_t* col, int k, const void* q, const void* scale, const int8_t* zp,
                      int64_t rows, int S, const void* grad, float oscale, void* ao, cudaStream_t st) {
-  HYC_LANE_DISPATCH(launch_restore, val, col, k, q, scale, zp, rows, grad, oscale, ao, st);
+#define FN(L, RG) launch_restore<QB, L, RG>
+  HYC_LANE_DISPATCH(FN, val, col, k, q, scale, zp, rows, S / 64, grad, oscale, ao, st);
+#undef FN
   return HYC_OK;
 }
 
@@ -524,12 +533,12 @@ int topk_lane_compress(const void* a, int64_t rows, int S, int k, void* val_out,
 }
 
 // scores [rows, S] -> probabilities (written to `dense`) and their saved form, one pass.  Covered: the shapes of
-// topk_lane_ok with M a multiple of the rows a warp takes and mask rows S apart; HYC_ERR_UNSUPPORTED otherwise
+// topk_lane_ok with S a power of two, M a multiple of the rows a warp takes and mask rows S apart; HYC_ERR_UNSUPPORTED otherwise
 // (nothing launched: the caller runs the softmax and the compress kernels one after the other).
 int topk_lane_softmax_compress(const void* scores, float sc, const void* mask, int64_t mb, int64_t mh, int64_t mr, int heads,
                                int M, int64_t rows, int S, int k, void* dense, void* val_out, uint16_t* col_out,
                                void* q_out, void* scale_out, int8_t* zp_out, int q_bit, cudaStream_t st) {
-  if (!topk_lane_ok(S, k)) return HYC_ERR_UNSUPPORTED;
+  if (!topk_lane_ok(S, k) || (S & (S - 1)) != 0) return HYC_ERR_UNSUPPORTED;
   const int rpw = 32 / (S / 64);
   if (M % rpw != 0 || (mask != nullptr && mr != S) || !aligned(scores, 32) || !aligned(dense, 32) || !aligned(q_out, 32) ||
       (mask != nullptr && (!aligned(mask, 32) || (mb & 15) != 0 || (mh & 15) != 0)))

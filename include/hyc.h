@@ -185,7 +185,7 @@ int hyc_softmax_topk_restore(const void* val, const uint16_t* col, int k,
  * followed by `softmax_backward`): out = (g - sum_row(bf16(y * g))) * y with y the restored map, which is
  * never written to HBM.  grad, out [rows, S] bf16.  out_scale != 1 multiplies the bf16 result once more (a second
  * bf16 operation: the layer's `grad_s / sqrt(head_dim)`, :436).  Returns HYC_ERR_UNSUPPORTED for shapes outside the
- * lane-per-group kernels (S not 64 * 2^n <= 2048, very large k): restore, then hyc_softmax_bwd. */
+ * lane-per-group kernels (S > 2048, very large k): restore, then hyc_softmax_bwd. */
 int hyc_softmax_topk_restore_bwd(const void* val, const uint16_t* col, int k,
                                  const void* q, const void* scale, const int8_t* zp,
                                  int64_t rows, int S, const void* grad, void* out, int q_bit, float out_scale,

@@ -163,6 +163,28 @@ def test_topk_ties_lane_layout(cf, S, rows):
             assert torch.equal(m.to_dense().cpu(), oracle.topk_decompress(vals, cols, pk, sc, zp, q, x.shape))
 
 
+@pytest.mark.parametrize("S,rows", [(192, 37), (320, 11), (448, 5), (576, 9), (960, 4), (1088, 3), (1984, 2)])
+def test_topk_rows_of_other_group_counts(cf, S, rows):
+    """Rows whose groups are not a power of two share the lanes of the next one: least and most idle lanes of every lane count, a
+    ragged last warp, ties; the fused softmax backward against the oracle (the fp32 row sum has another order: one
+    rounding of the bf16 result and the cancellation in g - sum, as in the test below)."""
+    g = torch.Generator().manual_seed(S + rows)
+    ties = (torch.randint(-2, 3, (rows, S), generator=g).float() * 0.5).to(torch.bfloat16)
+    soft = torch.softmax(3 * torch.randn(rows, S, generator=g), -1).to(torch.bfloat16)
+    grad = torch.randn(rows, S, generator=g).to(torch.bfloat16)
+    for x in (ties, soft):
+        for q in (2, 4, 8):
+            m = cf.compression_softmax_topk(x.to(DEV), 0.05, q)
+            vals, cols, pk, sc, zp = oracle.topk_compress(x, 0.05, q)
+            assert torch.equal(m.col.cpu().to(torch.int64) & 0xFFFF, cols) and torch.equal(m.val.cpu(), vals)
+            assert torch.equal(m.q.cpu(), pk) and torch.equal(m.scale.cpu(), sc) and torch.equal(m.zp.cpu(), zp)
+            y = oracle.topk_decompress(vals, cols, pk, sc, zp, q, x.shape)
+            assert torch.equal(m.to_dense().cpu(), y)
+            ref = oracle.ref_softmax_backward(y.view(1, 1, rows, S), grad.view(1, 1, rows, S)).view(rows, S).float()
+            out = m.softmax_backward(grad.to(DEV)).float().cpu()
+            assert (out - ref).abs().max() <= 1e-2 * ref.abs().max()
+
+
 def test_topk_reused_buffers(cf):
     """``out=`` writes into the buffers of an earlier handle / an existing dense tensor, bit-identically."""
     a = _softmax_map(1, 2, 512, seed=3).to(DEV)
