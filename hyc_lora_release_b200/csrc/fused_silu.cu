@@ -603,8 +603,7 @@ dequant_lora_add_kernel(const RebuildJobs jobs, int64_t rows) {
 template <typename K>
 static inline dim3 wide_grid(K kern, int64_t rows, int cgroups) {
   const int64_t tiles = (rows + 15) / 16;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 2;
+  const int per_sm = resident_blocks(kern, 256, 0, 2);
   int64_t slots = ((int64_t)num_sms() * per_sm) / cgroups;
   if (slots > tiles) slots = tiles;
   if (slots < 1) slots = 1;

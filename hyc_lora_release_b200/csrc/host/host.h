@@ -56,7 +56,7 @@ Tensor topk_restore(const Tensor& val, const Tensor& col, const Tensor& q, const
                     at::IntArrayRef shape, int64_t q_bit, const OptTensor& out);
 Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
                              at::IntArrayRef shape, int64_t q_bit, const Tensor& grad, const OptTensor& out, double scale);
-Tensor prune_sparse(const Tensor& x, double thr);
+Tensor prune_sparse(const Tensor& x, double thr, const OptTensor& thr_dev);
 Tensor prune_restore(const Tensor& idx, const Tensor& val, int64_t numel);
 std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity);
 Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out);

@@ -36,6 +36,22 @@ inline int current_device_slot() {
   return dev;
 }
 
+// Resident blocks per SM of a kernel, asked of the runtime once per thread, kernel, launch shape and device (a query costs
+// one to two microseconds, as much as a launch; the lane kernels ask for four block widths): a direct-mapped table.
+template <typename K>
+inline int resident_blocks(K kern, int threads, size_t smem, int otherwise) {
+  struct Entry { const void* kern; size_t smem; int threads, device, blocks; };
+  static thread_local Entry table[128] = {};
+  const void* f = reinterpret_cast<const void*>(kern);
+  const int dev = current_device_slot();
+  Entry& e = table[((reinterpret_cast<uintptr_t>(f) >> 4) ^ (uintptr_t)(threads >> 5) * 37u ^ (uintptr_t)(smem >> 10)) & 127];
+  if (dev >= 0 && e.kern == f && e.threads == threads && e.smem == smem && e.device == dev) return e.blocks;
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess || n < 1) return otherwise;
+  e = {f, smem, threads, dev, n};
+  return n;
+}
+
 // Programmatic dependent launch: a kernel launched with launch_pdl may begin before the kernel in front of it in the
 // stream has ended, and has to call pdl_wait() before it touches memory (pdl_wait returns once that kernel, and with
 // it everything before, is complete and visible).  pdl_trigger() in the kernel in front lets the launch go out.

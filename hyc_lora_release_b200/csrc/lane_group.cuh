@@ -232,8 +232,7 @@ inline void lane_launch_shape(K kern, int64_t rows, int rows_per_warp, int& grid
   double best = -1.0;
   grid = 1; threads = 256;
   for (int w = 8; w >= 5; --w) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * w, (size_t)w * smem_per_warp) != cudaSuccess || per_sm < 1) per_sm = 1;
+    const int per_sm = resident_blocks(kern, 32 * w, (size_t)w * smem_per_warp, 1);
     const int64_t resident = (int64_t)num_sms() * per_sm * w;
     int64_t blocks = (items + w - 1) / w;
     if (blocks > (int64_t)num_sms() * per_sm) blocks = (int64_t)num_sms() * per_sm;

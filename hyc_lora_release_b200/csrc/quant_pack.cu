@@ -472,8 +472,7 @@ template <typename Kernel>
 static inline dim3 stream_grid(Kernel kern, int threads, size_t smem, int64_t rows, int n_ct, int unroll) {
   const int col_tiles = (n_ct + threads - 1) / threads;
   const int64_t groups = (rows + unroll - 1) / unroll;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 2;
+  const int per_sm = resident_blocks(kern, threads, smem, 2);
   int64_t slots = ((int64_t)num_sms() * per_sm) / col_tiles;
   if (slots > groups) slots = groups;
   if (slots < 1) slots = 1;

@@ -69,10 +69,10 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int& total) {
 // (four loads in flight per lane and 32 registers: all 64 warp slots of an SM are taken, one wave for 9472 tiles)
 template <bool NEG>
 __global__ void __launch_bounds__(kTileThreads, 8)
-prune_count_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, int64_t n_tiles,
+prune_count_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, const float* __restrict__ thr_dev, int64_t n_tiles,
                    int64_t* __restrict__ ws) {
   constexpr int CB = 4;
-  const __nv_bfloat162 t2 = __float2bfloat162_rn(thr);
+  const __nv_bfloat162 t2 = __float2bfloat162_rn(thr_dev ? *thr_dev : thr);
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   for (int64_t tile = warp0; tile < n_tiles; tile += (int64_t)gridDim.x * kWarpsPerBlock) {
@@ -159,11 +159,11 @@ constexpr int kFillTrips = 4;
 
 template <bool NEG>
 __global__ void __launch_bounds__(kTileThreads, 4)
-prune_fill_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, int64_t n_tiles,
+prune_fill_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, const float* __restrict__ thr_dev, int64_t n_tiles,
                   const int64_t* __restrict__ ws, int64_t* __restrict__ idx_out,
                   __nv_bfloat16* __restrict__ val_out, int64_t capacity) {
   __shared__ uint32_t s_stage[kWarpsPerBlock][256 * kFillTrips];
-  const __nv_bfloat162 t2 = __float2bfloat162_rn(thr);
+  const __nv_bfloat162 t2 = __float2bfloat162_rn(thr_dev ? *thr_dev : thr);
   const int lane = threadIdx.x & 31;
   uint32_t* stage = s_stage[threadIdx.x >> 5];
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -481,15 +481,16 @@ static inline float thr_bf16(float t) {
   return r;
 }
 
-// thr is the bf16-rounded threshold; a negative one (or NaN) takes the kernels that also test for zero
-static inline void launch_count(const __nv_bfloat16* a, int64_t numel, float thr, int64_t nt, int64_t* ws, cudaStream_t st) {
-  if (thr >= 0.f) prune_count_kernel<false><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nt, ws);
-  else prune_count_kernel<true><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nt, ws);
+// thr is the bf16-rounded threshold; a negative one (or NaN), and one that only the device knows, takes the kernels that also
+// test for zero
+static inline void launch_count(const __nv_bfloat16* a, int64_t numel, float thr, const float* thr_dev, int64_t nt, int64_t* ws, cudaStream_t st) {
+  if (thr >= 0.f && !thr_dev) prune_count_kernel<false><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nullptr, nt, ws);
+  else prune_count_kernel<true><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, thr_dev, nt, ws);
 }
-static inline void launch_fill(const __nv_bfloat16* a, int64_t numel, float thr, int64_t nt, const int64_t* ws,
+static inline void launch_fill(const __nv_bfloat16* a, int64_t numel, float thr, const float* thr_dev, int64_t nt, const int64_t* ws,
                                int64_t* idx_out, __nv_bfloat16* val_out, int64_t capacity, cudaStream_t st) {
-  if (thr >= 0.f) prune_fill_kernel<false><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nt, ws, idx_out, val_out, capacity);
-  else prune_fill_kernel<true><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nt, ws, idx_out, val_out, capacity);
+  if (thr >= 0.f && !thr_dev) prune_fill_kernel<false><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nullptr, nt, ws, idx_out, val_out, capacity);
+  else prune_fill_kernel<true><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, thr_dev, nt, ws, idx_out, val_out, capacity);
 }
 
 }  // namespace hyc
@@ -501,34 +502,51 @@ extern "C" HYC_API size_t hyc_softmax_prune_workspace_bytes(int64_t numel) {
   return (size_t)(1 + n_tiles_of(numel)) * sizeof(int64_t);
 }
 
-extern "C" HYC_API int hyc_softmax_prune_count(const void* a, int64_t numel, float threshold,
-                                       void* workspace, size_t workspace_bytes, void* stream) {
+static int prune_count(const void* a, int64_t numel, float thr, const float* thr_dev, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   if (!a || !workspace) return HYC_ERR_NULL;
   if (numel <= 0) return HYC_ERR_SHAPE;
   if (!aligned(a, 16) || !aligned(workspace, 8)) return HYC_ERR_ALIGN;
   if (workspace_bytes < hyc_softmax_prune_workspace_bytes(numel)) return HYC_ERR_WORKSPACE;
   const int64_t nt = n_tiles_of(numel);
-  cudaStream_t st = (cudaStream_t)stream;
-  launch_count((const __nv_bfloat16*)a, numel, thr_bf16(threshold), nt, (int64_t*)workspace, st);
+  launch_count((const __nv_bfloat16*)a, numel, thr, thr_dev, nt, (int64_t*)workspace, st);
   HYC_CHECK_LAUNCH();
   prune_scan_kernel<<<1, 1024, 0, st>>>((int64_t*)workspace, nt, nullptr);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
-
-extern "C" HYC_API int hyc_softmax_prune_fill(const void* a, int64_t numel, float threshold,
-                                      const void* workspace, int64_t* idx_out, void* val_out,
-                                      int64_t capacity, void* stream) {
+static int prune_fill(const void* a, int64_t numel, float thr, const float* thr_dev, const void* workspace, int64_t* idx_out, void* val_out,
+                      int64_t capacity, cudaStream_t st) {
   if (!a || !workspace) return HYC_ERR_NULL;
   if (capacity > 0 && (!idx_out || !val_out)) return HYC_ERR_NULL;
   if (numel <= 0 || capacity < 0) return HYC_ERR_SHAPE;
   if (!aligned(a, 16) || !aligned(workspace, 8)) return HYC_ERR_ALIGN;
   if (capacity == 0) return HYC_OK;
   const int64_t nt = n_tiles_of(numel);
-  launch_fill((const __nv_bfloat16*)a, numel, thr_bf16(threshold), nt, (const int64_t*)workspace, idx_out,
-              (__nv_bfloat16*)val_out, capacity, (cudaStream_t)stream);
+  launch_fill((const __nv_bfloat16*)a, numel, thr, thr_dev, nt, (const int64_t*)workspace, idx_out, (__nv_bfloat16*)val_out, capacity, st);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
+}
+
+extern "C" HYC_API int hyc_softmax_prune_count(const void* a, int64_t numel, float threshold,
+                                       void* workspace, size_t workspace_bytes, void* stream) {
+  return prune_count(a, numel, thr_bf16(threshold), nullptr, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+extern "C" HYC_API int hyc_softmax_prune_count_dev(const void* a, int64_t numel, const float* threshold,
+                                                   void* workspace, size_t workspace_bytes, void* stream) {
+  if (!threshold) return HYC_ERR_NULL;
+  return prune_count(a, numel, 0.f, threshold, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+extern "C" HYC_API int hyc_softmax_prune_fill(const void* a, int64_t numel, float threshold,
+                                      const void* workspace, int64_t* idx_out, void* val_out,
+                                      int64_t capacity, void* stream) {
+  return prune_fill(a, numel, thr_bf16(threshold), nullptr, workspace, idx_out, val_out, capacity, (cudaStream_t)stream);
+}
+extern "C" HYC_API int hyc_softmax_prune_fill_dev(const void* a, int64_t numel, const float* threshold,
+                                                  const void* workspace, int64_t* idx_out, void* val_out,
+                                                  int64_t capacity, void* stream) {
+  if (!threshold) return HYC_ERR_NULL;
+  return prune_fill(a, numel, 0.f, threshold, workspace, idx_out, val_out, capacity, (cudaStream_t)stream);
 }
 
 extern "C" HYC_API int hyc_softmax_prune_restore(const int64_t* idx, const void* val, int64_t nnz,
@@ -681,12 +699,12 @@ extern "C" HYC_API int hyc_softmax_prune_static(const void* a, int64_t numel, fl
   if (!ws) { hyc_set_last_cuda_error(err); return HYC_ERR_LAUNCH; }
   cudaStream_t st = (cudaStream_t)stream;
   const float thr = thr_bf16(threshold);
-  launch_count((const __nv_bfloat16*)a, numel, thr, nt, ws, st);
+  launch_count((const __nv_bfloat16*)a, numel, thr, nullptr, nt, ws, st);
   HYC_CHECK_LAUNCH();
   prune_scan_kernel<<<1, 1024, 0, st>>>(ws, nt, nnz_out);
   HYC_CHECK_LAUNCH();
   if (capacity > 0) {
-    launch_fill((const __nv_bfloat16*)a, numel, thr, nt, ws, idx_out, (__nv_bfloat16*)val_out, capacity, st);
+    launch_fill((const __nv_bfloat16*)a, numel, thr, nullptr, nt, ws, idx_out, (__nv_bfloat16*)val_out, capacity, st);
     HYC_CHECK_LAUNCH();
   }
   return HYC_OK;

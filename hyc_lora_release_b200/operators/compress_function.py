@@ -190,6 +190,8 @@ def compression_softmax(x: torch.Tensor, outlier):
     of the flattened map (int64 indices, values in x's dtype), built by a two-phase stream
     compaction.  One device-to-host copy of the count sizes the result, as in ``to_sparse``."""
     require_cuda(x)
+    if isinstance(outlier, torch.Tensor) and outlier.device == x.device and outlier.numel() == 1:
+        return host.prune_sparse(x, 0.0, outlier)
     return host.prune_sparse(x, float(outlier))
 
 

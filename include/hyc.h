@@ -140,6 +140,12 @@ int hyc_softmax_prune_tiled(const void* a, int64_t numel, float threshold,
 int hyc_softmax_prune_tiled_restore(const uint32_t* words, int64_t capacity, const void* directory,
                                     void* a_out, int64_t numel, void* stream);
 
+/* hyc_softmax_prune_count / _fill with the threshold read from device memory (fp32, rounded to bf16 like the other form): a
+ * calibrated threshold that lives on the device needs no copy to the host first. */
+int hyc_softmax_prune_count_dev(const void* a, int64_t numel, const float* threshold, void* workspace, size_t workspace_bytes, void* stream);
+int hyc_softmax_prune_fill_dev(const void* a, int64_t numel, const float* threshold, const void* workspace,
+                               int64_t* idx_out, void* val_out, int64_t capacity, void* stream);
+
 /* *flag += 1 if *nnz > capacity (entries of a fixed-capacity save were dropped). */
 int hyc_prune_overflow_flag(const int64_t* nnz, int64_t capacity, int* flag, void* stream);
 

@@ -163,6 +163,16 @@ def test_topk_ties_lane_layout(cf, S, rows):
             assert torch.equal(m.to_dense().cpu(), oracle.topk_decompress(vals, cols, pk, sc, zp, q, x.shape))
 
 
+@pytest.mark.parametrize("thr,dtype", [(0.01, torch.float32), (0.0100001, torch.bfloat16), (-0.5, torch.float32), (0.0, torch.float64)])
+def test_prune_with_the_threshold_on_the_device(cf, thr, dtype):
+    """A threshold tensor on the map's device is read by the kernels; same list as with the number, whatever its dtype."""
+    a = _softmax_map(1, 3, 136, seed=11)
+    t = torch.tensor(thr, dtype=dtype)
+    idx, val = oracle.ref_softmax_prune(a, t)
+    sp = cf.compression_softmax(a.to(DEV), t.to(DEV))
+    assert torch.equal(sp.indices().reshape(-1).cpu(), idx) and torch.equal(sp.values().cpu(), val)
+
+
 @pytest.mark.parametrize("S,rows", [(192, 37), (320, 11), (448, 5), (576, 9), (960, 4), (1088, 3), (1984, 2)])
 def test_topk_rows_of_other_group_counts(cf, S, rows):
     """Rows whose groups are not a power of two share the lanes of the next one: least and most idle lanes of every lane count, a
