@@ -55,6 +55,7 @@ SIGNATURES = {
     "hyc_fused_lora_silu_hadamard_bwd": (_i, [_p] * 12 + [_l, _i, _i, _i, _p]),
     "hyc_softmax_prune_count_dev": (_i, [_p, _l, _p, _p, _z, _p]),
     "hyc_softmax_prune_fill_dev": (_i, [_p, _l, _p, _p, _p, _p, _l, _p]),
+    "hyc_dequant_nf4_many": (_i, [_i, _p, _p]),
     "hyc_prune_overflow_flag": (_i, [_p, _l, _p, _p]),
     "hyc_rebuild_qkv": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _l, _i, _l, _i, _i, _p]),
     "hyc_rope_pair": (_i, [_p, _i, _p, _i, _p, _p, _l, _i, _l, _i, _i, _i, _p]),

@@ -99,12 +99,42 @@ Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64
   return out;
 }
 
+// a frozen projection: a bf16 matrix, or 4-bit codes that become one for the product that uses it
+struct FrozenWeight {
+  Tensor plain;
+  Tensor packed, code, absmax;
+  OptTensor code2, absmax2;
+  int64_t blocksize2 = 1, blocksize = 64;
+  double offset = 0;
+  std::vector<int64_t> shape;
+};
+// the matrices of up to four weights, one launch for all that are codes.  Called directly before the product that reads them:
+// what fits of the matrices is then still in L2
+static std::vector<Tensor> matrices(std::initializer_list<const FrozenWeight*> ws) {
+  std::vector<Tensor> out;
+  hyc_nf4_job jobs[4] = {};
+  int n = 0;
+  for (const FrozenWeight* f : ws) {
+    if (f->plain.defined()) { out.push_back(f->plain); continue; }
+    out.push_back(empty(f->shape, f->packed));
+    const bool nested = given(f->code2);
+    jobs[n++] = {data(f->packed), (const float*)data(f->code), nested ? nullptr : (const float*)data(f->absmax),
+                 nested ? (const uint8_t*)data(f->absmax) : nullptr, (const float*)data(f->code2), (const float*)data(f->absmax2),
+                 data(out.back()), out.back().numel(), (int)f->blocksize, (int)f->blocksize2, (float)f->offset};
+  }
+  if (n) {
+    OnDevice on(out[0]);
+    check(hyc_dequant_nf4_many(n, jobs, on.stream), "hyc_dequant_nf4_many");
+  }
+  return out;
+}
+
 // ------------------------------------------------------------------ MLP half
 struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa, down_xa64; };
 
 static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
-                                       const OptTensor& bias_d, int64_t q, double eps, const Tensor& status) {
-  const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &wd = w[3], &bg = w[4], &bu = w[5], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
+                                       const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const FrozenWeight* wd_later = nullptr) {
+  const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &bg = w[4], &bu = w[5], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
   const Tensor gs = vec(stats[3]), us = vec(stats[4]);
   require_cuda({&x_medium, &wg});
@@ -119,7 +149,7 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
                                    data(gs), data(us), data(q1), data(q2), data(had), nullptr, nullptr, (int)q, status_ptr(status), on.stream),
         "hyc_mlp_gateup_fwd_tcgen05");
   const Tensor down_xa64 = at::mm(had, ad_cols);
-  const Tensor res = bf16c(x_medium);
+  const Tensor res = bf16c(x_medium), wd = wd_later ? matrices({wd_later})[0] : w[3];
   Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, false, &res, status);
   if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
   return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
@@ -384,19 +414,6 @@ static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads,
 // dictionary look-ups, argument conversion), which cost more than the kernels of a short sequence run for.
 // 128 tokens, Llama-2-7B, bf16 weights, host work per forward + backward: 863 us as ten calls.
 
-// a frozen projection: a bf16 matrix, or 4-bit codes that become one for the half of the pass that uses it
-struct FrozenWeight {
-  Tensor plain;
-  Tensor packed, code, absmax;
-  OptTensor code2, absmax2;
-  int64_t blocksize2 = 1, blocksize = 64;
-  double offset = 0;
-  std::vector<int64_t> shape;
-  Tensor get() const {
-    return plain.defined() ? plain : dequant_nf4(packed, code, absmax, code2, absmax2, blocksize2, offset, blocksize, shape);
-  }
-};
-
 enum { PQ, PK, PV, PO, PGATE, PUP, PDOWN, PROJECTIONS };
 enum { AQKV_T, AQKV_ROWS, AO_COLS, AO_ROWS, BO_COLS, AGU_T, AGU_ROWS, AD_ROWS, AD_COLS, BD_COLS, PADS };
 
@@ -481,9 +498,11 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
   {
     Tensor a, o2;
     OptTensor o_codes;
+    std::vector<Tensor> w = matrices({&p.w[PQ], &p.w[PK], &p.w[PV]});
     std::tie(a, o2, s->rstd, s->x_o, s->x_q, s->xn_q, s->q_q, s->k_q, s->v_q, s->xa3, o_codes, s->cls, s->cls_b, s->cls_h) = attn_forward_map(
-        x, {p.norm1, p.w[PQ].get(), p.w[PK].get(), p.w[PV].get(), p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
+        x, {p.norm1, w[0], w[1], w[2], p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
         {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status);
+    w.clear();
     if (map_q > 0) {
       auto [val, col, q, sc, z] = topk_compress(a, map_k, map_q);
       s->map = {val, col, q, sc, z};
@@ -492,12 +511,13 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
       s->map = {words, directory, nnz};
     }
     a.reset();
-    auto out = attn_forward_out(x, o2, p.w[PO].get(), p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
+    auto out = attn_forward_out(x, o2, matrices({&p.w[PO]})[0], p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
     x_medium = out[0]; s->o_q = out[1]; s->o_xa64 = out[2];
   }
-  s->mlp = mlp_forward(x_medium, {p.norm2, p.w[PGATE].get(), p.w[PUP].get(), p.w[PDOWN].get(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
+  std::vector<Tensor> w = matrices({&p.w[PGATE], &p.w[PUP]});
+  s->mlp = mlp_forward(x_medium, {p.norm2, std::move(w[0]), std::move(w[1]), Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
                                   p.pad[AGU_T], p.pad[AD_COLS], p.pad[BD_COLS]},
-                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status);
+                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, &p.w[PDOWN]);
   Tensor y = std::move(s->mlp.x_out);
   s->mlp.x_out = Tensor();
   return {y.to(s->x_type), s};
@@ -527,19 +547,20 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   {
     const Tensor g = bf16c(grad_y).view({T, s.H});
     const MlpForward& m = s.mlp;
-    auto r = mlp_backward_lora(g, {p.w[PDOWN].get(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
+    auto r = mlp_backward_lora(g, {matrices({&p.w[PDOWN]})[0], p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
                                {m.q1, m.gs, m.q2, m.us, m.gu_xa, m.down_xa64, m.xn_q, st[XN2_SCALE]}, s.q_mlp, status);
     lora(PGATE, r[5].narrow(0, 0, 16), r[6].select(0, 0));
     lora(PUP, r[5].narrow(0, 16, 16), r[6].select(0, 1));
     lora(PDOWN, r[4], r[3]);
     report({{"g", PGATE}, {"u", PUP}, {"d", PDOWN}});
     r[0].reset();
-    g_medium = mlp_backward_x(g, r[1], r[2], {p.w[PGATE].get(), p.w[PUP].get(), p.pad[AGU_ROWS], p.norm2},
+    const std::vector<Tensor> w = matrices({&p.w[PGATE], &p.w[PUP]});
+    g_medium = mlp_backward_x(g, r[1], r[2], {w[0], w[1], p.pad[AGU_ROWS], p.norm2},
                               {m.xm_q, st[XM_SCALE], m.xm_o, st[XM_IDX], m.rstd}, shape, s.q_mlp, status).view({T, s.H});
   }
   std::vector<Tensor> grads;
   {
-    auto r = attn_backward_out(g_medium, p.w[PO].get(), p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
+    auto r = attn_backward_out(g_medium, matrices({&p.w[PO]})[0], p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
     lora(PO, r[1], r[0]);
     const std::vector<int64_t> a_shape = {s.B, s.nh, s.M, s.M};
     const bool topk = s.map_q > 0;
@@ -555,7 +576,8 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   auto r = attn_backward_lora(grads, {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.xa3, s.xn_q, st[XN1_SCALE], s.q_attn, status);
   for (int i = 0; i < 3; ++i) lora(PQ + i, r[1].narrow(0, 16 * i, 16), r[2 + i]);
   report({{"q", PQ}, {"k", PK}, {"v", PV}, {"o", PO}});
-  out[0] = attn_backward_x(g_medium, grads, r[0], {p.w[PQ].get(), p.w[PK].get(), p.w[PV].get(), p.pad[AQKV_ROWS], p.norm1},
+  const std::vector<Tensor> w = matrices({&p.w[PQ], &p.w[PK], &p.w[PV]});
+  out[0] = attn_backward_x(g_medium, grads, r[0], {w[0], w[1], w[2], p.pad[AQKV_ROWS], p.norm1},
                            {s.x_q, st[X_SCALE], s.x_o, st[X_IDX], s.rstd}, shape, s.q_attn, status).to(s.x_type);
   return out;
 }

@@ -294,6 +294,19 @@ int hyc_dequant_nf4(const void* packed, const float* code16, const float* absmax
                     const uint8_t* absmax_q, const float* code256, const float* absmax2,
                     int blocksize2, float offset, int64_t numel, int blocksize, void* out, void* stream);
 
+/* The same for up to four weights in one launch. */
+typedef struct hyc_nf4_job {
+  const void* packed;
+  const float *code16, *absmax;      /* absmax NULL: double quantization */
+  const uint8_t* absmax_q;
+  const float *code256, *absmax2;
+  void* out;
+  int64_t numel;
+  int blocksize, blocksize2;
+  float offset;
+} hyc_nf4_job;
+int hyc_dequant_nf4_many(int count, const hyc_nf4_job* jobs, void* stream);
+
 /* ---- tcgen05 / TMEM GEMMs of the LoRA MLP (activation compression in the epilogue) ------------
  * bf16 operands, fp32 accumulation in tensor memory, operands staged by TMA.  `status` is a
  * caller-provided device int, zero before the call; a non-zero value afterwards means a bounded
