@@ -603,11 +603,7 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
 static int choose_wide(int tiles_m, int columns, int units) {
   int best = columns;
   float best_cost = 1e30f;
-#ifdef HYC_TUNE
-  const float half = getenv("HYC_HALF") ? (float)atof(getenv("HYC_HALF")) : 0.68f;
-#else
   const float half = 0.68f;
-#endif
   for (int w = columns; w >= 0; --w) {
     const int wide = tiles_m * w, narrow = tiles_m * 2 * (columns - w);
     const int rounds = wide / units, rest = wide % units;            // the first `rest` workers have one wide tile more
@@ -666,9 +662,6 @@ static int launch_as(const Operands& ops, const Params& p, cudaStream_t st) {
   // half-width tiles only: the B part of a stage is half as big and the ring has more stages
   pp.stage_bytes = STAGE_A_BYTES + Geo<PAIR>::STAGE_B_BYTES / (pp.n_wide == 0 ? 2 : 1);
   pp.stages = PIPE_BYTES / pp.stage_bytes < MAX_STAGES ? PIPE_BYTES / pp.stage_bytes : MAX_STAGES;
-#ifdef HYC_TUNE
-  if (getenv("HYC_STAGES")) pp.stages = atoi(getenv("HYC_STAGES"));
-#endif
   const int tiles = tiles_m * (pp.n_wide + 2 * (columns - pp.n_wide));
   cfg.gridDim = dim3((unsigned)((PAIR ? 2 : 1) * (tiles < units ? tiles : units)));
 #ifdef HYC_TC_PROF
@@ -689,9 +682,6 @@ static int launch(const Operands& ops, const Params& p, cudaStream_t st) {
   if (plan.split > 0) return launch_split(EPI, QBIT, B_MN, plan, ops, p, st);
   // pairs, except where few rows would leave half of the tile empty
   bool pair = p.M > BM;
-#ifdef HYC_TUNE
-  if (const char* e = getenv("HYC_SPLIT")) { int v = atoi(e); if (v >= 200) pair = v >= 300; }
-#endif
   return pair ? launch_as<EPI, QBIT, B_MN, true>(ops, p, st) : launch_as<EPI, QBIT, B_MN, false>(ops, p, st);
 }
 

@@ -755,12 +755,6 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-#ifdef HYC_TUNE
-#include <stdlib.h>
-#define HYC_PROMO (getenv("HYC_P256") ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B)
-#else
-#define HYC_PROMO CU_TENSOR_MAP_L2_PROMOTION_L2_128B
-#endif
 inline EncodeTiledFn get_encode() {
   // the encoder is a driver function: a thread whose first CUDA work is this call has no context current yet (the
   // runtime binds the device's primary context, once per thread)
@@ -790,7 +784,7 @@ inline bool make_map(CUtensorMap* m, const void* ptr, int64_t rows, int64_t cols
   cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1u, 1u};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, HYC_PROMO,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

@@ -343,9 +343,6 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
 // together (with 2-bit codes one that flips moves a value by a third of its range).  That leaves 5 us on the o projection.
 SplitPlan choose_split(int epi, bool b_mn, const Params& p) {
   SplitPlan plan = {0, false};
-#ifdef HYC_TUNE
-  if (const char* e = getenv("HYC_SPLIT")) { if (atoi(e) >= 100) return plan; plan.split = atoi(e) % 10; plan.pair = atoi(e) >= 10; return plan; }
-#endif
   if (epi == EPI_GRADDOWN || p.M > 2 * BM) return plan;
   if (epi == EPI_STORE && p.l1.bt != nullptr) return plan;         // a second LoRA term: the persistent kernel's own epilogue
   const int tiles = p.N / (epi == EPI_GATEUP ? SBN / 2 : SBN), sms = num_sms();

@@ -67,3 +67,54 @@ def test_projections_in_one_launch(T, ns):
         assert bool(((y.double() - main - lora).abs() <= bound).all())
         flips = ((codes ^ q1) != 0).double().mean()
         assert float(flips) < 2e-3 and bool(((y.double() - y1.double()).abs() <= 2 * bound).all())
+
+
+def _lora_b(g, n, transposed):
+    """-> (the [n, 16] factor, the tensor that is passed, its column stride, its rank stride)"""
+    b = _rn(g, n, 16, scale=0.3)
+    if transposed:
+        t = b.t().contiguous()
+        return b, t, 1, n
+    return b, b, 16, 1
+
+
+@pytest.mark.parametrize("T", [129, 256, 300, 700, 1500])
+@pytest.mark.parametrize("I,q,transposed", [(256, 4, False), (1280, 2, True), (2816, 8, False)])
+def test_lora_terms_of_the_pair_form(T, I, q, transposed):
+    """Gate/up forward and grad_down backward with LoRA terms as large as the main branches (a term in the wrong row or
+    column is an error of the order of the result), wide and half-width tiles, a ragged last row block, both layouts of B.
+    Forward and backward round to bf16 at most eight times on the way from exact products, each at most 2^-8 of the value:
+    2-norm of the difference below 8 * 2^-8 of the result's."""
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(T + I)
+    H = 512
+    x, wg, wu = _rn(g, T, H), _rn(g, I, H, scale=0.04), _rn(g, I, H, scale=0.04)
+    xa1, xa2 = _rn(g, T, 16), _rn(g, T, 16)
+    (b1, p1, c1, r1), (b2, p2, c2, r2) = _lora_b(g, I, transposed), _lora_b(g, I, transposed)
+    s = torch.full((I,), 0.25 if q > 2 else 1.0, dtype=BF16, device=DEV)
+    q1, q2 = (torch.zeros(T, I * q // 8, dtype=torch.uint8, device=DEV) for _ in range(2))
+    o, m1, m2, had, gg, gu = (torch.full((T, I), float("nan"), dtype=BF16, device=DEV) for _ in range(6))
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    check(lib.hyc_mlp_gateup_fwd_tcgen05(ptr(x), ptr(wg), ptr(wu), T, H, I, ptr(xa1), ptr(p1), c1, r1, ptr(xa2), ptr(p2), c2, r2, ptr(s), ptr(s),
+                                         ptr(q1), ptr(q2), ptr(o), ptr(m1), ptr(m2), q, ptr(st), stream_of(x)), "gateup")
+    assert int(st.item()) == 0
+
+    def near(got, want):
+        assert float((got.double() - want).norm()) <= 8 * 2.0 ** -8 * float(want.norm())
+    l1, l2 = xa1.double() @ b1.double().t(), xa2.double() @ b2.double().t()
+    near(m1, x.double() @ wg.double().t())
+    near(m2, x.double() @ wu.double().t())
+    near(o, torch.nn.functional.silu(m1.double() + l1) * (m2.double() + l2))
+
+    wd, gy = _rn(g, H, I, scale=0.04), _rn(g, T, H)
+    from hyc_lora_release_b200.operators import compress_function as cf
+    d1, d2 = (cf.decompression_dequantization(c.view(1, T, -1), s.view(1, 1, -1), q).view(T, I).double() for c in (q1, q2))
+    check(lib.hyc_mlp_graddown_bwd_tcgen05(ptr(gy), ptr(wd), T, H, I, None, None, 0, ptr(xa1), ptr(p1), c1, r1, ptr(xa2), ptr(p2), c2, r2,
+                                           ptr(q1), ptr(s), ptr(q2), ptr(s), None, None, 0, ptr(had), ptr(gg), ptr(gu), q, ptr(st),
+                                           stream_of(x)), "graddown")
+    assert int(st.item()) == 0
+    y1, y2, gd = d1 + l1, d2 + l2, gy.double() @ wd.double()
+    sig = torch.sigmoid(y1)
+    near(had, y1 * sig * y2)
+    near(gu, gd * y1 * sig)
+    near(gg, gd * y2 * sig * (1 + y1 * (1 - sig)))
