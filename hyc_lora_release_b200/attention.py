@@ -6,18 +6,19 @@ in its grouped key/value heads, which are covered) with plain bf16 frozen weight
 
   forward : RMSNorm fused with the saves of x (outlier channels + codes) and x_norm (codes) -> q/k/v
             projections on the tcgen05 GEMM whose epilogue also packs the codes of the main branch ->
-            rotary embedding in place -> scores (library batched GEMM) -> scale + mask + softmax in one pass
-            -> save of the probability map (per-row top-k + 4-bit groups, or the reference's threshold
-            prune) -> P.V (library batched GEMM) -> save of o -> o projection with the LoRA product as one
-            more K block and the residual in the GEMM epilogue;
-  backward: o projection backward (LoRA-A gradient straight from the packed o) -> restored map -> grad_v,
-            grad_a -> restore fused with the softmax backward -> q, k rebuilt by de-quantize + LoRA re-add +
-            rotary -> grad_q, grad_k -> inverse rotary -> LoRA gradients of q/k/v (A side from the packed
-            x_norm in one pass for the three adapters) -> grad_x as ONE GEMM over the three K segments ->
-            RMSNorm backward from the packed x with the residual gradient added in the same pass.
+            rotary embedding of q and k in place -> one attention kernel from q, k, v to the probability map, o
+            and the codes of o -> save of the map (per-row top-k + 4-bit groups, or the reference's threshold
+            prune) -> o projection with the LoRA product as one more K block and the residual in the GEMM
+            epilogue;
+  backward: o projection backward (LoRA-A gradient straight from the packed o) -> q, k (rotated) and v rebuilt
+            from their codes in one launch -> restored map -> two attention kernels: softmax backward and
+            grad_q, then grad_k and grad_v -> inverse rotary -> LoRA gradients of q/k/v (A side from the packed
+            x_norm in one pass for the three adapters) -> grad_x as ONE GEMM over four K segments -> RMSNorm
+            backward from the packed x with the residual gradient added in the same pass.
+Head sizes other than 128 and sequences that are no multiple of 8 take library batched products for the attention part.
 
 Weights use the nn.Linear layout ([out, in]); LoRA factors are ``lora_A.weight`` [r, in] and
-``lora_B.weight`` [out, r].  The two batched attention products are plain library GEMMs (torch.matmul).
+``lora_B.weight`` [out, r].
 """
 import math
 from dataclasses import dataclass, field

@@ -24,6 +24,9 @@
 //   warps 2..9  : epilogue (both CTAs).  Warp w reads TMEM lanes 32*(w%4).. (tcgen05.ld 32x32b.x32) for half
 //                 of the tile's columns, so the epilogue of tile i overlaps the MMAs of tile i+1; when a warp
 //                 is done with an accumulator it arrives on the leader's "accumulator empty" barrier.
+// LoRA terms of the pair form: the epilogue warps first take the whole main branch of the tile into registers and report it
+// ("main read"); the MMA warp, between two k-blocks of the next tile, writes the K = 16 products xa B^T into the freed
+// columns ("LoRA full"), and the warps come back for them.  grad_down has two terms per column and does this in two rounds.
 // The B operand is either K-major ([N,K] row-major, the forward weights) or MN-major ([K,N]
 // row-major: the same weights read for the backward products, no transposed copy).
 // Every wait is bounded: when a limit is hit the kernel records a code in *status and drains; both CTAs of a
