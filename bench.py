@@ -767,11 +767,18 @@ def layer_workload(dev, dist=None, steps=80, warmup=3, graph=True):
     if graph:
         # the steady-state step (module forward + autograd backward) is a fixed launch sequence: captured once,
         # replayed without host work between the launches
+        # (autograd nodes of earlier steps that a reference cycle still holds belong to the default stream, which a
+        # capture must not touch)
+        import gc
+        args[0] = None
+        gc.collect()
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
             step(0)
         torch.cuda.current_stream().wait_stream(side)
+        args[0] = None
+        gc.collect()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             step(0)
