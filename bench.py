@@ -807,7 +807,7 @@ def layer_workload(dev, dist=None, steps=80, warmup=3, graph=False):
                     "[1,32,2048,2048] map (softmax, save, restore, softmax backward), bound by HBM, not by the tensor cores"}
 
 
-def model_workload(dev, dist=None, steps=4, warmup=3, n_layers=32, graph=True):
+def model_workload(dev, dist=None, steps=4, warmup=3, n_layers=32, graph=False):
     """One training step (forward + backward) of the whole 32-layer stack of BASELINE configs[4]: token embedding
     (vocabulary 32000, hidden 4096), 32 fused decoder layers driven through the layer module (32 heads of 128,
     intermediate 11008, LoRA rank 16 on q/k/v/o/gate/up/down, 4-bit saves, top-k map), final RMSNorm, the
