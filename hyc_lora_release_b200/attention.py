@@ -60,7 +60,8 @@ class AttnWeights:
     bias_v: Optional[torch.Tensor] = None
     bias_o: Optional[torch.Tensor] = None
 
-    def padded(self):
+    @torch.no_grad()      # as part of a graph they would keep the adapters' AccumulateGrad nodes, and with them the stream of
+    def padded(self):     # the step that made them, alive: a later step could not be captured on another stream
         """LoRA factors zero-padded to a K of 64 so that a rank-16 product rides along a GEMM as one more K block
         (rebuilt when a factor changes):
           ao_cols  [heads*d, 64]  columns 0..15 = Ao^T   (o -> padded LoRA activation of the o projection)

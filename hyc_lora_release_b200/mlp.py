@@ -115,7 +115,8 @@ class MLPWeights:
     bd: torch.Tensor       # down lora_B.weight [H, r]
     bias_d: Optional[torch.Tensor] = None    # bias of the down projection ([H] bf16) or None; no gradient
 
-    def padded(self):
+    @torch.no_grad()      # as part of a graph they would keep the adapters' AccumulateGrad nodes, and with them the stream of
+    def padded(self):     # the step that made them, alive: a later step could not be captured on another stream
         """LoRA factors zero-padded to a K of 64 so that a rank-16 product can ride along a GEMM as one more
         K block (built once per optimizer step; a few hundred KB):
           ad_rows  [64, I]  rows 0..15 = Ad            (second operand of grad_down's LoRA part, [K, N])

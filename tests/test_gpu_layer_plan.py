@@ -1,0 +1,95 @@
+"""The calibrated layer through its plan (one native call forward, one backward) on the GPU."""
+import os
+import sys
+import types
+
+import pytest
+import torch
+
+sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden"))
+from test_gpu_layer import BF16, DEV, _Holder, _base  # noqa: E402
+from test_oracle_layer import layer_problem  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+NAMES = ("q", "k", "v", "o", "gate", "up", "down")
+
+
+class Problem:
+    """A calibrated layer with its modules and inputs.  ``seed`` fixes the frozen weights and the inputs."""
+
+    def __init__(self, B=1, M=128, heads=4, kv=2, d=128, I=512, q=4, map_mode="topk", seed=5, bias=()):
+        from hyc_lora_release_b200.layer import FusedLlamaLayerIntraInterFullFuse
+        g = torch.Generator().manual_seed(seed)
+        self.geometry = heads, d, kv
+        x, p, cos, sin, mask = layer_problem(g, B, M, heads * d, heads, d, kv, I)
+        self.x, self.cos, self.sin, self.mask = x.to(DEV), cos.to(DEV), sin.to(DEV), mask.to(DEV)
+        self.gy = torch.randn(x.shape, generator=g).to(BF16).to(DEV)
+        self.norms = p["norm_w1"].to(DEV), p["norm_w2"].to(DEV)
+        self.mods = {n: (_base(p["w" + n].t().to(DEV), 0.1 * torch.ones(p["w" + n].shape[1], dtype=BF16) if n in bias else None),
+                         _Holder(p["a" + n].t().to(DEV)), _Holder(p["b" + n].t().to(DEV))) for n in NAMES}
+        self.config = types.SimpleNamespace(use_hyclora=True, iteration_threshold=2, softmax_outlier_ratio=0.05,
+                                            layernorm_outlier_ratio=0.01, q_bit=q, softmax_map_mode=map_mode)
+        self.layer = FusedLlamaLayerIntraInterFullFuse()
+        self.layer.set_hyclora_config(self.config)
+        for _ in range(2):
+            self.step()
+
+    def lora(self):
+        return [self.mods[n][j].default.weight for n in NAMES for j in (1, 2)]
+
+    def forward(self, x, layer=None, mods=None, mask=None):
+        mods = mods or self.mods
+        args = [x, self.norms[0], None, self.cos, self.sin]
+        for n in ("q", "k", "v", "o"):
+            args += list(mods[n])
+        args += [self.norms[1], None]
+        for n in ("gate", "up", "down"):
+            args += list(mods[n])
+        return (layer or self.layer)(*args, self.mask if mask is None else mask, *self.geometry)
+
+    def step(self, layer=None, x=None):
+        """-> [y, grad_x, the fourteen adapter gradients]"""
+        x = (self.x if x is None else x).detach().requires_grad_(True)
+        y = self.forward(x, layer)
+        return [y.detach(), *torch.autograd.grad(y, [x, *self.lora()], self.gy)]
+
+    def fresh_layer(self):
+        """A layer that has seen none of the earlier steps but has their statistics."""
+        from hyc_lora_release_b200.layer import FusedLlamaLayerIntraInterFullFuse
+        layer = FusedLlamaLayerIntraInterFullFuse()
+        layer.set_hyclora_config(self.config)
+        for mine, theirs in ((layer.attn_state, self.layer.attn_state), (layer.mlp_state, self.layer.mlp_state)):
+            mine.iteration = theirs.iteration
+            mine.static_value = {k: dict(v) for k, v in theirs.static_value.items()}
+        return layer
+
+
+def _same(got, want):
+    return all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
+
+
+@pytest.mark.parametrize("map_mode", ["topk", "prune"])
+@pytest.mark.parametrize("stepwise", [False, True])
+def test_step_captured_after_eager_steps(map_mode, stepwise):
+    """Eager steps on the default stream, then the capture of a step on another one: what the layer keeps between steps must
+    not tie a later step to the stream of an earlier one.  The replay on other inputs equals the eager step bit for bit."""
+    p = Problem(map_mode=map_mode)
+    p.layer.keep_saved = stepwise             # the step-wise path
+    for _ in range(3):
+        p.step()
+    torch.manual_seed(0)
+    other = torch.randn(p.x.shape, device=DEV).to(BF16)
+    want = p.step(x=other)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        p.step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    x = p.x.clone()
+    with torch.cuda.graph(graph):
+        got = p.step(x=x)
+    x.copy_(other)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert _same(got, want)
