@@ -678,7 +678,7 @@ def mlp_workload(dev, dist=None, steps=200, warmup=5, shape="llama", q_bit=4, ea
     return line
 
 
-def layer_workload(dev, dist=None, steps=80, warmup=3, graph=False):
+def layer_workload(dev, dist=None, steps=80, warmup=3, graph=True):
     """One fused decoder layer (attention + MLP) forward + backward at the Llama-2-7B geometry of BASELINE
     hidden 4096, 32 heads of 128, intermediate 11008, sequence 2048, batch 1 per GPU, causal mask,
     LoRA rank 16 on q/k/v/o/gate/up/down, saved activations 4-bit with 0.5 % outlier channels, the probability
@@ -767,18 +767,11 @@ def layer_workload(dev, dist=None, steps=80, warmup=3, graph=False):
     if graph:
         # the steady-state step (module forward + autograd backward) is a fixed launch sequence: captured once,
         # replayed without host work between the launches
-        # (autograd nodes of earlier steps that a reference cycle still holds belong to the default stream, which a
-        # capture must not touch)
-        import gc
-        args[0] = None
-        gc.collect()
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
             step(0)
         torch.cuda.current_stream().wait_stream(side)
-        args[0] = None
-        gc.collect()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             step(0)
@@ -807,7 +800,7 @@ def layer_workload(dev, dist=None, steps=80, warmup=3, graph=False):
                     "[1,32,2048,2048] map (softmax, save, restore, softmax backward), bound by HBM, not by the tensor cores"}
 
 
-def model_workload(dev, dist=None, steps=4, warmup=3, n_layers=32, graph=False):
+def model_workload(dev, dist=None, steps=4, warmup=3, n_layers=32, graph=True):
     """One training step (forward + backward) of the whole 32-layer stack of BASELINE configs[4]: token embedding
     (vocabulary 32000, hidden 4096), 32 fused decoder layers driven through the layer module (32 heads of 128,
     intermediate 11008, LoRA rank 16 on q/k/v/o/gate/up/down, 4-bit saves, top-k map), final RMSNorm, the
