@@ -526,7 +526,9 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
 // -> grad_x and the fourteen LoRA gradients (A, B of q, k, v, o, gate, up, down).  hook: see mlp.mlp_backward
 static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad_y, LayerSaved& s, const pybind11::object& hook, const Tensor& overflow,
                                           const Tensor& status) {
-  at::AutoDispatchBelowADInplaceOrView below;
+  // the steps run below the dispatch keys of autograd and version counting, the hook above them: it is the caller's code, and
+  // an update in place that it makes has to bump the versions that fresh() goes by
+  std::optional<at::AutoDispatchBelowADInplaceOrView> below(std::in_place);
   const std::vector<Tensor>& st = s.stats;
   const int64_t T = s.B * s.M;
   const std::vector<int64_t> shape = {s.B, s.M, s.H};
@@ -541,7 +543,9 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
       d[(std::string("grad_a") + name).c_str()] = out[1 + 2 * proj];
       d[(std::string("grad_b") + name).c_str()] = out[2 + 2 * proj];
     }
+    below.reset();
     hook(d);
+    below.emplace();
   };
   Tensor g_medium;
   {

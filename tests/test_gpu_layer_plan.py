@@ -93,3 +93,23 @@ def test_step_captured_after_eager_steps(map_mode, stepwise):
     graph.replay()
     torch.cuda.synchronize()
     assert _same(got, want)
+
+
+def test_hook_that_updates_adapters_in_place():
+    """An update of the adapters inside ``on_lora_grads`` counts as one: the next step uses the new factors everywhere."""
+    p = Problem()
+    p.step()
+    seen = []
+
+    def hook(grads):
+        named = p.layer.named_lora_weights()
+        with torch.no_grad():
+            for name, grad in grads.items():
+                before = named[name]._version
+                named[name].add_(grad.reshape(named[name].shape), alpha=0.5)
+                seen.append(named[name]._version > before)
+    p.layer.on_lora_grads = hook
+    p.step()
+    p.layer.on_lora_grads = None
+    assert len(seen) == 14 and all(seen)
+    assert _same(p.step(), p.step(layer=p.fresh_layer()))
