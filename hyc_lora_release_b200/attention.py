@@ -27,7 +27,7 @@ from typing import Optional
 import torch
 
 from ._lib import host, require_cuda
-from .mlp import _status_tensor, gemm, linear_lora_save, lora_a_products
+from .mlp import _status_tensor, contents_key, gemm, linear_lora_save, lora_a_products
 from .operators import compress_function as cf
 from .operators.rmsnorm_kernels import rmsnorm_forward, rmsnorm_forward_save
 from .operators.rope_kernels import rope_inplace
@@ -71,7 +71,7 @@ class AttnWeights:
         and the transposed factors of the rank-16 products:
           aqkv_t   [3, H, r]        Aq^T, Ak^T, Av^T (x_norm @ all three in one call)"""
         ts = (self.aq, self.ak, self.av, self.ao, self.bo, self.bq, self.bk, self.bv)
-        key = tuple((t.data_ptr(), t._version) for t in ts)
+        key = contents_key(ts)
         if getattr(self, "_pad_key", None) != key:
             r, D = self.ao.shape
             H = self.bo.shape[0]
@@ -83,7 +83,7 @@ class AttnWeights:
             aqkv_t = torch.stack((self.aq.t(), self.ak.t(), self.av.t())).contiguous()      # [3, H, r]
             self._pad = dict(ao_rows=ao_rows, ao_cols=ao_rows.t().contiguous(), bo_cols=bo_cols, aqkv_rows=aqkv,
                              aqkv_t=aqkv_t)
-            self._pad_key = key
+            self._pad_key, self._pad_of = key, [t.detach() for t in ts]
         return self._pad
 
 

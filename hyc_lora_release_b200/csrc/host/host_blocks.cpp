@@ -417,11 +417,22 @@ static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads,
 enum { PQ, PK, PV, PO, PGATE, PUP, PDOWN, PROJECTIONS };
 enum { AQKV_T, AQKV_ROWS, AO_COLS, AO_ROWS, BO_COLS, AGU_T, AGU_ROWS, AD_ROWS, AD_COLS, BD_COLS, PADS };
 
-struct Stamp {                                  // a tensor as it was: the same storage, nothing written since
-  const void* p = nullptr;
+// What a tensor was: the same memory, seen the same way, nothing written since.  Holding the storage keeps its address from
+// being handed out again, so that an adapter whose `.data` was replaced cannot look unchanged.
+struct Stamp {
+  c10::Storage storage;
+  int64_t offset = 0;
   uint32_t version = 0;
-  static Stamp of(const Tensor& t) { return {t.data_ptr(), t.is_inference() ? 0u : (uint32_t)t._version()}; }
-  bool operator==(const Stamp& o) const { return p == o.p && version == o.version; }
+  at::ScalarType type = at::kBFloat16;
+  at::DimVector sizes, strides;
+  static uint32_t version_of(const Tensor& t) { return t.is_inference() ? 0u : (uint32_t)t._version(); }
+  static Stamp of(const Tensor& t) {
+    return {t.storage(), t.storage_offset(), version_of(t), t.scalar_type(), at::DimVector(t.sizes()), at::DimVector(t.strides())};
+  }
+  bool fits(const Tensor& t) const {
+    return t.storage().unsafeGetStorageImpl() == storage.unsafeGetStorageImpl() && t.storage_offset() == offset && version_of(t) == version &&
+           t.scalar_type() == type && t.sizes() == at::IntArrayRef(sizes) && t.strides() == at::IntArrayRef(strides);
+  }
 };
 
 struct LayerPlan {
@@ -440,7 +451,7 @@ struct LayerPlan {
     for (const FrozenWeight& f : w)
       if (f.plain.defined() && f.plain.scalar_type() != at::kBFloat16) return false;
     for (int i = 0; i < 2 * PROJECTIONS; ++i)
-      if (lora[i].scalar_type() != at::kBFloat16 || !(Stamp::of(lora[i]) == pad_of[i])) return false;
+      if (lora[i].scalar_type() != at::kBFloat16 || !pad_of[i].fits(lora[i])) return false;
     return true;
   }
   void set_padded(const std::vector<Tensor>& p) {
@@ -450,7 +461,7 @@ struct LayerPlan {
   }
   void set_stats(const std::vector<Tensor>& s) {
     bool same = s.size() == stats_in.size();
-    for (size_t i = 0; same && i < s.size(); ++i) same = s[i].unsafeGetTensorImpl() == stats_in[i].unsafeGetTensorImpl() && Stamp::of(s[i]) == stats_of[i];
+    for (size_t i = 0; same && i < s.size(); ++i) same = s[i].unsafeGetTensorImpl() == stats_in[i].unsafeGetTensorImpl() && stats_of[i].fits(s[i]);
     if (same) return;
     stats_in = s;
     stats.clear();

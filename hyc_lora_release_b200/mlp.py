@@ -100,6 +100,12 @@ def lora_grad_a(q, scale, gm, r2, q_bit):
     return host.lora_grad_a(q, scale, gm, r2, q_bit)
 
 
+def contents_key(tensors):
+    """Equal keys: the tensors hold what they held, as long as an alias of each is kept beside the key (``_pad_of`` of the
+    weight records; without it another tensor's storage may come to lie at the old address)."""
+    return tuple((t.data_ptr(), t._version, t.shape, t.stride(), t.dtype) for t in tensors)
+
+
 @dataclass
 class MLPWeights:
     """Frozen bf16 weights ([out, in]) and LoRA factors of one MLP."""
@@ -125,7 +131,8 @@ class MLPWeights:
           agu_rows [64, H]  rows 0..15 = Ag, 16..31 = Au (second operand of grad_x's LoRA part, [K, N])
         and the transposed factors of the rank-16 products:
           agu_t    [2, H, r]  Ag^T, Au^T  (x_norm @ both in one call)"""
-        key = tuple(t._version for t in (self.ag, self.au, self.ad, self.bd, self.bg, self.bu))
+        ts = (self.ag, self.au, self.ad, self.bd, self.bg, self.bu)
+        key = contents_key(ts)
         if getattr(self, "_pad_key", None) != key:
             r, I = self.ad.shape
             H = self.bd.shape[0]
@@ -136,7 +143,7 @@ class MLPWeights:
             agu_t = torch.stack((self.ag.t(), self.au.t())).contiguous()      # [2, H, r]
             self._pad = dict(ad_rows=ad_rows, ad_cols=ad_rows.t().contiguous(), bd_cols=bd_cols, agu_rows=agu_rows,
                              agu_t=agu_t)
-            self._pad_key = key
+            self._pad_key, self._pad_of = key, [t.detach() for t in ts]
         return self._pad
 
 

@@ -92,7 +92,7 @@ class QuantizedWeight:
         return host.dequant_nf4(self.packed, self.code, self.absmax, None, None, 1, 0.0, self.blocksize, self.shape)
 
 
-_CACHE_ATTRS = ("_pad", "_pad_key")      # what AttnWeights / MLPWeights keep between steps
+_CACHE_ATTRS = ("_pad", "_pad_key", "_pad_of")      # what AttnWeights / MLPWeights keep between steps
 
 
 def materialize(record):

@@ -31,3 +31,48 @@ def test_padded_factors_are_no_part_of_a_graph(bound):
     for record in (aw, mw):
         for name, t in record.padded().items():
             assert not t.requires_grad and t.grad_fn is None, name
+
+
+def _padded(layer):
+    return {**layer._weights[1].padded(), **layer._weights[2].padded()}
+
+
+@pytest.mark.parametrize("change", ["data", "in place", "view"])
+def test_padded_factors_follow_the_adapters(bound, change):
+    """A record bound after the change is the measure: ``.data`` replaced (the version stays), written in place (the storage
+    stays), another view of the same storage (both stay)."""
+    from hyc_lora_release_b200.layer import FusedLlamaLayerIntraInterFullFuse
+    layer, bind, mods = bound
+    bind()
+    before = {k: t.clone() for k, t in _padded(layer).items()}
+    for i, name in enumerate(ADAPTERS):
+        for j in (1, 2):
+            w = mods[name][j].default.weight
+            if change == "data":
+                w.data = w.data + 1 + i
+            elif change == "in place":
+                with torch.no_grad():
+                    w.add_(1 + i)
+            else:
+                w.data = w.data.as_strided(w.shape, (1, w.shape[0]))
+    assert not layer._plan.fresh()
+    bind()
+    assert layer._plan.fresh()
+    got = _padded(layer)
+    case_layer = FusedLlamaLayerIntraInterFullFuse()
+    case_layer.set_hyclora_config(layer.hyclora_config)
+    case_layer._bind(layer._weights[1].norm_w, layer._weights[2].norm_w, mods)
+    for k, t in _padded(case_layer).items():
+        assert torch.equal(got[k], t) and not torch.equal(got[k], before[k]), k
+
+
+def test_replaced_adapter_memory_is_not_handed_out_again(bound):
+    """The address of a factor identifies it only while its memory is held."""
+    layer, bind, mods = bound
+    bind()
+    ws = [mods[n][j].default.weight for n in ADAPTERS for j in (1, 2)]
+    old = {w.data_ptr() for w in ws}
+    for w in ws:
+        w.data = torch.zeros_like(w.data)
+    later = [torch.empty_like(w) for w in ws for _ in range(20)]
+    assert not old & {t.data_ptr() for t in later}
