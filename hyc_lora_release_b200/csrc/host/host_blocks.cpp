@@ -534,9 +534,10 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
   return {y.to(s->x_type), s};
 }
 
-// -> grad_x and the fourteen LoRA gradients (A, B of q, k, v, o, gate, up, down).  hook: see mlp.mlp_backward
-static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad_y, LayerSaved& s, const pybind11::object& hook, const Tensor& overflow,
-                                          const Tensor& status) {
+// -> grad_x and the fourteen LoRA gradients (A, B of q, k, v, o, gate, up, down).  hook: see mlp.mlp_backward; refresh: makes the
+// padded factors again
+static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad_y, LayerSaved& s, const pybind11::object& hook,
+                                          const pybind11::object& refresh, const Tensor& overflow, const Tensor& status) {
   // the steps run below the dispatch keys of autograd and version counting, the hook above them: it is the caller's code, and
   // an update in place that it makes has to bump the versions that fresh() goes by
   std::optional<at::AutoDispatchBelowADInplaceOrView> below(std::in_place);
@@ -572,6 +573,11 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
     const std::vector<Tensor> w = matrices({&p.w[PGATE], &p.w[PUP]});
     g_medium = mlp_backward_x(g, r[1], r[2], {w[0], w[1], p.pad[AGU_ROWS], p.norm2},
                               {m.xm_q, st[XM_SCALE], m.xm_o, st[XM_IDX], m.rstd}, shape, s.q_mlp, status).view({T, s.H});
+  }
+  if (!hook.is_none() && !p.fresh()) {           // the hook of the MLP half changed factors of this one
+    below.reset();
+    refresh();
+    below.emplace();
   }
   std::vector<Tensor> grads;
   {

@@ -99,24 +99,32 @@ class FusedLayerFunction(torch.autograd.Function):
 
 class SteadyLayerFunction(torch.autograd.Function):
     """The calibrated layer through the native host path: one call forward, one backward.  Arguments as in
-    ``FusedLayerFunction`` with the layer's plan in place of the two weight records."""
+    ``FusedLayerFunction``, the layer's plan and the two weight records it was made of as one tuple."""
 
     @staticmethod
-    def forward(ctx, x, module, plan, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, *lora):
+    def forward(ctx, x, module, bound, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, *lora):
         st = module._status_for(x.device)
-        y, saved = module._steady_forward(plan, x, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, st)
-        ctx.hyc = (saved, plan, st, module)
+        y, saved = module._steady_forward(bound[0], x, cos, sin, attention_mask, num_heads, head_dim, num_key_value_heads, st)
+        ctx.hyc = (saved, bound, st, module)
         return y
 
     @staticmethod
     def backward(ctx, grad_y):
-        saved, plan, st, module = ctx.hyc
+        saved, bound, st, module = ctx.hyc
         ctx.hyc = None
+        plan = bound[0]
         if not plan.fresh():
-            module._refresh_plan(plan)
-        grads = plan.backward(grad_y, saved, module.on_lora_grads, module._overflow, st)
+            _refresh_plan(*bound)
+        grads = plan.backward(grad_y, saved, module.on_lora_grads, lambda: _refresh_plan(*bound), module._overflow, st)
         module._after_backward()
         return (grads[0], None, None, None, None, None, None, None, None, *grads[1:])
+
+
+def _refresh_plan(plan, aw, mw):
+    """The LoRA factors of the plan's own records in the layouts of the kernels, rebuilt where one changed."""
+    a, m = aw.padded(), mw.padded()
+    plan.set_padded([a["aqkv_t"], a["aqkv_rows"], a["ao_cols"], a["ao_rows"], a["bo_cols"], m["agu_t"], m["agu_rows"], m["ad_rows"],
+                     m["ad_cols"], m["bd_cols"]])
 
 
 def _frozen(base, name):
@@ -289,14 +297,8 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
                 n1, n2, [w.native() if isinstance(w, nf4.QuantizedWeight) else host.FrozenWeight(w) for w in (wq, wk, wv, wo, wg, wu, wd)],
                 list(lora), biases["o"], biases["down"])
         if self._plan is not None:
-            self._refresh_plan(self._plan)
+            _refresh_plan(self._plan, *self._weights[1:3])
         return self._weights[1:]
-
-    def _refresh_plan(self, plan):
-        """The LoRA factors in the layouts of the kernels, rebuilt when one changed."""
-        a, m = self._weights[1].padded(), self._weights[2].padded()
-        plan.set_padded([a["aqkv_t"], a["aqkv_rows"], a["ao_cols"], a["ao_rows"], a["bo_cols"], m["agu_t"], m["agu_rows"], m["ad_rows"],
-                         m["ad_cols"], m["bd_cols"]])
 
     def _steady(self):
         """True when a call is one of the fixed launch sequence: statistics calibrated and nothing wanted of the steps between."""
@@ -347,7 +349,7 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
                     down=(down_proj_base, down_proj_lora_a, down_proj_lora_b))
         aw, mw, lora = self._bind(norm_weight_1, norm_weight_2, mods)
         if self._steady():
-            return SteadyLayerFunction.apply(input, self, self._plan, cos, sin, attention_mask, num_heads, head_dim,
+            return SteadyLayerFunction.apply(input, self, (self._plan, aw, mw), cos, sin, attention_mask, num_heads, head_dim,
                                              num_key_value_heads, *lora)
         return FusedLayerFunction.apply(input, self, aw, mw, cos, sin, attention_mask, num_heads, head_dim,
                                         num_key_value_heads, *lora)

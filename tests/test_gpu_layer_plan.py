@@ -113,3 +113,37 @@ def test_hook_that_updates_adapters_in_place():
     p.layer.on_lora_grads = None
     assert len(seen) == 14 and all(seen)
     assert _same(p.step(), p.step(layer=p.fresh_layer()))
+
+
+def test_backward_after_another_adapter_was_bound():
+    """The backward pass of a step goes by the factors of its own forward pass, also when these have changed and the layer
+    has been called with other adapters in between."""
+    def run(switch):
+        p = Problem()
+        x = p.x.detach().requires_grad_(True)
+        y = p.forward(x)
+        with torch.no_grad():
+            for w in p.lora():
+                w.mul_(1.5)
+        if switch:
+            other = {n: (m[0], _Holder(3 * m[1].default.weight), _Holder(3 * m[2].default.weight)) for n, m in p.mods.items()}
+            with torch.no_grad():
+                p.forward(p.x, mods=other)
+        return torch.autograd.grad(y, [x, *p.lora()], p.gy)
+    assert _same(run(True), run(False))
+
+
+def test_hook_of_the_mlp_half_that_changes_the_attention_half():
+    """Both paths take the attention half's factors as the hook left them."""
+    def run(stepwise):
+        p = Problem()
+        p.layer.keep_saved = stepwise
+
+        def hook(grads):
+            if "grad_ag" in grads:
+                with torch.no_grad():
+                    for w in p.lora()[:8]:
+                        w.mul_(1.5)
+        p.layer.on_lora_grads = hook
+        return p.step()
+    assert _same(run(False), run(True))
