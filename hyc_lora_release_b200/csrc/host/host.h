@@ -28,7 +28,15 @@ struct OnDevice {
   explicit OnDevice(const Tensor& t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.get_device()).stream()) {}
 };
 
-void require_cuda(std::initializer_list<const Tensor*> ts);
+void require_cuda(std::initializer_list<const Tensor*> ts);      // null entries are skipped
+// the same for what the blocks take as lists: everything that a kernel reads by its address alone (index lists are moved
+// to the device by the operators that read them)
+struct SameDevice {
+  const Tensor& first;
+  SameDevice& with(const Tensor& t) { if (t.defined() && t.scalar_type() != at::kLong) require_cuda({&first, &t}); return *this; }
+  SameDevice& with(const OptTensor& t) { return t.has_value() ? with(*t) : *this; }
+  SameDevice& with(const std::vector<Tensor>& ts) { for (const Tensor& t : ts) with(t); return *this; }
+};
 void check_q(int64_t q);
 inline const Tensor* opt(const OptTensor& t) { return t.has_value() && t->defined() ? &*t : nullptr; }
 inline bool given(const OptTensor& t) { return t.has_value() && t->defined(); }

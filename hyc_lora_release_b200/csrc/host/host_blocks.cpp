@@ -116,6 +116,7 @@ static std::vector<Tensor> matrices(std::initializer_list<const FrozenWeight*> w
   int n = 0;
   for (const FrozenWeight* f : ws) {
     if (f->plain.defined()) { out.push_back(f->plain); continue; }
+    require_cuda({&f->packed, &f->code, &f->absmax, opt(f->code2), opt(f->absmax2)});
     out.push_back(empty(f->shape, f->packed));
     const bool nested = given(f->code2);
     jobs[n++] = {data(f->packed), (const float*)data(f->code), nested ? nullptr : (const float*)data(f->absmax),
@@ -137,7 +138,7 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &bg = w[4], &bu = w[5], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
   const Tensor gs = vec(stats[3]), us = vec(stats[4]);
-  require_cuda({&x_medium, &wg});
+  SameDevice{x_medium}.with(w).with(stats).with(bias_d).with(status);
   OnDevice on(x_medium);
   const int64_t B = x_medium.size(0), M = x_medium.size(1), H = x_medium.size(2), T = B * M, I = wg.size(0);
   auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale);
@@ -150,6 +151,7 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
         "hyc_mlp_gateup_fwd_tcgen05");
   const Tensor down_xa64 = at::mm(had, ad_cols);
   const Tensor res = bf16c(x_medium), wd = wd_later ? matrices({wd_later})[0] : w[3];
+  require_cuda({&x_medium, &wd});
   Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, false, &res, status);
   if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
   return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
@@ -162,6 +164,7 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<
   const Tensor bg = w[1].contiguous(), bu = w[2].contiguous(), bd = w[3].contiguous();
   const Tensor &gate_q = saved[0], &gate_s = saved[1], &up_q = saved[2], &up_s = saved[3], &gu_xa = saved[4], &down_xa = saved[5],
                &xn_q = saved[6], &xn_scale = saved[7];
+  SameDevice{g}.with(w).with(saved).with(status);
   OnDevice on(g);
   const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
   Tensor grad_bd = empty({H, 16}, g), gdm64 = empty({T, 64}, g), gm64 = empty({T, 64}, g), grad_ad = empty({16, I}, g),
@@ -185,6 +188,7 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<
 static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
                              at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wg = w[0], &wu = w[1], &agu_rows = w[2], &norm_w = w[3];
+  SameDevice{g}.with(ggu).with(gm64).with(w).with(saved).with(status);
   const Tensor g0 = ggu[0], g1 = ggu[1];
   Tensor grad_xn = gemm({{&g0, &wg}, {&g1, &wu}, {&gm64, &agu_rows}}, true, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
@@ -244,7 +248,6 @@ RopeTables rope_tables(const Tensor& cos_in, const Tensor& sin_in, int64_t seq, 
 // q and k (contiguous [rows, heads*d]) in place
 static void rope_pair(const Tensor& q, int64_t nh, const Tensor& k, int64_t nkv, const RopeTables& t, int64_t seq, int64_t d, bool backward,
                       void* stream) {
-  require_cuda({&q, &k, &t.cos, &t.sin});
   check(hyc_rope_pair(data(q), (int)nh, data(k), (int)nkv, data(t.cos), data(t.sin), t.cos.stride(0), t.f32(), q.size(0), (int)seq, (int)d,
                       backward ? 1 : 0, stream), "hyc_rope_pair");
 }
@@ -255,7 +258,7 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
                                    const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status) {
   const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
-  require_cuda({&x, &wq});
+  SameDevice{x}.with(w).with(stats).with(tables.cos).with(tables.sin).with(mask).with(status);
   OnDevice on(x);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M, rep = nh / nkv;
   auto [x_norm, rstd, x_o, x_q, xn_q] = rmsnorm_save(x, norm_w, eps, q, x_scale, x_idx, xn_scale);
@@ -294,6 +297,7 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
 // o projection with residual and the save of its input
 static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols,
                                             const Tensor& o_scale, const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& status) {
+  SameDevice{x}.with(o2).with(wo).with(ao_cols).with(bo_cols).with(o_scale).with(o_codes).with(bias_o).with(status);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
   const Tensor o_xa64 = at::mm(o2, ao_cols);
   const Tensor res = bf16c(x);
@@ -311,6 +315,7 @@ static Tensor rebuild(const Tensor& codes, const Tensor& scale, const Tensor& xa
 // o projection backward: -> grad_bo, grad_ao, grad_o2
 static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, const Tensor& bo_in, const Tensor& ao_rows, const Tensor& o_xa,
                                              const Tensor& o_q, const Tensor& o_scale, int64_t q, const Tensor& status) {
+  SameDevice{g}.with(wo).with(bo_in).with(ao_rows).with(o_xa).with(o_q).with(o_scale).with(status);
   OnDevice on(g);
   const int64_t T = g.size(0);
   const Tensor bo = bo_in.contiguous();
@@ -330,6 +335,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
                                                 const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status) {
   const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
                &v_s = saved[7], &v_xa = saved[8];
+  SameDevice{grad_o2}.with(a).with(topk).with(saved).with(w).with(tables.cos).with(tables.sin).with(cls).with(status);
   OnDevice on(grad_o2);
   const int64_t T = B * M, rep = nh / nkv;
   const double scale = 1.0 / std::sqrt((double)d);
@@ -345,7 +351,6 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
       cp[i] = data(keep[3 * i] = saved[3 * i].contiguous()); sp[i] = data(keep[3 * i + 1] = vec(saved[3 * i + 1]));
       xp[i] = data(saved[3 * i + 2]); bp[i] = data(keep[3 * i + 2] = w[i].contiguous()); yp[i] = data(rebuilt[i]);
     }
-    require_cuda({&q_q, &k_q, &v_q, &w[0], &tables.cos, &tables.sin});
     check(hyc_rebuild_qkv(cp, sp, xp, bp, yp, n, data(tables.cos), data(tables.sin), tables.cos.stride(0), tables.f32(), T, (int)M, (int)q, on.stream),
           "hyc_rebuild_qkv");
     const Tensor &q2 = rebuilt[0], &k2 = rebuilt[1], &v2 = rebuilt[2];
@@ -388,6 +393,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
 // LoRA gradients of q/k/v: -> gmq [T, 64], ga [48, H], grad_bq, grad_bk, grad_bv
 static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, const std::vector<Tensor>& b_in, const Tensor& qkv_xa, const Tensor& xn_q,
                                               const Tensor& xn_scale, int64_t q, const Tensor& status) {
+  SameDevice{grads[0]}.with(grads).with(b_in).with(qkv_xa).with(xn_q).with(xn_scale).with(status);
   OnDevice on(grads[0]);
   const int64_t T = grads[0].size(0);
   Tensor gmq = empty({T, 64}, grads[0]), gb[3], b[3];
@@ -405,6 +411,7 @@ static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, 
 static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wq = w[0], &wk = w[1], &wv = w[2], &aqkv_rows = w[3], &norm_w = w[4];
+  SameDevice{g}.with(grads).with(gmq).with(w).with(saved).with(status);
   Tensor grad_xn = gemm({{&grads[0], &wq}, {&grads[1], &wk}, {&grads[2], &wv}, {&gmq, &aqkv_rows}}, true, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
@@ -495,7 +502,7 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
   at::AutoDispatchBelowADInplaceOrView below;
   TORCH_CHECK_VALUE((int)stats.size() == STATS, "layer_forward: ", (int)STATS, " statistics expected");
   TORCH_CHECK_VALUE(x_in.dim() == 3, "expected a [B, M, H] input, got shape ", x_in.sizes());
-  require_cuda({&x_in, &p.norm1, &p.lora[0], &status});
+  require_cuda({&x_in, &status});
   p.set_stats(stats);
   const std::vector<Tensor>& st = p.stats;
   const Tensor x = bf16c(x_in);

@@ -349,6 +349,7 @@ Tensor rope(const Tensor& x, const Tensor& cos_in, const Tensor& sin_in, bool ba
 
 Tensor dequant_nf4(const Tensor& packed, const Tensor& code, const Tensor& absmax, const OptTensor& code2, const OptTensor& absmax2,
                    int64_t blocksize2, double offset, int64_t blocksize, at::IntArrayRef shape) {
+  require_cuda({&packed, &code, &absmax, opt(code2), opt(absmax2)});
   OnDevice on(packed);
   Tensor out = empty(shape, packed);
   const bool nested = given(code2);

@@ -185,6 +185,7 @@ def mlp_forward(x_medium, w: MLPWeights, state: MLPState, eps=1e-5, status=None)
 
 def _mlp_forward_calibrating(x_medium, w, state, eps, st):
     """A calibration iteration: every save takes its statistics from the finished tensor."""
+    require_cuda(x_medium, w.wg, w.wu, w.bg, w.bu)
     B, M, H = x_medium.shape
     T, I, q, it, thd = B * M, w.wg.shape[0], state.q_bit, state.iteration, state.iteration_threshold
     sv, dev = state.static_value, x_medium.device

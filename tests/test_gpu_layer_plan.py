@@ -147,3 +147,32 @@ def test_hook_of_the_mlp_half_that_changes_the_attention_half():
         p.layer.on_lora_grads = hook
         return p.step()
     assert _same(run(False), run(True))
+
+
+@pytest.mark.parametrize("stepwise", [False, True])
+@pytest.mark.parametrize("what", ["mask", "cos", "q", "k", "v", "o", "gate", "up", "down", "q scale", "o scale", "gate scale"])
+def test_tensor_on_another_device_is_refused(what, stepwise):
+    """A tensor on the host is an error of the call, never an address that a kernel reads."""
+    p = Problem()
+    p.layer.keep_saved = stepwise
+    x, mask, attn, mlp = p.x, p.mask, p.layer.attn_state.static_value, p.layer.mlp_state.static_value
+    if what == "mask":
+        mask = mask.cpu()
+    elif what == "cos":
+        p.cos, p.sin = p.cos.cpu(), p.sin.cpu()
+    elif what.endswith(" scale"):
+        entry = {**attn, **mlp}[what.split()[0]]
+        entry["scale"] = entry["scale"].cpu()
+    else:
+        p.mods[what][0].cpu()
+    with pytest.raises(RuntimeError, match="device|CUDA"):
+        p.forward(x, mask=mask)
+    assert int(p.layer._status.item()) == 0
+
+
+def test_outlier_indices_may_lie_on_the_host():
+    p = Problem()
+    want = p.step()
+    for entry in (p.layer.attn_state.static_value["x"], p.layer.mlp_state.static_value["x_medium"]):
+        entry["outlier_channel_index"] = entry["outlier_channel_index"].cpu()
+    assert _same(p.step(), want)
