@@ -245,6 +245,15 @@ RopeTables rope_tables(const Tensor& cos_in, const Tensor& sin_in, int64_t seq, 
   if (t.cos.stride(1) != 1 || t.sin.stride(1) != 1 || t.sin.stride(0) != t.cos.stride(0)) { t.cos = t.cos.contiguous(); t.sin = t.sin.contiguous(); }
   return t;
 }
+// Projections and head geometry have to agree: the kernels take rows of heads * d elements as they are told
+static void check_geometry(const std::array<int64_t, 3>& widths, int64_t nh, int64_t d, int64_t nkv) {
+  if (nh < 1 || nkv < 1 || d < 1 || nh % nkv != 0)
+    throw std::runtime_error("invalid head geometry: " + std::to_string(nh) + " heads, " + std::to_string(nkv) + " key/value heads of " + std::to_string(d));
+  for (int i = 0; i < 3; ++i)
+    if (widths[i] != (i == 0 ? nh : nkv) * d)
+      throw std::runtime_error(std::string("the ") + "qkv"[i] + " projection has " + std::to_string(widths[i]) + " outputs, not " +
+                               std::to_string(i == 0 ? nh : nkv) + " heads of " + std::to_string(d));
+}
 // q and k (contiguous [rows, heads*d]) in place
 static void rope_pair(const Tensor& q, int64_t nh, const Tensor& k, int64_t nkv, const RopeTables& t, int64_t seq, int64_t d, bool backward,
                       void* stream) {
@@ -258,6 +267,7 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
                                    const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status) {
   const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
+  check_geometry({wq.size(0), wk.size(0), wv.size(0)}, nh, d, nkv);
   SameDevice{x}.with(w).with(stats).with(tables.cos).with(tables.sin).with(mask).with(status);
   OnDevice on(x);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M, rep = nh / nkv;
@@ -273,7 +283,7 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
     // one kernel from q, k, v to the probabilities, o and the codes of o
     const MaskView mv = mask_view(mask, B, nh, M);
     Tensor cls, a = empty({B, nh, M, M}, x_norm), o2 = empty({T, nh * d}, x_norm), o_q = empty({T, nh * d * q / 8}, x_norm, at::kByte);
-    const Tensor os = vec(stats[6]);
+    const Tensor os = scale_vec(stats[6], nh * d);
     int64_t cls_b = 0, cls_h = 0;
     if (mv.t.defined()) {
       const int64_t nb = mv.t.size(0), nhm = mv.t.size(1);
@@ -335,6 +345,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
                                                 const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status) {
   const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
                &v_s = saved[7], &v_xa = saved[8];
+  check_geometry({w[0].size(0), w[1].size(0), w[2].size(0)}, nh, d, nkv);
   SameDevice{grad_o2}.with(a).with(topk).with(saved).with(w).with(tables.cos).with(tables.sin).with(cls).with(status);
   OnDevice on(grad_o2);
   const int64_t T = B * M, rep = nh / nkv;

@@ -176,3 +176,25 @@ def test_outlier_indices_may_lie_on_the_host():
     for entry in (p.layer.attn_state.static_value["x"], p.layer.mlp_state.static_value["x_medium"]):
         entry["outlier_channel_index"] = entry["outlier_channel_index"].cpu()
     assert _same(p.step(), want)
+
+
+@pytest.mark.parametrize("stepwise", [False, True])
+def test_head_geometry_and_scale_that_do_not_fit_are_refused(stepwise):
+    p = Problem()
+    p.layer.keep_saved = stepwise
+    want = p.step()
+    fits = p.geometry
+    for geometry in ((4, 128, 4), (2, 128, 2), (4, 64, 2), (4, 128, 0)):
+        p.geometry = geometry
+        with pytest.raises(RuntimeError, match="head"):
+            p.forward(p.x)
+    p.geometry = fits
+    entry = p.layer.attn_state.static_value["o"]
+    scale = entry["scale"]
+    entry["scale"] = scale.reshape(-1)[:1]
+    with pytest.raises(ValueError, match="per-channel scale"):
+        p.forward(p.x)
+    entry["scale"] = scale
+    # (a failed call may have advanced one half: what counts is that the launches of a right call are unharmed)
+    p.layer.iteration = 10
+    assert _same(p.step(), want)

@@ -76,3 +76,16 @@ def test_replaced_adapter_memory_is_not_handed_out_again(bound):
         w.data = torch.zeros_like(w.data)
     later = [torch.empty_like(w) for w in ws for _ in range(20)]
     assert not old & {t.data_ptr() for t in later}
+
+
+@pytest.mark.parametrize("heads,d,kv", [(4, 128, 4), (2, 128, 2), (8, 128, 2), (4, 64, 2), (4, 128, 0), (0, 128, 2), (4, 128, 3), (4, 256, 1)])
+def test_head_geometry_is_checked_against_the_projections(heads, d, kv):
+    """4 query and 2 key/value heads of 128 are what the weights hold; the check comes before anything is launched."""
+    from hyc_lora_release_b200._lib import host
+    H, t = 512, lambda *s: torch.zeros(*s, dtype=torch.bfloat16)
+    w = [t(H), t(512, H), t(256, H), t(256, H), t(512, 16), t(256, 16), t(256, 16), t(3, H, 16)]
+    with pytest.raises(RuntimeError, match="head"):
+        host.attn_forward_map(t(1, 8, H), w, [t(1)] * 7, t(8, 128), t(8, 128), None, heads, d, kv, 4, 1e-5, torch.zeros(1, dtype=torch.int32))
+    with pytest.raises(RuntimeError, match="head"):
+        host.attn_backward_map(t(8, 512), t(1, 4, 8, 8), [], 0, [t(8, 1)] * 9, w[4:7], t(8, 128), t(8, 128), 1, 8, heads, d, kv, 4, None, 0, 0,
+                               torch.zeros(1, dtype=torch.int32))
