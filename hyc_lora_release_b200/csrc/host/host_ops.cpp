@@ -29,6 +29,13 @@ Tensor scale_vec(const Tensor& s, int64_t n) {
   return v;
 }
 
+// length of the rows of a tensor that is taken as rows; a caller divides by it
+static int64_t row_length(const Tensor& t) {
+  const int64_t n = t.size(-1);
+  TORCH_CHECK_VALUE(n > 0, "the last dimension is empty (shape ", t.sizes(), ")");
+  return n;
+}
+
 // [B, M, N] (or [B, heads, M, d], which becomes [B, M, heads*d]) -> bf16 with one row stride
 static Tensor rows_view(const Tensor& x_in) {
   Tensor x = x_in;
@@ -94,19 +101,19 @@ Tensor dequant(const Tensor& q_in, const Tensor& s_in, int64_t q_bit, const OptT
 // ---- attention map, per-row top-k
 void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& val, const Tensor& col, const Tensor& q,
                         const Tensor& s, const Tensor& z) {
+  const int64_t S = row_length(x), rows = x.numel() / S;
   require_cuda({&x});
   check_q(q_bit);
   OnDevice on(x);
   const Tensor xb = bf16c(x);
-  const int64_t S = xb.size(-1), rows = xb.numel() / S;
   check(hyc_softmax_topk_compress(data(xb), rows, (int)S, (int)k, k ? data(val) : nullptr, k ? (uint16_t*)data(col) : nullptr, data(q),
                                   data(s), (int8_t*)data(z), (int)q_bit, on.stream), "hyc_softmax_topk_compress");
 }
 
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit) {
+  const int64_t S = row_length(x), rows = x.numel() / S;
   require_cuda({&x});
   check_q(q_bit);
-  const int64_t S = x.size(-1), rows = x.numel() / S;
   Tensor val = empty({rows, k}, x), col = empty({rows, k}, x, at::kShort), q = empty({rows, S * q_bit / 8}, x, at::kByte),
          s = empty({rows, S / 64}, x), z = empty({rows, S / 64}, x, at::kChar);
   topk_compress_into(x, k, q_bit, val, col, q, s, z);
@@ -260,11 +267,11 @@ Tensor dequant_lora_add(const Tensor& q, const Tensor& s, const Tensor& xa, cons
 // ---- norms, softmax, rotary embedding
 std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor& x, const Tensor& w_in, double eps, int64_t q_bit,
                                                                    const Tensor& sx_in, const OptTensor& idx_in, const OptTensor& sy_in) {
+  const int64_t N = row_length(x), rows = x.numel() / N;
   require_cuda({&x, &w_in, &sx_in});
   check_q(q_bit);
   OnDevice on(x);
   const Tensor xc = bf16c(x), w = bf16c(w_in);
-  const int64_t N = xc.size(-1), rows = xc.numel() / N;
   const Tensor sx = scale_vec(sx_in, N);
   Tensor idx, sy;
   int64_t k = 0;
@@ -285,10 +292,10 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor&
 
 Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor& sx_in, const OptTensor& xo_in, const OptTensor& idx_in,
                                const Tensor& w_in, const Tensor& rstd, int64_t q_bit, const OptTensor& res_in) {
+  const int64_t N = row_length(dy), rows = dy.numel() / N;
   require_cuda({&dy, &qx, &sx_in, &w_in, &rstd});
   OnDevice on(dy);
   const Tensor dyc = bf16c(dy), sx = vec(sx_in), w = bf16c(w_in), q = qx.contiguous(), rs = rstd.contiguous();
-  const int64_t N = dyc.size(-1), rows = dyc.numel() / N;
   Tensor idx, xo, res;
   int64_t k = 0;
   if (given(idx_in)) { idx = index_of(*idx_in, dy); k = idx.numel(); }
@@ -302,11 +309,11 @@ Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor&
 }
 
 Tensor softmax_backward(const Tensor& y, const Tensor& g, double scale) {
+  const int64_t S = row_length(y);
   require_cuda({&y, &g});
   OnDevice on(y);
   const Tensor yc = bf16c(y), gc = bf16c(g);
   Tensor o = at::empty_like(yc);
-  const int64_t S = yc.size(-1);
   check(hyc_softmax_bwd(data(yc), data(gc), data(o), yc.numel() / S, (int)S, (float)scale, on.stream), "hyc_softmax_bwd");
   return o;
 }

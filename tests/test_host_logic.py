@@ -1,4 +1,5 @@
-"""Host-side logic that needs no device: the calibration running mean."""
+"""Host-side logic that needs no device: the calibration running mean, checks before any launch."""
+import pytest
 import torch
 
 from hyc_lora_release_b200.operators.compress_function import (
@@ -17,3 +18,14 @@ def test_update_dict_matches_reference(golden):
 def test_head_hidden_roundtrip():
     x = torch.arange(2 * 3 * 8, dtype=torch.float32).reshape(2, 3, 8)
     assert torch.equal(head_to_hidden_shape(hidden_to_head_shape(x, 4)), x)
+
+
+def test_rows_of_no_columns_are_an_error():
+    """An integer division by zero in native code would end the process, not raise."""
+    from hyc_lora_release_b200.operators import compress_function as cf, rmsnorm_kernels as rn, softmax_kernels as sk
+    none, one = torch.zeros(2, 3, 4, 0), torch.zeros(1)
+    for call in (lambda: sk.softmax_backward(none, none), lambda: cf.compression_softmax_topk(none, 0.05),
+                 lambda: rn.rmsnorm_forward_save(none, one, 1e-5, 4, one, None, one),
+                 lambda: rn.rmsnorm_backward_packed(none, one, one, None, None, one, one, 4)):
+        with pytest.raises(ValueError, match="empty"):
+            call()
