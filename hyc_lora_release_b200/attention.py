@@ -144,7 +144,7 @@ def _project(xn2, w, a, b, q_bit, calib, sv, it, thd, status, B, bias=None, xa=N
         y, qm, xa = linear_lora_save(xn2, w, a, b, scale, q_bit, status=status, xa=xa)
         return y, qm, scale, xa
     # calibration iterations (the scale depends on the finished main branch) and projections with a bias
-    main = gemm(xn2, w, status=status)
+    main = gemm(xn2, w, status=status, fixed_order=True)
     if bias is not None:
         main = main + bias.to(main.dtype)
     qm, scale = cf.compression_pack_quant_base(main.view(B, main.shape[0] // B, -1), q_bit, 'per-channel', it, thd, sv)
@@ -250,7 +250,8 @@ def _attention_forward_stepwise(x, w, state, cos, sin, attention_mask, num_heads
 
     pad = w.padded()
     o_xa64 = o2 @ pad["ao_cols"]
-    x_medium = gemm(o2, w.wo, a2=o_xa64, b2=pad["bo_cols"], residual=x.reshape(T, H).to(BF16).contiguous(), status=st)
+    x_medium = gemm(o2, w.wo, a2=o_xa64, b2=pad["bo_cols"], residual=x.reshape(T, H).to(BF16).contiguous(), status=st,
+                    fixed_order=True)
     if w.bias_o is not None:
         x_medium += w.bias_o.to(BF16)
     o_q, o_scale = cf.compression_pack_quant_base(o2.view(B, M, -1), q, 'per-channel', it, thd, sv['o'])

@@ -11,15 +11,15 @@ static int* status_ptr(const Tensor& st) { return (int*)st.data_ptr(); }
 
 // sum of a_i op(b_i) (+ residual), one to four K segments
 struct Segment { const Tensor *a, *b; };
-static Tensor gemm(std::initializer_list<Segment> segs, bool b_is_kn, const Tensor* residual, const Tensor& status) {
+static Tensor gemm(std::initializer_list<Segment> segs, int form, const Tensor* residual, const Tensor& status) {
   const Tensor& a = *segs.begin()->a;
   OnDevice on(a);
-  const int64_t M = a.size(0), N = segs.begin()->b->size(b_is_kn ? 1 : 0);
+  const int64_t M = a.size(0), N = segs.begin()->b->size(form & HYC_GEMM_B_KN ? 1 : 0);
   const void *pa[4], *pb[4];
   int k[4], n = 0;
   for (const Segment& s : segs) { pa[n] = data(*s.a); pb[n] = data(*s.b); k[n++] = (int)s.a->size(1); }
   Tensor d = empty({M, N}, a);
-  check(hyc_gemm_segments_tcgen05(n, pa, pb, k, (int)M, (int)N, b_is_kn ? 1 : 0, residual ? data(*residual) : nullptr, data(d),
+  check(hyc_gemm_segments_tcgen05(n, pa, pb, k, (int)M, (int)N, form, residual ? data(*residual) : nullptr, data(d),
                                   status_ptr(status), on.stream), "hyc_gemm_segments_tcgen05");
   return d;
 }
@@ -152,7 +152,7 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   const Tensor down_xa64 = at::mm(had, ad_cols);
   const Tensor res = bf16c(x_medium), wd = wd_later ? matrices({wd_later})[0] : w[3];
   require_cuda({&x_medium, &wd});
-  Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, false, &res, status);
+  Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, 0, &res, status);
   if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
   return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
 }
@@ -190,7 +190,7 @@ static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& g
   const Tensor &wg = w[0], &wu = w[1], &agu_rows = w[2], &norm_w = w[3];
   SameDevice{g}.with(ggu).with(gm64).with(w).with(saved).with(status);
   const Tensor g0 = ggu[0], g1 = ggu[1];
-  Tensor grad_xn = gemm({{&g0, &wg}, {&g1, &wu}, {&gm64, &agu_rows}}, true, nullptr, status);
+  Tensor grad_xn = gemm({{&g0, &wg}, {&g1, &wu}, {&gm64, &agu_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 
@@ -311,7 +311,7 @@ static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, c
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
   const Tensor o_xa64 = at::mm(o2, ao_cols);
   const Tensor res = bf16c(x);
-  Tensor x_medium = gemm({{&o2, &wo}, {&o_xa64, &bo_cols}}, false, &res, status);
+  Tensor x_medium = gemm({{&o2, &wo}, {&o_xa64, &bo_cols}}, HYC_GEMM_FIXED_ORDER, &res, status);
   if (given(bias_o)) x_medium.add_(bias_o->to(at::kBFloat16));
   const Tensor o_q = given(o_codes) ? *o_codes : std::get<0>(quant(o2.view({B, M, -1}), o_scale, q, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
   return {x_medium.view({B, M, H}), o_q.view({T, -1}), o_xa64};
@@ -332,7 +332,7 @@ static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, 
   Tensor gm64 = empty({T, 64}, g), grad_bo = empty({g.size(1), 16}, g);
   Skinny().on(g).rows(data(bo), 16, gm64, 0, 64, 48).cols(data(o_xa), o_xa.stride(0), data(grad_bo)).run(T, g, status, on.stream);
   Tensor grad_ao = lora_grad_a(o_q, vec(o_scale), gm64, 16, q);
-  Tensor grad_o2 = gemm({{&g, &wo}, {&gm64, &ao_rows}}, true, nullptr, status);
+  Tensor grad_o2 = gemm({{&g, &wo}, {&gm64, &ao_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return {grad_bo, grad_ao, grad_o2};
 }
 
@@ -423,7 +423,7 @@ static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads,
                               const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wq = w[0], &wk = w[1], &wv = w[2], &aqkv_rows = w[3], &norm_w = w[4];
   SameDevice{g}.with(grads).with(gmq).with(w).with(saved).with(status);
-  Tensor grad_xn = gemm({{&grads[0], &wq}, {&grads[1], &wk}, {&grads[2], &wv}, {&gmq, &aqkv_rows}}, true, nullptr, status);
+  Tensor grad_xn = gemm({{&grads[0], &wq}, {&grads[1], &wk}, {&grads[2], &wv}, {&gmq, &aqkv_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 

@@ -681,7 +681,7 @@ static int launch_as(const Operands& ops, const Params& p, cudaStream_t st) {
 
 template <int EPI, int QBIT, bool B_MN>
 static int launch(const Operands& ops, const Params& p, cudaStream_t st) {
-  const SplitPlan plan = choose_split(EPI, B_MN, p);
+  const SplitPlan plan = choose_split(EPI, p);
   if (plan.split > 0) return launch_split(EPI, QBIT, B_MN, plan, ops, p, st);
   // pairs, except where few rows would leave half of the tile empty
   bool pair = p.M > BM;
@@ -694,6 +694,8 @@ static int launch(const Operands& ops, const Params& p, cudaStream_t st) {
 using namespace hyc;
 using namespace hyc::tc;
 
+static constexpr int kGemmForms = HYC_GEMM_B_KN | HYC_GEMM_FIXED_ORDER;
+
 static LoraTerm make_term(const void* xa, const void* bt, int64_t ld_col, int64_t ld_r) {
   LoraTerm t;
   t.xa = (const __nv_bfloat16*)xa;
@@ -704,12 +706,14 @@ static LoraTerm make_term(const void* xa, const void* bt, int64_t ld_col, int64_
 }
 
 extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
-    const void* A, const void* B, int M, int N, int K, int b_is_kn,
+    const void* A, const void* B, int M, int N, int K, int form,
     const void* A2, const void* B2, int K2, const void* A3, const void* B3, int K3,
     const void* xa0, const void* bt0, int64_t bt0_ld_col, int64_t bt0_ld_r,
     const void* xa1, const void* bt1, int64_t bt1_ld_col, int64_t bt1_ld_r,
     const void* residual, void* D, int* status, void* stream) {
   if (!A || !B || !D || !status) return HYC_ERR_NULL;
+  if (form & ~kGemmForms) return HYC_ERR_SHAPE;
+  const bool b_is_kn = (form & HYC_GEMM_B_KN) != 0;
   if ((K2 > 0) != (A2 != nullptr && B2 != nullptr)) return HYC_ERR_NULL;
   if ((K3 > 0) != (A3 != nullptr && B3 != nullptr)) return HYC_ERR_NULL;
   if (M <= 0 || N <= 0 || K <= 0 || N % BN != 0 || K % BK != 0 || K2 < 0 || K2 % BK != 0 || K3 < 0 || K3 % BK != 0)
@@ -725,6 +729,7 @@ extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
   if (K3 > 0) { ops.a[2] = {A3, M, K3}; ops.b[2] = b_is_kn ? Matrix{B3, K3, N} : Matrix{B3, N, K3}; }
   Params p = {};
   p.M = M; p.N = N; p.K1 = K; p.K2 = K2; p.K3 = K3; p.epi = EPI_STORE; p.q_bit = 0;
+  p.fixed_order = (form & HYC_GEMM_FIXED_ORDER) != 0;
   p.l0 = make_term(xa0, bt0, bt0_ld_col, bt0_ld_r);
   p.l1 = make_term(xa1, bt1, bt1_ld_col, bt1_ld_r);
   p.l2 = make_term(nullptr, nullptr, 0, 0);
@@ -737,8 +742,10 @@ extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
 }
 
 extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
-                                                int b_is_kn, const void* residual, void* D, int* status, void* stream) {
+                                                int form, const void* residual, void* D, int* status, void* stream) {
   if (!A || !B || !K || !D || !status) return HYC_ERR_NULL;
+  if (form & ~kGemmForms) return HYC_ERR_SHAPE;
+  const bool b_is_kn = (form & HYC_GEMM_B_KN) != 0;
   if (count < 1 || count > 4 || M <= 0 || N <= 0 || N % BN != 0) return HYC_ERR_SHAPE;
   if (!aligned(D, 16) || (residual && !aligned(residual, 16))) return HYC_ERR_ALIGN;
   Operands ops = {};
@@ -751,6 +758,7 @@ extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A
   }
   Params p = {};
   p.M = M; p.N = N; p.epi = EPI_STORE;
+  p.fixed_order = (form & HYC_GEMM_FIXED_ORDER) != 0;
   p.K1 = K[0]; p.K2 = count > 1 ? K[1] : 0; p.K3 = count > 2 ? K[2] : 0; p.K4 = count > 3 ? K[3] : 0;
   p.residual = (const __nv_bfloat16*)residual;
   p.out0 = (__nv_bfloat16*)D;

@@ -69,6 +69,7 @@ struct Params {
   // Column tiles: the first n_wide are TILE_N columns wide, the rest half of that
   int n_wide;
   int stages, stage_bytes;    // ring of the main loop
+  bool fixed_order;           // for the launch: K is not split
   int* status;
 #ifdef HYC_TC_PROF
   long long* prof;            // debug builds only: clock64 stamps of CTA 0, [role][tile][8]

@@ -338,16 +338,17 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
 //   512 tokens: 45 / 47, 75 / 77: persistent
 // A CTA keeps at least 16 k-blocks: below that its share of the main loop is shorter than set-up and reduction (about
 // 3 us), and the sum over all of K stays in one accumulator.
-// Products whose results the layer quantizes, or that feed tensors it quantizes (gate/up, q/k/v, the K-major ones of fewer
-// than 128 k-blocks: the o projection), are not split: the saved codes then do not depend on how many rows are computed
-// together (with 2-bit codes one that flips moves a value by a third of its range).  That leaves 5 us on the o projection.
-SplitPlan choose_split(int epi, bool b_mn, const Params& p) {
+// Products whose results the layer quantizes, or that feed tensors it quantizes in the same pass, are not split (gate/up, q/k/v,
+// and what the caller marks as such: the o projection): the saved codes of a layer then do not depend through them on how many
+// rows are computed together (with 2-bit codes one that flips moves a value by a third of its range).  That leaves 5 us on
+// the o projection.  The down projection may be split, so the input of the next layer does depend on it in its last bits.
+SplitPlan choose_split(int epi, const Params& p) {
   SplitPlan plan = {0, false};
   if (epi == EPI_GRADDOWN || p.M > 2 * BM) return plan;
   if (epi == EPI_STORE && p.l1.bt != nullptr) return plan;         // a second LoRA term: the persistent kernel's own epilogue
   const int tiles = p.N / (epi == EPI_GATEUP ? SBN / 2 : SBN), sms = num_sms();
   const int kb = (p.K1 + p.K2 + p.K3 + p.K4) / BK;
-  const bool whole = epi == EPI_GATEUP || p.q1 != nullptr || (!b_mn && kb < 128);
+  const bool whole = epi == EPI_GATEUP || p.q1 != nullptr || p.fixed_order;
   if (whole) {
     if (p.M <= BM && tiles >= sms / 4) plan.split = 1;      // fewer tiles: half-width tiles of the persistent kernel
   } else if (p.M <= BM) {

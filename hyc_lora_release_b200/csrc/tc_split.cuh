@@ -7,7 +7,7 @@ namespace tc {
 
 // split > 0: launch with the split kernels, the pair form (256-row tiles) if `pair`; split = 0: the persistent kernel
 struct SplitPlan { int split; bool pair; };
-SplitPlan choose_split(int epi, bool b_mn, const Params& p);
+SplitPlan choose_split(int epi, const Params& p);
 int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Operands& ops, const Params& p, cudaStream_t st);
 
 }  // namespace tc

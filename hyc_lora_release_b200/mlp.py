@@ -46,10 +46,11 @@ def _lora(xa, bt, ld_col, ld_r):
 
 
 def gemm(a, b, *, b_is_kn=False, a2=None, b2=None, a3=None, b3=None, lora0=None, lora1=None, residual=None,
-         status=None):
+         status=None, fixed_order=False):
     """D = a @ op(b) (+ a2 @ op(b2)) (+ a3 @ op(b3)) (+ LoRA terms) (+ residual) on the tcgen05 kernel.
 
     a [M,K] bf16; b [N,K] (b_is_kn=False) or [K,N] (b_is_kn=True), both row-major.
+    fixed_order: the order of summation does not depend on M (for results that are quantized, or feed what is).
     lora = (xa [M,16], bt, ld_col, ld_r): adds xa @ Bt^T with Bt(col, r) = bt[col*ld_col + r*ld_r]."""
     require_cuda(a, b)
     M, K = a.shape
@@ -60,7 +61,7 @@ def gemm(a, b, *, b_is_kn=False, a2=None, b2=None, a3=None, b3=None, lora0=None,
     st = status if status is not None else _status_tensor(a.device)
     l0 = _lora(*lora0) if lora0 else [None, None, 0, 0]
     l1 = _lora(*lora1) if lora1 else [None, None, 0, 0]
-    check(lib.hyc_gemm_bf16_tcgen05(ptr(a), ptr(b), M, N, K, 1 if b_is_kn else 0, ptr(a2), ptr(b2), K2,
+    check(lib.hyc_gemm_bf16_tcgen05(ptr(a), ptr(b), M, N, K, (1 if b_is_kn else 0) | (2 if fixed_order else 0), ptr(a2), ptr(b2), K2,
                                     ptr(a3), ptr(b3), K3, *l0, *l1, ptr(residual), ptr(d), ptr(st), stream_of(a)),
           "hyc_gemm_bf16_tcgen05")
     return d

@@ -315,16 +315,19 @@ int hyc_dequant_nf4_many(int count, const hyc_nf4_job* jobs, void* stream);
  * factor as element (column, r) at bt[column * ld_col + r * ld_r], so both the [out, r] weight and
  * its [r, out] transpose can be passed without a copy. */
 
+#define HYC_GEMM_B_KN 1
+#define HYC_GEMM_FIXED_ORDER 2
 /* D[M,N] = A[M,K] * B (+ A2[M,K2] * B2) (+ A3[M,K3] * B3) (+ xa0 * bt0^T) (+ xa1 * bt1^T) (+ residual).
  * Up to three (A, B) pairs accumulate in the same tensor-memory tile; K2, K3 may be 0.  A rank-16 LoRA
  * product can be passed either as an extra pair whose K is padded with zeros to 64 (it then costs one more
  * MMA block and nothing in the epilogue) or as xa/bt, evaluated per element in the epilogue and rounded to
  * bf16 separately like the reference's tensor-by-tensor code.
- * b_is_kn = 0: every B is [N,K] row-major (an nn.Linear weight, forward use); 1: every B is [K,N] row-major
- * (the same weight used for a backward product, read in place).  N % 256 == 0, K, K2, K3 % 64 == 0.
+ * form: 0 or any of HYC_GEMM_B_KN (every B is [K,N] row-major, an nn.Linear weight used for a backward product and read in
+ * place; without it every B is [N,K] row-major, forward use) and HYC_GEMM_FIXED_ORDER (the order in which a result is summed
+ * up does not depend on M; without it products of up to 256 rows may split K).  N % 256 == 0, K, K2, K3 % 64 == 0.
  * Replaces the matmuls of lora_forward / lora_backward (models/utils/compute_utils.py:18-36) and the
  * hand-inlined copies (models/llama/fused_llama_layer_intra_inter_full_fuse.py:247, 359-364, 379-384). */
-int hyc_gemm_bf16_tcgen05(const void* A, const void* B, int M, int N, int K, int b_is_kn,
+int hyc_gemm_bf16_tcgen05(const void* A, const void* B, int M, int N, int K, int form,
                           const void* A2, const void* B2, int K2, const void* A3, const void* B3, int K3,
                           const void* xa0, const void* bt0, int64_t bt0_ld_col, int64_t bt0_ld_r,
                           const void* xa1, const void* bt1, int64_t bt1_ld_col, int64_t bt1_ld_r,
@@ -332,7 +335,7 @@ int hyc_gemm_bf16_tcgen05(const void* A, const void* B, int M, int N, int K, int
 
 /* The same without LoRA terms for one to four (A, B) pairs: host arrays of `count` entries, A[i] [M, K[i]]. */
 int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
-                              int b_is_kn, const void* residual_or_null, void* D, int* status, void* stream);
+                              int form, const void* residual_or_null, void* D, int* status, void* stream);
 
 /* A LoRA projection with the save of its main branch in the GEMM epilogue (the q/k/v/o projections of the
  * attention half: `lora_forward` followed by `compression_pack_quant_base(x=q_main, ...)`,

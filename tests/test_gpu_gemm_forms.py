@@ -118,3 +118,32 @@ def test_lora_terms_of_the_pair_form(T, I, q, transposed):
     near(had, y1 * sig * y2)
     near(gu, gd * y1 * sig)
     near(gg, gd * y2 * sig * (1 + y1 * (1 - sig)))
+
+
+@pytest.mark.parametrize("N,K", [(512, 4096), (1024, 8192), (256, 12288)])
+def test_fixed_order_does_not_depend_on_the_rows(N, K):
+    """A row's sum is the same bits whatever else is computed with it, on every form that the row count selects."""
+    from hyc_lora_release_b200 import mlp
+    g = torch.Generator().manual_seed(K)
+    a, a2, b, b2, res = _rn(g, 700, K), _rn(g, 700, 64), _rn(g, N, K, scale=0.02), _rn(g, N, 64, scale=0.1), _rn(g, 700, N)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    run = lambda M, **kw: mlp.gemm(a[:M], b, a2=a2[:M], b2=b2, residual=res[:M], status=st, **kw)
+    whole = run(700, fixed_order=True)
+    for M in (1, 64, 128, 129, 256, 257, 512):
+        assert torch.equal(run(M, fixed_order=True), whole[:M]), M
+    assert int(st.item()) == 0
+
+
+def test_o_projection_does_not_depend_on_the_rows():
+    """The o projection of the layer at a hidden size whose K is as long as a down projection's: x_medium, which is quantized
+    next, is the same bits (the library's LoRA-A product aside: its factor is zero here)."""
+    from hyc_lora_release_b200._lib import host
+    g = torch.Generator().manual_seed(3)
+    H = 8192
+    wo, zero, bo = _rn(g, H, H, scale=0.01), torch.zeros(H, 64, dtype=BF16, device=DEV), _rn(g, H, 64)
+    x, o = _rn(g, 1, 300, H), _rn(g, 300, H)
+    st, sc = torch.zeros(1, dtype=torch.int32, device=DEV), torch.ones(H, dtype=BF16, device=DEV)
+    run = lambda M: host.attn_forward_out(x[:, :M], o[:M], wo, zero, bo, sc, None, None, 4, st)[0]
+    whole = run(300)
+    for M in (64, 128, 200, 256):
+        assert torch.equal(run(M), whole[:, :M]), M
