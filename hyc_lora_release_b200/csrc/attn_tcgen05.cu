@@ -104,9 +104,9 @@ __device__ __forceinline__ float ex2(float x) {
 }
 __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return as_u32(__hmax2(as_bf2(a), as_bf2(b))); }
 constexpr float kLog2e = 1.4426950408889634f;
-// exp(u - m) is evaluated as 2^(u * k - m * k).  Where m itself is a masked score m * log2(e) would overflow; any k that
-// keeps equal scores equal and -inf at -inf does there (the whole row part is masked)
-__device__ __forceinline__ float exp_scale(float m) { return m <= kMaskedOut ? 1e-38f : kLog2e; }
+// exp(u - m) is evaluated as 2^(u * k - m * k).  Where m itself is a masked score m * log2(e) could overflow.  k = 1 does there:
+// u and m are bf16 values, so they are equal (2^0) or at least 2^-8 of 1e30 apart (2^-inf = 0), whatever the base
+__device__ __forceinline__ float exp_scale(float m) { return m <= kMaskedOut ? 1.f : kLog2e; }
 constexpr uint32_t kNegInf2 = 0xff80ff80u;
 
 // a warp's [32 rows][32 columns] tile to rows of `ld` elements, clipped to `cols` columns (a multiple of 8)

@@ -85,3 +85,35 @@ def test_attention_forward_backward(B, M, h, kv, kind, q):
     # shapes outside the kernels are refused before any launch
     assert lib.hyc_attn_fwd_tcgen05(ptr(qx), ptr(kx), ptr(vx), B, M, h, kv, 64, scale, None, 0, 0, 0, None, 0, 0, None, ptr(o), None, None,
                                     q, ptr(st), stream_of(qx)) == -8
+
+
+@pytest.mark.parametrize("case", ["levels", "lowest"])
+def test_rows_without_a_passing_entry(case):
+    """Rows masked everywhere, with masks of two levels (the higher one takes all) and with the type's lowest value next to -inf
+    (equal shares of the former): the probabilities of the reference."""
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(11)
+    B, M, h, d = 1, 264, 2, 128
+    rn = lambda *s: torch.randn(*s, generator=g).to(BF16).to(DEV)
+    qx, kx, vx = rn(B, M, h * d), rn(B, M, h * d), rn(B, M, h * d)
+    mask = torch.zeros(1, 1, M, M)
+    if case == "levels":
+        mask[..., :M // 2, :] = -2e30
+        mask[..., :M // 2, ::3] = -4e30
+        mask[..., :M // 2, 200:] = -8e30
+    else:
+        mask[..., :M // 2, :] = float("-inf")
+        mask[..., :M // 2, 40:200] = torch.finfo(BF16).min
+    mask = mask.to(BF16).to(DEV)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    a, o = torch.zeros((B, h, M, M), dtype=BF16, device=DEV), torch.empty((B, M, h * d), dtype=BF16, device=DEV)
+    cls = torch.empty(lib.hyc_attn_mask_class_bytes(1, 1, M), dtype=torch.uint8, device=DEV)
+    check(lib.hyc_attn_mask_class(ptr(mask), 0, 0, M, 1, 1, M, ptr(cls), stream_of(qx)), "class")
+    check(lib.hyc_attn_fwd_tcgen05(ptr(qx), ptr(kx), ptr(vx), B, M, h, h, d, 1 / math.sqrt(d), ptr(mask), 0, 0, M, ptr(cls), 0, 0, ptr(a), ptr(o),
+                                   None, None, 4, ptr(st), stream_of(qx)), "fwd")
+    assert int(st.item()) == 0
+    heads = lambda t: t.view(B, M, h, d).transpose(1, 2).float()
+    t = ((heads(qx) @ heads(kx).transpose(-1, -2)).to(BF16).float() / math.sqrt(d)).to(BF16) + mask
+    ref = torch.softmax(t.float(), -1)
+    assert torch.equal(a.isnan(), ref.isnan())
+    assert _rel(a.nan_to_num(), ref.nan_to_num()) < 2 ** -8
