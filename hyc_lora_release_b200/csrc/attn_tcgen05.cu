@@ -417,7 +417,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
           sum *= ex2((m - tm) * kLog2e);
           m = tm;
         }
-        if (tm > -INFINITY) {
+        if (tm != -INFINITY) {      // (a NaN has to reach the sum: the whole row becomes NaN)
           const float k = exp_scale(m);
           const float2 ml = both(-m * k);
           float2 s2[2] = {both(0.f), both(0.f)};

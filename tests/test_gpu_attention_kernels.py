@@ -87,10 +87,11 @@ def test_attention_forward_backward(B, M, h, kv, kind, q):
                                     q, ptr(st), stream_of(qx)) == -8
 
 
-@pytest.mark.parametrize("case", ["levels", "lowest"])
-def test_rows_without_a_passing_entry(case):
+@pytest.mark.parametrize("case", ["levels", "lowest", "nan"])
+def test_rows_without_a_passing_or_a_finite_entry(case):
     """Rows masked everywhere, with masks of two levels (the higher one takes all) and with the type's lowest value next to -inf
-    (equal shares of the former): the probabilities of the reference."""
+    (equal shares of the former), and NaN scores that fill whole quarters of a row's tile (the whole row is NaN, as in a
+    softmax): the probabilities of the reference."""
     from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
     g = torch.Generator().manual_seed(11)
     B, M, h, d = 1, 264, 2, 128
@@ -101,9 +102,11 @@ def test_rows_without_a_passing_entry(case):
         mask[..., :M // 2, :] = -2e30
         mask[..., :M // 2, ::3] = -4e30
         mask[..., :M // 2, 200:] = -8e30
-    else:
+    elif case == "lowest":
         mask[..., :M // 2, :] = float("-inf")
         mask[..., :M // 2, 40:200] = torch.finfo(BF16).min
+    else:
+        kx[:, 32:96, :d] = float("nan")          # head 0
     mask = mask.to(BF16).to(DEV)
     st = torch.zeros(1, dtype=torch.int32, device=DEV)
     a, o = torch.zeros((B, h, M, M), dtype=BF16, device=DEV), torch.empty((B, M, h * d), dtype=BF16, device=DEV)
