@@ -422,7 +422,7 @@ __device__ __forceinline__ void lora_load_a(const __nv_bfloat16* xa, int64_t row
 }
 __device__ __forceinline__ void lora_load_b(const LoraTerm& l, int64_t n, int lane, LoraB& b) {
   const int g = lane >> 2, t = lane & 3;
-  const bool fast = l.ld_r == 1 && (l.ld_col & 1) == 0;
+  const bool fast = l.ld_r == 1 && (l.ld_col & 1) == 0 && (reinterpret_cast<uintptr_t>(l.bt) & 3) == 0;
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt) {
     const __nv_bfloat16* p = l.bt + (n + 8 * nt + g) * l.ld_col;

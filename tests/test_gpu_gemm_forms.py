@@ -147,3 +147,30 @@ def test_o_projection_does_not_depend_on_the_rows():
     whole = run(300)
     for M in (64, 128, 200, 256):
         assert torch.equal(run(M), whole[:, :M]), M
+
+
+@pytest.mark.parametrize("T", [40, 100, 300])
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_lora_factors_at_any_address(T, offset):
+    """LoRA-B factors that start at an odd element, or off a 16-byte boundary (slices of a flat buffer): the same bits."""
+    from hyc_lora_release_b200 import mlp
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(T)
+    H, I, q = 512, 4352, 4
+    x, wg, wu, wd, gy = _rn(g, T, H), _rn(g, I, H, scale=0.04), _rn(g, I, H, scale=0.04), _rn(g, H, I, scale=0.04), _rn(g, T, H)
+    xa, b, s = _rn(g, T, 16), _rn(g, I, 16, scale=0.3), torch.full((I,), 0.25, dtype=BF16, device=DEV)
+    flat = torch.empty(b.numel() + offset, dtype=BF16, device=DEV)[offset:]
+    moved = flat.copy_(b.reshape(-1)).view(I, 16)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(b):
+        q1, q2 = (torch.zeros(T, I * q // 8, dtype=torch.uint8, device=DEV) for _ in range(2))
+        o, had, gg, gu = (torch.zeros((T, I), dtype=BF16, device=DEV) for _ in range(4))
+        check(lib.hyc_mlp_gateup_fwd_tcgen05(ptr(x), ptr(wg), ptr(wu), T, H, I, ptr(xa), ptr(b), 16, 1, ptr(xa), ptr(b), 16, 1, ptr(s), ptr(s),
+                                             ptr(q1), ptr(q2), ptr(o), None, None, q, ptr(st), stream_of(x)), "gateup")
+        check(lib.hyc_mlp_graddown_bwd_tcgen05(ptr(gy), ptr(wd), T, H, I, None, None, 0, ptr(xa), ptr(b), 16, 1, ptr(xa), ptr(b), 16, 1,
+                                               ptr(q1), ptr(s), ptr(q2), ptr(s), None, None, 0, ptr(had), ptr(gg), ptr(gu), q, ptr(st),
+                                               stream_of(x)), "graddown")
+        return [o, q1, q2, had, gg, gu, *mlp.linear_lora_save(x, wg, None, b, s, q, xa=xa, status=st)]
+    assert all(torch.equal(u, v) for u, v in zip(run(moved), run(b)))
+    assert int(st.item()) == 0
