@@ -6,8 +6,12 @@ PYBIND11_MODULE(_hyc_host, m) {
   pybind11::register_exception_translator([](std::exception_ptr p) {
     try {
       if (p) std::rethrow_exception(p);
+    } catch (const Error& e) {
+      PyErr_SetString(error.ptr(), e.what());
     } catch (const c10::ValueError& e) {
       PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
+    } catch (const c10::IndexError& e) {
+      PyErr_SetString(PyExc_IndexError, e.what_without_backtrace());
     } catch (const c10::OutOfMemoryError& e) {
       PyErr_SetString(pybind11::module_::import("torch").attr("OutOfMemoryError").ptr(), e.what_without_backtrace());
     } catch (const c10::Error& e) {

@@ -29,3 +29,12 @@ def test_rows_of_no_columns_are_an_error():
                  lambda: rn.rmsnorm_backward_packed(none, one, one, None, None, one, one, 4)):
         with pytest.raises(ValueError, match="empty"):
             call()
+
+
+@pytest.mark.gpu
+def test_error_codes_become_hyc_errors():
+    """A code that the library returns is a HycError on both paths to it."""
+    from hyc_lora_release_b200._lib import HycError
+    from hyc_lora_release_b200.operators import compress_function as cf
+    with pytest.raises(HycError, match="hyc_softmax_topk_compress"):
+        cf.compression_softmax_topk(torch.zeros(1, 1, 8, 72, device="cuda"), 0.05)
