@@ -847,7 +847,7 @@ extern "C" HYC_API int hyc_attn_fwd_tcgen05(
   if (!q || !k || !v || !o || !status || (o_codes != nullptr) != (o_scale != nullptr) || (cls && !mask)) return HYC_ERR_NULL;
   if (const int rc = at_check(B, M, heads, kv_heads, head_dim)) return rc;
   if (o_codes && q_bit != 2 && q_bit != 4 && q_bit != 8) return HYC_ERR_QBIT;
-  const void* al[] = {q, k, v, o, map, mask, cls, o_codes};
+  const void* al[] = {q, k, v, o, map, mask, cls, o_codes, o_scale};
   for (const void* x : al) if (x && !aligned(x, 16)) return HYC_ERR_ALIGN;
   if (mask && ((mask_b | mask_h | mask_row) & 7)) return HYC_ERR_ALIGN;
   FwdMaps maps;

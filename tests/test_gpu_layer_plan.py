@@ -198,3 +198,19 @@ def test_head_geometry_and_scale_that_do_not_fit_are_refused(stepwise):
     # (a failed call may have advanced one half: what counts is that the launches of a right call are unharmed)
     p.layer.iteration = 10
     assert _same(p.step(), want)
+
+
+def _at_offset(t, n):
+    """A copy of ``t`` that starts n elements behind a 16-byte boundary."""
+    flat = torch.empty(t.numel() + n, dtype=t.dtype, device=t.device)[n:]
+    return flat.copy_(t.reshape(-1)).view(t.shape)
+
+
+@pytest.mark.parametrize("n", [1, 2, 4])
+def test_misaligned_scale_of_o_is_refused(n):
+    from hyc_lora_release_b200._lib import HycError
+    p = Problem()
+    entry = p.layer.attn_state.static_value["o"]
+    entry["scale"] = _at_offset(entry["scale"].to(BF16), n)
+    with pytest.raises(HycError, match="align"):
+        p.forward(p.x)
