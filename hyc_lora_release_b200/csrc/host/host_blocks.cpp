@@ -9,6 +9,12 @@ namespace hyc_host {
 
 static int* status_ptr(const Tensor& st) { return (int*)st.data_ptr(); }
 
+// a LoRA-B factor as the kernels load it: contiguous and on a 16-byte boundary (one that is a slice of a flat buffer is copied)
+static Tensor factor(const Tensor& b) {
+  const Tensor c = b.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
+}
+
 // sum of a_i op(b_i) (+ residual), one to four K segments
 struct Segment { const Tensor *a, *b; };
 static Tensor gemm(std::initializer_list<Segment> segs, int form, const Tensor* residual, const Tensor& status) {
@@ -78,7 +84,7 @@ static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, c
     n[i] = (int)w[i]->size(0);
     out[i] = {empty({T, n[i]}, x), empty({T, n[i] * q_bit / 8}, x, at::kByte)};
     keep[2 * i] = vec(*scale[i]);
-    keep[2 * i + 1] = b[i]->contiguous();
+    keep[2 * i + 1] = factor(*b[i]);
     wp[i] = data(*w[i]); xp[i] = (const char*)xa3.data_ptr() + i * T * 16 * 2; bp[i] = data(keep[2 * i + 1]); sp[i] = data(keep[2 * i]);
     yp[i] = data(out[i].first); qp[i] = data(out[i].second);
   }
@@ -135,11 +141,11 @@ struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa,
 
 static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
                                        const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const FrozenWeight* wd_later = nullptr) {
-  const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &bg = w[4], &bu = w[5], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
+  const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
-  const Tensor gs = vec(stats[3]), us = vec(stats[4]);
   SameDevice{x_medium}.with(w).with(stats).with(bias_d).with(status);
   OnDevice on(x_medium);
+  const Tensor gs = vec(stats[3]), us = vec(stats[4]), bg = factor(w[4]), bu = factor(w[5]);
   const int64_t B = x_medium.size(0), M = x_medium.size(1), H = x_medium.size(2), T = B * M, I = wg.size(0);
   auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale);
   const Tensor xn2 = x_norm.view({T, H});
@@ -161,11 +167,11 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
 static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q,
                                              const Tensor& status) {
   const Tensor &wd = w[0], &ad_rows = w[4];
-  const Tensor bg = w[1].contiguous(), bu = w[2].contiguous(), bd = w[3].contiguous();
   const Tensor &gate_q = saved[0], &gate_s = saved[1], &up_q = saved[2], &up_s = saved[3], &gu_xa = saved[4], &down_xa = saved[5],
                &xn_q = saved[6], &xn_scale = saved[7];
   SameDevice{g}.with(w).with(saved).with(status);
   OnDevice on(g);
+  const Tensor bg = factor(w[1]), bu = factor(w[2]), bd = factor(w[3]);
   const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
   Tensor grad_bd = empty({H, 16}, g), gdm64 = empty({T, 64}, g), gm64 = empty({T, 64}, g), grad_ad = empty({16, I}, g),
          grad_bgu = empty({2, I, 16}, g);
@@ -328,7 +334,7 @@ static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, 
   SameDevice{g}.with(wo).with(bo_in).with(ao_rows).with(o_xa).with(o_q).with(o_scale).with(status);
   OnDevice on(g);
   const int64_t T = g.size(0);
-  const Tensor bo = bo_in.contiguous();
+  const Tensor bo = factor(bo_in);
   Tensor gm64 = empty({T, 64}, g), grad_bo = empty({g.size(1), 16}, g);
   Skinny().on(g).rows(data(bo), 16, gm64, 0, 64, 48).cols(data(o_xa), o_xa.stride(0), data(grad_bo)).run(T, g, status, on.stream);
   Tensor grad_ao = lora_grad_a(o_q, vec(o_scale), gm64, 16, q);
@@ -360,7 +366,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
       n[i] = (int)((i == 0 ? nh : nkv) * d);
       rebuilt[i] = empty({T, n[i]}, grad_o2);
       cp[i] = data(keep[3 * i] = saved[3 * i].contiguous()); sp[i] = data(keep[3 * i + 1] = vec(saved[3 * i + 1]));
-      xp[i] = data(saved[3 * i + 2]); bp[i] = data(keep[3 * i + 2] = w[i].contiguous()); yp[i] = data(rebuilt[i]);
+      xp[i] = data(saved[3 * i + 2]); bp[i] = data(keep[3 * i + 2] = factor(w[i])); yp[i] = data(rebuilt[i]);
     }
     check(hyc_rebuild_qkv(cp, sp, xp, bp, yp, n, data(tables.cos), data(tables.sin), tables.cos.stride(0), tables.f32(), T, (int)M, (int)q, on.stream),
           "hyc_rebuild_qkv");
@@ -411,7 +417,7 @@ static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, 
   Skinny s;
   for (int i = 0; i < 3; ++i) {
     gb[i] = empty({grads[i].size(1), 16}, grads[0]);
-    b[i] = b_in[i].contiguous();
+    b[i] = factor(b_in[i]);
     s.on(grads[i]).rows(data(b[i]), 16, gmq, 16 * i, 64, i == 2 ? 16 : 0).cols(at_row(qkv_xa, i), 16, data(gb[i]));
   }
   s.run(T, gmq, status, on.stream);

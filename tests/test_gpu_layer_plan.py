@@ -214,3 +214,15 @@ def test_misaligned_scale_of_o_is_refused(n):
     entry["scale"] = _at_offset(entry["scale"].to(BF16), n)
     with pytest.raises(HycError, match="align"):
         p.forward(p.x)
+
+
+@pytest.mark.parametrize("stepwise", [False, True])
+@pytest.mark.parametrize("n", [2, 4])
+def test_adapters_off_a_16_byte_boundary(n, stepwise):
+    """Adapters that are slices of a flat buffer: the same step, bit for bit."""
+    p = Problem()
+    p.layer.keep_saved = stepwise
+    want = p.step()
+    for w in p.lora():
+        w.data = _at_offset(w.data, n)
+    assert _same(p.step(), want)
