@@ -210,6 +210,10 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
         self._weights = None
         self._plan = None
 
+    def __getstate__(self):
+        """For copies and files: without what the next call binds anew (the plan is a native object of this process)."""
+        return {**self.__dict__, "_weights": None, "_plan": None}
+
     def _status_for(self, device):
         if self._status is None or self._status.device != device:
             self._status = torch.zeros(1, dtype=torch.int32, device=device)

@@ -89,3 +89,23 @@ def test_head_geometry_is_checked_against_the_projections(heads, d, kv):
     with pytest.raises(RuntimeError, match="head"):
         host.attn_backward_map(t(8, 512), t(1, 4, 8, 8), [], 0, [t(8, 1)] * 9, w[4:7], t(8, 128), t(8, 128), 1, 8, heads, d, kv, 4, None, 0, 0,
                                torch.zeros(1, dtype=torch.int32))
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "file"])
+def test_a_bound_layer_can_be_copied_and_saved(bound, how):
+    import copy
+    import io
+    layer, bind, mods = bound
+    bind()
+    layer.iteration = 7
+    if how == "deepcopy":
+        other = copy.deepcopy(layer)
+    else:
+        f = io.BytesIO()
+        torch.save(layer, f)
+        f.seek(0)
+        other = torch.load(f, weights_only=False)
+    assert other.iteration == 7 and layer._plan is not None
+    norms = layer._weights[1].norm_w, layer._weights[2].norm_w
+    other._bind(*norms, mods)
+    assert other._plan.fresh() and other._plan is not layer._plan
