@@ -474,6 +474,8 @@ struct LayerPlan {
     if ((int)pad.size() != PADS) return false;
     for (const FrozenWeight& f : w)
       if (f.plain.defined() && f.plain.scalar_type() != at::kBFloat16) return false;
+    for (const OptTensor* b : {&bias_o, &bias_d})
+      if (given(*b) && (*b)->scalar_type() != at::kBFloat16) return false;
     for (int i = 0; i < 2 * PROJECTIONS; ++i)
       if (lora[i].scalar_type() != at::kBFloat16 || !pad_of[i].fits(lora[i])) return false;
     return true;

@@ -281,7 +281,8 @@ class FusedLlamaLayerIntraInterFullFuse(torch.nn.Module):
             # (a 4-bit weight is wrapped once: the parameter and its quant state are what identify it)
             key += (id(w), id(w.__dict__.get("quant_state") if type(w) is torch.nn.Parameter else getattr(w, "quant_state", None)),
                     id(_adapter_weight(la)), id(_adapter_weight(lb)), id(_entry(base, "_parameters", "bias", None)))
-        if self._weights is not None and self._weights[0] == key and (self._plan is None or self._plan.fresh()):
+        # fresh() looks at what the checks below look at (without a plan they are made on every call)
+        if self._weights is not None and self._weights[0] == key and self._plan is not None and self._plan.fresh():
             return self._weights[1:]
         tensors = [norm_w1, norm_w2]
         biases = {}

@@ -109,3 +109,22 @@ def test_a_bound_layer_can_be_copied_and_saved(bound, how):
     norms = layer._weights[1].norm_w, layer._weights[2].norm_w
     other._bind(*norms, mods)
     assert other._plan.fresh() and other._plan is not layer._plan
+
+
+@pytest.mark.parametrize("with_plan", [True, False])
+@pytest.mark.parametrize("what", ["weight", "adapter type", "adapter rank", "o bias", "down bias"])
+def test_a_parameter_that_stops_fitting_is_refused(bound, what, with_plan):
+    """The parameters are the same objects; what ``.data`` holds has become something that the layer refuses."""
+    layer, bind, mods = bound
+    biased = ("o", "down") if with_plan else ("o", "down", "q")
+    for n in biased:
+        base = mods[n][0]
+        base.bias = torch.nn.Parameter(torch.zeros(base.weight.shape[0], dtype=torch.bfloat16), requires_grad=False)
+    bind()
+    assert (layer._plan is not None) == with_plan
+    bind()
+    p = {"weight": mods["up"][0].weight, "adapter type": mods["k"][1].default.weight, "adapter rank": mods["k"][1].default.weight,
+         "o bias": mods["o"][0].bias, "down bias": mods["down"][0].bias}[what]
+    p.data = p.data[:8] if what == "adapter rank" else p.data.float()
+    with pytest.raises(NotImplementedError):
+        bind()
