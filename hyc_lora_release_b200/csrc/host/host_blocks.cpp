@@ -485,16 +485,19 @@ struct LayerPlan {
     pad = p;
     for (int i = 0; i < 2 * PROJECTIONS; ++i) pad_of[i] = Stamp::of(lora[i]);
   }
+  // A statistic that the kernels read where it lies is looked up once.  One that has to be converted is converted on every
+  // call: the copy could not follow a write that bumps no version (through `.data`, or to an inference tensor).
   void set_stats(const std::vector<Tensor>& s) {
-    bool same = s.size() == stats_in.size();
-    for (size_t i = 0; same && i < s.size(); ++i) same = s[i].unsafeGetTensorImpl() == stats_in[i].unsafeGetTensorImpl() && stats_of[i].fits(s[i]);
-    if (same) return;
-    stats_in = s;
-    stats.clear();
-    stats_of.clear();
-    for (const Tensor& t : s) {
-      stats_of.push_back(Stamp::of(t));
-      stats.push_back(t.scalar_type() == at::kLong ? t.contiguous() : vec(t));
+    stats_in.resize(s.size());
+    stats.resize(s.size());
+    stats_of.resize(s.size());
+    for (size_t i = 0; i < s.size(); ++i) {
+      if (stats_in[i].defined() && s[i].unsafeGetTensorImpl() == stats_in[i].unsafeGetTensorImpl() && stats_of[i].fits(s[i])) continue;
+      Tensor now = s[i].scalar_type() == at::kLong ? s[i].contiguous() : vec(s[i]);
+      const bool in_place = now.storage().unsafeGetStorageImpl() == s[i].storage().unsafeGetStorageImpl();
+      stats[i] = std::move(now);
+      stats_in[i] = in_place ? s[i] : Tensor();
+      if (in_place) stats_of[i] = Stamp::of(s[i]);
     }
   }
 };

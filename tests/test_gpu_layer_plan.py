@@ -226,3 +226,19 @@ def test_adapters_off_a_16_byte_boundary(n, stepwise):
     for w in p.lora():
         w.data = _at_offset(w.data, n)
     assert _same(p.step(), want)
+
+
+def test_statistics_written_behind_the_version_counter():
+    """Statistics that the kernels read as a converted copy (here fp32) count as they are at the call."""
+    p = Problem()
+    for state in (p.layer.attn_state, p.layer.mlp_state):
+        for entry in state.static_value.values():
+            if entry.get("scale") is not None:
+                entry["scale"] = entry["scale"].float()
+    before = p.step()
+    for state in (p.layer.attn_state, p.layer.mlp_state):
+        for entry in state.static_value.values():
+            if entry.get("scale") is not None:
+                entry["scale"].data.mul_(2)
+    after = p.step()
+    assert not _same(after, before) and _same(after, p.step(layer=p.fresh_layer()))
