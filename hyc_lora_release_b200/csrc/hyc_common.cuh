@@ -54,9 +54,8 @@ inline int resident_blocks(K kern, int threads, size_t smem, int otherwise) {
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may begin before the kernel in front of it in the
 // stream has ended, and has to call pdl_wait() before it touches memory (pdl_wait returns once that kernel, and with
-// it everything before, is complete and visible).  pdl_trigger() in the kernel in front lets the launch go out.
+// it everything before, is complete and visible).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename K, typename... A>
 inline int launch_pdl(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -9,7 +9,6 @@
 // of the B block), which cuts what an SM pulls out of L2 per k-block from 32 to 24 KB; a cluster is then 2 S CTAs.
 // The reduction order is fixed (rank 0, 1, ...), so results do not depend on the run.
 #include "tc_split.cuh"
-#include <stdlib.h>
 
 namespace hyc {
 namespace tc {
@@ -20,7 +19,7 @@ constexpr int S_MAX_STAGES = 8;
 constexpr int S_EPI_BYTES = 1024;                 // per-column constants
 constexpr int S_THREADS = 64 + 128;
 constexpr int S_PART_BYTES = SBN * BM * 4;        // the CTA's accumulators as [column][row], over the drained stages
-static_assert(S_PART_BYTES + 4 * 4096 <= S_PIPE_BYTES, "partials and the GRADDOWN tiles fit in the drained pipeline");
+static_assert(S_PART_BYTES + 4 * 4096 <= S_PIPE_BYTES, "partials and the epilogue's tiles fit in the drained pipeline");
 constexpr int split_smem_bytes(int pipe) { return 1024 + pipe + S_EPI_BYTES + 256; }
 
 __device__ __forceinline__ void s_epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
@@ -54,6 +53,7 @@ __device__ __forceinline__ void gather32(int split, int first, int step, uint32_
 template <int EPI, int QBIT, bool B_MN, bool PAIR>
 __global__ void __launch_bounds__(S_THREADS, 2)
 split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, int stages, int a_bytes) {
+  static_assert(EPI == EPI_STORE || (EPI == EPI_GATEUP && !PAIR && !B_MN), "the forms that choose_split picks");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
@@ -104,12 +104,10 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
   const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
   float* part = reinterpret_cast<float*>(smem);
   float* sV = reinterpret_cast<float*>(epi);                       // quantizer constants (GATEUP: second vector at sV + 64)
-  __nv_bfloat16* sS = reinterpret_cast<__nv_bfloat16*>(sV);        // GRADDOWN: two bf16 scale vectors of 128
   const int per = UNITS / split, first = rank * per;               // the 32-column blocks this CTA finishes
   LoraA a1, a2;
   LoraB b1, b2;
   uint4 res[4];
-  GdInputs<QBIT> gin;
   bool ok = true;
 
   if (warp == 0) {
@@ -131,12 +129,8 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
         if (elect_one()) {
         if (half == 0) mbar_expect_tx(&full[stage], (uint32_t)((PAIR ? 2 : 1) * stage_bytes));      // the leader counts both CTAs' bytes
         if (EPI == EPI_GATEUP) {
-          if (PAIR) {
-            tma_load_2d<PAIR>(sb, half == 0 ? &maps.b[0] : &maps.b[1], fbar, k0, n0);
-          } else {
-            tma_load_2d<PAIR>(sb, &maps.b[0], fbar, k0, n0);
-            tma_load_2d<PAIR>(sb + 8192, &maps.b[1], fbar, k0, n0);
-          }
+          tma_load_2d<PAIR>(sb, &maps.b[0], fbar, k0, n0);
+          tma_load_2d<PAIR>(sb + 8192, &maps.b[1], fbar, k0, n0);
         } else if (B_MN) {
           tma_load_2d<PAIR>(sb, mb, fbar, n0 + 64 * half, k0);
           if (!PAIR) tma_load_2d<PAIR>(sb + 8192, mb, fbar, n0 + 64, k0);
@@ -189,7 +183,7 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
         lora_load_b(sv.l0, (int64_t)sv.n0 + 32 * first, lane, b1);
       }
       if (sv.residual != nullptr) tile_fetch(sv.residual, row0, p.M, sv.ld, (int64_t)sv.n0 + 32 * first, lane, res);
-    } else if (EPI == EPI_GATEUP) {
+    } else {
       if (et < TILE_N) {
         sV[et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(p.s1[nt + et])));
         sV[64 + et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(p.s2[nt + et])));
@@ -198,12 +192,6 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
       lora_load_a(p.l1.xa, row0, p.M, lane, a2);
       lora_load_b(p.l0, (int64_t)nt + 32 * first, lane, b1);
       lora_load_b(p.l1, (int64_t)nt + 32 * first, lane, b2);
-    } else {
-      sS[et] = p.s1[nt + et];
-      sS[128 + et] = p.s2[nt + et];
-      lora_load_a(p.l1.xa, row0, p.M, lane, a1);
-      lora_load_a(p.l2.xa, row0, p.M, lane, a2);
-      gd_fetch<QBIT>(p, row0, lane, (int64_t)nt + 32 * first, gin);
     }
     s_epi_sync();
     ok = mbar_wait(acc_full, 0, abort_flag);
@@ -244,19 +232,13 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
         gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
         gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, TILE_N + cb, r, up);
         epi_gateup_block<QBIT>(p, row0, lane, nt, cb, acc, up, a1, a2, n1, n2, sV, sV + 64, R1, R2);
-      } else if (EPI == EPI_STORE) {
+      } else {
         const uint4 now[4] = {res[0], res[1], res[2], res[3]};
         const LoraB n1 = b1;
         if (more && sv.residual != nullptr) tile_fetch(sv.residual, row0, p.M, sv.ld, (int64_t)sv.n0 + cb + 32, lane, res);
         if (more && sv.l0.bt != nullptr) lora_load_b(sv.l0, (int64_t)sv.n0 + cb + 32, lane, b1);
         gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
         epi_store_block<QBIT>(sv, row0, lane, p.M, cb, acc, a1, n1, sV, now, R1, R2);
-      } else {
-        const GdInputs<QBIT> cur = gin;
-        if (more) gd_fetch<QBIT>(p, row0, lane, (int64_t)nt + cb + 32, gin);
-        gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
-        epi_graddown_block<QBIT>(p, row0, lane, nt, cb, acc, cur, a1, a2, R1, R2, reinterpret_cast<const uint32_t*>(sS),
-                                 reinterpret_cast<const uint32_t*>(sS + 128));
       }
     }
   }
@@ -310,24 +292,21 @@ static int launch_one(int split, const Operands& ops, const Params& p, cudaStrea
   return HYC_OK;
 }
 
+// (only the forms that choose_split picks: products with codes in their epilogue are never split, so never paired)
 int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Operands& ops, const Params& p, cudaStream_t st) {
-#define HYC_SPLIT(E, Q, MN) \
-  return plan.pair ? launch_one<E, Q, MN, true>(plan.split, ops, p, st) : launch_one<E, Q, MN, false>(plan.split, ops, p, st)
-  if (epi == EPI_STORE) {
-    if (b_mn) HYC_SPLIT(EPI_STORE, 4, true);
-    if (q_bit == 2) HYC_SPLIT(EPI_STORE, 2, false);
-    if (q_bit == 8) HYC_SPLIT(EPI_STORE, 8, false);
-    HYC_SPLIT(EPI_STORE, 4, false);
-  }
   if (epi == EPI_GATEUP) {
-    if (q_bit == 2) HYC_SPLIT(EPI_GATEUP, 2, false);
-    if (q_bit == 8) HYC_SPLIT(EPI_GATEUP, 8, false);
-    HYC_SPLIT(EPI_GATEUP, 4, false);
+    if (q_bit == 2) return launch_one<EPI_GATEUP, 2, false, false>(plan.split, ops, p, st);
+    if (q_bit == 8) return launch_one<EPI_GATEUP, 8, false, false>(plan.split, ops, p, st);
+    return launch_one<EPI_GATEUP, 4, false, false>(plan.split, ops, p, st);
   }
-  if (q_bit == 2) HYC_SPLIT(EPI_GRADDOWN, 2, true);
-  if (q_bit == 8) HYC_SPLIT(EPI_GRADDOWN, 8, true);
-  HYC_SPLIT(EPI_GRADDOWN, 4, true);
-#undef HYC_SPLIT
+  if (b_mn) {
+    if (plan.pair) return launch_one<EPI_STORE, 4, true, true>(plan.split, ops, p, st);
+    return launch_one<EPI_STORE, 4, true, false>(plan.split, ops, p, st);
+  }
+  if (plan.pair) return launch_one<EPI_STORE, 4, false, true>(plan.split, ops, p, st);
+  if (q_bit == 2) return launch_one<EPI_STORE, 2, false, false>(plan.split, ops, p, st);
+  if (q_bit == 8) return launch_one<EPI_STORE, 8, false, false>(plan.split, ops, p, st);
+  return launch_one<EPI_STORE, 4, false, false>(plan.split, ops, p, st);
 }
 
 // Where the line lies (B200, Llama-2-7B weights, us per product, persistent / split):
