@@ -68,6 +68,38 @@ def _same(got, want):
     return all(torch.equal(a, b) for a, b in zip(got, want, strict=True))
 
 
+@pytest.mark.parametrize("shape", [dict(), dict(map_mode="prune", q=2), dict(B=2, M=200, map_mode="prune", kv=4, q=8), dict(M=320, q=8),
+                                   dict(B=3, M=8, map_mode="prune"), dict(M=264, map_mode="prune", heads=6), dict(M=64, bias=("o", "down")),
+                                   dict(heads=8, kv=4, d=64, M=136, map_mode="prune"), dict(heads=8, d=64, kv=8, M=128), dict(M=1088, map_mode="topk")])
+def test_plan_equals_the_stepwise_path(shape):
+    """The step-wise path is what the oracle tests hold; the plan runs the same launches: equal bits, also after the adapters
+    have changed between two steps."""
+    p = Problem(**shape)
+    for _ in range(2):
+        assert p.layer._steady()
+        got = p.step()
+        p.layer.keep_saved = True
+        want = p.step()
+        p.layer.keep_saved = False
+        assert _same(got, want) and _same(got, p.step(layer=p.fresh_layer()))
+        with torch.no_grad():
+            for i, w in enumerate(p.lora()):
+                w.mul_(1 + 0.1 * i)
+    p.layer.raise_on_device_errors()
+
+
+@pytest.mark.parametrize("stepwise", [False, True])
+@pytest.mark.parametrize("M", [100, 4104])
+def test_lengths_outside_the_softmax_kernels_are_refused(M, stepwise):
+    from hyc_lora_release_b200._lib import HycError
+    p = Problem(heads=2, map_mode="prune")
+    p.layer.keep_saved = stepwise
+    x = torch.zeros(1, M, 256, dtype=BF16, device=DEV)
+    p.cos, p.sin = torch.ones(M, 128, dtype=BF16, device=DEV), torch.zeros(M, 128, dtype=BF16, device=DEV)
+    with pytest.raises(HycError, match="shape"):
+        p.forward(x, mask=torch.zeros(1, 1, M, M, dtype=BF16, device=DEV))
+
+
 @pytest.mark.parametrize("map_mode", ["topk", "prune"])
 @pytest.mark.parametrize("stepwise", [False, True])
 def test_step_captured_after_eager_steps(map_mode, stepwise):
