@@ -590,8 +590,8 @@ def mlp_eager_baseline(dev, B, M, H, I, R, steps=200, warmup=5):
 
 
 def mlp_workload(dev, dist=None, steps=200, warmup=5, shape="llama", q_bit=4, eager=False):
-    """Fused LoRA-SiLU-Hadamard MLP forward + backward.  shape "llama" = BASELINE configs[2]: x [4,512,4096] per
-    GPU, intermediate 11008, 0.5 % outlier channels x30; shape "mistral" = BASELINE configs[3]: 8192 tokens per GPU,
+    """Fused LoRA-SiLU-Hadamard MLP forward + backward.  shape "llama": x [4,512,4096] per
+    GPU, intermediate 11008, 0.5 % outlier channels x30; shape "mistral": 8192 tokens per GPU,
     intermediate 14336, 1 % outlier channels x20.  Frozen W ~ N(0, .02), LoRA rank 16, saved activations q_bit
     wide; calibration (5 iterations, statistics synchronised across ranks) happens before the timed region.  With
     several ranks every rank runs its OWN token shard (inputs seeded per rank, weights shared) and the six LoRA
@@ -679,8 +679,8 @@ def mlp_workload(dev, dist=None, steps=200, warmup=5, shape="llama", q_bit=4, ea
 
 
 def layer_workload(dev, dist=None, steps=80, warmup=3, graph=True):
-    """One fused decoder layer (attention + MLP) forward + backward at the Llama-2-7B geometry of BASELINE
-    configs[4]: hidden 4096, 32 heads of 128, intermediate 11008, sequence 2048, batch 1 per GPU, causal mask,
+    """One fused decoder layer (attention + MLP) forward + backward at the Llama-2-7B geometry:
+    hidden 4096, 32 heads of 128, intermediate 11008, sequence 2048, batch 1 per GPU, causal mask,
     LoRA rank 16 on q/k/v/o/gate/up/down, saved activations 4-bit with 0.5 % outlier channels, the probability
     map [1,32,2048,2048] saved as per-row top-k (5 %) + 4-bit groups.  Driven through the layer module and
     autograd (the call a model fork makes); calibration happens before the timed region."""
@@ -796,12 +796,12 @@ def layer_workload(dev, dist=None, steps=80, warmup=3, graph=True):
             "identical_grads_on_all_ranks": ranks_hold_identical(reducer, dist),
             "roofline": {"bound": "tensor", "achieved": tf, "peak": sustained, "unit": "TFLOP/s", "frac": tf / sustained,
                          "peak_source": src + " (sustained)"},
-            "note": "the two attention products per direction are library batched GEMMs and, like every pass over the "
-                    "[1,32,2048,2048] map (softmax, save, restore, softmax backward), bound by HBM, not by the tensor cores"}
+            "note": "attention runs on tcgen05 kernels (one forward, two backward) bound by their element-wise work; the save of "
+                    "the [1,32,2048,2048] map is bound by instruction issue, its restore by HBM, not by the tensor cores"}
 
 
 def model_workload(dev, dist=None, steps=4, warmup=3, n_layers=32, graph=True):
-    """One training step (forward + backward) of the whole 32-layer stack of BASELINE configs[4]: token embedding
+    """One training step (forward + backward) of the whole 32-layer Llama-2-7B stack: token embedding
     (vocabulary 32000, hidden 4096), 32 fused decoder layers driven through the layer module (32 heads of 128,
     intermediate 11008, LoRA rank 16 on q/k/v/o/gate/up/down, 4-bit saves, top-k map), final RMSNorm, the
     vocabulary projection and a cross-entropy loss on random token ids uniform in [0,32000), sequence 2048,
@@ -957,7 +957,7 @@ def model_workload(dev, dist=None, steps=4, warmup=3, n_layers=32, graph=True):
            "roofline": {"bound": "tensor", "achieved": tf, "peak": sustained, "unit": "TFLOP/s", "frac": tf / sustained,
                         "peak_source": src + " (sustained)"},
            "note": "embedding lookup and the cross-entropy are torch glue; every other launch is a kernel of this library "
-                   "except the batched attention products and the rank-16 skinny products (library GEMMs)"}
+                   "except the forward rank-16 products of the LoRA-A factors (library GEMMs)"}
     return out
 
 

@@ -15,7 +15,8 @@ in its grouped key/value heads, which are covered) with plain bf16 frozen weight
             grad_q, then grad_k and grad_v -> inverse rotary -> LoRA gradients of q/k/v (A side from the packed
             x_norm in one pass for the three adapters) -> grad_x as ONE GEMM over four K segments -> RMSNorm
             backward from the packed x with the residual gradient added in the same pass.
-Head sizes other than 128 and sequences that are no multiple of 8 take library batched products for the attention part.
+Head sizes other than 128 take library batched products for the attention part.  Sequences that are no multiple of 8 or longer
+than 4096 are refused by the softmax that these products need, and by the attention kernels.
 
 Weights use the nn.Linear layout ([out, in]); LoRA factors are ``lora_A.weight`` [r, in] and
 ``lora_B.weight`` [out, r].

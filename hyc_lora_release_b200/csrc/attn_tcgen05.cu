@@ -16,14 +16,15 @@
 //
 // CTA (one per SM): warp 0 loads (TMA, ring of 32 KB tiles), warp 1 issues the MMAs, the other sixteen (kv kernel: eight)
 // do the element-wise work, each a 32-row quadrant and a quarter of the tile's columns (with eight warps of 64 columns
-// the schedulers issued 0.3 instructions a cycle; [1,32,2048,2048] forward 173 us against 143 us with sixteen).  Scores /
+// the schedulers issued 0.3 instructions a cycle; [1,32,2048,2048] forward 173 us against 139 us with sixteen).  Scores /
 // dP are double-buffered in tensor memory, so the next tile's product runs while this one is worked on; P and dS go back
 // to tensor memory as the A operand of the second product.  Every wait is bounded (see tc_common.cuh).
 //
-// What bounds them: the forward and q kernels the element-wise work (issue slots 0.4 of one per cycle and scheduler,
-// waits on tensor memory and barriers in between), the kv kernel its loads (two 32 KB tiles per product).  Measured
-// [1,32,2048,2048] causal: forward 143 us for 512 MB of map traffic saved, backward 195 us; the separate steps took
-// 110 + 104 + 107 us (products, softmax) and 330 us.
+// What bounds them: the forward and q kernels the element-wise work (issue slots 0.47 and 0.39 of one per cycle and
+// scheduler, waits on tensor memory and loads in between; DRAM at 28 and 46 %), the kv kernel its loads (two 32 KB tiles per
+// product; issue slots 0.08, DRAM 56 %).  The tensor pipe is busy a fifth of the time in all three.  Measured
+// [1,32,2048,2048] causal: forward 139 us for 512 MB of map traffic saved, backward 117 + 76 us (204 us as a call from a cold
+// L2); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
 #include "tc_common.cuh"
 #include <math.h>
 

@@ -315,6 +315,8 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
 //     more column tiles than SMs can take at once either way and stays persistent: 28.8 / 30.3
 //   129 to 256 tokens, pair form, S = 2: 21.8 / 19.0, 43 / 30.6, 69 / 45; wider products fill the chip without it
 //   512 tokens: 45 / 47, 75 / 77: persistent
+//   (cold L2, each call with its own pair of events, which adds about 5 us: x[4096,11008] of 128 tokens 57 / 35, of 200 tokens
+//   51 / 41, grad_o 27 / 23 and 27 / 25)
 // A CTA keeps at least 16 k-blocks: below that its share of the main loop is shorter than set-up and reduction (about
 // 3 us), and the sum over all of K stays in one accumulator.
 // Products whose results the layer quantizes, or that feed tensors it quantizes in the same pass, are not split (gate/up, q/k/v,
