@@ -9,6 +9,16 @@ namespace hyc_host {
 
 static int* status_ptr(const Tensor& st) { return (int*)st.data_ptr(); }
 
+// what the kernels read by address and stride alone: a contiguous bf16 matrix of the size that the product needs
+static void expect(const Tensor& t, int64_t rows, int64_t cols, const char* what) {
+  TORCH_CHECK(t.dim() == 2 && t.size(0) == rows && t.size(1) == cols && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), what,
+              ": expected a contiguous bf16 [", rows, ", ", cols, "] matrix, got ", t.scalar_type(), " ", t.sizes(), " with strides ", t.strides());
+}
+static void expect_factor(const Tensor& b, int64_t rows, const char* what) {      // any strides
+  TORCH_CHECK(b.dim() == 2 && b.size(0) == rows && b.size(1) == 16 && b.scalar_type() == at::kBFloat16, what, ": expected a bf16 [", rows,
+              ", 16] factor, got ", b.scalar_type(), " ", b.sizes());
+}
+
 // a LoRA-B factor as the kernels load it: contiguous and on a 16-byte boundary (one that is a slice of a flat buffer is copied)
 static Tensor factor(const Tensor& b) {
   const Tensor c = b.contiguous();
@@ -143,10 +153,16 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
                                        const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const FrozenWeight* wd_later = nullptr) {
   const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
+  const int64_t B = x_medium.size(0), M = x_medium.size(1), H = x_medium.size(2), T = B * M, I = wg.size(0);
+  expect(wg, I, H, "gate projection");
+  expect(wu, I, H, "up projection");
+  expect_factor(w[4], I, "gate lora_B");
+  expect_factor(w[5], I, "up lora_B");
+  expect(bd_cols, H, 64, "down lora_B");
+  const Tensor gs = scale_vec(stats[3], I), us = scale_vec(stats[4], I);
   SameDevice{x_medium}.with(w).with(stats).with(bias_d).with(status);
   OnDevice on(x_medium);
-  const Tensor gs = vec(stats[3]), us = vec(stats[4]), bg = factor(w[4]), bu = factor(w[5]);
-  const int64_t B = x_medium.size(0), M = x_medium.size(1), H = x_medium.size(2), T = B * M, I = wg.size(0);
+  const Tensor bg = factor(w[4]), bu = factor(w[5]);
   auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale);
   const Tensor xn2 = x_norm.view({T, H});
   const Tensor gu_xa = lora_a_products(xn2, agu_t);
@@ -158,6 +174,7 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   const Tensor down_xa64 = at::mm(had, ad_cols);
   const Tensor res = bf16c(x_medium), wd = wd_later ? matrices({wd_later})[0] : w[3];
   require_cuda({&x_medium, &wd});
+  expect(wd, H, I, "down projection");
   Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, 0, &res, status);
   if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
   return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
@@ -169,10 +186,15 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<
   const Tensor &wd = w[0], &ad_rows = w[4];
   const Tensor &gate_q = saved[0], &gate_s = saved[1], &up_q = saved[2], &up_s = saved[3], &gu_xa = saved[4], &down_xa = saved[5],
                &xn_q = saved[6], &xn_scale = saved[7];
+  const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
+  expect(wd, H, I, "down projection");
+  expect_factor(w[1], I, "gate lora_B");
+  expect_factor(w[2], I, "up lora_B");
+  expect_factor(w[3], H, "down lora_B");
+  expect(ad_rows, 64, I, "down lora_A");
   SameDevice{g}.with(w).with(saved).with(status);
   OnDevice on(g);
   const Tensor bg = factor(w[1]), bu = factor(w[2]), bd = factor(w[3]);
-  const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
   Tensor grad_bd = empty({H, 16}, g), gdm64 = empty({T, 64}, g), gm64 = empty({T, 64}, g), grad_ad = empty({16, I}, g),
          grad_bgu = empty({2, I, 16}, g);
   Skinny().on(g).rows(data(bd), 16, gdm64, 0, 64, 48).cols(data(down_xa), down_xa.stride(0), data(grad_bd)).run(T, g, status, on.stream);
@@ -194,6 +216,9 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<
 static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
                              at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wg = w[0], &wu = w[1], &agu_rows = w[2], &norm_w = w[3];
+  expect(wg, ggu.size(2), g.size(1), "gate projection");
+  expect(wu, ggu.size(2), g.size(1), "up projection");
+  expect(agu_rows, 64, g.size(1), "gate and up lora_A");
   SameDevice{g}.with(ggu).with(gm64).with(w).with(saved).with(status);
   const Tensor g0 = ggu[0], g1 = ggu[1];
   Tensor grad_xn = gemm({{&g0, &wg}, {&g1, &wu}, {&gm64, &agu_rows}}, HYC_GEMM_B_KN, nullptr, status);
@@ -274,6 +299,12 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
   const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
   check_geometry({wq.size(0), wk.size(0), wv.size(0)}, nh, d, nkv);
+  for (int i = 0; i < 3; ++i) {
+    const char* const names[3][2] = {{"q projection", "q lora_B"}, {"k projection", "k lora_B"}, {"v projection", "v lora_B"}};
+    expect(w[1 + i], w[1 + i].size(0), x.size(2), names[i][0]);
+    expect_factor(w[4 + i], w[1 + i].size(0), names[i][1]);
+    scale_vec(stats[3 + i], w[1 + i].size(0));
+  }
   SameDevice{x}.with(w).with(stats).with(tables.cos).with(tables.sin).with(mask).with(status);
   OnDevice on(x);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M, rep = nh / nkv;
@@ -313,6 +344,8 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
 // o projection with residual and the save of its input
 static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols,
                                             const Tensor& o_scale, const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& status) {
+  expect(wo, x.size(2), o2.size(1), "o projection");
+  expect(bo_cols, x.size(2), 64, "o lora_B");
   SameDevice{x}.with(o2).with(wo).with(ao_cols).with(bo_cols).with(o_scale).with(o_codes).with(bias_o).with(status);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
   const Tensor o_xa64 = at::mm(o2, ao_cols);
@@ -331,6 +364,9 @@ static Tensor rebuild(const Tensor& codes, const Tensor& scale, const Tensor& xa
 // o projection backward: -> grad_bo, grad_ao, grad_o2
 static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, const Tensor& bo_in, const Tensor& ao_rows, const Tensor& o_xa,
                                              const Tensor& o_q, const Tensor& o_scale, int64_t q, const Tensor& status) {
+  expect(wo, g.size(1), wo.size(1), "o projection");
+  expect_factor(bo_in, g.size(1), "o lora_B");
+  expect(ao_rows, 64, wo.size(1), "o lora_A");
   SameDevice{g}.with(wo).with(bo_in).with(ao_rows).with(o_xa).with(o_q).with(o_scale).with(status);
   OnDevice on(g);
   const int64_t T = g.size(0);
@@ -352,6 +388,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
   const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
                &v_s = saved[7], &v_xa = saved[8];
   check_geometry({w[0].size(0), w[1].size(0), w[2].size(0)}, nh, d, nkv);
+  for (int i = 0; i < 3; ++i) expect_factor(w[i], w[i].size(0), "lora_B of q, k or v");
   SameDevice{grad_o2}.with(a).with(topk).with(saved).with(w).with(tables.cos).with(tables.sin).with(cls).with(status);
   OnDevice on(grad_o2);
   const int64_t T = B * M, rep = nh / nkv;
@@ -410,6 +447,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
 // LoRA gradients of q/k/v: -> gmq [T, 64], ga [48, H], grad_bq, grad_bk, grad_bv
 static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, const std::vector<Tensor>& b_in, const Tensor& qkv_xa, const Tensor& xn_q,
                                               const Tensor& xn_scale, int64_t q, const Tensor& status) {
+  for (int i = 0; i < 3; ++i) expect_factor(b_in[i], grads[i].size(1), "lora_B of q, k or v");
   SameDevice{grads[0]}.with(grads).with(b_in).with(qkv_xa).with(xn_q).with(xn_scale).with(status);
   OnDevice on(grads[0]);
   const int64_t T = grads[0].size(0);
@@ -428,6 +466,8 @@ static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, 
 static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
   const Tensor &wq = w[0], &wk = w[1], &wv = w[2], &aqkv_rows = w[3], &norm_w = w[4];
+  for (int i = 0; i < 3; ++i) expect(w[i], grads[i].size(1), g.size(1), "q, k or v projection");
+  expect(aqkv_rows, 64, g.size(1), "lora_A of q, k and v");
   SameDevice{g}.with(grads).with(gmq).with(w).with(saved).with(status);
   Tensor grad_xn = gemm({{&grads[0], &wq}, {&grads[1], &wk}, {&grads[2], &wv}, {&gmq, &aqkv_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));

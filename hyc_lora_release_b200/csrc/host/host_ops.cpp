@@ -276,7 +276,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor&
   Tensor idx, sy;
   int64_t k = 0;
   if (given(idx_in)) { idx = index_of(*idx_in, x); k = idx.numel(); }
-  if (given(sy_in)) sy = vec(*sy_in);
+  if (given(sy_in)) sy = scale_vec(*sy_in, N);
+  TORCH_CHECK_VALUE(w.numel() == N, "norm weight with ", w.numel(), " entries for ", N, " channels");
   std::vector<int64_t> qs(xc.sizes().begin(), xc.sizes().end()), os = qs;
   qs.back() = N * q_bit / 8;
   os.back() = k;
@@ -295,7 +296,8 @@ Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor&
   const int64_t N = row_length(dy), rows = dy.numel() / N;
   require_cuda({&dy, &qx, &sx_in, &w_in, &rstd});
   OnDevice on(dy);
-  const Tensor dyc = bf16c(dy), sx = vec(sx_in), w = bf16c(w_in), q = qx.contiguous(), rs = rstd.contiguous();
+  const Tensor dyc = bf16c(dy), sx = scale_vec(sx_in, N), w = bf16c(w_in), q = qx.contiguous(), rs = rstd.contiguous();
+  TORCH_CHECK_VALUE(w.numel() == N, "norm weight with ", w.numel(), " entries for ", N, " channels");
   Tensor idx, xo, res;
   int64_t k = 0;
   if (given(idx_in)) { idx = index_of(*idx_in, dy); k = idx.numel(); }

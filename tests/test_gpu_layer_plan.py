@@ -274,3 +274,15 @@ def test_statistics_written_behind_the_version_counter():
                 entry["scale"].data.mul_(2)
     after = p.step()
     assert not _same(after, before) and _same(after, p.step(layer=p.fresh_layer()))
+
+
+def test_norm_weights_and_scales_of_another_length_are_refused():
+    from hyc_lora_release_b200.operators import rmsnorm_kernels as rk
+    x, w, s = torch.randn(8, 256, device=DEV).to(BF16), torch.ones(256, dtype=BF16, device=DEV), torch.ones(1, 256, dtype=BF16, device=DEV)
+    for ww, sx, sy in ((w[:128], s, s), (w, s[:, :64], s), (w, s, s[:, :64])):
+        with pytest.raises(ValueError, match="entries"):
+            rk.rmsnorm_forward_save(x, ww, 1e-5, 4, sx, None, sy)
+    _, rstd, _, q, _ = rk.rmsnorm_forward_save(x, w, 1e-5, 4, s, None, s)
+    for ww, sx in ((w[:128], s), (w, s[:, :64])):
+        with pytest.raises(ValueError, match="entries"):
+            rk.rmsnorm_backward_packed(x, q, sx, None, None, ww, rstd, 4)

@@ -128,3 +128,48 @@ def test_a_parameter_that_stops_fitting_is_refused(bound, what, with_plan):
     p.data = p.data[:8] if what == "adapter rank" else p.data.float()
     with pytest.raises(NotImplementedError):
         bind()
+
+
+def _bad(t, how):
+    return {"rows": lambda: t[:-8], "columns": lambda: t[:, :-8].contiguous(), "type": lambda: t.float(),
+            "strides": lambda: t.t().contiguous().t()}[how]()
+
+
+@pytest.mark.parametrize("how", ["rows", "columns", "type", "strides"])
+@pytest.mark.parametrize("which", [1, 2, 3, 4, 5, 6])
+def test_projections_and_factors_that_do_not_fit_are_refused(which, how):
+    """The kernels read weights and factors by address: a matrix of another size, type or (weights) layout is an error before
+    anything is launched.  A factor of other strides is copied, so it gets as far as the check for the device."""
+    from hyc_lora_release_b200._lib import host
+    H, I, t, st = 512, 1024, lambda *s: torch.zeros(*s, dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32)
+    match = "CUDA" if which > 3 and how == "strides" else "expected|head|projection"
+    w = [t(H), t(512, H), t(256, H), t(256, H), t(512, 16), t(256, 16), t(256, 16), t(3, H, 16)]
+    w[which] = _bad(w[which], how)
+    with pytest.raises(RuntimeError, match=match):
+        host.attn_forward_map(t(1, 8, H), w, [t(1), t(H), t(H), t(512), t(256), t(256), t(512)], t(8, 128), t(8, 128), None, 4, 128, 2, 4, 1e-5, st)
+    if which in (1, 2):
+        w = [t(H), t(I, H), t(I, H), t(H, I), t(I, 16), t(I, 16), t(2, H, 16), t(I, 64), t(H, 64)]
+        w[which] = _bad(w[which], how)
+        with pytest.raises(RuntimeError, match="expected"):
+            host.mlp_forward(t(1, 8, H), w, [t(1), t(H), t(H), t(I), t(I)], None, 4, 1e-5, st)
+        w = [t(H, I), t(I, 16), t(I, 16), t(H, 16), t(64, I)]
+        w[0] = _bad(w[0], how)
+        with pytest.raises(RuntimeError, match="expected"):
+            host.mlp_backward_lora(t(8, H), w, [t(1)] * 8, 4, st)
+
+
+@pytest.mark.parametrize("which", [3, 4, 5])
+def test_scales_of_another_length_are_refused(which):
+    from hyc_lora_release_b200._lib import host
+    H, t, st = 512, lambda *s: torch.zeros(*s, dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32)
+    w = [t(H), t(512, H), t(256, H), t(256, H), t(512, 16), t(256, 16), t(256, 16), t(3, H, 16)]
+    stats = [t(1), t(H), t(H), t(512), t(256), t(256), t(512)]
+    stats[which] = t(1)
+    with pytest.raises(ValueError, match="per-channel scale"):
+        host.attn_forward_map(t(1, 8, H), w, stats, t(8, 128), t(8, 128), None, 4, 128, 2, 4, 1e-5, st)
+    if which < 5:
+        w = [t(H), t(1024, H), t(1024, H), t(H, 1024), t(1024, 16), t(1024, 16), t(2, H, 16), t(1024, 64), t(H, 64)]
+        stats = [t(1), t(H), t(H), t(1024), t(1024)]
+        stats[which] = t(1)
+        with pytest.raises(ValueError, match="per-channel scale"):
+            host.mlp_forward(t(1, 8, H), w, stats, None, 4, 1e-5, st)
