@@ -49,6 +49,14 @@ static Tensor rows_view(const Tensor& x_in) {
   return x;
 }
 
+// a caller's buffer that a kernel writes by its address
+static const Tensor& buffer(const Tensor& t, at::IntArrayRef shape, at::ScalarType type, const Tensor& like, const char* what) {
+  TORCH_CHECK_VALUE(t.numel() >= c10::multiply_integers(shape) && t.scalar_type() == type && t.is_contiguous() && t.device() == like.device(), what,
+                    ": expected a contiguous ", type, " buffer for ", shape, " on ", like.device(), ", got ", t.scalar_type(), " ", t.sizes(),
+                    " on ", t.device());
+  return t;
+}
+
 static Tensor index_of(const Tensor& channel, const Tensor& like) {
   return channel.to(like.device(), at::kLong).contiguous();
 }
@@ -66,8 +74,12 @@ std::tuple<Tensor, OptTensor> quant(const Tensor& x_in, const Tensor& s_in, int6
   if (given(z)) zt = z->reshape({-1}).to(at::kChar).contiguous();
   int64_t k = 0;
   if (given(channel)) { idx = index_of(*channel, x); k = idx.numel(); }
-  Tensor q = given(out_q) ? *out_q : empty({B, M, N * q_bit / 8}, x, at::kByte);
+  Tensor q = given(out_q) ? buffer(*out_q, {B, M, N * q_bit / 8}, at::kByte, x, "codes") : empty({B, M, N * q_bit / 8}, x, at::kByte);
   OptTensor xo = out_xo;
+  if (k && given(out_q)) {
+    TORCH_CHECK_VALUE(given(xo), "a buffer for the outlier values is needed beside the one for the codes");
+    buffer(*xo, {B, M, k}, at::kBFloat16, x, "outlier values");
+  }
   if (!given(out_q) && given(channel)) xo = empty({B, M, k}, x);
   if (rows > 0)
     check(hyc_quant_pack(data(x), rows, (int)N, x.stride(1), data(s), (const int8_t*)data(zt), k ? (const int64_t*)data(idx) : nullptr,
@@ -85,7 +97,7 @@ Tensor dequant(const Tensor& q_in, const Tensor& s_in, int64_t q_bit, const OptT
   const Tensor q = q_in.contiguous(), s = scale_vec(s_in, N);
   Tensor zt, idx, xo;
   if (given(z)) zt = z->reshape({-1}).to(at::kChar).contiguous();
-  Tensor x = given(out) ? *out : empty({B, M, N}, q);
+  Tensor x = given(out) ? buffer(*out, {B, M, N}, at::kBFloat16, q, "out") : empty({B, M, N}, q);
   if (B * M == 0) return x;
   int64_t k = 0;
   if (given(channel)) {
@@ -136,7 +148,10 @@ Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor&
   OnDevice on(q);
   const Tensor g = bf16c(grad);
   TORCH_CHECK_VALUE(g.sizes() == shape, "the gradient must have the map's shape ", shape);
-  Tensor o = given(out) ? *out : empty(shape, q);
+  // (a buffer of another layout or type receives a copy)
+  const bool direct = !given(out) || (out->numel() == c10::multiply_integers(shape) && out->scalar_type() == at::kBFloat16 && out->is_contiguous() && out->device() == q.device());
+  Tensor o = given(out) && direct ? *out : empty(shape, q);
+  auto result = [&]() { return direct ? o : out->copy_(o); };
   const int64_t k = val.size(1);
   const int rc = hyc_softmax_topk_restore_bwd(k ? data(val) : nullptr, k ? (const uint16_t*)data(col) : nullptr, (int)k, data(q), data(s),
                                               (const int8_t*)data(z), q.size(0), (int)shape.back(), data(g), data(o), (int)q_bit,
@@ -144,10 +159,10 @@ Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor&
   if (rc == HYC_ERR_UNSUPPORTED) {      // shape outside the fused kernel: restore, then the softmax backward in place
     Tensor a = topk_restore(val, col, q, s, z, shape, q_bit, std::nullopt);
     check(hyc_softmax_bwd(data(a), data(g), data(o), a.numel() / shape.back(), (int)shape.back(), (float)scale, on.stream), "hyc_softmax_bwd");
-    return o;
+    return result();
   }
   check(rc, "hyc_softmax_topk_restore_bwd");
-  return o;
+  return result();
 }
 
 // ---- attention map, threshold prune

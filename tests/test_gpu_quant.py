@@ -211,3 +211,34 @@ def test_idempotent_requantization(cf):
         xr = cf.decompression_dequantization(pk, s, q)
         # bf16 rounding moves code*s by at most 2^-9 relative, i.e. less than half a step
         assert torch.equal(cf.compression_quantization(xr, s, q), pk)
+
+
+def test_buffers_that_do_not_fit_are_refused():
+    """Buffers handed in for the results are checked before a kernel writes to them."""
+    from hyc_lora_release_b200.operators import compress_function as cf
+    x = torch.randn(2, 8, 256, device="cuda").to(torch.bfloat16)
+    s, idx = torch.ones(1, 256, dtype=torch.bfloat16, device="cuda"), torch.tensor([3, 70], device="cuda")
+    q, xo, r = torch.empty(2, 8, 128, dtype=torch.uint8, device="cuda"), torch.empty(2, 8, 2, dtype=torch.bfloat16, device="cuda"), torch.empty_like(x)
+    want = cf.outlier_subtraction_fuse_compression_quantization(x, s, idx, 4)
+    got = cf.outlier_subtraction_fuse_compression_quantization(x, s, idx, 4, out=(q, xo))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    back = cf.outlier_addition_fuse_decompression_dequantization(q, s, xo, idx, 4)
+    assert torch.equal(cf.outlier_addition_fuse_decompression_dequantization(q, s, xo, idx, 4, out=r), back)
+    for bad in ((q[:1], xo), (q, xo[:1]), (q.int(), xo), (q, xo.float()), (q.cpu(), xo), (q, None)):
+        with pytest.raises((ValueError, RuntimeError)):
+            cf.outlier_subtraction_fuse_compression_quantization(x, s, idx, 4, out=bad)
+    for bad in (r[:1], r.float(), r.transpose(0, 1), r.cpu()):
+        with pytest.raises((ValueError, RuntimeError)):
+            cf.outlier_addition_fuse_decompression_dequantization(q, s, xo, idx, 4, out=bad)
+
+
+def test_topk_backward_into_any_buffer():
+    from hyc_lora_release_b200.operators import compress_function as cf
+    a = torch.softmax(torch.randn(1, 2, 64, 128, device="cuda"), -1).to(torch.bfloat16)
+    m, g = cf.compression_softmax_topk(a, 0.05), torch.randn_like(a)
+    want = m.softmax_backward(g)
+    flat, strided = torch.empty_like(a), torch.empty(1, 64, 2, 128, dtype=torch.bfloat16, device="cuda").transpose(1, 2)
+    for out in (flat, strided, torch.empty(a.shape, device="cuda")):
+        assert torch.equal(m.softmax_backward(g, out=out).to(torch.bfloat16), want) and torch.equal(out.to(torch.bfloat16), want)
+    with pytest.raises(RuntimeError):
+        m.softmax_backward(g, out=flat[:, :1, :8])
