@@ -499,6 +499,17 @@ struct Stamp {
   }
 };
 
+// The stream capture that work on the device of `t` is being recorded into, 0 if it runs.  What is computed inside a capture holds
+// nothing until the graph is replayed, and a replay computes anew only what was recorded: copies of things that change between
+// replays (adapters) are made inside each capture that reads them, and made again outside of it.
+static int64_t capture_of(const Tensor& t) {
+  if (!t.is_cuda()) return 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(c10::cuda::getCurrentCUDAStream(t.get_device()).stream(), &status, &id) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  return status == cudaStreamCaptureStatusNone ? 0 : (int64_t)id;
+}
+
 struct LayerPlan {
   Tensor norm1, norm2;
   FrozenWeight w[PROJECTIONS];
@@ -506,12 +517,13 @@ struct LayerPlan {
   OptTensor bias_o, bias_d;
   std::vector<Tensor> pad;                      // what AttnWeights.padded / MLPWeights.padded make of the LoRA factors
   Stamp pad_of[2 * PROJECTIONS];
+  int64_t pad_capture = 0;
   std::vector<Tensor> stats_in, stats;          // calibrated statistics as given, and as the kernels read them
   std::vector<Stamp> stats_of;
 
   // false: the padded factors are out of date, or a weight is no longer what it was checked to be
   bool fresh() const {
-    if ((int)pad.size() != PADS) return false;
+    if ((int)pad.size() != PADS || pad_capture != capture_of(lora[0])) return false;
     for (const FrozenWeight& f : w)
       if (f.plain.defined() && f.plain.scalar_type() != at::kBFloat16) return false;
     for (const OptTensor* b : {&bias_o, &bias_d})
@@ -524,6 +536,7 @@ struct LayerPlan {
     TORCH_CHECK_VALUE((int)p.size() == PADS, "LayerPlan: ", (int)PADS, " padded factors expected");
     pad = p;
     for (int i = 0; i < 2 * PROJECTIONS; ++i) pad_of[i] = Stamp::of(lora[i]);
+    pad_capture = capture_of(lora[0]);
   }
   // A statistic that the kernels read where it lies is looked up once.  One that has to be converted is converted on every
   // call: the copy could not follow a write that bumps no version (through `.data`, or to an inference tensor).
@@ -674,6 +687,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
 
 void bind_blocks(pybind11::module_& m) {
   m.def("lora_grad_a", &lora_grad_a);
+  m.def("capture_of", &capture_of);
   m.def("mlp_forward", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const OptTensor& bias_d, int64_t q,
                           double eps, const Tensor& st) {
     MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st);

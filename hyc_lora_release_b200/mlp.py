@@ -103,8 +103,9 @@ def lora_grad_a(q, scale, gm, r2, q_bit):
 
 def contents_key(tensors):
     """Equal keys: the tensors hold what they held, as long as an alias of each is kept beside the key (``_pad_of`` of the
-    weight records; without it another tensor's storage may come to lie at the old address)."""
-    return tuple((t.data_ptr(), t._version, t.shape, t.stride(), t.dtype) for t in tensors)
+    weight records; without it another tensor's storage may come to lie at the old address), and what was made of them
+    was made in the same stream capture (a replay makes again only what was recorded) or outside of one."""
+    return (host.capture_of(tensors[0]), *((t.data_ptr(), t._version, t.shape, t.stride(), t.dtype) for t in tensors))
 
 
 @dataclass

@@ -286,3 +286,32 @@ def test_norm_weights_and_scales_of_another_length_are_refused():
     for ww, sx in ((w[:128], s), (w, s[:, :64])):
         with pytest.raises(ValueError, match="entries"):
             rk.rmsnorm_backward_packed(x, q, sx, None, None, ww, rstd, 4)
+
+
+@pytest.mark.parametrize("stepwise", [False, True])
+def test_replay_follows_the_adapters_and_leaves_eager_steps_alone(stepwise):
+    """Adapters updated in place between replays count in the next one, and a step that runs after a capture does not read what
+    the capture only recorded (nothing was replayed in between)."""
+    p = Problem()
+    p.layer.keep_saved = stepwise
+
+    def update(f):
+        with torch.no_grad():
+            for i, w in enumerate(p.lora()):
+                w.mul_(f + 0.05 * i)
+    p.step()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        p.step()
+    torch.cuda.current_stream().wait_stream(side)
+    update(1.1)                               # the copies of the adapters are out of date when the capture begins
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = p.step()
+    assert _same(p.step(), p.step(layer=p.fresh_layer()))
+    for f in (0.9, 1.2):
+        update(f)
+        graph.replay()
+        want = p.step(layer=p.fresh_layer())
+        assert _same(got, want) and _same(p.step(), want)
