@@ -134,6 +134,7 @@ __device__ __forceinline__ void at_sync() { asm volatile("bar.sync 1, %0;" ::"n"
 // ------------------------------------------------------------------ mask classes
 __global__ void __launch_bounds__(256)
 mask_class_kernel(const __nv_bfloat16* __restrict__ mask, int64_t mb, int64_t mh, int64_t mr, int M, int tiles, int mask_heads, TileClass* __restrict__ out) {
+  pdl_wait();
   __shared__ uint32_t s_rows[4], s_nonzero;
   const int kt = blockIdx.x, qt = blockIdx.y, z = blockIdx.z;
   if (threadIdx.x < 4) s_rows[threadIdx.x] = 0u;
@@ -238,6 +239,7 @@ __device__ __forceinline__ uint32_t at_setup(const AttnParams& p, const Bars& ba
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(bar.tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  pdl_wait();
   if (warp == 2 && lane < p.tiles) bar.cls[lane] = (uint8_t)(fixed_is_q ? class_of(p, b, h, fixed, lane) : class_of(p, b, h, lane, fixed));
   tc_fence_before();
   __syncthreads();
@@ -813,7 +815,7 @@ template <int QBIT>
 static int launch_fwd(const FwdMaps& maps, const AttnParams& p, cudaStream_t st) {
   static bool done[64] = {false};
   if (const int rc = at_prepare(attn_fwd_kernel<QBIT>, AT_SMEM, done)) return rc;
-  attn_fwd_kernel<QBIT><<<p.tiles * p.B * p.heads, AT_THREADS, AT_SMEM, st>>>(maps, p);
+  launch_pdl(attn_fwd_kernel<QBIT>, dim3((unsigned)(p.tiles * p.B * p.heads)), dim3(AT_THREADS), AT_SMEM, st, maps, p);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
@@ -835,7 +837,7 @@ extern "C" HYC_API int hyc_attn_mask_class(const void* mask, int64_t stride_b, i
   if (mask_batch < 1 || mask_heads < 1 || M < 1 || M % 8 != 0 || M > MAX_TILES * TILE) return HYC_ERR_SHAPE;
   if (!aligned(mask, 16) || !aligned(out, 16) || ((stride_b | stride_h | stride_row) & 7)) return HYC_ERR_ALIGN;
   const int t = (M + TILE - 1) / TILE;
-  mask_class_kernel<<<dim3(t, t, mask_batch * mask_heads), 256, 0, (cudaStream_t)stream>>>(
+  launch_pdl(mask_class_kernel, dim3(t, t, mask_batch * mask_heads), dim3(256), 0, (cudaStream_t)stream, 
       (const __nv_bfloat16*)mask, stride_b, stride_h, stride_row, M, t, mask_heads, (TileClass*)out);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
@@ -890,10 +892,10 @@ extern "C" HYC_API int hyc_attn_bwd_tcgen05(
   if (const int rc = at_prepare(attn_bwd_q_kernel, AT_SMEM, done_q)) return rc;
   if (const int rc = at_prepare(attn_bwd_kv_kernel, KV_SMEM, done_kv)) return rc;
   p.out0 = (__nv_bfloat16*)grad_q; p.map = (__nv_bfloat16*)grad_s;
-  attn_bwd_q_kernel<<<p.tiles * B * heads, AT_THREADS, AT_SMEM, st>>>(mq, p);
+  launch_pdl(attn_bwd_q_kernel, dim3((unsigned)(p.tiles * B * heads)), dim3(AT_THREADS), AT_SMEM, st, mq, p);
   HYC_CHECK_LAUNCH();
   p.out0 = (__nv_bfloat16*)grad_k; p.out1 = (__nv_bfloat16*)grad_v;
-  attn_bwd_kv_kernel<<<p.tiles * B * kv_heads, KV_THREADS, KV_SMEM, st>>>(mk, p);
+  launch_pdl(attn_bwd_kv_kernel, dim3((unsigned)(p.tiles * B * kv_heads)), dim3(KV_THREADS), KV_SMEM, st, mk, p);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }

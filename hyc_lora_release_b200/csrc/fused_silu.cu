@@ -47,6 +47,7 @@ fused_silu_kernel(const __nv_bfloat16* __restrict__ xa1, const __nv_bfloat16* __
                   const __nv_bfloat16* __restrict__ go,                                         // backward input
                   __nv_bfloat16* __restrict__ o, __nv_bfloat16* __restrict__ gg, __nv_bfloat16* __restrict__ gu,
                   int64_t rows, int N) {
+  pdl_wait();
   using G = FGeo<QBIT>;
   constexpr int EPP = G::EPP, NPS = G::NT_PER_SLAB;
   constexpr uint32_t CM = (1u << QBIT) - 1u;
@@ -242,6 +243,7 @@ fused_silu_wide_kernel(const __nv_bfloat16* __restrict__ xa1, const __nv_bfloat1
                        const __nv_bfloat16* __restrict__ go,                                         // backward input
                        __nv_bfloat16* __restrict__ o, __nv_bfloat16* __restrict__ gg, __nv_bfloat16* __restrict__ gu,
                        int64_t rows, int N) {
+  pdl_wait();
   constexpr int EPP = 8 / QBIT;
   constexpr uint32_t CM = (1u << QBIT) - 1u, BM = CM * 0x01010101u;
   __shared__ __align__(16) uint32_t s_l[8][2][16 * kWideLd];
@@ -479,6 +481,7 @@ __device__ __forceinline__ float rotate_f32(float own, float other, float c, flo
 template <int QBIT, bool HEADS>
 __global__ void __launch_bounds__(256, HYC_FUSED_MINB)
 dequant_lora_add_kernel(const RebuildJobs jobs, int64_t rows) {
+  pdl_wait();
   const int which = !HEADS || jobs.count < 2 || (int)blockIdx.x < jobs.job[1].first_block ? 0 : ((int)blockIdx.x < jobs.job[2].first_block ? 1 : 2);
   const __nv_bfloat16* __restrict__ xa = jobs.job[which].xa;
   const __nv_bfloat16* __restrict__ bt = jobs.job[which].bt;
@@ -648,7 +651,7 @@ extern "C" HYC_API int hyc_fused_lora_silu_hadamard_fwd(const void* xa1, const v
   bool wide = true;
   for (const void* p : ps) wide = wide && aligned(p, 16);
   dim3 grid = fused_grid(rows, N);
-#define FWW(QB) fused_silu_wide_kernel<QB, false><<<fused_wide_grid(fused_silu_wide_kernel<QB, false>, rows, N), 256, 0, (cudaStream_t)stream>>>(                    \
+#define FWW(QB) launch_pdl(fused_silu_wide_kernel<QB, false>, fused_wide_grid(fused_silu_wide_kernel<QB, false>, rows, N), dim3(256), 0, (cudaStream_t)stream,                     \
       (const __nv_bfloat16*)xa1, (const __nv_bfloat16*)bt1, (const __nv_bfloat16*)xa2, (const __nv_bfloat16*)bt2, \
       (const __nv_bfloat16*)s1, (const __nv_bfloat16*)s2, (const __nv_bfloat16*)x1, (const __nv_bfloat16*)x2,     \
       (uint8_t*)q1, (uint8_t*)q2, nullptr, (__nv_bfloat16*)o, nullptr, nullptr, rows, N)
@@ -658,7 +661,7 @@ extern "C" HYC_API int hyc_fused_lora_silu_hadamard_fwd(const void* xa1, const v
     return HYC_OK;
   }
 #undef FWW
-#define FW(QB) fused_silu_kernel<QB, false><<<grid, 256, 0, (cudaStream_t)stream>>>(                         \
+#define FW(QB) launch_pdl(fused_silu_kernel<QB, false>, grid, dim3(256), 0, (cudaStream_t)stream,                          \
       (const __nv_bfloat16*)xa1, (const __nv_bfloat16*)bt1, (const __nv_bfloat16*)xa2, (const __nv_bfloat16*)bt2, \
       (const __nv_bfloat16*)s1, (const __nv_bfloat16*)s2, (const __nv_bfloat16*)x1, (const __nv_bfloat16*)x2,     \
       (uint8_t*)q1, (uint8_t*)q2, nullptr, (__nv_bfloat16*)o, nullptr, nullptr, rows, N)
@@ -681,7 +684,7 @@ extern "C" HYC_API int hyc_fused_lora_silu_hadamard_bwd(const void* xa1, const v
   bool wide = true;
   for (const void* p : ps) wide = wide && aligned(p, 16);
   dim3 grid = fused_grid(rows, N);
-#define BWW(QB) fused_silu_wide_kernel<QB, true><<<fused_wide_grid(fused_silu_wide_kernel<QB, true>, rows, N), 256, 0, (cudaStream_t)stream>>>(                     \
+#define BWW(QB) launch_pdl(fused_silu_wide_kernel<QB, true>, fused_wide_grid(fused_silu_wide_kernel<QB, true>, rows, N), dim3(256), 0, (cudaStream_t)stream,                      \
       (const __nv_bfloat16*)xa1, (const __nv_bfloat16*)bt1, (const __nv_bfloat16*)xa2, (const __nv_bfloat16*)bt2, \
       (const __nv_bfloat16*)s1, (const __nv_bfloat16*)s2, nullptr, nullptr,                                       \
       (uint8_t*)q1, (uint8_t*)q2, (const __nv_bfloat16*)grad_o, (__nv_bfloat16*)o, (__nv_bfloat16*)grad_gate,     \
@@ -692,7 +695,7 @@ extern "C" HYC_API int hyc_fused_lora_silu_hadamard_bwd(const void* xa1, const v
     return HYC_OK;
   }
 #undef BWW
-#define BW(QB) fused_silu_kernel<QB, true><<<grid, 256, 0, (cudaStream_t)stream>>>(                          \
+#define BW(QB) launch_pdl(fused_silu_kernel<QB, true>, grid, dim3(256), 0, (cudaStream_t)stream,                           \
       (const __nv_bfloat16*)xa1, (const __nv_bfloat16*)bt1, (const __nv_bfloat16*)xa2, (const __nv_bfloat16*)bt2, \
       (const __nv_bfloat16*)s1, (const __nv_bfloat16*)s2, nullptr, nullptr,                                       \
       (uint8_t*)q1, (uint8_t*)q2, (const __nv_bfloat16*)grad_o, (__nv_bfloat16*)o, (__nv_bfloat16*)grad_gate,     \
@@ -713,7 +716,7 @@ extern "C" HYC_API int hyc_dequant_lora_add(const void* q, const void* scale, co
   RebuildJobs jobs = {};
   jobs.job[0] = {(const __nv_bfloat16*)xa, (const __nv_bfloat16*)bt, (const __nv_bfloat16*)scale, (const uint8_t*)q, (__nv_bfloat16*)y, N, 0, false};
   jobs.count = 1;
-#define DL(QB) dequant_lora_add_kernel<QB, false><<<fused_wide_grid(dequant_lora_add_kernel<QB, false>, rows, N), 256, 0, (cudaStream_t)stream>>>(jobs, rows)
+#define DL(QB) launch_pdl(dequant_lora_add_kernel<QB, false>, fused_wide_grid(dequant_lora_add_kernel<QB, false>, rows, N), dim3(256), 0, (cudaStream_t)stream, jobs, rows)
   if (q_bit == 2) DL(2); else if (q_bit == 4) DL(4); else DL(8);
 #undef DL
   HYC_CHECK_LAUNCH();
@@ -740,7 +743,7 @@ extern "C" HYC_API int hyc_rebuild_qkv(const void* const* q, const void* const* 
   }
   jobs.cos = cos_t; jobs.sin = sin_t; jobs.ld_table = ld_table; jobs.table_f32 = table_is_f32; jobs.seq_len = seq_len; jobs.count = 3;
   if (rows == 0) return HYC_OK;
-#define DL(QB) dequant_lora_add_kernel<QB, true><<<wide_grid(dequant_lora_add_kernel<QB, true>, rows, blocks), 256, 0, (cudaStream_t)stream>>>(jobs, rows)
+#define DL(QB) launch_pdl(dequant_lora_add_kernel<QB, true>, wide_grid(dequant_lora_add_kernel<QB, true>, rows, blocks), dim3(256), 0, (cudaStream_t)stream, jobs, rows)
   if (q_bit == 2) DL(2); else if (q_bit == 4) DL(4); else DL(8);
 #undef DL
   HYC_CHECK_LAUNCH();

@@ -124,6 +124,7 @@ template <int QBIT>
 __global__ void __launch_bounds__(256)
 group_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int N, int64_t ldx,
                    uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scale, int8_t* __restrict__ zp) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int steps = (N + 511) / 512;
   const int64_t items = rows * steps;
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(256)
 group_dequant_kernel(const uint8_t* __restrict__ q, int64_t rows, int N,
                      const __nv_bfloat16* __restrict__ scale, const int8_t* __restrict__ zp,
                      __nv_bfloat16* __restrict__ xo, int64_t ldx) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int steps = (N + 511) / 512;
   const int64_t items = rows * steps;
@@ -183,6 +185,7 @@ template <int QBIT>
 __global__ void __launch_bounds__(256, HYC_LANE_MINB)
 group_flat_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t n_groups, uint8_t* __restrict__ q,
                         __nv_bfloat16* __restrict__ scale, int8_t* __restrict__ zp) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   __shared__ __align__(16) uint32_t s_x[8][32 * 32];
   const int64_t items = (n_groups + 31) / 32;
@@ -209,6 +212,7 @@ template <int QBIT>
 __global__ void __launch_bounds__(256, HYC_LANE_MINB)
 group_flat_dequant_kernel(const uint8_t* __restrict__ q, int64_t n_groups, const __nv_bfloat16* __restrict__ scale,
                           const int8_t* __restrict__ zp, __nv_bfloat16* __restrict__ xo) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   __shared__ __align__(16) uint32_t s_x[8][32 * 32];
   const int64_t items = (n_groups + 31) / 32;
@@ -249,6 +253,7 @@ __global__ void __launch_bounds__(256)
 topk_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int S, int k,
                      __nv_bfloat16* __restrict__ val_out, uint16_t* __restrict__ col_out,
                      uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scale, int8_t* __restrict__ zp) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t qld = (int64_t)S * QBIT / 8, gld = S / 64;
   __shared__ __align__(16) uint32_t s_x[8][32][8];          // the lane's 16 values, per warp
@@ -426,6 +431,7 @@ __global__ void __launch_bounds__(256)
 topk_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* __restrict__ colv, int k,
                     const uint8_t* __restrict__ q, const __nv_bfloat16* __restrict__ scale,
                     const int8_t* __restrict__ zp, int64_t rows, int S, __nv_bfloat16* __restrict__ ao) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int steps = (S + 511) / 512;
   const int64_t qld = (int64_t)S * QBIT / 8, gld = S / 64;
@@ -492,14 +498,14 @@ extern "C" HYC_API int hyc_group_quant_pack(const void* x, int64_t rows, int N, 
     const int64_t n_groups = rows * (N / 64);
     int grid, threads;
 #define GFQ(QB) do { auto kern = group_flat_quant_kernel<QB>; lane_launch_shape(kern, n_groups, 32, grid, threads); \
-      kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)x, n_groups, (uint8_t*)q_out, (__nv_bfloat16*)scale_out, zp_out); } while (0)
+      launch_pdl(kern, dim3((unsigned)grid), dim3(threads), 0, st, (const __nv_bfloat16*)x, n_groups, (uint8_t*)q_out, (__nv_bfloat16*)scale_out, zp_out); } while (0)
     if (q_bit == 2) GFQ(2); else if (q_bit == 4) GFQ(4); else GFQ(8);
 #undef GFQ
     HYC_CHECK_LAUNCH();
     return HYC_OK;
   }
   const int64_t items = rows * ((N + 511) / 512);
-#define GQ(QB) group_quant_kernel<QB><<<warp_grid(items), 256, 0, st>>>((const __nv_bfloat16*)x, rows, N, ldx, \
+#define GQ(QB) launch_pdl(group_quant_kernel<QB>, dim3((unsigned)warp_grid(items)), dim3(256), 0, st, (const __nv_bfloat16*)x, rows, N, ldx, \
       (uint8_t*)q_out, (__nv_bfloat16*)scale_out, zp_out)
   if (q_bit == 2) GQ(2); else if (q_bit == 4) GQ(4); else GQ(8);
 #undef GQ
@@ -520,14 +526,14 @@ extern "C" HYC_API int hyc_group_unpack_dequant(const void* q, int64_t rows, int
     const int64_t n_groups = rows * (N / 64);
     int grid, threads;
 #define GFD(QB) do { auto kern = group_flat_dequant_kernel<QB>; lane_launch_shape(kern, n_groups, 32, grid, threads); \
-      kern<<<grid, threads, 0, st>>>((const uint8_t*)q, n_groups, (const __nv_bfloat16*)scale, zp, (__nv_bfloat16*)x_out); } while (0)
+      launch_pdl(kern, dim3((unsigned)grid), dim3(threads), 0, st, (const uint8_t*)q, n_groups, (const __nv_bfloat16*)scale, zp, (__nv_bfloat16*)x_out); } while (0)
     if (q_bit == 2) GFD(2); else if (q_bit == 4) GFD(4); else GFD(8);
 #undef GFD
     HYC_CHECK_LAUNCH();
     return HYC_OK;
   }
   const int64_t items = rows * ((N + 511) / 512);
-#define GD(QB) group_dequant_kernel<QB><<<warp_grid(items), 256, 0, st>>>((const uint8_t*)q, rows, N, \
+#define GD(QB) launch_pdl(group_dequant_kernel<QB>, dim3((unsigned)warp_grid(items)), dim3(256), 0, st, (const uint8_t*)q, rows, N, \
       (const __nv_bfloat16*)scale, zp, (__nv_bfloat16*)x_out, ldx)
   if (q_bit == 2) GD(2); else if (q_bit == 4) GD(4); else GD(8);
 #undef GD
@@ -570,7 +576,7 @@ extern "C" HYC_API int hyc_softmax_topk_compress(const void* a, int64_t rows, in
   }
   const int steps = (S + 511) / 512;
   const int grid = warp_grid(rows);
-#define TK(QB, ST) topk_compress_kernel<QB, ST><<<grid, 256, 0, st>>>((const __nv_bfloat16*)a, rows, S, k, \
+#define TK(QB, ST) launch_pdl(topk_compress_kernel<QB, ST>, dim3((unsigned)grid), dim3(256), 0, st, (const __nv_bfloat16*)a, rows, S, k, \
       (__nv_bfloat16*)val_out, col_out, (uint8_t*)q_out, (__nv_bfloat16*)scale_out, zp_out)
 #define TKQ(QB) do { if (steps <= 1) TK(QB, 1); else if (steps <= 2) TK(QB, 2); else if (steps <= 4) TK(QB, 4); else TK(QB, 8); } while (0)
   if (q_bit == 2) TKQ(2); else if (q_bit == 4) TKQ(4); else TKQ(8);
@@ -596,7 +602,7 @@ extern "C" HYC_API int hyc_softmax_topk_restore(const void* val, const uint16_t*
     HYC_CHECK_LAUNCH();
     return HYC_OK;
   }
-#define TR(QB) topk_restore_kernel<QB><<<warp_grid(rows), 256, 0, st>>>((const __nv_bfloat16*)val, col, k, \
+#define TR(QB) launch_pdl(topk_restore_kernel<QB>, dim3((unsigned)warp_grid(rows)), dim3(256), 0, st, (const __nv_bfloat16*)val, col, k, \
       (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows, S, (__nv_bfloat16*)a_out)
   if (q_bit == 2) TR(2); else if (q_bit == 4) TR(4); else TR(8);
 #undef TR

@@ -53,11 +53,15 @@ inline int resident_blocks(K kern, int threads, size_t smem, int otherwise) {
 }
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may begin before the kernel in front of it in the
-// stream has ended, and has to call pdl_wait() before it touches memory (pdl_wait returns once that kernel, and with
-// it everything before, is complete and visible).
+// stream has ended, and has to call pdl_wait() before it touches global memory (pdl_wait returns once that kernel is
+// complete and its writes are visible; since every such kernel waits, so is everything before it).  The kernel in front lets it
+// begin by ending: with griddepcontrol.launch_dependents early on, blocks that only wait take the places of the last working
+// ones, and streaming kernels got slower (save, restore and softmax backward of a [4,32,512,512] map 96.6 us against
+// 85.3; without any of this 93.3).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// (errors stay in cudaGetLastError, as with <<<>>>)
 template <typename K, typename... A>
-inline int launch_pdl(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+inline void launch_pdl(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -65,11 +69,7 @@ inline int launch_pdl(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t s
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, kern, args...) != cudaSuccess) {
-    hyc_set_last_cuda_error((int)cudaGetLastError());
-    return HYC_ERR_LAUNCH;
-  }
-  return HYC_OK;
+  (void)cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 __host__ __device__ inline bool aligned(const void* p, size_t a) {

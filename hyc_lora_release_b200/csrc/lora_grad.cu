@@ -75,6 +75,7 @@ template <int QBIT, int RT>   // RT = number of 16-row tiles of the LoRA dimensi
 __global__ void __launch_bounds__(128)
 lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restrict__ scale,
                    const __nv_bfloat16* __restrict__ gm, int64_t ldg, int T, int H, float* __restrict__ ws) {
+  pdl_wait();
   constexpr int R2 = 16 * RT;
   __shared__ __align__(16) __nv_bfloat16 xs[kGaStep][kGaCols + 8];
   __shared__ __align__(16) __nv_bfloat16 gs[kGaStep][R2 + 8];
@@ -155,6 +156,7 @@ lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restric
 
 __global__ void __launch_bounds__(256)
 lora_grad_a_reduce_kernel(const float* __restrict__ ws, int splits, int64_t n, __nv_bfloat16* __restrict__ out) {
+  pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
     float s = 0.f;
     for (int k = 0; k < splits; ++k) s += ws[(int64_t)k * n + i];
@@ -182,7 +184,7 @@ extern "C" HYC_API int hyc_lora_grad_a_dequant(const void* q, const void* scale,
   cudaStream_t st = (cudaStream_t)stream;
   const int splits = (T + kGaChunk - 1) / kGaChunk;
   dim3 grid(H / kGaCols, splits);
-#define GA(QB, RT) lora_grad_a_kernel<QB, RT><<<grid, 128, 0, st>>>((const uint8_t*)q, (const __nv_bfloat16*)scale, \
+#define GA(QB, RT) launch_pdl(lora_grad_a_kernel<QB, RT>, grid, dim3(128), 0, st, (const uint8_t*)q, (const __nv_bfloat16*)scale, \
       (const __nv_bfloat16*)gm, ldg, T, H, (float*)workspace)
 #define GAQ(QB) do { switch (R2 / 16) { case 1: GA(QB, 1); break; case 2: GA(QB, 2); break; case 3: GA(QB, 3); break; default: GA(QB, 4); } } while (0)
   if (q_bit == 2) GAQ(2); else if (q_bit == 4) GAQ(4); else GAQ(8);
@@ -192,7 +194,7 @@ extern "C" HYC_API int hyc_lora_grad_a_dequant(const void* q, const void* scale,
   const int64_t n = (int64_t)R2 * H;
   int64_t rb = (n + 255) / 256;
   if (rb > num_sms() * 8) rb = num_sms() * 8;
-  lora_grad_a_reduce_kernel<<<(int)rb, 256, 0, st>>>((const float*)workspace, splits, n, (__nv_bfloat16*)out);
+  launch_pdl(lora_grad_a_reduce_kernel, dim3((unsigned)rb), dim3(256), 0, st, (const float*)workspace, splits, n, (__nv_bfloat16*)out);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }

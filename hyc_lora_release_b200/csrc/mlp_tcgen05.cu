@@ -118,6 +118,7 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
   __syncthreads();
   if (PAIR) cluster_sync_all();      // the peer's barriers are initialised before anything is signalled there
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -641,11 +642,13 @@ static int launch_as(const Operands& ops, const Params& p, cudaStream_t st) {
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = PAIR ? 1 : 0;
+  cfg.numAttrs = PAIR ? 2 : 1;
   // the kernel is persistent: one CTA per SM, or one pair per two neighbouring SMs (as many as can be resident)
   int units = num_sms();
   if (PAIR) {

@@ -39,6 +39,7 @@ __device__ __forceinline__ float nf4_scale(const Nf4Job& j, int64_t e) {
 
 __global__ void __launch_bounds__(256)
 dequant_nf4_kernel(const __grid_constant__ Nf4Jobs jobs) {
+  pdl_wait();
   __shared__ float s_code[kNf4Jobs][16];
   if (threadIdx.x < 16 * jobs.count) s_code[threadIdx.x >> 4][threadIdx.x & 15] = jobs.job[threadIdx.x >> 4].code16[threadIdx.x & 15];
   __syncthreads();
@@ -123,7 +124,7 @@ extern "C" HYC_API int hyc_dequant_nf4_many(int count, const hyc_nf4_job* in, vo
   const int64_t cap = (int64_t)num_sms() * 8;
   if (grid > cap) grid = cap;
   if (grid < 1) grid = 1;
-  dequant_nf4_kernel<<<(int)grid, 256, 0, (cudaStream_t)stream>>>(jobs);
+  launch_pdl(dequant_nf4_kernel, dim3((unsigned)grid), dim3(256), 0, (cudaStream_t)stream, jobs);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }

@@ -54,6 +54,7 @@ template <int NV>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, float eps,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int64_t rows, int N) {
+  pdl_wait();
   const int nvec = N / 8;
   // NV octets per thread; the next row of the block is in flight while the current one is reduced and written
   uint4 xnext[NV];
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kNormThreads, NV <= 2 ? 4 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    __nv_bfloat16* __restrict__ dx, int64_t rows, int N) {
+  pdl_wait();
   const int nvec = N / 8;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const float rs = rstd[row];
@@ -171,6 +173,7 @@ rmsnorm_fwd_save_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
                         const __nv_bfloat16* __restrict__ scale_y,
                         __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, uint8_t* __restrict__ qx,
                         __nv_bfloat16* __restrict__ oout, uint8_t* __restrict__ qy, int64_t rows, int N) {
+  pdl_wait();
   extern __shared__ __align__(16) int16_t s_map[];
   constexpr bool CACHED = NV <= 2;
   const int nvec = N / 8;
@@ -289,6 +292,7 @@ rmsnorm_bwd_packed_kernel(const __nv_bfloat16* __restrict__ dy, const uint8_t* _
                           const __nv_bfloat16* __restrict__ oin, const __nv_bfloat16* __restrict__ w,
                           const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ res,
                           __nv_bfloat16* __restrict__ dx, int64_t rows, int N) {
+  pdl_wait();
   extern __shared__ __align__(16) int16_t s_map[];
   if (k > 0) build_full_map(s_map, N, oidx, k);
   const int nvec = N / 8;
@@ -367,6 +371,7 @@ constexpr int kSmMaxVec = 16;   // 16 x (32 lanes x 8 elements) = 4096 columns
 __global__ void __launch_bounds__(256)
 softmax_bwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ g,
                    __nv_bfloat16* __restrict__ o, int64_t rows, int S, float oscale) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = S / 8;
   for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (int64_t)gridDim.x * 8) {
@@ -421,6 +426,7 @@ __global__ void __launch_bounds__(256, NV <= 8 ? 3 : 1)
 softmax_fwd_kernel(const __nv_bfloat16* __restrict__ sc, float scale, const __nv_bfloat16* __restrict__ mask,
                    int64_t mb, int64_t mh, int64_t mr, int heads, int M, __nv_bfloat16* __restrict__ a,
                    int64_t rows, int S) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = S / 8;
   constexpr float kLog2e = 1.4426950408889634f;
@@ -500,10 +506,10 @@ extern "C" HYC_API int hyc_rmsnorm_fwd(const void* x, const void* w, float eps, 
   if (rows == 0) return HYC_OK;
   int64_t grid = rows < (int64_t)num_sms() * 8 ? rows : (int64_t)num_sms() * 8;
   if (N <= 2 * kNormThreads * 8)
-    rmsnorm_fwd_kernel<2><<<(int)grid, kNormThreads, 0, (cudaStream_t)stream>>>(
+    launch_pdl(rmsnorm_fwd_kernel<2>, dim3((unsigned)grid), dim3(kNormThreads), 0, (cudaStream_t)stream, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)y, rstd, rows, N);
   else
-    rmsnorm_fwd_kernel<kNormMaxVec><<<(int)grid, kNormThreads, 0, (cudaStream_t)stream>>>(
+    launch_pdl(rmsnorm_fwd_kernel<kNormMaxVec>, dim3((unsigned)grid), dim3(kNormThreads), 0, (cudaStream_t)stream, 
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)y, rstd, rows, N);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
@@ -527,7 +533,7 @@ extern "C" HYC_API int hyc_rmsnorm_fwd_save(const void* x, const void* w, float 
   const int64_t grid = rows < cap ? rows : cap;
   const size_t smem = k > 0 ? (size_t)N * 2 : 0;
 #define FS(QB) if (N <= 2 * kNormThreads * 8) FSV(QB, 2); else FSV(QB, kNormMaxVec)
-#define FSV(QB, NVV) rmsnorm_fwd_save_kernel<QB, NVV><<<(int)grid, kNormThreads, smem, (cudaStream_t)stream>>>(       \
+#define FSV(QB, NVV) launch_pdl(rmsnorm_fwd_save_kernel<QB, NVV>, dim3((unsigned)grid), dim3(kNormThreads), smem, (cudaStream_t)stream,        \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, eps, (const __nv_bfloat16*)scale_x, outlier_idx, k,          \
       (const __nv_bfloat16*)scale_y, (__nv_bfloat16*)y, rstd, (uint8_t*)qx, (__nv_bfloat16*)outlier_out, (uint8_t*)qy, rows, N)
   if (q_bit == 2) { FS(2); } else if (q_bit == 4) { FS(4); } else { FS(8); }
@@ -552,7 +558,7 @@ extern "C" HYC_API int hyc_rmsnorm_bwd_packed(const void* dy, const void* qx, co
   const int64_t cap = (int64_t)num_sms() * (N <= 2 * kNormThreads * 8 ? 4 : 1);
   const int64_t grid = rows < cap ? rows : cap;
   const size_t smem = k > 0 ? (size_t)N * 2 : 0;
-#define BPN(QB, NV) rmsnorm_bwd_packed_kernel<QB, NV><<<(int)grid, kNormThreads, smem, (cudaStream_t)stream>>>(      \
+#define BPN(QB, NV) launch_pdl(rmsnorm_bwd_packed_kernel<QB, NV>, dim3((unsigned)grid), dim3(kNormThreads), smem, (cudaStream_t)stream,       \
       (const __nv_bfloat16*)dy, (const uint8_t*)qx, (const __nv_bfloat16*)scale_x, outlier_idx, k,                   \
       (const __nv_bfloat16*)outlier, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)residual_grad,             \
       (__nv_bfloat16*)dx, rows, N)
@@ -572,10 +578,10 @@ extern "C" HYC_API int hyc_rmsnorm_bwd(const void* dy, const void* x, const void
   if (rows == 0) return HYC_OK;
   int64_t grid = rows < (int64_t)num_sms() * 8 ? rows : (int64_t)num_sms() * 8;
   if (N <= 2 * kNormThreads * 8)
-    rmsnorm_bwd_kernel<2><<<(int)grid, kNormThreads, 0, (cudaStream_t)stream>>>(
+    launch_pdl(rmsnorm_bwd_kernel<2>, dim3((unsigned)grid), dim3(kNormThreads), 0, (cudaStream_t)stream, 
         (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, rows, N);
   else
-    rmsnorm_bwd_kernel<kNormMaxVec><<<(int)grid, kNormThreads, 0, (cudaStream_t)stream>>>(
+    launch_pdl(rmsnorm_bwd_kernel<kNormMaxVec>, dim3((unsigned)grid), dim3(kNormThreads), 0, (cudaStream_t)stream, 
         (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd, (__nv_bfloat16*)dx, rows, N);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
@@ -592,7 +598,7 @@ extern "C" HYC_API int hyc_softmax_bwd(const void* y, const void* g, void* o, in
   }
   int64_t grid = (rows + 7) / 8;
   if (grid > (int64_t)num_sms() * 8) grid = (int64_t)num_sms() * 8;
-  softmax_bwd_kernel<<<(int)grid, 256, 0, (cudaStream_t)stream>>>(
+  launch_pdl(softmax_bwd_kernel, dim3((unsigned)grid), dim3(256), 0, (cudaStream_t)stream, 
       (const __nv_bfloat16*)y, (const __nv_bfloat16*)g, (__nv_bfloat16*)o, rows, S, out_scale);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
@@ -608,7 +614,7 @@ extern "C" HYC_API int hyc_softmax_fwd_scale_mask(const void* scores, float scal
   if (rows == 0) return HYC_OK;
   int64_t grid = (rows + 7) / 8;
   if (grid > (int64_t)num_sms() * 8) grid = (int64_t)num_sms() * 8;
-#define SF(NV) softmax_fwd_kernel<NV><<<(int)grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)scores, scale, \
+#define SF(NV) launch_pdl(softmax_fwd_kernel<NV>, dim3((unsigned)grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)scores, scale, \
       (const __nv_bfloat16*)mask_or_null, mask_stride_b, mask_stride_h, mask_stride_row, heads, M, (__nv_bfloat16*)a, rows, S)
   if (S <= 512) SF(2); else if (S <= 1024) SF(4); else if (S <= 2048) SF(8); else SF(16);
 #undef SF

@@ -126,6 +126,7 @@ quant_pack_kernel(const __nv_bfloat16* __restrict__ x, int64_t rows, int N, int6
                   const __nv_bfloat16* __restrict__ scale, const int8_t* __restrict__ zp,
                   const int64_t* __restrict__ oidx, int k,
                   uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ oout) {
+  pdl_wait();
   using G = Geo<QBIT>;
   constexpr int EPP = G::EPP;
   const int ct = blockIdx.x * blockDim.x + threadIdx.x;
@@ -272,6 +273,7 @@ unpack_dequant_kernel(const uint8_t* __restrict__ q, int64_t rows, int N,
                       const __nv_bfloat16* __restrict__ scale, const int8_t* __restrict__ zp,
                       const int64_t* __restrict__ oidx, int k, const __nv_bfloat16* __restrict__ oin,
                       __nv_bfloat16* __restrict__ xo, int64_t ldx) {
+  pdl_wait();
   using G = Geo<QBIT>;
   constexpr int EPP = G::EPP;
   constexpr uint32_t MASK = (1u << QBIT) - 1u;
@@ -508,7 +510,7 @@ extern "C" HYC_API int hyc_quant_pack(const void* x, int64_t rows, int N, int64_
   const int threads = pick_threads(N / cpt);
   size_t smem = k > 0 ? (size_t)threads * cpt * 2 + (size_t)(threads / 32) * kWarpList * 4 : 0;   // int16 column map + per-warp lists
 #define LAUNCH_Q(QB, ZP)                                                                          \
-  quant_pack_kernel<QB, ZP><<<stream_grid(quant_pack_kernel<QB, ZP>, threads, smem, rows, N / cpt, kRowUnroll), threads, smem, st>>>( \
+  launch_pdl(quant_pack_kernel<QB, ZP>, stream_grid(quant_pack_kernel<QB, ZP>, threads, smem, rows, N / cpt, kRowUnroll), dim3(threads), smem, st,  \
       (const __nv_bfloat16*)x, rows, N, ldx, (const __nv_bfloat16*)scale, zp, outlier_idx, k,      \
       (uint8_t*)q_out, (__nv_bfloat16*)outlier_out)
   if (zp) {
@@ -538,7 +540,7 @@ extern "C" HYC_API int hyc_unpack_dequant(const void* q, int64_t rows, int N,
   const int threads = pick_threads(N / cpt);
   size_t smem = k > 0 ? (size_t)threads * cpt * 2 + (size_t)(threads / 32) * kWarpList * 4 : 0;
 #define LAUNCH_D(QB, ZP)                                                                          \
-  unpack_dequant_kernel<QB, ZP><<<stream_grid(unpack_dequant_kernel<QB, ZP>, threads, smem, rows, N / cpt, kDeqUnroll), threads, smem, st>>>(                                        \
+  launch_pdl(unpack_dequant_kernel<QB, ZP>, stream_grid(unpack_dequant_kernel<QB, ZP>, threads, smem, rows, N / cpt, kDeqUnroll), dim3(threads), smem, st,                                         \
       (const uint8_t*)q, rows, N, (const __nv_bfloat16*)scale, zp, outlier_idx, k,                 \
       (const __nv_bfloat16*)outlier, (__nv_bfloat16*)x_out, ldx)
   if (zp) {

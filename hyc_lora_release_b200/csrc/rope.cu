@@ -26,6 +26,7 @@ template <bool TABLE_F32>
 __global__ void __launch_bounds__(256)
 rope_kernel(const RopeTensor t0, const RopeTensor t1, const void* __restrict__ cos_t, const void* __restrict__ sin_t, int64_t ld_table,
             int64_t rows, int seq_len, int head_dim, float sin_sign) {
+  pdl_wait();
   const int half = head_dim >> 1;
   const int per_head = half >> 3;                       // octets of j per head
   const int w = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -101,9 +102,9 @@ static int launch_rope(const RopeTensor& t0, const RopeTensor& t1, const void* c
   const dim3 grid((unsigned)bx, (unsigned)by);
   const float sgn = backward ? -1.f : 1.f;
   if (table_is_f32)
-    rope_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(t0, t1, cos_t, sin_t, ld_table, rows, seq_len, head_dim, sgn);
+    launch_pdl(rope_kernel<true>, grid, dim3(256), 0, (cudaStream_t)stream, t0, t1, cos_t, sin_t, ld_table, rows, seq_len, head_dim, sgn);
   else
-    rope_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(t0, t1, cos_t, sin_t, ld_table, rows, seq_len, head_dim, sgn);
+    launch_pdl(rope_kernel<false>, grid, dim3(256), 0, (cudaStream_t)stream, t0, t1, cos_t, sin_t, ld_table, rows, seq_len, head_dim, sgn);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }

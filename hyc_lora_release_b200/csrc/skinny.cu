@@ -100,6 +100,7 @@ skinny_kernel(const __grid_constant__ Args a) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem = *tmem_slot;
   const uint32_t ring = smem_u32(smem), aux = ring + AUX_AT;
   // xa blocks first, then W blocks [column tile][w]; accumulators: Y [row tile][w], then Z [column tile]
@@ -195,8 +196,8 @@ skinny_kernel(const __grid_constant__ Args a) {
 // shared memory (one thread adding 43 of them one after the other took 5 us at 2048 rows).
 __global__ void __launch_bounds__(256)
 sum_kernel(const __grid_constant__ Args a) {
-  __shared__ float4 s_part[8][32];
   pdl_wait();
+  __shared__ float4 s_part[8][32];
   const Job& j = a.job[blockIdx.y];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ny = (int64_t)j.n_w * a.T * 4, nz = j.z != nullptr ? (int64_t)j.n * 4 : 0;
@@ -354,8 +355,10 @@ extern "C" HYC_API int hyc_skinny_products(int count, const hyc_skinny_job* jobs
     if (slot >= 0) attr[slot] = true;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  skinny_kernel<<<first, SK_THREADS, SK_SMEM, st>>>(a);
+  launch_pdl(skinny_kernel, dim3((unsigned)first), dim3(SK_THREADS), SK_SMEM, st, a);
   HYC_CHECK_LAUNCH();
   const int64_t grid = (most + 31) / 32;
-  return launch_pdl(sum_kernel, dim3((unsigned)(grid < 4096 ? grid : 4096), count), dim3(256), 0, st, a);
+  launch_pdl(sum_kernel, dim3((unsigned)(grid < 4096 ? grid : 4096), count), dim3(256), 0, st, a);
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
 }

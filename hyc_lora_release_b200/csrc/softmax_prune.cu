@@ -71,6 +71,7 @@ template <bool NEG>
 __global__ void __launch_bounds__(kTileThreads, 8)
 prune_count_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, const float* __restrict__ thr_dev, int64_t n_tiles,
                    int64_t* __restrict__ ws) {
+  pdl_wait();
   constexpr int CB = 4;
   const __nv_bfloat162 t2 = __float2bfloat162_rn(thr_dev ? *thr_dev : thr);
   const int lane = threadIdx.x & 31;
@@ -99,6 +100,7 @@ prune_count_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr
 // block-wide scans chained by a carry.
 __global__ void __launch_bounds__(1024)
 prune_scan_kernel(int64_t* __restrict__ ws, int64_t n_tiles, int64_t* __restrict__ total_out) {
+  pdl_wait();
   constexpr int U = 8;
   __shared__ int64_t s_off[U][32];      // per scan: inclusive warp totals, then the warps' exclusive offsets
   __shared__ int64_t s_tot[U];
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
 prune_fill_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, const float* __restrict__ thr_dev, int64_t n_tiles,
                   const int64_t* __restrict__ ws, int64_t* __restrict__ idx_out,
                   __nv_bfloat16* __restrict__ val_out, int64_t capacity) {
+  pdl_wait();
   __shared__ uint32_t s_stage[kWarpsPerBlock][256 * kFillTrips];
   const __nv_bfloat162 t2 = __float2bfloat162_rn(thr_dev ? *thr_dev : thr);
   const int lane = threadIdx.x & 31;
@@ -220,6 +223,7 @@ prune_fill_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr,
 __global__ void __launch_bounds__(256)
 prune_scatter_kernel(const int64_t* __restrict__ idx, const __nv_bfloat16* __restrict__ val, int64_t nnz,
                      __nv_bfloat16* __restrict__ out, int64_t numel) {
+  pdl_wait();
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * 256) {
     const int64_t p = idx[i];
     if (p >= 0 && p < numel) out[p] = val[i];
@@ -231,6 +235,7 @@ __global__ void __launch_bounds__(256)
 prune_scatter_counted_kernel(const int64_t* __restrict__ idx, const __nv_bfloat16* __restrict__ val,
                              const int64_t* __restrict__ nnz_dev, int64_t capacity,
                              __nv_bfloat16* __restrict__ out, int64_t numel) {
+  pdl_wait();
   int64_t nnz = *nnz_dev;
   if (nnz > capacity) nnz = capacity;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * 256) {
@@ -294,6 +299,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
 prune_tiled_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, int64_t n_tiles,
                    uint32_t* __restrict__ words, uint32_t capacity, uint2* __restrict__ dir,
                    unsigned long long* __restrict__ counters, int64_t* __restrict__ nnz_out) {
+  pdl_wait();
   // A warp walks batches with a fixed stride.  Per batch: masks and counts from the eight chunks in registers, ONE
   // atomic add for the span, the entries staged in shared memory, and -- before anything waits for the atomic's
   // answer -- the loads of the warp's NEXT batch: the round trip of the atomic and the write-out of this batch run
@@ -427,6 +433,7 @@ prune_tiled_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr
 __global__ void __launch_bounds__(kTileThreads, 4)
 prune_tiled_restore_kernel(const uint32_t* __restrict__ words, uint32_t capacity, const uint2* __restrict__ dir,
                            __nv_bfloat16* __restrict__ out, int64_t numel, int64_t n_batches) {
+  pdl_wait();
   __shared__ __align__(16) uint16_t s_tile[kWarpsPerBlock][kBatchElems];
   const int lane = threadIdx.x & 31;
   uint16_t* tile = s_tile[threadIdx.x >> 5];
@@ -494,13 +501,13 @@ static inline float thr_bf16(float t) {
 // thr is the bf16-rounded threshold; a negative one (or NaN), and one that only the device knows, takes the kernels that also
 // test for zero
 static inline void launch_count(const __nv_bfloat16* a, int64_t numel, float thr, const float* thr_dev, int64_t nt, int64_t* ws, cudaStream_t st) {
-  if (thr >= 0.f && !thr_dev) prune_count_kernel<false><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nullptr, nt, ws);
-  else prune_count_kernel<true><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, thr_dev, nt, ws);
+  if (thr >= 0.f && !thr_dev) launch_pdl(prune_count_kernel<false>, dim3((unsigned)tile_grid(nt)), dim3(kTileThreads), 0, st, a, numel, thr, nullptr, nt, ws);
+  else launch_pdl(prune_count_kernel<true>, dim3((unsigned)tile_grid(nt)), dim3(kTileThreads), 0, st, a, numel, thr, thr_dev, nt, ws);
 }
 static inline void launch_fill(const __nv_bfloat16* a, int64_t numel, float thr, const float* thr_dev, int64_t nt, const int64_t* ws,
                                int64_t* idx_out, __nv_bfloat16* val_out, int64_t capacity, cudaStream_t st) {
-  if (thr >= 0.f && !thr_dev) prune_fill_kernel<false><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, nullptr, nt, ws, idx_out, val_out, capacity);
-  else prune_fill_kernel<true><<<tile_grid(nt), kTileThreads, 0, st>>>(a, numel, thr, thr_dev, nt, ws, idx_out, val_out, capacity);
+  if (thr >= 0.f && !thr_dev) launch_pdl(prune_fill_kernel<false>, dim3((unsigned)tile_grid(nt)), dim3(kTileThreads), 0, st, a, numel, thr, nullptr, nt, ws, idx_out, val_out, capacity);
+  else launch_pdl(prune_fill_kernel<true>, dim3((unsigned)tile_grid(nt)), dim3(kTileThreads), 0, st, a, numel, thr, thr_dev, nt, ws, idx_out, val_out, capacity);
 }
 
 }  // namespace hyc
@@ -520,7 +527,7 @@ static int prune_count(const void* a, int64_t numel, float thr, const float* thr
   const int64_t nt = n_tiles_of(numel);
   launch_count((const __nv_bfloat16*)a, numel, thr, thr_dev, nt, (int64_t*)workspace, st);
   HYC_CHECK_LAUNCH();
-  prune_scan_kernel<<<1, 1024, 0, st>>>((int64_t*)workspace, nt, nullptr);
+  launch_pdl(prune_scan_kernel, dim3(1), dim3(1024), 0, st, (int64_t*)workspace, nt, nullptr);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
@@ -568,7 +575,7 @@ extern "C" HYC_API int hyc_softmax_prune_restore(const int64_t* idx, const void*
   if (nnz > 0) {
     int64_t g = (nnz + 255) / 256;
     if (g > (int64_t)num_sms() * 16) g = (int64_t)num_sms() * 16;
-    prune_scatter_kernel<<<(int)g, 256, 0, st>>>(idx, (const __nv_bfloat16*)val, nnz, (__nv_bfloat16*)a_out, numel);
+    launch_pdl(prune_scatter_kernel, dim3((unsigned)g), dim3(256), 0, st, idx, (const __nv_bfloat16*)val, nnz, (__nv_bfloat16*)a_out, numel);
     HYC_CHECK_LAUNCH();
   }
   return HYC_OK;
@@ -583,7 +590,7 @@ extern "C" HYC_API int hyc_softmax_prune_restore_counted(const int64_t* idx, con
   if (capacity > 0) {
     int64_t g = (capacity + 255) / 256;
     if (g > (int64_t)num_sms() * 16) g = (int64_t)num_sms() * 16;
-    prune_scatter_counted_kernel<<<(int)g, 256, 0, st>>>(idx, (const __nv_bfloat16*)val, nnz_dev, capacity,
+    launch_pdl(prune_scatter_counted_kernel, dim3((unsigned)g), dim3(256), 0, st, idx, (const __nv_bfloat16*)val, nnz_dev, capacity,
                                                          (__nv_bfloat16*)a_out, numel);
     HYC_CHECK_LAUNCH();
   }
@@ -616,10 +623,10 @@ extern "C" HYC_API int hyc_softmax_prune_tiled(const void* a, int64_t numel, flo
   int64_t g = (nbt + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (g > (int64_t)num_sms() * 4) g = (int64_t)num_sms() * 4;
   if (thr >= 0.f)
-    prune_tiled_kernel<false><<<(int)g, kTileThreads, 0, st>>>((const __nv_bfloat16*)a, numel, thr, nt, words_out, (uint32_t)capacity,
+    launch_pdl(prune_tiled_kernel<false>, dim3((unsigned)g), dim3(kTileThreads), 0, st, (const __nv_bfloat16*)a, numel, thr, nt, words_out, (uint32_t)capacity,
                                                             (uint2*)directory_out, counters, nnz_out);
   else
-    prune_tiled_kernel<true><<<(int)g, kTileThreads, 0, st>>>((const __nv_bfloat16*)a, numel, thr, nt, words_out, (uint32_t)capacity,
+    launch_pdl(prune_tiled_kernel<true>, dim3((unsigned)g), dim3(kTileThreads), 0, st, (const __nv_bfloat16*)a, numel, thr, nt, words_out, (uint32_t)capacity,
                                                            (uint2*)directory_out, counters, nnz_out);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
@@ -633,19 +640,20 @@ extern "C" HYC_API int hyc_softmax_prune_tiled_restore(const uint32_t* words, in
   const int64_t nb = (numel + kBatchElems - 1) / kBatchElems;
   int64_t g = (nb + kWarpsPerBlock - 1) / kWarpsPerBlock;
   if (g > (int64_t)num_sms() * 4) g = (int64_t)num_sms() * 4;
-  prune_tiled_restore_kernel<<<(int)g, kTileThreads, 0, (cudaStream_t)stream>>>(words, (uint32_t)capacity, (const uint2*)directory,
+  launch_pdl(prune_tiled_restore_kernel, dim3((unsigned)g), dim3(kTileThreads), 0, (cudaStream_t)stream, words, (uint32_t)capacity, (const uint2*)directory,
                                                                              (__nv_bfloat16*)a_out, numel, nb);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
 
 static __global__ void prune_overflow_kernel(const int64_t* nnz, int64_t capacity, int* flag) {
+  pdl_wait();
   if (*nnz > capacity) *flag += 1;
 }
 
 extern "C" HYC_API int hyc_prune_overflow_flag(const int64_t* nnz, int64_t capacity, int* flag, void* stream) {
   if (!nnz || !flag) return HYC_ERR_NULL;
-  prune_overflow_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(nnz, capacity, flag);
+  launch_pdl(prune_overflow_kernel, dim3(1), dim3(1), 0, (cudaStream_t)stream, nnz, capacity, flag);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
@@ -711,7 +719,7 @@ extern "C" HYC_API int hyc_softmax_prune_static(const void* a, int64_t numel, fl
   const float thr = thr_bf16(threshold);
   launch_count((const __nv_bfloat16*)a, numel, thr, nullptr, nt, ws, st);
   HYC_CHECK_LAUNCH();
-  prune_scan_kernel<<<1, 1024, 0, st>>>(ws, nt, nnz_out);
+  launch_pdl(prune_scan_kernel, dim3(1), dim3(1024), 0, st, ws, nt, nnz_out);
   HYC_CHECK_LAUNCH();
   if (capacity > 0) {
     launch_fill((const __nv_bfloat16*)a, numel, thr, nullptr, nt, ws, idx_out, (__nv_bfloat16*)val_out, capacity, st);

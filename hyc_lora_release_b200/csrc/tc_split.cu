@@ -97,6 +97,7 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
   __syncthreads();
   if (PAIR) cluster_sync_all();      // the peer's barriers exist before anything is signalled there
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   const int et = (int)threadIdx.x - 64, quad = warp & 3;
@@ -276,11 +277,13 @@ static int launch_one(int split, const Operands& ops, const Params& p, cudaStrea
   cfg.blockDim = dim3(S_THREADS);
   cfg.dynamicSmemBytes = split_smem_bytes(pipe);
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   int stages = pipe / stage_bytes;
   if (stages > S_MAX_STAGES) stages = S_MAX_STAGES;
   Maps maps;

@@ -70,6 +70,7 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
                           __nv_bfloat16* __restrict__ val_out, uint16_t* __restrict__ col_out,
                           uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scale, int8_t* __restrict__ zp,
                           SoftmaxPrologue sp) {
+  pdl_wait();
   constexpr int RPW = 32 / LPR;          // rows per warp
   const int GPR = RAGGED ? groups : LPR; // groups per row
   const int S = 64 * GPR;
@@ -278,6 +279,7 @@ topk_lane_restore_kernel(const __nv_bfloat16* __restrict__ val, const uint16_t* 
                          const uint8_t* __restrict__ q, const __nv_bfloat16* __restrict__ scale,
                          const int8_t* __restrict__ zp, int64_t rows, int groups, const __nv_bfloat16* __restrict__ grad,
                          float oscale, __nv_bfloat16* __restrict__ ao) {
+  pdl_wait();
   constexpr int RPW = 32 / LPR;
   const int GPR = RAGGED ? groups : LPR;
   const int S = 64 * GPR;
@@ -384,6 +386,7 @@ template <int LPR, bool RAGGED>
 __global__ void __launch_bounds__(256, 3)
 softmax_bwd_lane_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ g, int64_t rows, int groups,
                         float oscale, __nv_bfloat16* __restrict__ out) {
+  pdl_wait();
   constexpr int RPW = 32 / LPR;
   const int GPR = RAGGED ? groups : LPR;
   const int S = 64 * GPR;
@@ -442,7 +445,7 @@ static void launch_softmax_bwd(const void* y, const void* g, int64_t rows, int g
   }
   int grid, threads;
   lane_launch_shape(kern, rows, 32 / LPR, grid, threads, 8192);
-  kern<<<grid, threads, (threads / 32) * 8192, st>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)g, rows, groups, oscale,
+  launch_pdl(kern, dim3((unsigned)grid), dim3(threads), (threads / 32) * 8192, st, (const __nv_bfloat16*)y, (const __nv_bfloat16*)g, rows, groups, oscale,
                                                      (__nv_bfloat16*)out);
 }
 
@@ -473,12 +476,12 @@ static void launch_compress(const void* a, int64_t rows, int groups, int k, void
   if (sp == nullptr) {
     auto kern = topk_lane_compress_kernel<QBIT, LPR, false, RAGGED>;
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads);
-    kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)a, rows, groups, k, (__nv_bfloat16*)val, col,
+    launch_pdl(kern, dim3((unsigned)grid), dim3(threads), 0, st, (const __nv_bfloat16*)a, rows, groups, k, (__nv_bfloat16*)val, col,
                                    (uint8_t*)q, (__nv_bfloat16*)scale, zp, SoftmaxPrologue{});
   } else if constexpr (!RAGGED) {
     auto kern = topk_lane_compress_kernel<QBIT, LPR, true, false>;
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads);
-    kern<<<grid, threads, 0, st>>>((const __nv_bfloat16*)a, rows, groups, k, (__nv_bfloat16*)val, col,
+    launch_pdl(kern, dim3((unsigned)grid), dim3(threads), 0, st, (const __nv_bfloat16*)a, rows, groups, k, (__nv_bfloat16*)val, col,
                                    (uint8_t*)q, (__nv_bfloat16*)scale, zp, *sp);
   }
 }
@@ -489,7 +492,7 @@ static void launch_restore(const void* val, const uint16_t* col, int k, const vo
   if (grad == nullptr) {
     auto kern = topk_lane_restore_kernel<QBIT, LPR, false, RAGGED>;
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads, 4096);
-    kern<<<grid, threads, (threads / 32) * 4096, st>>>((const __nv_bfloat16*)val, col, k, k > 0 ? 1.0f / (float)k : 0.f,
+    launch_pdl(kern, dim3((unsigned)grid), dim3(threads), (threads / 32) * 4096, st, (const __nv_bfloat16*)val, col, k, k > 0 ? 1.0f / (float)k : 0.f,
                                    (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows, groups, nullptr, 1.f, (__nv_bfloat16*)ao);
   } else {
     auto kern = topk_lane_restore_kernel<QBIT, LPR, true, RAGGED>;
@@ -501,7 +504,7 @@ static void launch_restore(const void* val, const uint16_t* col, int k, const vo
       if (slot >= 0) attr[slot] = true;
     }
     lane_launch_shape(kern, rows, 32 / LPR, grid, threads, 8192);
-    kern<<<grid, threads, (threads / 32) * 8192, st>>>((const __nv_bfloat16*)val, col, k, k > 0 ? 1.0f / (float)k : 0.f,
+    launch_pdl(kern, dim3((unsigned)grid), dim3(threads), (threads / 32) * 8192, st, (const __nv_bfloat16*)val, col, k, k > 0 ? 1.0f / (float)k : 0.f,
                                    (const uint8_t*)q, (const __nv_bfloat16*)scale, zp, rows, groups,
                                    (const __nv_bfloat16*)grad, oscale, (__nv_bfloat16*)ao);
   }
