@@ -8,14 +8,19 @@
 // matching 32 x R tile of gm on the tensor cores (m16n8k16, fp32 accumulate; both operands are
 // read from shared memory with transposing ldmatrix).  x_hat never goes to HBM: the kernel reads
 // T*H*q/8 bytes of codes where the two-step version reads and writes 2*T*H bytes twice.
-// Token chunks leave fp32 partials in a workspace; a second tiny kernel sums them in a fixed order.
+// The up to eight token chunks of the same columns are a cluster: their fp32 partials meet in distributed shared memory and
+// are added up in the order of the chunks.  The codes and gm rows of the next kGaAhead steps are on their way while a step is
+// worked on: the kernel waits for memory (issue slots 0.1 without that, every step a full round trip).
+// us, cold, with the second kernel that added the partials up before / now: 2048 tokens of 4096, 4 bits, one adapter 15.7 / 10.9,
+// three 22.4 / 14.1; 128 tokens, 8 bits, two adapters 11.6 / 7.5; 8192 tokens, 8 bits, two 35.5 / 28.9.
 #include "hyc_common.cuh"
 
 namespace hyc {
 
 constexpr int kGaCols = 128;      // hidden columns per block
 constexpr int kGaStep = 32;       // tokens per step
-constexpr int kGaChunk = 256;     // tokens per block
+constexpr int kGaMaxSplits = 8;   // token chunks = blocks of a cluster
+constexpr int kGaAhead = 4;
 constexpr int kGaMaxR = 64;
 
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_ptr) {
@@ -31,14 +36,29 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
 }
 
 // de-quantize one 32-column block of one row into 32 bf16 (16 packed words), reference rounding
+template <int QBIT> struct GaCodes { uint32_t w[QBIT]; };      // the packed bytes of a block
 template <int QBIT>
-__device__ __forceinline__ void dequant_block32(const uint8_t* __restrict__ src, const uint32_t (&s2)[16], uint32_t (&out)[16]) {
+__device__ __forceinline__ void load_codes32(const uint8_t* __restrict__ src, bool valid, GaCodes<QBIT>& c) {
+#pragma unroll
+  for (int i = 0; i < QBIT; ++i) c.w[i] = 0u;
+  if (!valid) return;
+  if constexpr (QBIT == 2) {
+    const uint2 a = *reinterpret_cast<const uint2*>(src);
+    c.w[0] = a.x; c.w[1] = a.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < QBIT / 4; ++i) {
+      const uint4 a = *reinterpret_cast<const uint4*>(src + 16 * i);
+      c.w[4 * i] = a.x; c.w[4 * i + 1] = a.y; c.w[4 * i + 2] = a.z; c.w[4 * i + 3] = a.w;
+    }
+  }
+}
+template <int QBIT>
+__device__ __forceinline__ void dequant_block32(const GaCodes<QBIT>& c, const uint32_t (&s2)[16], uint32_t (&out)[16]) {
   constexpr int EPP = 8 / QBIT, SLAB = 32 / EPP;
   constexpr uint32_t MASK = (1u << QBIT) - 1u, BM = MASK * 0x01010101u;
-  uint32_t w[8];
-  if (QBIT == 8) {
-    const uint4 a = *reinterpret_cast<const uint4*>(src), b = *reinterpret_cast<const uint4*>(src + 16);
-    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+  const uint32_t (&w)[QBIT] = c.w;
+  if constexpr (QBIT == 8) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {     // columns 2j, 2j+1 = bytes 2j, 2j+1
       const float f0 = (byte_to_magic_float(w[j >> 1], (2 * j) & 3) - 8388736.f) * bf16lo_to_f32(s2[j]);
@@ -46,13 +66,6 @@ __device__ __forceinline__ void dequant_block32(const uint8_t* __restrict__ src,
       out[j] = pack_bf16x2_rn(f0, f1);
     }
   } else {
-    if (QBIT == 4) {
-      const uint4 a = *reinterpret_cast<const uint4*>(src);
-      w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-    } else {
-      const uint2 a = *reinterpret_cast<const uint2*>(src);
-      w[0] = a.x; w[1] = a.y;
-    }
     constexpr uint32_t C1 = 0x4300u | (uint32_t)(1 << (QBIT - 1));
     const uint32_t c1 = C1 | (C1 << 16);
 #pragma unroll
@@ -71,22 +84,60 @@ __device__ __forceinline__ void dequant_block32(const uint8_t* __restrict__ src,
   }
 }
 
-template <int QBIT, int RT>   // RT = number of 16-row tiles of the LoRA dimension (R2 = 16 * RT)
+__device__ __forceinline__ uint32_t cluster_block_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_v4(const void* own, uint32_t rank) {      // the same variable in another block
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(own);
+  uint32_t r;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r) : "memory");
+  return v;
+}
+
+// grid (hidden blocks, chunks), cluster (1, chunks).  RT = number of 16-row tiles of the LoRA dimension (R2 = 16 * RT)
+template <int QBIT, int RT>
 __global__ void __launch_bounds__(128)
 lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restrict__ scale,
-                   const __nv_bfloat16* __restrict__ gm, int64_t ldg, int T, int H, float* __restrict__ ws) {
+                   const __nv_bfloat16* __restrict__ gm, int64_t ldg, int T, int H, int chunk, __nv_bfloat16* __restrict__ out) {
   pdl_wait();
-  constexpr int R2 = 16 * RT;
-  __shared__ __align__(16) __nv_bfloat16 xs[kGaStep][kGaCols + 8];
-  __shared__ __align__(16) __nv_bfloat16 gs[kGaStep][R2 + 8];
+  constexpr int R2 = 16 * RT, PIECES = kGaStep * (R2 / 8), PPT = (PIECES + 127) / 128;      // 16-byte pieces of a gm tile, per thread
+  constexpr int X_LD = kGaCols + 8, G_LD = R2 + 8;
+  // the tiles of two steps; after the last one the partials take their place
+  constexpr int X_BYTES = 2 * kGaStep * X_LD * 2, TILE_BYTES = X_BYTES + 2 * kGaStep * G_LD * 2, PART_BYTES = R2 * (kGaCols + 4) * 4;
+  __shared__ __align__(16) uint8_t s_raw[TILE_BYTES > PART_BYTES ? TILE_BYTES : PART_BYTES];
+  auto xs = reinterpret_cast<__nv_bfloat16 (*)[kGaStep][X_LD]>(s_raw);
+  auto gs = reinterpret_cast<__nv_bfloat16 (*)[kGaStep][G_LD]>(s_raw + X_BYTES);
+  auto part = reinterpret_cast<float (*)[kGaCols + 4]>(s_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h0 = blockIdx.x * kGaCols;
-  const int t_begin = blockIdx.y * kGaChunk;
-  const int t_end = min(T, t_begin + kGaChunk);
+  const int t_begin = blockIdx.y * chunk;
+  const int t_end = min(T, t_begin + chunk);
   const int64_t qld = (int64_t)H * QBIT / 8;
 
   // this thread de-quantizes block `blk` (32 columns) of row `lrow` of every step
   const int lrow = tid >> 2, blk = tid & 3;
+  const uint8_t* qp = q + (int64_t)(t_begin + lrow) * qld + (int64_t)(h0 + 32 * blk) * QBIT / 8;
+  GaCodes<QBIT> codes[kGaAhead];
+  uint4 gmv[kGaAhead][PPT];
+  auto fetch = [&](int t0, int slot) {
+    load_codes32<QBIT>(qp + (int64_t)(t0 - t_begin) * qld, t0 + lrow < t_end, codes[slot]);
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      const int p = tid + 128 * i, r = p / (R2 / 8), c = p % (R2 / 8);
+      gmv[slot][i] = make_uint4(0u, 0u, 0u, 0u);
+      if (p < PIECES && t0 + r < t_end) gmv[slot][i] = *reinterpret_cast<const uint4*>(gm + (int64_t)(t0 + r) * ldg + 8 * c);
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < kGaAhead; ++i) fetch(t_begin + kGaStep * i, i);
   uint32_t s2[16];
   {
     const uint4* sp = reinterpret_cast<const uint4*>(scale + h0 + 32 * blk);
@@ -101,67 +152,70 @@ lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restric
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
 
-  for (int t0 = t_begin; t0 < t_end; t0 += kGaStep) {
-    const int row = t0 + lrow;
-    uint32_t xv[16];
-    if (row < t_end) {
-      dequant_block32<QBIT>(q + row * qld + (int64_t)(h0 + 32 * blk) * QBIT / 8, s2, xv);
-    } else {
+  for (int tb = t_begin; tb < t_end; tb += kGaStep * kGaAhead) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) xv[j] = 0u;
-    }
-    uint4* xdst = reinterpret_cast<uint4*>(&xs[lrow][32 * blk]);
+    for (int u = 0; u < kGaAhead; ++u) {
+      const int t0 = tb + kGaStep * u, buf = u & 1;
+      if (t0 >= t_end) break;
+      uint32_t xv[16];
+      dequant_block32<QBIT>(codes[u], s2, xv);
+      if (t0 + lrow >= t_end) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) xdst[i] = make_uint4(xv[4 * i], xv[4 * i + 1], xv[4 * i + 2], xv[4 * i + 3]);
-    // gm tile: 32 rows x R2 columns, 16-byte pieces
-    for (int i = tid; i < kGaStep * (R2 / 8); i += 128) {
-      const int r = i / (R2 / 8), c = i % (R2 / 8);
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (t0 + r < t_end) v = *reinterpret_cast<const uint4*>(gm + (int64_t)(t0 + r) * ldg + 8 * c);
-      *reinterpret_cast<uint4*>(&gs[r][8 * c]) = v;
-    }
-    __syncthreads();
+        for (int j = 0; j < 16; ++j) xv[j] = 0u;
+      }
+      uint4* xdst = reinterpret_cast<uint4*>(&xs[buf][lrow][32 * blk]);
 #pragma unroll
-    for (int kk = 0; kk < kGaStep / 16; ++kk) {
-      const int k0 = 16 * kk;
-      uint32_t a[RT][4];
+      for (int i = 0; i < 4; ++i) xdst[i] = make_uint4(xv[4 * i], xv[4 * i + 1], xv[4 * i + 2], xv[4 * i + 3]);
 #pragma unroll
-      for (int m = 0; m < RT; ++m)
-        ldmatrix_x4_trans(a[m], &gs[k0 + (lane & 7) + ((lane >> 4) & 1) * 8][16 * m + ((lane >> 3) & 1) * 8]);
+      for (int i = 0; i < PPT; ++i) {
+        const int p = tid + 128 * i;
+        if (p < PIECES) *reinterpret_cast<uint4*>(&gs[buf][p / (R2 / 8)][8 * (p % (R2 / 8))]) = gmv[u][i];
+      }
+      fetch(t0 + kGaStep * kGaAhead, u);
+      __syncthreads();      // (one barrier per step: the tile written next was read a step ago)
 #pragma unroll
-      for (int np = 0; np < 2; ++np) {     // two 8-column tiles per ldmatrix
-        uint32_t b[4];
-        ldmatrix_x4_trans(b, &xs[k0 + (lane & 7) + ((lane >> 3) & 1) * 8][32 * warp + 16 * np + ((lane >> 4) & 1) * 8]);
+      for (int kk = 0; kk < kGaStep / 16; ++kk) {
+        const int k0 = 16 * kk;
+        uint32_t a[RT][4];
 #pragma unroll
-        for (int m = 0; m < RT; ++m) {
-          mma16816(acc[m][2 * np], a[m], b[0], b[1]);
-          mma16816(acc[m][2 * np + 1], a[m], b[2], b[3]);
+        for (int m = 0; m < RT; ++m)
+          ldmatrix_x4_trans(a[m], &gs[buf][k0 + (lane & 7) + ((lane >> 4) & 1) * 8][16 * m + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+        for (int np = 0; np < 2; ++np) {     // two 8-column tiles per ldmatrix
+          uint32_t b[4];
+          ldmatrix_x4_trans(b, &xs[buf][k0 + (lane & 7) + ((lane >> 3) & 1) * 8][32 * warp + 16 * np + ((lane >> 4) & 1) * 8]);
+#pragma unroll
+          for (int m = 0; m < RT; ++m) {
+            mma16816(acc[m][2 * np], a[m], b[0], b[1]);
+            mma16816(acc[m][2 * np + 1], a[m], b[2], b[3]);
+          }
         }
       }
     }
-    __syncthreads();
   }
-  // fp32 partials: ws[split][r][h]
-  float* wbase = ws + (int64_t)blockIdx.y * R2 * H;
+  __syncthreads();
   const int g = lane >> 2, tq = lane & 3;
 #pragma unroll
   for (int m = 0; m < RT; ++m)
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-      const int h = h0 + 32 * warp + 8 * n + 2 * tq;
-      *reinterpret_cast<float2*>(wbase + (int64_t)(16 * m + g) * H + h) = make_float2(acc[m][n][0], acc[m][n][1]);
-      *reinterpret_cast<float2*>(wbase + (int64_t)(16 * m + g + 8) * H + h) = make_float2(acc[m][n][2], acc[m][n][3]);
+      const int h = 32 * warp + 8 * n + 2 * tq;
+      *reinterpret_cast<float2*>(&part[16 * m + g][h]) = make_float2(acc[m][n][0], acc[m][n][1]);
+      *reinterpret_cast<float2*>(&part[16 * m + g + 8][h]) = make_float2(acc[m][n][2], acc[m][n][3]);
     }
-}
-
-__global__ void __launch_bounds__(256)
-lora_grad_a_reduce_kernel(const float* __restrict__ ws, int splits, int64_t n, __nv_bfloat16* __restrict__ out) {
-  pdl_wait();
-  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += ws[(int64_t)k * n + i];
-    out[i] = __ushort_as_bfloat16(f32_to_bf16bits_rn(s));
+  // every block of the cluster adds up its share of the rows
+  const int splits = (int)gridDim.y;
+  if (splits > 1) cluster_barrier(); else __syncthreads();
+  for (int r = (splits > 1 ? (int)cluster_block_rank() : 0) * 4 + warp; r < R2; r += 4 * splits) {
+    const int h = 4 * lane;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < splits; ++k) {
+      const float4 v = splits > 1 ? ld_cluster_v4(&part[r][h], (uint32_t)k) : *reinterpret_cast<const float4*>(&part[r][h]);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    *reinterpret_cast<uint2*>(out + (int64_t)r * H + h0 + h) = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
   }
+  if (splits > 1) cluster_barrier();      // nobody leaves while its partials may be read
 }
 
 }  // namespace hyc
@@ -169,8 +223,33 @@ lora_grad_a_reduce_kernel(const float* __restrict__ ws, int splits, int64_t n, _
 using namespace hyc;
 
 extern "C" HYC_API size_t hyc_lora_grad_a_workspace_bytes(int T, int H, int R2) {
-  if (T <= 0 || H <= 0 || R2 <= 0) return 0;
-  return (size_t)((T + kGaChunk - 1) / kGaChunk) * (size_t)R2 * (size_t)H * sizeof(float);
+  return T <= 0 || H <= 0 || R2 <= 0 ? 0 : 16;      // (the partial sums stay on chip)
+}
+
+// tokens per block: eight blocks at most share the tokens, whole steps each
+static int ga_chunk(int T) {
+  const int steps = (T + kGaStep - 1) / kGaStep;
+  return (steps + kGaMaxSplits - 1) / kGaMaxSplits * kGaStep;
+}
+
+template <int QBIT, int RT>
+static int launch_ga(const void* q, const void* scale, const void* gm, int64_t ldg, int T, int H, void* out, cudaStream_t st) {
+  const int chunk = ga_chunk(T), splits = (T + chunk - 1) / chunk;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(H / kGaCols), (unsigned)splits);
+  cfg.blockDim = dim3(128);
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)splits; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = splits > 1 ? 2 : 1;
+  (void)cudaLaunchKernelEx(&cfg, lora_grad_a_kernel<QBIT, RT>, (const uint8_t*)q, (const __nv_bfloat16*)scale, (const __nv_bfloat16*)gm, ldg, T, H,
+                           chunk, (__nv_bfloat16*)out);
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
 }
 
 extern "C" HYC_API int hyc_lora_grad_a_dequant(const void* q, const void* scale, const void* gm, int64_t ldg, int R2,
@@ -182,19 +261,11 @@ extern "C" HYC_API int hyc_lora_grad_a_dequant(const void* q, const void* scale,
   if (!aligned(q, 16) || !aligned(scale, 16) || !aligned(gm, 16) || ldg % 8 != 0 || !aligned(workspace, 16)) return HYC_ERR_ALIGN;
   if (workspace_bytes < hyc_lora_grad_a_workspace_bytes(T, H, R2)) return HYC_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  const int splits = (T + kGaChunk - 1) / kGaChunk;
-  dim3 grid(H / kGaCols, splits);
-#define GA(QB, RT) launch_pdl(lora_grad_a_kernel<QB, RT>, grid, dim3(128), 0, st, (const uint8_t*)q, (const __nv_bfloat16*)scale, \
-      (const __nv_bfloat16*)gm, ldg, T, H, (float*)workspace)
-#define GAQ(QB) do { switch (R2 / 16) { case 1: GA(QB, 1); break; case 2: GA(QB, 2); break; case 3: GA(QB, 3); break; default: GA(QB, 4); } } while (0)
-  if (q_bit == 2) GAQ(2); else if (q_bit == 4) GAQ(4); else GAQ(8);
+#define GA(QB, RT) return launch_ga<QB, RT>(q, scale, gm, ldg, T, H, out, st)
+#define GAQ(QB) switch (R2 / 16) { case 1: GA(QB, 1); case 2: GA(QB, 2); case 3: GA(QB, 3); default: GA(QB, 4); }
+  if (q_bit == 2) { GAQ(2) }
+  if (q_bit == 4) { GAQ(4) }
+  GAQ(8)
 #undef GAQ
 #undef GA
-  HYC_CHECK_LAUNCH();
-  const int64_t n = (int64_t)R2 * H;
-  int64_t rb = (n + 255) / 256;
-  if (rb > num_sms() * 8) rb = num_sms() * 8;
-  launch_pdl(lora_grad_a_reduce_kernel, dim3((unsigned)rb), dim3(256), 0, st, (const float*)workspace, splits, n, (__nv_bfloat16*)out);
-  HYC_CHECK_LAUNCH();
-  return HYC_OK;
 }

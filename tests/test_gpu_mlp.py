@@ -114,6 +114,23 @@ def test_lora_grad_a_with_dequant_inside(mlp, q, T, H, R2, ldg):
     assert out.shape == (R2, H) and close(out, ref, rel=4e-3)
 
 
+@pytest.mark.parametrize("q", (2, 4, 8))
+@pytest.mark.parametrize("T,R2", [(1, 16), (31, 48), (32, 64), (33, 32), (129, 16), (255, 64), (289, 48), (2100, 32)])
+def test_lora_grad_a_shares_of_the_tokens(mlp, q, T, R2):
+    """One to eight blocks share the tokens, in whole steps of 32, the last one with what is left."""
+    g = torch.Generator().manual_seed(T + q)
+    H = 256
+    codes = torch.randint(0, 256, (T, H * q // 8), generator=g).to(torch.uint8)
+    s = (torch.rand(H, generator=g) + 0.01).to(BF16)
+    s[3] = float("inf")                   # a column of its own: it must not reach others, nor rows behind the last token
+    gm = _randn(g, T, R2)
+    out = mlp.lora_grad_a(codes.to(DEV), s.to(DEV), gm.to(DEV), R2, q).float().cpu()
+    xhat = oracle.ref_decompress(codes[None], s[None], q)[0].float()
+    keep = torch.arange(H) != 3
+    ref = gm.float().t() @ xhat
+    assert not out[:, 3].isfinite().any() and close(out[:, keep], ref[:, keep], rel=4e-3)
+
+
 def _mlp_problem(g, B, M, H, I, R=16):
     x = _randn(g, B, M, H)
     x[:, :, torch.randperm(H, generator=g)[: max(1, H // 200)]] *= 20
