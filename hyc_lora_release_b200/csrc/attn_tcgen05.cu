@@ -322,7 +322,7 @@ template <int QBIT>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   const Bars bar(smem + AT_BARS);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // the query tiles with the most key tiles (a causal map's last ones) start first
@@ -523,7 +523,7 @@ struct BwdQMaps { CUtensorMap g, v, k, p; };
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   const Bars bar(smem + AT_BARS);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int bh = (int)blockIdx.x % (p.B * p.heads), qt = p.tiles - 1 - (int)blockIdx.x / (p.B * p.heads);
@@ -704,7 +704,7 @@ struct BwdKvMaps { CUtensorMap p, s, g, q; };
 __global__ void __launch_bounds__(KV_THREADS, 1)
 attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   const Bars bar(smem + KV_BARS);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // the first key tiles have the most query tiles under a causal mask: they start first

@@ -56,8 +56,7 @@ template <int EPI, int QBIT, bool B_MN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
   extern __shared__ uint8_t smem_raw[];
-  // 1024-byte alignment for the 128-byte swizzle atoms
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   uint8_t* stage_base = smem;
   const int stages = p.stages, stage_bytes = p.stage_bytes;
   constexpr int TILE_M = Geo<PAIR>::TILE_M;

@@ -69,7 +69,7 @@ constexpr uint32_t kAMn = 1u << 15;
 __global__ void __launch_bounds__(SK_THREADS, 1)
 skinny_kernel(const __grid_constant__ Args a) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BARS_AT);
   uint64_t *full = bars, *empty = bars + RING, *aux_full = bars + 2 * RING, *acc_full = aux_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);

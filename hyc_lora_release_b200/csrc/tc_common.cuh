@@ -103,6 +103,11 @@ __device__ __forceinline__ StoreView store_view(const Params& p, int n0) {
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Dynamic shared memory from the next 1024-byte boundary on (swizzle atoms).  By an offset and not by rounding the address: a
+// pointer that went through an integer is no longer known to be a shared one, and every access through it is a generic one (us,
+// cold, generic / shared: attention forward 126 / 119, its q side backward 118 / 113, down projection of 2048 tokens 139 / 136).
+__device__ __forceinline__ uint8_t* align_shared(uint8_t* raw) { return raw + ((0u - smem_u32(raw)) & 1023u); }
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(S_THREADS, 2)
 split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, int stages, int a_bytes) {
   static_assert(EPI == EPI_STORE || (EPI == EPI_GATEUP && !PAIR && !B_MN), "the forms that choose_split picks");
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = align_shared(smem_raw);
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
   constexpr int B_BYTES = (PAIR ? SBN / 2 : SBN) * BK * 2;        // this CTA's part of the B block
   const int stage_bytes = a_bytes + B_BYTES;
