@@ -81,6 +81,12 @@ SIGNATURES = {
     "hyc_attn_mask_class_bytes": (_z, [_i, _i, _i]),
     "hyc_attn_mask_class": (_i, [_p, _l, _l, _l, _i, _i, _i, _p, _p]),
     "hyc_attn_fwd_tcgen05": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _f, _p, _l, _l, _l, _p, _l, _l, _p, _p, _p, _p, _i, _p, _p]),
+    "hyc_attn_fwd_cols_tcgen05": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _f, _p, _l, _l, _l, _p, _l, _l, _p, _p, _p, _p, _p, _i, _p, _p]),
+    "hyc_softmax_prune_tiled_cols": (_i, [_p, _l, _i, _p, _f, _p, _l, _p, _p, _p]),
+    "hyc_softmax_prune_tiled_restore_cols": (_i, [_p, _l, _p, _i, _p, _p, _l, _p]),
+    "hyc_softmax_topk_cols_supported": (_i, [_i, _i]),
+    "hyc_softmax_topk_compress_cols": (_i, [_p, _l, _i, _p, _i, _p, _p, _p, _p, _p, _i, _p]),
+    "hyc_softmax_topk_restore_cols": (_i, [_p, _p, _i, _p, _p, _p, _l, _i, _p, _p, _i, _p]),
     "hyc_attn_bwd_tcgen05": (_i, [_p] * 6 + [_i] * 5 + [_f, _p, _l, _l, _p, _p, _p, _p, _p]),
     "hyc_linears_lora_save_fwd_tcgen05": (_i, [_p, _i, _i, _i] + [_p] * 7 + [_i, _p, _p]),
     "hyc_mlp_graddown_bwd_tcgen05": (_i, [_p, _p, _i, _i, _i, _p, _p, _i, _p, _p, _l, _l, _p, _p, _l, _l,

@@ -597,7 +597,7 @@ extern "C" HYC_API int hyc_softmax_topk_restore(const void* val, const uint16_t*
   if (rows == 0) return HYC_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (topk_lane_ok(S, k) && aligned(q, 32)) {
-    const int rc = topk_lane_restore(val, col, k, q, scale, zp, rows, S, nullptr, 1.f, a_out, q_bit, st);
+    const int rc = topk_lane_restore(val, col, k, q, scale, zp, rows, S, nullptr, nullptr, 1.f, a_out, q_bit, st);
     if (rc) return rc;
     HYC_CHECK_LAUNCH();
     return HYC_OK;
@@ -621,8 +621,41 @@ extern "C" HYC_API int hyc_softmax_topk_restore_bwd(const void* val, const uint1
   if (!aligned(out, 32) || !aligned(grad, 32) || !aligned(q, 16)) return HYC_ERR_ALIGN;
   if (!topk_lane_ok(S, k) || !aligned(q, 32)) return HYC_ERR_UNSUPPORTED;   // caller: restore, then hyc_softmax_bwd
   if (rows == 0) return HYC_OK;
-  const int rc = topk_lane_restore(val, col, k, q, scale, zp, rows, S, grad, out_scale, out, q_bit, (cudaStream_t)stream);
+  const int rc = topk_lane_restore(val, col, k, q, scale, zp, rows, S, nullptr, grad, out_scale, out, q_bit, (cudaStream_t)stream);
   if (rc) return rc;
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
+}
+
+extern "C" HYC_API int hyc_softmax_topk_cols_supported(int M, int k) { return topk_lane_cols_ok(M, k) ? 1 : 0; }
+
+// square maps of M rows; group numbers have 32 bits
+static int check_topk_cols(int64_t rows, int M, int k, int q_bit) {
+  if (q_bit != 2 && q_bit != 4 && q_bit != 8) return HYC_ERR_QBIT;
+  if (rows < 0 || M <= 0 || rows % M != 0 || k < 0 || k > M) return HYC_ERR_SHAPE;
+  return topk_lane_cols_ok(M, k) && rows * (M / 64) < 0x7fffffffll ? HYC_OK : HYC_ERR_UNSUPPORTED;
+}
+
+extern "C" HYC_API int hyc_softmax_topk_compress_cols(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val_out,
+                                                      uint16_t* col_out, void* q_out, void* scale_out, int8_t* zp_out, int q_bit, void* stream) {
+  if (!a || !row_cols || !q_out || !scale_out || !zp_out) return HYC_ERR_NULL;
+  if (k > 0 && (!val_out || !col_out)) return HYC_ERR_NULL;
+  if (const int rc = check_topk_cols(rows, M, k, q_bit)) return rc;
+  if (!aligned(a, 32) || !aligned(q_out, 32) || !aligned(row_cols, 2)) return HYC_ERR_ALIGN;
+  if (rows == 0) return HYC_OK;
+  if (const int rc = topk_lane_compress_cols(a, rows, M, row_cols, k, val_out, col_out, q_out, scale_out, zp_out, q_bit, (cudaStream_t)stream)) return rc;
+  HYC_CHECK_LAUNCH();
+  return HYC_OK;
+}
+
+extern "C" HYC_API int hyc_softmax_topk_restore_cols(const void* val, const uint16_t* col, int k, const void* q, const void* scale, const int8_t* zp,
+                                                     int64_t rows, int M, const uint16_t* row_cols, void* a_out, int q_bit, void* stream) {
+  if (!q || !scale || !zp || !a_out || !row_cols) return HYC_ERR_NULL;
+  if (k > 0 && (!val || !col)) return HYC_ERR_NULL;
+  if (const int rc = check_topk_cols(rows, M, k, q_bit)) return rc;
+  if (!aligned(a_out, 32) || !aligned(q, 32) || !aligned(row_cols, 2)) return HYC_ERR_ALIGN;
+  if (rows == 0) return HYC_OK;
+  if (const int rc = topk_lane_restore(val, col, k, q, scale, zp, rows, M, row_cols, nullptr, 1.f, a_out, q_bit, (cudaStream_t)stream)) return rc;
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }

@@ -57,17 +57,17 @@ std::tuple<Tensor, OptTensor> quant(const Tensor& x, const Tensor& s, int64_t q_
                                     const OptTensor& out_q, const OptTensor& out_xo);
 Tensor dequant(const Tensor& q, const Tensor& s, int64_t q_bit, const OptTensor& z, const OptTensor& channel, const OptTensor& xo,
                const OptTensor& out);
-std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit);
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& row_cols = {});
 void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& val, const Tensor& col, const Tensor& q,
                         const Tensor& s, const Tensor& z);
 Tensor topk_restore(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
-                    at::IntArrayRef shape, int64_t q_bit, const OptTensor& out);
+                    at::IntArrayRef shape, int64_t q_bit, const OptTensor& out, const Tensor& row_cols = {});
 Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
                              at::IntArrayRef shape, int64_t q_bit, const Tensor& grad, const OptTensor& out, double scale);
 Tensor prune_sparse(const Tensor& x, double thr, const OptTensor& thr_dev);
 Tensor prune_restore(const Tensor& idx, const Tensor& val, int64_t numel);
-std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity);
-Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out);
+std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity, const Tensor& row_cols = {});
+Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out, const Tensor& row_cols = {});
 std::tuple<Tensor, Tensor, Tensor> silu_forward(const Tensor& xa1, const Tensor& b1, const Tensor& x1, const Tensor& s1,
                                                 const Tensor& xa2, const Tensor& b2, const Tensor& x2, const Tensor& s2, int64_t q_bit);
 std::tuple<Tensor, Tensor, Tensor> silu_backward(const Tensor& xa1, const Tensor& b1, const Tensor& q1, const Tensor& s1,

@@ -294,8 +294,11 @@ static void rope_pair(const Tensor& q, int64_t nh, const Tensor& k, int64_t nkv,
 
 // the q, k, v projections with their saves, rotary embedding, scores and probabilities
 using MapForward = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor, OptTensor, int64_t, int64_t>;
+// row_cols (wanted if not null): how far each row of the probabilities reaches; what lies behind is zero and then not written.
+// Left undefined where the rows are whole
 static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const RopeTables& tables,
-                                   const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status) {
+                                   const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status,
+                                   Tensor* row_cols = nullptr) {
   const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
   check_geometry({wq.size(0), wk.size(0), wv.size(0)}, nh, d, nkv);
@@ -328,10 +331,12 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
       check(hyc_attn_mask_class(data(mv.t), mv.b, mv.h, mv.row, (int)nb, (int)nhm, (int)M, data(cls), on.stream), "hyc_attn_mask_class");
       cls_b = nb == 1 ? 0 : nhm;
       cls_h = nhm == 1 ? 0 : 1;
+      // (a mask per head with grouped heads: the backward kernels read the whole map)
+      if (row_cols && !(cls_h != 0 && nh != nkv)) *row_cols = empty({B * nh * M}, x_norm, at::kShort);
     }
-    check(hyc_attn_fwd_tcgen05(data(qy), data(ky), data(vy), (int)B, (int)M, (int)nh, (int)nkv, (int)d, (float)(1.0 / std::sqrt((double)d)),
-                               data(mv.t), mv.b, mv.h, mv.row, data(cls), cls_b, cls_h, data(a), data(o2), data(os), data(o_q), (int)q,
-                               status_ptr(status), on.stream), "hyc_attn_fwd_tcgen05");
+    check(hyc_attn_fwd_cols_tcgen05(data(qy), data(ky), data(vy), (int)B, (int)M, (int)nh, (int)nkv, (int)d, (float)(1.0 / std::sqrt((double)d)),
+                               data(mv.t), mv.b, mv.h, mv.row, data(cls), cls_b, cls_h, data(a), row_cols ? (uint16_t*)data(*row_cols) : nullptr,
+                               data(o2), data(os), data(o_q), (int)q, status_ptr(status), on.stream), "hyc_attn_fwd_cols_tcgen05");
     return {a, o2, rstd, x_o, x_q, *xn_q, q_q, k_q, v_q, xa3, o_q, cls, cls_b, cls_h};
   }
   const Tensor kh = repeat_kv(heads(ky, B, M, nkv), rep), vh = repeat_kv(heads(vy, B, M, nkv), rep);
@@ -564,6 +569,7 @@ struct LayerSaved {
   std::vector<Tensor> map;                      // top-k form: five tensors; pruned form: words, directory, nnz
   OptTensor cls;
   int64_t cls_b = 0, cls_h = 0;
+  Tensor row_cols;                              // how far the rows of the map reach; undefined: they are whole
   std::vector<Tensor> stats;
   RopeTables tables;
   int64_t B, M, H, nh, d, nkv, q_attn, q_mlp, map_q;    // map_q = 0: pruned form
@@ -592,15 +598,17 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
     Tensor a, o2;
     OptTensor o_codes;
     std::vector<Tensor> w = matrices({&p.w[PQ], &p.w[PK], &p.w[PV]});
+    // where the save and the restore know how to leave out what the mask rules out
+    const bool cols = map_q == 0 ? s->M % 256 == 0 : hyc_softmax_topk_cols_supported((int)s->M, (int)map_k) == 1;
     std::tie(a, o2, s->rstd, s->x_o, s->x_q, s->xn_q, s->q_q, s->k_q, s->v_q, s->xa3, o_codes, s->cls, s->cls_b, s->cls_h) = attn_forward_map(
         x, {p.norm1, w[0], w[1], w[2], p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
-        {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status);
+        {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status, cols ? &s->row_cols : nullptr);
     w.clear();
     if (map_q > 0) {
-      auto [val, col, q, sc, z] = topk_compress(a, map_k, map_q);
+      auto [val, col, q, sc, z] = topk_compress(a, map_k, map_q, s->row_cols);
       s->map = {val, col, q, sc, z};
     } else {
-      auto [words, directory, nnz] = prune_tiled(a, threshold, capacity);
+      auto [words, directory, nnz] = prune_tiled(a, threshold, capacity, s->row_cols);
       s->map = {words, directory, nnz};
     }
     a.reset();
@@ -667,8 +675,8 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
     lora(PO, r[1], r[0]);
     const std::vector<int64_t> a_shape = {s.B, s.nh, s.M, s.M};
     const bool topk = s.map_q > 0;
-    Tensor a = topk ? topk_restore(s.map[0], s.map[1], s.map[2], s.map[3], s.map[4], a_shape, s.map_q, std::nullopt)
-                    : prune_tiled_restore(s.map[0], s.map[1], a_shape, std::nullopt);
+    Tensor a = topk ? topk_restore(s.map[0], s.map[1], s.map[2], s.map[3], s.map[4], a_shape, s.map_q, std::nullopt, s.row_cols)
+                    : prune_tiled_restore(s.map[0], s.map[1], a_shape, std::nullopt, s.row_cols);
     grads = attn_backward_map(r[2], std::move(a), topk ? s.map : std::vector<Tensor>(), s.map_q,
                               {s.q_q, st[Q_SCALE], s.xa3.select(0, 0), s.k_q, st[K_SCALE], s.xa3.select(0, 1), s.v_q, st[V_SCALE], s.xa3.select(0, 2)},
                               {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.tables, s.B, s.M, s.nh, s.d, s.nkv, s.q_attn,

@@ -122,21 +122,34 @@ void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor&
                                   data(s), (int8_t*)data(z), (int)q_bit, on.stream), "hyc_softmax_topk_compress");
 }
 
-std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit) {
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& row_cols) {
   const int64_t S = row_length(x), rows = x.numel() / S;
   require_cuda({&x});
   check_q(q_bit);
   Tensor val = empty({rows, k}, x), col = empty({rows, k}, x, at::kShort), q = empty({rows, S * q_bit / 8}, x, at::kByte),
          s = empty({rows, S / 64}, x), z = empty({rows, S / 64}, x, at::kChar);
-  topk_compress_into(x, k, q_bit, val, col, q, s, z);
+  if (row_cols.defined()) {
+    OnDevice on(x);
+    check(hyc_softmax_topk_compress_cols(data(x), rows, (int)S, (const uint16_t*)data(row_cols), (int)k, k ? data(val) : nullptr,
+                                         k ? (uint16_t*)data(col) : nullptr, data(q), data(s), (int8_t*)data(z), (int)q_bit, on.stream),
+          "hyc_softmax_topk_compress_cols");
+  } else {
+    topk_compress_into(x, k, q_bit, val, col, q, s, z);
+  }
   return {val, col, q, s, z};
 }
 
 Tensor topk_restore(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
-                    at::IntArrayRef shape, int64_t q_bit, const OptTensor& out) {
+                    at::IntArrayRef shape, int64_t q_bit, const OptTensor& out, const Tensor& row_cols) {
   OnDevice on(q);
   Tensor x = given(out) ? *out : empty(shape, q);
   const int64_t k = val.size(1);
+  if (row_cols.defined()) {
+    check(hyc_softmax_topk_restore_cols(k ? data(val) : nullptr, k ? (const uint16_t*)data(col) : nullptr, (int)k, data(q), data(s),
+                                        (const int8_t*)data(z), q.size(0), (int)shape.back(), (const uint16_t*)data(row_cols), data(x), (int)q_bit,
+                                        on.stream), "hyc_softmax_topk_restore_cols");
+    return x;
+  }
   check(hyc_softmax_topk_restore(k ? data(val) : nullptr, k ? (const uint16_t*)data(col) : nullptr, (int)k, data(q), data(s),
                                  (const int8_t*)data(z), q.size(0), (int)shape.back(), data(x), (int)q_bit, on.stream), "hyc_softmax_topk_restore");
   return x;
@@ -202,21 +215,30 @@ Tensor prune_restore(const Tensor& idx_in, const Tensor& val_in, int64_t numel) 
   return out;
 }
 
-std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity) {
+std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity, const Tensor& row_cols) {
   require_cuda({&x});
   OnDevice on(x);
   const Tensor xf = bf16c(x);
   const int64_t numel = xf.numel();
   Tensor nnz = empty({1}, x, at::kLong), words = empty({capacity}, x, at::kInt),
          dir = empty({(int64_t)(hyc_softmax_prune_tiled_directory_bytes(numel) / 4)}, x, at::kInt);
-  check(hyc_softmax_prune_tiled(data(xf), numel, (float)thr, (uint32_t*)data(words), capacity, data(dir), (int64_t*)data(nnz), on.stream),
-        "hyc_softmax_prune_tiled");
+  if (row_cols.defined())
+    check(hyc_softmax_prune_tiled_cols(data(xf), numel, (int)x.size(-1), (const uint16_t*)data(row_cols), (float)thr, (uint32_t*)data(words), capacity,
+                                       data(dir), (int64_t*)data(nnz), on.stream), "hyc_softmax_prune_tiled_cols");
+  else
+    check(hyc_softmax_prune_tiled(data(xf), numel, (float)thr, (uint32_t*)data(words), capacity, data(dir), (int64_t*)data(nnz), on.stream),
+          "hyc_softmax_prune_tiled");
   return {words, dir, nnz};
 }
 
-Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out) {
+Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out, const Tensor& row_cols) {
   OnDevice on(words);
   Tensor x = given(out) ? *out : empty(shape, words);
+  if (row_cols.defined()) {
+    check(hyc_softmax_prune_tiled_restore_cols((const uint32_t*)data(words), words.numel(), data(directory), (int)shape.back(),
+                                               (const uint16_t*)data(row_cols), data(x), x.numel(), on.stream), "hyc_softmax_prune_tiled_restore_cols");
+    return x;
+  }
   check(hyc_softmax_prune_tiled_restore((const uint32_t*)data(words), words.numel(), data(directory), data(x), x.numel(), on.stream),
         "hyc_softmax_prune_tiled_restore");
   return x;
@@ -386,7 +408,7 @@ Tensor dequant_nf4(const Tensor& packed, const Tensor& code, const Tensor& absma
 void bind_ops(pybind11::module_& m) {
   m.def("quant", &quant);
   m.def("dequant", &dequant);
-  m.def("topk_compress", &topk_compress);
+  m.def("topk_compress", [](const Tensor& x, int64_t k, int64_t q_bit) { return topk_compress(x, k, q_bit); });
   m.def("topk_compress_into", &topk_compress_into);
   m.def("topk_restore", [](const Tensor& v, const Tensor& c, const Tensor& q, const Tensor& s, const Tensor& z, std::vector<int64_t> shape,
                            int64_t q_bit, const OptTensor& out) { return topk_restore(v, c, q, s, z, shape, q_bit, out); });
@@ -395,7 +417,7 @@ void bind_ops(pybind11::module_& m) {
     return topk_softmax_backward(v, c, q, s, z, shape, q_bit, g, out, scale); });
   m.def("prune_sparse", &prune_sparse, pybind11::arg("x"), pybind11::arg("thr"), pybind11::arg("thr_dev") = pybind11::none());
   m.def("prune_restore", &prune_restore);
-  m.def("prune_tiled", &prune_tiled);
+  m.def("prune_tiled", [](const Tensor& x, double thr, int64_t capacity) { return prune_tiled(x, thr, capacity); });
   m.def("prune_tiled_restore", [](const Tensor& w, const Tensor& d, std::vector<int64_t> shape, const OptTensor& out) {
     return prune_tiled_restore(w, d, shape, out); });
   m.def("silu_forward", &silu_forward);

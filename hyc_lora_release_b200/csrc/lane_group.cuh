@@ -193,10 +193,10 @@ __device__ __forceinline__ void lane_run_to_shared_async(const __nv_bfloat16* __
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void lane_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-// shared -> global
+// shared -> global; owners: the lanes whose groups are written
 template <typename MAP = LaneMapWhole>
 __device__ __forceinline__ void lane_shared_to_run(const uint32_t* slots, __nv_bfloat16* __restrict__ run, int n_pieces, int lane,
-                                                   const MAP& map = MAP(32)) {
+                                                   const MAP& map = MAP(32), uint32_t owners = 0xffffffffu) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int p = 32 * i + lane;
@@ -206,7 +206,7 @@ __device__ __forceinline__ void lane_shared_to_run(const uint32_t* slots, __nv_b
     const uint4 t0 = *reinterpret_cast<const uint4*>(src + park_chunk(c0, owner));
     const uint4 t1 = *reinterpret_cast<const uint4*>(src + park_chunk(c0 + 1, owner));
     const uint32_t t[8] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
-    if (p < n_pieces) st_stream_v8(run + 16 * p, t);
+    if (p < n_pieces && ((owners >> owner) & 1u)) st_stream_v8(run + 16 * p, t);
   }
 }
 // the lane's own slot <-> registers

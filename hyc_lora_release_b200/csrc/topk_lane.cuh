@@ -21,6 +21,13 @@ inline bool topk_lane_ok(int S, int k) {
   return (int64_t)rows_per_warp * k <= kLaneStageEntries;
 }
 
+// square maps whose rows end early: the lists of two rows per segment have to fit
+inline bool topk_lane_cols_ok(int M, int k) {
+  return k >= 0 && k <= M && topk_lane_ok(M, k) && 2 * (32 / topk_lanes_per_row(M)) * (int64_t)k <= kLaneStageEntries;
+}
+int topk_lane_compress_cols(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val_out, uint16_t* col_out,
+                            void* q_out, void* scale_out, int8_t* zp_out, int q_bit, cudaStream_t st);
+
 // both return 0 or a negative HYC_ERR_* (arguments already validated by the caller)
 int topk_lane_compress(const void* a, int64_t rows, int S, int k, void* val_out, uint16_t* col_out,
                        void* q_out, void* scale_out, int8_t* zp_out, int q_bit, cudaStream_t st);
@@ -30,9 +37,10 @@ int topk_lane_softmax_compress(const void* scores, float scale, const void* mask
                                int M, int64_t rows, int S, int k, void* dense, void* val_out, uint16_t* col_out,
                                void* q_out, void* scale_out, int8_t* zp_out, int q_bit, cudaStream_t st);
 // grad_or_null != NULL: a_out receives bf16(softmax_backward(restored map, grad) * out_scale) instead of the
-// restored map (out_scale == 1: no second operation)
+// restored map (out_scale == 1: no second operation); row_cols (only without a gradient): row r is written up to column
+// row_cols[r]
 int topk_lane_restore(const void* val, const uint16_t* col, int k, const void* q, const void* scale,
-                      const int8_t* zp, int64_t rows, int S, const void* grad_or_null, float out_scale, void* a_out,
+                      const int8_t* zp, int64_t rows, int S, const uint16_t* row_cols, const void* grad_or_null, float out_scale, void* a_out,
                       int q_bit, cudaStream_t st);
 
 // softmax backward on dense maps in the same layout; false = shape or alignment not covered, nothing launched

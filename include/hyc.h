@@ -140,6 +140,14 @@ int hyc_softmax_prune_tiled(const void* a, int64_t numel, float threshold,
 int hyc_softmax_prune_tiled_restore(const uint32_t* words, int64_t capacity, const void* directory,
                                     void* a_out, int64_t numel, void* stream);
 
+/* Both for square maps [rows / M][M][M] (M a multiple of 256, numel = rows * M) whose rows end early: row r has row_cols[r]
+ * (device uint16, a multiple of 8) columns that may hold something, the rest is zero.  The save does not read the rest and
+ * stores what hyc_softmax_prune_tiled stores; the restore does not write it. */
+int hyc_softmax_prune_tiled_cols(const void* a, int64_t numel, int M, const uint16_t* row_cols, float threshold,
+                                 uint32_t* words_out, int64_t capacity, void* directory_out, int64_t* nnz_out, void* stream);
+int hyc_softmax_prune_tiled_restore_cols(const uint32_t* words, int64_t capacity, const void* directory, int M, const uint16_t* row_cols,
+                                         void* a_out, int64_t numel, void* stream);
+
 /* hyc_softmax_prune_count / _fill with the threshold read from device memory (fp32, rounded to bf16 like the other form): a
  * calibrated threshold that lives on the device needs no copy to the host first. */
 int hyc_softmax_prune_count_dev(const void* a, int64_t numel, const float* threshold, void* workspace, size_t workspace_bytes, void* stream);
@@ -170,6 +178,14 @@ int hyc_softmax_prune_static(const void* a, int64_t numel, float threshold,
 int hyc_softmax_topk_compress(const void* a, int64_t rows, int S, int k,
                               void* val_out, uint16_t* col_out,
                               void* q_out, void* scale_out, int8_t* zp_out, int q_bit, void* stream);
+/* The same for square maps [rows / M][M][M] whose rows end early: row r has row_cols[r] (device uint16, a multiple of 64)
+ * columns that may hold something, the rest is zero and is neither read nor (restore) written.  The stored bytes are those of
+ * hyc_softmax_topk_compress.  Covered where hyc_softmax_topk_cols_supported says 1; HYC_ERR_UNSUPPORTED elsewhere. */
+int hyc_softmax_topk_cols_supported(int M, int k);
+int hyc_softmax_topk_compress_cols(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val_out, uint16_t* col_out,
+                                   void* q_out, void* scale_out, int8_t* zp_out, int q_bit, void* stream);
+int hyc_softmax_topk_restore_cols(const void* val, const uint16_t* col, int k, const void* q, const void* scale, const int8_t* zp,
+                                  int64_t rows, int M, const uint16_t* row_cols, void* a_out, int q_bit, void* stream);
 /* The forward side of the attention map in ONE pass: s = q k^T / sqrt(d) is already computed (library batched GEMM);
  * this call does  a = softmax(bf16(bf16(s * scale) + mask))  (fused_llama_layer_intra_inter_full_fuse.py:152-167, the
  * three tensor operations of the layer with their bf16 rounding points), writes the dense probabilities to a_out
@@ -425,6 +441,12 @@ int hyc_attn_fwd_tcgen05(const void* q, const void* k, const void* v, int B, int
                          const void* mask_or_null, int64_t mask_b, int64_t mask_h, int64_t mask_row,
                          const void* cls_or_null, int64_t cls_b, int64_t cls_h, void* map_or_null, void* o,
                          const void* o_scale_or_null, void* o_codes_or_null, int q_bit, int* status, void* stream);
+/* The same; row_cols [B * heads * M] (optional) receives for every row of the map the number of its leading columns that were
+ * written: a multiple of 128 or M.  What lies behind them is zero and is not written: for consumers that take row_cols. */
+int hyc_attn_fwd_cols_tcgen05(const void* q, const void* k, const void* v, int B, int M, int heads, int kv_heads, int head_dim, float scale,
+                              const void* mask_or_null, int64_t mask_b, int64_t mask_h, int64_t mask_row,
+                              const void* cls_or_null, int64_t cls_b, int64_t cls_h, void* map_or_null, uint16_t* row_cols_or_null, void* o,
+                              const void* o_scale_or_null, void* o_codes_or_null, int q_bit, int* status, void* stream);
 int hyc_attn_bwd_tcgen05(const void* q, const void* k, const void* v, const void* grad_o, const void* map, void* grad_s,
                          int B, int M, int heads, int kv_heads, int head_dim, float scale,
                          const void* cls_or_null, int64_t cls_b, int64_t cls_h, void* grad_q, void* grad_k, void* grad_v,

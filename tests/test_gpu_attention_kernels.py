@@ -120,3 +120,30 @@ def test_rows_without_a_passing_or_a_finite_entry(case):
     ref = torch.softmax(t.float(), -1)
     assert torch.equal(a.isnan(), ref.isnan())
     assert _rel(a.nan_to_num(), ref.nan_to_num()) < 2 ** -8
+
+
+@pytest.mark.parametrize("B,M,h,kv,kind", [(1, 8, 1, 1, None), (2, 136, 4, 2, "causal"), (1, 264, 2, 1, "padded"), (1, 1096, 2, 2, "causal")])
+def test_map_up_to_the_columns_that_are_reported(B, M, h, kv, kind):
+    """With row_cols the map is the same up to those columns, nothing is written behind them and zeros would have been."""
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(M)
+    d, scale = 128, 128 ** -0.5
+    rn = lambda *s: torch.randn(*s, generator=g).to(BF16).to(DEV)
+    qx, kx, vx = rn(B, M, h * d), rn(B, M, kv * d), rn(B, M, kv * d)
+    mask, st = _mask(kind, g, B, h, M), torch.zeros(1, dtype=torch.int32, device=DEV)
+    cls, cb, strides = None, 0, (0, 0, 0)
+    if mask is not None:
+        nb = mask.shape[0]
+        cb, strides = 0 if nb == 1 else 1, (0 if nb == 1 else mask.stride(0), 0, mask.stride(2))
+        cls = torch.empty(lib.hyc_attn_mask_class_bytes(nb, 1, M), dtype=torch.uint8, device=DEV)
+        check(lib.hyc_attn_mask_class(ptr(mask), *strides, nb, 1, M, ptr(cls), stream_of(qx)), "class")
+    maps, outs = [torch.full((B, h, M, M), -1.0, dtype=BF16, device=DEV) for _ in range(2)], [torch.empty_like(qx) for _ in range(2)]
+    cols = torch.empty(B * h * M, dtype=torch.int16, device=DEV)
+    fwd = (ptr(qx), ptr(kx), ptr(vx), B, M, h, kv, d, scale, ptr(mask), *strides, ptr(cls), cb, 0)
+    check(lib.hyc_attn_fwd_tcgen05(*fwd, ptr(maps[0]), ptr(outs[0]), None, None, 4, ptr(st), stream_of(qx)), "fwd")
+    check(lib.hyc_attn_fwd_cols_tcgen05(*fwd, ptr(maps[1]), ptr(cols), ptr(outs[1]), None, None, 4, ptr(st), stream_of(qx)), "fwd")
+    inside = (torch.arange(M, device=DEV)[None] < cols[:, None]).view(B, h, M, M)
+    assert int(st.item()) == 0 and torch.equal(*outs)
+    assert torch.equal(maps[0][inside], maps[1][inside]) and bool((maps[0][~inside] == 0).all()) and bool((maps[1][~inside] == -1).all())
+    if kind == "causal":
+        assert torch.equal(cols.view(B * h, M)[0], ((torch.arange(M) // 128 + 1) * 128).clamp(max=M).to(torch.int16).to(DEV))

@@ -1,0 +1,97 @@
+"""Probability maps whose rows end early: the save and restore kernels that do not touch what lies behind the rows' ends,
+against the whole-row kernels on the same map with zeros there."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _map(maps, M, kind, seed):
+    """-> (map with NaN behind the rows' ends, the same with zeros there, row_cols)"""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    unit = 128 if M > 64 else 64
+    r = torch.arange(M, device="cuda")
+    if kind == "causal":
+        cols = ((r // unit + 1) * unit).clamp(max=M).repeat(maps)
+    elif kind == "whole":
+        cols = torch.full((maps * M,), M, device="cuda")
+    else:      # any multiple of 64 (M itself among them), none as well
+        cols = (torch.randint(0, M // 64 + 2, (maps * M,), generator=g, device="cuda") * 64).clamp(max=M)
+    a = torch.softmax(3 * torch.randn(maps * M, M, generator=g, device="cuda"), -1).to(torch.bfloat16)
+    behind = torch.arange(M, device="cuda")[None] >= cols[:, None]
+    return a.masked_fill(behind, float("nan")), a.masked_fill(behind, 0.0), cols.to(torch.int16), behind
+
+
+def _call(name, *args):
+    from hyc_lora_release_b200._lib import lib, check, stream_of
+    args = [ctypes.c_void_p(x.data_ptr()) if isinstance(x, torch.Tensor) else x for x in args]
+    check(getattr(lib, name)(*args, stream_of(torch.empty(0, device="cuda"))), name)
+
+
+def _topk_buffers(rows, M, k, q):
+    e = lambda *s, dt: torch.empty(*s, dtype=dt, device="cuda")
+    return [e(rows, k, dt=torch.bfloat16), e(rows, k, dt=torch.int16), e(rows, M * q // 8, dt=torch.uint8), e(rows, M // 64, dt=torch.bfloat16),
+            e(rows, M // 64, dt=torch.int8)]
+
+
+@pytest.mark.parametrize("kind", ["causal", "whole", "any"])
+@pytest.mark.parametrize("M,k,q", [(64, 3, 4), (128, 6, 2), (192, 9, 4), (192, 10, 8), (448, 22, 4), (704, 35, 4), (704, 0, 2), (1024, 51, 4),
+                                   (1984, 99, 2), (2048, 102, 4), (2048, 128, 8)])
+def test_topk_rows_that_end_early(M, k, q, kind):
+    from hyc_lora_release_b200._lib import lib
+    assert lib.hyc_softmax_topk_cols_supported(M, k) == 1
+    maps = 3
+    a, dense, cols, behind = _map(maps, M, kind, M + k)
+    rows = maps * M
+    whole, early = _topk_buffers(rows, M, k, q), _topk_buffers(rows, M, k, q)
+    _call("hyc_softmax_topk_compress", dense, rows, M, k, *whole, q)
+    _call("hyc_softmax_topk_compress_cols", a, rows, M, cols, k, *early, q)
+    for w, e in zip(whole, early):
+        assert torch.equal(w.view(torch.uint8), e.view(torch.uint8))
+    val, col, codes, scale, zp = whole
+    full = torch.empty(rows, M, dtype=torch.bfloat16, device="cuda")
+    _call("hyc_softmax_topk_restore", val, col, k, codes, scale, zp, rows, M, full, q)
+    out = torch.full_like(full, -7.0)
+    _call("hyc_softmax_topk_restore_cols", val, col, k, codes, scale, zp, rows, M, cols, out, q)
+    assert torch.equal(out, full.masked_fill(behind, -7.0))
+
+
+def test_topk_lists_that_do_not_fit_are_refused():
+    from hyc_lora_release_b200._lib import lib
+    assert lib.hyc_softmax_topk_cols_supported(2048, 129) == 0      # two lists of a warp need 258 staged entries
+    assert lib.hyc_softmax_topk_cols_supported(4096, 10) == 0 and lib.hyc_softmax_topk_cols_supported(96, 4) == 0
+
+
+@pytest.mark.parametrize("kind", ["causal", "whole", "any"])
+@pytest.mark.parametrize("M,maps,thr", [(256, 3, 0.01), (768, 2, 0.004), (1024, 2, 0.003), (2048, 1, 0.002), (4096, 1, 0.001), (256, 2, -1.0)])
+def test_pruned_rows_that_end_early(M, maps, thr, kind):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    numel = maps * M * M
+    r = torch.arange(M, device="cuda")
+    if kind == "causal":
+        cols = ((r // 128 + 1) * 128).clamp(max=M).repeat(maps)
+    elif kind == "whole":
+        cols = torch.full((maps * M,), M, device="cuda")
+    else:
+        cols = torch.randint(0, M // 8 + 1, (maps * M,), generator=g, device="cuda") * 8
+    a = torch.softmax(3 * torch.randn(maps * M, M, generator=g, device="cuda"), -1).to(torch.bfloat16)
+    behind = torch.arange(M, device="cuda")[None] >= cols[:, None]
+    dense = a.masked_fill(behind, 0.0)
+    a = a.masked_fill(behind, float("inf"))
+    cols = cols.to(torch.int16)
+    from hyc_lora_release_b200._lib import lib
+    words = torch.empty(2 * numel, dtype=torch.int32, device="cuda")
+    directory = torch.empty(lib.hyc_softmax_prune_tiled_directory_bytes(numel) // 4, dtype=torch.int32, device="cuda")
+    nnz = torch.empty(1, dtype=torch.int64, device="cuda")
+    _call("hyc_softmax_prune_tiled_cols", a, numel, M, cols, thr, words, words.numel(), directory, nnz)
+    want = torch.where((dense > torch.tensor(thr, dtype=torch.bfloat16)) & (dense != 0), dense, torch.zeros_like(dense))
+    assert int(nnz) == int((want != 0).sum())
+    out = torch.full_like(dense, -7.0)
+    _call("hyc_softmax_prune_tiled_restore_cols", words, words.numel(), directory, M, cols, out, numel)
+    assert torch.equal(out, want.masked_fill(behind, -7.0))
+    _call("hyc_softmax_prune_tiled_restore", words, words.numel(), directory, out, numel)
+    assert torch.equal(out, want)
+    assert lib.hyc_softmax_prune_tiled_restore_cols(None, 0, ctypes.c_void_p(directory.data_ptr()), M - 8, ctypes.c_void_p(cols.data_ptr()),
+                                                    ctypes.c_void_p(out.data_ptr()), numel, None) == -3
