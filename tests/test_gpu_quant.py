@@ -242,3 +242,30 @@ def test_topk_backward_into_any_buffer():
         assert torch.equal(m.softmax_backward(g, out=out).to(torch.bfloat16), want) and torch.equal(out.to(torch.bfloat16), want)
     with pytest.raises(RuntimeError):
         m.softmax_backward(g, out=flat[:, :1, :8])
+
+
+@pytest.mark.parametrize("q", QS)
+@pytest.mark.parametrize("rows,N,k", [(1, 32, 0), (3, 96, 5), (37, 4096, 41), (5, 14336, 143)])
+def test_rebuild_into_rows_of_any_alignment(q, rows, N, k):
+    """Rows that start on 32-byte boundaries leave in wider stores than rows that only keep the 16 bytes that are asked for (an
+    offset of 8 columns, a row stride of 8 more than N): the same values either way, and nothing beside the rows is touched."""
+    import ctypes
+    from hyc_lora_release_b200._lib import check, lib, stream_of
+    g = torch.Generator().manual_seed(N + q)
+    codes = torch.randint(0, 256, (rows, N * q // 8), dtype=torch.uint8, generator=g)
+    s = (torch.rand(1, N, generator=g) + 0.5).to(torch.bfloat16)
+    idx = torch.randperm(N, generator=g)[:k]
+    xo = torch.randn(rows, k, generator=g).to(torch.bfloat16)
+    want = oracle.ref_decompress(codes[None], s, q)[0].to(torch.bfloat16)
+    want[:, idx] = xo
+    d = [t.to(DEV) for t in (codes, s, idx, xo)]
+    p = [ctypes.c_void_p(t.data_ptr()) for t in d]
+    for offset, ld in ((0, N), (16, N + 16), (8, N), (0, N + 8), (8, N + 24)):
+        if q == 2 and (offset % 16 or ld % 16):      # (2-bit rows are asked to start on 32-byte boundaries)
+            continue
+        buf = torch.full((offset + rows * ld + 32,), -3.0, dtype=torch.bfloat16, device=DEV)
+        check(lib.hyc_unpack_dequant(p[0], rows, N, p[1], None, p[2] if k else None, k, p[3] if k else None,
+                                     ctypes.c_void_p(buf.data_ptr() + 2 * offset), ld, q, stream_of(buf)), "hyc_unpack_dequant")
+        got = buf[offset:offset + rows * ld].view(rows, ld).cpu()
+        assert torch.equal(got[:, :N], want)
+        assert (got[:, N:] == -3.0).all() and (buf[:offset] == -3.0).all() and (buf[offset + rows * ld:] == -3.0).all()
