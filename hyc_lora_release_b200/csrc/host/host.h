@@ -40,9 +40,11 @@ struct SameDevice {
 void check_q(int64_t q);
 inline const Tensor* opt(const OptTensor& t) { return t.has_value() && t->defined() ? &*t : nullptr; }
 inline bool given(const OptTensor& t) { return t.has_value() && t->defined(); }
-inline Tensor bf16c(const Tensor& t) { return t.to(at::kBFloat16).contiguous(); }
+// (what is there already is returned without a trip through the dispatcher, which costs more than half a launch)
+inline Tensor bf16c(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? t.contiguous() : t.to(at::kBFloat16).contiguous(); }
+// a per-channel vector as the kernels read it: contiguous bf16, of any shape
 inline Tensor vec(const Tensor& s) {
-  if (s.dim() == 1 && s.scalar_type() == at::kBFloat16 && s.is_contiguous()) return s;
+  if (s.scalar_type() == at::kBFloat16 && s.is_contiguous()) return s;
   return s.to(at::kBFloat16).reshape({-1}).contiguous();
 }
 inline Tensor empty(at::IntArrayRef sz, const Tensor& like, at::ScalarType ty = at::kBFloat16) {

@@ -41,7 +41,7 @@ static Tensor rows_view(const Tensor& x_in) {
   Tensor x = x_in;
   if (x.dim() == 4) x = x.transpose(1, 2).reshape({x.size(0), x.size(2), -1});
   TORCH_CHECK_VALUE(x.dim() == 3, "expected a [B, M, N] or [B, heads, M, d] tensor, got shape ", x_in.sizes());
-  x = x.to(at::kBFloat16);
+  if (x.scalar_type() != at::kBFloat16) x = x.to(at::kBFloat16);
   const int64_t M = x.size(1), N = x.size(2);
   if (x.stride(2) != 1 || (x.size(0) > 1 && x.stride(0) != M * x.stride(1)) || x.stride(1) < N || x.stride(1) % 8 != 0 ||
       reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0)
@@ -58,6 +58,7 @@ static const Tensor& buffer(const Tensor& t, at::IntArrayRef shape, at::ScalarTy
 }
 
 static Tensor index_of(const Tensor& channel, const Tensor& like) {
+  if (channel.scalar_type() == at::kLong && channel.device() == like.device()) return channel.contiguous();
   return channel.to(like.device(), at::kLong).contiguous();
 }
 
@@ -71,7 +72,7 @@ std::tuple<Tensor, OptTensor> quant(const Tensor& x_in, const Tensor& s_in, int6
   TORCH_CHECK_VALUE(N % 32 == 0, "the hidden size must be a multiple of 32");
   const Tensor s = scale_vec(s_in, N);
   Tensor zt, idx;
-  if (given(z)) zt = z->reshape({-1}).to(at::kChar).contiguous();
+  if (given(z)) zt = z->scalar_type() == at::kChar && z->is_contiguous() ? *z : z->reshape({-1}).to(at::kChar).contiguous();
   int64_t k = 0;
   if (given(channel)) { idx = index_of(*channel, x); k = idx.numel(); }
   Tensor q = given(out_q) ? buffer(*out_q, {B, M, N * q_bit / 8}, at::kByte, x, "codes") : empty({B, M, N * q_bit / 8}, x, at::kByte);
@@ -96,7 +97,7 @@ Tensor dequant(const Tensor& q_in, const Tensor& s_in, int64_t q_bit, const OptT
   const int64_t B = q_in.size(0), M = q_in.size(1), N = s_in.size(-1);
   const Tensor q = q_in.contiguous(), s = scale_vec(s_in, N);
   Tensor zt, idx, xo;
-  if (given(z)) zt = z->reshape({-1}).to(at::kChar).contiguous();
+  if (given(z)) zt = z->scalar_type() == at::kChar && z->is_contiguous() ? *z : z->reshape({-1}).to(at::kChar).contiguous();
   Tensor x = given(out) ? buffer(*out, {B, M, N}, at::kBFloat16, q, "out") : empty({B, M, N}, q);
   if (B * M == 0) return x;
   int64_t k = 0;
@@ -318,7 +319,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor&
   std::vector<int64_t> qs(xc.sizes().begin(), xc.sizes().end()), os = qs;
   qs.back() = N * q_bit / 8;
   os.back() = k;
-  Tensor y = at::empty_like(xc), rstd = empty({rows}, x, at::kFloat), qx = empty(qs, x, at::kByte), xo = empty(os, x);
+  Tensor y = empty(xc.sizes(), x), rstd = empty({rows}, x, at::kFloat), qx = empty(qs, x, at::kByte), xo = empty(os, x);
   OptTensor qy;
   if (sy.defined()) qy = empty(qs, x, at::kByte);
   if (rows)
@@ -340,7 +341,7 @@ Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor&
   if (given(idx_in)) { idx = index_of(*idx_in, dy); k = idx.numel(); }
   if (k) xo = bf16c(*xo_in);
   if (given(res_in)) res = bf16c(*res_in);
-  Tensor dx = at::empty_like(dyc);
+  Tensor dx = empty(dyc.sizes(), dyc);
   if (rows)
     check(hyc_rmsnorm_bwd_packed(data(dyc), data(q), data(sx), k ? (const int64_t*)data(idx) : nullptr, (int)k, data(xo), data(w),
                                  (const float*)data(rs), data(res), data(dx), rows, (int)N, (int)q_bit, on.stream), "hyc_rmsnorm_bwd_packed");
