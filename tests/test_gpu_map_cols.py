@@ -95,3 +95,22 @@ def test_pruned_rows_that_end_early(M, maps, thr, kind):
     assert torch.equal(out, want)
     assert lib.hyc_softmax_prune_tiled_restore_cols(None, 0, ctypes.c_void_p(directory.data_ptr()), M - 8, ctypes.c_void_p(cols.data_ptr()),
                                                     ctypes.c_void_p(out.data_ptr()), numel, None) == -3
+
+
+@pytest.mark.parametrize("thr", [0.25, -1.0])
+@pytest.mark.parametrize("numel", [8, 1024, 4096 + 8, 3 * 4096 + 1000])
+def test_ordered_list_at_any_density(numel, thr):
+    """The ordered fill packs four trips of a warp at once: none, one entry per lane, whole lanes, everything, and ends."""
+    from hyc_lora_release_b200._lib import lib
+    i = torch.arange(numel, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(numel)
+    for keep in (i < 0, i % 8 == 7, i // 8 % 32 == 5, i >= 0, i // 256 % 4 == 2, torch.rand(numel, generator=g, device="cuda") < 0.3):
+        # (what is dropped is a zero or, where the threshold allows it, below it)
+        a = torch.where(keep, 0.5 + (i % 61).float() / 128, torch.where(i % 2 == 0, 0.0, -2.0)).to(torch.bfloat16)
+        ws = torch.empty(lib.hyc_softmax_prune_workspace_bytes(numel) // 8 + 1, dtype=torch.int64, device="cuda")
+        _call("hyc_softmax_prune_count", a, numel, thr, ws, ws.numel() * 8)
+        n = int(ws[0])
+        idx, val = torch.empty(max(n, 1), dtype=torch.int64, device="cuda"), torch.empty(max(n, 1), dtype=torch.bfloat16, device="cuda")
+        _call("hyc_softmax_prune_fill", a, numel, thr, ws, idx, val, n)
+        want = keep.nonzero().flatten()
+        assert n == want.numel() and torch.equal(idx[:n], want) and torch.equal(val[:n], a[want])
