@@ -91,3 +91,26 @@ def test_nf4_weights_in_one_launch(parts):
     check(lib.hyc_dequant_nf4_many(len(parts), jobs, stream_of(keep[0][0])), "hyc_dequant_nf4_many")
     for t, w in zip(keep, want):
         assert torch.equal(t[3].cpu(), w)
+
+
+@pytest.mark.parametrize("nested", [False, True])
+@pytest.mark.parametrize("blocksize,packed_off,out_off", [(64, 0, 0), (64, 4, 0), (64, 0, 8), (48, 8, 16), (16, 0, 0), (8, 0, 0), (4096, 8, 16)])
+def test_nf4_lanes_of_sixteen_and_of_eight(blocksize, packed_off, out_off, nested):
+    """16 elements per lane where they share a scale and the tensors start on 8 and 32 bytes, eight elsewhere: the same values."""
+    from hyc_lora_release_b200._lib import check, lib, stream_of
+    g = torch.Generator().manual_seed(blocksize + packed_off)
+    w = (torch.randn(3, 1024 * 5 + 62, generator=g) * 0.03).to(BF16)
+    packed, qs = onf4.quantize_4bit(w, onf4.normal_float_table(), blocksize=blocksize, nested=nested, blocksize2=32)
+    want = onf4.ref_dequantize_4bit(packed, qs).flatten()
+    n = want.numel()
+    p = torch.zeros(packed.numel() + 16, dtype=torch.uint8, device=DEV)
+    p[packed_off:packed_off + packed.numel()] = packed.flatten().to(DEV)
+    out = torch.full((n + 48,), -3.0, dtype=BF16, device=DEV)
+    t = [qs.code.to(DEV), qs.absmax.to(DEV)] + ([qs.state2.code.to(DEV), qs.state2.absmax.to(DEV)] if nested else [])
+    v = lambda x: ctypes.c_void_p(x.data_ptr())
+    check(lib.hyc_dequant_nf4(ctypes.c_void_p(p.data_ptr() + packed_off), v(t[0]), None if nested else v(t[1]), v(t[1]) if nested else None,
+                              v(t[2]) if nested else None, v(t[3]) if nested else None, 32, float(qs.offset) if nested else 0.0, n, blocksize,
+                              ctypes.c_void_p(out.data_ptr() + 2 * out_off), stream_of(out)), "hyc_dequant_nf4")
+    got = out.cpu()
+    assert torch.equal(got[out_off:out_off + n], want)
+    assert (got[:out_off] == -3.0).all() and (got[out_off + n:] == -3.0).all()
