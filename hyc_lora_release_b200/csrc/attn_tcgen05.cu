@@ -236,11 +236,11 @@ __device__ __forceinline__ uint32_t at_setup(const AttnParams& p, const Bars& ba
     *bar.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();      // before tensor memory is taken: see launch_pdl
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(bar.tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();
   if (warp == 2 && lane < p.tiles) bar.cls[lane] = (uint8_t)(fixed_is_q ? class_of(p, b, h, fixed, lane) : class_of(p, b, h, lane, fixed));
   tc_fence_before();
   __syncthreads();

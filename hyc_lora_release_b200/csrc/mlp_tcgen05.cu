@@ -104,6 +104,7 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();      // before tensor memory is taken: see launch_pdl
   if (warp == 1) {
     if (PAIR) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
@@ -117,7 +118,6 @@ mlp_gemm_kernel(const __grid_constant__ Maps maps, const Params p) {
   __syncthreads();
   if (PAIR) cluster_sync_all();      // the peer's barriers are initialised before anything is signalled there
   tc_fence_after();
-  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {

@@ -93,6 +93,7 @@ skinny_kernel(const __grid_constant__ Args a) {
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();      // before tensor memory is taken: see launch_pdl
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -100,7 +101,6 @@ skinny_kernel(const __grid_constant__ Args a) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_wait();
   const uint32_t tmem = *tmem_slot;
   const uint32_t ring = smem_u32(smem), aux = ring + AUX_AT;
   // xa blocks first, then W blocks [column tile][w]; accumulators: Y [row tile][w], then Z [column tile]

@@ -84,6 +84,7 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();      // before tensor memory is taken: see launch_pdl
   if (warp == 1) {
     if (PAIR) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(SBN) : "memory");
@@ -97,7 +98,6 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
   __syncthreads();
   if (PAIR) cluster_sync_all();      // the peer's barriers exist before anything is signalled there
   tc_fence_after();
-  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   const int et = (int)threadIdx.x - 64, quad = warp & 3;

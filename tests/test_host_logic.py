@@ -1,4 +1,7 @@
 """Host-side logic that needs no device: the calibration running mean, checks before any launch."""
+import pathlib
+import re
+
 import pytest
 import torch
 
@@ -29,6 +32,20 @@ def test_rows_of_no_columns_are_an_error():
                  lambda: rn.rmsnorm_backward_packed(none, one, one, None, None, one, one, 4)):
         with pytest.raises(ValueError, match="empty"):
             call()
+
+
+def test_tensor_memory_is_taken_after_the_wait():
+    """A kernel that may start before the one in front of it has ended takes no tensor memory until that one has: the kernel in
+    front may still want some, and would wait for good.  Read from the sources, since a failure would hang the GPU."""
+    csrc = pathlib.Path(__file__).resolve().parent.parent / "hyc_lora_release_b200" / "csrc"
+    seen = 0
+    for path in sorted(csrc.glob("*.cu*")):
+        text = path.read_text()
+        for at in [m.start() for m in re.finditer(r"tcgen05\.alloc", text)]:
+            function = max(text.rfind("\n" + word, 0, at) for word in ("__global__", "__device__", "template", "static", "inline"))
+            assert re.search(r"^ *pdl_wait\(\);", text[function:at], re.M), f"{path.name}: tensor memory before pdl_wait()"
+            seen += 1
+    assert seen >= 4
 
 
 @pytest.mark.gpu
