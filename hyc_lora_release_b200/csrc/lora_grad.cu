@@ -213,7 +213,14 @@ lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restric
       const float4 v = splits > 1 ? ld_cluster_v4(&part[r][h], (uint32_t)k) : *reinterpret_cast<const float4*>(&part[r][h]);
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    *reinterpret_cast<uint2*>(out + (int64_t)r * H + h0 + h) = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
+    const uint2 w = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
+    __nv_bfloat16* at = out + (int64_t)r * H + h0 + h;
+    if (aligned(out, 8)) {
+      *reinterpret_cast<uint2*>(at) = w;
+    } else {      // a gradient that starts anywhere in a caller's buffer
+      at[0] = __ushort_as_bfloat16((uint16_t)w.x); at[1] = __ushort_as_bfloat16((uint16_t)(w.x >> 16));
+      at[2] = __ushort_as_bfloat16((uint16_t)w.y); at[3] = __ushort_as_bfloat16((uint16_t)(w.y >> 16));
+    }
   }
   if (splits > 1) cluster_barrier();      // nobody leaves while its partials may be read
 }

@@ -131,6 +131,24 @@ def test_lora_grad_a_shares_of_the_tokens(mlp, q, T, R2):
     assert not out[:, 3].isfinite().any() and close(out[:, keep], ref[:, keep], rel=4e-3)
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3, 4])
+@pytest.mark.parametrize("q,T", [(2, 40), (4, 300), (8, 7)])
+def test_lora_grad_a_into_a_buffer_of_any_alignment(mlp, q, T, offset):
+    """A gradient may start at any element of a caller's buffer: the same bits, and nothing beside it is touched."""
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(T)
+    H, R2 = 256, 32
+    codes = torch.randint(0, 256, (T, H * q // 8), generator=g).to(torch.uint8).to(DEV)
+    s, gm = (torch.rand(H, generator=g) + 0.01).to(BF16).to(DEV), _randn(g, T, R2).to(DEV)
+    want = mlp.lora_grad_a(codes, s, gm, R2, q).flatten()
+    buf = torch.full((want.numel() + 16,), -3.0, dtype=BF16, device=DEV)
+    ws = torch.empty(max(16, lib.hyc_lora_grad_a_workspace_bytes(T, H, R2)), dtype=torch.uint8, device=DEV)
+    check(lib.hyc_lora_grad_a_dequant(ptr(codes), ptr(s), ptr(gm), R2, R2, T, H, q, ptr(buf[offset:]), ptr(ws), ws.numel(), stream_of(buf)),
+          "hyc_lora_grad_a_dequant")
+    assert torch.equal(buf[offset:offset + want.numel()], want)
+    assert bool((buf[:offset] == -3.0).all()) and bool((buf[offset + want.numel():] == -3.0).all())
+
+
 def _mlp_problem(g, B, M, H, I, R=16):
     x = _randn(g, B, M, H)
     x[:, :, torch.randperm(H, generator=g)[: max(1, H // 200)]] *= 20
