@@ -337,17 +337,18 @@ topk_lane_compress_cols_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows
     const uint32_t seg = item * RPW + rw;
     const bool valid = seg < n_items;
     uint32_t rowa = 0u, rowb = NONE;
-    int ga = 0, gb = 0, la = 0, lb = 0;                     // groups the row takes up here, groups it has in memory
+    // groups the row takes up here, groups it has in memory (its lanes write a row of GPR groups: a row_cols above M must not count)
+    int ga = 0, gb = 0, la = 0, lb = 0;
     if (valid) {
       const uint32_t map = seg / (uint32_t)sm.items;
       int ra, rb;
       paired_rows((int)(seg - map * (uint32_t)sm.items), sm.M, ra, rb);
       rowa = map * (uint32_t)sm.M + (uint32_t)ra;
-      la = (int)__ldg(row_cols + rowa) / 64;
+      la = min((int)__ldg(row_cols + rowa) / 64, GPR);
       ga = max(la, kg);
       if (rb >= 0) {
         rowb = map * (uint32_t)sm.M + (uint32_t)rb;
-        lb = (int)__ldg(row_cols + rowb) / 64;
+        lb = min((int)__ldg(row_cols + rowb) / 64, GPR);
         gb = max(lb, kg);
       }
     }

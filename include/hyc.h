@@ -141,7 +141,7 @@ int hyc_softmax_prune_tiled_restore(const uint32_t* words, int64_t capacity, con
                                     void* a_out, int64_t numel, void* stream);
 
 /* Both for square maps [rows / M][M][M] (M a multiple of 256, numel = rows * M) whose rows end early: row r has row_cols[r]
- * (device uint16, a multiple of 8) columns that may hold something, the rest is zero.  The save does not read the rest and
+ * (device uint16, a multiple of 8; M if above) columns that may hold something, the rest is zero.  The save does not read the rest and
  * stores what hyc_softmax_prune_tiled stores; the restore does not write it. */
 int hyc_softmax_prune_tiled_cols(const void* a, int64_t numel, int M, const uint16_t* row_cols, float threshold,
                                  uint32_t* words_out, int64_t capacity, void* directory_out, int64_t* nnz_out, void* stream);
@@ -178,8 +178,8 @@ int hyc_softmax_prune_static(const void* a, int64_t numel, float threshold,
 int hyc_softmax_topk_compress(const void* a, int64_t rows, int S, int k,
                               void* val_out, uint16_t* col_out,
                               void* q_out, void* scale_out, int8_t* zp_out, int q_bit, void* stream);
-/* The same for square maps [rows / M][M][M] whose rows end early: row r has row_cols[r] (device uint16, a multiple of 64)
- * columns that may hold something, the rest is zero and is neither read nor (restore) written.  The stored bytes are those of
+/* The same for square maps [rows / M][M][M] whose rows end early: row r has row_cols[r] (device uint16, a multiple of
+ * 64; M if above) columns that may hold something, the rest is zero and is neither read nor (restore) written.  The stored bytes are those of
  * hyc_softmax_topk_compress.  Covered where hyc_softmax_topk_cols_supported says 1; HYC_ERR_UNSUPPORTED elsewhere. */
 int hyc_softmax_topk_cols_supported(int M, int k);
 int hyc_softmax_topk_compress_cols(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val_out, uint16_t* col_out,

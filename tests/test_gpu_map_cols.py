@@ -58,6 +58,29 @@ def test_topk_rows_that_end_early(M, k, q, kind):
     assert torch.equal(out, full.masked_fill(behind, -7.0))
 
 
+@pytest.mark.parametrize("beyond", [64, 320, 65535 - 704])
+@pytest.mark.parametrize("M,q", [(192, 2), (704, 4), (1984, 8), (512, 4)])
+def test_row_ends_beyond_the_row_are_its_end(M, q, beyond):
+    """A reported end above M counts as M: no group behind the row is read or written, in the middle of the buffers or after them."""
+    maps, k = 2, 5
+    rows = maps * M
+    a, dense, cols, behind = _map(maps, M, "any", M)
+    too_far = torch.where(cols.int() == M, torch.minimum(cols.int() + beyond, torch.full_like(cols.int(), 65535)), cols.int()).to(torch.uint16)
+    assert bool((cols == M).any())
+    fill = lambda bufs: [t.view(torch.uint8).fill_(0xa5).view(t.dtype) for t in bufs]
+    exact, far = fill(_topk_buffers(rows, M, k, q)), fill(_topk_buffers(rows + 64, M, k, q))
+    _call("hyc_softmax_topk_compress_cols", a, rows, M, cols, k, *exact, q)
+    _call("hyc_softmax_topk_compress_cols", a, rows, M, too_far, k, *far, q)
+    for e, f in zip(exact, far):
+        e, f = e.flatten().view(torch.uint8), f.flatten().view(torch.uint8)
+        assert torch.equal(e, f[:e.numel()]) and bool((f[e.numel():] == 0xa5).all())
+    out = [torch.full((rows + 8, M), -7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    for o, c in zip(out, (cols, too_far)):
+        val, col, codes, scale, zp = exact
+        _call("hyc_softmax_topk_restore_cols", val, col, k, codes, scale, zp, rows, M, c, o, q)
+    assert torch.equal(*out) and bool((out[1][rows:] == -7.0).all())
+
+
 def test_topk_lists_that_do_not_fit_are_refused():
     from hyc_lora_release_b200._lib import lib
     assert lib.hyc_softmax_topk_cols_supported(2048, 129) == 0      # two lists of a warp need 258 staged entries
