@@ -109,7 +109,8 @@ Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64
   const int64_t T = q.size(0), H = scale.numel();
   Tensor out = empty({r2, H}, q);
   const size_t nbytes = hyc_lora_grad_a_workspace_bytes((int)T, (int)H, (int)r2);
-  Tensor ws = empty({(int64_t)(nbytes / 4)}, q, at::kFloat);
+  Tensor ws;
+  if (nbytes > 0) ws = empty({(int64_t)(nbytes / 4)}, q, at::kFloat);
   check(hyc_lora_grad_a_dequant(data(q), data(scale), data(gm), gm.stride(0), (int)r2, (int)T, (int)H, (int)q_bit, data(out), data(ws),
                                 nbytes, on.stream), "hyc_lora_grad_a_dequant");
   return out;

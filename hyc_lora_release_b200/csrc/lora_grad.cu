@@ -8,8 +8,8 @@
 // matching 32 x R tile of gm on the tensor cores (m16n8k16, fp32 accumulate; both operands are
 // read from shared memory with transposing ldmatrix).  x_hat never goes to HBM: the kernel reads
 // T*H*q/8 bytes of codes where the two-step version reads and writes 2*T*H bytes twice.
-// The up to eight token chunks of the same columns are a cluster: their fp32 partials meet in distributed shared memory and
-// are added up in the order of the chunks.  The codes and gm rows of the next kGaAhead steps are on their way while a step is
+// Up to eight token chunks of the same columns are a cluster: their fp32 partials meet in distributed shared memory and
+// are added up in the order of the chunks (narrow products of many tokens: several clusters, ga_shares).  The codes and gm rows of the next kGaAhead steps are on their way while a step is
 // worked on: the kernel waits for memory (issue slots 0.1 without that, every step a full round trip).
 // us, cold, with the second kernel that added the partials up before / now: 2048 tokens of 4096, 4 bits, one adapter 15.7 / 10.9,
 // three 22.4 / 14.1; 128 tokens, 8 bits, two adapters 11.6 / 7.5; 8192 tokens, 8 bits, two 35.5 / 28.9.
@@ -21,6 +21,7 @@ constexpr int kGaCols = 128;      // hidden columns per block
 constexpr int kGaStep = 32;       // tokens per step
 constexpr int kGaMaxSplits = 8;   // token chunks = blocks of a cluster
 constexpr int kGaAhead = 4;
+constexpr int kGaMinSteps = 16;   // several clusters: steps per block at least
 constexpr int kGaMaxR = 64;
 
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_ptr) {
@@ -102,11 +103,24 @@ __device__ __forceinline__ float4 ld_cluster_v4(const void* own, uint32_t rank) 
   return v;
 }
 
-// grid (hidden blocks, chunks), cluster (1, chunks).  RT = number of 16-row tiles of the LoRA dimension (R2 = 16 * RT)
+// four sums of a row of out, which may start at any element of a caller's buffer
+__device__ __forceinline__ void store_sums(__nv_bfloat16* __restrict__ out, int64_t i, float4 s) {
+  const uint2 w = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
+  if (aligned(out, 8)) {
+    *reinterpret_cast<uint2*>(out + i) = w;
+  } else {
+    out[i] = __ushort_as_bfloat16((uint16_t)w.x); out[i + 1] = __ushort_as_bfloat16((uint16_t)(w.x >> 16));
+    out[i + 2] = __ushort_as_bfloat16((uint16_t)w.y); out[i + 3] = __ushort_as_bfloat16((uint16_t)(w.y >> 16));
+  }
+}
+
+// grid (hidden blocks, chunks, clusters), cluster (1, chunks).  RT = number of 16-row tiles of the LoRA dimension (R2 = 16 * RT).
+// ws: null, or where each cluster of several leaves its sums, [cluster][R2][H]
 template <int QBIT, int RT>
 __global__ void __launch_bounds__(128)
 lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restrict__ scale,
-                   const __nv_bfloat16* __restrict__ gm, int64_t ldg, int T, int H, int chunk, __nv_bfloat16* __restrict__ out) {
+                   const __nv_bfloat16* __restrict__ gm, int64_t ldg, int T, int H, int chunk, __nv_bfloat16* __restrict__ out,
+                   float* __restrict__ ws) {
   pdl_wait();
   constexpr int R2 = 16 * RT, PIECES = kGaStep * (R2 / 8), PPT = (PIECES + 127) / 128;      // 16-byte pieces of a gm tile, per thread
   constexpr int X_LD = kGaCols + 8, G_LD = R2 + 8;
@@ -118,7 +132,7 @@ lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restric
   auto part = reinterpret_cast<float (*)[kGaCols + 4]>(s_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h0 = blockIdx.x * kGaCols;
-  const int t_begin = blockIdx.y * chunk;
+  const int t_begin = (blockIdx.z * gridDim.y + blockIdx.y) * chunk;
   const int t_end = min(T, t_begin + chunk);
   const int64_t qld = (int64_t)H * QBIT / 8;
 
@@ -213,16 +227,42 @@ lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restric
       const float4 v = splits > 1 ? ld_cluster_v4(&part[r][h], (uint32_t)k) : *reinterpret_cast<const float4*>(&part[r][h]);
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    const uint2 w = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
-    __nv_bfloat16* at = out + (int64_t)r * H + h0 + h;
-    if (aligned(out, 8)) {
-      *reinterpret_cast<uint2*>(at) = w;
-    } else {      // a gradient that starts anywhere in a caller's buffer
-      at[0] = __ushort_as_bfloat16((uint16_t)w.x); at[1] = __ushort_as_bfloat16((uint16_t)(w.x >> 16));
-      at[2] = __ushort_as_bfloat16((uint16_t)w.y); at[3] = __ushort_as_bfloat16((uint16_t)(w.y >> 16));
-    }
+    const int64_t i = (int64_t)r * H + h0 + h;
+    if (ws != nullptr) *reinterpret_cast<float4*>(ws + (int64_t)blockIdx.z * R2 * H + i) = s;
+    else store_sums(out, i, s);
   }
   if (splits > 1) cluster_barrier();      // nobody leaves while its partials may be read
+}
+
+// the clusters' sums, in their order (n = R2 * H)
+__global__ void __launch_bounds__(128)
+lora_grad_a_sum_kernel(const float* __restrict__ ws, int clusters, int64_t n, __nv_bfloat16* __restrict__ out) {
+  pdl_wait();
+  const int64_t i = 4 * ((int64_t)blockIdx.x * 128 + threadIdx.x);      // (n is a multiple of 2048)
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int k = 0; k < clusters; ++k) {
+    const float4 v = *reinterpret_cast<const float4*>(ws + k * n + i);
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  store_sums(out, i, s);
+}
+
+// How the tokens are shared: whole steps each, eight blocks at most per cluster.  One cluster per 128 columns where these fill
+// the GPU or the tokens are few; narrower products of many tokens take several (four blocks per SM, 512 tokens per block at
+// least), which meet in a workspace.  us, one cluster / several, 4 bits, two adapters: 32768 tokens of 1024 columns 54.8 / 21.8, of
+// 2048 65.5 / 34.6, of 128 51.2 / 12.5; 8192 of 1024 16.8 / 13.7 (256 tokens per block: 10.8, but 4096 of 1024 then take 9.5
+// against 8.9 of one cluster).
+struct GaShares { int clusters, blocks, chunk; };
+static GaShares ga_shares(int T, int H) {
+  const int steps = (T + kGaStep - 1) / kGaStep, one = H / kGaCols * kGaMaxSplits;
+  int clusters = 1;
+  if (one < num_sms()) {
+    const int room = 4 * num_sms() / one, wanted = steps / (kGaMaxSplits * kGaMinSteps);
+    clusters = wanted < 1 ? 1 : (wanted < room ? wanted : room);
+  }
+  const int shares = clusters * kGaMaxSplits, chunk = (steps + shares - 1) / shares * kGaStep;
+  return {clusters, clusters > 1 ? kGaMaxSplits : (T + chunk - 1) / chunk, chunk};
 }
 
 }  // namespace hyc
@@ -230,45 +270,49 @@ lora_grad_a_kernel(const uint8_t* __restrict__ q, const __nv_bfloat16* __restric
 using namespace hyc;
 
 extern "C" HYC_API size_t hyc_lora_grad_a_workspace_bytes(int T, int H, int R2) {
-  return T <= 0 || H <= 0 || R2 <= 0 ? 0 : 16;      // (the partial sums stay on chip)
-}
-
-// tokens per block: eight blocks at most share the tokens, whole steps each
-static int ga_chunk(int T) {
-  const int steps = (T + kGaStep - 1) / kGaStep;
-  return (steps + kGaMaxSplits - 1) / kGaMaxSplits * kGaStep;
+  if (T <= 0 || H < kGaCols || R2 <= 0) return 0;
+  const GaShares g = ga_shares(T, H);
+  return g.clusters > 1 ? (size_t)g.clusters * (size_t)R2 * (size_t)H * sizeof(float) : 0;
 }
 
 template <int QBIT, int RT>
-static int launch_ga(const void* q, const void* scale, const void* gm, int64_t ldg, int T, int H, void* out, cudaStream_t st) {
-  const int chunk = ga_chunk(T), splits = (T + chunk - 1) / chunk;
+static int launch_ga(const void* q, const void* scale, const void* gm, int64_t ldg, int T, int H, void* out, void* workspace, cudaStream_t st) {
+  const GaShares g = ga_shares(T, H);
+  float* ws = g.clusters > 1 ? (float*)workspace : nullptr;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(H / kGaCols), (unsigned)splits);
+  cfg.gridDim = dim3((unsigned)(H / kGaCols), (unsigned)g.blocks, (unsigned)g.clusters);
   cfg.blockDim = dim3(128);
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)splits; at[1].val.clusterDim.z = 1;
+  at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)g.blocks; at[1].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = splits > 1 ? 2 : 1;
+  cfg.numAttrs = g.blocks > 1 ? 2 : 1;
   (void)cudaLaunchKernelEx(&cfg, lora_grad_a_kernel<QBIT, RT>, (const uint8_t*)q, (const __nv_bfloat16*)scale, (const __nv_bfloat16*)gm, ldg, T, H,
-                           chunk, (__nv_bfloat16*)out);
+                           g.chunk, (__nv_bfloat16*)out, ws);
   HYC_CHECK_LAUNCH();
+  if (ws != nullptr) {
+    const int64_t n = (int64_t)16 * RT * H;
+    launch_pdl(lora_grad_a_sum_kernel, dim3((unsigned)(n / 512)), dim3(128), 0, st, (const float*)ws, g.clusters, n, (__nv_bfloat16*)out);
+    HYC_CHECK_LAUNCH();
+  }
   return HYC_OK;
 }
 
 extern "C" HYC_API int hyc_lora_grad_a_dequant(const void* q, const void* scale, const void* gm, int64_t ldg, int R2,
                                                int T, int H, int q_bit, void* out, void* workspace, size_t workspace_bytes,
                                                void* stream) {
-  if (!q || !scale || !gm || !out || !workspace) return HYC_ERR_NULL;
+  if (!q || !scale || !gm || !out) return HYC_ERR_NULL;
   if (q_bit != 2 && q_bit != 4 && q_bit != 8) return HYC_ERR_QBIT;
   if (T <= 0 || H <= 0 || H % kGaCols != 0 || R2 <= 0 || R2 % 16 != 0 || R2 > kGaMaxR || ldg < R2) return HYC_ERR_SHAPE;
   if (!aligned(q, 16) || !aligned(scale, 16) || !aligned(gm, 16) || ldg % 8 != 0 || !aligned(workspace, 16)) return HYC_ERR_ALIGN;
-  if (workspace_bytes < hyc_lora_grad_a_workspace_bytes(T, H, R2)) return HYC_ERR_WORKSPACE;
+  const size_t need = hyc_lora_grad_a_workspace_bytes(T, H, R2);
+  if (need > 0 && !workspace) return HYC_ERR_NULL;
+  if (workspace_bytes < need) return HYC_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-#define GA(QB, RT) return launch_ga<QB, RT>(q, scale, gm, ldg, T, H, out, st)
+#define GA(QB, RT) return launch_ga<QB, RT>(q, scale, gm, ldg, T, H, out, workspace, st)
 #define GAQ(QB) switch (R2 / 16) { case 1: GA(QB, 1); case 2: GA(QB, 2); case 3: GA(QB, 3); default: GA(QB, 4); }
   if (q_bit == 2) { GAQ(2) }
   if (q_bit == 4) { GAQ(4) }

@@ -459,8 +459,8 @@ int hyc_attn_bwd_tcgen05(const void* q, const void* k, const void* v, const void
  * packed codes are unpacked into shared-memory tiles and fed to the tensor cores; x_hat is never written to
  * HBM.  q [T, H*q_bit/8], scale [H] bf16, gm [T, ldg] bf16 of which the first R2 columns are used (R2 a
  * multiple of 16, <= 64: several LoRA adapters that share the input can be stacked), out [R2, H] bf16.
- * H % 128 == 0.  workspace: hyc_lora_grad_a_workspace_bytes(T, H, R2) bytes (the partial sums
- * stay on chip). */
+ * H % 128 == 0.  workspace: hyc_lora_grad_a_workspace_bytes(T, H, R2) bytes, 16-byte aligned; where that is
+ * 0 (the partial sums stay on chip) it may be null. */
 size_t hyc_lora_grad_a_workspace_bytes(int T, int H, int R2);
 int hyc_lora_grad_a_dequant(const void* q, const void* scale, const void* gm, int64_t ldg, int R2,
                             int T, int H, int q_bit, void* out, void* workspace, size_t workspace_bytes,

@@ -49,6 +49,13 @@ def test_argument_validation_without_device():
     assert lib.hyc_softmax_fwd_scale_mask(p, 1.0, p, 0, 0, 68, 1, 4, p, 4, 64, None) == -4         # mask row stride
     assert lib.hyc_softmax_fwd_scale_mask(p, 1.0, None, 0, 0, 0, 1, 4, p, 0, 64, None) == 0        # no rows
     assert lib.hyc_softmax_bwd(p, p, None, 4, 64, 1.0, None) == -1
+    # LoRA-A gradients need a workspace only where several clusters share the tokens of few columns
+    size = lib.hyc_lora_grad_a_workspace_bytes
+    assert size(2048, 4096, 48) == size(8192, 14336, 32) == size(131072, 4096, 64) == size(4096, 128, 16) == 0
+    need = size(32768, 512, 32)
+    assert need > 0 and need % (32 * 512 * 4) == 0
+    assert lib.hyc_lora_grad_a_dequant(p, p, p, 32, 32, 32768, 512, 4, p, None, 0, None) == -1
+    assert lib.hyc_lora_grad_a_dequant(p, p, p, 32, 32, 32768, 512, 4, p, p, need - 1, None) == -5
     assert b"q_bit" in lib.hyc_strerror(-2)
 
 

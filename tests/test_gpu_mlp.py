@@ -131,8 +131,22 @@ def test_lora_grad_a_shares_of_the_tokens(mlp, q, T, R2):
     assert not out[:, 3].isfinite().any() and close(out[:, keep], ref[:, keep], rel=4e-3)
 
 
+@pytest.mark.parametrize("q,T,H,R2,clusters", [(4, 8160, 128, 32, 1), (8, 8161, 384, 48, 2), (4, 12300, 256, 16, 3), (8, 12300, 2304, 64, 3), (8, 12300, 2432, 16, 1),
+                                               (2, 122900, 128, 16, 30), (4, 20000, 2176, 32, 4)])
+def test_lora_grad_a_of_narrow_products(mlp, q, T, H, R2, clusters):
+    """Many tokens by few columns: several clusters share the tokens and meet in a workspace (the last shares may be empty)."""
+    from hyc_lora_release_b200._lib import lib
+    assert lib.hyc_lora_grad_a_workspace_bytes(T, H, R2) == (clusters * R2 * H * 4 if clusters > 1 else 0)
+    g = torch.Generator().manual_seed(T + H)
+    codes = torch.randint(0, 256, (T, H * q // 8), generator=g).to(torch.uint8)
+    s, gm = (torch.rand(H, generator=g) + 0.01).to(BF16), _randn(g, T, R2)
+    out = mlp.lora_grad_a(codes.to(DEV), s.to(DEV), gm.to(DEV), R2, q).float().cpu()
+    ref = gm.float().t() @ oracle.ref_decompress(codes[None], s[None], q)[0].float()
+    assert close(out, ref, rel=4e-3)
+
+
 @pytest.mark.parametrize("offset", [1, 2, 3, 4])
-@pytest.mark.parametrize("q,T", [(2, 40), (4, 300), (8, 7)])
+@pytest.mark.parametrize("q,T", [(2, 40), (4, 300), (8, 7), (2, 8200)])
 def test_lora_grad_a_into_a_buffer_of_any_alignment(mlp, q, T, offset):
     """A gradient may start at any element of a caller's buffer: the same bits, and nothing beside it is touched."""
     from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
