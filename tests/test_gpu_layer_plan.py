@@ -17,12 +17,12 @@ NAMES = ("q", "k", "v", "o", "gate", "up", "down")
 class Problem:
     """A calibrated layer with its modules and inputs.  ``seed`` fixes the frozen weights and the inputs."""
 
-    def __init__(self, B=1, M=128, heads=4, kv=2, d=128, I=512, q=4, map_mode="topk", seed=5, bias=()):
+    def __init__(self, B=1, M=128, heads=4, kv=2, d=128, I=512, q=4, map_mode="topk", seed=5, bias=(), mask=None):
         from hyc_lora_release_b200.layer import FusedLlamaLayerIntraInterFullFuse
         g = torch.Generator().manual_seed(seed)
         self.geometry = heads, d, kv
-        x, p, cos, sin, mask = layer_problem(g, B, M, heads * d, heads, d, kv, I)
-        self.x, self.cos, self.sin, self.mask = x.to(DEV), cos.to(DEV), sin.to(DEV), mask.to(DEV)
+        x, p, cos, sin, own_mask = layer_problem(g, B, M, heads * d, heads, d, kv, I)
+        self.x, self.cos, self.sin, self.mask = x.to(DEV), cos.to(DEV), sin.to(DEV), own_mask.to(DEV) if mask is None else mask
         self.gy = torch.randn(x.shape, generator=g).to(BF16).to(DEV)
         self.norms = p["norm_w1"].to(DEV), p["norm_w2"].to(DEV)
         self.mods = {n: (_base(p["w" + n].t().to(DEV), 0.1 * torch.ones(p["w" + n].shape[1], dtype=BF16) if n in bias else None),
@@ -70,7 +70,8 @@ def _same(got, want):
 
 @pytest.mark.parametrize("shape", [dict(), dict(map_mode="prune", q=2), dict(B=2, M=200, map_mode="prune", kv=4, q=8), dict(M=320, q=8),
                                    dict(B=3, M=8, map_mode="prune"), dict(M=264, map_mode="prune", heads=6), dict(M=64, bias=("o", "down")),
-                                   dict(heads=8, kv=4, d=64, M=136, map_mode="prune"), dict(heads=8, d=64, kv=8, M=128), dict(M=1088, map_mode="topk")])
+                                   dict(heads=8, kv=4, d=64, M=136, map_mode="prune"), dict(heads=8, d=64, kv=8, M=128), dict(M=1088, map_mode="topk"),
+                                   dict(B=2, M=256, map_mode="prune"), dict(M=768, map_mode="prune", heads=8, kv=2, q=2), dict(B=2, M=192)])
 def test_plan_equals_the_stepwise_path(shape):
     """The step-wise path is what the oracle tests hold; the plan runs the same launches: equal bits, also after the adapters
     have changed between two steps."""
@@ -85,6 +86,40 @@ def test_plan_equals_the_stepwise_path(shape):
         with torch.no_grad():
             for i, w in enumerate(p.lora()):
                 w.mul_(1 + 0.1 * i)
+    p.layer.raise_on_device_errors()
+
+
+def _masks(kind, B, heads, M):
+    """Additive masks whose rows of tiles end at different places: per batch entry, per head, with a gap, or nowhere."""
+    i = torch.arange(M, device=DEV)
+    dead = i[None] > i[:, None]
+    if kind == "padded":         # the entries of a batch are of different lengths: the last keys of each are ruled out
+        length = torch.tensor([M - 200 * b for b in range(B)], device=DEV)
+        dead = (dead[None] | (i[None, None] >= length[:, None, None]))[:, None]
+    elif kind == "heads":        # heads look back different distances
+        back = torch.tensor([M, 130, 300, 64][:heads], device=DEV)
+        dead = (dead[None] | (i[None] < i[:, None] - back[:, None, None]))[None]
+    elif kind == "gap":          # a tile in the middle of the rows is ruled out
+        dead = (dead & (i[:, None] >= 256) | ((i >= 128) & (i < 256))[None])[None, None]
+    else:                        # "open": nothing is ruled out but a few keys
+        dead = (i < 5).expand(M, M)[None, None]
+    return torch.zeros(dead.shape, dtype=BF16, device=DEV).masked_fill(dead, torch.finfo(BF16).min)
+
+
+@pytest.mark.parametrize("map_mode", ["topk", "prune"])
+@pytest.mark.parametrize("kind,B,heads,kv", [("padded", 2, 4, 2), ("heads", 1, 4, 4), ("heads", 2, 4, 2), ("gap", 1, 4, 2), ("open", 1, 2, 2)])
+def test_plan_equals_the_stepwise_path_for_any_mask(kind, B, heads, kv, map_mode):
+    """The plan leaves what the mask rules out of the map unwritten, the step-wise path writes zeros there: equal bits, also where
+    the memory that the maps get holds NaN."""
+    M = 512
+    p = Problem(B=B, M=M, heads=heads, kv=kv, map_mode=map_mode, mask=_masks(kind, B, heads, M))
+    p.layer.keep_saved = True
+    want = p.step()
+    p.layer.keep_saved = False
+    for _ in range(2):
+        used = [torch.full((B, heads, M, M), float("nan"), dtype=BF16, device=DEV) for _ in range(8)]
+        del used
+        assert _same(p.step(), want) and all(bool(t.isfinite().all()) for t in want)
     p.layer.raise_on_device_errors()
 
 
