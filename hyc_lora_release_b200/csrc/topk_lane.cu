@@ -170,6 +170,36 @@ __device__ __forceinline__ void select_top(const uint32_t (&xw)[32], uint32_t* s
         }
 }
 
+// The lists and codes of the warp's rows row0 .. row0 + n_rows - 1 (row: the lane's), whose groups are in xw and parked at sx
+template <int QBIT, int LPR>
+__device__ __forceinline__ void save_rows(uint32_t (&xw)[32], uint32_t* sx, uint32_t* so, int64_t row0, int n_rows, int64_t row, int GPR, int k,
+                                          bool owns, bool valid, int lr, int rw, int lane, __nv_bfloat16* __restrict__ val_out,
+                                          uint16_t* __restrict__ col_out, uint8_t* __restrict__ q, __nv_bfloat16* __restrict__ scale,
+                                          int8_t* __restrict__ zp) {
+  if (k > 0) {
+    select_top<LPR, false>(xw, sx, so + rw * k, k, owns, valid, 0, 64u * (uint32_t)lr, lr, lane);
+    __syncwarp();
+    lane_slot_load(sx, lane, xw);
+    // the lists of the warp's rows are one contiguous run
+    const int n_ent = n_rows * k;
+    __nv_bfloat16* vrun = val_out + row0 * k;
+    uint16_t* crun = col_out + row0 * k;
+    for (int j = lane; j < n_ent; j += 32) {
+      const uint32_t w = so[j];
+      vrun[j] = __ushort_as_bfloat16((uint16_t)(w & 0xffffu));
+      crun[j] = (uint16_t)(w >> 16);
+    }
+  }
+  float mn, mx;
+  lane_minmax(xw, mn, mx);
+  const GroupParams p = group_params<QBIT>(mn, mx);
+  if (valid && owns) {
+    lane_quant_store<QBIT>(xw, p, q + row * ((int64_t)GPR * (8 * QBIT)) + (64 * QBIT / 8) * lr);
+    scale[row * GPR + lr] = __ushort_as_bfloat16(f32_to_bf16bits_rn(p.s));
+    zp[row * GPR + lr] = (int8_t)(int)p.z;
+  }
+}
+
 // What the SOFTMAX form of the compress kernel needs besides the map itself: the raw scores are read from `a`, turned
 // into probabilities (scale, additive mask, softmax with the rounding points of softmax_fwd_kernel in
 // norm_softmax.cu), written to `dense` for the P.V product, and saved in the same pass.
@@ -192,7 +222,6 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
   constexpr int RPW = 32 / LPR;          // rows per warp
   const int GPR = RAGGED ? groups : LPR; // groups per row
   const int S = 64 * GPR;
-  const int64_t QLD = (int64_t)S * QBIT / 8;
   const LaneMap<LPR, RAGGED> map(GPR);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int lr = lane & (LPR - 1), rw = lane / LPR;
@@ -264,29 +293,7 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
       __syncwarp();
     }
 
-    if (k > 0) {
-      select_top<LPR, false>(xw, sx, so + rw * k, k, owns, valid, 0, 64u * (uint32_t)lr, lr, lane);
-      __syncwarp();
-      lane_slot_load(sx, lane, xw);
-      // the lists of the warp's rows are one contiguous run
-      const int n_ent = n_rows * k;
-      __nv_bfloat16* vrun = val_out + row0 * k;
-      uint16_t* crun = col_out + row0 * k;
-      for (int j = lane; j < n_ent; j += 32) {
-        const uint32_t w = so[j];
-        vrun[j] = __ushort_as_bfloat16((uint16_t)(w & 0xffffu));
-        crun[j] = (uint16_t)(w >> 16);
-      }
-    }
-
-    float mn, mx;
-    lane_minmax(xw, mn, mx);
-    const GroupParams p = group_params<QBIT>(mn, mx);
-    if (valid && owns) {
-      lane_quant_store<QBIT>(xw, p, q + row * QLD + (64 * QBIT / 8) * lr);
-      scale[row * GPR + lr] = __ushort_as_bfloat16(f32_to_bf16bits_rn(p.s));
-      zp[row * GPR + lr] = (int8_t)(int)p.z;
-    }
+    save_rows<QBIT, LPR>(xw, sx, so, row0, n_rows, row, GPR, k, owns, valid, lr, rw, lane, val_out, col_out, q, scale, zp);
     __syncwarp();   // the slots and the staging area are rewritten by other lanes in the next round
   }
 }
@@ -297,7 +304,12 @@ topk_lane_compress_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, int
 // tiles before them are paired outside in (the longest with the shortest), a tile left over in the middle with itself.
 // Which rows fit is decided by their lengths; two that do not take the segment one after the other.  Groups behind a
 // row's end are not read; they get the codes of a group of zeros.  What is stored is what the kernel above stores.
-// [1,32,2048,2048] causal, 5 %, 4 bits: 111 us against 144.
+// That pays where rows end early: whole rows, taken two to a segment one after the other, make items twice as long and a last
+// round half empty.  So the first row decides: where it is whole (no causal map), rows go one by one.  The shape of the launch
+// is that of rows one by one, too: with the one that suits the pairs, five warps per block, fewer warps share an SM (31 % of them
+// against 39 %).  us, 5 %, 4 bits, the kernel above / this one: causal [1,32,2048,2048] 142 / 104, [4,32,1024,1024]
+// 154 / 116, [4,32,256,256] 12.0 / 11.6; nothing ruled out 130 / 126, 138 / 136, 11.7 / 12.0 (before the first row decided and with
+// the other shape: 108, 126, 11.9; 160, 178, 17.1).
 struct SquareMap { int M, items; };      // columns and rows of a map; segments of work per map
 inline SquareMap square_map(int M) {
   const int full = (M - 1) / 128;
@@ -313,7 +325,7 @@ __device__ __forceinline__ void paired_rows(int i, int M, int& ra, int& rb) {
   ra = rb + 64;
 }
 
-template <int QBIT, int LPR>
+template <int QBIT, int LPR, bool RAGGED>
 __global__ void __launch_bounds__(256, HYC_LANE_MINB)
 topk_lane_compress_cols_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows, SquareMap sm, const uint16_t* __restrict__ row_cols, int k,
                                __nv_bfloat16* __restrict__ val_out, uint16_t* __restrict__ col_out,
@@ -328,6 +340,28 @@ topk_lane_compress_cols_kernel(const __nv_bfloat16* __restrict__ a, int64_t rows
   __shared__ uint32_t s_out[8][kLaneStageEntries];
   uint32_t* sx = s_x[warp] + lane * 32;
   uint32_t* so = s_out[warp] + 2 * rw * k;                 // the lists of the segment's two rows
+  if ((int)__ldg(row_cols) >= sm.M) {
+    // rows one by one, as in the kernel above but for the lanes behind their ends
+    const LaneMap<LPR, RAGGED> map(GPR);
+    const bool owns = !RAGGED || lr < GPR;
+    const int64_t items = rows / RPW;                      // (M is a multiple of 64)
+    for (int64_t item = (int64_t)blockIdx.x * nwarps + warp; item < items; item += (int64_t)gridDim.x * nwarps) {
+      const int64_t row0 = item * RPW, row = row0 + rw;
+      const bool inside = 64 * lr < (int)__ldg(row_cols + row);
+      lane_run_to_shared(a + row0 * sm.M, RPW * GPR * 4, s_x[warp], lane, map);
+      __syncwarp();
+      uint32_t xw[32];
+      lane_slot_load(sx, lane, xw);
+      if (!inside) {                                        // whatever lies there
+#pragma unroll
+        for (int j = 0; j < 32; ++j) xw[j] = 0u;
+        lane_slot_store(sx, lane, xw);
+      }
+      save_rows<QBIT, LPR>(xw, sx, s_out[warp], row0, RPW, row, GPR, k, owns, true, lr, rw, lane, val_out, col_out, q, scale, zp);
+      __syncwarp();
+    }
+    return;
+  }
   const GroupParams zero = group_params<QBIT>(0.f, 0.f);
   const uint32_t zero_scale = f32_to_bf16bits_rn(zero.s);
   // a byte of codes of zeros, four times
@@ -633,13 +667,13 @@ static void launch_compress(const void* a, int64_t rows, int groups, int k, void
                                    (uint8_t*)q, (__nv_bfloat16*)scale, zp, *sp);
   }
 }
-template <int QBIT, int LPR>
+template <int QBIT, int LPR, bool RAGGED>
 static void launch_compress_cols(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val, uint16_t* col, void* q, void* scale,
                                  int8_t* zp, cudaStream_t st) {
   const SquareMap sm = square_map(M);
-  auto kern = topk_lane_compress_cols_kernel<QBIT, LPR>;
+  auto kern = topk_lane_compress_cols_kernel<QBIT, LPR, RAGGED>;
   int grid, threads;
-  lane_launch_shape(kern, rows / M * sm.items, 32 / LPR, grid, threads);
+  lane_launch_shape(kern, rows, 32 / LPR, grid, threads);
   launch_pdl(kern, dim3((unsigned)grid), dim3(threads), 0, st, (const __nv_bfloat16*)a, rows, sm, row_cols, k, (__nv_bfloat16*)val, col,
              (uint8_t*)q, (__nv_bfloat16*)scale, zp);
 }
@@ -725,12 +759,10 @@ int topk_lane_restore(const void* val, const uint16_t* col, int k, const void* q
 template <int QB>
 static int compress_cols_q(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val, uint16_t* col, void* q, void* scale,
                            int8_t* zp, cudaStream_t st) {
-  switch (topk_lanes_per_row(M)) {
-#define CC(L) case L: launch_compress_cols<QB, L>(a, rows, M, row_cols, k, val, col, q, scale, zp, st); break
-    CC(1); CC(2); CC(4); CC(8); CC(16);
-    default: launch_compress_cols<QB, 32>(a, rows, M, row_cols, k, val, col, q, scale, zp, st);
-#undef CC
-  }
+  const int S = M;
+#define FN(L, RG) launch_compress_cols<QB, L, RG>
+  HYC_LANE_DISPATCH(FN, a, rows, M, row_cols, k, val, col, q, scale, zp, st);
+#undef FN
   return HYC_OK;
 }
 int topk_lane_compress_cols(const void* a, int64_t rows, int M, const uint16_t* row_cols, int k, void* val_out, uint16_t* col_out,

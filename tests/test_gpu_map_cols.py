@@ -19,6 +19,8 @@ def _map(maps, M, kind, seed):
         cols = torch.full((maps * M,), M, device="cuda")
     else:      # any multiple of 64 (M itself among them), none as well
         cols = (torch.randint(0, M // 64 + 2, (maps * M,), generator=g, device="cuda") * 64).clamp(max=M)
+        if kind != "any":
+            cols[0] = M if kind == "any, the first whole" else 0
     a = torch.softmax(3 * torch.randn(maps * M, M, generator=g, device="cuda"), -1).to(torch.bfloat16)
     behind = torch.arange(M, device="cuda")[None] >= cols[:, None]
     return a.masked_fill(behind, float("nan")), a.masked_fill(behind, 0.0), cols.to(torch.int16), behind
@@ -36,7 +38,7 @@ def _topk_buffers(rows, M, k, q):
             e(rows, M // 64, dt=torch.int8)]
 
 
-@pytest.mark.parametrize("kind", ["causal", "whole", "any"])
+@pytest.mark.parametrize("kind", ["causal", "whole", "any, the first empty", "any, the first whole"])      # (the first row decides on the order)
 @pytest.mark.parametrize("M,k,q", [(64, 3, 4), (128, 6, 2), (192, 9, 4), (192, 10, 8), (448, 22, 4), (704, 35, 4), (704, 0, 2), (1024, 51, 4),
                                    (1984, 99, 2), (2048, 102, 4), (2048, 128, 8)])
 def test_topk_rows_that_end_early(M, k, q, kind):
@@ -60,11 +62,12 @@ def test_topk_rows_that_end_early(M, k, q, kind):
 
 @pytest.mark.parametrize("beyond", [64, 320, 65535 - 704])
 @pytest.mark.parametrize("M,q", [(192, 2), (704, 4), (1984, 8), (512, 4)])
-def test_row_ends_beyond_the_row_are_its_end(M, q, beyond):
+@pytest.mark.parametrize("kind", ["any, the first empty", "any, the first whole"])
+def test_row_ends_beyond_the_row_are_its_end(M, q, beyond, kind):
     """A reported end above M counts as M: no group behind the row is read or written, in the middle of the buffers or after them."""
     maps, k = 2, 5
     rows = maps * M
-    a, dense, cols, behind = _map(maps, M, "any", M)
+    a, dense, cols, behind = _map(maps, M, kind, M)
     too_far = torch.where(cols.int() == M, torch.minimum(cols.int() + beyond, torch.full_like(cols.int(), 65535)), cols.int()).to(torch.uint16)
     assert bool((cols == M).any())
     fill = lambda bufs: [t.view(torch.uint8).fill_(0xa5).view(t.dtype) for t in bufs]
