@@ -306,18 +306,28 @@ __device__ __forceinline__ void tiled_finish(const unsigned long long* counters,
 // Maps whose rows end early, in rows of a multiple of 256 columns: a trip of a batch (256 elements) lies in one row.  Lane j (of
 // every eight) asks how many elements of trip j of a batch count; that is asked a batch ahead, so that the loads of the map do
 // not wait for it.
-struct TripEnds {
+struct TripEnds { const uint16_t* row_cols; uint32_t per_row, rows; };
+struct TripCursor {
   const uint16_t* row_cols;
-  uint32_t per_row, rows;
-  __device__ __forceinline__ int ask(int64_t batch, int lane) const {
-    const uint32_t trip = (uint32_t)batch * kBatch + (uint32_t)(lane & 7), row = trip / per_row;
-    return row < rows ? (int)__ldg(row_cols + row) - 256 * (int)(trip - row * per_row) : 0;
+  uint32_t per_row, rows, row, rem, d_row, d_rem;      // the lane's trip, and how far a batch stride takes it
+  __device__ __forceinline__ TripCursor(const TripEnds& e, int64_t batch, int64_t stride, int lane) : row_cols(e.row_cols), per_row(e.per_row), rows(e.rows) {
+    const uint32_t trip = (uint32_t)batch * kBatch + (uint32_t)(lane & 7), step = (uint32_t)stride * kBatch;
+    row = trip / per_row; rem = trip - row * per_row;
+    d_row = step / per_row; d_rem = step - d_row * per_row;
+  }
+  // of the lane's trip; the next call answers for a stride further
+  __device__ __forceinline__ int ask() {
+    const int n = row < rows ? (int)__ldg(row_cols + row) - 256 * (int)rem : 0;
+    row += d_row; rem += d_rem;
+    if (rem >= per_row) { rem -= per_row; ++row; }
+    return n;
   }
 };
 
-// COLS: rows that end early (M, row_cols); nothing behind their ends is read.  For [4,32,1024,1024] causal the save takes 61 us
-// against 56 (what it reads is half, what it does per batch is not), the restore 37 against 52, and the attention kernel that
-// leaves the zeros out 150 against 165
+// COLS: rows that end early (M, row_cols); nothing behind their ends is read.  us without / with: [4,32,1024,1024] causal, save 58 / 62
+// (what it reads is half, what it does per batch is not), restore 54 / 35, and the attention kernel that leaves the zeros
+// out 143 / 134; a mask that rules out nothing, save 57 / 61, the others alike (save 64 with a division per trip and every load
+// behind a test)
 template <bool NEG, bool COLS>
 __global__ void __launch_bounds__(kTileThreads, 4)
 prune_tiled_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr, int64_t n_tiles,
@@ -342,17 +352,24 @@ prune_tiled_kernel(const __nv_bfloat16* __restrict__ a, int64_t numel, float thr
   const uint32_t sub_cap = capacity / n_sub;          // words per sub-list
   (void)n_tiles;
   uint4 u[kBatch];
-  int next_ends = COLS ? ends.ask(batch, lane) : 0;
+  TripCursor cursor(COLS ? ends : TripEnds{nullptr, 1u, 0u}, batch, stride, lane);
+  int next_ends = COLS ? cursor.ask() : 0;
   auto load_batch = [&](int64_t bt) {
     const int64_t t0 = bt * kBatchElems + 8 * lane;
     if (COLS) {
+      if (!__any_sync(0xffffffffu, next_ends < 256)) {
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) u[j] = ld_stream_v4(a + t0 + 256 * j);
+        next_ends = cursor.ask();
+        return;
+      }
 #pragma unroll
       for (int j = 0; j < kBatch; ++j) {
         const int n = __shfl_sync(0xffffffffu, next_ends, j);
         u[j] = make_uint4(0u, 0u, 0u, 0u);
         if (8 * lane < n) u[j] = ld_stream_v4(a + t0 + 256 * j);
       }
-      next_ends = ends.ask(bt + stride, lane);
+      next_ends = cursor.ask();
       return;
     }
     if ((bt + 1) * kBatchElems <= numel) {
@@ -477,12 +494,13 @@ prune_tiled_restore_kernel(const uint32_t* __restrict__ words, uint32_t capacity
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
   uint2 d = warp0 < n_batches ? __ldg(dir + warp0) : make_uint2(0u, 0u);
-  int next_ends = COLS ? ends.ask(warp0, lane) : 0;
+  TripCursor cursor(COLS ? ends : TripEnds{nullptr, 1u, 0u}, warp0, stride, lane);
+  int next_ends = COLS ? cursor.ask() : 0;
   for (int64_t batch = warp0; batch < n_batches; batch += stride) {
     const uint2 cur = d;
     const int cur_ends = next_ends;
     if (COLS) {
-      next_ends = ends.ask(batch + stride, lane);
+      next_ends = cursor.ask();
       if (!__any_sync(0xffffffffu, cur_ends > 0)) {          // nothing of the batch is wanted (and nothing of it was saved)
         if (batch + stride < n_batches) d = __ldg(dir + batch + stride);
         continue;
