@@ -12,19 +12,20 @@
 //             kv kernel: per 128 keys dV += P^T dO and dK += dS^T Q over the query tiles and the heads of the group.
 //
 // Tiles that the additive mask rules out completely (a causal map: nearly half) are skipped everywhere; a small kernel
-// classifies the mask's tiles on every call.
+// classifies the mask's tiles on every call.  In the map they are written as zeros, or, where the caller takes the ends of the
+// rows (row_cols), only those in front of a tile that is not ruled out.
 //
 // CTA (one per SM): warp 0 loads (TMA, ring of 32 KB tiles), warp 1 issues the MMAs, the other sixteen (kv kernel: eight)
 // do the element-wise work, each a 32-row quadrant and a quarter of the tile's columns (with eight warps of 64 columns
-// the schedulers issued 0.3 instructions a cycle; [1,32,2048,2048] forward 173 us against 139 us with sixteen).  Scores /
+// the schedulers issued 0.3 instructions a cycle; [1,32,2048,2048] forward, in an earlier state, 173 us against 139 us with sixteen).  Scores /
 // dP are double-buffered in tensor memory, so the next tile's product runs while this one is worked on; P and dS go back
 // to tensor memory as the A operand of the second product.  Every wait is bounded (see tc_common.cuh).
 //
 // What bounds them: the forward and q kernels the element-wise work (issue slots 0.47 and 0.39 of one per cycle and
 // scheduler, waits on tensor memory and loads in between; DRAM at 28 and 46 %), the kv kernel its loads (two 32 KB tiles per
 // product; issue slots 0.08, DRAM 56 %).  The tensor pipe is busy a fifth of the time in all three.  Measured
-// [1,32,2048,2048] causal: forward 139 us for 512 MB of map traffic saved, backward 117 + 76 us (204 us as a call from a cold
-// L2); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
+// [1,32,2048,2048] causal, cold: forward 106 us with the ends of the rows and 122 with the whole map, for 512 MB of map traffic saved;
+// backward 185 (111 + 74 as single launches); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
 #include "tc_common.cuh"
 #include <math.h>
 
@@ -452,7 +453,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
     // ---- second pass: probabilities to tensor memory and to the map
     __nv_bfloat16* map = p.map + (int64_t)bh * p.M * p.M;
     // tiles of the map that are written: all, or up to the last one that is not ruled out.  Half of a causal map are zeros that
-    // cost as much to write as probabilities: 140 -> 120 us for [1,32,2048,2048], 165 -> 150 for [4,32,1024,1024]
+    // cost as much to write as probabilities: 122 -> 106 us for [1,32,2048,2048], 143 -> 134 for [4,32,1024,1024]
     int written = nt;
     if (p.row_cols != nullptr) {
       while (written > 0 && bar.cls[written - 1] == 2) --written;

@@ -52,14 +52,16 @@ inline int resident_blocks(K kern, int threads, size_t smem, int otherwise) {
   return n;
 }
 
-// Programmatic dependent launch: a kernel launched with launch_pdl may begin before the kernel in front of it in the
-// stream has ended, and has to call pdl_wait() before it touches global memory (pdl_wait returns once that kernel is
-// complete and its writes are visible; since every such kernel waits, so is everything before it).  It also waits before it takes
-// tensor memory: a library's kernel in front may let its successor in before it has taken its own, and would then wait for columns
-// that the successor keeps until that kernel has ended.  The kernel in front lets it
-// begin by ending: with griddepcontrol.launch_dependents early on, blocks that only wait take the places of the last working
-// ones, and streaming kernels got slower (save, restore and softmax backward of a [4,32,512,512] map 96.6 us against
-// 85.3; without any of this 93.3).
+// Programmatic dependent launch: a kernel launched with launch_pdl (GEMMs and kernels in clusters set the attribute in launch code
+// of their own) may begin before the kernel in front of it in the stream has ended, and has to call pdl_wait() before it touches
+// global memory (pdl_wait returns once that kernel is complete and its writes are visible; since every such kernel waits, so is
+// everything before it).  It also waits before it takes tensor memory: a library's kernel in front may let its successor in
+// before it has taken its own, and would then wait for columns that the successor keeps until that kernel has ended.  The
+// calibration kernels (stats.cu) are launched plainly and do not wait.
+// It saves time between calls that queue up; a single call on an idle GPU gains next to nothing.  The kernel in front lets its
+// successor begin by ending: with griddepcontrol.launch_dependents at the start of every kernel, blocks that only wait take the
+// places of the last working ones, and streaming kernels got slower (save, restore and softmax backward of a
+// [4,32,512,512] map 96.6 us against 85.3; without any of this 93.3).  Letting it in at a block's last tile was not measured.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // (errors stay in cudaGetLastError, as with <<<>>>)
 template <typename K, typename... A>

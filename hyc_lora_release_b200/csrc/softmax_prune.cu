@@ -156,7 +156,7 @@ prune_scan_kernel(int64_t* __restrict__ ws, int64_t n_tiles, int64_t* __restrict
 // bytes, and one store instruction per entry and lane would cost a 32-byte memory transaction for each of them.
 // A lane parks its 64 bytes of the four trips in shared memory and walks the set bits of its mask; four trips without any
 // entry are skipped.  Bound by instructions: with a scan per trip and a test per element the save and restore of a sparse
-// [2,32,696,696] map took 83.4 us, 79.0 now.
+// [2,32,696,696] map took 83.4 us, 79.0 now (count and fill of 31 M elements of which 60 % are kept, which no pruned map is: 74.3, 76.9).
 constexpr int kBatch = 8;                       // chunks a lane has in flight: a tile is two batches
 constexpr int kFillTrips = 4;
 
