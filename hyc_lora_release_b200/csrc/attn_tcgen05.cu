@@ -21,9 +21,9 @@
 // dP are double-buffered in tensor memory, so the next tile's product runs while this one is worked on; P and dS go back
 // to tensor memory as the A operand of the second product.  Every wait is bounded (see tc_common.cuh).
 //
-// What bounds them: the forward and q kernels the element-wise work (issue slots 0.47 and 0.39 of one per cycle and
-// scheduler, waits on tensor memory and loads in between; DRAM at 28 and 46 %), the kv kernel its loads (two 32 KB tiles per
-// product; issue slots 0.08, DRAM 56 %).  The tensor pipe is busy a fifth of the time in all three.  Measured
+// What bounds them: the forward and q kernels the element-wise work (issue slots 0.46 and 0.36 of one per cycle and
+// scheduler, waits on tensor memory and loads in between; DRAM at 21 and 49 %), the kv kernel its loads (two 32 KB tiles per
+// product; issue slots 0.07, DRAM 59 %).  The tensor pipe is busy a quarter of the time in all three.  Measured
 // [1,32,2048,2048] causal, cold: forward 106 us with the ends of the rows and 122 with the whole map, for 512 MB of map traffic saved;
 // backward 185 (111 + 74 as single launches); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
 #include "tc_common.cuh"
