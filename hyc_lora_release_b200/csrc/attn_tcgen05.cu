@@ -25,7 +25,7 @@
 // scheduler, waits on tensor memory and loads in between; DRAM at 21 and 49 %), the kv kernel its loads (two 32 KB tiles per
 // product; issue slots 0.07, DRAM 59 %).  The tensor pipe is busy a quarter of the time in all three.  Measured
 // [1,32,2048,2048] causal, cold: forward 106 us with the ends of the rows and 122 with the whole map, for 512 MB of map traffic saved;
-// backward 185 (111 + 74 as single launches); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
+// backward 171 (105.5 + 65.4 as single launches); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
 #include "tc_common.cuh"
 #include <math.h>
 
@@ -36,7 +36,8 @@ using namespace tc;
 
 constexpr int TILE = 128, TILE_BYTES = TILE * TILE * 2;
 constexpr int EW = 16;                           // element-wise warps of the forward and q kernels
-constexpr int AT_THREADS = 64 + 32 * EW, KV_THREADS = 64 + 32 * 8;
+constexpr int KV_WARPS = 8;                      // of the kv kernel
+constexpr int AT_THREADS = 64 + 32 * EW, KV_THREADS = 64 + 32 * KV_WARPS;
 constexpr int MAX_TILES = 32;                    // sequence lengths up to 4096
 
 // one entry per 128 x 128 tile of the mask: 0 all zero, 1 mixed, 2 nothing passes; rows: bit set = the row has an entry
@@ -198,14 +199,17 @@ __device__ __forceinline__ uint32_t class_of(const AttnParams& p, int b, int h, 
 }
 
 // ------------------------------------------------------------------ shared-memory plan
-//   forward, q kernel: the resident tile (Q, dO), RING ring slots, a 2 KB tile per element-wise warp, row values
-//   kv kernel:         KV_SLOTS ring slots, eight 2 KB tiles
+//   forward:   the resident tile (Q), RING ring slots, a 2 KB tile per element-wise warp, row values
+//   q kernel:  the resident tile (dO), Q_RING ring slots, row values
+//   kv kernel: KV_SLOTS ring slots, eight 2 KB tiles
 // then the barriers
 constexpr int RING = 4, KV_SLOTS = 6;
 constexpr int AT_EPI = TILE_BYTES * (1 + RING), KV_EPI = TILE_BYTES * KV_SLOTS;
 constexpr int AT_ROWS = AT_EPI + EW * 2048;
-constexpr int AT_BARS = AT_ROWS + 8 * TILE * 4, KV_BARS = KV_EPI + 8 * 2048;
-constexpr int AT_SMEM = 1024 + AT_BARS + 512, KV_SMEM = 1024 + KV_BARS + 512;
+constexpr int AT_BARS = AT_ROWS + 8 * TILE * 4, KV_BARS = KV_EPI + KV_WARPS * 2048;
+constexpr int Q_RING = 6, Q_ROWS = TILE_BYTES * (1 + Q_RING), Q_BARS = Q_ROWS + 2 * TILE * 4;
+constexpr int AT_SMEM = 1024 + AT_BARS + 512, KV_SMEM = 1024 + KV_BARS + 512, Q_SMEM = 1024 + Q_BARS + 512;
+static_assert(Q_SMEM <= 227 * 1024 && AT_SMEM <= 227 * 1024 && KV_SMEM <= 227 * 1024, "shared memory of a block");
 constexpr int MAX_SLOTS = 6;
 
 struct Bars {
@@ -214,6 +218,7 @@ struct Bars {
   uint64_t *s_full, *s_free;     // [2] a product is in its buffer / has been read (first pass)
   uint64_t *p_full;              // [2] the element-wise result is in tensor memory
   uint64_t* acc_full;            // accumulator complete
+  uint64_t* ds_out;              // [2] q kernel: dS has left its slot
   uint32_t* tmem_slot;
   volatile int* abort_flag;
   uint8_t* cls;                  // [MAX_TILES]
@@ -221,18 +226,19 @@ struct Bars {
     uint64_t* b = reinterpret_cast<uint64_t*>(at);
     full = b; empty = b + MAX_SLOTS; res_full = b + 2 * MAX_SLOTS;
     s_full = res_full + 1; s_free = s_full + 2; p_full = s_free + 2; acc_full = p_full + 2;
-    tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    ds_out = acc_full + 1;
+    tmem_slot = reinterpret_cast<uint32_t*>(ds_out + 2);
     abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     cls = reinterpret_cast<uint8_t*>(tmem_slot + 2);
   }
 };
 
-// barriers, tensor memory (all 512 columns) and the class list; returns the tensor memory's base
-__device__ __forceinline__ uint32_t at_setup(const AttnParams& p, const Bars& bar, int warp, int lane, int b, int h, int fixed, bool fixed_is_q) {
+// barriers and tensor memory (all 512 columns)
+__device__ __forceinline__ void at_begin(const Bars& bar, int warp, int warps) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < MAX_SLOTS; ++i) { mbar_init(&bar.full[i], 1); mbar_init(&bar.empty[i], 1); }
     mbar_init(bar.res_full, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&bar.s_full[i], 1); mbar_init(&bar.s_free[i], EW); mbar_init(&bar.p_full[i], EW); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bar.s_full[i], 1); mbar_init(&bar.s_free[i], warps); mbar_init(&bar.p_full[i], warps); mbar_init(&bar.ds_out[i], warps); }
     mbar_init(bar.acc_full, 1);
     *bar.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -242,11 +248,18 @@ __device__ __forceinline__ uint32_t at_setup(const AttnParams& p, const Bars& ba
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(bar.tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  if (warp == 2 && lane < p.tiles) bar.cls[lane] = (uint8_t)(fixed_is_q ? class_of(p, b, h, fixed, lane) : class_of(p, b, h, lane, fixed));
+}
+__device__ __forceinline__ uint32_t at_ready(const Bars& bar) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   return *bar.tmem_slot;
+}
+// the same and the class list of query tile qt
+__device__ __forceinline__ uint32_t at_setup(const AttnParams& p, const Bars& bar, int warp, int lane, int b, int h, int qt) {
+  at_begin(bar, warp, EW);
+  if (warp == 2 && lane < p.tiles) bar.cls[lane] = (uint8_t)class_of(p, b, h, qt, lane);
+  return at_ready(bar);
 }
 __device__ __forceinline__ void at_teardown(int warp, uint32_t tmem_base) {
   tc_fence_before();
@@ -330,7 +343,7 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
   // the query tiles with the most key tiles (a causal map's last ones) start first
   const int bh = (int)blockIdx.x % (p.B * p.heads), qt = p.tiles - 1 - (int)blockIdx.x / (p.B * p.heads);
   const int b = bh / p.heads, h = bh % p.heads, kvh = h / (p.heads / p.kv_heads);
-  const uint32_t tmem = at_setup(p, bar, warp, lane, b, h, qt, true);
+  const uint32_t tmem = at_setup(p, bar, warp, lane, b, h, qt);
   const uint32_t res = smem_u32(smem), ring = res + TILE_BYTES;
   // tensor memory: scores / P in two buffers of 128 columns, O in columns 256..383
   const uint32_t t_o = tmem + 256;
@@ -529,15 +542,17 @@ attn_fwd_kernel(const __grid_constant__ FwdMaps maps, const AttnParams p) {
 // maps: dO (hidden layout), V, K (hidden layout), P (the restored map [B * heads, M, M])
 struct BwdQMaps { CUtensorMap g, v, k, p; };
 
+// dS leaves through the ring slot of the P that it was made from: what a staging tile of its own would take buys two more slots, so that
+// two steps of three tiles are in flight ([1,32,2048,2048] causal, cold: 111.8 -> 105.5 us).
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_shared(smem_raw);
-  const Bars bar(smem + AT_BARS);
+  const Bars bar(smem + Q_BARS);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int bh = (int)blockIdx.x % (p.B * p.heads), qt = p.tiles - 1 - (int)blockIdx.x / (p.B * p.heads);
   const int b = bh / p.heads, h = bh % p.heads, kvh = h / (p.heads / p.kv_heads);
-  const uint32_t tmem = at_setup(p, bar, warp, lane, b, h, qt, true);
+  const uint32_t tmem = at_setup(p, bar, warp, lane, b, h, qt);
   const uint32_t res = smem_u32(smem), ring = res + TILE_BYTES;
   // tensor memory: dP / dS in two buffers of 128 columns, dQ in columns 256..383
   const uint32_t t_acc = tmem + 256;
@@ -550,14 +565,21 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
     __syncwarp();
     for (int kt = 0; kt < nt && ok; ++kt) {
       if (bar.cls[kt] == 2) continue;
-      ok = ring_load(p, bar, pos, ring, &maps.v, kvh * TILE, kt * TILE, b, lane);
-      ok = ok && ring_load(p, bar, pos, ring, &maps.p, kt * TILE, qt * TILE, bh, lane);
+      ok = ring_load(p, bar, pos, ring, &maps.v, kvh * TILE, kt * TILE, b, lane, Q_RING);
+      ok = ok && ring_load(p, bar, pos, ring, &maps.p, kt * TILE, qt * TILE, bh, lane, Q_RING);
     }
+    // a step takes three of the six slots, so the P of step j lies where that of step j - 2 was: its dS has to be out
+    int j = 0;
     for (int kt = 0; kt < nt && ok; ++kt) {
       if (bar.cls[kt] == 2) continue;
-      ok = ring_load(p, bar, pos, ring, &maps.v, kvh * TILE, kt * TILE, b, lane);
-      ok = ok && ring_load(p, bar, pos, ring, &maps.p, kt * TILE, qt * TILE, bh, lane);
-      ok = ok && ring_load(p, bar, pos, ring, &maps.k, kvh * TILE, kt * TILE, b, lane);
+      ok = ring_load(p, bar, pos, ring, &maps.v, kvh * TILE, kt * TILE, b, lane, Q_RING);
+      if (ok && j >= 2 && !mbar_wait_warp(&bar.ds_out[j & 1], (uint32_t)((j >> 1) - 1) & 1u, bar.abort_flag)) {
+        if (lane == 0) give_up(p, bar, ST_TIMEOUT_PRODUCER);
+        ok = false;
+      }
+      ok = ok && ring_load(p, bar, pos, ring, &maps.p, kt * TILE, qt * TILE, bh, lane, Q_RING);
+      ok = ok && ring_load(p, bar, pos, ring, &maps.k, kvh * TILE, kt * TILE, b, lane, Q_RING);
+      ++j;
     }
   } else if (warp == 1) {
     RingPos pos;
@@ -565,7 +587,7 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
     for (int kt = 0; kt < nt; ++kt) n1 += bar.cls[kt] != 2;
     bool ok = mma_wait(p, bar, bar.res_full, 0, lane);
     // dP = dO V^T of step t (both passes counted) into buffer t & 1
-    auto grad_map = [&](RingPos& at, int t) {
+    auto grad_map = [&](const RingPos& at, int t) {
       if (!mma_wait(p, bar, &bar.full[at.slot], at.phase, lane)) return false;
       const uint32_t v_addr = ring + (uint32_t)at.slot * TILE_BYTES;
       if (elect_one()) {
@@ -580,13 +602,13 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
     // first pass, slots of step t: V, P.  A step that has been read frees its buffer and its P
     auto step_read = [&](int t) {
       if (!mma_wait(p, bar, &bar.s_free[t & 1], (uint32_t)(t >> 1) & 1u, lane)) return false;
-      if (elect_one()) mbar_arrive(&bar.empty[(2 * t + 1) % RING]);
+      if (elect_one()) mbar_arrive(&bar.empty[(2 * t + 1) % Q_RING]);
       __syncwarp();
       return true;
     };
     for (int t = 0; t < n1 && ok; ++t) {
       ok = (t < 2 || step_read(t - 2)) && grad_map(pos, t);
-      pos.step(RING); pos.step(RING);
+      pos.step(Q_RING); pos.step(Q_RING);
     }
     for (int t = n1 > 1 ? n1 - 2 : 0; t < n1 && ok; ++t) ok = step_read(t);
     // second pass, slots of step j: V, P, K
@@ -594,17 +616,17 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
     if (ok && n1 > 0) ok = grad_map(pv, n1);
     for (int j = 0; j < n1 && ok; ++j) {
       const int t = n1 + j, buf = t & 1;
-      pv.step(RING); pv.step(RING); pv.step(RING);
+      pv.step(Q_RING); pv.step(Q_RING); pv.step(Q_RING);
       if (j + 1 < n1) ok = grad_map(pv, t + 1);
       ok = ok && mma_wait(p, bar, &bar.p_full[buf], (uint32_t)((t >> 1) - ((n1 + (buf ^ (n1 & 1))) >> 1)) & 1u, lane);
-      pos.step(RING);                            // V
+      pos.step(Q_RING);                          // V
       const int p_slot = pos.slot;
-      pos.step(RING);
+      pos.step(Q_RING);
       ok = ok && mma_wait(p, bar, &bar.full[pos.slot], pos.phase, lane);
       if (!ok) break;
       const uint32_t k_addr = ring + (uint32_t)pos.slot * TILE_BYTES, t_s = tmem + (uint32_t)(buf * TILE);
       if (elect_one()) {
-        mbar_arrive(&bar.empty[p_slot]);         // dS is there, so every warp has read its part of P
+        mbar_arrive(&bar.empty[p_slot]);         // (dS still leaves through it: the producer waits for that too)
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
           tc_mma_ta(t_acc, t_s + (uint32_t)((kk >> 1) * 32 + (kk & 1) * 8), desc_mn(k_addr, kk), kIdesc | kBMn, (j > 0 || kk > 0) ? 1u : 0u);
@@ -612,18 +634,17 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
         if (j + 1 == n1) tc_commit<false>(bar.acc_full);
       }
       __syncwarp();
-      pos.step(RING);
+      pos.step(Q_RING);
     }
   } else {
     const int quad = warp & 3, part = (warp - 2) >> 2;
     const int r = quad * 32 + lane;
     const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(32 * part);
-    uint32_t* R = reinterpret_cast<uint32_t*>(smem + AT_EPI) + (warp - 2) * 512;
-    float* s_val = reinterpret_cast<float*>(smem + AT_ROWS);
+    float* s_val = reinterpret_cast<float*>(smem + Q_ROWS);
     bool fine = true;
-    // 16-byte chunk c of the thread's quarter row (a 128-byte row of a swizzled sub-tile holds two quarters)
-    auto row_chunk = [&](const uint8_t* tile, int c) {
-      return *reinterpret_cast<const uint4*>(tile + (part >> 1) * (TILE_BYTES / 2) + r * 128 + (((4 * (part & 1) + c) ^ (r & 7)) << 4));
+    // 16-byte chunk c of this warp's quarter of row rr (a 128-byte row of a swizzled sub-tile holds two quarters)
+    auto chunk_at = [&](uint8_t* tile, int rr, int c) {
+      return reinterpret_cast<uint4*>(tile + (part >> 1) * (TILE_BYTES / 2) + rr * 128 + (((4 * (part & 1) + c) ^ (rr & 7)) << 4));
     };
     // ---- D = rowsum of the bf16 products P * bf16(dP)
     float2 d2 = both(0.f);
@@ -636,12 +657,12 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
       fine = fine && epi_wait(p, bar, &bar.full[pp.slot], pp.phase);
       fine = fine && epi_wait(p, bar, &bar.s_full[buf], (uint32_t)(t >> 1) & 1u);
       if (fine) {
-        const uint8_t* pt = smem + TILE_BYTES * (1 + pp.slot);
+        uint8_t* pt = smem + TILE_BYTES * (1 + pp.slot);
         uint32_t acc[32];
         tc_ld32(t_lane + (uint32_t)(buf * TILE), acc);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const uint4 q4 = row_chunk(pt, e);
+          const uint4 q4 = *chunk_at(pt, r, e);
           const uint32_t pw[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -651,27 +672,31 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar.s_free[buf]);
       }
-      pp.step(RING); pp.step(RING);
+      pp.step(Q_RING); pp.step(Q_RING);
       ++t;
     }
-    s_val[part * TILE + r] = d2.x + d2.y;
+    // (as (0 + 1) + (2 + 3) of the four parts)
+    if (part & 1) s_val[(part >> 1) * TILE + r] = d2.x + d2.y;
     at_sync();
-    const float2 minus_d = both(-((s_val[r] + s_val[TILE + r]) + (s_val[2 * TILE + r] + s_val[3 * TILE + r])));
+    if (!(part & 1)) s_val[(part >> 1) * TILE + r] += d2.x + d2.y;
+    at_sync();
+    const float2 minus_d = both(-(s_val[r] + s_val[TILE + r]));
     // ---- dS = bf16(bf16((bf16(dP) - D) * P) * scale)
     __nv_bfloat16* ds = p.map + (int64_t)bh * p.M * p.M;
     // pp stands one slot behind the first V of this pass: its P
+    int j = 0;
     for (int kt = 0; kt < nt; ++kt) {
       if (bar.cls[kt] == 2) continue;
       const int buf = t & 1;
       fine = fine && epi_wait(p, bar, &bar.full[pp.slot], pp.phase);
       fine = fine && epi_wait(p, bar, &bar.s_full[buf], (uint32_t)(t >> 1) & 1u);
       if (fine) {
-        const uint8_t* pt = smem + TILE_BYTES * (1 + pp.slot);
+        uint8_t* pt = smem + TILE_BYTES * (1 + pp.slot);
         uint32_t w[16], acc[32];
         tc_ld32(t_lane + (uint32_t)(buf * TILE), acc);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const uint4 q4 = row_chunk(pt, e);
+          const uint4 q4 = *chunk_at(pt, r, e);
           const uint32_t pw[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -685,16 +710,27 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar.p_full[buf]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) *reinterpret_cast<uint4*>(R + gd_chunk(lane, e)) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+        for (int e = 0; e < 4; ++e) *chunk_at(pt, r, e) = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
         __syncwarp();
-        flush_clipped(R, ds, qt * TILE + quad * 32, p.M, p.M, kt * TILE + 32 * part, p.M, lane);
+        // eight lanes read two rows whose chunks the swizzle puts on different banks
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int rr = quad * 32 + 8 * k + (lane >> 3) + 4 * ((lane >> 2) & 1), row = qt * TILE + rr, c = kt * TILE + 32 * part + 8 * (lane & 3);
+          const uint4 v = *chunk_at(pt, rr, lane & 3);
+          if (row < p.M && c < p.M) *reinterpret_cast<uint4*>(ds + (int64_t)row * p.M + c) = v;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the next tile of this slot comes by TMA
         __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.ds_out[j & 1]);
       }
-      pp.step(RING); pp.step(RING); pp.step(RING);
+      pp.step(Q_RING); pp.step(Q_RING); pp.step(Q_RING);
       ++t;
+      ++j;
     }
-    fine = fine && t > 0 && epi_wait(p, bar, bar.acc_full, 0);
+    fine = fine && j > 0 && epi_wait(p, bar, bar.acc_full, 0);
     if (fine) {
+      // through the dO tile: its last readers were the products that came before the last of dQ
+      uint32_t* R = reinterpret_cast<uint32_t*>(smem) + (warp - 2) * 512;
       const int64_t ld = (int64_t)p.heads * TILE;
       uint32_t acc[32];
       tc_ld32(t_lane + 256u, acc);
@@ -710,80 +746,135 @@ attn_bwd_q_kernel(const __grid_constant__ BwdQMaps maps, const AttnParams p) {
 // maps: P, dS ([B * heads, M, M]), dO, Q (hidden layout)
 struct BwdKvMaps { CUtensorMap p, s, g, q; };
 
+// the query tiles that do not rule key tile kt out, one bit each (all lanes get all of them)
+__device__ __forceinline__ uint32_t live_query_tiles(const AttnParams& p, int b, int h, int kt, int lane) {
+  return __ballot_sync(0xffffffffu, lane < p.tiles && class_of(p, b, h, lane, kt) != 2u);
+}
+// item -> batch, key/value head, key tile.  The first key tiles have the most query tiles under a causal mask: they come first
+struct KvItem {
+  int b, kvh, kt;
+  __device__ __forceinline__ KvItem(const AttnParams& p, int item) {
+    const int bk = item % (p.B * p.kv_heads);
+    kt = item / (p.B * p.kv_heads); b = bk / p.kv_heads; kvh = bk % p.kv_heads;
+  }
+};
+// The items of a block: one of every `gridDim.x`, taken in turn from either end, so that long and short ones add up to the same.
+// All roles walk the same list.
+__device__ __forceinline__ int kv_item(int round) {
+  const int g = (int)gridDim.x;
+  return round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
+}
+
+// Persistent where that gives a block two items and more: the loads of the next item run while the gradients of this one leave, which is
+// why each item has accumulators of its own (dV and dK, two sets).  [1,32,2048,2048] causal, cold, 512 blocks of one item each / 148 of three
+// or four: 72.4 / 65.4 us.  Both backward kernels, us before / now: 191.5 / 177.1, [4,32,1024,1024] 246.8 / 226.3 (with 8 key/value heads,
+// 256 blocks of one item: 195.6 / 193.5), [2,32,696,696] 80.9 / 74.8, [1,32,2048,2048] with an open mask 356 / 321.  Below two items per
+// SM the fixed shares cost what the overlap gives ([4,32,512,512], 8 key/value heads, 128 items: 78.8 / 80.7 with them).
 __global__ void __launch_bounds__(KV_THREADS, 1)
 attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_shared(smem_raw);
   const Bars bar(smem + KV_BARS);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  // the first key tiles have the most query tiles under a causal mask: they start first
-  const int bk = (int)blockIdx.x % (p.B * p.kv_heads), kt = (int)blockIdx.x / (p.B * p.kv_heads);
-  const int b = bk / p.kv_heads, kvh = bk % p.kv_heads, rep = p.heads / p.kv_heads;
-  const uint32_t tmem = at_setup(p, bar, warp, lane, b, kvh * rep, kt, false);
+  const int rep = p.heads / p.kv_heads, items = p.tiles * p.B * p.kv_heads;
+  at_begin(bar, warp, KV_WARPS);
+  const uint32_t tmem = at_ready(bar);
   const uint32_t ring = smem_u32(smem);
   constexpr int SLOTS = KV_SLOTS;
-  const int nt = p.tiles;
 
   if (warp == 0) {
     bool ok = true;
     RingPos pos;
-    for (int g = 0; g < rep && ok; ++g) {
-      const int h = kvh * rep + g, bh = b * p.heads + h;
-      for (int qt = 0; qt < nt && ok; ++qt) {
-        if (bar.cls[qt] == 2) continue;
-        ok = ring_load(p, bar, pos, ring, &maps.p, kt * TILE, qt * TILE, bh, lane, SLOTS) &&
-             ring_load(p, bar, pos, ring, &maps.g, h * TILE, qt * TILE, b, lane, SLOTS) &&
-             ring_load(p, bar, pos, ring, &maps.s, kt * TILE, qt * TILE, bh, lane, SLOTS) &&
-             ring_load(p, bar, pos, ring, &maps.q, h * TILE, qt * TILE, b, lane, SLOTS);
+    int item = kv_item(0);
+    uint32_t next = 0u;
+    if (item < items) { const KvItem w(p, item); next = live_query_tiles(p, w.b, w.kvh * rep, w.kt, lane); }
+    for (int round = 0; item < items && ok; ++round) {
+      const KvItem w(p, item);
+      const uint32_t live = next;
+      item = kv_item(round + 1);
+      bool asked = false;
+      // the classes of the next item are looked up while the first tiles of this one are on their way
+      auto ask = [&]() {
+        if (!asked && item < items) { const KvItem n(p, item); next = live_query_tiles(p, n.b, n.kvh * rep, n.kt, lane); }
+        asked = true;
+      };
+      for (int g = 0; g < rep && ok; ++g) {
+        const int h = w.kvh * rep + g, bh = w.b * p.heads + h;
+        for (uint32_t left = live; left != 0u && ok; left &= left - 1u) {
+          const int qt = __ffs(left) - 1;
+          ok = ring_load(p, bar, pos, ring, &maps.p, w.kt * TILE, qt * TILE, bh, lane, SLOTS) &&
+               ring_load(p, bar, pos, ring, &maps.g, h * TILE, qt * TILE, w.b, lane, SLOTS) &&
+               ring_load(p, bar, pos, ring, &maps.s, w.kt * TILE, qt * TILE, bh, lane, SLOTS) &&
+               ring_load(p, bar, pos, ring, &maps.q, h * TILE, qt * TILE, w.b, lane, SLOTS);
+          ask();
+        }
       }
+      ask();
     }
   } else if (warp == 1) {
     RingPos pos;
-    int n1 = 0;
-    for (int qt = 0; qt < nt; ++qt) n1 += bar.cls[qt] != 2;
-    const int steps = 2 * rep * n1;               // a product each: dV from P and dO, dK from dS and Q
     bool ok = true;
-    for (int i = 0; i < steps && ok; ++i) {
-      RingPos pb = pos;
-      pb.step(SLOTS);
-      ok = mma_wait(p, bar, &bar.full[pos.slot], pos.phase, lane) && mma_wait(p, bar, &bar.full[pb.slot], pb.phase, lane);
-      if (!ok) break;
-      const uint32_t a_addr = ring + (uint32_t)pos.slot * TILE_BYTES, b_addr = ring + (uint32_t)pb.slot * TILE_BYTES;
-      if (elect_one()) {
+    int used = 0;                                   // items with products so far
+    for (int round = 0, item; (item = kv_item(round)) < items && ok; ++round) {
+      const KvItem w(p, item);
+      const int steps = 2 * rep * __popc(live_query_tiles(p, w.b, w.kvh * rep, w.kt, lane));      // dV from P and dO, dK from dS and Q
+      if (steps == 0) continue;
+      const int set = used & 1;
+      if (used >= 2) ok = mma_wait(p, bar, &bar.s_free[set], (uint32_t)((used >> 1) - 1) & 1u, lane);
+      for (int i = 0; i < steps && ok; ++i) {
+        RingPos pb = pos;
+        pb.step(SLOTS);
+        ok = mma_wait(p, bar, &bar.full[pos.slot], pos.phase, lane) && mma_wait(p, bar, &bar.full[pb.slot], pb.phase, lane);
+        if (!ok) break;
+        const uint32_t a_addr = ring + (uint32_t)pos.slot * TILE_BYTES, b_addr = ring + (uint32_t)pb.slot * TILE_BYTES;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          tc_mma<false>(tmem + (uint32_t)((i & 1) * TILE), desc_mn(a_addr, kk), desc_mn(b_addr, kk), kIdesc | kAMn | kBMn, (i > 1 || kk > 0) ? 1u : 0u);
-        tc_commit<false>(&bar.empty[pos.slot]);
-        tc_commit<false>(&bar.empty[pb.slot]);
-        if (i + 1 == steps) tc_commit<false>(bar.acc_full);
+          for (int kk = 0; kk < 8; ++kk)
+            tc_mma<false>(tmem + (uint32_t)((2 * set + (i & 1)) * TILE), desc_mn(a_addr, kk), desc_mn(b_addr, kk), kIdesc | kAMn | kBMn, (i > 1 || kk > 0) ? 1u : 0u);
+          tc_commit<false>(&bar.empty[pos.slot]);
+          tc_commit<false>(&bar.empty[pb.slot]);
+          if (i + 1 == steps) tc_commit<false>(&bar.s_full[set]);
+        }
+        __syncwarp();
+        pos = pb;
+        pos.step(SLOTS);
       }
-      __syncwarp();
-      pos = pb;
-      pos.step(SLOTS);
+      ++used;
     }
   } else {
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const uint32_t t_lane = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(64 * half);
     uint32_t* R = reinterpret_cast<uint32_t*>(smem + KV_EPI) + (warp - 2) * 512;
-    int n1 = 0;
-    for (int qt = 0; qt < nt; ++qt) n1 += bar.cls[qt] != 2;
-    // keys that no query row attends to (n1 = 0) get zero gradients
-    const bool fine = n1 == 0 || epi_wait(p, bar, bar.acc_full, 0);
-    if (fine) {
-      const int64_t ld = (int64_t)p.kv_heads * TILE;
+    const int64_t ld = (int64_t)p.kv_heads * TILE;
+    bool fine = true;
+    int used = 0;
+    for (int round = 0, item; (item = kv_item(round)) < items && fine; ++round) {
+      const KvItem w(p, item);
+      // keys that no query row attends to get zero gradients
+      const bool any = live_query_tiles(p, w.b, w.kvh * rep, w.kt, lane) != 0u;
+      const int set = used & 1;
+      fine = !any || epi_wait(p, bar, &bar.s_full[set], (uint32_t)(used >> 1) & 1u);
+      if (!fine) break;
 #pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         uint32_t acc[32];
-        if (n1 > 0) tc_ld32(t_lane + (uint32_t)((c >> 1) * TILE + 32 * (c & 1)), acc);
-        if (n1 == 0) {
+        if (any) {
+          tc_ld32(t_lane + (uint32_t)((2 * set + (c >> 1)) * TILE + 32 * (c & 1)), acc);
+          if (c == 3) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar.s_free[set]);
+          }
+        } else {
 #pragma unroll
           for (int e = 0; e < 32; ++e) acc[e] = 0u;
         }
         put_row_bf16(R, lane, acc);
         __syncwarp();
-        flush_clipped(R, (c < 2 ? p.out1 : p.out0) + (int64_t)b * p.M * ld, kt * TILE + quad * 32, p.M, ld, kvh * TILE + 64 * half + 32 * (c & 1), (int)ld, lane);
+        flush_clipped(R, (c < 2 ? p.out1 : p.out0) + (int64_t)w.b * p.M * ld, w.kt * TILE + quad * 32, p.M, ld, w.kvh * TILE + 64 * half + 32 * (c & 1), (int)ld, lane);
         __syncwarp();
       }
+      if (any) ++used;
     }
   }
   at_teardown(warp, tmem);
@@ -907,13 +998,15 @@ extern "C" HYC_API int hyc_attn_bwd_tcgen05(
   p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
   static bool done_q[64] = {false}, done_kv[64] = {false};
-  if (const int rc = at_prepare(attn_bwd_q_kernel, AT_SMEM, done_q)) return rc;
+  if (const int rc = at_prepare(attn_bwd_q_kernel, Q_SMEM, done_q)) return rc;
   if (const int rc = at_prepare(attn_bwd_kv_kernel, KV_SMEM, done_kv)) return rc;
   p.out0 = (__nv_bfloat16*)grad_q; p.map = (__nv_bfloat16*)grad_s;
-  launch_pdl(attn_bwd_q_kernel, dim3((unsigned)(p.tiles * B * heads)), dim3(AT_THREADS), AT_SMEM, st, mq, p);
+  launch_pdl(attn_bwd_q_kernel, dim3((unsigned)(p.tiles * B * heads)), dim3(AT_THREADS), Q_SMEM, st, mq, p);
   HYC_CHECK_LAUNCH();
   p.out0 = (__nv_bfloat16*)grad_k; p.out1 = (__nv_bfloat16*)grad_v;
-  launch_pdl(attn_bwd_kv_kernel, dim3((unsigned)(p.tiles * B * kv_heads)), dim3(KV_THREADS), KV_SMEM, st, mk, p);
+  // fewer than two items per SM: a block each (measured at the kernel)
+  const int items = p.tiles * B * kv_heads, sms = num_sms();
+  launch_pdl(attn_bwd_kv_kernel, dim3((unsigned)(items < 2 * sms ? items : sms)), dim3(KV_THREADS), KV_SMEM, st, mk, p);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
