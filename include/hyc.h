@@ -99,7 +99,7 @@ int hyc_group_unpack_dequant(const void* q, int64_t rows, int N,
 
 /* compression_softmax (compress_function.py:309-313): keep a[i] > bf16(threshold) and
  * a[i] != 0, as the COO list of the flattened map.  Two phases because the caller owns the
- * output: phase 1 counts per tile and leaves exclusive offsets plus the total in `workspace`
+ * output: phase 1 counts per tile and leaves what phase 2 starts from plus the total in `workspace`
  * (copy the int64 at workspace[0] to the host to size idx/val); phase 2 writes them.
  * workspace bytes: hyc_softmax_prune_workspace_bytes(numel). */
 size_t hyc_softmax_prune_workspace_bytes(int64_t numel);
