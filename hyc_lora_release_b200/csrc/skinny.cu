@@ -3,7 +3,7 @@
 //
 // The backward pass needs both forms of every gradient (g B for the input's gradient, g^T xa for B's).  Each is bound by
 // reading X; as library calls they read it twice, and each call costs the host 10 us.  One call for grad_gate, grad_up and
-// hadamard of 2048 tokens (three X of [2048, 11008], 135 MB from HBM): 48 us with its sums, 33 of them the first kernel's,
+// hadamard of 2048 tokens (three X of [2048, 11008], 135 MB from HBM): 37 us with its sums, 31 of them the first kernel's,
 // which is then at 52 % of the DRAM rate (issue slots 7 %: it waits for its tiles).
 //
 // A CTA owns a region of R x C tiles of 128 x 128 of one X.  A tile arrives by TMA (128-byte swizzle) and is the A operand
@@ -192,8 +192,43 @@ skinny_kernel(const __grid_constant__ Args a) {
   }
 }
 
-// Sums of the partials.  A block makes 32 x four values; its eight warps take every eighth partial each and meet in
-// shared memory (one thread adding 43 of them one after the other took 5 us at 2048 rows).
+// Sums of the partials, four values of the result at a time: partials k, k + 8, ... first, then these eight in order.
+struct SumAt {
+  const float* p;                 // its first partial
+  int64_t e, stride;
+  int w, parts;
+  bool is_y;
+  __device__ __forceinline__ SumAt(const Args& a, const Job& j, int64_t i, int64_t ny) {
+    is_y = i < ny;
+    w = is_y ? (int)(i / ((int64_t)a.T * 4)) : 0;
+    e = is_y ? i - (int64_t)w * a.T * 4 : i - ny;
+    stride = is_y ? (int64_t)a.T * 16 : (int64_t)j.n * 16;
+    parts = is_y ? j.col_regions : a.row_regions;
+    p = (is_y ? j.yp + (int64_t)w * j.col_regions * a.T * 16 : j.zp) + e * 4;
+  }
+};
+__device__ __forceinline__ void add4(float4& s, const float4& v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+__device__ __forceinline__ void sum_store(const Job& j, const SumAt& t, const float4& s) {
+  const int64_t at = t.e >> 2;
+  const int r = 4 * (int)(t.e & 3);
+  const uint2 out = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
+  if (t.is_y) {
+    __nv_bfloat16* y = j.y[t.w] + at * j.ld_y + r;
+    *reinterpret_cast<uint2*>(y) = out;
+    // zero columns behind the last product of the job (it rides a GEMM as part of a K block of 64)
+    if (t.w == j.n_w - 1)
+      for (int c = 0; c < j.y_pad; c += 16) *reinterpret_cast<uint2*>(y + 16 + c) = make_uint2(0u, 0u);
+  } else if (j.z_transposed) {
+    const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) j.z[(int64_t)(r + c) * j.n + at] = __float2bfloat16_rn(v[c]);
+  } else {
+    *reinterpret_cast<uint2*>(j.z + at * 16 + r) = out;
+  }
+}
+
+// Many partials: the eight warps of a block take every eighth partial of 32 results each and meet in shared memory
+// (one thread adding 43 of them one after the other took 5 us at 2048 rows).
 __global__ void __launch_bounds__(256)
 sum_kernel(const __grid_constant__ Args a) {
   pdl_wait();
@@ -202,44 +237,50 @@ sum_kernel(const __grid_constant__ Args a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ny = (int64_t)j.n_w * a.T * 4, nz = j.z != nullptr ? (int64_t)j.n * 4 : 0;
   for (int64_t base = (int64_t)blockIdx.x * 32; base < ny + nz; base += (int64_t)gridDim.x * 32) {
-    const int64_t i = base + lane;
-    const bool is_y = i < ny, valid = i < ny + nz;
-    const int w = is_y ? (int)(i / ((int64_t)a.T * 4)) : 0;
-    const int64_t e = is_y ? i - (int64_t)w * a.T * 4 : i - ny, stride = is_y ? (int64_t)a.T * 16 : (int64_t)j.n * 16;
-    const int parts = is_y ? j.col_regions : a.row_regions;
-    const float* p = (is_y ? j.yp + (int64_t)w * j.col_regions * a.T * 16 : j.zp) + e * 4;
+    const bool valid = base + lane < ny + nz;
+    const SumAt t(a, j, base + lane, ny);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
     if (valid) {
 #pragma unroll 4
-      for (int k = warp; k < parts; k += 8) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p + k * stride));
-        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-      }
+      for (int k = warp; k < t.parts; k += 8) add4(s, __ldcg(reinterpret_cast<const float4*>(t.p + k * t.stride)));
     }
     s_part[warp][lane] = s;
     __syncthreads();
     if (warp == 0 && valid) {
 #pragma unroll
-      for (int k = 1; k < 8; ++k) { const float4 v = s_part[k][lane]; s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
-      const int64_t at = e >> 2;
-      const int r = 4 * (int)(e & 3);
-      const uint2 out = make_uint2(pack_bf16x2_rn(s.x, s.y), pack_bf16x2_rn(s.z, s.w));
-      if (is_y) {
-        __nv_bfloat16* y = j.y[w] + at * j.ld_y + r;
-        *reinterpret_cast<uint2*>(y) = out;
-        // zero columns behind the last product of the job (it rides a GEMM as part of a K block of 64)
-        if (w == j.n_w - 1)
-          for (int c = 0; c < j.y_pad; c += 16) *reinterpret_cast<uint2*>(y + 16 + c) = make_uint2(0u, 0u);
-      } else if (j.z_transposed) {
-        const float v[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) j.z[(int64_t)(r + c) * j.n + at] = __float2bfloat16_rn(v[c]);
-      } else {
-        *reinterpret_cast<uint2*>(j.z + at * 16 + r) = out;
-      }
+      for (int k = 1; k < 8; ++k) add4(s, s_part[k][lane]);
+      sum_store(j, t, s);
     }
     __syncthreads();
   }
+}
+
+// Up to sixteen partials: a thread has them all on their way at once.  Taken where that makes a block per SM: three X of [2048, 11008] 10.2 ->
+// 6.0 us (the other way it is 4896 blocks of a barrier and a few loads each); one X of [2048, 4096], 96 blocks, would take 5.1 for 4.4.
+constexpr int kFewParts = 16;
+__global__ void __launch_bounds__(256)
+sum_few_kernel(const __grid_constant__ Args a) {
+  pdl_wait();
+  const Job& j = a.job[blockIdx.y];
+  const int64_t ny = (int64_t)j.n_w * a.T * 4, nz = j.z != nullptr ? (int64_t)j.n * 4 : 0;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= ny + nz) return;
+  const SumAt t(a, j, i, ny);
+  float4 v[kFewParts];
+#pragma unroll
+  for (int k = 0; k < kFewParts; ++k) {
+    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k < t.parts) v[k] = __ldcg(reinterpret_cast<const float4*>(t.p + k * t.stride));
+  }
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float4 pair = v[k];
+    add4(pair, v[k + 8]);
+    if (k == 0) s = pair;
+    else add4(s, pair);
+  }
+  sum_store(j, t, s);
 }
 
 // row-major bf16 [rows, cols] with a row stride of its own; box = box_cols x 128 rows
@@ -357,8 +398,15 @@ extern "C" HYC_API int hyc_skinny_products(int count, const hyc_skinny_job* jobs
   cudaStream_t st = (cudaStream_t)stream;
   launch_pdl(skinny_kernel, dim3((unsigned)first), dim3(SK_THREADS), SK_SMEM, st, a);
   HYC_CHECK_LAUNCH();
-  const int64_t grid = (most + 31) / 32;
-  launch_pdl(sum_kernel, dim3((unsigned)(grid < 4096 ? grid : 4096), count), dim3(256), 0, st, a);
+  int parts = a.row_regions;
+  for (int i = 0; i < count; ++i) parts = a.job[i].n_w > 0 && a.job[i].col_regions > parts ? a.job[i].col_regions : parts;
+  const int64_t few = (most + 255) / 256;
+  if (parts <= kFewParts && few * count >= num_sms()) {
+    launch_pdl(sum_few_kernel, dim3((unsigned)few, count), dim3(256), 0, st, a);
+  } else {
+    const int64_t grid = (most + 31) / 32;
+    launch_pdl(sum_kernel, dim3((unsigned)(grid < 4096 ? grid : 4096), count), dim3(256), 0, st, a);
+  }
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }
