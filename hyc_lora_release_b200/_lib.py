@@ -74,8 +74,12 @@ SIGNATURES = {
                                    _p, _p, _l, _l, _p, _p, _l, _l, _p, _p, _p, _p]),
     "hyc_mlp_gateup_fwd_tcgen05": (_i, [_p, _p, _p, _i, _i, _i, _p, _p, _l, _l, _p, _p, _l, _l,
                                         _p, _p, _p, _p, _p, _p, _p, _i, _p, _p]),
+    "hyc_mlp_gateup_fwd_nf4_tcgen05": (_i, [_p, _p, _i, _i, _i, _p, _p, _l, _l, _p, _p, _l, _l,
+                                        _p, _p, _p, _p, _p, _p, _p, _i, _p, _p]),
     "hyc_linear_lora_save_fwd_tcgen05": (_i, [_p, _p, _i, _i, _i, _p, _p, _l, _l, _p, _p, _p, _p, _i, _p, _p]),
     "hyc_gemm_segments_tcgen05": (_i, [_i, _p, _p, _p, _i, _i, _i, _p, _p, _p, _p]),
+    "hyc_gemm_segments_nf4_tcgen05": (_i, [_i, _p, _p, _p, _p, _i, _i, _i, _p, _p, _p, _p]),
+    "hyc_nf4_product_supported": (_i, [_p, _i, _i]),
     "hyc_skinny_workspace_bytes": (_z, [_i, _p, _i]),
     "hyc_skinny_products": (_i, [_i, _p, _i, _p, _z, _p, _p]),
     "hyc_attn_mask_class_bytes": (_z, [_i, _i, _i]),
@@ -89,7 +93,10 @@ SIGNATURES = {
     "hyc_softmax_topk_restore_cols": (_i, [_p, _p, _i, _p, _p, _p, _l, _i, _p, _p, _i, _p]),
     "hyc_attn_bwd_tcgen05": (_i, [_p] * 6 + [_i] * 5 + [_f, _p, _l, _l, _p, _p, _p, _p, _p]),
     "hyc_linears_lora_save_fwd_tcgen05": (_i, [_p, _i, _i, _i] + [_p] * 7 + [_i, _p, _p]),
+    "hyc_linears_lora_save_fwd_nf4_tcgen05": (_i, [_p, _i, _i, _i] + [_p] * 8 + [_i, _p, _p]),
     "hyc_mlp_graddown_bwd_tcgen05": (_i, [_p, _p, _i, _i, _i, _p, _p, _i, _p, _p, _l, _l, _p, _p, _l, _l,
+                                          _p, _p, _p, _p, _p, _p, _l, _p, _p, _p, _i, _p, _p]),
+    "hyc_mlp_graddown_bwd_nf4_tcgen05": (_i, [_p, _p, _i, _i, _i, _p, _p, _i, _p, _p, _l, _l, _p, _p, _l, _l,
                                           _p, _p, _p, _p, _p, _p, _l, _p, _p, _p, _i, _p, _p]),
 }
 

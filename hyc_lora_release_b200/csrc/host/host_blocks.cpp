@@ -2,7 +2,10 @@
 // What each step is and which rounding points it has is documented in mlp.py and attention.py, which own the
 // calibration branch and the weight records.
 #include "host.h"
+#include <ATen/cuda/CUDAContext.h>
+#include <algorithm>
 #include <array>
+#include <climits>
 #include <cmath>
 
 namespace hyc_host {
@@ -25,17 +28,56 @@ static Tensor factor(const Tensor& b) {
   return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
 }
 
+// a frozen projection: a bf16 matrix, or 4-bit codes, which become one for the product that uses it or are read by it as they are
+struct FrozenWeight {
+  Tensor plain;
+  Tensor packed, code, absmax;
+  OptTensor code2, absmax2;
+  int64_t blocksize2 = 1, blocksize = 64;
+  double offset = 0;
+  std::vector<int64_t> shape;
+  hyc_nf4_weight codes() const {
+    const bool nested = given(code2);
+    return {data(packed), (const float*)data(code), nested ? nullptr : (const float*)data(absmax), nested ? (const uint8_t*)data(absmax) : nullptr,
+            (const float*)data(code2), (const float*)data(absmax2), (int)blocksize, (int)blocksize2, (float)offset};
+  }
+};
+// what a product gets of it
+struct Weight {
+  Tensor m;
+  const FrozenWeight* f = nullptr;          // m undefined: the codes
+  Weight(const Tensor& t) : m(t) {}
+  explicit Weight(const FrozenWeight* w) : f(w) {}
+  int64_t size(int i) const { return f ? f->shape[i] : m.size(i); }
+  hyc_nf4_weight codes() const { return f ? f->codes() : hyc_nf4_weight{}; }
+};
+static void expect(const Weight& w, int64_t rows, int64_t cols, const Tensor& like, const char* what) {
+  if (!w.f) return expect(w.m, rows, cols, what);
+  TORCH_CHECK(w.size(0) == rows && w.size(1) == cols, what, ": expected a [", rows, ", ", cols, "] weight, got ", w.f->shape);
+  require_cuda({&like, &w.f->packed, &w.f->code, &w.f->absmax, opt(w.f->code2), opt(w.f->absmax2)});
+}
+
 // sum of a_i op(b_i) (+ residual), one to four K segments
-struct Segment { const Tensor *a, *b; };
+struct Segment { const Tensor* a; Weight b; };
 static Tensor gemm(std::initializer_list<Segment> segs, int form, const Tensor* residual, const Tensor& status) {
   const Tensor& a = *segs.begin()->a;
   OnDevice on(a);
-  const int64_t M = a.size(0), N = segs.begin()->b->size(form & HYC_GEMM_B_KN ? 1 : 0);
+  const int64_t M = a.size(0), N = segs.begin()->b.size(form & HYC_GEMM_B_KN ? 1 : 0);
   const void *pa[4], *pb[4];
+  hyc_nf4_weight codes[4];
+  bool coded = false;
   int k[4], n = 0;
-  for (const Segment& s : segs) { pa[n] = data(*s.a); pb[n] = data(*s.b); k[n++] = (int)s.a->size(1); }
+  for (const Segment& s : segs) {
+    pa[n] = data(*s.a); pb[n] = data(s.b.m); codes[n] = s.b.codes(); k[n] = (int)s.a->size(1);
+    coded = coded || s.b.f != nullptr;
+    ++n;
+  }
   Tensor d = empty({M, N}, a);
-  check(hyc_gemm_segments_tcgen05(n, pa, pb, k, (int)M, (int)N, form, residual ? data(*residual) : nullptr, data(d),
+  if (coded)
+    check(hyc_gemm_segments_nf4_tcgen05(n, pa, pb, codes, k, (int)M, (int)N, form, residual ? data(*residual) : nullptr, data(d),
+                                        status_ptr(status), on.stream), "hyc_gemm_segments_nf4_tcgen05");
+  else
+    check(hyc_gemm_segments_tcgen05(n, pa, pb, k, (int)M, (int)N, form, residual ? data(*residual) : nullptr, data(d),
                                   status_ptr(status), on.stream), "hyc_gemm_segments_tcgen05");
   return d;
 }
@@ -80,7 +122,7 @@ struct Skinny {
 static const char* at_row(const Tensor& t, int64_t i) { return (const char*)t.data_ptr() + i * t.stride(0) * t.element_size(); }
 
 // the q, k and v projections with the saves of their main branches in one launch: -> {y, codes} of each
-static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, const std::array<const Tensor*, 3>& w, const Tensor& xa3,
+static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, const std::vector<Weight>& w, const Tensor& xa3,
                                                               const std::array<const Tensor*, 3>& b, const std::array<const Tensor*, 3>& scale,
                                                               int64_t q_bit, const Tensor& status) {
   OnDevice on(x);
@@ -89,16 +131,22 @@ static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, c
   Tensor keep[6];
   const void *wp[3], *xp[3], *bp[3], *sp[3];
   void *qp[3], *yp[3];
+  hyc_nf4_weight codes[3];
   int n[3];
   for (int i = 0; i < 3; ++i) {
-    n[i] = (int)w[i]->size(0);
+    n[i] = (int)w[i].size(0);
+    codes[i] = w[i].codes();
     out[i] = {empty({T, n[i]}, x), empty({T, n[i] * q_bit / 8}, x, at::kByte)};
     keep[2 * i] = vec(*scale[i]);
     keep[2 * i + 1] = factor(*b[i]);
-    wp[i] = data(*w[i]); xp[i] = (const char*)xa3.data_ptr() + i * T * 16 * 2; bp[i] = data(keep[2 * i + 1]); sp[i] = data(keep[2 * i]);
+    wp[i] = data(w[i].m); xp[i] = (const char*)xa3.data_ptr() + i * T * 16 * 2; bp[i] = data(keep[2 * i + 1]); sp[i] = data(keep[2 * i]);
     yp[i] = data(out[i].first); qp[i] = data(out[i].second);
   }
-  check(hyc_linears_lora_save_fwd_tcgen05(data(x), (int)T, (int)K, 3, wp, n, xp, bp, sp, qp, yp, (int)q_bit, status_ptr(status), on.stream),
+  if (w[0].f || w[1].f || w[2].f)
+    check(hyc_linears_lora_save_fwd_nf4_tcgen05(data(x), (int)T, (int)K, 3, wp, codes, n, xp, bp, sp, qp, yp, (int)q_bit, status_ptr(status), on.stream),
+          "hyc_linears_lora_save_fwd_nf4_tcgen05");
+  else
+    check(hyc_linears_lora_save_fwd_tcgen05(data(x), (int)T, (int)K, 3, wp, n, xp, bp, sp, qp, yp, (int)q_bit, status_ptr(status), on.stream),
         "hyc_linears_lora_save_fwd_tcgen05");
   return out;
 }
@@ -116,15 +164,6 @@ Tensor lora_grad_a(const Tensor& q, const Tensor& scale, const Tensor& gm, int64
   return out;
 }
 
-// a frozen projection: a bf16 matrix, or 4-bit codes that become one for the product that uses it
-struct FrozenWeight {
-  Tensor plain;
-  Tensor packed, code, absmax;
-  OptTensor code2, absmax2;
-  int64_t blocksize2 = 1, blocksize = 64;
-  double offset = 0;
-  std::vector<int64_t> shape;
-};
 // the matrices of up to four weights, one launch for all that are codes.  Called directly before the product that reads them:
 // what fits of the matrices is then still in L2
 static std::vector<Tensor> matrices(std::initializer_list<const FrozenWeight*> ws) {
@@ -147,21 +186,50 @@ static std::vector<Tensor> matrices(std::initializer_list<const FrozenWeight*> w
   return out;
 }
 
+// The same for a product of T rows: the codes as they are where it takes them (BOTH: where it takes all of them).
+// WHOLE: a product whose K is not split has a CTA per 128 outputs, and each decodes at a rate of its own (0.65 us for 64 x 128
+// elements): on less than half of the SMs a launch of all of them is faster.  us for 128 rows, de-quantizing and product / decoded inside:
+// q, k and v of 4096 (96 CTAs) 55 / 54, o of 4096 (32) 33 / 46; split or wide enough anyway: gate and up of 11008 85 / 77, down 48 / 35,
+// backward of down 50 / 47, grad_x of gate and up 79 / 56, grad_o 26 / 21, grad_x of q, k and v 51 / 37.
+enum class Use { ANY, BOTH, WHOLE };
+static std::vector<Weight> weights(std::initializer_list<const FrozenWeight*> ws, int64_t T, Use use = Use::ANY) {
+  size_t coded = 0;
+  int64_t outputs = 0;
+  for (const FrozenWeight* f : ws) {
+    outputs += f->plain.defined() ? f->plain.size(0) : f->shape[0];
+    if (f->plain.defined()) continue;
+    const hyc_nf4_weight c = f->codes();
+    if (f->shape.size() == 2 && hyc_nf4_product_supported(&c, (int)std::min<int64_t>(T, INT_MAX), (int)f->shape[1])) ++coded;
+    else coded = ws.size() + 1;
+    if (coded > ws.size()) break;
+  }
+  if (coded > 0 && use == Use::WHOLE && outputs / 128 * 2 < at::cuda::getCurrentDeviceProperties()->multiProcessorCount) coded = 0;
+  std::vector<Weight> out;
+  if (coded == 0 || coded > ws.size() || (use == Use::BOTH && coded < ws.size())) {
+    for (const Tensor& m : matrices(ws)) out.emplace_back(m);
+  } else {
+    for (const FrozenWeight* f : ws) f->plain.defined() ? out.emplace_back(f->plain) : out.emplace_back(f);
+  }
+  return out;
+}
+
 // ------------------------------------------------------------------ MLP half
 struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa, down_xa64; };
 
 static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
-                                       const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const FrozenWeight* wd_later = nullptr) {
-  const Tensor &norm_w = w[0], &wg = w[1], &wu = w[2], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
+                                       const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const std::vector<Weight>& gate_up,
+                                       const Weight* wd_now, const FrozenWeight* wd_later = nullptr) {
+  const Weight &wg = gate_up[0], &wu = gate_up[1];
+  const Tensor &norm_w = w[0], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
   const int64_t B = x_medium.size(0), M = x_medium.size(1), H = x_medium.size(2), T = B * M, I = wg.size(0);
-  expect(wg, I, H, "gate projection");
-  expect(wu, I, H, "up projection");
+  expect(wg, I, H, x_medium, "gate projection");
+  expect(wu, I, H, x_medium, "up projection");
   expect_factor(w[4], I, "gate lora_B");
   expect_factor(w[5], I, "up lora_B");
   expect(bd_cols, H, 64, "down lora_B");
   const Tensor gs = scale_vec(stats[3], I), us = scale_vec(stats[4], I);
-  SameDevice{x_medium}.with(w).with(stats).with(bias_d).with(status);
+  SameDevice{x_medium}.with(w).with(wg.m).with(wu.m).with(stats).with(bias_d).with(status);
   OnDevice on(x_medium);
   const Tensor bg = factor(w[4]), bu = factor(w[5]);
   auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale);
@@ -169,31 +237,39 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   const Tensor gu_xa = lora_a_products(xn2, agu_t);
   const char* xa = (const char*)gu_xa.data_ptr();
   Tensor q1 = empty({B, M, I * q / 8}, x_norm, at::kByte), q2 = empty({B, M, I * q / 8}, x_norm, at::kByte), had = empty({T, I}, x_norm);
-  check(hyc_mlp_gateup_fwd_tcgen05(data(xn2), data(wg), data(wu), (int)T, (int)H, (int)I, xa, data(bg), 16, 1, xa + T * 16 * 2, data(bu), 16, 1,
-                                   data(gs), data(us), data(q1), data(q2), data(had), nullptr, nullptr, (int)q, status_ptr(status), on.stream),
-        "hyc_mlp_gateup_fwd_tcgen05");
+  if (wg.f) {
+    const hyc_nf4_weight codes[2] = {wg.codes(), wu.codes()};
+    check(hyc_mlp_gateup_fwd_nf4_tcgen05(data(xn2), codes, (int)T, (int)H, (int)I, xa, data(bg), 16, 1, xa + T * 16 * 2, data(bu), 16, 1, data(gs),
+                                         data(us), data(q1), data(q2), data(had), nullptr, nullptr, (int)q, status_ptr(status), on.stream),
+          "hyc_mlp_gateup_fwd_nf4_tcgen05");
+  } else {
+    check(hyc_mlp_gateup_fwd_tcgen05(data(xn2), data(wg.m), data(wu.m), (int)T, (int)H, (int)I, xa, data(bg), 16, 1, xa + T * 16 * 2, data(bu), 16, 1,
+                                     data(gs), data(us), data(q1), data(q2), data(had), nullptr, nullptr, (int)q, status_ptr(status), on.stream),
+          "hyc_mlp_gateup_fwd_tcgen05");
+  }
   const Tensor down_xa64 = at::mm(had, ad_cols);
-  const Tensor res = bf16c(x_medium), wd = wd_later ? matrices({wd_later})[0] : w[3];
-  require_cuda({&x_medium, &wd});
-  expect(wd, H, I, "down projection");
-  Tensor x_out = gemm({{&had, &wd}, {&down_xa64, &bd_cols}}, 0, &res, status);
+  const Tensor res = bf16c(x_medium);
+  const Weight wd = wd_later ? weights({wd_later}, T)[0] : *wd_now;
+  if (!wd.f) require_cuda({&x_medium, &wd.m});
+  expect(wd, H, I, x_medium, "down projection");
+  Tensor x_out = gemm({{&had, wd}, {&down_xa64, bd_cols}}, 0, &res, status);
   if (given(bias_d)) x_out.add_(bias_d->to(at::kBFloat16));
   return {x_out.view({B, M, H}), rstd, xm_o, xm_q, *xn_q, q1, q2, gs, us, gu_xa, down_xa64};
 }
 
 // up to and including the six LoRA gradients: -> had, ggu, gm64, grad_bd, grad_ad, ga, grad_bgu
-static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q,
+static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const Weight& wd, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q,
                                              const Tensor& status) {
-  const Tensor &wd = w[0], &ad_rows = w[4];
+  const Tensor& ad_rows = w[4];
   const Tensor &gate_q = saved[0], &gate_s = saved[1], &up_q = saved[2], &up_s = saved[3], &gu_xa = saved[4], &down_xa = saved[5],
                &xn_q = saved[6], &xn_scale = saved[7];
   const int64_t T = g.size(0), H = g.size(1), I = wd.size(1);
-  expect(wd, H, I, "down projection");
+  expect(wd, H, I, g, "down projection");
   expect_factor(w[1], I, "gate lora_B");
   expect_factor(w[2], I, "up lora_B");
   expect_factor(w[3], H, "down lora_B");
   expect(ad_rows, 64, I, "down lora_A");
-  SameDevice{g}.with(w).with(saved).with(status);
+  SameDevice{g}.with(wd.m).with(w).with(saved).with(status);
   OnDevice on(g);
   const Tensor bg = factor(w[1]), bu = factor(w[2]), bd = factor(w[3]);
   Tensor grad_bd = empty({H, 16}, g), gdm64 = empty({T, 64}, g), gm64 = empty({T, 64}, g), grad_ad = empty({16, I}, g),
@@ -202,9 +278,16 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<
   Tensor had = empty({T, I}, g), ggu = empty({2, T, I}, g);
   char* gp = (char*)ggu.data_ptr();
   const char* xa = (const char*)gu_xa.data_ptr();
-  check(hyc_mlp_graddown_bwd_tcgen05(data(g), data(wd), (int)T, (int)H, (int)I, data(gdm64), data(ad_rows), 64, xa, data(bg), 16, 1,
-                                     xa + T * 16 * 2, data(bu), 16, 1, data(gate_q), data(gate_s), data(up_q), data(up_s), nullptr, nullptr, 0,
-                                     data(had), gp, gp + T * I * 2, (int)q, status_ptr(status), on.stream), "hyc_mlp_graddown_bwd_tcgen05");
+  if (wd.f) {
+    const hyc_nf4_weight codes = wd.codes();
+    check(hyc_mlp_graddown_bwd_nf4_tcgen05(data(g), &codes, (int)T, (int)H, (int)I, data(gdm64), data(ad_rows), 64, xa, data(bg), 16, 1,
+                                           xa + T * 16 * 2, data(bu), 16, 1, data(gate_q), data(gate_s), data(up_q), data(up_s), nullptr, nullptr, 0,
+                                           data(had), gp, gp + T * I * 2, (int)q, status_ptr(status), on.stream), "hyc_mlp_graddown_bwd_nf4_tcgen05");
+  } else {
+    check(hyc_mlp_graddown_bwd_tcgen05(data(g), data(wd.m), (int)T, (int)H, (int)I, data(gdm64), data(ad_rows), 64, xa, data(bg), 16, 1,
+                                       xa + T * 16 * 2, data(bu), 16, 1, data(gate_q), data(gate_s), data(up_q), data(up_s), nullptr, nullptr, 0,
+                                       data(had), gp, gp + T * I * 2, (int)q, status_ptr(status), on.stream), "hyc_mlp_graddown_bwd_tcgen05");
+  }
   // g_gate Bg | g_up Bu side by side, the two B gradients and grad_ad, each operand read once
   const Tensor g0 = ggu[0], g1 = ggu[1];
   Skinny().on(g0).rows(data(bg), 16, gm64, 0, 64).cols(xa, 16, data(grad_bgu))
@@ -214,15 +297,16 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const std::vector<
   return {had, ggu, gm64, grad_bd, grad_ad, ga, grad_bgu};
 }
 
-static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
-                             at::IntArrayRef shape, int64_t q, const Tensor& status) {
-  const Tensor &wg = w[0], &wu = w[1], &agu_rows = w[2], &norm_w = w[3];
-  expect(wg, ggu.size(2), g.size(1), "gate projection");
-  expect(wu, ggu.size(2), g.size(1), "up projection");
+static Tensor mlp_backward_x(const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Weight>& gate_up, const std::vector<Tensor>& w,
+                             const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
+  const Weight &wg = gate_up[0], &wu = gate_up[1];
+  const Tensor &agu_rows = w[0], &norm_w = w[1];
+  expect(wg, ggu.size(2), g.size(1), g, "gate projection");
+  expect(wu, ggu.size(2), g.size(1), g, "up projection");
   expect(agu_rows, 64, g.size(1), "gate and up lora_A");
-  SameDevice{g}.with(ggu).with(gm64).with(w).with(saved).with(status);
+  SameDevice{g}.with(ggu).with(gm64).with(wg.m).with(wu.m).with(w).with(saved).with(status);
   const Tensor g0 = ggu[0], g1 = ggu[1];
-  Tensor grad_xn = gemm({{&g0, &wg}, {&g1, &wu}, {&gm64, &agu_rows}}, HYC_GEMM_B_KN, nullptr, status);
+  Tensor grad_xn = gemm({{&g0, wg}, {&g1, wu}, {&gm64, agu_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 
@@ -297,25 +381,26 @@ static void rope_pair(const Tensor& q, int64_t nh, const Tensor& k, int64_t nkv,
 using MapForward = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, OptTensor, OptTensor, int64_t, int64_t>;
 // row_cols (wanted if not null): how far each row of the probabilities reaches; what lies behind is zero and then not written.
 // Left undefined where the rows are whole
-static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const RopeTables& tables,
+static MapForward attn_forward_map(const Tensor& x, const std::vector<Weight>& qkv, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const RopeTables& tables,
                                    const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status,
                                    Tensor* row_cols = nullptr) {
-  const Tensor &norm_w = w[0], &wq = w[1], &wk = w[2], &wv = w[3], &bq = w[4], &bk = w[5], &bv = w[6], &aqkv_t = w[7];
+  const Tensor &norm_w = w[0], &bq = w[1], &bk = w[2], &bv = w[3], &aqkv_t = w[4];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
-  check_geometry({wq.size(0), wk.size(0), wv.size(0)}, nh, d, nkv);
+  check_geometry({qkv[0].size(0), qkv[1].size(0), qkv[2].size(0)}, nh, d, nkv);
   for (int i = 0; i < 3; ++i) {
     const char* const names[3][2] = {{"q projection", "q lora_B"}, {"k projection", "k lora_B"}, {"v projection", "v lora_B"}};
-    expect(w[1 + i], w[1 + i].size(0), x.size(2), names[i][0]);
-    expect_factor(w[4 + i], w[1 + i].size(0), names[i][1]);
-    scale_vec(stats[3 + i], w[1 + i].size(0));
+    expect(qkv[i], qkv[i].size(0), x.size(2), x, names[i][0]);
+    expect_factor(w[1 + i], qkv[i].size(0), names[i][1]);
+    scale_vec(stats[3 + i], qkv[i].size(0));
   }
+  for (const Weight& f : qkv) SameDevice{x}.with(f.m);
   SameDevice{x}.with(w).with(stats).with(tables.cos).with(tables.sin).with(mask).with(status);
   OnDevice on(x);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M, rep = nh / nkv;
   auto [x_norm, rstd, x_o, x_q, xn_q] = rmsnorm_save(x, norm_w, eps, q, x_scale, x_idx, xn_scale);
   const Tensor xn2 = x_norm.view({T, H});
   const Tensor xa3 = lora_a_products(xn2, aqkv_t);
-  auto p3 = qkv_lora_save(xn2, {&wq, &wk, &wv}, xa3, {&bq, &bk, &bv}, {&q_scale, &k_scale, &v_scale}, q, status);
+  auto p3 = qkv_lora_save(xn2, qkv, xa3, {&bq, &bk, &bv}, {&q_scale, &k_scale, &v_scale}, q, status);
   const auto &[qy, q_q] = p3[0];
   const auto &[ky, k_q] = p3[1];
   const auto &[vy, v_q] = p3[2];
@@ -348,15 +433,15 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Tensor>& w
 }
 
 // o projection with residual and the save of its input
-static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols,
+static std::vector<Tensor> attn_forward_out(const Tensor& x, const Tensor& o2, const Weight& wo, const Tensor& ao_cols, const Tensor& bo_cols,
                                             const Tensor& o_scale, const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& status) {
-  expect(wo, x.size(2), o2.size(1), "o projection");
+  expect(wo, x.size(2), o2.size(1), x, "o projection");
   expect(bo_cols, x.size(2), 64, "o lora_B");
-  SameDevice{x}.with(o2).with(wo).with(ao_cols).with(bo_cols).with(o_scale).with(o_codes).with(bias_o).with(status);
+  SameDevice{x}.with(o2).with(wo.m).with(ao_cols).with(bo_cols).with(o_scale).with(o_codes).with(bias_o).with(status);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M;
   const Tensor o_xa64 = at::mm(o2, ao_cols);
   const Tensor res = bf16c(x);
-  Tensor x_medium = gemm({{&o2, &wo}, {&o_xa64, &bo_cols}}, HYC_GEMM_FIXED_ORDER, &res, status);
+  Tensor x_medium = gemm({{&o2, wo}, {&o_xa64, bo_cols}}, HYC_GEMM_FIXED_ORDER, &res, status);
   if (given(bias_o)) x_medium.add_(bias_o->to(at::kBFloat16));
   const Tensor o_q = given(o_codes) ? *o_codes : std::get<0>(quant(o2.view({B, M, -1}), o_scale, q, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
   return {x_medium.view({B, M, H}), o_q.view({T, -1}), o_xa64};
@@ -368,19 +453,19 @@ static Tensor rebuild(const Tensor& codes, const Tensor& scale, const Tensor& xa
 }
 
 // o projection backward: -> grad_bo, grad_ao, grad_o2
-static std::vector<Tensor> attn_backward_out(const Tensor& g, const Tensor& wo, const Tensor& bo_in, const Tensor& ao_rows, const Tensor& o_xa,
+static std::vector<Tensor> attn_backward_out(const Tensor& g, const Weight& wo, const Tensor& bo_in, const Tensor& ao_rows, const Tensor& o_xa,
                                              const Tensor& o_q, const Tensor& o_scale, int64_t q, const Tensor& status) {
-  expect(wo, g.size(1), wo.size(1), "o projection");
+  expect(wo, g.size(1), wo.size(1), g, "o projection");
   expect_factor(bo_in, g.size(1), "o lora_B");
   expect(ao_rows, 64, wo.size(1), "o lora_A");
-  SameDevice{g}.with(wo).with(bo_in).with(ao_rows).with(o_xa).with(o_q).with(o_scale).with(status);
+  SameDevice{g}.with(wo.m).with(bo_in).with(ao_rows).with(o_xa).with(o_q).with(o_scale).with(status);
   OnDevice on(g);
   const int64_t T = g.size(0);
   const Tensor bo = factor(bo_in);
   Tensor gm64 = empty({T, 64}, g), grad_bo = empty({g.size(1), 16}, g);
   Skinny().on(g).rows(data(bo), 16, gm64, 0, 64, 48).cols(data(o_xa), o_xa.stride(0), data(grad_bo)).run(T, g, status, on.stream);
   Tensor grad_ao = lora_grad_a(o_q, vec(o_scale), gm64, 16, q);
-  Tensor grad_o2 = gemm({{&g, &wo}, {&gm64, &ao_rows}}, HYC_GEMM_B_KN, nullptr, status);
+  Tensor grad_o2 = gemm({{&g, wo}, {&gm64, ao_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return {grad_bo, grad_ao, grad_o2};
 }
 
@@ -469,13 +554,16 @@ static std::vector<Tensor> attn_backward_lora(const std::vector<Tensor>& grads, 
   return {gmq, ga, gb[0], gb[1], gb[2]};
 }
 
-static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
+static Tensor attn_backward_x(const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Weight>& qkv, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, at::IntArrayRef shape, int64_t q, const Tensor& status) {
-  const Tensor &wq = w[0], &wk = w[1], &wv = w[2], &aqkv_rows = w[3], &norm_w = w[4];
-  for (int i = 0; i < 3; ++i) expect(w[i], grads[i].size(1), g.size(1), "q, k or v projection");
+  const Tensor &aqkv_rows = w[0], &norm_w = w[1];
+  for (int i = 0; i < 3; ++i) {
+    expect(qkv[i], grads[i].size(1), g.size(1), g, "q, k or v projection");
+    SameDevice{g}.with(qkv[i].m);
+  }
   expect(aqkv_rows, 64, g.size(1), "lora_A of q, k and v");
   SameDevice{g}.with(grads).with(gmq).with(w).with(saved).with(status);
-  Tensor grad_xn = gemm({{&grads[0], &wq}, {&grads[1], &wk}, {&grads[2], &wv}, {&gmq, &aqkv_rows}}, HYC_GEMM_B_KN, nullptr, status);
+  Tensor grad_xn = gemm({{&grads[0], qkv[0]}, {&grads[1], qkv[1]}, {&grads[2], qkv[2]}, {&gmq, aqkv_rows}}, HYC_GEMM_B_KN, nullptr, status);
   return rmsnorm_backward_packed(grad_xn.view(shape), saved[0], saved[1], saved[2], saved[3], norm_w, saved[4], q, g.view(shape));
 }
 
@@ -598,13 +686,13 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
   {
     Tensor a, o2;
     OptTensor o_codes;
-    std::vector<Tensor> w = matrices({&p.w[PQ], &p.w[PK], &p.w[PV]});
+    std::vector<Weight> w = weights({&p.w[PQ], &p.w[PK], &p.w[PV]}, s->B * s->M, Use::WHOLE);
     // where the save and the restore know how to leave out what the mask rules out (tiles of 128 columns: not in maps of one tile).
     // us of the attention kernel, save and restore without / with, 5 % kept: causal [4,32,1024,1024] top-k 364 / 300, pruned 254 / 231,
     // [4,32,256,256] 41 / 40 and 42 / 41; a mask that rules out nothing, which is not known here, 396 / 392 and 304 / 308
     const bool cols = s->M > 128 && (map_q == 0 ? s->M % 256 == 0 : hyc_softmax_topk_cols_supported((int)s->M, (int)map_k) == 1);
     std::tie(a, o2, s->rstd, s->x_o, s->x_q, s->xn_q, s->q_q, s->k_q, s->v_q, s->xa3, o_codes, s->cls, s->cls_b, s->cls_h) = attn_forward_map(
-        x, {p.norm1, w[0], w[1], w[2], p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
+        x, w, {p.norm1, p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
         {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status, cols ? &s->row_cols : nullptr);
     w.clear();
     if (map_q > 0) {
@@ -615,13 +703,13 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
       s->map = {words, directory, nnz};
     }
     a.reset();
-    auto out = attn_forward_out(x, o2, matrices({&p.w[PO]})[0], p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
+    auto out = attn_forward_out(x, o2, weights({&p.w[PO]}, s->B * s->M, Use::WHOLE)[0], p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
     x_medium = out[0]; s->o_q = out[1]; s->o_xa64 = out[2];
   }
-  std::vector<Tensor> w = matrices({&p.w[PGATE], &p.w[PUP]});
-  s->mlp = mlp_forward(x_medium, {p.norm2, std::move(w[0]), std::move(w[1]), Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
+  std::vector<Weight> w = weights({&p.w[PGATE], &p.w[PUP]}, s->B * s->M, Use::BOTH);
+  s->mlp = mlp_forward(x_medium, {p.norm2, Tensor(), Tensor(), Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
                                   p.pad[AGU_T], p.pad[AD_COLS], p.pad[BD_COLS]},
-                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, &p.w[PDOWN]);
+                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, w, nullptr, &p.w[PDOWN]);
   Tensor y = std::move(s->mlp.x_out);
   s->mlp.x_out = Tensor();
   return {y.to(s->x_type), s};
@@ -656,15 +744,14 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   {
     const Tensor g = bf16c(grad_y).view({T, s.H});
     const MlpForward& m = s.mlp;
-    auto r = mlp_backward_lora(g, {matrices({&p.w[PDOWN]})[0], p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
+    auto r = mlp_backward_lora(g, weights({&p.w[PDOWN]}, T)[0], {Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
                                {m.q1, m.gs, m.q2, m.us, m.gu_xa, m.down_xa64, m.xn_q, st[XN2_SCALE]}, s.q_mlp, status);
     lora(PGATE, r[5].narrow(0, 0, 16), r[6].select(0, 0));
     lora(PUP, r[5].narrow(0, 16, 16), r[6].select(0, 1));
     lora(PDOWN, r[4], r[3]);
     report({{"g", PGATE}, {"u", PUP}, {"d", PDOWN}});
     r[0].reset();
-    const std::vector<Tensor> w = matrices({&p.w[PGATE], &p.w[PUP]});
-    g_medium = mlp_backward_x(g, r[1], r[2], {w[0], w[1], p.pad[AGU_ROWS], p.norm2},
+    g_medium = mlp_backward_x(g, r[1], r[2], weights({&p.w[PGATE], &p.w[PUP]}, T), {p.pad[AGU_ROWS], p.norm2},
                               {m.xm_q, st[XM_SCALE], m.xm_o, st[XM_IDX], m.rstd}, shape, s.q_mlp, status).view({T, s.H});
   }
   if (!hook.is_none() && !p.fresh()) {           // the hook of the MLP half changed factors of this one
@@ -674,7 +761,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   }
   std::vector<Tensor> grads;
   {
-    auto r = attn_backward_out(g_medium, matrices({&p.w[PO]})[0], p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
+    auto r = attn_backward_out(g_medium, weights({&p.w[PO]}, T)[0], p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
     lora(PO, r[1], r[0]);
     const std::vector<int64_t> a_shape = {s.B, s.nh, s.M, s.M};
     const bool topk = s.map_q > 0;
@@ -690,8 +777,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   auto r = attn_backward_lora(grads, {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.xa3, s.xn_q, st[XN1_SCALE], s.q_attn, status);
   for (int i = 0; i < 3; ++i) lora(PQ + i, r[1].narrow(0, 16 * i, 16), r[2 + i]);
   report({{"q", PQ}, {"k", PK}, {"v", PV}, {"o", PO}});
-  const std::vector<Tensor> w = matrices({&p.w[PQ], &p.w[PK], &p.w[PV]});
-  out[0] = attn_backward_x(g_medium, grads, r[0], {w[0], w[1], w[2], p.pad[AQKV_ROWS], p.norm1},
+  out[0] = attn_backward_x(g_medium, grads, r[0], weights({&p.w[PQ], &p.w[PK], &p.w[PV]}, T), {p.pad[AQKV_ROWS], p.norm1},
                            {s.x_q, st[X_SCALE], s.x_o, st[X_IDX], s.rstd}, shape, s.q_attn, status).to(s.x_type);
   return out;
 }
@@ -701,16 +787,22 @@ void bind_blocks(pybind11::module_& m) {
   m.def("capture_of", &capture_of);
   m.def("mlp_forward", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const OptTensor& bias_d, int64_t q,
                           double eps, const Tensor& st) {
-    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st);
+    const Weight wd(w[3]);
+    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st, {Weight(w[1]), Weight(w[2])}, &wd);
     return std::vector<Tensor>{f.x_out, f.rstd, f.xm_o, f.xm_q, f.xn_q, f.q1, f.q2, f.gs, f.us, f.gu_xa, f.down_xa64}; });
-  m.def("mlp_backward_lora", &mlp_backward_lora);
+  m.def("mlp_backward_lora", [](const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q, const Tensor& st) {
+    return mlp_backward_lora(g, w[0], w, saved, q, st); });
   m.def("mlp_backward_x", [](const Tensor& g, const Tensor& ggu, const Tensor& gm64, const std::vector<Tensor>& w, const std::vector<Tensor>& saved,
-                             std::vector<int64_t> shape, int64_t q, const Tensor& st) { return mlp_backward_x(g, ggu, gm64, w, saved, shape, q, st); });
+                             std::vector<int64_t> shape, int64_t q, const Tensor& st) { return mlp_backward_x(g, ggu, gm64, {Weight(w[0]), Weight(w[1])}, {w[2], w[3]}, saved, shape, q, st); });
   m.def("attn_forward_map", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos, const Tensor& sin,
                                const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& st) {
-    return attn_forward_map(x, w, stats, rope_tables(cos, sin, x.size(1), d), mask, nh, d, nkv, q, eps, st); });
-  m.def("attn_forward_out", &attn_forward_out);
-  m.def("attn_backward_out", &attn_backward_out);
+    return attn_forward_map(x, {Weight(w[1]), Weight(w[2]), Weight(w[3])}, {w[0], w[4], w[5], w[6], w[7]}, stats, rope_tables(cos, sin, x.size(1), d), mask, nh, d, nkv, q, eps, st); });
+  m.def("attn_forward_out", [](const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols, const Tensor& o_scale,
+                               const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& st) {
+    return attn_forward_out(x, o2, wo, ao_cols, bo_cols, o_scale, o_codes, bias_o, q, st); });
+  m.def("attn_backward_out", [](const Tensor& g, const Tensor& wo, const Tensor& bo, const Tensor& ao_rows, const Tensor& o_xa, const Tensor& o_q,
+                                const Tensor& o_scale, int64_t q, const Tensor& st) {
+    return attn_backward_out(g, wo, bo, ao_rows, o_xa, o_q, o_scale, q, st); });
   m.def("attn_backward_map", [](const Tensor& grad_o2, const Tensor& a, const std::vector<Tensor>& topk, int64_t map_q_bit, const std::vector<Tensor>& saved,
                                 const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin, int64_t B, int64_t M, int64_t nh, int64_t d,
                                 int64_t nkv, int64_t q, const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& st) {
@@ -718,7 +810,7 @@ void bind_blocks(pybind11::module_& m) {
   m.def("attn_backward_lora", &attn_backward_lora);
   m.def("attn_backward_x", [](const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, std::vector<int64_t> shape, int64_t q, const Tensor& st) {
-    return attn_backward_x(g, grads, gmq, w, saved, shape, q, st); });
+    return attn_backward_x(g, grads, gmq, {Weight(w[0]), Weight(w[1]), Weight(w[2])}, {w[3], w[4]}, saved, shape, q, st); });
   pybind11::class_<FrozenWeight>(m, "FrozenWeight")
       .def(pybind11::init([](const Tensor& w) { FrozenWeight f; f.plain = w; return f; }))
       .def(pybind11::init([](const Tensor& packed, const Tensor& code, const Tensor& absmax, const OptTensor& code2, const OptTensor& absmax2,

@@ -684,7 +684,8 @@ static int launch_as(const Operands& ops, const Params& p, cudaStream_t st) {
 }
 
 template <int EPI, int QBIT, bool B_MN>
-static int launch(const Operands& ops, const Params& p, cudaStream_t st) {
+static int launch(const Operands& ops, const Params& p, cudaStream_t st, const FourWeights* four = nullptr) {
+  if (four != nullptr) return launch_four(EPI, QBIT, B_MN, ops, p, *four, st);
   const SplitPlan plan = choose_split(EPI, p);
   if (plan.split > 0) return launch_split(EPI, QBIT, B_MN, plan, ops, p, st);
   // pairs, except where few rows would leave half of the tile empty
@@ -708,6 +709,25 @@ static LoraTerm make_term(const void* xa, const void* bt, int64_t ld_col, int64_
   t.ld_r = ld_r;
   return t;
 }
+
+// the weights of a product as the split kernel decodes them; `w`: null, or one entry per B operand (its `packed` null: that one is bf16)
+static int shift_of(int blocksize) {
+  int s = 0;
+  while ((1 << s) < blocksize && s < 30) ++s;
+  return (1 << s) == blocksize ? s : -1;
+}
+static bool four_takes(const hyc_nf4_weight& w, int rows, int cols) {
+  if (!w.packed || !w.code16 || (!w.absmax && (!w.absmax_q || !w.code256 || !w.absmax2))) return false;
+  return rows >= 1 && rows <= BM && cols % 64 == 0 && w.blocksize >= 64 && shift_of(w.blocksize) >= 0 && aligned(w.packed, 32) && aligned(w.code16, 4) &&
+         (w.absmax || (w.blocksize2 >= 1 && shift_of(w.blocksize2) >= 0));
+}
+static FourView four_view(const hyc_nf4_weight& w, int64_t cols) {
+  return {(const uint8_t*)w.packed, w.code16, w.absmax, w.absmax_q, w.code256, w.absmax2, cols, shift_of(w.blocksize),
+          w.absmax ? 0 : shift_of(w.blocksize2), w.offset};
+}
+static bool has_four(const hyc_nf4_weight* w, int i) { return w != nullptr && w[i].packed != nullptr; }
+
+extern "C" HYC_API int hyc_nf4_product_supported(const hyc_nf4_weight* w, int rows, int cols) { return w && four_takes(*w, rows, cols) ? 1 : 0; }
 
 extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
     const void* A, const void* B, int M, int N, int K, int form,
@@ -745,17 +765,25 @@ extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
   return b_is_kn ? launch<EPI_STORE, 4, true>(ops, p, st) : launch<EPI_STORE, 4, false>(ops, p, st);
 }
 
-extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
-                                                int form, const void* residual, void* D, int* status, void* stream) {
+static int gemm_segments(int count, const void* const* A, const void* const* B, const hyc_nf4_weight* B4, const int* K, int M, int N,
+                         int form, const void* residual, void* D, int* status, void* stream) {
   if (!A || !B || !K || !D || !status) return HYC_ERR_NULL;
   if (form & ~kGemmForms) return HYC_ERR_SHAPE;
   const bool b_is_kn = (form & HYC_GEMM_B_KN) != 0;
   if (count < 1 || count > 4 || M <= 0 || N <= 0 || N % BN != 0) return HYC_ERR_SHAPE;
   if (!aligned(D, 16) || (residual && !aligned(residual, 16))) return HYC_ERR_ALIGN;
   Operands ops = {};
+  FourWeights four = {};
   for (int i = 0; i < count; ++i) {
-    if (!A[i] || !B[i]) return HYC_ERR_NULL;
+    if (!A[i] || (!B[i] && !has_four(B4, i))) return HYC_ERR_NULL;
     if (K[i] <= 0 || K[i] % BK != 0) return HYC_ERR_SHAPE;
+    if (has_four(B4, i)) {
+      if (!four_takes(B4[i], M, b_is_kn ? N : K[i])) return HYC_ERR_UNSUPPORTED;
+      if (!aligned(A[i], 16)) return HYC_ERR_ALIGN;
+      ops.a[i] = {A[i], M, K[i]};
+      four.w[i] = four_view(B4[i], b_is_kn ? N : K[i]);
+      continue;
+    }
     if (!aligned(A[i], 16) || !aligned(B[i], 16)) return HYC_ERR_ALIGN;
     ops.a[i] = {A[i], M, K[i]};
     ops.b[i] = b_is_kn ? Matrix{B[i], K[i], N} : Matrix{B[i], N, K[i]};
@@ -769,24 +797,38 @@ extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A
   p.status = status;
   p.g_end0 = p.g_end1 = N;
   cudaStream_t st = (cudaStream_t)stream;
-  return b_is_kn ? launch<EPI_STORE, 4, true>(ops, p, st) : launch<EPI_STORE, 4, false>(ops, p, st);
+  const FourWeights* f4 = B4 ? &four : nullptr;
+  return b_is_kn ? launch<EPI_STORE, 4, true>(ops, p, st, f4) : launch<EPI_STORE, 4, false>(ops, p, st, f4);
+}
+extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
+                                                int form, const void* residual, void* D, int* status, void* stream) {
+  return gemm_segments(count, A, B, nullptr, K, M, N, form, residual, D, status, stream);
+}
+extern "C" HYC_API int hyc_gemm_segments_nf4_tcgen05(int count, const void* const* A, const void* const* B, const hyc_nf4_weight* B4, const int* K,
+                                                    int M, int N, int form, const void* residual, void* D, int* status, void* stream) {
+  if (!B4) return HYC_ERR_NULL;
+  return gemm_segments(count, A, B, B4, K, M, N, form, residual, D, status, stream);
 }
 
-extern "C" HYC_API int hyc_mlp_gateup_fwd_tcgen05(
-    const void* x, const void* wg, const void* wu, int T, int H, int I,
+static int gateup_fwd(
+    const void* x, const void* wg, const void* wu, const hyc_nf4_weight* w4, int T, int H, int I,
     const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
     const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
     const void* s1, const void* s2, void* q1, void* q2, void* o, void* main1_or_null, void* main2_or_null,
     int q_bit, int* status, void* stream) {
-  if (!x || !wg || !wu || !xa1 || !b1t || !xa2 || !b2t || !s1 || !s2 || !q1 || !q2 || !o || !status) return HYC_ERR_NULL;
+  if (!x || (!w4 && (!wg || !wu)) || !xa1 || !b1t || !xa2 || !b2t || !s1 || !s2 || !q1 || !q2 || !o || !status) return HYC_ERR_NULL;
   if (q_bit != 2 && q_bit != 4 && q_bit != 8) return HYC_ERR_QBIT;
   if (T <= 0 || H <= 0 || I <= 0 || I % (BN / 2) != 0 || H % BK != 0) return HYC_ERR_SHAPE;
+  if (w4 && (!four_takes(w4[0], T, H) || !four_takes(w4[1], T, H))) return HYC_ERR_UNSUPPORTED;
   const void* al[] = {x, wg, wu, xa1, xa2, q1, q2, o};
   for (const void* q : al) if (!aligned(q, 16)) return HYC_ERR_ALIGN;
   Operands ops = {};
   ops.a[0] = {x, T, H};
   ops.b[0] = {wg, I, H};
   ops.b[1] = {wu, I, H};
+  FourWeights four = {};
+  if (w4) { four.w[0] = four_view(w4[0], H); four.w[1] = four_view(w4[1], H); }
+  const FourWeights* f4 = w4 ? &four : nullptr;
   Params p = {};
   p.M = T; p.N = I; p.K1 = H; p.K2 = 0; p.K3 = 0; p.epi = EPI_GATEUP; p.q_bit = q_bit;
   p.l0 = make_term(xa1, b1t, b1_ld_col, b1_ld_r);
@@ -799,20 +841,42 @@ extern "C" HYC_API int hyc_mlp_gateup_fwd_tcgen05(
   p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
   p.g_end0 = p.g_end1 = I;
-  if (q_bit == 2) return launch<EPI_GATEUP, 2, false>(ops, p, st);
-  if (q_bit == 4) return launch<EPI_GATEUP, 4, false>(ops, p, st);
-  return launch<EPI_GATEUP, 8, false>(ops, p, st);
+  if (q_bit == 2) return launch<EPI_GATEUP, 2, false>(ops, p, st, f4);
+  if (q_bit == 4) return launch<EPI_GATEUP, 4, false>(ops, p, st, f4);
+  return launch<EPI_GATEUP, 8, false>(ops, p, st, f4);
 }
 
-extern "C" HYC_API int hyc_mlp_graddown_bwd_tcgen05(
-    const void* g, const void* wd, int T, int H, int I,
+extern "C" HYC_API int hyc_mlp_gateup_fwd_tcgen05(
+    const void* x, const void* wg, const void* wu,
+    int T, int H, int I,
+    const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
+    const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
+    const void* s1, const void* s2, void* q1, void* q2, void* o, void* main1_or_null, void* main2_or_null,
+    int q_bit, int* status, void* stream) {
+  return gateup_fwd(x, wg, wu, nullptr, T, H, I, xa1, b1t, b1_ld_col, b1_ld_r, xa2, b2t, b2_ld_col, b2_ld_r, s1, s2, q1, q2, o,
+                    main1_or_null, main2_or_null, q_bit, status, stream);
+}
+extern "C" HYC_API int hyc_mlp_gateup_fwd_nf4_tcgen05(
+    const void* x, const hyc_nf4_weight* gate_up,
+    int T, int H, int I,
+    const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
+    const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
+    const void* s1, const void* s2, void* q1, void* q2, void* o, void* main1_or_null, void* main2_or_null,
+    int q_bit, int* status, void* stream) {
+  if (!gate_up) return HYC_ERR_NULL;
+  return gateup_fwd(x, nullptr, nullptr, gate_up, T, H, I, xa1, b1t, b1_ld_col, b1_ld_r, xa2, b2t, b2_ld_col, b2_ld_r, s1, s2, q1, q2, o,
+                    main1_or_null, main2_or_null, q_bit, status, stream);
+}
+
+static int graddown_bwd(
+    const void* g, const void* wd, const hyc_nf4_weight* w4, int T, int H, int I,
     const void* a_lora, const void* b_lora, int k_lora,
     const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
     const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
     const void* q1, const void* s1, const void* q2, const void* s2,
     const void* lora_gate, const void* lora_up, int64_t ld_lora,
     void* o, void* grad_gate, void* grad_up, int q_bit, int* status, void* stream) {
-  if (!g || !wd || !q1 || !s1 || !q2 || !s2 || !o || !grad_gate || !grad_up || !status) return HYC_ERR_NULL;
+  if (!g || (!w4 && !wd) || !q1 || !s1 || !q2 || !s2 || !o || !grad_gate || !grad_up || !status) return HYC_ERR_NULL;
   const bool pre = lora_gate != nullptr || lora_up != nullptr;
   if (pre) {
     if (!lora_gate || !lora_up) return HYC_ERR_NULL;
@@ -824,6 +888,7 @@ extern "C" HYC_API int hyc_mlp_graddown_bwd_tcgen05(
   if ((k_lora > 0) != (a_lora != nullptr && b_lora != nullptr)) return HYC_ERR_NULL;
   if (q_bit != 2 && q_bit != 4 && q_bit != 8) return HYC_ERR_QBIT;
   if (T <= 0 || H <= 0 || I <= 0 || I % BN != 0 || H % BK != 0 || k_lora < 0 || k_lora % BK != 0) return HYC_ERR_SHAPE;
+  if (w4 && !four_takes(*w4, T, I)) return HYC_ERR_UNSUPPORTED;
   const void* al[] = {g, wd, q1, q2, o, grad_gate, grad_up};
   for (const void* q : al) if (!aligned(q, 16)) return HYC_ERR_ALIGN;
   if (!pre && (!aligned(xa1, 16) || !aligned(xa2, 16))) return HYC_ERR_ALIGN;
@@ -832,6 +897,9 @@ extern "C" HYC_API int hyc_mlp_graddown_bwd_tcgen05(
   ops.a[0] = {g, T, H};
   ops.b[0] = {wd, H, I};      // [H, I] row-major: the K = H rows are the reduction dimension, so B is MN-major
   if (k_lora > 0) { ops.a[1] = {a_lora, T, k_lora}; ops.b[1] = {b_lora, k_lora, I}; }
+  FourWeights four = {};
+  if (w4) four.w[0] = four_view(*w4, I);
+  const FourWeights* f4 = w4 ? &four : nullptr;
   Params p = {};
   p.M = T; p.N = I; p.K1 = H; p.K2 = k_lora; p.K3 = 0; p.epi = EPI_GRADDOWN; p.q_bit = q_bit;
   p.l0 = make_term(nullptr, nullptr, 0, 0);
@@ -844,28 +912,58 @@ extern "C" HYC_API int hyc_mlp_graddown_bwd_tcgen05(
   p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
   p.g_end0 = p.g_end1 = I;
-  if (q_bit == 2) return launch<EPI_GRADDOWN, 2, true>(ops, p, st);
-  if (q_bit == 4) return launch<EPI_GRADDOWN, 4, true>(ops, p, st);
-  return launch<EPI_GRADDOWN, 8, true>(ops, p, st);
+  if (q_bit == 2) return launch<EPI_GRADDOWN, 2, true>(ops, p, st, f4);
+  if (q_bit == 4) return launch<EPI_GRADDOWN, 4, true>(ops, p, st, f4);
+  return launch<EPI_GRADDOWN, 8, true>(ops, p, st, f4);
+}
+
+extern "C" HYC_API int hyc_mlp_graddown_bwd_tcgen05(
+    const void* g, const void* wd,
+    int T, int H, int I,
+    const void* a_lora, const void* b_lora, int k_lora,
+    const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
+    const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
+    const void* q1, const void* s1, const void* q2, const void* s2,
+    const void* lora_gate, const void* lora_up, int64_t ld_lora,
+    void* o, void* grad_gate, void* grad_up, int q_bit, int* status, void* stream) {
+  return graddown_bwd(g, wd, nullptr, T, H, I, a_lora, b_lora, k_lora, xa1, b1t, b1_ld_col, b1_ld_r, xa2, b2t, b2_ld_col, b2_ld_r, q1, s1, q2, s2,
+                      lora_gate, lora_up, ld_lora, o, grad_gate, grad_up, q_bit, status, stream);
+}
+extern "C" HYC_API int hyc_mlp_graddown_bwd_nf4_tcgen05(
+    const void* g, const hyc_nf4_weight* down,
+    int T, int H, int I,
+    const void* a_lora, const void* b_lora, int k_lora,
+    const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
+    const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
+    const void* q1, const void* s1, const void* q2, const void* s2,
+    const void* lora_gate, const void* lora_up, int64_t ld_lora,
+    void* o, void* grad_gate, void* grad_up, int q_bit, int* status, void* stream) {
+  if (!down) return HYC_ERR_NULL;
+  return graddown_bwd(g, nullptr, down, T, H, I, a_lora, b_lora, k_lora, xa1, b1t, b1_ld_col, b1_ld_r, xa2, b2t, b2_ld_col, b2_ld_r, q1, s1, q2, s2,
+                      lora_gate, lora_up, ld_lora, o, grad_gate, grad_up, q_bit, status, stream);
 }
 
 // The LoRA projections of up to three weights on one x, with the saves of their main branches, in ONE launch: the tiles
 // of all weights are dealt out together (separately every launch ends with a round of tiles that leaves SMs idle).
-extern "C" HYC_API int hyc_linears_lora_save_fwd_tcgen05(
-    const void* x, int T, int K, int count, const void* const* w, const int* n, const void* const* xa, const void* const* bt,
+static int linears_lora_save(
+    const void* x, int T, int K, int count, const void* const* w, const hyc_nf4_weight* w4, const int* n, const void* const* xa, const void* const* bt,
     const void* const* scale, void* const* q_out, void* const* y, int q_bit, int* status, void* stream) {
-  if (!x || !w || !n || !xa || !bt || !scale || !q_out || !y || !status) return HYC_ERR_NULL;
+  if (!x || (!w && !w4) || !n || !xa || !bt || !scale || !q_out || !y || !status) return HYC_ERR_NULL;
   if (q_bit != 2 && q_bit != 4 && q_bit != 8) return HYC_ERR_QBIT;
   if (count < 1 || count > 3 || T <= 0 || K <= 0 || K % BK != 0) return HYC_ERR_SHAPE;
   if (!aligned(x, 16)) return HYC_ERR_ALIGN;
   int total = 0;
   Operands ops = {};
+  FourWeights four = {};
   ops.a[0] = {x, T, K};
   for (int i = 0; i < count; ++i) {
-    if (!w[i] || !xa[i] || !bt[i] || !scale[i] || !q_out[i] || !y[i]) return HYC_ERR_NULL;
+    const bool coded = has_four(w4, i);
+    if ((!coded && (!w || !w[i])) || !xa[i] || !bt[i] || !scale[i] || !q_out[i] || !y[i]) return HYC_ERR_NULL;
     if (n[i] <= 0 || n[i] % BN != 0) return HYC_ERR_SHAPE;
-    if (!aligned(w[i], 16) || !aligned(xa[i], 16) || !aligned(q_out[i], 16) || !aligned(y[i], 16)) return HYC_ERR_ALIGN;
-    ops.b[i] = {w[i], n[i], K};
+    if (coded && !four_takes(w4[i], T, K)) return HYC_ERR_UNSUPPORTED;
+    if ((!coded && !aligned(w[i], 16)) || !aligned(xa[i], 16) || !aligned(q_out[i], 16) || !aligned(y[i], 16)) return HYC_ERR_ALIGN;
+    if (coded) four.w[i] = four_view(w4[i], K);
+    else ops.b[i] = {w[i], n[i], K};
     total += n[i];
   }
   Params p = {};
@@ -879,9 +977,22 @@ extern "C" HYC_API int hyc_linears_lora_save_fwd_tcgen05(
     *g[i - 1] = {(__nv_bfloat16*)y[i], (uint8_t*)q_out[i], (const __nv_bfloat16*)scale[i], make_term(xa[i], bt[i], 16, 1)};
   p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
-  if (q_bit == 2) return launch<EPI_STORE, 2, false>(ops, p, st);
-  if (q_bit == 4) return launch<EPI_STORE, 4, false>(ops, p, st);
-  return launch<EPI_STORE, 8, false>(ops, p, st);
+  const FourWeights* f4 = w4 ? &four : nullptr;
+  if (q_bit == 2) return launch<EPI_STORE, 2, false>(ops, p, st, f4);
+  if (q_bit == 4) return launch<EPI_STORE, 4, false>(ops, p, st, f4);
+  return launch<EPI_STORE, 8, false>(ops, p, st, f4);
+}
+
+extern "C" HYC_API int hyc_linears_lora_save_fwd_tcgen05(
+    const void* x, int T, int K, int count, const void* const* w, const int* n, const void* const* xa, const void* const* bt,
+    const void* const* scale, void* const* q_out, void* const* y, int q_bit, int* status, void* stream) {
+  return linears_lora_save(x, T, K, count, w, nullptr, n, xa, bt, scale, q_out, y, q_bit, status, stream);
+}
+extern "C" HYC_API int hyc_linears_lora_save_fwd_nf4_tcgen05(
+    const void* x, int T, int K, int count, const void* const* w, const hyc_nf4_weight* w4, const int* n, const void* const* xa,
+    const void* const* bt, const void* const* scale, void* const* q_out, void* const* y, int q_bit, int* status, void* stream) {
+  if (!w4) return HYC_ERR_NULL;
+  return linears_lora_save(x, T, K, count, w, w4, n, xa, bt, scale, q_out, y, q_bit, status, stream);
 }
 
 extern "C" HYC_API int hyc_linear_lora_save_fwd_tcgen05(

@@ -8,6 +8,16 @@
 // from L2.  With 129 tokens and more the tile belongs to a CTA pair (M 256, tcgen05 cta_group::2, each CTA loading half
 // of the B block), which cuts what an SM pulls out of L2 per k-block from 32 to 24 KB; a cluster is then 2 S CTAs.
 // The reduction order is fixed (rank 0, 1, ...), so results do not depend on the run.
+//
+// FOUR: frozen weights that are 4-bit codes.  Up to 128 rows every element of a weight is read by one CTA alone, so that decoding it there
+// costs no more than decoding it once, and what a launch of its own would write and the product read back, 2 + 2 bytes per element, is not
+// moved at all.  Eight warps write the B blocks where TMA would have put them, two k-blocks at a time, a thread the 64 elements of a
+// 128-byte row (32 bytes of codes under one scale): the sixteen values that a scale makes of the table as byte planes in registers, then
+// byte permutes (3.7 instructions per element).  Bound by instructions (issue slots 0.37, two and a half warps per scheduler) and by the
+// requests for codes and scales, 32 and 4 bytes per thread from rows of their own: 0.65 us per k-block, 0.59 without the arithmetic, 0.42
+// without the requests.  The products of a layer of 128 tokens that take codes, us: 395 as de-quantizing launches and products, 328 so; the layer
+// 577 -> 517 to 538 (its host work takes about as long).  More codes in flight (cp.async, eight slots), sixteen warps, and addresses carried
+// from block to block gave nothing or cost some.  Which products: see weights() in host/host_blocks.cpp.
 #include "tc_split.cuh"
 
 namespace hyc {
@@ -50,10 +60,66 @@ __device__ __forceinline__ void gather32(int split, int first, int step, uint32_
   for (int c = 0; c < 32; ++c) acc[c] = __float_as_uint(f[c]);
 }
 
-template <int EPI, int QBIT, bool B_MN, bool PAIR>
-__global__ void __launch_bounds__(S_THREADS, 2)
-split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, int stages, int a_bytes) {
-  static_assert(EPI == EPI_STORE || (EPI == EPI_GATEUP && !PAIR && !B_MN), "the forms that choose_split picks");
+// ---- 4-bit weights
+constexpr int S_FOUR_WARPS = 8, S_FOUR_AT = 512;      // decoding warps; where the tables lie in the epilogue's constants
+static_assert(S_FOUR_AT + 4 * 64 <= S_EPI_BYTES, "the tables fit behind the constants");
+// 64 elements on their way: their codes and what makes their scale
+struct FourUnit {
+  uint32_t w[8];
+  float s, c;                               // absmax; two-level: the second-level factor and the table value
+  uint32_t q;                               // two-level: the code
+  int which;                                // weight, -1: nothing to decode
+};
+__device__ __forceinline__ void four_fetch(const FourView& v, int which, int64_t e, FourUnit& u) {
+  asm volatile("ld.global.L2::128B.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]), "=r"(u.w[4]), "=r"(u.w[5]), "=r"(u.w[6]), "=r"(u.w[7]) : "l"(v.packed + e / 2));
+  const int64_t blk = e >> v.shift;
+  u.which = which;
+  u.q = 0u;
+  if (v.absmax) {
+    u.s = v.absmax[blk];
+  } else {
+    u.q = v.absmax_q[blk];
+    u.s = v.absmax2[blk >> v.shift2];
+  }
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {      // bit 3 of a selector: the byte's sign, eight times
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+// to the 128-byte row at `row`, whose 16-byte chunks lie permuted by `swz`
+__device__ __forceinline__ void four_decode(const FourUnit& u, float s, const float* code, uint8_t* row, int swz) {
+  uint32_t lo[4], hi[4];                    // the low and the high bytes of the sixteen values
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 c = *reinterpret_cast<const float4*>(code + 4 * i);
+    const uint32_t a = pack_bf16x2_rn(__fmul_rn(c.x, s), __fmul_rn(c.y, s)), b = pack_bf16x2_rn(__fmul_rn(c.z, s), __fmul_rn(c.w, s));
+    lo[i] = prmt(a, b, 0x6420u);
+    hi[i] = prmt(a, b, 0x7531u);
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const uint32_t sel = u.w[c] & 0x77777777u, z = u.w[c] << 4;
+    uint32_t o[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      // four codes, the low nibble of a byte before the high one; which of them are in the upper half of the table
+      const uint32_t k = h ? sel >> 16 : sel, up = prmt(u.w[c], z, h ? 0xbfaeu : 0x9d8cu);
+      const uint32_t l = (prmt(lo[0], lo[1], k) & ~up) | (prmt(lo[2], lo[3], k) & up);
+      const uint32_t m = (prmt(hi[0], hi[1], k) & ~up) | (prmt(hi[2], hi[3], k) & up);
+      o[2 * h] = prmt(l, m, 0x4051u);       // (the high nibble is the first element)
+      o[2 * h + 1] = prmt(l, m, 0x6273u);
+    }
+    *reinterpret_cast<uint4*>(row + ((c ^ swz) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+template <int EPI, int QBIT, bool B_MN, bool PAIR, bool FOUR>
+__global__ void __launch_bounds__(FOUR ? 64 + 32 * S_FOUR_WARPS : S_THREADS, 2)
+split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, int stages, int a_bytes, const __grid_constant__ FourWeights four) {
+  static_assert(EPI == EPI_STORE || (EPI == EPI_GATEUP && !PAIR && !B_MN) || (EPI == EPI_GRADDOWN && FOUR && B_MN), "the forms that are launched");
+  static_assert(!(FOUR && PAIR), "a pair would decode everything twice");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align_shared(smem_raw);
   constexpr int TILE_M = PAIR ? 2 * BM : BM;
@@ -79,12 +145,17 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
   const StoreView sv = store_view(p, nt);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    // (FOUR: a B block is there when the four warps that decode it have arrived)
+    for (int s = 0; s < stages; ++s) { mbar_init(&full[s], FOUR ? 1 + S_FOUR_WARPS / 2 : 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   pdl_wait();      // before tensor memory is taken: see launch_pdl
+  if (FOUR && threadIdx.x >= 64 && threadIdx.x < 64 + 64) {
+    const int i = (int)threadIdx.x - 64;
+    if (four.w[i >> 4].packed != nullptr) reinterpret_cast<float*>(epi + S_FOUR_AT)[i] = four.w[i >> 4].code16[i & 15];
+  }
   if (warp == 1) {
     if (PAIR) {
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(SBN) : "memory");
@@ -128,8 +199,10 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
         const uint32_t sa = smem_u32(smem + stage * stage_bytes), sb = sa + (uint32_t)a_bytes;
         const uint32_t fbar = PAIR ? map_to_cta(&full[stage], leader) : smem_u32(&full[stage]);
         if (elect_one()) {
-        if (half == 0) mbar_expect_tx(&full[stage], (uint32_t)((PAIR ? 2 : 1) * stage_bytes));      // the leader counts both CTAs' bytes
-        if (EPI == EPI_GATEUP) {
+        const bool decoded = FOUR && four.w[wsel].packed != nullptr;
+        if (half == 0) mbar_expect_tx(&full[stage], (uint32_t)((PAIR ? 2 : 1) * (decoded ? a_bytes : stage_bytes)));      // the leader counts both CTAs' bytes
+        if (decoded) {
+        } else if (EPI == EPI_GATEUP) {
           tma_load_2d<PAIR>(sb, &maps.b[0], fbar, k0, n0);
           tma_load_2d<PAIR>(sb + 8192, &maps.b[1], fbar, k0, n0);
         } else if (B_MN) {
@@ -176,8 +249,62 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
     }
     __syncwarp();
   } else {
+    if constexpr (FOUR) {
+      // warps 2..5 decode the even k-blocks of this CTA's share, warps 6..9 the odd ones; codes and scales are two blocks of theirs ahead
+      const int group = (warp - 2) >> 2, i = ((int)threadIdx.x - 64) & 127;
+      auto fetch = [&](int kb, FourUnit& u) {
+        u.which = -1;
+        if (kb >= kb_hi) return;
+        const int seg = kb < kb1 ? 0 : (kb < kb2 ? 1 : (kb < kb3 ? 2 : 3));
+        const int k0 = (kb - (seg == 0 ? 0 : (seg == 1 ? kb1 : (seg == 2 ? kb2 : kb3)))) * BK;
+        const int which = EPI == EPI_GATEUP ? i >> 6 : (EPI == EPI_STORE && sv.group > 0 ? sv.group : seg);
+        const FourView& v = four.w[which];
+        if (v.packed == nullptr) return;      // (TMA brings it)
+        const int n0 = EPI == EPI_STORE ? sv.n0 : nt;
+        if (B_MN) four_fetch(v, which, (int64_t)(k0 + (i >> 1)) * v.ld + n0 + 64 * (i & 1), u);
+        else four_fetch(v, which, (int64_t)(n0 + (EPI == EPI_GATEUP ? i & 63 : i)) * v.ld + k0, u);
+      };
+      auto table_value = [&](FourUnit& u) {
+        if (u.which >= 0 && four.w[u.which].absmax == nullptr) u.c = __ldg(four.w[u.which].code256 + u.q);
+      };
+      const float* code = reinterpret_cast<const float*>(epi + S_FOUR_AT);
+      const uint32_t row_at = B_MN ? (uint32_t)((i & 1) * 8192 + (i >> 1) * 128) : (uint32_t)(i * 128);
+      const int swz = B_MN ? (i >> 1) & 7 : i & 7;
+      int stage = group;
+      uint32_t phase = 0;
+      FourUnit n1, n2;
+      fetch(kb_lo + group, n1);
+      table_value(n1);
+      fetch(kb_lo + group + 2, n2);
+      for (int kb = kb_lo + group; kb < kb_hi; kb += 2) {
+        const FourUnit u = n1;
+        n1 = n2;
+        table_value(n1);
+        fetch(kb + 4, n2);
+        if (!mbar_wait_warp(&empty[stage], phase ^ 1u, abort_flag)) {
+          if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ST_TIMEOUT_PRODUCER); }
+          break;
+        }
+        if (u.which >= 0) {
+          const FourView& v = four.w[u.which];
+          const float s = v.absmax ? u.s : __fadd_rn(__fmul_rn(u.c, u.s), v.offset);
+          four_decode(u, s, code + 16 * u.which, smem + stage * stage_bytes + a_bytes + row_at, swz);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[stage]);
+        stage += 2;
+        if (stage >= stages) { stage -= stages; phase ^= 1u; }
+      }
+    }
+    if (!FOUR || warp < 6) {
     // what the epilogue needs besides the accumulators is fetched while the main loop runs
-    if (EPI == EPI_STORE) {
+    if (EPI == EPI_GRADDOWN) {
+      reinterpret_cast<__nv_bfloat16*>(sV)[et] = p.s1[nt + et];
+      reinterpret_cast<__nv_bfloat16*>(sV)[SBN + et] = p.s2[nt + et];
+      lora_load_a(p.l1.xa, row0, p.M, lane, a1);
+      lora_load_a(p.l2.xa, row0, p.M, lane, a2);
+    } else if (EPI == EPI_STORE) {
       if (sv.q != nullptr) sV[et] = fastq_scale<QBIT>(__frcp_rn(__bfloat162float(sv.s[sv.n0 + et])));
       if (sv.l0.bt != nullptr) {
         lora_load_a(sv.l0.xa, row0, p.M, lane, a1);
@@ -209,11 +336,12 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
         for (int c = 0; c < 32; ++c) part[(c0 + c) * BM + quad * 32 + lane] = __uint_as_float(v[c]);
       }
     }
+    }
   }
   // every CTA of the cluster has its partial sums in place (or has given up: the status word says so)
   if (split > 1) cluster_sync_all();
 
-  if (warp >= 2 && ok) {
+  if (warp >= 2 && warp < 6 && ok) {
     const uint32_t part_addr = smem_u32(part);
     const int r = quad * 32 + lane;
     // behind the partial sums
@@ -233,6 +361,12 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
         gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, cb, r, acc);
         gather32(split, half, PAIR ? 2 : 1, t_lane, part_addr, TILE_N + cb, r, up);
         epi_gateup_block<QBIT>(p, row0, lane, nt, cb, acc, up, a1, a2, n1, n2, sV, sV + 64, R1, R2);
+      } else if constexpr (EPI == EPI_GRADDOWN) {
+        GdInputs<QBIT> in;
+        gd_fetch<QBIT>(p, row0, lane, (int64_t)nt + cb, in);
+        gather32(split, half, 1, t_lane, part_addr, cb, r, acc);
+        epi_graddown_block<QBIT>(p, row0, lane, nt, cb, acc, in, a1, a2, R1, R2, reinterpret_cast<const uint32_t*>(sV),
+                                 reinterpret_cast<const uint32_t*>(sV) + SBN / 2);
       } else {
         const uint4 now[4] = {res[0], res[1], res[2], res[3]};
         const LoraB n1 = b1;
@@ -254,9 +388,9 @@ split_gemm_kernel(const __grid_constant__ Maps maps, const Params p, int split, 
   }
 }
 
-template <int EPI, int QBIT, bool B_MN, bool PAIR>
-static int launch_one(int split, const Operands& ops, const Params& p, cudaStream_t st) {
-  auto kern = split_gemm_kernel<EPI, QBIT, B_MN, PAIR>;
+template <int EPI, int QBIT, bool B_MN, bool PAIR, bool FOUR = false>
+static int launch_one(int split, const Operands& ops, const Params& p, cudaStream_t st, const FourWeights& four = {}) {
+  auto kern = split_gemm_kernel<EPI, QBIT, B_MN, PAIR, FOUR>;
   static bool attr[64] = {false};
   const int slot = current_device_slot();
   if (slot < 0 || !attr[slot]) {
@@ -274,7 +408,7 @@ static int launch_one(int split, const Operands& ops, const Params& p, cudaStrea
   const int stage_bytes = a_bytes + (PAIR ? SBN / 2 : SBN) * BK * 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(S_THREADS);
+  cfg.blockDim = dim3(FOUR ? 64 + 32 * S_FOUR_WARPS : S_THREADS);
   cfg.dynamicSmemBytes = split_smem_bytes(pipe);
   cfg.stream = st;
   cudaLaunchAttribute at[2];
@@ -286,9 +420,9 @@ static int launch_one(int split, const Operands& ops, const Params& p, cudaStrea
   cfg.numAttrs = cluster > 1 ? 2 : 1;
   int stages = pipe / stage_bytes;
   if (stages > S_MAX_STAGES) stages = S_MAX_STAGES;
-  Maps maps;
+  Maps maps = {};      // (FOUR: some weights have none)
   if (!make_maps(&maps, ops, B_MN, a_bytes / (BK * 2), EPI == EPI_GATEUP || PAIR ? 64 : 128, false)) return HYC_ERR_UNSUPPORTED;
-  if (cudaLaunchKernelEx(&cfg, kern, maps, p, split, stages, a_bytes) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, kern, maps, p, split, stages, a_bytes, four) != cudaSuccess) {
     hyc_set_last_cuda_error((int)cudaGetLastError());
     return HYC_ERR_LAUNCH;
   }
@@ -310,6 +444,27 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
   if (q_bit == 2) return launch_one<EPI_STORE, 2, false, false>(plan.split, ops, p, st);
   if (q_bit == 8) return launch_one<EPI_STORE, 8, false, false>(plan.split, ops, p, st);
   return launch_one<EPI_STORE, 4, false, false>(plan.split, ops, p, st);
+}
+
+// the split that a product of up to 128 rows has either way: the same sums for a weight as for its codes
+int launch_four(int epi, int q_bit, bool b_mn, const Operands& ops, const Params& p, const FourWeights& four, cudaStream_t st) {
+  if (p.M > BM) return HYC_ERR_UNSUPPORTED;
+  const SplitPlan plan = choose_split(epi, p);
+  const int split = plan.split > 0 ? plan.split : 1;
+  if (epi == EPI_GRADDOWN) {
+    if (q_bit == 2) return launch_one<EPI_GRADDOWN, 2, true, false, true>(split, ops, p, st, four);
+    if (q_bit == 8) return launch_one<EPI_GRADDOWN, 8, true, false, true>(split, ops, p, st, four);
+    return launch_one<EPI_GRADDOWN, 4, true, false, true>(split, ops, p, st, four);
+  }
+  if (epi == EPI_GATEUP) {
+    if (q_bit == 2) return launch_one<EPI_GATEUP, 2, false, false, true>(split, ops, p, st, four);
+    if (q_bit == 8) return launch_one<EPI_GATEUP, 8, false, false, true>(split, ops, p, st, four);
+    return launch_one<EPI_GATEUP, 4, false, false, true>(split, ops, p, st, four);
+  }
+  if (b_mn) return launch_one<EPI_STORE, 4, true, false, true>(split, ops, p, st, four);
+  if (q_bit == 2) return launch_one<EPI_STORE, 2, false, false, true>(split, ops, p, st, four);
+  if (q_bit == 8) return launch_one<EPI_STORE, 8, false, false, true>(split, ops, p, st, four);
+  return launch_one<EPI_STORE, 4, false, false, true>(split, ops, p, st, four);
 }
 
 // Where the line lies (B200, Llama-2-7B weights, us per product, persistent / split):

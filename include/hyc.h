@@ -323,6 +323,19 @@ typedef struct hyc_nf4_job {
 } hyc_nf4_job;
 int hyc_dequant_nf4_many(int count, const hyc_nf4_job* jobs, void* stream);
 
+/* A weight [rows, cols] in that form as an operand: products of up to 128 rows (hyc_nf4_product_supported: cols % 64 == 0, block sizes
+ * powers of two, at least 64 elements under a scale, packed 32-byte aligned) decode it on its way in.  The *_nf4_tcgen05 entries are
+ * their namesakes without the suffix, with the same results for the same weights; where `packed` is NULL the bf16 matrix counts. */
+typedef struct hyc_nf4_weight {
+  const void* packed;
+  const float *code16, *absmax;      /* absmax NULL: double quantization */
+  const uint8_t* absmax_q;
+  const float *code256, *absmax2;
+  int blocksize, blocksize2;
+  float offset;
+} hyc_nf4_weight;
+int hyc_nf4_product_supported(const hyc_nf4_weight* w, int rows, int cols);
+
 /* ---- tcgen05 / TMEM GEMMs of the LoRA MLP (activation compression in the epilogue) ------------
  * bf16 operands, fp32 accumulation in tensor memory, operands staged by TMA.  `status` is a
  * caller-provided device int, zero before the call; a non-zero value afterwards means a bounded
@@ -352,6 +365,8 @@ int hyc_gemm_bf16_tcgen05(const void* A, const void* B, int M, int N, int K, int
 /* The same without LoRA terms for one to four (A, B) pairs: host arrays of `count` entries, A[i] [M, K[i]]. */
 int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
                               int form, const void* residual_or_null, void* D, int* status, void* stream);
+int hyc_gemm_segments_nf4_tcgen05(int count, const void* const* A, const void* const* B, const hyc_nf4_weight* B4, const int* K, int M, int N,
+                              int form, const void* residual_or_null, void* D, int* status, void* stream);
 
 /* A LoRA projection with the save of its main branch in the GEMM epilogue (the q/k/v/o projections of the
  * attention half: `lora_forward` followed by `compression_pack_quant_base(x=q_main, ...)`,
@@ -371,6 +386,9 @@ int hyc_linear_lora_save_fwd_tcgen05(const void* x, const void* w, int T, int K,
 int hyc_linears_lora_save_fwd_tcgen05(const void* x, int T, int K, int count, const void* const* w, const int* n,
                                       const void* const* xa, const void* const* bt, const void* const* scale,
                                       void* const* q_out, void* const* y, int q_bit, int* status, void* stream);
+int hyc_linears_lora_save_fwd_nf4_tcgen05(const void* x, int T, int K, int count, const void* const* w, const hyc_nf4_weight* w4, const int* n,
+                                      const void* const* xa, const void* const* bt, const void* const* scale,
+                                      void* const* q_out, void* const* y, int q_bit, int* status, void* stream);
 
 /* gate/up projections and triton_fuse_silu_forward in one kernel
  * (fused_llama_layer_intra_inter_full_fuse.py:218-235 + triton_fuse_lora_silu_hadamard_forward_kernels.py):
@@ -379,6 +397,11 @@ int hyc_linears_lora_save_fwd_tcgen05(const void* x, int T, int K, int count, co
  * x [T,H], wg/wu [I,H], s1/s2 [I] bf16, q1/q2 [T, I*q_bit/8], o [T,I].  I % 128 == 0, H % 64 == 0.
  * main1/main2 (optional, [T,I] bf16) receive the bf16 main branches for inspection. */
 int hyc_mlp_gateup_fwd_tcgen05(const void* x, const void* wg, const void* wu, int T, int H, int I,
+                               const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
+                               const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
+                               const void* s1, const void* s2, void* q1, void* q2, void* o,
+                               void* main1_or_null, void* main2_or_null, int q_bit, int* status, void* stream);
+int hyc_mlp_gateup_fwd_nf4_tcgen05(const void* x, const hyc_nf4_weight* gate_up, int T, int H, int I,
                                const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
                                const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
                                const void* s1, const void* s2, void* q1, void* q2, void* o,
@@ -396,6 +419,13 @@ int hyc_mlp_gateup_fwd_tcgen05(const void* x, const void* wg, const void* wu, in
  * or read from lora_gate / lora_up ([T, ld_lora] bf16, ld_lora >= I, a multiple of 8), which one launch of
  * hyc_gemm_bf16_tcgen05 on the zero-padded rank-16 operands prepares; xa1/b1t/xa2/b2t may then be NULL. */
 int hyc_mlp_graddown_bwd_tcgen05(const void* g, const void* wd, int T, int H, int I,
+                                 const void* a_lora, const void* b_lora, int k_lora,
+                                 const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
+                                 const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
+                                 const void* q1, const void* s1, const void* q2, const void* s2,
+                                 const void* lora_gate, const void* lora_up, int64_t ld_lora,
+                                 void* o, void* grad_gate, void* grad_up, int q_bit, int* status, void* stream);
+int hyc_mlp_graddown_bwd_nf4_tcgen05(const void* g, const hyc_nf4_weight* down, int T, int H, int I,
                                  const void* a_lora, const void* b_lora, int k_lora,
                                  const void* xa1, const void* b1t, int64_t b1_ld_col, int64_t b1_ld_r,
                                  const void* xa2, const void* b2t, int64_t b2_ld_col, int64_t b2_ld_r,
