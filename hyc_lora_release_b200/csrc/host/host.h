@@ -6,6 +6,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <array>
 #include <initializer_list>
 #include <optional>
 #include <stdexcept>
@@ -49,6 +50,27 @@ inline Tensor vec(const Tensor& s) {
 }
 inline Tensor empty(at::IntArrayRef sz, const Tensor& like, at::ScalarType ty = at::kBFloat16) {
   return at::detail::empty_cuda(sz, ty, like.device(), std::nullopt);
+}
+// Results that are kept and dropped together, in one allocation (an allocation and its release cost the host 0.8 us, a tensor more on
+// the same storage 0.2; a layer step made seventy).  Each starts on a 256-byte boundary, none overlap.
+struct Want { at::DimVector sizes; at::ScalarType type; };
+template <size_t N>
+std::array<Tensor, N> together(const Tensor& like, const Want (&wants)[N]) {
+  int64_t at[N], bytes = 0;
+  for (size_t i = 0; i < N; ++i) {
+    at[i] = bytes;
+    bytes += (c10::multiply_integers(wants[i].sizes) * (int64_t)c10::elementSize(wants[i].type) + 255) / 256 * 256;
+  }
+  const Tensor all = empty({bytes}, like, at::kByte);
+  std::array<Tensor, N> out;
+  for (size_t i = 0; i < N; ++i) {
+    out[i] = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(all.storage()), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                      c10::scalarTypeToTypeMeta(wants[i].type));
+    c10::TensorImpl* t = out[i].unsafeGetTensorImpl();
+    t->set_storage_offset(at[i] / (int64_t)c10::elementSize(wants[i].type));
+    t->set_sizes_contiguous(wants[i].sizes);
+  }
+  return out;
 }
 inline void* data(const Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr; }
 inline void* data(const OptTensor& t) { return given(t) ? data(*t) : nullptr; }

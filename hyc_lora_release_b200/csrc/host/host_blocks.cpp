@@ -128,6 +128,10 @@ static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, c
   OnDevice on(x);
   const int64_t T = x.size(0), K = x.size(1);
   std::array<std::pair<Tensor, Tensor>, 3> out;
+  const int64_t n0 = w[0].size(0), n1 = w[1].size(0), n2 = w[2].size(0);
+  // (the projections themselves are gone behind the attention kernel, the codes stay for the backward pass)
+  const auto y3 = together(x, {{{T, n0}, at::kBFloat16}, {{T, n1}, at::kBFloat16}, {{T, n2}, at::kBFloat16}});
+  const auto q3 = together(x, {{{T, n0 * q_bit / 8}, at::kByte}, {{T, n1 * q_bit / 8}, at::kByte}, {{T, n2 * q_bit / 8}, at::kByte}});
   Tensor keep[6];
   const void *wp[3], *xp[3], *bp[3], *sp[3];
   void *qp[3], *yp[3];
@@ -136,7 +140,7 @@ static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, c
   for (int i = 0; i < 3; ++i) {
     n[i] = (int)w[i].size(0);
     codes[i] = w[i].codes();
-    out[i] = {empty({T, n[i]}, x), empty({T, n[i] * q_bit / 8}, x, at::kByte)};
+    out[i] = {y3[i], q3[i]};
     keep[2 * i] = vec(*scale[i]);
     keep[2 * i + 1] = factor(*b[i]);
     wp[i] = data(w[i].m); xp[i] = (const char*)xa3.data_ptr() + i * T * 16 * 2; bp[i] = data(keep[2 * i + 1]); sp[i] = data(keep[2 * i]);
@@ -236,7 +240,8 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   const Tensor xn2 = x_norm.view({T, H});
   const Tensor gu_xa = lora_a_products(xn2, agu_t);
   const char* xa = (const char*)gu_xa.data_ptr();
-  Tensor q1 = empty({B, M, I * q / 8}, x_norm, at::kByte), q2 = empty({B, M, I * q / 8}, x_norm, at::kByte), had = empty({T, I}, x_norm);
+  const auto [q1, q2] = together(x_norm, {{{B, M, I * q / 8}, at::kByte}, {{B, M, I * q / 8}, at::kByte}});
+  const Tensor had = empty({T, I}, x_norm);
   if (wg.f) {
     const hyc_nf4_weight codes[2] = {wg.codes(), wu.codes()};
     check(hyc_mlp_gateup_fwd_nf4_tcgen05(data(xn2), codes, (int)T, (int)H, (int)I, xa, data(bg), 16, 1, xa + T * 16 * 2, data(bu), 16, 1, data(gs),
@@ -272,8 +277,8 @@ static std::vector<Tensor> mlp_backward_lora(const Tensor& g, const Weight& wd, 
   SameDevice{g}.with(wd.m).with(w).with(saved).with(status);
   OnDevice on(g);
   const Tensor bg = factor(w[1]), bu = factor(w[2]), bd = factor(w[3]);
-  Tensor grad_bd = empty({H, 16}, g), gdm64 = empty({T, 64}, g), gm64 = empty({T, 64}, g), grad_ad = empty({16, I}, g),
-         grad_bgu = empty({2, I, 16}, g);
+  const auto [gdm64, gm64] = together(g, {{{T, 64}, at::kBFloat16}, {{T, 64}, at::kBFloat16}});
+  Tensor grad_bd = empty({H, 16}, g), grad_ad = empty({16, I}, g), grad_bgu = empty({2, I, 16}, g);
   Skinny().on(g).rows(data(bd), 16, gdm64, 0, 64, 48).cols(data(down_xa), down_xa.stride(0), data(grad_bd)).run(T, g, status, on.stream);
   Tensor had = empty({T, I}, g), ggu = empty({2, T, I}, g);
   char* gp = (char*)ggu.data_ptr();
@@ -486,13 +491,13 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
   const double scale = 1.0 / std::sqrt((double)d);
   if (attn_kernels_take(M, d)) {
     // q, k (rotated) and v from their codes in one launch
-    Tensor rebuilt[3], keep[9];
+    const auto rebuilt = together(grad_o2, {{{T, nh * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}});
+    Tensor keep[9];
     const void *cp[3], *sp[3], *xp[3], *bp[3];
     void* yp[3];
     int n[3];
     for (int i = 0; i < 3; ++i) {
       n[i] = (int)((i == 0 ? nh : nkv) * d);
-      rebuilt[i] = empty({T, n[i]}, grad_o2);
       cp[i] = data(keep[3 * i] = saved[3 * i].contiguous()); sp[i] = data(keep[3 * i + 1] = vec(saved[3 * i + 1]));
       xp[i] = data(saved[3 * i + 2]); bp[i] = data(keep[3 * i + 2] = factor(w[i])); yp[i] = data(rebuilt[i]);
     }
@@ -500,7 +505,7 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
           "hyc_rebuild_qkv");
     const Tensor &q2 = rebuilt[0], &k2 = rebuilt[1], &v2 = rebuilt[2];
     Tensor gs = empty({B, nh, M, M}, grad_o2);
-    Tensor gq = empty({T, nh * d}, grad_o2), gk = empty({T, nkv * d}, grad_o2), gv = empty({T, nkv * d}, grad_o2);
+    const auto [gq, gk, gv] = together(grad_o2, {{{T, nh * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}});
     check(hyc_attn_bwd_tcgen05(data(q2), data(k2), data(v2), data(grad_o2), data(a), data(gs), (int)B, (int)M, (int)nh, (int)nkv, (int)d,
                                (float)scale, data(cls), cls_b, cls_h, data(gq), data(gk), data(gv), status_ptr(status), on.stream),
           "hyc_attn_bwd_tcgen05");

@@ -127,8 +127,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x
   const int64_t S = row_length(x), rows = x.numel() / S;
   require_cuda({&x});
   check_q(q_bit);
-  Tensor val = empty({rows, k}, x), col = empty({rows, k}, x, at::kShort), q = empty({rows, S * q_bit / 8}, x, at::kByte),
-         s = empty({rows, S / 64}, x), z = empty({rows, S / 64}, x, at::kChar);
+  const auto [q, val, col, s, z] = together(x, {{{rows, S * q_bit / 8}, at::kByte}, {{rows, k}, at::kBFloat16}, {{rows, k}, at::kShort},
+                                                {{rows, S / 64}, at::kBFloat16}, {{rows, S / 64}, at::kChar}});
   if (row_cols.defined()) {
     OnDevice on(x);
     check(hyc_softmax_topk_compress_cols(data(x), rows, (int)S, (const uint16_t*)data(row_cols), (int)k, k ? data(val) : nullptr,
@@ -221,8 +221,8 @@ std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int6
   OnDevice on(x);
   const Tensor xf = bf16c(x);
   const int64_t numel = xf.numel();
-  Tensor nnz = empty({1}, x, at::kLong), words = empty({capacity}, x, at::kInt),
-         dir = empty({(int64_t)(hyc_softmax_prune_tiled_directory_bytes(numel) / 4)}, x, at::kInt);
+  const auto [dir, nnz, words] = together(x, {{{(int64_t)(hyc_softmax_prune_tiled_directory_bytes(numel) / 4)}, at::kInt}, {{1}, at::kLong},
+                                              {{capacity}, at::kInt}});
   if (row_cols.defined())
     check(hyc_softmax_prune_tiled_cols(data(xf), numel, (int)x.size(-1), (const uint16_t*)data(row_cols), (float)thr, (uint32_t*)data(words), capacity,
                                        data(dir), (int64_t*)data(nnz), on.stream), "hyc_softmax_prune_tiled_cols");
@@ -247,8 +247,10 @@ Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::Int
 
 // ---- fused LoRA-SiLU-Hadamard
 // [R, N] LoRA-B operand -> the [N, R] row-major matrix the kernels read; ``lora_B.weight.T`` is a view of exactly that storage
+// (only its memory is read)
 static Tensor b_transposed(const Tensor& b) {
   TORCH_CHECK_VALUE(b.dim() == 2, "LoRA B must be [R, N]");
+  if (b.scalar_type() == at::kBFloat16 && b.stride(0) == 1 && b.stride(1) == b.size(0)) return b;
   return b.t().to(at::kBFloat16).contiguous();
 }
 
@@ -316,12 +318,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor&
   if (given(idx_in)) { idx = index_of(*idx_in, x); k = idx.numel(); }
   if (given(sy_in)) sy = scale_vec(*sy_in, N);
   TORCH_CHECK_VALUE(w.numel() == N, "norm weight with ", w.numel(), " entries for ", N, " channels");
-  std::vector<int64_t> qs(xc.sizes().begin(), xc.sizes().end()), os = qs;
+  at::DimVector qs(xc.sizes()), os = qs, none = {0};
   qs.back() = N * q_bit / 8;
   os.back() = k;
-  Tensor y = empty(xc.sizes(), x), rstd = empty({rows}, x, at::kFloat), qx = empty(qs, x, at::kByte), xo = empty(os, x);
+  const Tensor y = empty(xc.sizes(), x);
+  const auto [rstd, qx, xo, codes_y] = together(x, {{{rows}, at::kFloat}, {qs, at::kByte}, {os, at::kBFloat16}, {sy.defined() ? qs : none, at::kByte}});
   OptTensor qy;
-  if (sy.defined()) qy = empty(qs, x, at::kByte);
+  if (sy.defined()) qy = codes_y;
   if (rows)
     check(hyc_rmsnorm_fwd_save(data(xc), data(w), (float)eps, rows, (int)N, data(sx), k ? (const int64_t*)data(idx) : nullptr, (int)k,
                                data(sy), data(y), (float*)data(rstd), data(qx), k ? data(xo) : nullptr, data(qy), (int)q_bit, on.stream),
