@@ -51,11 +51,19 @@ inline Tensor vec(const Tensor& s) {
 inline Tensor empty(at::IntArrayRef sz, const Tensor& like, at::ScalarType ty = at::kBFloat16) {
   return at::detail::empty_cuda(sz, ty, like.device(), std::nullopt);
 }
-// Results that are kept and dropped together, in one allocation (an allocation and its release cost the host 0.8 us, a tensor more on
-// the same storage 0.2; a layer step made seventy).  Each starts on a 256-byte boundary, none overlap.
+// Tensors that are kept and dropped together, in one allocation (an allocation and its release cost the host 0.8 us, a tensor more on
+// the same storage 0.2; a layer step made seventy).  Each starts on a 256-byte boundary, none overlap.  SHARED only for what no caller
+// gets hold of (the temporaries of a call, what the record of a layer step keeps): a tensor on a storage with others keeps them alive, is
+// written to a file with them and frees them when its storage is emptied, so whatever is handed out has a storage of its own.
+enum class Keep { OWN, SHARED };
 struct Want { at::DimVector sizes; at::ScalarType type; };
 template <size_t N>
-std::array<Tensor, N> together(const Tensor& like, const Want (&wants)[N]) {
+std::array<Tensor, N> together(const Tensor& like, const Want (&wants)[N], Keep keep = Keep::SHARED) {
+  if (keep == Keep::OWN) {
+    std::array<Tensor, N> out;
+    for (size_t i = 0; i < N; ++i) out[i] = empty(wants[i].sizes, like, wants[i].type);
+    return out;
+  }
   int64_t at[N], bytes = 0;
   for (size_t i = 0; i < N; ++i) {
     at[i] = bytes;
@@ -81,7 +89,8 @@ std::tuple<Tensor, OptTensor> quant(const Tensor& x, const Tensor& s, int64_t q_
                                     const OptTensor& out_q, const OptTensor& out_xo);
 Tensor dequant(const Tensor& q, const Tensor& s, int64_t q_bit, const OptTensor& z, const OptTensor& channel, const OptTensor& xo,
                const OptTensor& out);
-std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& row_cols = {});
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& row_cols = {},
+                                                                 Keep keep = Keep::OWN);
 void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& val, const Tensor& col, const Tensor& q,
                         const Tensor& s, const Tensor& z);
 Tensor topk_restore(const Tensor& val, const Tensor& col, const Tensor& q, const Tensor& s, const Tensor& z,
@@ -90,7 +99,7 @@ Tensor topk_softmax_backward(const Tensor& val, const Tensor& col, const Tensor&
                              at::IntArrayRef shape, int64_t q_bit, const Tensor& grad, const OptTensor& out, double scale);
 Tensor prune_sparse(const Tensor& x, double thr, const OptTensor& thr_dev);
 Tensor prune_restore(const Tensor& idx, const Tensor& val, int64_t numel);
-std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity, const Tensor& row_cols = {});
+std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity, const Tensor& row_cols = {}, Keep keep = Keep::OWN);
 Tensor prune_tiled_restore(const Tensor& words, const Tensor& directory, at::IntArrayRef shape, const OptTensor& out, const Tensor& row_cols = {});
 std::tuple<Tensor, Tensor, Tensor> silu_forward(const Tensor& xa1, const Tensor& b1, const Tensor& x1, const Tensor& s1,
                                                 const Tensor& xa2, const Tensor& b2, const Tensor& x2, const Tensor& s2, int64_t q_bit);
@@ -98,7 +107,7 @@ std::tuple<Tensor, Tensor, Tensor> silu_backward(const Tensor& xa1, const Tensor
                                                  const Tensor& xa2, const Tensor& b2, const Tensor& q2, const Tensor& s2,
                                                  const Tensor& grad_o, int64_t q_bit);
 std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor& x, const Tensor& w, double eps, int64_t q_bit,
-                                                                   const Tensor& sx, const OptTensor& idx, const OptTensor& sy);
+                                                                   const Tensor& sx, const OptTensor& idx, const OptTensor& sy, Keep keep = Keep::OWN);
 Tensor rmsnorm_backward_packed(const Tensor& dy, const Tensor& qx, const Tensor& sx, const OptTensor& xo, const OptTensor& idx,
                                const Tensor& w, const Tensor& rstd, int64_t q_bit, const OptTensor& res);
 Tensor softmax_backward(const Tensor& y, const Tensor& g, double scale);

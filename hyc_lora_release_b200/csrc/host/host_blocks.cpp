@@ -124,14 +124,14 @@ static const char* at_row(const Tensor& t, int64_t i) { return (const char*)t.da
 // the q, k and v projections with the saves of their main branches in one launch: -> {y, codes} of each
 static std::array<std::pair<Tensor, Tensor>, 3> qkv_lora_save(const Tensor& x, const std::vector<Weight>& w, const Tensor& xa3,
                                                               const std::array<const Tensor*, 3>& b, const std::array<const Tensor*, 3>& scale,
-                                                              int64_t q_bit, const Tensor& status) {
+                                                              int64_t q_bit, const Tensor& status, Keep keep_codes) {
   OnDevice on(x);
   const int64_t T = x.size(0), K = x.size(1);
   std::array<std::pair<Tensor, Tensor>, 3> out;
   const int64_t n0 = w[0].size(0), n1 = w[1].size(0), n2 = w[2].size(0);
   // (the projections themselves are gone behind the attention kernel, the codes stay for the backward pass)
   const auto y3 = together(x, {{{T, n0}, at::kBFloat16}, {{T, n1}, at::kBFloat16}, {{T, n2}, at::kBFloat16}});
-  const auto q3 = together(x, {{{T, n0 * q_bit / 8}, at::kByte}, {{T, n1 * q_bit / 8}, at::kByte}, {{T, n2 * q_bit / 8}, at::kByte}});
+  const auto q3 = together(x, {{{T, n0 * q_bit / 8}, at::kByte}, {{T, n1 * q_bit / 8}, at::kByte}, {{T, n2 * q_bit / 8}, at::kByte}}, keep_codes);
   Tensor keep[6];
   const void *wp[3], *xp[3], *bp[3], *sp[3];
   void *qp[3], *yp[3];
@@ -222,7 +222,7 @@ struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa,
 
 static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
                                        const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const std::vector<Weight>& gate_up,
-                                       const Weight* wd_now, const FrozenWeight* wd_later = nullptr) {
+                                       const Weight* wd_now, const FrozenWeight* wd_later, Keep keep) {
   const Weight &wg = gate_up[0], &wu = gate_up[1];
   const Tensor &norm_w = w[0], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
@@ -236,11 +236,11 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   SameDevice{x_medium}.with(w).with(wg.m).with(wu.m).with(stats).with(bias_d).with(status);
   OnDevice on(x_medium);
   const Tensor bg = factor(w[4]), bu = factor(w[5]);
-  auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale);
+  auto [x_norm, rstd, xm_o, xm_q, xn_q] = rmsnorm_save(x_medium, norm_w, eps, q, xm_scale, xm_idx, xn_scale, keep);
   const Tensor xn2 = x_norm.view({T, H});
   const Tensor gu_xa = lora_a_products(xn2, agu_t);
   const char* xa = (const char*)gu_xa.data_ptr();
-  const auto [q1, q2] = together(x_norm, {{{B, M, I * q / 8}, at::kByte}, {{B, M, I * q / 8}, at::kByte}});
+  const auto [q1, q2] = together(x_norm, {{{B, M, I * q / 8}, at::kByte}, {{B, M, I * q / 8}, at::kByte}}, keep);
   const Tensor had = empty({T, I}, x_norm);
   if (wg.f) {
     const hyc_nf4_weight codes[2] = {wg.codes(), wu.codes()};
@@ -388,7 +388,7 @@ using MapForward = std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Te
 // Left undefined where the rows are whole
 static MapForward attn_forward_map(const Tensor& x, const std::vector<Weight>& qkv, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const RopeTables& tables,
                                    const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& status,
-                                   Tensor* row_cols = nullptr) {
+                                   Keep keep, Tensor* row_cols = nullptr) {
   const Tensor &norm_w = w[0], &bq = w[1], &bk = w[2], &bv = w[3], &aqkv_t = w[4];
   const Tensor &x_idx = stats[0], &x_scale = stats[1], &xn_scale = stats[2], &q_scale = stats[3], &k_scale = stats[4], &v_scale = stats[5];
   check_geometry({qkv[0].size(0), qkv[1].size(0), qkv[2].size(0)}, nh, d, nkv);
@@ -402,10 +402,10 @@ static MapForward attn_forward_map(const Tensor& x, const std::vector<Weight>& q
   SameDevice{x}.with(w).with(stats).with(tables.cos).with(tables.sin).with(mask).with(status);
   OnDevice on(x);
   const int64_t B = x.size(0), M = x.size(1), H = x.size(2), T = B * M, rep = nh / nkv;
-  auto [x_norm, rstd, x_o, x_q, xn_q] = rmsnorm_save(x, norm_w, eps, q, x_scale, x_idx, xn_scale);
+  auto [x_norm, rstd, x_o, x_q, xn_q] = rmsnorm_save(x, norm_w, eps, q, x_scale, x_idx, xn_scale, keep);
   const Tensor xn2 = x_norm.view({T, H});
   const Tensor xa3 = lora_a_products(xn2, aqkv_t);
-  auto p3 = qkv_lora_save(xn2, qkv, xa3, {&bq, &bk, &bv}, {&q_scale, &k_scale, &v_scale}, q, status);
+  auto p3 = qkv_lora_save(xn2, qkv, xa3, {&bq, &bk, &bv}, {&q_scale, &k_scale, &v_scale}, q, status, keep);
   const auto &[qy, q_q] = p3[0];
   const auto &[ky, k_q] = p3[1];
   const auto &[vy, v_q] = p3[2];
@@ -480,7 +480,7 @@ static std::vector<Tensor> attn_backward_out(const Tensor& g, const Weight& wo, 
 static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, const std::vector<Tensor>& topk, int64_t map_q_bit,
                                                 const std::vector<Tensor>& saved, const std::vector<Tensor>& w, const RopeTables& tables,
                                                 int64_t B, int64_t M, int64_t nh, int64_t d, int64_t nkv, int64_t q,
-                                                const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status) {
+                                                const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& status, Keep keep) {
   const Tensor &q_q = saved[0], &q_s = saved[1], &q_xa = saved[2], &k_q = saved[3], &k_s = saved[4], &k_xa = saved[5], &v_q = saved[6],
                &v_s = saved[7], &v_xa = saved[8];
   check_geometry({w[0].size(0), w[1].size(0), w[2].size(0)}, nh, d, nkv);
@@ -492,20 +492,20 @@ static std::vector<Tensor> attn_backward_map(const Tensor& grad_o2, Tensor a, co
   if (attn_kernels_take(M, d)) {
     // q, k (rotated) and v from their codes in one launch
     const auto rebuilt = together(grad_o2, {{{T, nh * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}});
-    Tensor keep[9];
+    Tensor held[9];
     const void *cp[3], *sp[3], *xp[3], *bp[3];
     void* yp[3];
     int n[3];
     for (int i = 0; i < 3; ++i) {
       n[i] = (int)((i == 0 ? nh : nkv) * d);
-      cp[i] = data(keep[3 * i] = saved[3 * i].contiguous()); sp[i] = data(keep[3 * i + 1] = vec(saved[3 * i + 1]));
-      xp[i] = data(saved[3 * i + 2]); bp[i] = data(keep[3 * i + 2] = factor(w[i])); yp[i] = data(rebuilt[i]);
+      cp[i] = data(held[3 * i] = saved[3 * i].contiguous()); sp[i] = data(held[3 * i + 1] = vec(saved[3 * i + 1]));
+      xp[i] = data(saved[3 * i + 2]); bp[i] = data(held[3 * i + 2] = factor(w[i])); yp[i] = data(rebuilt[i]);
     }
     check(hyc_rebuild_qkv(cp, sp, xp, bp, yp, n, data(tables.cos), data(tables.sin), tables.cos.stride(0), tables.f32(), T, (int)M, (int)q, on.stream),
           "hyc_rebuild_qkv");
     const Tensor &q2 = rebuilt[0], &k2 = rebuilt[1], &v2 = rebuilt[2];
     Tensor gs = empty({B, nh, M, M}, grad_o2);
-    const auto [gq, gk, gv] = together(grad_o2, {{{T, nh * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}});
+    const auto [gq, gk, gv] = together(grad_o2, {{{T, nh * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}, {{T, nkv * d}, at::kBFloat16}}, keep);
     check(hyc_attn_bwd_tcgen05(data(q2), data(k2), data(v2), data(grad_o2), data(a), data(gs), (int)B, (int)M, (int)nh, (int)nkv, (int)d,
                                (float)scale, data(cls), cls_b, cls_h, data(gq), data(gk), data(gv), status_ptr(status), on.stream),
           "hyc_attn_bwd_tcgen05");
@@ -698,13 +698,13 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
     const bool cols = s->M > 128 && (map_q == 0 ? s->M % 256 == 0 : hyc_softmax_topk_cols_supported((int)s->M, (int)map_k) == 1);
     std::tie(a, o2, s->rstd, s->x_o, s->x_q, s->xn_q, s->q_q, s->k_q, s->v_q, s->xa3, o_codes, s->cls, s->cls_b, s->cls_h) = attn_forward_map(
         x, w, {p.norm1, p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1], p.pad[AQKV_T]},
-        {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status, cols ? &s->row_cols : nullptr);
+        {st[X_IDX], st[X_SCALE], st[XN1_SCALE], st[Q_SCALE], st[K_SCALE], st[V_SCALE], st[O_SCALE]}, s->tables, mask, nh, d, nkv, q_attn, eps, status, Keep::SHARED, cols ? &s->row_cols : nullptr);
     w.clear();
     if (map_q > 0) {
-      auto [val, col, q, sc, z] = topk_compress(a, map_k, map_q, s->row_cols);
+      auto [val, col, q, sc, z] = topk_compress(a, map_k, map_q, s->row_cols, Keep::SHARED);
       s->map = {val, col, q, sc, z};
     } else {
-      auto [words, directory, nnz] = prune_tiled(a, threshold, capacity, s->row_cols);
+      auto [words, directory, nnz] = prune_tiled(a, threshold, capacity, s->row_cols, Keep::SHARED);
       s->map = {words, directory, nnz};
     }
     a.reset();
@@ -714,7 +714,7 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
   std::vector<Weight> w = weights({&p.w[PGATE], &p.w[PUP]}, s->B * s->M, Use::BOTH);
   s->mlp = mlp_forward(x_medium, {p.norm2, Tensor(), Tensor(), Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
                                   p.pad[AGU_T], p.pad[AD_COLS], p.pad[BD_COLS]},
-                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, w, nullptr, &p.w[PDOWN]);
+                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, w, nullptr, &p.w[PDOWN], Keep::SHARED);
   Tensor y = std::move(s->mlp.x_out);
   s->mlp.x_out = Tensor();
   return {y.to(s->x_type), s};
@@ -775,7 +775,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
     grads = attn_backward_map(r[2], std::move(a), topk ? s.map : std::vector<Tensor>(), s.map_q,
                               {s.q_q, st[Q_SCALE], s.xa3.select(0, 0), s.k_q, st[K_SCALE], s.xa3.select(0, 1), s.v_q, st[V_SCALE], s.xa3.select(0, 2)},
                               {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.tables, s.B, s.M, s.nh, s.d, s.nkv, s.q_attn,
-                              s.cls, s.cls_b, s.cls_h, status);
+                              s.cls, s.cls_b, s.cls_h, status, Keep::SHARED);
     if (!topk)
       check(hyc_prune_overflow_flag((const int64_t*)data(s.map[2]), s.map[0].numel(), (int*)data(overflow), on.stream), "hyc_prune_overflow_flag");
   }
@@ -793,7 +793,7 @@ void bind_blocks(pybind11::module_& m) {
   m.def("mlp_forward", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const OptTensor& bias_d, int64_t q,
                           double eps, const Tensor& st) {
     const Weight wd(w[3]);
-    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st, {Weight(w[1]), Weight(w[2])}, &wd);
+    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st, {Weight(w[1]), Weight(w[2])}, &wd, nullptr, Keep::OWN);
     return std::vector<Tensor>{f.x_out, f.rstd, f.xm_o, f.xm_q, f.xn_q, f.q1, f.q2, f.gs, f.us, f.gu_xa, f.down_xa64}; });
   m.def("mlp_backward_lora", [](const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q, const Tensor& st) {
     return mlp_backward_lora(g, w[0], w, saved, q, st); });
@@ -801,7 +801,7 @@ void bind_blocks(pybind11::module_& m) {
                              std::vector<int64_t> shape, int64_t q, const Tensor& st) { return mlp_backward_x(g, ggu, gm64, {Weight(w[0]), Weight(w[1])}, {w[2], w[3]}, saved, shape, q, st); });
   m.def("attn_forward_map", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const Tensor& cos, const Tensor& sin,
                                const OptTensor& mask, int64_t nh, int64_t d, int64_t nkv, int64_t q, double eps, const Tensor& st) {
-    return attn_forward_map(x, {Weight(w[1]), Weight(w[2]), Weight(w[3])}, {w[0], w[4], w[5], w[6], w[7]}, stats, rope_tables(cos, sin, x.size(1), d), mask, nh, d, nkv, q, eps, st); });
+    return attn_forward_map(x, {Weight(w[1]), Weight(w[2]), Weight(w[3])}, {w[0], w[4], w[5], w[6], w[7]}, stats, rope_tables(cos, sin, x.size(1), d), mask, nh, d, nkv, q, eps, st, Keep::OWN); });
   m.def("attn_forward_out", [](const Tensor& x, const Tensor& o2, const Tensor& wo, const Tensor& ao_cols, const Tensor& bo_cols, const Tensor& o_scale,
                                const OptTensor& o_codes, const OptTensor& bias_o, int64_t q, const Tensor& st) {
     return attn_forward_out(x, o2, wo, ao_cols, bo_cols, o_scale, o_codes, bias_o, q, st); });
@@ -811,7 +811,7 @@ void bind_blocks(pybind11::module_& m) {
   m.def("attn_backward_map", [](const Tensor& grad_o2, const Tensor& a, const std::vector<Tensor>& topk, int64_t map_q_bit, const std::vector<Tensor>& saved,
                                 const std::vector<Tensor>& w, const Tensor& cos, const Tensor& sin, int64_t B, int64_t M, int64_t nh, int64_t d,
                                 int64_t nkv, int64_t q, const OptTensor& cls, int64_t cls_b, int64_t cls_h, const Tensor& st) {
-    return attn_backward_map(grad_o2, a, topk, map_q_bit, saved, w, rope_tables(cos, sin, M, d), B, M, nh, d, nkv, q, cls, cls_b, cls_h, st); });
+    return attn_backward_map(grad_o2, a, topk, map_q_bit, saved, w, rope_tables(cos, sin, M, d), B, M, nh, d, nkv, q, cls, cls_b, cls_h, st, Keep::OWN); });
   m.def("attn_backward_lora", &attn_backward_lora);
   m.def("attn_backward_x", [](const Tensor& g, const std::vector<Tensor>& grads, const Tensor& gmq, const std::vector<Tensor>& w,
                               const std::vector<Tensor>& saved, std::vector<int64_t> shape, int64_t q, const Tensor& st) {

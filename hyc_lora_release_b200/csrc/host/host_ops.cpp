@@ -123,12 +123,12 @@ void topk_compress_into(const Tensor& x, int64_t k, int64_t q_bit, const Tensor&
                                   data(s), (int8_t*)data(z), (int)q_bit, on.stream), "hyc_softmax_topk_compress");
 }
 
-std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& row_cols) {
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> topk_compress(const Tensor& x, int64_t k, int64_t q_bit, const Tensor& row_cols, Keep keep) {
   const int64_t S = row_length(x), rows = x.numel() / S;
   require_cuda({&x});
   check_q(q_bit);
   const auto [q, val, col, s, z] = together(x, {{{rows, S * q_bit / 8}, at::kByte}, {{rows, k}, at::kBFloat16}, {{rows, k}, at::kShort},
-                                                {{rows, S / 64}, at::kBFloat16}, {{rows, S / 64}, at::kChar}});
+                                                {{rows, S / 64}, at::kBFloat16}, {{rows, S / 64}, at::kChar}}, keep);
   if (row_cols.defined()) {
     OnDevice on(x);
     check(hyc_softmax_topk_compress_cols(data(x), rows, (int)S, (const uint16_t*)data(row_cols), (int)k, k ? data(val) : nullptr,
@@ -216,13 +216,13 @@ Tensor prune_restore(const Tensor& idx_in, const Tensor& val_in, int64_t numel) 
   return out;
 }
 
-std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity, const Tensor& row_cols) {
+std::tuple<Tensor, Tensor, Tensor> prune_tiled(const Tensor& x, double thr, int64_t capacity, const Tensor& row_cols, Keep keep) {
   require_cuda({&x});
   OnDevice on(x);
   const Tensor xf = bf16c(x);
   const int64_t numel = xf.numel();
   const auto [dir, nnz, words] = together(x, {{{(int64_t)(hyc_softmax_prune_tiled_directory_bytes(numel) / 4)}, at::kInt}, {{1}, at::kLong},
-                                              {{capacity}, at::kInt}});
+                                              {{capacity}, at::kInt}}, keep);
   if (row_cols.defined())
     check(hyc_softmax_prune_tiled_cols(data(xf), numel, (int)x.size(-1), (const uint16_t*)data(row_cols), (float)thr, (uint32_t*)data(words), capacity,
                                        data(dir), (int64_t*)data(nnz), on.stream), "hyc_softmax_prune_tiled_cols");
@@ -306,7 +306,7 @@ Tensor dequant_lora_add(const Tensor& q, const Tensor& s, const Tensor& xa, cons
 
 // ---- norms, softmax, rotary embedding
 std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor& x, const Tensor& w_in, double eps, int64_t q_bit,
-                                                                   const Tensor& sx_in, const OptTensor& idx_in, const OptTensor& sy_in) {
+                                                                   const Tensor& sx_in, const OptTensor& idx_in, const OptTensor& sy_in, Keep keep) {
   const int64_t N = row_length(x), rows = x.numel() / N;
   require_cuda({&x, &w_in, &sx_in});
   check_q(q_bit);
@@ -322,7 +322,8 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, OptTensor> rmsnorm_save(const Tensor&
   qs.back() = N * q_bit / 8;
   os.back() = k;
   const Tensor y = empty(xc.sizes(), x);
-  const auto [rstd, qx, xo, codes_y] = together(x, {{{rows}, at::kFloat}, {qs, at::kByte}, {os, at::kBFloat16}, {sy.defined() ? qs : none, at::kByte}});
+  const auto [rstd, qx, xo, codes_y] = together(x, {{{rows}, at::kFloat}, {qs, at::kByte}, {os, at::kBFloat16}, {sy.defined() ? qs : none, at::kByte}},
+                                                    keep);
   OptTensor qy;
   if (sy.defined()) qy = codes_y;
   if (rows)
@@ -427,7 +428,8 @@ void bind_ops(pybind11::module_& m) {
   m.def("silu_forward", &silu_forward);
   m.def("silu_backward", &silu_backward);
   m.def("dequant_lora_add", &dequant_lora_add);
-  m.def("rmsnorm_save", &rmsnorm_save);
+  m.def("rmsnorm_save", [](const Tensor& x, const Tensor& w, double eps, int64_t q_bit, const Tensor& sx, const OptTensor& idx, const OptTensor& sy) {
+    return rmsnorm_save(x, w, eps, q_bit, sx, idx, sy); });
   m.def("rmsnorm_backward_packed", &rmsnorm_backward_packed);
   m.def("softmax_backward", &softmax_backward);
   m.def("softmax_forward", &softmax_forward);
