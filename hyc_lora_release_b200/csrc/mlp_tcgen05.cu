@@ -726,6 +726,12 @@ static FourView four_view(const hyc_nf4_weight& w, int64_t cols) {
           w.absmax ? 0 : shift_of(w.blocksize2), w.offset};
 }
 static bool has_four(const hyc_nf4_weight* w, int i) { return w != nullptr && w[i].packed != nullptr; }
+// (a product whose operands are all bf16 is its namesake's, with any number of rows)
+static bool any_four(const hyc_nf4_weight* w, int count) {
+  for (int i = 0; i < count; ++i)
+    if (has_four(w, i)) return true;
+  return false;
+}
 
 extern "C" HYC_API int hyc_nf4_product_supported(const hyc_nf4_weight* w, int rows, int cols) { return w && four_takes(*w, rows, cols) ? 1 : 0; }
 
@@ -797,7 +803,7 @@ static int gemm_segments(int count, const void* const* A, const void* const* B, 
   p.status = status;
   p.g_end0 = p.g_end1 = N;
   cudaStream_t st = (cudaStream_t)stream;
-  const FourWeights* f4 = B4 ? &four : nullptr;
+  const FourWeights* f4 = any_four(B4, count) ? &four : nullptr;
   return b_is_kn ? launch<EPI_STORE, 4, true>(ops, p, st, f4) : launch<EPI_STORE, 4, false>(ops, p, st, f4);
 }
 extern "C" HYC_API int hyc_gemm_segments_tcgen05(int count, const void* const* A, const void* const* B, const int* K, int M, int N,
@@ -977,7 +983,7 @@ static int linears_lora_save(
     *g[i - 1] = {(__nv_bfloat16*)y[i], (uint8_t*)q_out[i], (const __nv_bfloat16*)scale[i], make_term(xa[i], bt[i], 16, 1)};
   p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
-  const FourWeights* f4 = w4 ? &four : nullptr;
+  const FourWeights* f4 = any_four(w4, count) ? &four : nullptr;
   if (q_bit == 2) return launch<EPI_STORE, 2, false>(ops, p, st, f4);
   if (q_bit == 4) return launch<EPI_STORE, 4, false>(ops, p, st, f4);
   return launch<EPI_STORE, 8, false>(ops, p, st, f4);

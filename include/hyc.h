@@ -325,7 +325,9 @@ int hyc_dequant_nf4_many(int count, const hyc_nf4_job* jobs, void* stream);
 
 /* A weight [rows, cols] in that form as an operand: products of up to 128 rows (hyc_nf4_product_supported: cols % 64 == 0, block sizes
  * powers of two, at least 64 elements under a scale, packed 32-byte aligned) decode it on its way in.  The *_nf4_tcgen05 entries are
- * their namesakes without the suffix, with the same results for the same weights; where `packed` is NULL the bf16 matrix counts. */
+ * their namesakes without the suffix, with the same results for the same weights.  An entry of hyc_gemm_segments_nf4_tcgen05 and
+ * hyc_linears_lora_save_fwd_nf4_tcgen05 whose `packed` is NULL takes the bf16 matrix instead (rows: any number if all do); the weights of the
+ * other two are codes. */
 typedef struct hyc_nf4_weight {
   const void* packed;
   const float *code16, *absmax;      /* absmax NULL: double quantization */

@@ -108,3 +108,32 @@ def test_projections(T, q):
 
     assert all(torch.equal(a, b) for a, b in zip(graddown(True), graddown(False)))
     assert int(st.item()) == 0
+
+
+@pytest.mark.parametrize("T", [1, 128, 129, 300])
+def test_no_codes(T):
+    """Operands that are all bf16: the namesake's result, at any number of rows; a weight of codes behind 128 rows is refused."""
+    from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
+    g = torch.Generator().manual_seed(T)
+    rn = lambda *s: torch.randn(*s, generator=g).to(BF16).to(DEV)
+    K, N, q = 192, 256, 4
+    st, kk = torch.zeros(1, dtype=torch.int32, device=DEV), (ctypes.c_int * 2)(K, 64)
+    a, b, out = [rn(T, K), rn(T, 64)], [rn(N, K), rn(N, 64)], [torch.full((T, N), float("nan"), dtype=BF16, device=DEV) for _ in range(2)]
+    stream = stream_of(out[0])
+    check(lib.hyc_gemm_segments_tcgen05(2, _ptrs(a), _ptrs(b), kk, T, N, 0, None, ptr(out[0]), ptr(st), stream), "bf16")
+    check(lib.hyc_gemm_segments_nf4_tcgen05(2, _ptrs(a), _ptrs(b), (Codes * 2)(), kk, T, N, 0, None, ptr(out[1]), ptr(st), stream), "nf4")
+    assert torch.equal(*out)
+    xa, bt, sc = [rn(T, 16) for _ in b], [rn(N, 16) for _ in b], [rn(N).abs() + 0.1 for _ in b]
+    w = [b[0], rn(N, K)]
+
+    def linears(f, *codes):
+        qo, y = [torch.empty(T, N * q // 8, dtype=torch.uint8, device=DEV) for _ in w], [torch.empty(T, N, dtype=BF16, device=DEV) for _ in w]
+        check(f(ptr(a[0]), T, K, 2, _ptrs(w), *codes, (ctypes.c_int * 2)(N, N), _ptrs(xa), _ptrs(bt), _ptrs(sc), _ptrs(qo), _ptrs(y), q, ptr(st), stream), "linears")
+        return qo + y
+
+    assert all(torch.equal(x, y) for x, y in zip(linears(lib.hyc_linears_lora_save_fwd_tcgen05), linears(lib.hyc_linears_lora_save_fwd_nf4_tcgen05, (Codes * 2)())))
+    if T > 128:
+        w4 = _weight(g, N, K, 64, False)
+        coded = (Codes * 2)(w4[0], Codes())
+        assert lib.hyc_gemm_segments_nf4_tcgen05(2, _ptrs(a), _ptrs([None, b[1]]), coded, kk, T, N, 0, None, ptr(out[1]), ptr(st), stream) != 0
+    assert int(st.item()) == 0
