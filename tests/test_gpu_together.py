@@ -61,7 +61,7 @@ def test_halves_own_what_they_return():
     from hyc_lora_release_b200.mlp import MLPState, MLPWeights, mlp_forward
     from test_gpu_layer import _attn_weights, layer_problem
     g = torch.Generator().manual_seed(5)
-    B, M, heads, d, kv, I = 1, 128, 2, 128, 1, 512
+    B, M, heads, d, kv, I = 1, 128, 4, 128, 2, 512
     x, p, cos, sin, mask = layer_problem(g, B, M, heads * d, heads, d, kv, I)
     x, cos, sin, mask = (t.to(DEV) for t in (x, cos, sin, mask))
     t = lambda n: p[n].t().contiguous().to(DEV)
