@@ -25,7 +25,7 @@
 // scheduler, waits on tensor memory and loads in between; DRAM at 21 and 49 %), the kv kernel its loads (two 32 KB tiles per
 // product; issue slots 0.07, DRAM 59 %).  The tensor pipe is busy a quarter of the time in all three.  Measured
 // [1,32,2048,2048] causal, cold: forward 106 us with the ends of the rows and 122 with the whole map, for 512 MB of map traffic saved;
-// backward 171 (105.5 + 65.4 as single launches); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
+// backward 105.5 + 65.2 as single launches (the two between a pair of events: 179); the separate steps took 110 + 104 + 107 us (products, softmax) and 330 us.
 #include "tc_common.cuh"
 #include <math.h>
 
@@ -765,11 +765,16 @@ __device__ __forceinline__ int kv_item(int round) {
   return round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
 }
 
-// Persistent where that gives a block two items and more: the loads of the next item run while the gradients of this one leave, which is
-// why each item has accumulators of its own (dV and dK, two sets).  [1,32,2048,2048] causal, cold, 512 blocks of one item each / 148 of three
-// or four: 72.4 / 65.4 us.  Both backward kernels, us before / now: 191.5 / 177.1, [4,32,1024,1024] 246.8 / 226.3 (with 8 key/value heads,
-// 256 blocks of one item: 195.6 / 193.5), [2,32,696,696] 80.9 / 74.8, [1,32,2048,2048] with an open mask 356 / 321.  Below two items per
-// SM the fixed shares cost what the overlap gives ([4,32,512,512], 8 key/value heads, 128 items: 78.8 / 80.7 with them).
+// MANY: a block per SM and more items than blocks: the loads of the next item run while the gradients of this one leave, which is
+// why each item has accumulators of its own (dV and dK, two sets).  Without it a block has one item; a list of one would cost 0.1 to 0.5 us
+// of its fixed share.  Single launches, cold, us, a block per item / MANY: [1,32,2048,2048] causal, 512 items 73.5 / 65.2; 160 items
+// [5,32,128,128] 14.7 / 12.9; 192 [3,32,256,256] 16.1 / 14.2; 256 [1,32,1024,1024] 25.2 / 23.0; 288 [1,32,1152,1152] 28.9 / 26.3.  Items of
+// four heads each (8 key/value heads) keep their loads under way by themselves: 160 [5,32,512,512] 52.6 / 50.7 without a mask, 192 causal 35.5 / 35.1,
+// 256 [4,32,1024,1024] 68.4 / 68.5, 256 [8,32,512,512] causal 46.2 / 48.1, 288 without a mask 75.5 / 75.6.
+// Both backward kernels between a pair of events, four slots and a block per item / six slots and this: [1,32,2048,2048] causal 193 / 179, [4,32,1024,1024]
+// 250 / 232 (with 8 key/value heads 198 / 196), [2,32,696,696] 83.0 / 75.9, [1,32,2048,2048] without a mask 349 / 318, [3,32,256,256] 35.8 / 35.1;
+// short rows with 8 key/value heads lose by the q kernel's slots: [4,32,512,512] 101.6 / 103.2 without a mask (the q kernel 60.0 / 61.4), 79.8 / 80.3 causal.
+template <bool MANY>
 __global__ void __launch_bounds__(KV_THREADS, 1)
 attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -777,6 +782,12 @@ attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
   const Bars bar(smem + KV_BARS);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rep = p.heads / p.kv_heads, items = p.tiles * p.B * p.kv_heads;
+  // -1: there are no more of them
+  auto item_of = [&](int round) {
+    if (!MANY) return round == 0 ? (int)blockIdx.x : -1;
+    const int item = kv_item(round);
+    return item < items ? item : -1;
+  };
   at_begin(bar, warp, KV_WARPS);
   const uint32_t tmem = at_ready(bar);
   const uint32_t ring = smem_u32(smem);
@@ -785,17 +796,17 @@ attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
   if (warp == 0) {
     bool ok = true;
     RingPos pos;
-    int item = kv_item(0);
-    uint32_t next = 0u;
-    if (item < items) { const KvItem w(p, item); next = live_query_tiles(p, w.b, w.kvh * rep, w.kt, lane); }
-    for (int round = 0; item < items && ok; ++round) {
+    int item = item_of(0);
+    const KvItem first(p, item);
+    uint32_t next = live_query_tiles(p, first.b, first.kvh * rep, first.kt, lane);
+    for (int round = 0; item >= 0 && ok; ++round) {
       const KvItem w(p, item);
       const uint32_t live = next;
-      item = kv_item(round + 1);
+      item = item_of(round + 1);
       bool asked = false;
       // the classes of the next item are looked up while the first tiles of this one are on their way
       auto ask = [&]() {
-        if (!asked && item < items) { const KvItem n(p, item); next = live_query_tiles(p, n.b, n.kvh * rep, n.kt, lane); }
+        if (!asked && item >= 0) { const KvItem n(p, item); next = live_query_tiles(p, n.b, n.kvh * rep, n.kt, lane); }
         asked = true;
       };
       for (int g = 0; g < rep && ok; ++g) {
@@ -815,7 +826,7 @@ attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
     RingPos pos;
     bool ok = true;
     int used = 0;                                   // items with products so far
-    for (int round = 0, item; (item = kv_item(round)) < items && ok; ++round) {
+    for (int round = 0, item; (item = item_of(round)) >= 0 && ok; ++round) {
       const KvItem w(p, item);
       const int steps = 2 * rep * __popc(live_query_tiles(p, w.b, w.kvh * rep, w.kt, lane));      // dV from P and dO, dK from dS and Q
       if (steps == 0) continue;
@@ -848,7 +859,7 @@ attn_bwd_kv_kernel(const __grid_constant__ BwdKvMaps maps, const AttnParams p) {
     const int64_t ld = (int64_t)p.kv_heads * TILE;
     bool fine = true;
     int used = 0;
-    for (int round = 0, item; (item = kv_item(round)) < items && fine; ++round) {
+    for (int round = 0, item; (item = item_of(round)) >= 0 && fine; ++round) {
       const KvItem w(p, item);
       // keys that no query row attends to get zero gradients
       const bool any = live_query_tiles(p, w.b, w.kvh * rep, w.kt, lane) != 0u;
@@ -997,16 +1008,18 @@ extern "C" HYC_API int hyc_attn_bwd_tcgen05(
   if (cls && !(cls_h != 0 && heads != kv_heads)) { p.cls = (const TileClass*)cls; p.cls_b = cls_b; p.cls_h = cls_h; }
   p.status = status;
   cudaStream_t st = (cudaStream_t)stream;
-  static bool done_q[64] = {false}, done_kv[64] = {false};
+  static bool done_q[64] = {false}, done_kv[2][64] = {};
   if (const int rc = at_prepare(attn_bwd_q_kernel, Q_SMEM, done_q)) return rc;
-  if (const int rc = at_prepare(attn_bwd_kv_kernel, KV_SMEM, done_kv)) return rc;
+  if (const int rc = at_prepare(attn_bwd_kv_kernel<false>, KV_SMEM, done_kv[0])) return rc;
+  if (const int rc = at_prepare(attn_bwd_kv_kernel<true>, KV_SMEM, done_kv[1])) return rc;
   p.out0 = (__nv_bfloat16*)grad_q; p.map = (__nv_bfloat16*)grad_s;
   launch_pdl(attn_bwd_q_kernel, dim3((unsigned)(p.tiles * B * heads)), dim3(AT_THREADS), Q_SMEM, st, mq, p);
   HYC_CHECK_LAUNCH();
   p.out0 = (__nv_bfloat16*)grad_k; p.out1 = (__nv_bfloat16*)grad_v;
-  // fewer than two items per SM: a block each (measured at the kernel)
+  // up to an item per SM: a block each (measured at the kernel)
   const int items = p.tiles * B * kv_heads, sms = num_sms();
-  launch_pdl(attn_bwd_kv_kernel, dim3((unsigned)(items < 2 * sms ? items : sms)), dim3(KV_THREADS), KV_SMEM, st, mk, p);
+  if (items <= sms) launch_pdl(attn_bwd_kv_kernel<false>, dim3((unsigned)items), dim3(KV_THREADS), KV_SMEM, st, mk, p);
+  else launch_pdl(attn_bwd_kv_kernel<true>, dim3((unsigned)sms), dim3(KV_THREADS), KV_SMEM, st, mk, p);
   HYC_CHECK_LAUNCH();
   return HYC_OK;
 }

@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 DEV, BF16 = "cuda", torch.bfloat16
 
 
-@pytest.mark.parametrize("B,M,h,kv", [(5, 264, 40, 40), (7, 384, 32, 16), (3, 128, 148, 148)])
+@pytest.mark.parametrize("B,M,h,kv", [(5, 264, 40, 40), (7, 384, 32, 16), (3, 128, 148, 148), (2, 200, 40, 40), (2, 128, 149, 149)])
 @pytest.mark.parametrize("form", ["none", "causal", "dead keys"])
 def test_items(B, M, h, kv, form):
     from hyc_lora_release_b200._lib import check, lib, ptr, stream_of
