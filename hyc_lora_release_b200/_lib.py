@@ -80,6 +80,7 @@ SIGNATURES = {
     "hyc_gemm_segments_tcgen05": (_i, [_i, _p, _p, _p, _i, _i, _i, _p, _p, _p, _p]),
     "hyc_gemm_segments_nf4_tcgen05": (_i, [_i, _p, _p, _p, _p, _i, _i, _i, _p, _p, _p, _p]),
     "hyc_nf4_product_supported": (_i, [_p, _i, _i]),
+    "hyc_nf4_product_pays": (_i, [_i, _i, _i, _i, _i]),
     "hyc_skinny_workspace_bytes": (_z, [_i, _p, _i]),
     "hyc_skinny_products": (_i, [_i, _p, _i, _p, _z, _p, _p]),
     "hyc_attn_mask_class_bytes": (_z, [_i, _i, _i]),

@@ -2,7 +2,6 @@
 // What each step is and which rounding points it has is documented in mlp.py and attention.py, which own the
 // calibration branch and the weight records.
 #include "host.h"
-#include <ATen/cuda/CUDAContext.h>
 #include <algorithm>
 #include <array>
 #include <climits>
@@ -190,26 +189,32 @@ static std::vector<Tensor> matrices(std::initializer_list<const FrozenWeight*> w
   return out;
 }
 
-// The same for a product of T rows: the codes as they are where it takes them (BOTH: where it takes all of them).
-// WHOLE: a product whose K is not split has a CTA per 128 outputs, and each decodes at a rate of its own (0.65 us for 64 x 128
-// elements): on less than half of the SMs a launch of all of them is faster.  us for 128 rows, de-quantizing and product / decoded inside:
-// q, k and v of 4096 (96 CTAs) 55 / 54, o of 4096 (32) 33 / 46; split or wide enough anyway: gate and up of 11008 85 / 77, down 48 / 35,
-// backward of down 50 / 47, grad_x of gate and up 79 / 56, grad_o 26 / 21, grad_x of q, k and v 51 / 37.
-enum class Use { ANY, BOTH, WHOLE };
-static std::vector<Weight> weights(std::initializer_list<const FrozenWeight*> ws, int64_t T, Use use = Use::ANY) {
-  size_t coded = 0;
-  int64_t outputs = 0;
+// The same for a product of T rows: the codes as they are where it takes them (gate and up: where it takes both) and is faster for it
+// (the rule and its figures: tc_split.cu).  recorded: the product becomes part of a capture.
+enum class Use { QKV, O, GATE_UP, DOWN, GRAD_DOWN, GRAD_X };
+static std::vector<Weight> weights(std::initializer_list<const FrozenWeight*> ws, int64_t T, Use use, bool recorded) {
+  const bool backward = use == Use::GRAD_DOWN || use == Use::GRAD_X;
+  bool coded = false, refused = T > INT_MAX;
+  int64_t sum0 = 0, rows = 0, cols = 0;
   for (const FrozenWeight* f : ws) {
-    outputs += f->plain.defined() ? f->plain.size(0) : f->shape[0];
-    if (f->plain.defined()) continue;
+    const at::IntArrayRef shape = f->plain.defined() ? f->plain.sizes() : at::IntArrayRef(f->shape);
+    if (shape.size() != 2) { refused = true; break; }
+    sum0 += rows = shape[0];
+    cols = shape[1];
+    if (f->plain.defined()) { refused = refused || use == Use::GATE_UP; continue; }
     const hyc_nf4_weight c = f->codes();
-    if (f->shape.size() == 2 && hyc_nf4_product_supported(&c, (int)std::min<int64_t>(T, INT_MAX), (int)f->shape[1])) ++coded;
-    else coded = ws.size() + 1;
-    if (coded > ws.size()) break;
+    coded = true;
+    refused = refused || !hyc_nf4_product_supported(&c, (int)T, (int)cols);
+    if (refused) break;
   }
-  if (coded > 0 && use == Use::WHOLE && outputs / 128 * 2 < at::cuda::getCurrentDeviceProperties()->multiProcessorCount) coded = 0;
+  if (coded && !refused) {
+    // outputs side by side and depth (64: the LoRA products that ride along)
+    const int kind = use == Use::GATE_UP ? HYC_NF4_GATE_UP : (use == Use::GRAD_DOWN ? HYC_NF4_GRAD_DOWN : (use == Use::QKV || use == Use::O ? HYC_GEMM_FIXED_ORDER : 0));
+    const int64_t n = backward ? cols : (use == Use::GATE_UP ? rows : sum0), k = (backward ? sum0 : cols) + (use == Use::QKV || use == Use::GATE_UP ? 0 : 64);
+    refused = !hyc_nf4_product_pays(kind, (int)T, (int)std::min<int64_t>(n, INT_MAX), (int)std::min<int64_t>(k, INT_MAX), recorded);
+  }
   std::vector<Weight> out;
-  if (coded == 0 || coded > ws.size() || (use == Use::BOTH && coded < ws.size())) {
+  if (!coded || refused) {
     for (const Tensor& m : matrices(ws)) out.emplace_back(m);
   } else {
     for (const FrozenWeight* f : ws) f->plain.defined() ? out.emplace_back(f->plain) : out.emplace_back(f);
@@ -222,7 +227,7 @@ struct MlpForward { Tensor x_out, rstd, xm_o, xm_q, xn_q, q1, q2, gs, us, gu_xa,
 
 static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>& w, const std::vector<Tensor>& stats,
                                        const OptTensor& bias_d, int64_t q, double eps, const Tensor& status, const std::vector<Weight>& gate_up,
-                                       const Weight* wd_now, const FrozenWeight* wd_later, Keep keep) {
+                                       const Weight* wd_now, const FrozenWeight* wd_later, bool recorded, Keep keep) {
   const Weight &wg = gate_up[0], &wu = gate_up[1];
   const Tensor &norm_w = w[0], &agu_t = w[6], &ad_cols = w[7], &bd_cols = w[8];
   const Tensor &xm_idx = stats[0], &xm_scale = stats[1], &xn_scale = stats[2];
@@ -254,7 +259,7 @@ static MlpForward mlp_forward(const Tensor& x_medium, const std::vector<Tensor>&
   }
   const Tensor down_xa64 = at::mm(had, ad_cols);
   const Tensor res = bf16c(x_medium);
-  const Weight wd = wd_later ? weights({wd_later}, T)[0] : *wd_now;
+  const Weight wd = wd_later ? weights({wd_later}, T, Use::DOWN, recorded)[0] : *wd_now;
   if (!wd.f) require_cuda({&x_medium, &wd.m});
   expect(wd, H, I, x_medium, "down projection");
   Tensor x_out = gemm({{&had, wd}, {&down_xa64, bd_cols}}, 0, &res, status);
@@ -616,7 +621,7 @@ struct LayerPlan {
   OptTensor bias_o, bias_d;
   std::vector<Tensor> pad;                      // what AttnWeights.padded / MLPWeights.padded make of the LoRA factors
   Stamp pad_of[2 * PROJECTIONS];
-  int64_t pad_capture = 0;
+  int64_t pad_capture = 0;                      // where it is fresh: the capture that the calls are recorded into, 0 if they run
   std::vector<Tensor> stats_in, stats;          // calibrated statistics as given, and as the kernels read them
   std::vector<Stamp> stats_of;
 
@@ -687,11 +692,12 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
   s->stats = st;
   s->x_type = x_in.scalar_type();
   s->tables = rope_tables(cos, sin, s->M, d);
+  const bool recorded = p.pad_capture != 0;
   Tensor x_medium;
   {
     Tensor a, o2;
     OptTensor o_codes;
-    std::vector<Weight> w = weights({&p.w[PQ], &p.w[PK], &p.w[PV]}, s->B * s->M, Use::WHOLE);
+    std::vector<Weight> w = weights({&p.w[PQ], &p.w[PK], &p.w[PV]}, s->B * s->M, Use::QKV, recorded);
     // where the save and the restore know how to leave out what the mask rules out (tiles of 128 columns: not in maps of one tile).
     // us of the attention kernel, save and restore without / with, 5 % kept: causal [4,32,1024,1024] top-k 364 / 300, pruned 254 / 231,
     // [4,32,256,256] 41 / 40 and 42 / 41; a mask that rules out nothing, which is not known here, 396 / 392 and 304 / 308
@@ -708,13 +714,13 @@ static std::pair<Tensor, std::shared_ptr<LayerSaved>> layer_forward(LayerPlan& p
       s->map = {words, directory, nnz};
     }
     a.reset();
-    auto out = attn_forward_out(x, o2, weights({&p.w[PO]}, s->B * s->M, Use::WHOLE)[0], p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
+    auto out = attn_forward_out(x, o2, weights({&p.w[PO]}, s->B * s->M, Use::O, recorded)[0], p.pad[AO_COLS], p.pad[BO_COLS], st[O_SCALE], o_codes, p.bias_o, q_attn, status);
     x_medium = out[0]; s->o_q = out[1]; s->o_xa64 = out[2];
   }
-  std::vector<Weight> w = weights({&p.w[PGATE], &p.w[PUP]}, s->B * s->M, Use::BOTH);
+  std::vector<Weight> w = weights({&p.w[PGATE], &p.w[PUP]}, s->B * s->M, Use::GATE_UP, recorded);
   s->mlp = mlp_forward(x_medium, {p.norm2, Tensor(), Tensor(), Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1],
                                   p.pad[AGU_T], p.pad[AD_COLS], p.pad[BD_COLS]},
-                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, w, nullptr, &p.w[PDOWN], Keep::SHARED);
+                       {st[XM_IDX], st[XM_SCALE], st[XN2_SCALE], st[GATE_SCALE], st[UP_SCALE]}, p.bias_d, q_mlp, eps, status, w, nullptr, &p.w[PDOWN], recorded, Keep::SHARED);
   Tensor y = std::move(s->mlp.x_out);
   s->mlp.x_out = Tensor();
   return {y.to(s->x_type), s};
@@ -730,6 +736,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   const std::vector<Tensor>& st = s.stats;
   const int64_t T = s.B * s.M;
   const std::vector<int64_t> shape = {s.B, s.M, s.H};
+  const bool recorded = p.pad_capture != 0;
   require_cuda({&grad_y, &s.rstd});
   OnDevice on(s.rstd);
   std::vector<Tensor> out(1 + 2 * PROJECTIONS);
@@ -749,14 +756,14 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   {
     const Tensor g = bf16c(grad_y).view({T, s.H});
     const MlpForward& m = s.mlp;
-    auto r = mlp_backward_lora(g, weights({&p.w[PDOWN]}, T)[0], {Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
+    auto r = mlp_backward_lora(g, weights({&p.w[PDOWN]}, T, Use::GRAD_DOWN, recorded)[0], {Tensor(), p.lora[2 * PGATE + 1], p.lora[2 * PUP + 1], p.lora[2 * PDOWN + 1], p.pad[AD_ROWS]},
                                {m.q1, m.gs, m.q2, m.us, m.gu_xa, m.down_xa64, m.xn_q, st[XN2_SCALE]}, s.q_mlp, status);
     lora(PGATE, r[5].narrow(0, 0, 16), r[6].select(0, 0));
     lora(PUP, r[5].narrow(0, 16, 16), r[6].select(0, 1));
     lora(PDOWN, r[4], r[3]);
     report({{"g", PGATE}, {"u", PUP}, {"d", PDOWN}});
     r[0].reset();
-    g_medium = mlp_backward_x(g, r[1], r[2], weights({&p.w[PGATE], &p.w[PUP]}, T), {p.pad[AGU_ROWS], p.norm2},
+    g_medium = mlp_backward_x(g, r[1], r[2], weights({&p.w[PGATE], &p.w[PUP]}, T, Use::GRAD_X, recorded), {p.pad[AGU_ROWS], p.norm2},
                               {m.xm_q, st[XM_SCALE], m.xm_o, st[XM_IDX], m.rstd}, shape, s.q_mlp, status).view({T, s.H});
   }
   if (!hook.is_none() && !p.fresh()) {           // the hook of the MLP half changed factors of this one
@@ -766,7 +773,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   }
   std::vector<Tensor> grads;
   {
-    auto r = attn_backward_out(g_medium, weights({&p.w[PO]}, T)[0], p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
+    auto r = attn_backward_out(g_medium, weights({&p.w[PO]}, T, Use::GRAD_X, recorded)[0], p.lora[2 * PO + 1], p.pad[AO_ROWS], s.o_xa64, s.o_q, st[O_SCALE], s.q_attn, status);
     lora(PO, r[1], r[0]);
     const std::vector<int64_t> a_shape = {s.B, s.nh, s.M, s.M};
     const bool topk = s.map_q > 0;
@@ -782,7 +789,7 @@ static std::vector<Tensor> layer_backward(const LayerPlan& p, const Tensor& grad
   auto r = attn_backward_lora(grads, {p.lora[2 * PQ + 1], p.lora[2 * PK + 1], p.lora[2 * PV + 1]}, s.xa3, s.xn_q, st[XN1_SCALE], s.q_attn, status);
   for (int i = 0; i < 3; ++i) lora(PQ + i, r[1].narrow(0, 16 * i, 16), r[2 + i]);
   report({{"q", PQ}, {"k", PK}, {"v", PV}, {"o", PO}});
-  out[0] = attn_backward_x(g_medium, grads, r[0], weights({&p.w[PQ], &p.w[PK], &p.w[PV]}, T), {p.pad[AQKV_ROWS], p.norm1},
+  out[0] = attn_backward_x(g_medium, grads, r[0], weights({&p.w[PQ], &p.w[PK], &p.w[PV]}, T, Use::GRAD_X, recorded), {p.pad[AQKV_ROWS], p.norm1},
                            {s.x_q, st[X_SCALE], s.x_o, st[X_IDX], s.rstd}, shape, s.q_attn, status).to(s.x_type);
   return out;
 }
@@ -793,7 +800,7 @@ void bind_blocks(pybind11::module_& m) {
   m.def("mlp_forward", [](const Tensor& x, const std::vector<Tensor>& w, const std::vector<Tensor>& stats, const OptTensor& bias_d, int64_t q,
                           double eps, const Tensor& st) {
     const Weight wd(w[3]);
-    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st, {Weight(w[1]), Weight(w[2])}, &wd, nullptr, Keep::OWN);
+    MlpForward f = mlp_forward(x, w, stats, bias_d, q, eps, st, {Weight(w[1]), Weight(w[2])}, &wd, nullptr, false, Keep::OWN);
     return std::vector<Tensor>{f.x_out, f.rstd, f.xm_o, f.xm_q, f.xn_q, f.q1, f.q2, f.gs, f.us, f.gu_xa, f.down_xa64}; });
   m.def("mlp_backward_lora", [](const Tensor& g, const std::vector<Tensor>& w, const std::vector<Tensor>& saved, int64_t q, const Tensor& st) {
     return mlp_backward_lora(g, w[0], w, saved, q, st); });

@@ -734,6 +734,13 @@ static bool any_four(const hyc_nf4_weight* w, int count) {
 }
 
 extern "C" HYC_API int hyc_nf4_product_supported(const hyc_nf4_weight* w, int rows, int cols) { return w && four_takes(*w, rows, cols) ? 1 : 0; }
+extern "C" HYC_API int hyc_nf4_product_pays(int kind, int rows, int n, int k, int recorded) {
+  if (rows < 1 || rows > BM || n < 1 || k < 1) return 0;
+  Params p = {};
+  p.M = rows; p.N = n; p.K1 = k;
+  p.fixed_order = kind == HYC_GEMM_FIXED_ORDER;
+  return four_pays(kind == HYC_NF4_GATE_UP ? EPI_GATEUP : (kind == HYC_NF4_GRAD_DOWN ? EPI_GRADDOWN : EPI_STORE), p, recorded != 0) ? 1 : 0;
+}
 
 extern "C" HYC_API int hyc_gemm_bf16_tcgen05(
     const void* A, const void* B, int M, int N, int K, int form,

@@ -446,6 +446,27 @@ int launch_split(int epi, int q_bit, bool b_mn, const SplitPlan& plan, const Ope
   return launch_one<EPI_STORE, 4, false, false>(plan.split, ops, p, st);
 }
 
+// The codes of a CTA's share are decoded at a rate of its own (0.65 us for 64 x 128 elements), so a product on few SMs waits for that, while
+// a launch that de-quantizes them uses all.  By the CTAs that the product gets, for 128 rows, us with that launch / decoded inside (cold,
+// the launches between a pair of events):
+//   K in one CTA: o of 4096 (32 CTAs) 34 / 48; q, k and v of 3072 (72) 38 / 50, of 3328 (78) 42 / 51, of 5120 + 2 x 2560 (80) 61 / 66, of 3584
+//     (84) 46 / 54, of 4096 (96) 56 / 59 (one row: 57 / 56), of 5120 (120) 79 / 67; gate and up of 2048 x 5632 (88) 30 / 33, of 2048 x 6400 (100)
+//     32 / 33, of 2048 x 8192 (128) 36 / 32, of 4096 x 11008 (172) 92 / 80: five eighths of the SMs.  (K of 8192 and more would pay from 64 on.)
+//   K shared by the CTAs of a cluster, and the backward product of down, whose kernel for bf16 weights is the persistent one: down of 2048 x 5632 (64)
+//     25.6 / 27.6, of 2560 x 6912 (80) 29.9 / 30.7, of 3072 x 8192 (96) 34.2 / 33.2, of 4096 x 11008 (128) 48 / 40, of 5120 x 13824 (80) 79 / 70; grad_o of
+//     2048 (32) 21.5 / 23.6, of 5120 (80) 36 / 37, of 4096 (128) 27.6 / 25.6; grad_x of gate and up of 2048 x 8192 (64) 44 / 46, of 2560 x 6912 (80) 44 / 43;
+//     backward of down, 4096 x 8192 (64) 46.0 / 47.5, 4096 x 9728 (76) 49.9 / 48.6, 4096 x 11008 (86) 54 / 48: half of the SMs.
+// Without a capture the host has the launch and the allocation to make as well (5 us), and a layer of so few rows waits for the host up to
+// widths of 4096 (500 us a step): there only what loses more than that, the products with a fixed order on less than half of the SMs, is
+// de-quantized first.  Layer steps of 128 rows, us, by the first lines / by this one: launched 1024 wide 516 to 542 / 485, 2048 520 to 540 / 442 to 500, 3072
+// 498 to 523 / 490 to 503; replayed 1024 248 / 274, 2048 331 / 331, 3072 405 / 408.
+bool four_pays(int epi, const Params& p, bool recorded) {
+  const int split = choose_split(epi, p).split;
+  const int ctas = p.N / (epi == EPI_GATEUP ? SBN / 2 : SBN) * (split > 0 ? split : 1);
+  if (!recorded) return !p.fixed_order || 2 * ctas >= num_sms();
+  return epi == EPI_GRADDOWN || split > 1 ? 2 * ctas >= num_sms() : 8 * ctas >= 5 * num_sms();
+}
+
 // the split that a product of up to 128 rows has either way: the same sums for a weight as for its codes
 int launch_four(int epi, int q_bit, bool b_mn, const Operands& ops, const Params& p, const FourWeights& four, cudaStream_t st) {
   if (p.M > BM) return HYC_ERR_UNSUPPORTED;

@@ -18,6 +18,7 @@ struct FourView {
   float offset;
 };
 struct FourWeights { FourView w[4]; };      // as the B operands: K segments or weights side by side
+bool four_pays(int epi, const Params& p, bool recorded);
 int launch_four(int epi, int q_bit, bool b_mn, const Operands& ops, const Params& p, const FourWeights& four, cudaStream_t st);
 
 struct SplitPlan { int split; bool pair; };

@@ -337,6 +337,13 @@ typedef struct hyc_nf4_weight {
   float offset;
 } hyc_nf4_weight;
 int hyc_nf4_product_supported(const hyc_nf4_weight* w, int rows, int cols);
+/* 1 where the product is faster so than after a launch that de-quantizes its weights, by how much of the current device it fills (both sides
+ * measured at the rule, tc_split.cu).  recorded: 1 for a launch that a capture records, 0 for one that the host makes each time, whose
+ * cost counts then.  kind: HYC_GEMM_FIXED_ORDER or 0 for hyc_gemm_segments_nf4_tcgen05 with and without it (with it also
+ * hyc_linears_lora_save_fwd_nf4_tcgen05), or one of these; n: outputs of all weights side by side, k: K of all segments. */
+#define HYC_NF4_GATE_UP 16
+#define HYC_NF4_GRAD_DOWN 32
+int hyc_nf4_product_pays(int kind, int rows, int n, int k, int recorded);
 
 /* ---- tcgen05 / TMEM GEMMs of the LoRA MLP (activation compression in the epilogue) ------------
  * bf16 operands, fp32 accumulation in tensor memory, operands staged by TMA.  `status` is a

@@ -63,7 +63,8 @@ def test_dequantizer_matches_the_format_statement(shape, blocksize, nested):
 @pytest.mark.gpu
 def test_layer_with_4bit_frozen_weights():
     """The layer module with 4-bit frozen weights gives bit for bit what it gives with the de-quantized matrices
-    (the same kernels run on the same values), and it does not keep the bf16 matrices between the passes."""
+    (of 256 rows: a launch de-quantizes them, the same kernels run on the same values), and it does not keep the bf16 matrices between
+    the passes."""
     from hyc_lora_release_b200 import nf4
     from hyc_lora_release_b200.layer import FusedLlamaLayerIntraInterFullFuse
     from test_gpu_layer import layer_problem, _Holder, _base
@@ -124,3 +125,90 @@ def test_layer_with_4bit_frozen_weights():
     aw, mw, _ = layer4._weights[1:]
     assert isinstance(aw.wq, nf4.QuantizedWeight) and isinstance(mw.wd, nf4.QuantizedWeight)
     assert "_pad" in vars(aw) and "_pad" in vars(mw)          # the scratch of the passes came back to the records
+
+
+# which of a layer's products (q k v, o, gate and up, down, their backward products) decode their weights on the way in, by the SMs they fill
+PRODUCTS = ("qkv", "o", "gateup", "down", "graddown", "gradx gu", "grado", "gradx qkv")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,M,heads,kv,I,inside", [
+    (1, 128, 4, 2, 1024, ()), (1, 128, 32, 32, 11008, set(PRODUCTS) - {"o"}), (3, 40, 32, 32, 11008, set(PRODUCTS) - {"o"}),
+    (1, 64, 24, 8, 9472, {"gateup", "down", "graddown", "gradx gu", "gradx qkv"}), (1, 64, 38, 2, 11008, set(PRODUCTS) - {"qkv", "o"})])
+@pytest.mark.parametrize("coded,nested", [("q k v o gate up down", ""), ("q k v o gate up down", "q k v o gate up down"), ("q v gate down", "v down"), ("k o up", "k")])
+def test_short_layers_with_4bit_frozen_weights(B, M, heads, kv, I, inside, coded, nested):
+    """Up to 128 rows the products of a calibrated layer decode their weights where that pays, called and in a capture (``inside``): bit for bit
+    the layer with the de-quantized matrices, with one- and two-level scales and with some projections plain (gate and up then count as
+    matrices in the forward pass)."""
+    from hyc_lora_release_b200 import nf4
+    from hyc_lora_release_b200._lib import lib
+    from hyc_lora_release_b200.layer import FusedLlamaLayerIntraInterFullFuse
+    from test_gpu_layer import _Holder, _base
+    d, R = 128, 16
+    H, D, Dkv, T = heads * d, heads * d, kv * d, B * M
+    g = torch.Generator(device="cuda").manual_seed(H + T + len(coded))
+    rn = lambda *s, scale=1.0: (torch.randn(*s, generator=g, device="cuda") * scale).to(BF16)
+    fixed, gate_up, down = 2, 16, 32
+    want = {"qkv": (fixed, D + 2 * Dkv, H), "o": (fixed, H, D + 64), "gateup": (gate_up, I, H), "down": (0, H, I + 64), "graddown": (down, I, H + 64),
+            "gradx gu": (0, H, 2 * I + 64), "grado": (0, D, H + 64), "gradx qkv": (0, H, D + 2 * Dkv + 64)}
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert {n for n in PRODUCTS if lib.hyc_nf4_product_pays(want[n][0], T, *want[n][1:], 1)} == set(inside)
+        assert {n for n in PRODUCTS if lib.hyc_nf4_product_pays(want[n][0], T, *want[n][1:], 0)} == set(inside) | set(PRODUCTS) - {"qkv", "o"}
+    shapes = dict(q=(D, H), k=(Dkv, H), v=(Dkv, H), o=(H, D), gate=(I, H), up=(I, H), down=(H, I))
+    table = onf4.normal_float_table().cuda()
+    base4, base16, lora = {}, {}, {}
+    for n, (rows, cols) in shapes.items():
+        num = rows * cols
+        qs = types.SimpleNamespace(shape=(rows, cols), code=table, blocksize=64, dtype=BF16, nested=n in nested.split())
+        if qs.nested:
+            qs.absmax = torch.randint(0, 256, (num // 64,), generator=g, dtype=torch.uint8, device="cuda")
+            qs.state2 = types.SimpleNamespace(code=torch.linspace(0, 1, 256), blocksize=256, absmax=(torch.rand((num // 64 + 255) // 256, generator=g, device="cuda") + 0.5) * 0.03)
+            qs.offset = 0.01
+        else:
+            qs.absmax = (torch.rand(num // 64, generator=g, device="cuda") + 0.5) * 0.03
+        packed = torch.nn.Parameter(torch.randint(0, 256, (num // 2, 1), generator=g, dtype=torch.uint8, device="cuda"), requires_grad=False)
+        packed.quant_state = qs
+        base16[n] = _base(nf4.dequantize_nf4(packed))
+        base4[n] = base16[n]
+        if n in coded.split():
+            base4[n] = torch.nn.Module()
+            base4[n].weight, base4[n].bias = packed, None
+        lora[n] = _Holder(rn(R, cols, scale=cols ** -0.5)), _Holder(rn(rows, R, scale=0.05))
+    norms = [torch.nn.Parameter(1 + rn(H, scale=0.1), requires_grad=False) for _ in range(2)]
+    fr = torch.outer(torch.arange(M, dtype=torch.float32), 1.0 / (10000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d)))
+    emb = torch.cat([fr, fr], dim=-1)
+    cos, sin = emb.cos().to(BF16).cuda(), emb.sin().to(BF16).cuda()
+    mask = torch.full((M, M), torch.finfo(BF16).min).triu(1).to(BF16).reshape(1, 1, M, M).cuda()
+    x, gy = rn(B, M, H), rn(B, M, H)
+
+    def run(base):
+        layer = FusedLlamaLayerIntraInterFullFuse()
+        layer.set_hyclora_config(types.SimpleNamespace(use_hyclora=True, iteration_threshold=1, softmax_outlier_ratio=0.05, layernorm_outlier_ratio=0.01,
+                                                       q_bit=4, softmax_map_mode="prune"))
+        layer.attn_state.prune_capacity_margin = 4.0      # (few batches for the 64 lists of the saved map: they fill unevenly)
+        factors = [h.default.weight for n in lora for h in lora[n]]
+        xin = x.clone().requires_grad_(True)
+
+        def step():
+            args = [xin, norms[0], None, cos, sin]
+            for n in shapes:
+                args += ([norms[1], None] if n == "gate" else []) + [base[n], *lora[n]]
+            y = layer(*args, mask, heads, d, kv)
+            return [y, *torch.autograd.grad(y, [xin] + factors, gy)]
+
+        outs = [[t.detach().clone() for t in step()] for _ in range(3)]
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            step()
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                kept = step()
+        graph.replay()
+        torch.cuda.synchronize()
+        layer.raise_on_device_errors()
+        return outs + [[t.detach().clone() for t in kept]]
+
+    for a, b in zip(run(base4), run(base16)):
+        assert all(bool(torch.isfinite(t).all()) for t in a) and all(torch.equal(s, t) for s, t in zip(a, b))
