@@ -15,9 +15,10 @@
 // 128-byte row (32 bytes of codes under one scale): the sixteen values that a scale makes of the table as byte planes in registers, then
 // byte permutes (3.7 instructions per element).  Bound by instructions (issue slots 0.37, two and a half warps per scheduler) and by the
 // requests for codes and scales, 32 and 4 bytes per thread from rows of their own: 0.65 us per k-block, 0.59 without the arithmetic, 0.42
-// without the requests.  The products of a layer of 128 tokens that take codes, us: 395 as de-quantizing launches and products, 328 so; the layer
-// 577 -> 517 to 538 (its host work takes about as long).  More codes in flight (cp.async, eight slots), sixteen warps, and addresses carried
-// from block to block gave nothing or cost some.  Which products: see weights() in host/host_blocks.cpp.
+// without the requests.  The launch bound (two CTAs of 320 threads per SM, which only gate and up of a wide MLP fill) leaves 96 registers per
+// thread: the store forms spill 192 bytes per thread, gate/up about 400, grad_down up to 36.  The products of a layer of 128 tokens that take
+// codes, us: 395 as de-quantizing launches and products, 328 so; the layer step 577 -> 507 (its host work takes about as long).  More codes in
+// flight (cp.async, eight slots), sixteen warps, and addresses carried from block to block gave nothing or cost some.  Which products: four_pays().
 #include "tc_split.cuh"
 
 namespace hyc {
@@ -490,8 +491,8 @@ int launch_four(int epi, int q_bit, bool b_mn, const Operands& ops, const Params
 
 // Where the line lies (B200, Llama-2-7B weights, us per product, persistent / split):
 //   up to 128 tokens, S = the largest of 4, 2, 1 with at most one CTA per SM: x[4096,11008] 42 / 26.5, grad_o 21.8 / 16.6,
-//     the three-segment grad_x 67 / 37; unsplit (S = 1) gate/up 48.9 / 43.8, q/k/v 38 / 33.  The grad_down product has
-//     more column tiles than SMs can take at once either way and stays persistent: 28.8 / 30.3
+//     the three-segment grad_x 67 / 37; unsplit (S = 1) gate/up 48.9 / 43.8, q/k/v 38 / 33.  The grad_down product (bf16
+//     weight; as codes it is decoded here) stays persistent: 28.8 / 30.3
 //   129 to 256 tokens, pair form, S = 2: 21.8 / 19.0, 43 / 30.6, 69 / 45; wider products fill the chip without it
 //   512 tokens: 45 / 47, 75 / 77: persistent
 //   (cold L2, each call with its own pair of events, which adds about 5 us: x[4096,11008] of 128 tokens 57 / 35, of 200 tokens

@@ -1,5 +1,6 @@
 """Products that decode their 4-bit weights on the way in: the same bits as de-quantizing first, at the edges of the row tile, with K
-shared by one, two and four CTAs, an odd number of k-blocks, one- and two-level scales, and next to operands that are bf16."""
+shared by one, two and four CTAs, an odd number of k-blocks, one- and two-level scales, and next to operands that are bf16.  (The C entries; a
+layer that takes them: test_nf4.py.)"""
 import ctypes
 
 import pytest
