@@ -54,7 +54,8 @@ inline Tensor empty(at::IntArrayRef sz, const Tensor& like, at::ScalarType ty = 
 // Tensors that are kept and dropped together, in one allocation (an allocation and its release cost the host 0.8 us, a tensor more on
 // the same storage 0.2; a layer step made seventy).  Each starts on a 256-byte boundary, none overlap.  SHARED only for what no caller
 // gets hold of (the temporaries of a call, what the record of a layer step keeps): a tensor on a storage with others keeps them alive, is
-// written to a file with them and frees them when its storage is emptied, so whatever is handed out has a storage of its own.
+// written to a file with them and frees them when its storage is emptied, so whatever is handed out has a storage of its own (which costs
+// a small call: top-k save and restore of [1,8,64,64] 12.8 us, 10.5 with one storage; the norm with its saves 7.3, 5.7).
 enum class Keep { OWN, SHARED };
 struct Want { at::DimVector sizes; at::ScalarType type; };
 template <size_t N>

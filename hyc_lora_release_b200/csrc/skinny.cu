@@ -3,7 +3,7 @@
 //
 // The backward pass needs both forms of every gradient (g B for the input's gradient, g^T xa for B's).  Each is bound by
 // reading X; as library calls they read it twice, and each call costs the host 10 us.  One call for grad_gate, grad_up and
-// hadamard of 2048 tokens (three X of [2048, 11008], 135 MB from HBM): 37 us with its sums, 31 of them the first kernel's,
+// hadamard of 2048 tokens (three X of [2048, 11008], 135 MB from HBM): 39 us with its sums, 33 of them the first kernel's,
 // which is then at 52 % of the DRAM rate (issue slots 7 %: it waits for its tiles).
 //
 // A CTA owns a region of R x C tiles of 128 x 128 of one X.  A tile arrives by TMA (128-byte swizzle) and is the A operand

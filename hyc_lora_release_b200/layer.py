@@ -9,7 +9,8 @@ attention mask and the head geometry.  Differences, all deliberate:
 
   * frozen weights are plain bf16 ``[out, in]`` matrices, or 4-bit block-wise weights in the storage format of
     bitsandbytes (packed codes with a ``quant_state``), de-quantized to bf16 for each pass by a kernel of this
-    package (``nf4.py``; the library itself is not part of this build, parity with it is unpinned);
+    package, or by the products themselves where a calibrated step has up to 128 rows (``nf4.py``; the library itself is not
+    part of this build, parity with it is unpinned);
   * projection biases of q/k/v/o/down are added to the main branch (separate launches for such a projection);
     gate/up biases are refused (the reference's fused layer drops them);
   * ``hyclora_config.softmax_map_mode`` (optional, default ``"prune"`` = the reference's threshold prune) may
